@@ -20,6 +20,9 @@ LIB_PATH = Path(os.environ.get("DELTARULE_SM100_LIB", _PKG / "libdeltarule_sm100
 # the same sources with the index checks compiled in (-DDR_BOUNDS_CHECK); tests load it through DELTARULE_SM100_LIB
 BOUNDS_LIB_PATH = _PKG / "libdeltarule_sm100_bounds.so"
 _SOURCES = ["dr_api.cu", "dr_scans.cu"]   # translation units, compiled side by side
+# the native host path of the public calls (argument checks, allocation, C-ABI call): a CPython extension over torch
+HOST_PATH = _PKG / "_host_calls.so"
+_HOST_SOURCE = _PKG / "csrc" / "host_calls.cpp"
 _HEADERS = sorted(f.name for f in list((_PKG / "csrc").glob("*.cuh")) + list((_PKG / "csrc").glob("*.h")))
 
 # DrVariant / DrDtype / DrLayout / DrChunkPath (include/deltarule_sm100.h)
@@ -126,8 +129,33 @@ def build_library(force: bool = False, verbose: bool = False, bounds: bool = Fal
     return target
 
 
+def build_host_calls(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the CPython extension of the native host path (g++ against torch's headers)."""
+    deps = [_HOST_SOURCE, _ROOT / "include" / "deltarule_sm100.h"]
+    if not force and HOST_PATH.exists() and all(d.stat().st_mtime <= HOST_PATH.stat().st_mtime for d in deps):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", "/usr/local/cuda/include",
+           sysconfig.get_paths()["include"], _ROOT / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f"-I{i}" for i in inc]
+    cmd += ["-o", str(HOST_PATH), str(_HOST_SOURCE), f"-L{root / 'lib'}"]
+    cmd += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode:
+        print(" ".join(cmd))
+        print(res.stdout, res.stderr)
+    if res.returncode:
+        raise RuntimeError("g++ failed building _host_calls.so:\n" + res.stderr)
+    return HOST_PATH
+
+
 _lib = None
-_lock = threading.Lock()
+_host = None
+_lock = threading.RLock()
 
 
 def load() -> ctypes.CDLL:
@@ -202,6 +230,22 @@ def load() -> ctypes.CDLL:
         lib.dr_debug_umma_selftest.argtypes = [vp, vp, fp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ip, vp]
         _lib = lib
     return _lib
+
+
+def host_calls():
+    """The native host path, bound to the kernel library (both loaded once)."""
+    global _host
+    if _host is None:
+        with _lock:
+            if _host is None:
+                load()
+                if not HOST_PATH.exists():
+                    raise ImportError(
+                        f"{HOST_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+                from . import _host_calls
+                _host_calls.open(str(LIB_PATH))
+                _host = _host_calls
+    return _host
 
 
 def check(status: int, where: str) -> None:

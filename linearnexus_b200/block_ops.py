@@ -20,6 +20,7 @@ import torch
 
 from . import _lib
 from ._lib import DR_BF16, DR_F32, DR_LAYOUT_BHTD, DR_LAYOUT_BTHD
+from .ops import _native_calls
 
 Tensor = torch.Tensor
 _NATIVE = {torch.float32: DR_F32, torch.bfloat16: DR_BF16}
@@ -50,6 +51,10 @@ def depthwise_conv1d_causal(inputs: Tensor, weight: Tensor, bias: Optional[Tenso
     """``inputs`` [B,T,C], ``weight`` [kernel,C], ``bias`` [C] or None, ``cache`` [B,kernel-1,C] or None.
     Returns ``(conv_output, new_cache)`` as the reference; ``activation="silu"`` fuses the SiLU.  ``cache_out``
     may name the tensor that receives the new cache (``cache`` itself for a decode step)."""
+    if activation in (None, "silu"):
+        r = _native_calls().conv(inputs, weight, bias, cache, activation is not None, cache_out)
+        if r.__class__ is tuple:
+            return r
     _cuda(inputs, weight, bias, cache, cache_out)
     if inputs.dim() != 3:
         raise ValueError("inputs must be [batch, seq, channels]")
@@ -94,6 +99,9 @@ def short_conv_silu(inputs, weight, bias=None, *, cache=None, cache_out=None):
 
 
 def _gates(mode, a, b, A_log, bias, H, K, beta_scale, threshold):
+    r = _native_calls().gates(mode, a, b, A_log, bias, H, K, beta_scale, threshold)
+    if r.__class__ is tuple:
+        return r
     a2 = _act(a)
     b2 = None if b is None else _act(b)
     dev = a2.device
@@ -136,6 +144,11 @@ def rmsnorm_gated(o: Tensor, weight: Tensor, gate: Optional[Tensor] = None, eps:
                   o_layout: str = "bhtd", out_dtype: Optional[torch.dtype] = None) -> Tensor:
     """``o`` as the op returns it ([B,H,T,V], or [B,T,H,V] with ``o_layout="bthd"``), ``gate`` [B,T,H,V] or None,
     ``weight`` [V] -> ``RMSNorm(o) * sigmoid(gate)`` as [B,T,H,V]."""
+    out_code = -1 if out_dtype is None else _NATIVE.get(out_dtype)
+    if out_code is not None and o_layout in ("bhtd", "bthd"):
+        r = _native_calls().norm(o, weight, gate, eps, o_layout == "bthd", out_code)
+        if r.__class__ is Tensor:
+            return r
     _cuda(o, weight, gate)
     if o_layout not in ("bhtd", "bthd") or o.dim() != 4:
         raise ValueError("o must be 4-d with o_layout 'bhtd' or 'bthd'")

@@ -51,6 +51,7 @@ def _status(dev) -> Tensor:
     t = _status_words.get(idx)
     if t is None:
         t = _status_words[idx] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
+        _lib.host_calls().set_status(idx, t.data_ptr())
     return t
 
 
@@ -111,8 +112,28 @@ def _desc(variant, layout, B, H, T, K, V, chunk, qkv, g, out_dtype, l2norm, scal
     return d
 
 
+# Every public call tries the native host path first (csrc/host_calls.cpp): it answers with the results when the tensors
+# are what the kernels read as they are, and with something else otherwise; the functions below then cast, copy, check
+# and raise.
+_host = None
+
+
+def _native_calls():
+    global _host
+    if _host is None:
+        _host = _lib.host_calls()
+    return _host
+
+
 def _seq_forward(kind, variant, q, k, v, g, beta, initial_state, scale, chunk_size, l2norm,
                  out_dtype, path=None):
+    out_code = _NATIVE.get(out_dtype)
+    if out_code is not None:
+        path_code = _PATHS.get(path if path is not None else default_chunk_path, -1)
+        r = _native_calls().sequence(kind != "chunk", variant, q, k, v, g, beta, initial_state, scale, chunk_size,
+                                     bool(l2norm), out_code, path_code)
+        if r.__class__ is tuple:
+            return r
     _require_cuda(q, k, v, g, beta, initial_state)
     if (q.dim() != 4 or k.shape != q.shape or v.dim() != 4 or v.shape[0] != q.shape[0] or v.shape[2] != q.shape[2]
             or v.shape[1] % q.shape[1]):
@@ -164,6 +185,9 @@ def _seq_forward(kind, variant, q, k, v, g, beta, initial_state, scale, chunk_si
 
 
 def _step(variant, q, k, v, g, beta, state, scale, l2norm, out_dtype, inplace=False):
+    r = _native_calls().step(variant, q, k, v, g, beta, state, scale, bool(l2norm), bool(inplace))
+    if r.__class__ is tuple:
+        return r
     _require_cuda(q, k, v, g, beta, state)
     if q.dim() != 3 or k.shape != q.shape or v.dim() != 3 or v.shape[0] != q.shape[0] or v.shape[1] % q.shape[1]:
         raise ValueError("expected q,k [B,Hq,K] and v [B,H,V] with H a multiple of Hq")

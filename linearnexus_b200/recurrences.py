@@ -13,7 +13,7 @@ import torch
 
 from . import _lib
 from ._lib import DR_LAYOUT_BHTD, DR_LAYOUT_BTHD
-from .ops import _NATIVE, _is_bthd_view, _native, _ptr, _require_cuda, _status, _stream
+from .ops import _NATIVE, _is_bthd_view, _native, _native_calls, _ptr, _require_cuda, _status, _stream
 
 Tensor = torch.Tensor
 
@@ -54,6 +54,10 @@ def dplr_delta_rule_recurrent(q: Tensor, k: Tensor, v: Tensor, a: Tensor, b: Ten
                               ) -> Tuple[Tensor, Tensor]:
     """``h <- exp(gk) h + b (a^T h) + k v^T;  o = h^T (q scale)`` over the tokens (rwkv7.py:114-214).
     q, k, a, b, gk ``[B,H,T,K]``, v ``[B,H,T,V]`` -> o ``[B,H,T,V]`` in q's dtype, final state float32 ``[B,H,K,V]``."""
+    if _out_state is None:
+        r = _native_calls().scan(0, q, k, v, a, b, gk, scale, initial_state)
+        if r.__class__ is tuple:
+            return r
     _require_cuda(q, k, v, a, b, gk, initial_state)
     if q.dim() != 4 or any(t.shape != q.shape for t in (k, a, b, gk)) or v.shape[:3] != q.shape[:3]:
         raise ValueError("expected q, k, a, b, gk [B,H,T,K] and v [B,H,T,V]")
@@ -92,6 +96,10 @@ def rwkv6_recurrent(r: Tensor, k: Tensor, v: Tensor, w: Tensor, u: Tensor, scale
                     initial_state: Optional[Tensor] = None, _out_state: Optional[Tensor] = None) -> Tuple[Tensor, Tensor]:
     """``o = (h + (u k) v^T)^T (sigmoid(r) scale);  h <- exp(-exp(w)) h + k v^T`` (rwkv6.py:115-189).
     r, k, w ``[B,H,T,K]``, v ``[B,H,T,V]``, u ``[H,K]`` -> o in r's dtype, final state float32."""
+    if _out_state is None:
+        res = _native_calls().scan(1, r, k, v, u, None, w, scale, initial_state)
+        if res.__class__ is tuple:
+            return res
     _require_cuda(r, k, v, w, u, initial_state)
     if r.dim() != 4 or k.shape != r.shape or w.shape != r.shape or v.shape[:3] != r.shape[:3]:
         raise ValueError("expected r, k, w [B,H,T,K] and v [B,H,T,V]")
@@ -149,6 +157,10 @@ def ssd_chunk_scan(hidden_states: Tensor, dt: Tensor, A: Tensor, B: Tensor, C: T
     the result (the reference's chunked evaluation equals this recurrence); ``dt_min`` / ``dt_max`` are unused
     there as well."""
     x = hidden_states
+    if _out_state is None:
+        r = _native_calls().ssd(x, dt, A, B, C, D, n_groups, ssm_state, dt_bias, dt_limit[0], min(dt_limit[1], 3.0e38))
+        if r.__class__ is tuple:
+            return r
     _require_cuda(x, dt, A, B, C, D, ssm_state, dt_bias)
     if x.dim() != 4 or dt.shape != x.shape[:3] or B.dim() != 4 or C.shape != B.shape or B.shape[:2] != x.shape[:2]:
         raise ValueError("expected hidden_states [B,T,H,P], dt [B,T,H], B and C [B,T,G,N]")

@@ -61,9 +61,17 @@ def chunkwise_varlen(variant: str, q: Tensor, k: Tensor, v: Tensor, g: Optional[
     one by one through the autograd-aware ops and the results are concatenated."""
     if variant not in _VAR:
         raise ValueError(f"unknown variant {variant!r}")
+    cu = cu_seqlens.tolist() if isinstance(cu_seqlens, Tensor) else list(cu_seqlens)
+    odt = out_dtype if out_dtype is not None else torch.float32 if variant == "kda" else q.dtype
+    if odt in ops._NATIVE:
+        l2 = variant != "delta" if use_qk_l2norm is None else bool(use_qk_l2norm)
+        r = ops._native_calls().packed(_VAR[variant], q, k, v, g, beta, cu, initial_state, scale, chunk_size, l2,
+                                       ops._NATIVE[odt])
+        if r.__class__ is tuple:
+            return r
     if (g is None) != (variant == "delta"):
         raise ValueError("g must be given for 'gated' / 'kda' and omitted for 'delta'")
-    cu = [int(c) for c in (cu_seqlens.tolist() if isinstance(cu_seqlens, Tensor) else cu_seqlens)]
+    cu = [int(c) for c in cu]
     n = len(cu) - 1
     if n < 1 or cu[0] != 0 or cu[-1] != q.shape[0] or any(b <= a for a, b in zip(cu, cu[1:])):
         raise ValueError("cu_seqlens must rise strictly from 0 to the number of packed tokens")
