@@ -1,9 +1,11 @@
 // C ABI of the delta-rule kernels: argument validation and dispatch.  No device memory is
 // allocated here; every launch goes to the caller's stream.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "deltarule_sm100.h"
 #include "deltarule_sm100_debug.h"
@@ -230,6 +232,45 @@ int dr_chunk_fwd_varlen(const DrDesc* d, const void* q, const void* k, const voi
   if (n_seqs < 1 || d->layout != DR_LAYOUT_BTHD || cu[0] != 0) return DR_ERR_SHAPE;
   for (int i = 0; i < n_seqs; ++i)
     if (cu[i + 1] <= cu[i]) return DR_ERR_SHAPE;   // offsets strictly increasing: no empty sequence
+  const int path = resolve_chunk_path(d);
+  if ((path == DR_PATH_TCGEN05 && tcgen05_eligible(d)) || (path == DR_PATH_SPLIT && split_eligible(d))) {
+    // the tensor-core forwards take many sequences per launch
+    DrDesc da = *d;
+    da.B = 1;
+    da.T = cu[n_seqs];
+    int s = validate_common(&da, true);
+    if (s != DR_OK) return s;
+    s = validate_fwd_ptrs(&da, q, k, v, g, beta, h0, o, hT);
+    if (s != DR_OK) return s;
+    const bool split = path == DR_PATH_SPLIT;
+    // records the workspace holds per head; at least the longest sequence's
+    int64_t cap = (int64_t)1 << 30;
+    if (split) {
+      if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
+      cap = workspace ? (int64_t)workspace_bytes / dr::kda::workspace_bytes(d->H, 64) : 0;
+    }
+    const dr::FwdParams p = make_fwd(&da, q, k, v, g, beta, h0, o, hT, status_dev);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    std::vector<int32_t> order(n_seqs);   // longest first
+    for (int i = 0; i < n_seqs; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return cu[x + 1] - cu[x] > cu[y + 1] - cu[y]; });
+    tl_path = split ? "chunk_split_tcgen05" : "chunk_tcgen05";
+    for (int i = 0; i < n_seqs;) {
+      dr::SeqTable t{};
+      for (; i < n_seqs && t.n < dr::kMaxSeqs; ++i) {
+        const int32_t j = order[i], len = cu[j + 1] - cu[j], chunks = (len + 63) / 64;
+        if (t.chunks + chunks > cap) break;
+        t.start[t.n] = cu[j]; t.len[t.n] = len; t.index[t.n] = j; t.first[t.n] = t.chunks;
+        t.chunks += chunks;
+        ++t.n;
+      }
+      if (t.n == 0) return DR_ERR_WORKSPACE;
+      g_launches.fetch_add(split ? 2 : 1);
+      const cudaError_t e = split ? dr::kda::launch_chunk_packed(p, t, workspace, st) : dr::sm100::launch_chunk_packed(p, t, st);
+      if (e != cudaSuccess) return check_cuda(e);
+    }
+    return DR_OK;
+  }
   const int Hq = d->qk_heads > 0 ? d->qk_heads : d->H;
   const size_t es = d->qkv_dtype == DR_BF16 ? 2 : 4, eo = d->out_dtype == DR_BF16 ? 2 : 4, eg = d->g_dtype == DR_BF16 ? 2 : 4;
   const size_t g_row = d->variant == DR_KDA ? (size_t)d->H * d->K : (size_t)d->H;

@@ -1349,7 +1349,7 @@ inline cudaError_t bwd_side_stream(cudaStream_t* out) {
 // The checkpointing forward of the backward: state at the start of every chunk -> the head of the workspace.
 // With o / hT given it is also the forward a training step needs (dr_chunk_fwd_saving), so that step runs one
 // forward instead of two.  KDA at the tensor-core shape uses the two-kernel forward with its records parked in the
-// accumulator part of the workspace (262 KB per chunk there against 82 KB of records; the adjoint overwrites it).
+// accumulator part of the workspace (262 KB per chunk there against 66 KB of records; the adjoint overwrites it).
 // own_stream: the pre-pass may run on the library's side stream, forked from and joined to `stream` with events
 // (false for callers that must not create streams or events: the pre-pass then runs on `stream` before the forward).
 inline cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,

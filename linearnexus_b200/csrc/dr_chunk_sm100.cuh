@@ -13,8 +13,8 @@
 // (5) sit on the serial chain.
 //
 //   PA (warps 0-3)   state-independent, chunk n:
-//     K,Q rows land by TMA as one [K;Q] tile already in core-matrix order (4-slot ring; the copy of chunk n+2 is
-//     issued as soon as chunk n-2 has left the consumer, before this group waits for chunk n+1's tile).
+//     K,Q rows land by TMA as one [K;Q] tile in the 128-byte swizzle (4-slot ring; the copy of chunk n+2 is issued as
+//     soon as chunk n-2 has left the consumer, before this group waits for chunk n+1's tile).
 //     The l2 norms are not applied to the tiles: they are folded into row and column factors (rk from the
 //     diagonal of D1, rq from the raw Q rows).
 //     (1) D1 = [K;Q] K^T                             128x64x128  smem x smem, issued one chunk ahead
@@ -37,8 +37,9 @@
 //     (5) S^T += (V_new^T e^{G_L-G_c}) K   (K read MN-major)                                128x128x64
 //     (4) Do = V_new^T A_qk^T                                                              128x64x64
 //
-// The [K;Q] tile is stored once as 8x8 core matrices and serves as A and B of (1), MN-major
-// A of (2), K-major B of Dq and MN-major B of (5).  Hand-overs are mbarriers (arrive counts of a whole
+// The [K;Q] tile is stored once (two 64-column panels of 128 rows x 128 bytes, swizzled) and serves as A and B of (1),
+// MN-major A of (2), K-major B of Dq and MN-major B of (5).  A panel is one TMA box of 128-byte rows: 64 box rows per
+// tile half where un-swizzled core matrices take 1024 rows of 16 bytes.  Hand-overs are mbarriers (arrive counts of a whole
 // group, or tcgen05.commit for product completion); every wait is bounded: a wait that runs out sets
 // DR_DEV_TIMEOUT in the status word (with the barrier and group that gave up) and the kernel finishes without
 // further waiting.  A wait site is one mbarrier.try_wait; the bounded loop, the abort flag and the record live in
@@ -49,6 +50,7 @@
 #include <cuda.h>
 
 #include <cstring>
+#include <type_traits>
 
 #include "dr_common.cuh"
 #include "dr_sm100_common.cuh"
@@ -74,13 +76,15 @@ constexpr uint32_t TM_COLS = 512;
 
 // shared-memory map (bytes)
 constexpr int QK_TILE = 128 * 128 * 2;        // [K (64 rows); Q (64 rows)] x 128 raw bf16, 32 KB
+constexpr int QK_PANEL = 128 * 128;           //   as two panels of 64 columns
+constexpr int V_PANEL = 64 * 128;             // V: the same with 64 rows
 constexpr int kRing = 4;                      // K,Q tiles in flight: one each in PA, PB, the consumer + one landing
 constexpr int SM_QKR = 0;                     // ring of kRing such tiles (chunk n uses tile n % kRing)
 constexpr int W_TILE = 128 * 64 * 2;          // W as [128 k][64 c] core matrices, 16 KB
 constexpr int SM_W = kRing * QK_TILE;         // one W tile
 constexpr int AQK_TILE = 64 * 64 * 2;         // A_qk [64][64] bf16, 8 KB
 constexpr int SM_AQK = SM_W + W_TILE;         // three A_qk tiles (chunk n uses n % 3)
-constexpr int SM_V = SM_AQK + 3 * AQK_TILE;   // V [64][128] core-matrix tile, 16 KB
+constexpr int SM_V = SM_AQK + 3 * AQK_TILE;   // V [64][128] tile, 16 KB
 constexpr int AKK_BYTES = 64 * LDT * 4;       // X, then T in place (fp32 [64][68]), then the bf16 tiles
 constexpr int SM_AKK = SM_V + 64 * 128 * 2;   // two such buffers (chunk n uses n & 1)
 constexpr int XB_TB = 0;                      //   T diag(beta rk)         [64][64] bf16 core-matrix tile, 8 KB
@@ -102,12 +106,17 @@ struct alignas(16) Ctl {
                                      // was padding, the block is as large as without it
 };
 
-// Kernel parameters: the common forward parameters plus the TMA tensor maps (see make_input_map /
-// make_output_map); the map coordinates of a sequence are derived from (b, h) in the kernel.
+// Kernel parameters: the common forward parameters plus the TMA tensor maps (see make_panel_map); the map coordinates
+// of a sequence are derived from (b, h) in the kernel.
 struct alignas(64) Sm100Params {
   CUtensorMap tk, tq, tv;
   FwdParams p;
 };
+// The same for a packed batch: p.map describes the packed arrays (B = 1, T = all tokens), the table the sequences.
+struct alignas(64) Sm100PackedParams : Sm100Params {
+  SeqTable seqs;
+};
+static_assert(sizeof(Sm100PackedParams) <= 4096, "kernel parameters");
 
 // A shared-memory descriptor whose start address is `bytes` further on (the address field holds bytes / 16 and
 // cannot carry out of its 14 bits for addresses inside one CTA's shared memory).
@@ -115,8 +124,9 @@ __device__ __forceinline__ uint64_t desc_adv(uint64_t d, uint32_t bytes) { retur
 
 struct SyncPB { __device__ __forceinline__ void operator()() const { group_sync128(2); } };
 
-template <bool kTma>
-__global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_constant__ Sm100Params P) {
+template <class Params>
+__global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_constant__ Params P) {
+  constexpr bool kPacked = std::is_same<Params, Sm100PackedParams>::value;
   const FwdParams& p = P.p;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(16) Ctl ctl;   // its float arrays are read with 16-byte loads
@@ -125,16 +135,18 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
   const int grp = warp >> 2;             // 0 PA, 1 PB, 2 CA, 3 CB
   const int gt = tid & (kGrp - 1);       // thread index inside its group = tensor-memory lane it owns
   const int wq = warp & 3;
-  const int T = p.map.T;
-  const int unit = blockIdx.x;
-  const int b = unit / p.map.H, h = unit % p.map.H;
+  int T = p.map.T, unit = blockIdx.x, tok0 = 0;   // tok0: first token of a packed sequence
+  int b = unit / p.map.H;
+  const int h = unit % p.map.H;
+  if constexpr (kPacked) {
+    T = P.seqs.len[b];
+    tok0 = P.seqs.start[b];
+    unit = P.seqs.index[b] * p.map.H + h;
+    b = 0;
+  }
   const int hq = p.map.hq(h);
-  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
-  const int64_t vo_base = p.map.base(b, h, kD), vo_tok = p.map.tok(kD);         // v, o
-  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  // tensor-map coordinates of this sequence (column-block origin, outermost index)
-  const int qc2 = p.map.bthd ? 16 * hq : 0, qc4 = p.map.bthd ? b : b * p.map.Hq + hq;
-  const int vc2 = p.map.bthd ? 16 * h : 0, vc4 = p.map.bthd ? b : unit;
+  const int64_t vo_tok = p.map.tok(kD), vo_base = p.map.base(b, h, kD) + tok0 * vo_tok;   // v, o
+  const int64_t s_tok = p.map.tok(1), s_base = p.map.base(b, h, 1) + tok0 * s_tok;
 
   if (warp == 0) {
     tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), TM_COLS);
@@ -149,8 +161,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       tc::mbar_init(tc::smem_u32(&ctl.akk[i]), kGrp);
       tc::mbar_init(tc::smem_u32(&ctl.xfree[i]), 1);
     }
-    for (int i = 0; i < kRing; ++i) tc::mbar_init(tc::smem_u32(&ctl.kq[i]), kTma ? 1 : kGrp);
-    tc::mbar_init(tc::smem_u32(&ctl.vb), kTma ? 1 : kGrp);
+    for (int i = 0; i < kRing; ++i) tc::mbar_init(tc::smem_u32(&ctl.kq[i]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.vb), 1);
     tc::mbar_init(tc::smem_u32(&ctl.barP), 1);
     tc::mbar_init(tc::smem_u32(&ctl.barW), 1);
     tc::mbar_init(tc::smem_u32(&ctl.barUW), 1);
@@ -185,54 +197,48 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
 
   if (grp == 0) {
     // =========================== PA: K,Q tiles, D1, decay masks ======================================
-    const __nv_bfloat16* gq = reinterpret_cast<const __nv_bfloat16*>(p.q);
-    const __nv_bfloat16* gk = reinterpret_cast<const __nv_bfloat16*>(p.k);
     const float* gg = p.g ? reinterpret_cast<const float*>(p.g) + s_base : nullptr;
     const float* gbeta = p.beta + s_base;
 
     // K,Q rows (raw bf16), g and beta of chunk m -> ring tile m % kRing / raw scalars.  The l2 normalisation is
     // NOT applied to the tiles: it is folded into the factors rk, rs, rq.  Warp 0 fetches the scalars (and
-    // later scans them); with TMA its first lane also issues the tile copies.
+    // later scans them); its first lane also issues the tile copies.
     auto issue_kq = [&](int m) {
+      if (warp != 0) return;
       const int t0m = m * kC, rowsm = min(kC, T - t0m);
-      uint8_t* dQK = smem + SM_QKR + (m % kRing) * QK_TILE;
-      if (kTma) {
-        if (gt == 0) {
-          const uint32_t bar = tc::smem_u32(&ctl.kq[m % kRing]);
-          tc::mbar_arrive_expect_tx(bar, 2u * 64 * 256);
-          tc::tma_load_5d(tc::smem_u32(dQK), &P.tk, 0, 0, qc2, m * 8, qc4, bar);
-          tc::tma_load_5d(tc::smem_u32(dQK) + 64 * 256, &P.tq, 0, 0, qc2, m * 8, qc4, bar);
-        }
-      } else {
-        const int rin = gt & 7, kb = gt >> 3;
-#pragma unroll 2
-        for (int rb = 0; rb < 8; ++rb) {
-          const int r = rb * 8 + rin;
-          const bool live = r < rowsm;
-          const int64_t off = qk_base + (int64_t)(t0m + (live ? r : 0)) * qk_tok + kb * 8;
-          tc::cp_async16(tc::smem_u32(dQK + tc::core_off(r, kb * 8, RBS)), gk + off, live);
-          tc::cp_async16(tc::smem_u32(dQK + tc::core_off(64 + r, kb * 8, RBS)), gq + off, live);
-        }
+      if (lane == 0) {
+        const uint32_t dst = tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE);
+        const uint32_t bar = tc::smem_u32(&ctl.kq[m % kRing]);
+        tc::mbar_arrive_expect_tx(bar, QK_TILE);
+        tc::tma_load_4d(dst, &P.tk, 0, hq, tok0 + t0m, b, bar);
+        tc::tma_load_4d(dst + QK_PANEL, &P.tk, 64, hq, tok0 + t0m, b, bar);
+        tc::tma_load_4d(dst + QK_PANEL / 2, &P.tq, 0, hq, tok0 + t0m, b, bar);
+        tc::tma_load_4d(dst + QK_PANEL + QK_PANEL / 2, &P.tq, 64, hq, tok0 + t0m, b, bar);
       }
-      if (warp == 0) {
-        float* dG = ctl.gb;
+      float* dG = ctl.gb;
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int r = lane + 32 * hf;
-          const bool live = r < rowsm;
-          const int64_t off = live ? (int64_t)(t0m + r) * s_tok : 0;
-          tc::cp_async4(tc::smem_u32(dG + r), gbeta + off, live);                          // beta
-          tc::cp_async4(tc::smem_u32(dG + 64 + r), gg ? gg + off : gbeta, live && gg);     // g (0 without decay)
-        }
+      for (int hf = 0; hf < 2; ++hf) {
+        const int r = lane + 32 * hf;
+        const bool live = r < rowsm;
+        const int64_t off = live ? (int64_t)(t0m + r) * s_tok : 0;
+        tc::cp_async4(tc::smem_u32(dG + r), gbeta + off, live);                          // beta
+        tc::cp_async4(tc::smem_u32(dG + 64 + r), gg ? gg + off : gbeta, live && gg);     // g (0 without decay)
       }
       tc::cp_async_commit();
     };
-    // every thread: its copies of chunk m have landed (and, without TMA, are published on the tile's barrier)
-    auto land_kq = [&](int m) {
-      tc::cp_async_wait_all();
-      if (!kTma) {
+    // The last chunk of a packed sequence: the rows behind it belong to the next sequence.  Their beta is 0, so finite
+    // values would drop out of every product, but they are cleared (K here, V in CB) so that nothing of a neighbour,
+    // not even a NaN, can reach this sequence.  (Q rows behind the end only reach output rows that are not stored.)
+    auto clear_tail = [&](int m) {
+      if constexpr (kPacked) {
+        const int rowsm = T - m * kC;
+        if (rowsm >= kC) return;
+        wait_bar(&ctl.kq[m % kRing], (m / kRing) & 1);
+        uint8_t* tile = smem + SM_QKR + (m % kRing) * QK_TILE;
+        for (int i = gt; i < (kC - rowsm) * 16; i += kGrp)
+          *reinterpret_cast<uint4*>(tile + (i & 8) / 8 * QK_PANEL + (rowsm + (i >> 4)) * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
         tc::fence_async_smem();
-        arrive(&ctl.kq[m % kRing]);
+        group_sync128(1);
       }
     };
 
@@ -263,18 +269,18 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
     auto issue_d1 = [&](int m) {
       wait_bar(&ctl.kq[m % kRing], (m / kRing) & 1);
       tc::tc_fence_after();
-      const uint64_t ad0 = tc::smem_desc(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE), 128, RBS);
+      const uint64_t ad0 = tc::smem_desc_sw128(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE), 16, 1024);
 #pragma unroll 1
       for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t ad = desc_adv(ad0, ks * 256);
+        const uint64_t ad = desc_adv(ad0, (ks >> 2) * QK_PANEL + (ks & 3) * 32);
         tc::mma_ss(tbase + TM_D1, ad, ad, id_n64, ks > 0);
       }
       tc::mma_commit(tc::smem_u32(&ctl.barP));
     };
 
     issue_kq(0);
-    land_kq(0);
-    if (warp == 0) { __syncwarp(); scan_stage(0); }
+    clear_tail(0);
+    if (warp == 0) { tc::cp_async_wait_all(); __syncwarp(); scan_stage(0); }
     if (gt == 64) issue_d1(0);
     if (nchunks > 1) issue_kq(1);   // the copies run two chunks ahead of the masks (see the end of the loop body)
     uint32_t phP = 0;
@@ -352,9 +358,9 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       group_sync128(1);                      // every warp has drained D1 from tensor memory
       // what the NEXT chunk needs from this group, behind the hand-over
       if (n + 1 < nchunks) {
-        land_kq(n + 1);                      // the next chunk's beta, g (and, without TMA, its K,Q rows)
+        clear_tail(n + 1);
         if (gt == 64) issue_d1(n + 1);       // completes behind PB's inverse of this chunk
-        if (warp == 0) { __syncwarp(); scan_stage(n + 1); }
+        if (warp == 0) { tc::cp_async_wait_all(); __syncwarp(); scan_stage(n + 1); }
       }
       // chunk n-2 has left the consumer: its ring tile and its scalar and rq slots, (n+2) % 4, are free.  The copies of
       // chunk n+2 start here, BEFORE this group waits for chunk n+1's tile at the end of the next iteration: a tile
@@ -371,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       float* dst = ctl.rq[m % 4];
       const float scale = p.scale;
       const bool l2 = p.l2norm != 0;
-      row_sq_norms_64(smem + SM_QKR + (m % kRing) * QK_TILE, 64, wq, lane,
+      row_sq_norms_64(smem + SM_QKR + (m % kRing) * QK_TILE, QK_PANEL, 64, wq, lane,
                       [&](int r, float ss) { dst[r] = l2 ? scale / (sqrtf(ss) + 1e-6f) : scale; });
     };
     q_norms(0);
@@ -527,10 +533,10 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       // ---- (5) S^T += (decayed V_new^T) K^ ;  (4) Do = V_new^T A_qk^T -------------------------------------------
       if (gt == 0) {
         tc::tc_fence_after();
-        const uint64_t kd0 = tc::smem_desc(aQK, RBS, 128);  // K^ MN-major
+        const uint64_t kd0 = tc::smem_desc_sw128(aQK, QK_PANEL, 1024);  // K^ MN-major
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          tc::mma_ts(tbase + TM_S, tbase + TM_VB + ks * 8, desc_adv(kd0, ks * 2 * RBS), id_n128_bmn, 1);
+          tc::mma_ts(tbase + TM_S, tbase + TM_VB + ks * 8, desc_adv(kd0, ks * 2048), id_n128_bmn, 1);
         tc::mma_commit(tc::smem_u32(&ctl.bar2s));
         const uint64_t ad0 = tc::smem_desc(aAqk, 128, A_RBS);
 #pragma unroll
@@ -558,46 +564,28 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
     wait_bar(((nchunks - 1) & 1) ? &ctl.bar2b : &ctl.bar2, ((nchunks - 1) >> 1) & 1);   // every product has completed before tensor memory is released
   } else {
     // =========================== CB: q norms, W tile, U^T, output, Dq ==================================
-    const __nv_bfloat16* gv = reinterpret_cast<const __nv_bfloat16*>(p.v);
     __nv_bfloat16* go = reinterpret_cast<__nv_bfloat16*>(p.o);
     uint8_t* sV = smem + SM_V;
     // The group's three products per chunk are issued by threads of three different warps (a product blocks its issuing
     // thread for 330-540 cycles, and the warps meet again at the group's next barrier): W^T by thread 0, U^T and the V
     // copy by thread 32, Dq by thread 64.  Each commits to its own barrier.
     constexpr int kUThread = 32, kDqThread = 64;
-    // V rows of chunk m -> core-matrix tile
+    // V rows of chunk m -> tile (thread kUThread)
     auto issue_v = [&](int m) {
-      if (kTma) {
-        if (gt == kUThread) {
-          const uint32_t bar = tc::smem_u32(&ctl.vb);
-          tc::mbar_arrive_expect_tx(bar, 64u * 256);
-          tc::tma_load_5d(tc::smem_u32(sV), &P.tv, 0, 0, vc2, m * 8, vc4, bar);
-        }
-      } else {
-        const int t0m = m * kC, rowsm = min(kC, T - t0m);
-        const int rin = gt & 7, kb = gt >> 3;
-#pragma unroll 2
-        for (int rb = 0; rb < 8; ++rb) {
-          const int r = rb * 8 + rin;
-          const bool live = r < rowsm;
-          const __nv_bfloat16* src = gv + vo_base + (int64_t)(t0m + (live ? r : 0)) * vo_tok + kb * 8;
-          tc::cp_async16(tc::smem_u32(sV + tc::core_off(r, kb * 8, RBS)), src, live);
-        }
-        tc::cp_async_commit();
-        tc::cp_async_wait_all();
-        tc::fence_async_smem();
-        arrive(&ctl.vb);
-      }
+      const uint32_t bar = tc::smem_u32(&ctl.vb), dst = tc::smem_u32(sV);
+      tc::mbar_arrive_expect_tx(bar, 2 * V_PANEL);
+      tc::tma_load_4d(dst, &P.tv, 0, h, tok0 + m * kC, b, bar);
+      tc::tma_load_4d(dst + V_PANEL, &P.tv, 64, h, tok0 + m * kC, b, bar);
     };
     // Dq = S^T Q^T of chunk m (elected thread): the bf16 state copy of chunk m is ready and the Dq columns
     // have been read by the output epilogue of chunk m-1
     auto issue_dq = [&](int m) {
       wait_bar(&ctl.sbrdy, m & 1);
       tc::tc_fence_after();
-      const uint64_t qd0 = tc::smem_desc(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE) + 8 * RBS, 128, RBS);   // rows 64..127
+      const uint64_t qd0 = tc::smem_desc_sw128(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE) + QK_PANEL / 2, 16, 1024);   // rows 64..127
 #pragma unroll 1
       for (int ks = 0; ks < 8; ++ks)
-        tc::mma_ts(tbase + TM_DQ, tbase + TM_SB + ks * 8, desc_adv(qd0, ks * 256), id_n64, ks > 0);
+        tc::mma_ts(tbase + TM_DQ, tbase + TM_SB + ks * 8, desc_adv(qd0, (ks >> 2) * QK_PANEL + (ks & 3) * 32), id_n64, ks > 0);
       tc::mma_commit(tc::smem_u32(&ctl.barDq));
     };
     // O^T of chunk m: rq_i (e^{G_i} Dq + Do), straight from the accumulators to global memory.  Each thread owns
@@ -651,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       }
     };
 
-    issue_v(0);
+    if (gt == kUThread) issue_v(0);
     for (int n = 0; n < nchunks; ++n) {
       const int s = n & 1;
       const uint32_t aQK = tc::smem_u32(smem + SM_QKR + (n % kRing) * QK_TILE);
@@ -661,11 +649,11 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       tc::tc_fence_after();
       // ---- (2a) W^T = K^T Tw^T -> this stage's accumulator, idle until U^T is issued into it ---------------
       if (gt == 0) {
-        const uint64_t kd0 = tc::smem_desc(aQK, RBS, 128);   // K MN-major, 16 chunk rows per step
+        const uint64_t kd0 = tc::smem_desc_sw128(aQK, QK_PANEL, 1024);   // K MN-major, 16 chunk rows per step
         const uint64_t twd0 = tc::smem_desc(aXB + XB_TW, 128, A_RBS);
 #pragma unroll 1
         for (int ks = 0; ks < 4; ++ks)
-          tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(kd0, ks * 2 * RBS), desc_adv(twd0, ks * 256), id_n64_amn, ks > 0);
+          tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(kd0, ks * 2048), desc_adv(twd0, ks * 256), id_n64_amn, ks > 0);
         tc::mma_commit(tc::smem_u32(&ctl.barW));
       }
       // the scalars this chunk's output epilogue will need, kept where PA cannot overwrite them
@@ -698,22 +686,29 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       arrive(&ctl.wrdy);
       group_sync128(4);   // W^T has left the accumulator in every thread; the kept scalars are visible
       // ---- (2b) U^T = V^T Tb^T -> the same accumulator ---------------------------------------------------
+      if constexpr (kPacked) {
+        const int rowsn = T - n * kC;
+        if (rowsn < kC && wq == kUThread / 32) {   // see clear_tail
+          wait_bar(&ctl.vb, n & 1);
+          for (int i = lane; i < (kC - rowsn) * 16; i += 32)
+            *reinterpret_cast<uint4*>(sV + (i & 8) / 8 * V_PANEL + (rowsn + (i >> 4)) * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          tc::fence_async_smem();
+          __syncwarp();
+        }
+      }
       if (gt == kUThread) {
         tc::tc_fence_after();
         wait_bar(&ctl.vb, n & 1);
         tc::tc_fence_after();
-        const uint64_t vd0 = tc::smem_desc(tc::smem_u32(sV), RBS, 128);
+        const uint64_t vd0 = tc::smem_desc_sw128(tc::smem_u32(sV), V_PANEL, 1024);
         const uint64_t tbd0 = tc::smem_desc(aXB + XB_TB, 128, A_RBS);
 #pragma unroll 1
         for (int ks = 0; ks < 4; ++ks)
-          tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(vd0, ks * 2 * RBS), desc_adv(tbd0, ks * 256), id_n64_amn, ks > 0);
+          tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(vd0, ks * 2048), desc_adv(tbd0, ks * 256), id_n64_amn, ks > 0);
         tc::mma_commit(tc::smem_u32(&ctl.barUW));
         wait_bar(&ctl.barUW, n & 1);   // V, Tb, Tw have been read: release the X buffer, fetch the next chunk's V rows
         arrive(&ctl.xfree[s]);
-      }
-      if (n + 1 < nchunks) {
-        if (!kTma) wait_bar(&ctl.barUW, n & 1);   // every thread copies V rows
-        issue_v(n + 1);
+        if (n + 1 < nchunks) issue_v(n + 1);
       }
       // ---- output of the previous chunk, then Dq of this one ---------------------------------------------
       if (n >= 1) {
@@ -739,29 +734,37 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
   if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
 }
 
-inline cudaError_t launch_chunk(const FwdParams& p, cudaStream_t stream) {
-  // TMA inputs need whole 8-row blocks; otherwise the per-thread cp.async instantiation loads the tiles
-  // (same layout, same results).
-  Sm100Params P;
-  memset(&P, 0, sizeof(P));
-  P.p = p;
+template <class Params>
+inline cudaError_t launch_chunk_kernel(Params& P, const FwdParams& p, int64_t units, cudaStream_t stream) {
   const bool bthd = p.map.bthd != 0;
-  const bool tma_in = p.map.T % 8 == 0 && make_input_map(&P.tk, p.k, p.map.B, p.map.Hq, p.map.T, bthd) &&
-                      make_input_map(&P.tq, p.q, p.map.B, p.map.Hq, p.map.T, bthd) &&
-                      make_input_map(&P.tv, p.v, p.map.B, p.map.H, p.map.T, bthd);
-  auto kern = tma_in ? chunk_sm100_kernel<true> : chunk_sm100_kernel<false>;
-  thread_local int attr_dev[2] = {-1, -1};
+  P.p = p;
+  if (!make_panel_map(&P.tk, p.k, p.map.B, p.map.Hq, p.map.T, bthd) || !make_panel_map(&P.tq, p.q, p.map.B, p.map.Hq, p.map.T, bthd) ||
+      !make_panel_map(&P.tv, p.v, p.map.B, p.map.H, p.map.T, bthd))
+    return cudaErrorInvalidValue;
+  auto kern = chunk_sm100_kernel<Params>;
+  thread_local int attr_dev = -1;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (attr_dev[tma_in] != dev) {
+  if (attr_dev != dev) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
     if (e != cudaSuccess) return e;
-    attr_dev[tma_in] = dev;
+    attr_dev = dev;
   }
-  const dim3 grid((unsigned)((int64_t)p.map.B * p.map.H)), block(kThreads);
-  kern<<<grid, block, SM_TOTAL, stream>>>(P);
+  kern<<<dim3((unsigned)units), dim3(kThreads), SM_TOTAL, stream>>>(P);
   return cudaGetLastError();
+}
+
+inline cudaError_t launch_chunk(const FwdParams& p, cudaStream_t stream) {
+  Sm100Params P;
+  return launch_chunk_kernel(P, p, (int64_t)p.map.B * p.map.H, stream);
+}
+
+// Every sequence of `seqs` in one launch; p describes the packed arrays (map.B = 1, map.T = all tokens, token-major).
+inline cudaError_t launch_chunk_packed(const FwdParams& p, const SeqTable& seqs, cudaStream_t stream) {
+  Sm100PackedParams P;
+  P.seqs = seqs;
+  return launch_chunk_kernel(P, p, (int64_t)seqs.n * p.map.H, stream);
 }
 
 }  // namespace sm100

@@ -87,4 +87,16 @@ struct FwdParams {
   }
 };
 
+// The sequences of a packed batch that one launch works on, longest first (a CTA takes one sequence and head; CTAs
+// start in this order, so the long sequences are under way while the short ones fill the remaining SMs).  Travels as
+// a kernel parameter: no device memory, no copy.
+constexpr int kMaxSeqs = 192;   // per launch; with the tensor maps the parameters stay below 4 KB
+struct SeqTable {
+  int n, chunks;             // sequences; chunks of all of them together
+  int32_t start[kMaxSeqs];   // first token
+  int32_t len[kMaxSeqs];
+  int32_t index[kMaxSeqs];   // position in the caller's list (which state is its own)
+  int32_t first[kMaxSeqs];   // chunks of the sequences before it in the table
+};
+
 }  // namespace dr

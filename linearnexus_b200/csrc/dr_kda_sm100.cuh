@@ -41,11 +41,10 @@ constexpr int kThreads = 256;
 constexpr int WS_W = 0;                    // W   [64][128] bf16
 constexpr int WS_QG = WS_W + 16384;        // Qg  [64][128] bf16
 constexpr int WS_KD = WS_QG + 16384;       // Kd  [64][128] bf16
-constexpr int WS_V = WS_KD + 16384;        // V   [64][128] bf16 (rows past the end of the sequence zero)
-constexpr int WS_TB = WS_V + 16384;        // T diag(beta) [64][64] bf16
+constexpr int WS_TB = WS_KD + 16384;       // T diag(beta) [64][64] bf16
 constexpr int WS_AQK = WS_TB + 8192;       // A_qk         [64][64] bf16
 constexpr int WS_EGL = WS_AQK + 8192;      // e^{G_L}[128] fp32
-constexpr int WS_REC = WS_EGL + 512;       // 82432
+constexpr int WS_REC = WS_EGL + 512;       // 66048
 
 inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC - 1) / kC) * (int64_t)WS_REC; }
 
@@ -120,7 +119,20 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
 }
 
 
-__global__ void __launch_bounds__(kThreads, 2) intra_kernel(const FwdParams p, uint8_t* __restrict__ ws, const int copy_v) {
+// Kernel parameters of the intra pass; a packed batch adds the table of its sequences (p then describes the packed
+// arrays: B = 1, T = all tokens, token-major).
+struct IntraParams {
+  FwdParams p;
+  uint8_t* ws;
+};
+struct IntraPackedParams : IntraParams {
+  SeqTable seqs;
+};
+
+template <class Params>
+__global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constant__ Params P) {
+  constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value;
+  const FwdParams& p = P.p;
   extern __shared__ __align__(1024) uint8_t smem[];
   float* sG = reinterpret_cast<float*>(smem + IN_G);
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + IN_K);
@@ -135,15 +147,31 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const FwdParams p, u
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int T = p.map.T;
-  const int nchunks = (T + kC - 1) / kC;
-  const int unit = blockIdx.x / nchunks, n = blockIdx.x % nchunks;
-  const int b = unit / p.map.H, h = unit % p.map.H;
-  const int t0 = n * kC, rows = min(kC, T - t0);
+  int T = p.map.T, n, b, h, tok0 = 0;
+  uint8_t* rec = P.ws;
+  if constexpr (kPacked) {
+    h = blockIdx.x / P.seqs.chunks;
+    const int c = blockIdx.x % P.seqs.chunks;
+    int lo = 0, hi = P.seqs.n - 1;   // the last sequence that starts at or before chunk c
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (P.seqs.first[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    n = c - P.seqs.first[lo];
+    T = P.seqs.len[lo];
+    tok0 = P.seqs.start[lo];
+    b = 0;
+    rec += ((int64_t)P.seqs.first[lo] * p.map.H + (int64_t)h * ((T + kC - 1) / kC) + n) * WS_REC;
+  } else {
+    const int nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks;
+    n = blockIdx.x % nchunks;
+    b = unit / p.map.H; h = unit % p.map.H;
+    rec += ((int64_t)unit * nchunks + n) * WS_REC;
+  }
+  const int rows = min(kC, T - n * kC), t0 = tok0 + n * kC;
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
   const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);         // per-channel decay: per value head
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  uint8_t* rec = ws + ((int64_t)unit * nchunks + n) * WS_REC;
   constexpr float kLog2e = 1.4426950408889634f;
 
   // ---- load: raw k, q rows, their norm factors, the log decay (in log2 units); lane = four channels ---------
@@ -190,21 +218,6 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const FwdParams p, u
         sRk[c] = kmul;
         sRq[c] = qmul;
       }
-    }
-  }
-  // V rows -> the record's tile, 16 bytes per piece (coalesced writes); skipped when the state kernel can fetch
-  // the rows itself through a tensor map
-  if (copy_v) {
-    const __nv_bfloat16* gv = reinterpret_cast<const __nv_bfloat16*>(p.v);
-    const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int piece = tid + kThreads * it;
-      int row, col;
-      piece128(piece, row, col);
-      uint4 u = make_uint4(0u, 0u, 0u, 0u);
-      if (row < rows) u = *reinterpret_cast<const uint4*>(gv + v_base + (t0 + row) * v_tok + col);
-      *reinterpret_cast<uint4*>(rec + WS_V + piece * 16) = u;
     }
   }
   __syncthreads();
@@ -494,8 +507,12 @@ constexpr uint32_t TM_DU = 192;   // 2 x 64: U^T -> Vn^T -> Do
 constexpr uint32_t TM_DQ = 320;   // S^T Qg^T                          64
 constexpr uint32_t TM_VA = 384;   // Vn^T bf16                         32
 constexpr uint32_t TM_COLS = 512;
-// shared memory: two record buffers, then the fp32 output staging tile [64][128]
-constexpr int ST_O = 2 * WS_REC;
+// shared memory: two record buffers, two V tiles (two swizzled panels of 64 columns each, straight from the input by
+// TMA), then the fp32 output staging tile [64][128]
+constexpr int V_PANEL = 64 * 128, V_TILE = 2 * V_PANEL;
+constexpr int ST_V = 2 * WS_REC;
+constexpr int ST_O = ST_V + 2 * V_TILE;
+static_assert(ST_V % 1024 == 0, "swizzled tiles");
 constexpr int ST_TOTAL = ST_O + 64 * 128 * 4;
 
 struct StateCtl {
@@ -516,24 +533,41 @@ constexpr int kStateThreads = kThreads + 32;
 // o in its own dtype; one box {128, 64, 1, 1} stores a chunk's rows and clips the ragged tail).
 struct StateParams {
   CUtensorMap to;
-  CUtensorMap tv;   // 5-d view of v whose box is one 64x128 tile in core-matrix order (see sm100::make_input_map)
+  CUtensorMap tv;   // panels of v (see sm100::make_panel_map)
   FwdParams p;
   const uint8_t* ws;
-  int use_tma_out, use_tma_v;
+  int use_tma_out;
 };
+struct StatePackedParams : StateParams {
+  SeqTable seqs;
+};
+static_assert(sizeof(StatePackedParams) <= 4096, "kernel parameters");
 
-__global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_constant__ StateParams P) {
+template <class Params>
+__global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_constant__ Params P) {
+  constexpr bool kPacked = std::is_same<Params, StatePackedParams>::value;
   const FwdParams& p = P.p;
-  const uint8_t* __restrict__ ws = P.ws;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) StateCtl ctl;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int hs = (tid >> 7) & 1, l128 = tid & 127;
-  const int T = p.map.T, nchunks = (T + kC - 1) / kC;
-  const int unit = blockIdx.x;
-  const int b = unit / p.map.H, h = unit % p.map.H;
-  const int64_t o_base = p.map.base(b, h, kD), o_tok = p.map.tok(kD);
-  const uint8_t* recs = ws + (int64_t)unit * nchunks * WS_REC;
+  int T = p.map.T, unit = blockIdx.x, tok0 = 0;
+  int b = unit / p.map.H;
+  const int h = unit % p.map.H;
+  int64_t rec0;
+  if constexpr (kPacked) {
+    T = P.seqs.len[b];
+    tok0 = P.seqs.start[b];
+    unit = P.seqs.index[b] * p.map.H + h;
+    rec0 = (int64_t)P.seqs.first[b] * p.map.H + (int64_t)h * ((T + kC - 1) / kC);
+    b = 0;
+  }
+  const int nchunks = (T + kC - 1) / kC;
+  if constexpr (!kPacked) rec0 = (int64_t)unit * nchunks;
+  const int64_t o_tok = p.map.tok(kD), o_base = p.map.base(b, h, kD) + tok0 * o_tok;
+  const uint8_t* recs = P.ws + rec0 * WS_REC;
+  // the last chunk of a packed sequence: its V tile ends in rows of the next sequence, which the workers clear
+  auto packed_tail = [&](int n) { return kPacked && T - n * kC < kC; };
 
   if (warp == 0) {
     tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), TM_COLS);
@@ -566,23 +600,17 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   if (warp == 8) {
     // =========================== ISSUING WARP (one thread) ======================================================
     if (tid == kThreads) {
-      // the whole record of chunk m -> buffer m & 1 (the record is contiguous; four copies in flight)
+      // the record of chunk m -> buffer m & 1, the V rows straight from the input
       auto issue_load = [&](int m) {
         const uint32_t bar = tc::smem_u32(&ctl.full[m & 1]);
-        tc::mbar_arrive_expect_tx(bar, WS_REC);
-        const uint32_t dst = tc::smem_u32(smem + (m & 1) * WS_REC);
+        tc::mbar_arrive_expect_tx(bar, WS_REC + V_TILE);
+        const uint32_t dst = tc::smem_u32(smem + (m & 1) * WS_REC), dv = tc::smem_u32(smem + ST_V + (m & 1) * V_TILE);
         const uint8_t* src = recs + (int64_t)m * WS_REC;
-        if (P.use_tma_v) {
-          // the V rows straight from the input tensor; the record carries the other tiles
-          tc::tma_load_5d(dst + WS_V, &P.tv, 0, 0, 0, m * 8, unit, bar);
+        tc::tma_load_4d(dv, &P.tv, 0, h, tok0 + m * kC, b, bar);
+        tc::tma_load_4d(dv + V_PANEL, &P.tv, 64, h, tok0 + m * kC, b, bar);
 #pragma unroll
-          for (int i = 0; i < 3; ++i) tc::bulk_g2s(dst + i * 16384, src + i * 16384, 16384, bar);   // W, Qg, Kd
-          tc::bulk_g2s(dst + WS_TB, src + WS_TB, WS_REC - WS_TB, bar);                                   // Tb, A_qk, e^{G_L}
-        } else {
-          constexpr int Q4 = WS_REC / 4;   // 20608, a multiple of 16
-#pragma unroll
-          for (int i = 0; i < 4; ++i) tc::bulk_g2s(dst + i * Q4, src + i * Q4, Q4, bar);
-        }
+        for (int i = 0; i < 3; ++i) tc::bulk_g2s(dst + i * 16384, src + i * 16384, 16384, bar);   // W, Qg, Kd
+        tc::bulk_g2s(dst + WS_TB, src + WS_TB, WS_REC - WS_TB, bar);                                   // Tb, A_qk, e^{G_L}
       };
       if (nchunks > 0) issue_load(0);
       if (nchunks > 1) issue_load(1);
@@ -594,13 +622,14 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
         const int s = n & 1;
         const uint8_t* st = smem + s * WS_REC;
         const uint32_t aW = tc::smem_u32(st + WS_W), aQg = tc::smem_u32(st + WS_QG), aKd = tc::smem_u32(st + WS_KD);
-        const uint32_t aV = tc::smem_u32(st + WS_V), aTb = tc::smem_u32(st + WS_TB), aAqk = tc::smem_u32(st + WS_AQK);
+        const uint32_t aV = tc::smem_u32(smem + ST_V + s * V_TILE), aTb = tc::smem_u32(st + WS_TB), aAqk = tc::smem_u32(st + WS_AQK);
         wait_bar(&ctl.full[s], (n >> 1) & 1);
         // U^T = V^T Tb^T needs no state: issue it before the workers' state pass has finished
+        if (packed_tail(n)) wait_bar(&ctl.go1, n & 1);
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          const uint64_t ad = tc::smem_desc(aV + ks * 2 * RBS, RBS, 128);   // MN-major, 16 chunk rows per step
+          const uint64_t ad = tc::smem_desc_sw128(aV + ks * 2048, V_PANEL, 1024);   // MN-major, 16 chunk rows per step
           const uint64_t bd = tc::smem_desc(aTb + ks * 256, 128, A_RBS);
           tc::mma_ss(tbase + TM_DU + 64 * s, ad, bd, id_n64_amn, ks > 0);
         }
@@ -661,6 +690,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
     // tensor map, row copies by the threads)
     auto output_epilogue = [&](int m) {
       const int t0m = m * kC, rowsm = min(kC, T - t0m);
+      const bool tma_out = P.use_tma_out && !packed_tail(m);   // (a box would run into the next sequence)
       if (P.use_tma_out && tid == 0) tc::bulk_wait_read_all();   // the previous store has read the staging tile
       workers_sync();
       {
@@ -681,11 +711,11 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
         }
       }
       if (!p.o) return;
-      if (P.use_tma_out) {
+      if (tma_out) {
         tc::fence_async_smem();
         workers_sync();
         if (tid == 0) {
-          tc::tma_store_4d(&P.to, tc::smem_u32(sO), 0, t0m, h, b);
+          tc::tma_store_4d(&P.to, tc::smem_u32(sO), 0, tok0 + t0m, h, b);
           tc::bulk_commit();
         }
         return;
@@ -738,6 +768,13 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
         }
         tc::tc_wait_st();
       }
+      if (packed_tail(n)) {   // nothing of the next sequence, not even a NaN times 0, may reach this one
+        const int rowsn = T - n * kC;
+        for (int i = tid; i < (kC - rowsn) * 16; i += kThreads)
+          *reinterpret_cast<uint4*>(smem + ST_V + s * V_TILE + (i & 8) / 8 * V_PANEL + (rowsn + (i >> 4)) * 128 + (i & 7) * 16) =
+              make_uint4(0u, 0u, 0u, 0u);
+        tc::fence_async_smem();
+      }
       tc::tc_fence_before();
       arrive(&ctl.go1);
       if (n > 0) output_epilogue(n - 1);   // overlaps the products of this chunk
@@ -781,29 +818,46 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
 }
 
-inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches) {
-  cudaError_t e = cudaFuncSetAttribute(intra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+template <class IP, class SP>
+inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace, int64_t chunk_units, int64_t units, cudaStream_t stream) {
+  thread_local int attr_dev = -1;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_TOTAL);
-  if (e != cudaSuccess) return e;
-  const int64_t units = (int64_t)p.map.B * p.map.H;
-  const int nchunks = (p.map.T + kC - 1) / kC;
-  uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-  StateParams SP;
-  memset(&SP, 0, sizeof(SP));
-  SP.p = p;
-  SP.ws = ws;
-  // V rows by TMA need the rows of one sequence contiguous and whole 8-row blocks
-  SP.use_tma_v = !p.map.bthd && p.map.T % 8 == 0 && sm100::make_input_map(&SP.tv, p.v, units, p.map.T);
-  intra_kernel<<<(unsigned)(units * nchunks), kThreads, IN_TOTAL, stream>>>(p, ws, SP.use_tma_v ? 0 : 1);
+  if (attr_dev != dev) {
+    e = cudaFuncSetAttribute(intra_kernel<IP>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(state_kernel<SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_TOTAL);
+    if (e != cudaSuccess) return e;
+    attr_dev = dev;
+  }
+  I.p = p;
+  S.p = p;
+  S.ws = I.ws = reinterpret_cast<uint8_t*>(workspace);
+  if (!sm100::make_panel_map(&S.tv, p.v, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
+  intra_kernel<IP><<<(unsigned)chunk_units, kThreads, IN_TOTAL, stream>>>(I);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  SP.use_tma_out = p.o != nullptr && sm100::make_output_map(&SP.to, p.o, p.map, p.out_dt == DR_BF16 ? 2 : 4);
-  state_kernel<<<(unsigned)units, kStateThreads, ST_TOTAL, stream>>>(SP);
-  *launches = 2;
+  S.use_tma_out = p.o != nullptr && sm100::make_output_map(&S.to, p.o, p.map, p.out_dt == DR_BF16 ? 2 : 4);
+  state_kernel<SP><<<(unsigned)units, kStateThreads, ST_TOTAL, stream>>>(S);
   return cudaGetLastError();
+}
+
+inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches) {
+  IntraParams I;
+  StateParams S;
+  const int64_t units = (int64_t)p.map.B * p.map.H;
+  *launches = 2;
+  return launch_pair(I, S, p, workspace, units * ((p.map.T + kC - 1) / kC), units, stream);
+}
+
+// Every sequence of `seqs` in one pair of launches; the workspace holds seqs.chunks records per head.
+inline cudaError_t launch_chunk_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream) {
+  IntraPackedParams I;
+  StatePackedParams S;
+  I.seqs = S.seqs = seqs;
+  return launch_pair(I, S, p, workspace, (int64_t)seqs.chunks * p.map.H, (int64_t)seqs.n * p.map.H, stream);
 }
 
 }  // namespace kda
 }  // namespace dr
-

@@ -69,22 +69,22 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// ||x_r||^2 for 64 rows of a bf16 core-matrix tile (rows row0 .. row0+63, 128 columns, row-block stride RBS) on
-// the warp-level tensor cores: warp w of a four-warp group takes rows 16w .. 16w+15, forms their 16x16 Gram
-// block with mma.sync m16n8k16 (the A fragments double as the B fragments) and keeps the diagonal.  A core
-// matrix (8 rows x 16 bytes, 128 contiguous bytes) is exactly one ldmatrix 8x8 matrix.
+// ||x_r||^2 for 64 rows of a bf16 tile in the 128-byte swizzle (rows row0 .. row0+63; 128 columns as two 64-column
+// panels `panel` bytes apart) on the warp-level tensor cores: warp w of a four-warp group takes rows 16w .. 16w+15,
+// forms their 16x16 Gram block with mma.sync m16n8k16 (the A fragments double as the B fragments) and keeps the
+// diagonal.  ldmatrix takes eight 16-byte row pieces per 8x8 matrix; the swizzle spreads them over all banks.
 // out(r, value) is called once per row by the lane that holds its diagonal entry.
 template <class Out>
-__device__ __forceinline__ void row_sq_norms_64(const uint8_t* tile, int row0, int w, int lane, Out out) {
+__device__ __forceinline__ void row_sq_norms_64(const uint8_t* tile, int panel, int row0, int w, int lane, Out out) {
   const int mi = lane >> 3, rin = lane & 7;
-  const uint32_t base = tc::smem_u32(tile) + (uint32_t)(((row0 >> 3) + 2 * w + (mi & 1)) * RBS + (mi >> 1) * 128 + rin * 16);
+  const uint32_t base = tc::smem_u32(tile) + (uint32_t)((row0 + 16 * w + 8 * (mi & 1) + rin) * 128);
   float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     uint32_t a[4];
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-                 : "r"(base + ks * 256));
+                 : "r"(base + (ks >> 2) * panel + (((2 * (ks & 3) + (mi >> 1)) ^ rin) << 4)));
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d0[0]), "+f"(d0[1]), "+f"(d0[2]), "+f"(d0[3])
@@ -254,7 +254,7 @@ inline EncodeTiledFn encode_tiled_fn() {
 struct MapKey {
   const void* base;
   int64_t a, b, c;   // geometry (meaning depends on kind)
-  int kind;          // 0: [units][T][128] input, 1: [B][T][heads][128] input, 2: output
+  int kind;          // 0: swizzled panels of [B][heads][T][128], 1: of [B][T][heads][128], 2: output
   bool operator==(const MapKey& o) const { return base == o.base && a == o.a && b == o.b && c == o.c && kind == o.kind; }
 };
 struct MapCache {
@@ -277,39 +277,26 @@ struct MapCache {
 };
 inline MapCache& map_cache() { static MapCache c; return c; }
 
-// 5-d input view whose box {8,8,16,8,1} lands one 64x128 bf16 chunk in shared memory already in the
-// 8x8 core-matrix order the tensor cores read (needs T % 8 == 0).
-//   [B*heads, T, 128] storage ([B,H,T,D]): dims {8 elems, 8 rows, 16 column blocks, T/8 row blocks, B*heads};
-//     the chunk m of sequence u is at coordinates (0, 0, 0, 8m, u).
-//   [B, T, heads, 128] storage ([B,T,H,D]): dims {8 elems, 8 rows (stride heads*256 B), 16*heads column
-//     blocks, T/8 row blocks, B}; the chunk m of (b, h) is at coordinates (0, 0, 16h, 8m, b).
-// The maps cover this GPU's memory only and are used without multicast.
-inline bool make_input_map(CUtensorMap* m, const void* base, int64_t B, int64_t heads, int T, bool bthd) {
+// 4-d input view {128, heads, T, B} of [B,heads,T,128] or [B,T,heads,128] bf16 in the 128-byte swizzle: one box
+// {64,1,64,1} is a 64-column panel of 64 token rows (8 KB); rows past T arrive as zeros.  Any T, and a box may start at
+// any token (the sequences of a packed batch do).
+inline bool make_panel_map(CUtensorMap* m, const void* base, int64_t B, int64_t heads, int64_t T, bool bthd) {
   const MapKey key{base, B, heads, T, bthd ? 1 : 0};
   if (map_cache().find(key, m)) return true;
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return false;
-  cuuint64_t dims[5], strides[4];
-  if (bthd) {
-    dims[0] = 8; dims[1] = 8; dims[2] = 16 * (cuuint64_t)heads; dims[3] = (cuuint64_t)(T / 8); dims[4] = (cuuint64_t)B;
-    strides[0] = (cuuint64_t)heads * 256; strides[1] = 16; strides[2] = 8 * (cuuint64_t)heads * 256;
-    strides[3] = (cuuint64_t)T * heads * 256;
-  } else {
-    dims[0] = 8; dims[1] = 8; dims[2] = 16; dims[3] = (cuuint64_t)(T / 8); dims[4] = (cuuint64_t)(B * heads);
-    strides[0] = 256; strides[1] = 16; strides[2] = 2048; strides[3] = (cuuint64_t)T * 256;
-  }
-  const cuuint32_t box[5] = {8, 8, 16, 8, 1};
-  const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  if (fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, es,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const cuuint64_t dims[4] = {128, (cuuint64_t)heads, (cuuint64_t)T, (cuuint64_t)B};
+  cuuint64_t strides[3];
+  if (bthd) { strides[0] = 256; strides[1] = (cuuint64_t)heads * 256; strides[2] = (cuuint64_t)T * heads * 256; }
+  else { strides[0] = (cuuint64_t)T * 256; strides[1] = 256; strides[2] = (cuuint64_t)heads * T * 256; }
+  const cuuint32_t box[4] = {64, 1, 64, 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  if (fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
+         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   map_cache().put(key, *m);
   return true;
-}
-// the [B*heads][T][128] form with the units already flattened
-inline bool make_input_map(CUtensorMap* m, const void* base, int64_t units, int T) {
-  return make_input_map(m, base, units, 1, T, false);
 }
 
 // 4-d output view {128, T, H, B} of [B,H,T,128] or [B,T,H,128], bf16 (elem_bytes 2) or fp32 (4); one box

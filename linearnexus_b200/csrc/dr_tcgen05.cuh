@@ -102,12 +102,18 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void* src, uin
                : "memory");
 }
 // Tiled TMA copies through a tensor map (no multicast, this CTA's own shared memory only).
-// The innermost coordinate is always 0 here, so the 16-byte start rule holds by construction.
+// The innermost coordinate is a multiple of 64 elements here, so the 16-byte start rule holds by construction.
 __device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const void* tmap, int c0, int c1, int c2, int c3,
                                             int c4, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
       ::"r"(dst_smem), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst_smem, const void* tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst_smem), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void tma_store_4d(const void* tmap, uint32_t src_smem, int c0, int c1, int c2, int c3) {
@@ -173,6 +179,14 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version for sm_100
   return d;                // base offset 0, lbo mode 0, layout type 0 (no swizzle)
+}
+
+// The same for a tile in the 128-byte swizzle: rows of 128 bytes (64 bf16), groups of 8 rows = 1024 contiguous bytes, the
+// 16-byte piece c of row r at piece c ^ (r & 7) -- what a TMA box of 64 columns lands as.  K-major operands (rows along
+// M/N): sbo = 1024, lbo unused, 16 K elements further on = 32 bytes, the next 64 = the next panel.  MN-major operands
+// (rows along K): lbo = distance of 64-element panels along M/N, sbo = distance of 8-row groups along K.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return smem_desc(saddr, lbo, sbo) | ((uint64_t)2 << 61);
 }
 
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulation.

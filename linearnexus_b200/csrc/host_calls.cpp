@@ -18,6 +18,7 @@
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdint>
@@ -313,7 +314,9 @@ PyObject* py_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const double scale = a[8] == Py_None ? 1.0 / std::sqrt((double)K) : as_double(a[8]);
     const DrDesc d = make_desc(variant, DR_LAYOUT_BTHD, 1, H, longest, K, V, as_int(a[9]), dt, g_dt, (int)out, a[10] == Py_True, scale, 0, Hq);
     need(!PyErr_Occurred());
-    const int64_t ws_bytes = api.workspace_bytes(&d, 0);
+    DrDesc dw = d;   // room for every sequence's chunks at once (one launch over all of them)
+    dw.T = (int32_t)std::min<int64_t>(total + 64 * (int64_t)n_seqs, INT32_MAX);
+    const int64_t ws_bytes = api.workspace_bytes(&dw, 0);
     if (ws_bytes < 0) return PyLong_FromLong((long)ws_bytes);
     at::Tensor ws;
     if (ws_bytes > 0) ws = c.empty({ws_bytes}, at::kByte);

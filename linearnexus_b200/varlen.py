@@ -117,7 +117,9 @@ def chunkwise_varlen(variant: str, q: Tensor, k: Tensor, v: Tensor, g: Optional[
     d = ops._desc(_VAR[variant], DR_LAYOUT_BTHD, 1, H, longest, K, V, chunk_size, qn, gn, native_out, use_qk_l2norm, scale)
     d.qk_heads = Hq
     lib = _lib.load()
+    d.T = total + 64 * n   # room for every sequence's chunks at once (one launch over all of them)
     need = int(lib.dr_workspace_bytes(ctypes.byref(d), 0))
+    d.T = longest
     if need == -7:
         raise ValueError(f"chunk_size (BT={chunk_size}) must be divisible by BC=16.")
     _lib.check(need if need < 0 else 0, "dr_workspace_bytes")
