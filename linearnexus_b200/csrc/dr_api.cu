@@ -612,7 +612,7 @@ int dr_dplr_recurrent(const void* q, const void* k, const void* v, const void* a
   p.B = B; p.H = H; p.T = T; p.K = K; p.V = V; p.scale = scale;
   p.status = status_dev; p.n_o = ov.n; p.n_state = (int64_t)B * H * K * V;
   tl_path = "dplr_recurrent";
-  cudaError_t e = dr::launch_linrec(dr::LR_DPLR, io_dtype == DR_BF16, p, reinterpret_cast<cudaStream_t>(stream));
+  cudaError_t e = dr::launch_linrec(dr::LR_DPLR, io_dtype == DR_BF16, p, sm_count(), reinterpret_cast<cudaStream_t>(stream));
   g_launches.fetch_add(1);
   return check_cuda(e);
 }
@@ -637,7 +637,7 @@ int dr_rwkv6_recurrent(const void* r, const void* k, const void* v, const void* 
   p.B = B; p.H = H; p.T = T; p.K = K; p.V = V; p.scale = scale;
   p.status = status_dev; p.n_o = ov.n; p.n_state = (int64_t)B * H * K * V;
   tl_path = "rwkv6_recurrent";
-  cudaError_t e = dr::launch_linrec(dr::LR_RWKV6, io_dtype == DR_BF16, p, reinterpret_cast<cudaStream_t>(stream));
+  cudaError_t e = dr::launch_linrec(dr::LR_RWKV6, io_dtype == DR_BF16, p, sm_count(), reinterpret_cast<cudaStream_t>(stream));
   g_launches.fetch_add(1);
   return check_cuda(e);
 }
@@ -666,7 +666,7 @@ int dr_ssd_scan(const void* x, const void* dt, const float* A, const void* Bm, c
   p.B = B; p.H = H; p.T = T; p.K = N; p.V = P; p.scale = 1.f; p.dt_lo = dt_lo; p.dt_hi = dt_hi;
   p.status = status_dev; p.n_o = ov.n; p.n_state = (int64_t)B * H * P * N;
   tl_path = "ssd_scan";
-  cudaError_t e = dr::launch_linrec(dr::LR_SSD, io_dtype == DR_BF16, p, reinterpret_cast<cudaStream_t>(stream));
+  cudaError_t e = dr::launch_linrec(dr::LR_SSD, io_dtype == DR_BF16, p, sm_count(), reinterpret_cast<cudaStream_t>(stream));
   g_launches.fetch_add(1);
   return check_cuda(e);
 }

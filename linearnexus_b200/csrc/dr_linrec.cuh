@@ -330,7 +330,8 @@ inline cudaError_t launch_linrec_kind(const LinRecParams& p, cudaStream_t stream
   return cudaGetLastError();
 }
 
-cudaError_t launch_linrec(int kind, bool io_bf16, const LinRecParams& p, cudaStream_t stream) {
+// the launcher proper (chunk forms and this recurrence) is in dr_scans.cu
+inline cudaError_t launch_linrec_tokens(int kind, bool io_bf16, const LinRecParams& p, cudaStream_t stream) {
   if (io_bf16) {
     if (kind == LR_DPLR) return launch_linrec_kind<LR_DPLR, true>(p, stream);
     if (kind == LR_RWKV6) return launch_linrec_kind<LR_RWKV6, true>(p, stream);

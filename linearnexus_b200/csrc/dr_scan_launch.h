@@ -41,7 +41,7 @@ struct LinRecParams {
 };
 
 // io_bf16: the storage type of q, k, w, a, b, v (one type for all of them); dt of the SSD is float32
-cudaError_t launch_linrec(int kind, bool io_bf16, const LinRecParams& p, cudaStream_t stream);
+cudaError_t launch_linrec(int kind, bool io_bf16, const LinRecParams& p, int sms, cudaStream_t stream);
 // DeltaNet / Gated DeltaNet / KDA token recurrence (p.variant), any K <= 256
 cudaError_t launch_recurrent(const FwdParams& p, cudaStream_t stream);
 

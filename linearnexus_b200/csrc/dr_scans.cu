@@ -1,3 +1,14 @@
-// Translation unit of the token-recurrent scans: the delta-rule recurrence and the RWKV-7 / RWKV-6 / Mamba-2 scans.
+// Translation unit of the scans: the delta-rule recurrence and the RWKV-7 / RWKV-6 / Mamba-2 scans, token by token or in
+// chunk form by shape and storage type.
 #include "dr_linrec.cuh"
 #include "dr_recurrent.cuh"
+#include "dr_ssd_chunk.cuh"
+
+namespace dr {
+
+cudaError_t launch_linrec(int kind, bool io_bf16, const LinRecParams& p, int sms, cudaStream_t stream) {
+  if (kind == LR_SSD && io_bf16 && ssd::eligible(p)) return ssd::launch(p, sms, stream);
+  return launch_linrec_tokens(kind, io_bf16, p, stream);
+}
+
+}  // namespace dr

@@ -30,7 +30,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // Bounded; when the bound runs out every later wait of the CTA returns at once (abort flag), DR_DEV_TIMEOUT is set, and
 // the first such wait of the launch leaves its place in bits 8..15 of the status word (bits 8..13: the barrier's number
 // in the control block, 63 for one behind the float arrays; bits 14..15: the warp group).
-__device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int32_t* status, int* abort_flag, uint32_t bar_offset,
+static __device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int32_t* status, int* abort_flag, uint32_t bar_offset,
                                        uint32_t grp) {
   volatile int* ab = abort_flag;
   if (*ab) return;

@@ -67,7 +67,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 }
 // The same bound with the loop kept out of line: call sites inline one try_wait (the common case: the phase
 // has completed or completes within the hardware's own suspend window) and share this function for the rest.
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t limit) {
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t limit) {
   const long long t_start = clock64();
   for (uint32_t i = 0; i < limit; ++i) {
     if (mbar_try(bar, parity)) return true;
