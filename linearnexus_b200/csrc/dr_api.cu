@@ -10,14 +10,13 @@
 #include "deltarule_sm100.h"
 #include "deltarule_sm100_debug.h"
 #include "dr_chunk_fp32.cuh"
-#include "dr_chunk_sm100.cuh"
-#include "dr_kda_sm100.cuh"
 #include "dr_step_stream.cuh"
-#include "dr_bwd.cuh"
 #include "dr_block_ops.cuh"
 #include "dr_common.cuh"
+#include "dr_launch.h"
 #include "dr_scan_launch.h"
 #include "dr_step.cuh"
+#include "dr_umma_selftest.cuh"
 
 namespace {
 
@@ -100,14 +99,14 @@ int sm_count() {
 }
 
 bool tcgen05_eligible(const DrDesc* d) {
-  return dr::sm100::kAvailable && d->K == 128 && d->V == 128 && d->chunk == 64 &&
+  return d->K == 128 && d->V == 128 && d->chunk == 64 &&
          d->qkv_dtype == DR_BF16 && d->out_dtype == DR_BF16 && (d->variant == DR_GATED || d->variant == DR_DELTA) &&
          (d->variant == DR_DELTA || d->g_dtype == DR_F32);
 }
 
 // the two-kernel form (chunk-parallel intra pass + tcgen05 state pass over a workspace)
 bool split_eligible(const DrDesc* d) {
-  return dr::sm100::kAvailable && d->K == 128 && d->V == 128 && d->chunk == 64 && d->qkv_dtype == DR_BF16;
+  return d->K == 128 && d->V == 128 && d->chunk == 64 && d->qkv_dtype == DR_BF16;
 }
 // AUTO for a shape without a tensor-core kernel: the register-resident token recurrence.  It is the same function of
 // the inputs as the chunk form, does fewer multiply-adds (4 K V per token against the chunk form's 6CK + 4CV + 6KV
@@ -180,7 +179,7 @@ int64_t dr_workspace_bytes(const DrDesc* d, int op) {
   if (s != DR_OK) return s;
   if (op == 0)
     return (resolve_chunk_path(d) == DR_PATH_SPLIT && split_eligible(d))
-               ? dr::kda::workspace_bytes((int64_t)d->B * d->H, d->T) : 0;
+               ? dr::split_workspace_bytes((int64_t)d->B * d->H, d->T) : 0;
   if (op == 1) return dr::bwd_workspace_bytes(d);
   return DR_ERR_UNSUPPORTED;
 }
@@ -197,14 +196,14 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
   int path = resolve_chunk_path(d);
   if (path == DR_PATH_SPLIT) {
     if (!split_eligible(d)) return DR_ERR_UNSUPPORTED;
-    const int64_t need = dr::kda::workspace_bytes((int64_t)d->B * d->H, d->T);
+    const int64_t need = dr::split_workspace_bytes((int64_t)d->B * d->H, d->T);
     // no silent downgrade to the (much slower) kernel that needs no scratch: the caller asks for that one
     // with DR_PATH_FP32
     if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
     if (!workspace || (int64_t)workspace_bytes < need) return DR_ERR_WORKSPACE;
     tl_path = "chunk_split_tcgen05";
     int launches = 0;
-    cudaError_t e = dr::kda::launch_chunk(p, workspace, st, &launches);
+    cudaError_t e = dr::launch_chunk_split(p, workspace, st, &launches);
     g_launches.fetch_add(launches);
     return check_cuda(e);
   }
@@ -212,7 +211,7 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
     if (!tcgen05_eligible(d)) return DR_ERR_UNSUPPORTED;
     tl_path = "chunk_tcgen05";
     g_launches.fetch_add(1);
-    return check_cuda(dr::sm100::launch_chunk(p, st));
+    return check_cuda(dr::launch_chunk_fused(p, st));
   }
   if (path == DR_PATH_FP32 && fp32_chunk_eligible(d)) {
     tl_path = "chunk_fp32";
@@ -247,7 +246,7 @@ int dr_chunk_fwd_varlen(const DrDesc* d, const void* q, const void* k, const voi
     int64_t cap = (int64_t)1 << 30;
     if (split) {
       if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
-      cap = workspace ? (int64_t)workspace_bytes / dr::kda::workspace_bytes(d->H, 64) : 0;
+      cap = workspace ? (int64_t)workspace_bytes / dr::split_workspace_bytes(d->H, 64) : 0;
     }
     const dr::FwdParams p = make_fwd(&da, q, k, v, g, beta, h0, o, hT, status_dev);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -266,7 +265,7 @@ int dr_chunk_fwd_varlen(const DrDesc* d, const void* q, const void* k, const voi
       }
       if (t.n == 0) return DR_ERR_WORKSPACE;
       g_launches.fetch_add(split ? 2 : 1);
-      const cudaError_t e = split ? dr::kda::launch_chunk_packed(p, t, workspace, st) : dr::sm100::launch_chunk_packed(p, t, st);
+      const cudaError_t e = split ? dr::launch_chunk_split_packed(p, t, workspace, st) : dr::launch_chunk_fused_packed(p, t, st);
       if (e != cudaSuccess) return check_cuda(e);
     }
     return DR_OK;

@@ -29,11 +29,10 @@
 
 #include <mutex>
 
-#include "dr_chunk_fp32.cuh"
-#include "dr_scan_launch.h"
-#include "dr_chunk_sm100.cuh"
-#include "dr_kda_sm100.cuh"
 #include "dr_common.cuh"
+#include "dr_launch.h"
+#include "dr_scan_launch.h"
+#include "dr_sm100_common.cuh"
 
 namespace dr {
 
@@ -1276,7 +1275,7 @@ inline bool bwd_tensor_core_path(const DrDesc* d) {
   return d->variant != DR_KDA && d->qkv_dtype == DR_BF16 && d->chunk == 64 && d->K % 16 == 0 && d->V % 8 == 0;
 }
 
-inline int64_t bwd_workspace_bytes(const DrDesc* d) {
+int64_t bwd_workspace_bytes(const DrDesc* d) {
   if (!bwd_supported(d)) return DR_ERR_UNSUPPORTED;
   const int64_t N = (d->T + d->chunk - 1) / d->chunk;
   const int64_t units = (int64_t)d->B * d->H;
@@ -1352,9 +1351,9 @@ inline cudaError_t bwd_side_stream(cudaStream_t* out) {
 // accumulator part of the workspace (262 KB per chunk there against 66 KB of records; the adjoint overwrites it).
 // own_stream: the pre-pass may run on the library's side stream, forked from and joined to `stream` with events
 // (false for callers that must not create streams or events: the pre-pass then runs on `stream` before the forward).
-inline cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
+cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                                       const float* beta, const float* h0, void* o, float* hT, void* workspace,
-                                      int32_t* status, cudaStream_t stream, int* launches, bool own_stream = true) {
+                                      int32_t* status, cudaStream_t stream, int* launches, bool own_stream) {
   const int C = d->chunk, K = d->K, V = d->V;
   cudaEvent_t joined = nullptr;
   if (d->variant != DR_KDA && bwd_tensor_core_path(d)) {
@@ -1387,18 +1386,18 @@ inline cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void
   f.variant = d->variant; f.qkv_dt = d->qkv_dtype; f.g_dt = d->g_dtype; f.out_dt = o ? d->out_dtype : d->qkv_dtype;
   f.l2norm = d->use_qk_l2norm; f.scale = d->scale;
   f.set_extents();
-  const bool tc_shape = sm100::kAvailable && K == 128 && V == 128 && C == 64 && d->qkv_dtype == DR_BF16;
+  const bool tc_shape = K == 128 && V == 128 && C == 64 && d->qkv_dtype == DR_BF16;
   // the tensor-core forwards write the same checkpoints when the shape qualifies
   const bool fused = tc_shape && (d->variant == DR_DELTA || (d->variant == DR_GATED && d->g_dtype == DR_F32)) &&
                      (!o || d->out_dtype == DR_BF16);
   const bool split = tc_shape && !fused && d->variant == DR_KDA;
   cudaError_t e;
   if (fused) {
-    e = sm100::launch_chunk(f, stream);
+    e = launch_chunk_fused(f, stream);
     ++*launches;
   } else if (split) {
     int n2 = 0;
-    e = kda::launch_chunk(f, ckpt + units * N * K * V, stream, &n2);
+    e = launch_chunk_split(f, ckpt + units * N * K * V, stream, &n2);
     *launches += n2;
   } else {
     // every other shape: the token recurrence (the same function of the inputs as the chunk form, and on the CUDA
@@ -1414,7 +1413,7 @@ inline cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void
   return e;
 }
 
-inline cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
+cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                                       const float* beta, const void* d_o, const float* d_hT, void* dq, void* dk,
                                       void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
                                       cudaStream_t stream, int* launches) {
@@ -1478,10 +1477,10 @@ inline cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void
 }
 
 // forward recomputation + adjoint (dr_chunk_bwd)
-inline cudaError_t launch_bwd(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
+cudaError_t launch_bwd(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                               const float* beta, const float* h0, const void* d_o, const float* d_hT, void* dq,
                               void* dk, void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
-                              int32_t* status, cudaStream_t stream, int* launches, bool own_stream = true) {
+                              int32_t* status, cudaStream_t stream, int* launches, bool own_stream) {
   // only the forward has bounded waits that can report; the adjoint kernels synchronise with block barriers
   cudaError_t e = launch_bwd_forward(d, q, k, v, g, beta, h0, nullptr, nullptr, workspace, status, stream, launches,
                                      own_stream);

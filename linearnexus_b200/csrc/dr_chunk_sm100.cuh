@@ -55,12 +55,10 @@
 #include "dr_common.cuh"
 #include "dr_sm100_common.cuh"
 #include "dr_tcgen05.cuh"
-#include "dr_umma_selftest.cuh"
 
 namespace dr {
 namespace sm100 {
 
-constexpr bool kAvailable = true;
 constexpr int kThreads = 512;
 constexpr int kGrp = 128;
 

@@ -45,7 +45,7 @@ static __device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int
 // Test kernel of the record above: one thread waits, with this very routine and its full bound (about a second of SM
 // clock), on an mbarrier that nothing arrives on.  The status word gets DR_DEV_TIMEOUT and the site given here; a second
 // wait of the same CTA returns at once (abort flag) and leaves the record alone.  The kernel returns normally.
-__global__ void wait_site_kernel(int32_t* status, uint32_t barrier_number, uint32_t grp) {
+static __global__ void wait_site_kernel(int32_t* status, uint32_t barrier_number, uint32_t grp) {
   __shared__ __align__(8) uint64_t bar;
   __shared__ int abort_flag;
   if (threadIdx.x == 0) {

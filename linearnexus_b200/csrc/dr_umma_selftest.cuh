@@ -12,7 +12,7 @@
 namespace dr {
 namespace sm100 {
 
-__global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16* __restrict__ A,
+static __global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16* __restrict__ A,
                                                             const __nv_bfloat16* __restrict__ B,
                                                             float* __restrict__ D, int Kd, int N, int a_tmem,
                                                             int b_mn, int32_t* status) {
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16*
 
 // One warp waits on an mbarrier that nothing ever arrives on, with the bounded wait the kernels use and a
 // small attempt limit: the wait gives up, the status word gets DR_DEV_TIMEOUT, the kernel returns normally.
-__global__ void wait_timeout_kernel(int32_t* status, uint32_t attempts) {
+static __global__ void wait_timeout_kernel(int32_t* status, uint32_t attempts) {
   __shared__ __align__(8) uint64_t bar;
   if (threadIdx.x == 0) {
     tc::mbar_init(tc::smem_u32(&bar), 1);
