@@ -30,6 +30,7 @@
 #include <mutex>
 
 #include "dr_common.cuh"
+#include "dr_bwd_chunk.cuh"
 #include "dr_launch.h"
 #include "dr_scan_launch.h"
 #include "dr_sm100_common.cuh"
@@ -1277,6 +1278,7 @@ inline bool bwd_tensor_core_path(const DrDesc* d) {
 
 int64_t bwd_workspace_bytes(const DrDesc* d) {
   if (!bwd_supported(d)) return DR_ERR_UNSUPPORTED;
+  if (bwdc::eligible(d)) return bwdc::workspace_bytes(d);
   const int64_t N = (d->T + d->chunk - 1) / d->chunk;
   const int64_t units = (int64_t)d->B * d->H;
   const int64_t rows = units * N * d->chunk;
@@ -1356,7 +1358,11 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
                                       int32_t* status, cudaStream_t stream, int* launches, bool own_stream) {
   const int C = d->chunk, K = d->K, V = d->V;
   cudaEvent_t joined = nullptr;
-  if (d->variant != DR_KDA && bwd_tensor_core_path(d)) {
+  const bool chunked = bwdc::eligible(d);
+  auto pre = [&](cudaStream_t s) {
+    return chunked ? bwdc::launch_pre(d, q, k, g, beta, workspace, s, launches) : launch_bwd_pre(d, q, k, g, beta, workspace, s, launches);
+  };
+  if (chunked || bwd_tensor_core_path(d)) {
     cudaStream_t side = nullptr;
     cudaEvent_t forked = nullptr;
     if (own_stream && bwd_side_stream(&side) == cudaSuccess &&
@@ -1364,14 +1370,14 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
         cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess) {
       cudaError_t ef = cudaEventRecord(forked, stream);
       if (ef == cudaSuccess) ef = cudaStreamWaitEvent(side, forked, 0);
-      if (ef == cudaSuccess) ef = launch_bwd_pre(d, q, k, g, beta, workspace, side, launches);
+      if (ef == cudaSuccess) ef = pre(side);
       if (ef == cudaSuccess) ef = cudaEventRecord(joined, side);
       cudaEventDestroy(forked);   // released once the work recorded in it has completed
       if (ef != cudaSuccess) { cudaEventDestroy(joined); return ef; }
     } else {
       if (forked) cudaEventDestroy(forked);
       if (joined) { cudaEventDestroy(joined); joined = nullptr; }
-      const cudaError_t ep = launch_bwd_pre(d, q, k, g, beta, workspace, stream, launches);
+      const cudaError_t ep = pre(stream);
       if (ep != cudaSuccess) return ep;
     }
   }
@@ -1397,7 +1403,8 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
     ++*launches;
   } else if (split) {
     int n2 = 0;
-    e = launch_chunk_split(f, ckpt + units * N * K * V, stream, &n2);
+    // its records lie where dS1 of every chunk will be written (bwdc::Params)
+    e = launch_chunk_split(f, bwdc::make_params(d, workspace).ds, stream, &n2);
     *launches += n2;
   } else {
     // every other shape: the token recurrence (the same function of the inputs as the chunk form, and on the CUDA
@@ -1418,6 +1425,25 @@ cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, co
                                       void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
                                       cudaStream_t stream, int* launches) {
   const int C = d->chunk, K = d->K, V = d->V;
+  if (bwdc::eligible(d)) {
+    bwdc::Params p = bwdc::make_params(d, workspace);
+    p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta; p.d_o = d_o; p.d_hT = d_hT;
+    p.dq = dq; p.dk = dk; p.dv = dv; p.dbeta = dbeta; p.dg = dg; p.dh0 = dh0;
+    const int64_t units = (int64_t)d->B * d->H;
+    cudaError_t e = d->variant == DR_KDA ? bwdc::launch_adjoint_t<true>(p, units, stream) : bwdc::launch_adjoint_t<false>(p, units, stream);
+    *launches += 2;
+    if (e != cudaSuccess || p.map.Hq == p.map.H) return e;
+    // grouped q/k heads: the heads' dq^, dk^ summed over each group, then the chain rule
+    BwdFinalParams fp{};
+    fp.q = q; fp.k = k; fp.dq = dq; fp.dk = dk;
+    fp.dq_acc = p.part; fp.dk_acc = p.part + units * p.N * (C * K);
+    fp.map = p.map; fp.K = K; fp.C = C; fp.N = p.N; fp.variant = DR_DELTA; fp.qkv_dt = d->qkv_dtype;
+    fp.l2norm = d->use_qk_l2norm; fp.scale = d->scale;
+    fp.nvs = 1; fp.slice_stride = 0;
+    bwd_finalize_kernel<<<(unsigned)(units * p.N), 256, 0, stream>>>(fp);
+    ++*launches;
+    return cudaGetLastError();
+  }
   const BwdRegions rg = bwd_regions(d, workspace);
   const int64_t N = rg.N, units = rg.units, rows = rg.rows, nvs = rg.nvs;
   float *ckpt = rg.ckpt, *dq_acc = rg.dq_acc, *dk_acc = rg.dk_acc, *dg_acc = rg.dg_acc, *pre = rg.pre;

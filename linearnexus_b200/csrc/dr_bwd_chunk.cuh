@@ -1,0 +1,1281 @@
+// Backward of the chunkwise delta rule for bf16 inputs at K = V = 128, C = 64 (all three variants): the adjoint split
+// into what is serial over the chunks and what is not.  Formulas and names: header of dr_bwd.cuh.
+//
+// With W = T diag(beta) K^ e^G, Y = Q^ e^G - A W and N = -W^T Kd (Kd = K^ e^{G_L - G}) the state gradient obeys
+//     dS0 = e^{G_L} dS1 + N dS1 + Y^T dO
+// one [128 x 128] product per chunk and nothing else on the chain.  Three kernels:
+//
+//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as the A fragments of
+//                 mma.sync in the order the lanes of state_kernel load them (16 bytes per lane, no shared memory).
+//   state_kernel  one CTA per (sequence, 32 value columns) walks the chunks backwards; dS stays in accumulator
+//                 registers, its copy in shared memory is the B operand; stores dS1 of every chunk.
+//   local_kernel  one CTA per chunk, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1
+//                 and the chunk's inputs, looping over four value slices with the sums over v in registers; then the
+//                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
+//                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
+//                 finalize kernel).
+//
+// The one-CTA-per-sequence-slice adjoint it replaces here walked all of a chunk's work in sequence (B=2, T=4096, H=16:
+// 1.26 ms; with per-channel decay 12 ms on the CUDA cores) and stored four fp32 copies of dq^, dk^.
+//
+// Products are mma.sync tf32 with fp32 operands.  DeltaNet / Gated DeltaNet: one product (operands cut to tf32, as the
+// adjoint they replace).  KDA: three products per pair (x = hi + lo, lo lo dropped), i.e. float32 precision, as the
+// CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
+// referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
+// decay range exceeds 2^64 is summed exactly.
+#pragma once
+
+#include "dr_common.cuh"
+#include "dr_mma.cuh"
+#include "dr_sm100_common.cuh"
+
+namespace dr {
+namespace bwdc {
+
+using sm100::LDT;
+constexpr int kC = 64, kD = 128;
+constexpr int kVS = 32;   // value columns per slice
+
+struct Params {
+  const void* q; const void* k; const void* v; const void* g; const float* beta; const void* d_o; const float* d_hT;
+  void* dq; void* dk; void* dv; float* dbeta; float* dg; float* dh0;
+  const float* ckpt;    // [units][N][128][128] state at the start of every chunk
+  float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]
+  float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]
+  float* xat;           // [units][N][3][64][64] X, A, T
+  float* ds;            // [units][N][128][128] dS1
+  float* el;            // [units][N][128] e^{G_L}
+  float* part;          // grouped heads: dq^ [units][N*64][128], then dk^ (over nf)
+  SeqMap map;
+  int N, variant, g_dt, l2norm;
+  float scale;
+};
+
+// float2 from shared memory
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float bf(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ float ex2(float x) { return tc::fast_exp2(x); }
+constexpr float kLog2e = 1.4426950408889634f;
+
+// One operand of a tf32 product; X3: its leading 11 bits and the rest.
+template <bool X3>
+struct AFrag {
+  uint32_t h[4], l[X3 ? 4 : 1];
+  __device__ __forceinline__ void set(float a0, float a1, float a2, float a3) {
+    const float a[4] = {a0, a1, a2, a3};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      h[i] = __float_as_uint(a[i]);
+      if constexpr (X3) {
+        h[i] &= 0xffffe000u;
+        l[i] = __float_as_uint(a[i] - __uint_as_float(h[i]));
+      }
+    }
+  }
+};
+template <bool X3>
+struct BFrag {
+  uint32_t h[2], l[X3 ? 2 : 1];
+  __device__ __forceinline__ void set(float b0, float b1) {
+    h[0] = __float_as_uint(b0); h[1] = __float_as_uint(b1);
+    if constexpr (X3) {
+      h[0] &= 0xffffe000u; h[1] &= 0xffffe000u;
+      l[0] = __float_as_uint(b0 - __uint_as_float(h[0]));
+      l[1] = __float_as_uint(b1 - __uint_as_float(h[1]));
+    }
+  }
+};
+template <bool X3>
+__device__ __forceinline__ void fma(float (&d)[4], const AFrag<X3>& a, const BFrag<X3>& b) {
+  if constexpr (X3) {
+    sm100::mma_tf32(d, a.l, b.h);
+    sm100::mma_tf32(d, a.h, b.l);
+  }
+  sm100::mma_tf32(d, a.h, b.h);
+}
+__device__ __forceinline__ void zero4(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
+// value as the product will see it, rounded to nearest instead of cut (single-product operands that are stored)
+template <bool X3>
+__device__ __forceinline__ float stored(float x) { return X3 ? x : __uint_as_float(sm100::to_tf32(x)); }
+
+// In-place inclusive prefix sum over the 64 rows of sG [64][132] per channel; NTHR threads, `seg` scratch of
+// NTHR / 32 rows x 128 floats.  Ends with a barrier.
+template <int NTHR>
+__device__ __forceinline__ void scan_channels(float* sG, float* seg, int tid) {
+  constexpr int R = 64 / (NTHR / 32);   // rows per segment
+  const int s = tid >> 5, c4 = 4 * (tid & 31);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), loc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float4 x = *reinterpret_cast<const float4*>(sG + (R * s + r) * 132 + c4);
+    acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    loc[r] = acc;
+  }
+  *reinterpret_cast<float4*>(seg + s * 128 + c4) = acc;
+  __syncthreads();
+  float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s2 = 0; s2 < s; ++s2) {
+    const float4 x = *reinterpret_cast<const float4*>(seg + s2 * 128 + c4);
+    pre.x += x.x; pre.y += x.y; pre.z += x.z; pre.w += x.w;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    *reinterpret_cast<float4*>(sG + (R * s + r) * 132 + c4) =
+        make_float4(loc[r].x + pre.x, loc[r].y + pre.y, loc[r].z + pre.z, loc[r].w + pre.w);
+  __syncthreads();
+}
+// four channels of the log decay in log2 units
+__device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
+  float4 x;
+  if (dt == DR_BF16) {
+    const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(g) + at);
+    x = make_float4(mma::lo_f(u.x), mma::hi_f(u.x), mma::lo_f(u.y), mma::hi_f(u.y));
+  } else {
+    x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(g) + at);
+  }
+  return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
+}
+// inclusive sums of 64 scalars, rows lane and lane + 32
+__device__ __forceinline__ void scan_scalars(float& lo, float& hi, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float a = __shfl_up_sync(0xffffffffu, lo, o), b = __shfl_up_sync(0xffffffffu, hi, o);
+    if (lane >= o) { lo += a; hi += b; }
+  }
+  hi += __shfl_sync(0xffffffffu, lo, 31);
+}
+
+// =====================================================================================================================
+// pre_kernel
+// =====================================================================================================================
+constexpr int kPreThreads = 256;
+constexpr int LDH = 136;   // row stride (bf16) of the raw k, q rows
+constexpr int PR_K = 0, PR_Q = PR_K + 64 * LDH * 2, PR_X = PR_Q + 64 * LDH * 2, PR_A = PR_X + 64 * LDT * 4;
+constexpr int PR_SC = PR_A + 64 * 72 * 4;     // beta, rk, rq, G, fw, fd (64 each)
+constexpr int PR_G = PR_SC + 6 * 64 * 4;      // KDA: log2(e) G [64][132]; Kd [64][132] later takes the place of k, q
+template <bool KDA> constexpr int pre_smem() { return KDA ? PR_G + 64 * 132 * 4 : PR_G; }
+static_assert(2 * 64 * LDH * 2 >= 64 * 132 * 4 && 2 * (pre_smem<true>() + 1024) <= 233472, "two CTAs per SM");
+
+template <bool KDA>
+__global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + PR_K);
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + PR_Q);
+  float* sKd = reinterpret_cast<float*>(smem + PR_K);
+  float* sX = reinterpret_cast<float*>(smem + PR_X);
+  float* sA = reinterpret_cast<float*>(smem + PR_A);
+  float* sBeta = reinterpret_cast<float*>(smem + PR_SC);
+  float *sRk = sBeta + 64, *sRq = sBeta + 128, *sGs = sBeta + 192, *sFw = sBeta + 256, *sFd = sBeta + 320;
+  float* sG = reinterpret_cast<float*>(smem + PR_G);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
+  const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
+  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
+  const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);
+  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
+  const int64_t chunk = (int64_t)unit * p.N + n;
+
+  // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
+  {
+    uint2 qr[8], kr[8];
+    float4 gr[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = warp + 8 * i;
+      qr[i] = kr[i] = make_uint2(0u, 0u);
+      gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < rows) {
+        const int64_t at = qk_base + (t0 + c) * qk_tok + 4 * lane;
+        qr[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + at);
+        kr[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at);
+        if constexpr (KDA) gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
+      }
+    }
+    float bt = 0.f, g_lo = 0.f, g_hi = 0.f;
+    if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
+    if (!KDA && warp == 0 && p.variant == DR_GATED) {
+      if (lane < rows) g_lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
+      if (lane + 32 < rows) g_hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = warp + 8 * i;
+      *reinterpret_cast<uint2*>(sQ + c * LDH + 4 * lane) = qr[i];
+      *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kr[i];
+      if constexpr (KDA) *reinterpret_cast<float4*>(sG + c * 132 + 4 * lane) = gr[i];
+      float qmul = p.scale, kmul = 1.f;
+      if (p.l2norm) {
+        const float q0 = mma::lo_f(qr[i].x), q1 = mma::hi_f(qr[i].x), q2 = mma::lo_f(qr[i].y), q3 = mma::hi_f(qr[i].y);
+        const float k0 = mma::lo_f(kr[i].x), k1 = mma::hi_f(kr[i].x), k2 = mma::lo_f(kr[i].y), k3 = mma::hi_f(kr[i].y);
+        qmul = p.scale / (sqrtf(warp_sum(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3)) + 1e-6f);
+        kmul = 1.f / (sqrtf(warp_sum(k0 * k0 + k1 * k1 + k2 * k2 + k3 * k3)) + 1e-6f);
+      }
+      if (lane == i) { sBeta[c] = bt; sRk[c] = kmul; sRq[c] = qmul; }
+    }
+    if (!KDA && warp == 0) {
+      scan_scalars(g_lo, g_hi, lane);
+      sGs[lane] = g_lo; sGs[lane + 32] = g_hi;
+    }
+  }
+  __syncthreads();
+  if constexpr (KDA) {
+    scan_channels<kPreThreads>(sG, sX, tid);
+    if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * 132 + tid]);
+    if (tid < 64) { sFw[tid] = sBeta[tid] * sRk[tid]; }
+  } else {
+    const float gl = sGs[63];
+    if (tid < 128) p.el[chunk * 128 + tid] = expf(gl);
+    if (tid < 64) {   // factors of row j of k in W and in Kd
+      sFw[tid] = sBeta[tid] * sRk[tid] * expf(sGs[tid]);
+      sFd[tid] = sRk[tid] * expf(fminf(gl - sGs[tid], 0.f));
+    }
+  }
+  // ---- X = tril(K^K^^T.E, -1), A = tril(Q^K^^T.E): 20 tiles of 16 x 8 at or below the diagonal dealt to the warps ----------
+  auto unsafe = [&](int blk) -> bool {   // KDA, warp-uniform: the decay inside the block exceeds 2^64 in some channel
+    const float4 ga = *reinterpret_cast<const float4*>(sG + 16 * blk * 132 + 4 * lane);
+    const float4 gb = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
+    return __any_sync(0xffffffffu, !(fmaxf(fmaxf(ga.x - gb.x, ga.y - gb.y), fmaxf(ga.z - gb.z, ga.w - gb.w)) <= 64.f));
+  };
+#pragma unroll 1
+  for (int tile = warp; tile < 20; tile += kPreThreads / 32) {
+    const int mt = tile < 2 ? 0 : tile < 6 ? 1 : tile < 12 ? 2 : 3, nt = tile - mt * (mt + 1);
+    float dk[4], dq[4];
+    zero4(dk); zero4(dq);
+    if constexpr (KDA) {
+      if (nt >= 2 * mt && unsafe(mt)) continue;   // done exactly below
+      const int r0 = 16 * mt + g, r1 = r0 + 8, j = 8 * nt + g, nrow = 16 * mt;
+#pragma unroll 2
+      for (int ks = 0; ks < 16; ++ks) {
+        const int c0 = 8 * ks + t, c1 = c0 + 4;
+        const float n0 = sG[nrow * 132 + c0], n1 = sG[nrow * 132 + c1];
+        const float e00 = ex2(sG[r0 * 132 + c0] - n0), e10 = ex2(sG[r1 * 132 + c0] - n0);
+        const float e01 = ex2(sG[r0 * 132 + c1] - n1), e11 = ex2(sG[r1 * 132 + c1] - n1);
+        AFrag<true> ak, aq;
+        ak.set(bf(sK + r0 * LDH + c0) * e00, bf(sK + r1 * LDH + c0) * e10, bf(sK + r0 * LDH + c1) * e01, bf(sK + r1 * LDH + c1) * e11);
+        aq.set(bf(sQ + r0 * LDH + c0) * e00, bf(sQ + r1 * LDH + c0) * e10, bf(sQ + r0 * LDH + c1) * e01, bf(sQ + r1 * LDH + c1) * e11);
+        BFrag<true> bk;
+        bk.set(bf(sK + j * LDH + c0) * ex2(n0 - sG[j * 132 + c0]), bf(sK + j * LDH + c1) * ex2(n1 - sG[j * 132 + c1]));
+        fma<true>(dk, ak, bk);
+        fma<true>(dq, aq, bk);
+      }
+    } else {   // raw bf16 rows: exact products
+      const uint32_t aK = tc::smem_u32(sK), aQ = tc::smem_u32(sQ);
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) {
+        uint32_t a0[4], a1[4], q0[4], q1[4], bb[4];
+        mma::ldsm4(bb, aK + 2u * ((8 * nt + (lane & 7)) * LDH + 32 * k2 + (lane >> 3) * 8));
+        mma::ldsm4(a0, mma::frag_a(aK, LDH, 16 * mt, 32 * k2, lane));
+        mma::ldsm4(a1, mma::frag_a(aK, LDH, 16 * mt, 32 * k2 + 16, lane));
+        mma::ldsm4(q0, mma::frag_a(aQ, LDH, 16 * mt, 32 * k2, lane));
+        mma::ldsm4(q1, mma::frag_a(aQ, LDH, 16 * mt, 32 * k2 + 16, lane));
+        mma::bf16(dk, a0, bb[0], bb[1]);
+        mma::bf16(dq, q0, bb[0], bb[1]);
+        mma::bf16(dk, a1, bb[2], bb[3]);
+        mma::bf16(dq, q1, bb[2], bb[3]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 16 * mt + g + 8 * (e >> 1), j = 8 * nt + 2 * t + (e & 1);
+      const float f = KDA ? sRk[j] : sRk[j] * __expf(fminf(sGs[i] - sGs[j], 0.f));
+      sX[i * LDT + j] = j < i ? dk[e] * f * sRk[i] : 0.f;
+      sA[i * 72 + j] = j <= i ? dq[e] * f * sRq[i] : 0.f;
+    }
+  }
+  if constexpr (KDA) {   // diagonal blocks with too wide a decay range: exactly, one entry per thread
+    for (int blk = 0; blk < 4; ++blk) {
+      if (!unsafe(blk)) continue;
+      const int i = 16 * blk + (tid >> 4), j = 16 * blk + (tid & 15);
+      float ak = 0.f, aq = 0.f;
+      if (j <= i)
+        for (int c = 0; c < kD; ++c) {
+          const float w = bf(sK + j * LDH + c) * ex2(fminf(sG[i * 132 + c] - sG[j * 132 + c], 0.f));
+          ak += bf(sK + i * LDH + c) * w;
+          aq += bf(sQ + i * LDH + c) * w;
+        }
+      sX[i * LDT + j] = j < i ? ak * sRk[i] * sRk[j] : 0.f;
+      sA[i * 72 + j] = j <= i ? aq * sRq[i] * sRk[j] : 0.f;
+    }
+  }
+  __syncthreads();
+  // ---- X, A -> global (16 x 16 blocks at or below the diagonal), then T in place of X ----------------------------------------
+  float* xat = p.xat + chunk * (3 * 64 * 64);
+  for (int i = tid; i < 64 * 16; i += kPreThreads) {
+    const int r = i >> 4, c4 = (i & 15) * 4;
+    if ((c4 >> 4) <= (r >> 4)) {
+      *reinterpret_cast<float4*>(xat + r * 64 + c4) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
+    }
+  }
+  __syncthreads();
+  sm100::block_inverse_64(sX, sBeta, sX, tid);   // ends with a barrier
+  for (int i = tid; i < 64 * 16; i += kPreThreads) {
+    const int r = i >> 4, c4 = (i & 15) * 4;
+    if ((c4 >> 4) <= (r >> 4)) {
+      float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      if (c4 + 0 > r) v.x = 0.f;
+      if (c4 + 1 > r) v.y = 0.f;
+      if (c4 + 2 > r) v.z = 0.f;
+      if (c4 + 3 > r) v.w = 0.f;
+      *reinterpret_cast<float4*>(xat + 8192 + r * 64 + c4) = v;
+    }
+  }
+  // ---- W^T: rows = the warp's 16 channels, columns = tokens; W = T diag(beta) K^ e^G ----------------------------------------
+  constexpr bool X3 = KDA;
+  const int ch0 = 16 * warp + g, ch1 = ch0 + 8;
+  float W[8][4];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) zero4(W[nt]);
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    const int j0 = 8 * ks + t, j1 = j0 + 4;
+    float a0 = bf(sK + j0 * LDH + ch0), a1 = bf(sK + j0 * LDH + ch1), a2 = bf(sK + j1 * LDH + ch0), a3 = bf(sK + j1 * LDH + ch1);
+    if constexpr (KDA) {
+      a0 *= ex2(sG[j0 * 132 + ch0]); a1 *= ex2(sG[j0 * 132 + ch1]);
+      a2 *= ex2(sG[j1 * 132 + ch0]); a3 *= ex2(sG[j1 * 132 + ch1]);
+    }
+    AFrag<X3> a;
+    a.set(a0, a1, a2, a3);
+    const float f0 = sFw[j0], f1 = sFw[j1];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      if (nt >= ks) {
+        const int i = 8 * nt + g;
+        BFrag<X3> bt;
+        bt.set(j0 <= i ? sX[i * LDT + j0] * f0 : 0.f, j1 <= i ? sX[i * LDT + j1] * f1 : 0.f);
+        fma<X3>(W[nt], a, bt);
+      }
+    }
+  }
+  // ---- Y^T = (Q^ e^G)^T - W^T A^T -> fragments of the state kernel (an accumulator is a fragment with its columns as k) --------
+  {
+    float Y[8][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int ch = e < 2 ? ch0 : ch1, i = 8 * nt + 2 * t + (e & 1);
+        Y[nt][e] = bf(sQ + i * LDH + ch) * sRq[i] * (KDA ? ex2(sG[i * 132 + ch]) : expf(sGs[i]));
+      }
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      AFrag<X3> a;
+      a.set(-W[ks][0], -W[ks][2], -W[ks][1], -W[ks][3]);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        if (nt >= ks) {
+          const float2 y = ld2(sA + (8 * nt + g) * 72 + 8 * ks + 2 * t);
+          BFrag<X3> ba;
+          ba.set(y.x, y.y);
+          fma<X3>(Y[nt], a, ba);
+        }
+      }
+    }
+    float4* dst = p.yf + (chunk * 8 + warp) * 8 * 32 + lane;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+      dst[nt * 32] = make_float4(stored<X3>(Y[nt][0]), stored<X3>(Y[nt][2]), stored<X3>(Y[nt][1]), stored<X3>(Y[nt][3]));
+  }
+  // ---- N = -W^T Kd -> fragments -----------------------------------------------------------------------------------------------
+  if constexpr (KDA) {
+    float4 kd[8];
+    const float4 gl = *reinterpret_cast<const float4*>(sG + 63 * 132 + 4 * lane);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = warp + 8 * i;
+      const uint2 u = *reinterpret_cast<const uint2*>(sK + c * LDH + 4 * lane);
+      const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
+      const float r = sRk[c];
+      kd[i] = make_float4(mma::lo_f(u.x) * r * ex2(gl.x - gg.x), mma::hi_f(u.x) * r * ex2(gl.y - gg.y),
+                          mma::lo_f(u.y) * r * ex2(gl.z - gg.z), mma::hi_f(u.y) * r * ex2(gl.w - gg.w));
+    }
+    __syncthreads();   // every read of k and q is done
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(sKd + (warp + 8 * i) * 132 + 4 * lane) = kd[i];
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    float d[8][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) zero4(d[nt]);
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const int i0 = 8 * ks + 2 * t;
+      const float f0 = KDA ? -1.f : -sFd[i0], f1 = KDA ? -1.f : -sFd[i0 + 1];
+      AFrag<X3> a;
+      a.set(W[ks][0] * f0, W[ks][2] * f0, W[ks][1] * f1, W[ks][3] * f1);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        const int c = 64 * half + 8 * nt + g;
+        BFrag<X3> bk;
+        if constexpr (KDA) bk.set(sKd[i0 * 132 + c], sKd[(i0 + 1) * 132 + c]);
+        else bk.set(bf(sK + i0 * LDH + c), bf(sK + (i0 + 1) * LDH + c));
+        fma<X3>(d[nt], a, bk);
+      }
+    }
+    float4* dst = p.nf + ((chunk * 8 + warp) * 16 + 8 * half) * 32 + lane;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+      dst[nt * 32] = make_float4(stored<X3>(d[nt][0]), stored<X3>(d[nt][2]), stored<X3>(d[nt][1]), stored<X3>(d[nt][3]));
+  }
+}
+
+// =====================================================================================================================
+// state_kernel: eight warps, warp w owns channel rows 16 w .. 16 w + 15 of dS [128][32]
+// =====================================================================================================================
+constexpr int kStThreads = 256;
+constexpr int kStSmem = 2 * 96 * 72 * 4;
+constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved, [rows / 2][32 columns][2], 72 floats per pair
+
+template <bool X3>
+__global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * LDP]
+  float* sO = sS + 2 * 64 * LDP;                        // [2][32 * LDP]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int unit = blockIdx.x >> 2, v0 = (blockIdx.x & 3) * kVS;
+  const int b = unit / p.map.H, h = unit % p.map.H;
+  const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
+  const int r0 = 16 * warp + g, r1 = r0 + 8;
+  float S[4][4];   // tile nt: rows r0, r1; columns 8 nt + 2t, + 1
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    float2 lo = make_float2(0.f, 0.f), hi = lo;
+    if (p.d_hT) {
+      lo = *reinterpret_cast<const float2*>(p.d_hT + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t);
+      hi = *reinterpret_cast<const float2*>(p.d_hT + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t);
+    }
+    S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
+  }
+  const int orow = tid >> 2, ocol = (tid & 3) * 8;   // this thread's eight columns of dO
+  auto load_do = [&](int n) -> uint4 {
+    const int tok = n * kC + orow;
+    if (n < 0 || tok >= p.map.T) return make_uint4(0u, 0u, 0u, 0u);
+    return *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_o) + v_base + (int64_t)tok * v_tok + v0 + ocol);
+  };
+  const int64_t chunk0 = (int64_t)unit * p.N;
+  float4 nf[16], yf[8];
+  float el0, el1;
+  {
+    const int64_t c = chunk0 + p.N - 1;
+#pragma unroll
+    for (int ks = 0; ks < 16; ++ks) nf[ks] = __ldcs(p.nf + ((c * 8 + warp) * 16 + ks) * 32 + lane);
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) yf[ks] = __ldcs(p.yf + ((c * 8 + warp) * 8 + ks) * 32 + lane);
+    el0 = p.el[c * 128 + r0]; el1 = p.el[c * 128 + r1];
+  }
+  uint4 dor = load_do(p.N - 1);
+  for (int n = p.N - 1; n >= 0; --n) {
+    float* cS = sS + (n & 1) * 64 * LDP;
+    float* cO = sO + (n & 1) * 32 * LDP;
+    // dS1 of this chunk: to memory, and to the other warps
+    float* out = p.ds + (chunk0 + n) * (kD * kD) + v0;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = 8 * nt + 2 * t;
+      *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
+      float* w0 = cS + (r0 >> 1) * LDP + 2 * c + (r0 & 1);
+      float* w1 = cS + (r1 >> 1) * LDP + 2 * c + (r1 & 1);
+      w0[0] = S[nt][0]; w0[2] = S[nt][1];
+      w1[0] = S[nt][2]; w1[2] = S[nt][3];
+    }
+    {
+      const uint32_t w[4] = {dor.x, dor.y, dor.z, dor.w};
+      float* o = cO + (orow >> 1) * LDP + 2 * ocol + (orow & 1);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { o[4 * e] = mma::lo_f(w[e]); o[4 * e + 2] = mma::hi_f(w[e]); }
+    }
+    const int64_t cn = chunk0 + (n > 0 ? n - 1 : 0);   // the next chunk's operands replace this one's as they are used
+    dor = load_do(n - 1);
+    __syncthreads();
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) { S[nt][0] *= el0; S[nt][1] *= el0; S[nt][2] *= el1; S[nt][3] *= el1; }
+    el0 = p.el[cn * 128 + r0]; el1 = p.el[cn * 128 + r1];
+    float Z[4][4];   // second accumulator: shorter chains
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) zero4(Z[nt]);
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      AFrag<X3> a;
+      a.set(yf[ks].x, yf[ks].y, yf[ks].z, yf[ks].w);
+      yf[ks] = __ldcs(p.yf + ((cn * 8 + warp) * 8 + ks) * 32 + lane);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const float2 y = ld2(cO + (4 * ks + t) * LDP + 2 * (8 * nt + g));
+        BFrag<X3> bo;
+        bo.set(y.x, y.y);
+        fma<X3>(Z[nt], a, bo);
+      }
+    }
+#pragma unroll
+    for (int ks = 0; ks < 16; ++ks) {
+      AFrag<X3> a;
+      a.set(nf[ks].x, nf[ks].y, nf[ks].z, nf[ks].w);
+      nf[ks] = __ldcs(p.nf + ((cn * 8 + warp) * 16 + ks) * 32 + lane);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
+        BFrag<X3> bs;
+        bs.set(y.x, y.y);
+        if (ks & 1) fma<X3>(Z[nt], a, bs); else fma<X3>(S[nt], a, bs);
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[nt][e] += Z[nt][e];
+  }
+  if (p.dh0) {
+    float* out = p.dh0 + (int64_t)unit * kD * kD + v0;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = 8 * nt + 2 * t;
+      *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
+    }
+  }
+}
+
+// =====================================================================================================================
+// local_kernel: sixteen warps; warp w works on token rows 16 (w >> 2) .. and on a quarter of the columns, w & 3
+// =====================================================================================================================
+constexpr int kLoThreads = 512;
+constexpr int LDV = 40;    // row stride of the value-slice arrays
+constexpr int LDA = 72;    // of A, dA, dX
+// phase 1 (bytes): k^ (KDA: k^ e^G and k^ e^{G_L - G}), A, T, then V, dO, Vn, dR [64][40] and two buffers of S0, dS [128][40]
+template <bool KDA>
+struct LoSmem {
+  static constexpr int kK = 0, kKd = kK + 64 * 132 * 4;
+  static constexpr int kA = kKd + (KDA ? 64 * 132 * 4 : 0), kT = kA + 64 * LDA * 4;
+  static constexpr int kV = kT + 64 * LDT * 4, kSl = 64 * LDV * 4;   // V, dO, Vn, dR
+  static constexpr int kSD = kV + 4 * kSl, kS1 = 128 * LDV * 4;        // [2][S0, dS]
+  static constexpr int kSc = kSD + 4 * kS1;
+  static constexpr int kTotal = kSc + (10 * 64 + 3 * 128) * 4;
+  // final phase: DeltaNet / Gated: dX over V .. , q^ over the S0, dS buffers; KDA: its own map from 0
+  static constexpr int fX = kV, fQ = kSD;
+  static constexpr int gQS = 0, gKS = 64 * 132 * 4, gKE = 2 * gKS, gG = 3 * gKS, gA = 4 * gKS, gX = gA + 64 * LDA * 4, gD = gX + 64 * LDA * 4;
+  static constexpr int gSeg = gD + 4 * 128 * 4;   // [16][128] scan scratch
+  static_assert(64 * LDA * 4 <= 4 * kSl && 64 * 136 * 4 <= 4 * kS1 && gSeg + 16 * 128 * 4 <= kSc && kTotal <= 232448, "shared memory");
+};
+
+template <bool KDA>
+__global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
+  using L = LoSmem<KDA>;
+  constexpr bool X3 = KDA;
+  extern __shared__ __align__(16) uint8_t smem[];
+  auto F = [&](int off) { return reinterpret_cast<float*>(smem + off); };
+  float *sK = F(L::kK), *sKd = F(L::kKd), *sA = F(L::kA), *sT = F(L::kT);
+  float *sV = F(L::kV), *sdO = F(L::kV + L::kSl), *sVn = F(L::kV + 2 * L::kSl), *sdR = F(L::kV + 3 * L::kSl);
+  float* sBeta = F(L::kSc);
+  float *sEG = sBeta + 64, *sWd = sBeta + 128, *sGs = sBeta + 192, *sRk = sBeta + 256, *sRq = sBeta + 320;
+  float *sdB = sBeta + 384, *sdG = sBeta + 448, *sDq = sBeta + 512, *sDk = sBeta + 576;
+  float *sTS = sBeta + 640, *sEx = sBeta + 768, *sUn = sBeta + 896;   // <dS1, S0> per channel; KDA: sums for dG_L, block flags
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
+  const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
+  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
+  const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);
+  const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
+  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
+  const int64_t chunk = (int64_t)unit * p.N + n;
+  const float* xat = p.xat + chunk * (3 * 64 * 64);
+  const __nv_bfloat16 *gq = reinterpret_cast<const __nv_bfloat16*>(p.q), *gk = reinterpret_cast<const __nv_bfloat16*>(p.k);
+  const int m0 = 16 * (warp >> 2), wc = warp & 3;
+
+  // S0, dS columns of one value slice -> buffer, 16 bytes per copy
+  auto issue_slice = [&](int s) {
+    float* dst = F(L::kSD + (s & 1) * 2 * L::kS1);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int i = tid + kLoThreads * it, which = i >> 10, r = (i >> 3) & 127, c4 = (i & 7) * 4;
+      const float* src = (which ? p.ds : p.ckpt) + chunk * (kD * kD) + r * kD + s * kVS + c4;
+      tc::cp_async16(tc::smem_u32(dst + which * (128 * LDV) + r * LDV + c4), src, true);
+    }
+    tc::cp_async_commit();
+  };
+  // V, dO of one slice: thread = eight columns of one row of one of the two arrays
+  const int vrow = (tid & 255) >> 2, vcol = (tid & 3) * 8;
+  auto load_v = [&](int s) -> uint4 {
+    if (vrow >= rows) return make_uint4(0u, 0u, 0u, 0u);
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(tid < 256 ? p.v : p.d_o);
+    return *reinterpret_cast<const uint4*>(src + v_base + (int64_t)(t0 + vrow) * v_tok + s * kVS + vcol);
+  };
+  // ---- stage what all slices share ----------------------------------------------------------------------------------------------
+  for (int i = tid; i < 2 * 64 * 16; i += kLoThreads) {
+    const int m = i >> 10, r = (i >> 4) & 63, c4 = (i & 15) * 4;
+    if ((c4 >> 4) <= (r >> 4))
+      tc::cp_async16(tc::smem_u32((m ? sT + r * LDT : sA + r * LDA) + c4), xat + (1 + m) * 4096 + r * 64 + c4, true);
+  }
+  issue_slice(0);
+  uint4 vr = load_v(0);
+  {
+    uint2 kr[4];
+    float4 gr[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = warp + 16 * i;
+      kr[i] = make_uint2(0u, 0u);
+      gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < rows) {
+        kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
+        if constexpr (KDA) gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
+      }
+    }
+    if (tid < 64) {
+      sBeta[tid] = tid < rows ? p.beta[s_base + (t0 + tid) * s_tok] : 0.f;
+      sdB[tid] = sdG[tid] = sDq[tid] = sDk[tid] = 0.f;
+    }
+    if (tid < 128) sTS[tid] = sEx[tid] = 0.f;
+    if (!KDA && warp == 15) {
+      float lo = 0.f, hi = 0.f;
+      if (p.variant == DR_GATED) {
+        if (lane < rows) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
+        if (lane + 32 < rows) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
+      }
+      scan_scalars(lo, hi, lane);
+      const float gl = __shfl_sync(0xffffffffu, hi, 31);
+      sGs[lane] = lo; sGs[lane + 32] = hi;
+      sEG[lane] = expf(lo); sEG[lane + 32] = expf(hi);
+      sWd[lane] = expf(fminf(gl - lo, 0.f)); sWd[lane + 32] = expf(fminf(gl - hi, 0.f));
+    }
+    float* sG = F(L::kSD + 2 * L::kS1);   // KDA: the second slice buffer, not yet in use (behind it: scan scratch)
+    if constexpr (KDA) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
+      __syncthreads();
+      scan_channels<kLoThreads>(sG, sVn, tid);   // scratch 8 KB
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = warp + 16 * i;
+      const float k0 = mma::lo_f(kr[i].x), k1 = mma::hi_f(kr[i].x), k2 = mma::lo_f(kr[i].y), k3 = mma::hi_f(kr[i].y);
+      const float nrm = p.l2norm ? sqrtf(warp_sum(k0 * k0 + k1 * k1 + k2 * k2 + k3 * k3)) : 0.f;
+      const float m = p.l2norm ? 1.f / (nrm + 1e-6f) : 1.f;
+      if (lane == 0) sRk[c] = m;
+      if constexpr (KDA) {
+        const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane), gl = *reinterpret_cast<const float4*>(sG + 63 * 132 + 4 * lane);
+        *reinterpret_cast<float4*>(sK + c * 132 + 4 * lane) =
+            make_float4(k0 * m * ex2(gg.x), k1 * m * ex2(gg.y), k2 * m * ex2(gg.z), k3 * m * ex2(gg.w));
+        *reinterpret_cast<float4*>(sKd + c * 132 + 4 * lane) =
+            make_float4(k0 * m * ex2(gl.x - gg.x), k1 * m * ex2(gl.y - gg.y), k2 * m * ex2(gl.z - gg.z), k3 * m * ex2(gl.w - gg.w));
+      } else {
+        *reinterpret_cast<float4*>(sK + c * 132 + 4 * lane) = make_float4(k0 * m, k1 * m, k2 * m, k3 * m);
+      }
+    }
+  }
+  float dQ[4][4], dKr[4][4], dKc[4][4], da[2][4], dm[2][4];   // dQg, dKg (negated), dKt; dA, dR Vn^T
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { zero4(dQ[i]); zero4(dKr[i]); zero4(dKc[i]); }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) { zero4(da[i]); zero4(dm[i]); }
+
+#pragma unroll 1
+  for (int s = 0; s < kD / kVS; ++s) {
+    const float *sS0 = F(L::kSD + (s & 1) * 2 * L::kS1), *sdS = sS0 + 128 * LDV;
+    __syncthreads();   // the previous slice (s = 0: the scan scratch) is done with
+    {
+      const uint32_t w[4] = {vr.x, vr.y, vr.z, vr.w};
+      float* dst = (tid < 256 ? sV : sdO) + vrow * LDV + vcol;
+      *reinterpret_cast<float4*>(dst) = make_float4(mma::lo_f(w[0]), mma::hi_f(w[0]), mma::lo_f(w[1]), mma::hi_f(w[1]));
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(mma::lo_f(w[2]), mma::hi_f(w[2]), mma::lo_f(w[3]), mma::hi_f(w[3]));
+    }
+    tc::cp_async_wait_all();
+    __syncthreads();
+    if (s + 1 < kD / kVS) { issue_slice(s + 1); vr = load_v(s + 1); }
+    // ---- R = beta V - beta (K^ e^G) S0,  dVn = A^T dO + Kd dS1 (eight columns per warp) ------------------------------------------
+    const int n0 = 8 * wc;
+    {
+      float r0[4], r1[4], d0[4], d1[4];
+      zero4(r0); zero4(r1); zero4(d0); zero4(d1);
+#pragma unroll 4
+      for (int k0 = 0; k0 < kD; k0 += 16) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int k = k0 + 8 * hf + t;
+          AFrag<X3> a;
+          a.set(sK[(m0 + g) * 132 + k], sK[(m0 + g + 8) * 132 + k], sK[(m0 + g) * 132 + k + 4], sK[(m0 + g + 8) * 132 + k + 4]);
+          BFrag<X3> bs, bd;
+          bs.set(sS0[k * LDV + n0 + g], sS0[(k + 4) * LDV + n0 + g]);
+          bd.set(sdS[k * LDV + n0 + g], sdS[(k + 4) * LDV + n0 + g]);
+          fma<X3>(hf ? r1 : r0, a, bs);
+          if constexpr (KDA) a.set(sKd[(m0 + g) * 132 + k], sKd[(m0 + g + 8) * 132 + k], sKd[(m0 + g) * 132 + k + 4], sKd[(m0 + g + 8) * 132 + k + 4]);
+          fma<X3>(hf ? d1 : d0, a, bd);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { r0[e] += r1[e]; d0[e] += d1[e]; if (!KDA) d0[e] *= sWd[m0 + g + 8 * (e >> 1)]; }
+      for (int k0 = m0; k0 < kC; k0 += 8) {
+        const int k = k0 + t;
+        AFrag<X3> a;
+        a.set(sA[k * LDA + m0 + g], sA[k * LDA + m0 + g + 8], sA[(k + 4) * LDA + m0 + g], sA[(k + 4) * LDA + m0 + g + 8]);
+        BFrag<X3> bo;
+        bo.set(sdO[k * LDV + n0 + g], sdO[(k + 4) * LDV + n0 + g]);
+        fma<X3>(d0, a, bo);
+      }
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int c = m0 + g + 8 * hr, vv = n0 + 2 * t;
+        const float2 x = ld2(sV + c * LDV + vv);
+        const float bt = sBeta[c], eg = KDA ? 1.f : sEG[c];
+        *reinterpret_cast<float2*>(sVn + c * LDV + vv) = make_float2(bt * (x.x - eg * r0[2 * hr]), bt * (x.y - eg * r0[2 * hr + 1]));
+        *reinterpret_cast<float2*>(sdR + c * LDV + vv) = make_float2(d0[2 * hr], d0[2 * hr + 1]);
+      }
+    }
+    __syncthreads();
+    // ---- Vn = T R, dR = T^T dVn ------------------------------------------------------------------------------------------------------
+    {
+      float vn[4], dr[4];
+      zero4(vn); zero4(dr);
+      for (int k0 = 0; k0 < m0 + 16; k0 += 8) {
+        const int k = k0 + t;
+        AFrag<X3> a;
+        a.set(sT[(m0 + g) * LDT + k], sT[(m0 + g + 8) * LDT + k], sT[(m0 + g) * LDT + k + 4], sT[(m0 + g + 8) * LDT + k + 4]);
+        BFrag<X3> br;
+        br.set(sVn[k * LDV + n0 + g], sVn[(k + 4) * LDV + n0 + g]);
+        fma<X3>(vn, a, br);
+      }
+      for (int k0 = m0; k0 < kC; k0 += 8) {
+        const int k = k0 + t;
+        AFrag<X3> a;
+        a.set(sT[k * LDT + m0 + g], sT[k * LDT + m0 + g + 8], sT[(k + 4) * LDT + m0 + g], sT[(k + 4) * LDT + m0 + g + 8]);
+        BFrag<X3> bd;
+        bd.set(sdR[k * LDV + n0 + g], sdR[(k + 4) * LDV + n0 + g]);
+        fma<X3>(dr, a, bd);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int at = (m0 + g + 8 * hr) * LDV + n0 + 2 * t;
+        *reinterpret_cast<float2*>(sVn + at) = make_float2(vn[2 * hr], vn[2 * hr + 1]);
+        *reinterpret_cast<float2*>(sdR + at) = make_float2(dr[2 * hr], dr[2 * hr + 1]);
+      }
+    }
+    __syncthreads();
+    // ---- dV = beta dR, dbeta += dR . V (half of the threads); <dS1, S0> per channel (the other half) -----------------------------------
+    if (tid < 256) {
+      float x[8], acc = 0.f;
+      const float bt = sBeta[vrow];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        x[e] = sdR[vrow * LDV + vcol + e];
+        acc += x[e] * sV[vrow * LDV + vcol + e];
+        x[e] *= bt;
+      }
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      if ((tid & 3) == 0) sdB[vrow] += acc;
+      if (vrow < rows)
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dv) + v_base + (int64_t)(t0 + vrow) * v_tok + s * kVS + vcol) =
+            make_uint4(mma::pack(x[0], x[1]), mma::pack(x[2], x[3]), mma::pack(x[4], x[5]), mma::pack(x[6], x[7]));
+    } else {
+      const int u = tid - 256;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {   // eight lanes per channel row
+        const int k = 32 * it + (u >> 3), c4 = (u & 7) * 4;
+        const float4 x = *reinterpret_cast<const float4*>(sS0 + k * LDV + c4), y = *reinterpret_cast<const float4*>(sdS + k * LDV + c4);
+        float acc = x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+        if ((u & 7) == 0) sTS[k] += acc;
+      }
+    }
+    // ---- sums over v: dA += dO Vn^T, dM' += dR Vn^T; dQg += dO S0^T, dKg' += dR S0^T, dKt += Vn dS1^T (k taken in pairs) -----------------
+#pragma unroll
+    for (int k0 = 0; k0 < kVS; k0 += 8) {
+      const int k = k0 + 2 * t;
+      AFrag<X3> ao, ar, an;
+      {
+        const float2 x0 = ld2(sdO + (m0 + g) * LDV + k), x1 = ld2(sdO + (m0 + g + 8) * LDV + k);
+        ao.set(x0.x, x1.x, x0.y, x1.y);
+        const float2 y0 = ld2(sdR + (m0 + g) * LDV + k), y1 = ld2(sdR + (m0 + g + 8) * LDV + k);
+        ar.set(y0.x, y1.x, y0.y, y1.y);
+        const float2 z0 = ld2(sVn + (m0 + g) * LDV + k), z1 = ld2(sVn + (m0 + g + 8) * LDV + k);
+        an.set(z0.x, z1.x, z0.y, z1.y);
+      }
+      if (16 * wc <= m0) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const float2 y = ld2(sVn + (16 * wc + 8 * nt + g) * LDV + k);
+          BFrag<X3> bv;
+          bv.set(y.x, y.y);
+          fma<X3>(da[nt], ao, bv);
+          fma<X3>(dm[nt], ar, bv);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const int ch = 32 * wc + 8 * nt + g;
+        const float2 y = ld2(sS0 + ch * LDV + k), z = ld2(sdS + ch * LDV + k);
+        BFrag<X3> bs, bd;
+        bs.set(y.x, y.y);
+        bd.set(z.x, z.y);
+        fma<X3>(dQ[nt], ao, bs);
+        fma<X3>(dKr[nt], ar, bs);
+        fma<X3>(dKc[nt], an, bd);
+      }
+    }
+  }
+  // ---- dA, dX with their decay factors; dbeta += dM . X -------------------------------------------------------------------------------------
+  uint2 qr[4], kr[4];
+  float4 gr[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {   // the chunk's q (KDA: and k, g) rows once more, in flight behind the next lines
+    const int c = warp + 16 * i;
+    qr[i] = kr[i] = make_uint2(0u, 0u);
+    gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < rows) {
+      qr[i] = *reinterpret_cast<const uint2*>(gq + qk_base + (t0 + c) * qk_tok + 4 * lane);
+      if constexpr (KDA) {
+        kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
+        gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
+      }
+    }
+  }
+  __syncthreads();   // phase 1 is over: its arrays may be written
+  float* fA = KDA ? F(L::gA) : sA;
+  float* fX = KDA ? F(L::gX) : F(L::fX);
+  {
+    float dbacc[2] = {0.f, 0.f};
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int i = m0 + g + 8 * hr, j = 16 * wc + 8 * nt + 2 * t;
+        float2 xx = make_float2(0.f, 0.f);
+        if (16 * wc <= m0) xx = *reinterpret_cast<const float2*>(xat + i * 64 + j);   // zero at and above the diagonal
+        float av[2], xv[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float ee = (j + e <= i) ? (KDA ? 1.f : __expf(fminf(sGs[i] - sGs[j + e], 0.f))) : 0.f;
+          const float dmv = -dm[nt][2 * hr + e];
+          dbacc[hr] += dmv * (e ? xx.y : xx.x);   // X carries its decay factor
+          av[e] = da[nt][2 * hr + e] * ee;
+          xv[e] = (j + e < i) ? sBeta[i] * dmv * ee : 0.f;
+        }
+        *reinterpret_cast<float2*>(fA + i * LDA + j) = make_float2(av[0], av[1]);
+        *reinterpret_cast<float2*>(fX + i * LDA + j) = make_float2(xv[0], xv[1]);
+      }
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+      float x = dbacc[hr];
+      x += __shfl_xor_sync(0xffffffffu, x, 1);
+      x += __shfl_xor_sync(0xffffffffu, x, 2);
+      if (t == 0) atomicAdd(&sdB[m0 + g + 8 * hr], x);
+    }
+  }
+  // ---- q^ rows (KDA: the decayed forms of q^ and k^) ---------------------------------------------------------------------------------------
+  float* sQ = F(L::fQ);   // DeltaNet / Gated: [64][136]
+  float *sQS = F(L::gQS), *sKS = F(L::gKS), *sKE = F(L::gKE), *sG = F(L::gG), *sD = F(L::gD);
+  if constexpr (KDA) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
+    __syncthreads();
+    scan_channels<kLoThreads>(sG, F(L::gSeg), tid);
+    if (tid < 4) sUn[tid] = 0.f;
+    __syncthreads();
+    {   // total decay of each 16-row block; flag blocks whose range is too wide for the product form
+      const int blk = tid >> 7, c = tid & 127;
+      const float d = sG[(16 * blk + 15) * 132 + c] - (blk ? sG[(16 * blk - 1) * 132 + c] : 0.f);
+      sD[blk * 128 + c] = ex2(d);
+      if (!(d >= -64.f)) sUn[blk] = 1.f;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = warp + 16 * i;
+    const float q0 = mma::lo_f(qr[i].x), q1 = mma::hi_f(qr[i].x), q2 = mma::lo_f(qr[i].y), q3 = mma::hi_f(qr[i].y);
+    const float nrm = p.l2norm ? sqrtf(warp_sum(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3)) : 0.f;
+    const float m = p.l2norm ? p.scale / (nrm + 1e-6f) : p.scale;
+    if (lane == 0) sRq[c] = m;
+    if constexpr (KDA) {
+      const int blk = c >> 4;
+      const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
+      const float4 ge = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
+      float4 gn = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (blk) gn = *reinterpret_cast<const float4*>(sG + (16 * blk - 1) * 132 + 4 * lane);
+      const float mk = sRk[c];
+      const float k0 = mma::lo_f(kr[i].x) * mk, k1 = mma::hi_f(kr[i].x) * mk, k2 = mma::lo_f(kr[i].y) * mk, k3 = mma::hi_f(kr[i].y) * mk;
+      const float e0 = ex2(gg.x - gn.x), e1 = ex2(gg.y - gn.y), e2 = ex2(gg.z - gn.z), e3 = ex2(gg.w - gn.w);
+      *reinterpret_cast<float4*>(sQS + c * 132 + 4 * lane) = make_float4(q0 * m * e0, q1 * m * e1, q2 * m * e2, q3 * m * e3);
+      *reinterpret_cast<float4*>(sKS + c * 132 + 4 * lane) = make_float4(k0 * e0, k1 * e1, k2 * e2, k3 * e3);
+      *reinterpret_cast<float4*>(sKE + c * 132 + 4 * lane) =
+          make_float4(k0 * ex2(ge.x - gg.x), k1 * ex2(ge.y - gg.y), k2 * ex2(ge.z - gg.z), k3 * ex2(ge.w - gg.w));
+    } else {
+      *reinterpret_cast<float4*>(sQ + c * 136 + 4 * lane) = make_float4(q0 * m, q1 * m, q2 * m, q3 * m);
+    }
+  }
+  __syncthreads();
+  // ---- dQ^ = dQg e^G + (dA.E) K^ ; dK^ rows and columns (four channel tiles per warp: 32 wc ..) -------------------------------------------------
+  float dbrow[2] = {0.f, 0.f}, extra = 0.f;
+  float Dg[KDA ? 4 : 1][4];   // KDA: dG of this lane's entries
+  if constexpr (KDA) {
+    const int bi = warp >> 2;
+    const bool exact = sUn[bi] != 0.f;
+    // dbeta: -dKg . k^ e^G; dG_L: dKt . k^ e^{G_L - G}
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = 32 * wc + 8 * nt + 2 * t;
+      float2 en = make_float2(1.f, 1.f);   // decay before the block, and from its end to the chunk's
+      if (bi) { const float2 x = ld2(sG + (16 * bi - 1) * 132 + c); en = make_float2(ex2(x.x), ex2(x.y)); }
+      const float2 gl = ld2(sG + 63 * 132 + c), ge = ld2(sG + (16 * bi + 15) * 132 + c);
+      const float2 ee = make_float2(ex2(gl.x - ge.x), ex2(gl.y - ge.y));
+      float ex0 = 0.f, ex1 = 0.f;
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int i = m0 + g + 8 * hr;
+        const float2 ks = ld2(sKS + i * 132 + c), ke = ld2(sKE + i * 132 + c);
+        dbrow[hr] -= dKr[nt][2 * hr] * ks.x * en.x + dKr[nt][2 * hr + 1] * ks.y * en.y;
+        ex0 += dKc[nt][2 * hr] * ke.x * ee.x;
+        ex1 += dKc[nt][2 * hr + 1] * ke.y * ee.y;
+        dKr[nt][2 * hr] *= -sBeta[i];
+        dKr[nt][2 * hr + 1] *= -sBeta[i];
+      }
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        ex0 += __shfl_xor_sync(0xffffffffu, ex0, o);
+        ex1 += __shfl_xor_sync(0xffffffffu, ex1, o);
+      }
+      if (g == 0) { atomicAdd(&sEx[c], ex0); atomicAdd(&sEx[c + 1], ex1); }
+    }
+    auto carry = [&](float (&d)[4][4], int blk) {   // refer the sums to the end of block blk
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const float2 x = ld2(sD + blk * 128 + 32 * wc + 8 * nt + 2 * t);
+        d[nt][0] *= x.x; d[nt][1] *= x.y; d[nt][2] *= x.x; d[nt][3] *= x.y;
+      }
+    };
+    // rows: sums over the columns of earlier blocks, each block's decay carried on the way; then the diagonal block
+#pragma unroll 1
+    for (int bj = 0; bj <= bi; ++bj) {
+      const bool diag = bj == bi;
+      if (diag && exact) break;
+      if (!diag) { carry(dQ, bj); carry(dKr, bj); }
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int k = 16 * bj + 8 * hf + 2 * t;
+        AFrag<true> aa, ax;
+        const float2 x0 = ld2(fA + (m0 + g) * LDA + k), x1 = ld2(fA + (m0 + g + 8) * LDA + k);
+        aa.set(x0.x, x1.x, x0.y, x1.y);
+        const float2 y0 = ld2(fX + (m0 + g) * LDA + k), y1 = ld2(fX + (m0 + g + 8) * LDA + k);
+        ax.set(y0.x, y1.x, y0.y, y1.y);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const int c = 32 * wc + 8 * nt + g;
+          float b0 = sKE[k * 132 + c], b1 = sKE[(k + 1) * 132 + c];
+          if (diag) { const float iv = 1.f / sD[bi * 128 + c]; b0 *= iv; b1 *= iv; }
+          BFrag<true> bk;
+          bk.set(b0, b1);
+          fma<true>(dQ[nt], aa, bk);
+          fma<true>(dKr[nt], ax, bk);
+        }
+      }
+    }
+    // columns: the rows of later blocks, last first; then the diagonal block, referred to the block's start
+#pragma unroll 1
+    for (int bj = 3; bj >= bi; --bj) {
+      const bool diag = bj == bi;
+      if (diag && exact) break;
+      carry(dKc, bj);
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int k = 16 * bj + 8 * hf + t;
+        AFrag<true> aa, ax;
+        aa.set(fA[k * LDA + m0 + g], fA[k * LDA + m0 + g + 8], fA[(k + 4) * LDA + m0 + g], fA[(k + 4) * LDA + m0 + g + 8]);
+        ax.set(fX[k * LDA + m0 + g], fX[k * LDA + m0 + g + 8], fX[(k + 4) * LDA + m0 + g], fX[(k + 4) * LDA + m0 + g + 8]);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const int c = 32 * wc + 8 * nt + g;
+          BFrag<true> bq, bk;
+          bq.set(sQS[k * 132 + c], sQS[(k + 4) * 132 + c]);
+          bk.set(sKS[k * 132 + c], sKS[(k + 4) * 132 + c]);
+          fma<true>(dKc[nt], aa, bq);
+          fma<true>(dKc[nt], ax, bk);
+        }
+      }
+    }
+    // the factors of the entries' own rows; dG
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = 32 * wc + 8 * nt + 2 * t;
+      float2 gn = make_float2(0.f, 0.f);
+      if (bi) gn = ld2(sG + (16 * bi - 1) * 132 + c);
+      const float2 ge = ld2(sG + (16 * bi + 15) * 132 + c);
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int i = m0 + g + 8 * hr;
+        const float2 gi = ld2(sG + i * 132 + c);
+        float2 qh = make_float2(0.f, 0.f), kh = qh;
+        if (i < rows) {
+          const int64_t at = qk_base + (t0 + i) * qk_tok + c;
+          const uint32_t uq = *reinterpret_cast<const uint32_t*>(gq + at), uk = *reinterpret_cast<const uint32_t*>(gk + at);
+          qh = make_float2(mma::lo_f(uq) * sRq[i], mma::hi_f(uq) * sRq[i]);
+          kh = make_float2(mma::lo_f(uk) * sRk[i], mma::hi_f(uk) * sRk[i]);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int x = 2 * hr + e;
+          const float Gi = e ? gi.y : gi.x, Gn = e ? gn.y : gn.x, Ge = e ? ge.y : ge.x;
+          const float fr = ex2(Gi - Gn), fc = ex2((exact ? Ge : Gn) - Gi);
+          float dq = dQ[nt][x] * fr, dkr = dKr[nt][x] * fr, dkc = dKc[nt][x] * fc;
+          if (exact) {   // the diagonal block entry by entry
+            for (int j = m0; j < m0 + 16; ++j) {
+              const float Gj = sG[j * 132 + c + e];
+              if (j >= rows) break;
+              const int64_t at = qk_base + (t0 + j) * qk_tok + c + e;
+              const float kj = bf(gk + at) * sRk[j], qj = bf(gq + at) * sRq[j];
+              if (j <= i) {
+                const float w = ex2(Gi - Gj) * kj;
+                dq += fA[i * LDA + j] * w;
+                dkr += fX[i * LDA + j] * w;
+              }
+              if (j >= i) {
+                const float w = ex2(Gj - Gi);
+                dkc += w * (fA[j * LDA + i] * qj + fX[j * LDA + i] * kj);
+              }
+            }
+          }
+          Dg[nt][x] = (e ? qh.y : qh.x) * dq + (e ? kh.y : kh.x) * (dkr - dkc);
+          dQ[nt][x] = dq;
+          dKr[nt][x] = dkr + dkc;
+        }
+        float sq = qh.x * dQ[nt][2 * hr] + qh.y * dQ[nt][2 * hr + 1], sk = kh.x * dKr[nt][2 * hr] + kh.y * dKr[nt][2 * hr + 1];
+        sq += __shfl_xor_sync(0xffffffffu, sq, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+        sk += __shfl_xor_sync(0xffffffffu, sk, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+        if (t == 0) { atomicAdd(&sDq[i], sq); atomicAdd(&sDk[i], sk); }
+      }
+    }
+  } else {
+    const float eg[2] = {sEG[m0 + g], sEG[m0 + g + 8]}, el[2] = {sWd[m0 + g], sWd[m0 + g + 8]}, bt[2] = {sBeta[m0 + g], sBeta[m0 + g + 8]};
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const float2 kh = ld2(sK + (m0 + g + 8 * hr) * 132 + 32 * wc + 8 * nt + 2 * t);
+        const int e = 2 * hr;
+        dbrow[hr] -= (dKr[nt][e] * kh.x + dKr[nt][e + 1] * kh.y) * eg[hr];
+        extra += (dKc[nt][e] * kh.x + dKc[nt][e + 1] * kh.y) * el[hr];
+        dQ[nt][e] *= eg[hr]; dQ[nt][e + 1] *= eg[hr];
+        dKr[nt][e] *= -bt[hr] * eg[hr]; dKr[nt][e + 1] *= -bt[hr] * eg[hr];
+        dKc[nt][e] *= el[hr]; dKc[nt][e + 1] *= el[hr];
+      }
+    for (int k0 = 0; k0 < m0 + 16; k0 += 8) {
+      const int k = k0 + 2 * t;
+      AFrag<X3> aa, ax;
+      const float2 x0 = ld2(fA + (m0 + g) * LDA + k), x1 = ld2(fA + (m0 + g + 8) * LDA + k);
+      aa.set(x0.x, x1.x, x0.y, x1.y);
+      const float2 y0 = ld2(fX + (m0 + g) * LDA + k), y1 = ld2(fX + (m0 + g + 8) * LDA + k);
+      ax.set(y0.x, y1.x, y0.y, y1.y);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const int c = 32 * wc + 8 * nt + g;
+        BFrag<X3> bk;
+        bk.set(sK[k * 132 + c], sK[(k + 1) * 132 + c]);
+        fma<X3>(dQ[nt], aa, bk);
+        fma<X3>(dKr[nt], ax, bk);
+      }
+    }
+    for (int k0 = m0; k0 < kC; k0 += 8) {
+      const int k = k0 + t;
+      AFrag<X3> aa, ax;
+      aa.set(fA[k * LDA + m0 + g], fA[k * LDA + m0 + g + 8], fA[(k + 4) * LDA + m0 + g], fA[(k + 4) * LDA + m0 + g + 8]);
+      ax.set(fX[k * LDA + m0 + g], fX[k * LDA + m0 + g + 8], fX[(k + 4) * LDA + m0 + g], fX[(k + 4) * LDA + m0 + g + 8]);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const int c = 32 * wc + 8 * nt + g;
+        BFrag<X3> bq, bk;
+        bq.set(sQ[k * 136 + c], sQ[(k + 4) * 136 + c]);
+        bk.set(sK[k * 132 + c], sK[(k + 4) * 132 + c]);
+        fma<X3>(dKc[nt], aa, bq);
+        fma<X3>(dKc[nt], ax, bk);
+      }
+    }
+    float dgrow[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int i = m0 + g + 8 * hr, c = 32 * wc + 8 * nt + 2 * t, e = 2 * hr;
+        const float2 qh = ld2(sQ + i * 136 + c), kh = ld2(sK + i * 132 + c);
+        const float a = qh.x * dQ[nt][e] + qh.y * dQ[nt][e + 1];
+        const float kr_ = kh.x * dKr[nt][e] + kh.y * dKr[nt][e + 1], kc_ = kh.x * dKc[nt][e] + kh.y * dKc[nt][e + 1];
+        sq[hr] += a; sk[hr] += kr_ + kc_;
+        dgrow[hr] += a + kr_ - kc_;
+        dKr[nt][e] += dKc[nt][e]; dKr[nt][e + 1] += dKc[nt][e + 1];
+      }
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+      const int i = m0 + g + 8 * hr;
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        dgrow[hr] += __shfl_xor_sync(0xffffffffu, dgrow[hr], o);
+        sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
+        sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
+      }
+      if (t == 0) { atomicAdd(&sdG[i], dgrow[hr]); atomicAdd(&sDq[i], sq[hr]); atomicAdd(&sDk[i], sk[hr]); }
+    }
+    extra = warp_sum(extra);
+    if (lane == 0) atomicAdd(&sdG[63], extra);
+  }
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+    float db = dbrow[hr];
+    db += __shfl_xor_sync(0xffffffffu, db, 1); db += __shfl_xor_sync(0xffffffffu, db, 2);
+    if (t == 0) atomicAdd(&sdB[m0 + g + 8 * hr], db);
+  }
+  __syncthreads();
+  // ---- chain rule of the normalisation: y = s x / (|x| + eps), y^ = s x r:  dx = s r dy - y^ (y^ . dy) / (s |x|) ------------------------------------
+  const bool grouped = p.map.Hq != p.map.H;
+  __nv_bfloat16* oq = reinterpret_cast<__nv_bfloat16*>(KDA ? smem + L::gKS : smem + L::fX);   // staging [64][136] bf16, twice
+  __nv_bfloat16* ok = oq + 64 * 136;
+  float* sDG = F(L::gQS);   // KDA: dG [64][132]
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+    const int i = m0 + g + 8 * hr;
+    const float mq = sRq[i], mk = sRk[i];
+    float fq = 0.f, fk = 0.f;
+    if (p.l2norm) {
+      const float nq = p.scale / mq - 1e-6f, nk = 1.f / mk - 1e-6f;   // |q|, |k|
+      fq = nq > 0.f ? sDq[i] / (p.scale * nq) : 0.f;
+      fk = nk > 0.f ? sDk[i] / nk : 0.f;
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = 32 * wc + 8 * nt + 2 * t, e = 2 * hr;
+      if (grouped) {
+        const int64_t at = (chunk * kC + i) * kD + c;
+        *reinterpret_cast<float2*>(p.part + at) = make_float2(dQ[nt][e], dQ[nt][e + 1]);
+        *reinterpret_cast<float2*>(p.part + (int64_t)gridDim.x * (kC * kD) + at) = make_float2(dKr[nt][e], dKr[nt][e + 1]);
+      } else {
+        float2 qh = make_float2(0.f, 0.f), kh = qh;
+        if constexpr (KDA) {
+          if (i < rows) {
+            const int64_t at = qk_base + (t0 + i) * qk_tok + c;
+            const uint32_t uq = *reinterpret_cast<const uint32_t*>(gq + at), uk = *reinterpret_cast<const uint32_t*>(gk + at);
+            qh = make_float2(mma::lo_f(uq) * mq, mma::hi_f(uq) * mq);
+            kh = make_float2(mma::lo_f(uk) * mk, mma::hi_f(uk) * mk);
+          }
+        } else {
+          qh = ld2(sQ + i * 136 + c); kh = ld2(sK + i * 132 + c);
+        }
+        *reinterpret_cast<uint32_t*>(oq + i * 136 + c) = mma::pack(mq * dQ[nt][e] - qh.x * fq, mq * dQ[nt][e + 1] - qh.y * fq);
+        *reinterpret_cast<uint32_t*>(ok + i * 136 + c) = mma::pack(mk * dKr[nt][e] - kh.x * fk, mk * dKr[nt][e + 1] - kh.y * fk);
+      }
+      if constexpr (KDA) *reinterpret_cast<float2*>(sDG + i * 132 + c) = make_float2(Dg[nt][e], Dg[nt][e + 1]);
+    }
+  }
+  __syncthreads();
+  if (!grouped) {
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int i = tid + kLoThreads * it, which = i >> 10, r = (i >> 4) & 63, c8 = (i & 15) * 8;
+      if (r < rows)
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(which ? p.dk : p.dq) + qk_base + (t0 + r) * qk_tok + c8) =
+            *reinterpret_cast<const uint4*>((which ? ok : oq) + r * 136 + c8);
+    }
+  }
+  if (tid < rows) p.dbeta[s_base + (t0 + tid) * s_tok] = sdB[tid];
+  // ---- dg: reverse cumulative sum of dG inside the chunk ---------------------------------------------------------------------------------------
+  if constexpr (KDA) {
+    const int s = tid >> 7, c = tid & 127;   // 16-row segment, channel
+    float acc = 0.f, loc[16];
+    if (s == 3) acc = sEx[c] + sTS[c] * ex2(sG[63 * 132 + c]);
+#pragma unroll
+    for (int r = 15; r >= 0; --r) {
+      acc += sDG[(16 * s + r) * 132 + c];
+      loc[r] = acc;
+    }
+    sD[s * 128 + c] = acc;
+    __syncthreads();
+    float post = 0.f;
+    for (int s2 = s + 1; s2 < 4; ++s2) post += sD[s2 * 128 + c];
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (16 * s + r < rows) p.dg[gk_base + (int64_t)(t0 + 16 * s + r) * gk_tok + c] = loc[r] + post;
+  } else if (p.variant == DR_GATED && warp == 0) {
+    float ts = sTS[lane] + sTS[lane + 32] + sTS[lane + 64] + sTS[lane + 96];
+    ts = warp_sum(ts) * expf(sGs[63]);
+    float lo = sdG[lane], hi = sdG[lane + 32] + (lane == 31 ? ts : 0.f);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float a = __shfl_down_sync(0xffffffffu, lo, o), c = __shfl_down_sync(0xffffffffu, hi, o);
+      if (lane + o < 32) { lo += a; hi += c; }
+    }
+    lo += __shfl_sync(0xffffffffu, hi, 0);
+    if (lane < rows) p.dg[s_base + (t0 + lane) * s_tok] = lo;
+    if (lane + 32 < rows) p.dg[s_base + (t0 + lane + 32) * s_tok] = hi;
+  }
+}
+
+// =====================================================================================================================
+// host side
+// =====================================================================================================================
+inline bool eligible(const DrDesc* d) {
+  return d->K == kD && d->V == kD && d->chunk == kC && d->qkv_dtype == DR_BF16;
+}
+// floats per chunk: checkpoint, N (later the grouped heads' dq^, dk^), Y, X A T, dS1 (first the records of the two-kernel
+// forward: 66048 bytes), e^{G_L}
+constexpr int64_t kCkpt = 16384, kNf = 16384, kYf = 8192, kXat = 3 * 4096, kDs = 16512, kEl = 128;
+constexpr int64_t kFloats = kCkpt + kNf + kYf + kXat + kDs + kEl;
+inline int64_t workspace_bytes(const DrDesc* d) {
+  const int64_t N = (d->T + kC - 1) / kC;
+  return (int64_t)d->B * d->H * N * kFloats * 4;
+}
+inline Params make_params(const DrDesc* d, void* workspace) {
+  Params p{};
+  p.N = (d->T + kC - 1) / kC;
+  const int64_t nc = (int64_t)d->B * d->H * p.N;
+  float* f = reinterpret_cast<float*>(workspace);
+  p.ckpt = f; f += nc * kCkpt;
+  p.nf = reinterpret_cast<float4*>(f); p.part = f; f += nc * kNf;
+  p.yf = reinterpret_cast<float4*>(f); f += nc * kYf;
+  p.xat = f; f += nc * kXat;
+  p.ds = f; f += nc * kDs;
+  p.el = f;
+  p.map.B = d->B; p.map.H = d->H; p.map.T = d->T; p.map.bthd = d->layout == DR_LAYOUT_BTHD;
+  p.map.Hq = d->qk_heads > 0 ? d->qk_heads : d->H;
+  p.variant = d->variant; p.g_dt = d->g_dtype; p.l2norm = d->use_qk_l2norm; p.scale = d->scale;
+  return p;
+}
+template <bool KDA>
+inline cudaError_t set_attributes() {
+  thread_local int attr_dev = -1;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || attr_dev == dev) return e;
+  e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem<KDA>::kTotal);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(state_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem);
+  if (e == cudaSuccess) attr_dev = dev;
+  return e;
+}
+template <bool KDA>
+inline cudaError_t launch_pre_t(const Params& p, int64_t units, cudaStream_t stream) {
+  const cudaError_t e = set_attributes<KDA>();
+  if (e != cudaSuccess) return e;
+  pre_kernel<KDA><<<(unsigned)(units * p.N), kPreThreads, pre_smem<KDA>(), stream>>>(p);
+  return cudaGetLastError();
+}
+inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, const void* g, const float* beta, void* workspace,
+                              cudaStream_t stream, int* launches) {
+  Params p = make_params(d, workspace);
+  p.q = q; p.k = k; p.g = g; p.beta = beta;
+  ++*launches;
+  const int64_t units = (int64_t)d->B * d->H;
+  return d->variant == DR_KDA ? launch_pre_t<true>(p, units, stream) : launch_pre_t<false>(p, units, stream);
+}
+template <bool KDA>
+inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, cudaStream_t stream) {
+  cudaError_t e = set_attributes<KDA>();
+  if (e != cudaSuccess) return e;
+  state_kernel<KDA><<<(unsigned)(units * 4), kStThreads, kStSmem, stream>>>(p);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  local_kernel<KDA><<<(unsigned)(units * p.N), kLoThreads, LoSmem<KDA>::kTotal, stream>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace bwdc
+}  // namespace dr
