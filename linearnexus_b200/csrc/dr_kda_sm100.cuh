@@ -46,7 +46,10 @@ constexpr int WS_AQK = WS_TB + 8192;       // A_qk         [64][64] bf16
 constexpr int WS_EGL = WS_AQK + 8192;      // e^{G_L}[128] fp32
 constexpr int WS_REC = WS_EGL + 512;       // 66048
 
-inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC - 1) / kC) * (int64_t)WS_REC; }
+// What callers are asked for per record: the size the ABI has announced from the start (records once carried V, too).
+constexpr int WS_ASKED = 82432;
+static_assert(WS_REC <= WS_ASKED, "records fit what callers provide");
+inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC - 1) / kC) * (int64_t)WS_ASKED; }
 
 // ---- intra-chunk kernel ------------------------------------------------------------------------------------
 // Shared memory is kept under half an SM's worth so that two CTAs are resident and one chunk's latency
