@@ -124,6 +124,8 @@ const char* dr_last_path(void);
  * For op=0 the figure is what the path desc->path resolves to would use; a forward that is
  * given less returns DR_ERR_WORKSPACE (there is no silent downgrade to a slower kernel: ask for
  * DR_PATH_FP32 to run without scratch).
+ * op=2: scratch with which dr_chunk_fwd is at its fastest -- at least the op=0 figure; shapes that AUTO runs on the token
+ * recurrence without scratch (float32 storage with K = V = 64 or 128, more than one chunk) run chunk-parallel with it.
  * op=1 returns DR_ERR_UNSUPPORTED for shapes the backward does not cover: chunk > 64, K > 128,
  * or DR_KDA with K % 16 != 0 (the forward entry points accept those shapes). */
 int64_t dr_workspace_bytes(const DrDesc* desc, int op);

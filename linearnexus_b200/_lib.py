@@ -19,7 +19,7 @@ _ROOT = _PKG.parent
 LIB_PATH = Path(os.environ.get("DELTARULE_SM100_LIB", _PKG / "libdeltarule_sm100.so"))
 # the same sources with the index checks compiled in (-DDR_BOUNDS_CHECK); tests load it through DELTARULE_SM100_LIB
 BOUNDS_LIB_PATH = _PKG / "libdeltarule_sm100_bounds.so"
-_SOURCES = ["dr_api.cu", "dr_fwd.cu", "dr_bwd.cu", "dr_scans.cu"]   # translation units, compiled side by side
+_SOURCES = ["dr_api.cu", "dr_fwd.cu", "dr_trans.cu", "dr_bwd.cu", "dr_scans.cu"]   # translation units, compiled side by side
 # the native host path of the public calls (argument checks, allocation, C-ABI call): a CPython extension over torch
 HOST_PATH = _PKG / "_host_calls.so"
 _HOST_SOURCE = _PKG / "csrc" / "host_calls.cpp"

@@ -120,6 +120,14 @@ int resolve_chunk_path(const DrDesc* d) {
   return kPathRecurrence;
 }
 
+// AUTO without a tensor-core kernel: with scratch, whole chunks run in parallel (transition form); from two chunks on (one
+// chunk has no parallelism over the recurrence's), and up to 1 GB of scratch.
+int64_t trans_scratch(const DrDesc* d) {
+  if (resolve_chunk_path(d) != kPathRecurrence || d->K != d->V || (d->K != 64 && d->K != 128) || d->T <= 64) return 0;
+  const int64_t need = dr::trans_workspace_bytes((int64_t)d->B * d->H, d->T, d->K);
+  return need <= (int64_t)1 << 30 ? need : 0;
+}
+
 bool fp32_chunk_eligible(const DrDesc* d) { return d->chunk <= 64 && d->K <= 128; }
 
 // A [B,H,T,D] / [B,T,H,D] activation as the strided per-token vector the scans of dr_linrec.cuh read.
@@ -181,6 +189,10 @@ int64_t dr_workspace_bytes(const DrDesc* d, int op) {
     return (resolve_chunk_path(d) == DR_PATH_SPLIT && split_eligible(d))
                ? dr::split_workspace_bytes((int64_t)d->B * d->H, d->T) : 0;
   if (op == 1) return dr::bwd_workspace_bytes(d);
+  if (op == 2) {
+    const int64_t need = dr_workspace_bytes(d, 0);
+    return need != 0 ? need : trans_scratch(d);
+  }
   return DR_ERR_UNSUPPORTED;
 }
 
@@ -217,6 +229,12 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
     tl_path = "chunk_fp32";
     g_launches.fetch_add(1);
     return check_cuda(dr::launch_chunk_fp32(p, st));
+  }
+  const int64_t scratch = trans_scratch(d);
+  if (scratch > 0 && workspace && aligned16(workspace) && (int64_t)workspace_bytes >= scratch) {
+    tl_path = "chunk_transition";
+    g_launches.fetch_add(2);
+    return check_cuda(dr::launch_chunk_trans(p, workspace, sm_count(), st));
   }
   // AUTO without a tensor-core kernel for the shape, and DR_PATH_FP32 with chunks longer than 64 or K > 128
   tl_path = "recurrent";

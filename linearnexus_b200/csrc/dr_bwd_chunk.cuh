@@ -19,7 +19,7 @@
 // 1.26 ms; with per-channel decay 12 ms on the CUDA cores) and stored four fp32 copies of dq^, dk^.
 //
 // Products are mma.sync tf32 with fp32 operands.  DeltaNet / Gated DeltaNet: one product (operands cut to tf32, as the
-// adjoint they replace).  KDA: three products per pair (x = hi + lo, lo lo dropped), i.e. float32 precision, as the
+// adjoint they replace).  KDA: three products per pair (x = hi + lo; see dr_tf32.cuh), i.e. float32 precision, as the
 // CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
 // referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
 // decay range exceeds 2^64 is summed exactly.
@@ -28,6 +28,7 @@
 #include "dr_common.cuh"
 #include "dr_mma.cuh"
 #include "dr_sm100_common.cuh"
+#include "dr_tf32.cuh"
 
 namespace dr {
 namespace bwdc {
@@ -57,73 +58,14 @@ __device__ __forceinline__ float bf(const __nv_bfloat16* p) { return __bfloat162
 __device__ __forceinline__ float ex2(float x) { return tc::fast_exp2(x); }
 constexpr float kLog2e = 1.4426950408889634f;
 
-// One operand of a tf32 product; X3: its leading 11 bits and the rest.
-template <bool X3>
-struct AFrag {
-  uint32_t h[4], l[X3 ? 4 : 1];
-  __device__ __forceinline__ void set(float a0, float a1, float a2, float a3) {
-    const float a[4] = {a0, a1, a2, a3};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      h[i] = __float_as_uint(a[i]);
-      if constexpr (X3) {
-        h[i] &= 0xffffe000u;
-        l[i] = __float_as_uint(a[i] - __uint_as_float(h[i]));
-      }
-    }
-  }
-};
-template <bool X3>
-struct BFrag {
-  uint32_t h[2], l[X3 ? 2 : 1];
-  __device__ __forceinline__ void set(float b0, float b1) {
-    h[0] = __float_as_uint(b0); h[1] = __float_as_uint(b1);
-    if constexpr (X3) {
-      h[0] &= 0xffffe000u; h[1] &= 0xffffe000u;
-      l[0] = __float_as_uint(b0 - __uint_as_float(h[0]));
-      l[1] = __float_as_uint(b1 - __uint_as_float(h[1]));
-    }
-  }
-};
-template <bool X3>
-__device__ __forceinline__ void fma(float (&d)[4], const AFrag<X3>& a, const BFrag<X3>& b) {
-  if constexpr (X3) {
-    sm100::mma_tf32(d, a.l, b.h);
-    sm100::mma_tf32(d, a.h, b.l);
-  }
-  sm100::mma_tf32(d, a.h, b.h);
-}
+using mma::AFrag;
+using mma::BFrag;
+using mma::fma;
 __device__ __forceinline__ void zero4(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
 // value as the product will see it, rounded to nearest instead of cut (single-product operands that are stored)
 template <bool X3>
 __device__ __forceinline__ float stored(float x) { return X3 ? x : __uint_as_float(sm100::to_tf32(x)); }
 
-// In-place inclusive prefix sum over the 64 rows of sG [64][132] per channel; NTHR threads, `seg` scratch of
-// NTHR / 32 rows x 128 floats.  Ends with a barrier.
-template <int NTHR>
-__device__ __forceinline__ void scan_channels(float* sG, float* seg, int tid) {
-  constexpr int R = 64 / (NTHR / 32);   // rows per segment
-  const int s = tid >> 5, c4 = 4 * (tid & 31);
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), loc[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const float4 x = *reinterpret_cast<const float4*>(sG + (R * s + r) * 132 + c4);
-    acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
-    loc[r] = acc;
-  }
-  *reinterpret_cast<float4*>(seg + s * 128 + c4) = acc;
-  __syncthreads();
-  float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s2 = 0; s2 < s; ++s2) {
-    const float4 x = *reinterpret_cast<const float4*>(seg + s2 * 128 + c4);
-    pre.x += x.x; pre.y += x.y; pre.z += x.z; pre.w += x.w;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-    *reinterpret_cast<float4*>(sG + (R * s + r) * 132 + c4) =
-        make_float4(loc[r].x + pre.x, loc[r].y + pre.y, loc[r].z + pre.z, loc[r].w + pre.w);
-  __syncthreads();
-}
 // four channels of the log decay in log2 units
 __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   float4 x;
@@ -135,16 +77,6 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   }
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
-// inclusive sums of 64 scalars, rows lane and lane + 32
-__device__ __forceinline__ void scan_scalars(float& lo, float& hi, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float a = __shfl_up_sync(0xffffffffu, lo, o), b = __shfl_up_sync(0xffffffffu, hi, o);
-    if (lane >= o) { lo += a; hi += b; }
-  }
-  hi += __shfl_sync(0xffffffffu, lo, 31);
-}
-
 // =====================================================================================================================
 // pre_kernel
 // =====================================================================================================================
@@ -213,13 +145,13 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       if (lane == i) { sBeta[c] = bt; sRk[c] = kmul; sRq[c] = qmul; }
     }
     if (!KDA && warp == 0) {
-      scan_scalars(g_lo, g_hi, lane);
+      mma::scan_scalars(g_lo, g_hi, lane);
       sGs[lane] = g_lo; sGs[lane + 32] = g_hi;
     }
   }
   __syncthreads();
   if constexpr (KDA) {
-    scan_channels<kPreThreads>(sG, sX, tid);
+    mma::scan_channels<kPreThreads, kD>(sG, sX, tid);
     if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * 132 + tid]);
     if (tid < 64) { sFw[tid] = sBeta[tid] * sRk[tid]; }
   } else {
@@ -634,7 +566,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         if (lane < rows) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
         if (lane + 32 < rows) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
       }
-      scan_scalars(lo, hi, lane);
+      mma::scan_scalars(lo, hi, lane);
       const float gl = __shfl_sync(0xffffffffu, hi, 31);
       sGs[lane] = lo; sGs[lane + 32] = hi;
       sEG[lane] = expf(lo); sEG[lane + 32] = expf(hi);
@@ -645,7 +577,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
       __syncthreads();
-      scan_channels<kLoThreads>(sG, sVn, tid);   // scratch 8 KB
+      mma::scan_channels<kLoThreads, kD>(sG, sVn, tid);   // scratch 8 KB
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -873,7 +805,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
     __syncthreads();
-    scan_channels<kLoThreads>(sG, F(L::gSeg), tid);
+    mma::scan_channels<kLoThreads, kD>(sG, F(L::gSeg), tid);
     if (tid < 4) sUn[tid] = 0.f;
     __syncthreads();
     {   // total decay of each 16-row block; flag blocks whose range is too wide for the product form

@@ -1,5 +1,6 @@
 // Launchers of the kernels that are compiled in translation units of their own (dr_fwd.cu: the tensor-core forwards,
-// dr_bwd.cu: the backward), so that the library's units build side by side.
+// dr_trans.cu: the forward
+// in transition form, dr_bwd.cu: the backward), so that the library's units build side by side.
 #pragma once
 
 #include "dr_common.cuh"
@@ -13,6 +14,10 @@ cudaError_t launch_chunk_fused_packed(const FwdParams& p, const SeqTable& seqs, 
 int64_t split_workspace_bytes(int64_t units, int T);
 cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches);
 cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream);
+
+// forward in transition form (two kernels; K = V = 64 or 128, any storage types); the workspace holds trans_workspace_bytes
+int64_t trans_workspace_bytes(int64_t units, int T, int D);
+cudaError_t launch_chunk_trans(const FwdParams& p, void* workspace, int sms, cudaStream_t stream);
 
 // backward (see dr_bwd.cuh)
 int64_t bwd_workspace_bytes(const DrDesc* d);

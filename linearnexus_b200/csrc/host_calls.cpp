@@ -259,7 +259,7 @@ PyObject* py_sequence(PyObject*, PyObject* const* a, Py_ssize_t n) {
       Unlocked u;
       st = api.recurrent_fwd(&d, ptr(q), ptr(k), ptr(v), ptr(g), fptr(&beta), fptr(h0), o.mutable_data_ptr(), fmut(hT), c.status(), stream);
     } else {
-      const int64_t ws_bytes = api.workspace_bytes(&d, 0);
+      const int64_t ws_bytes = api.workspace_bytes(&d, 2);
       if (ws_bytes < 0) return PyLong_FromLong((long)ws_bytes);
       at::Tensor ws;
       if (ws_bytes > 0) ws = c.empty({ws_bytes}, at::kByte);

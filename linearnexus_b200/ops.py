@@ -170,7 +170,7 @@ def _seq_forward(kind, variant, q, k, v, g, beta, initial_state, scale, chunk_si
     lib = _lib.load()
     with torch.cuda.device(dev):
         if kind == "chunk":
-            need = int(lib.dr_workspace_bytes(ctypes.byref(d), 0))
+            need = int(lib.dr_workspace_bytes(ctypes.byref(d), 2))
             ws = torch.empty(need, dtype=torch.uint8, device=dev) if need > 0 else None
             st = lib.dr_chunk_fwd(ctypes.byref(d), _ptr(qn), _ptr(kn), _ptr(vn), _ptr(gn), _ptr(bn),
                                   _ptr(h0), _ptr(o), _ptr(hT), _ptr(ws), max(need, 0), _ptr(_status(dev)),
