@@ -484,12 +484,14 @@ struct LoSmem {
   static constexpr int kV = kT + 64 * LDT * 4, kSl = 64 * LDV * 4;   // V, dO, Vn, dR
   static constexpr int kSD = kV + 4 * kSl, kS1 = 128 * LDV * 4;        // [2][S0, dS]
   static constexpr int kSc = kSD + 4 * kS1;
-  static constexpr int kTotal = kSc + (10 * 64 + 3 * 128) * 4;
+  static constexpr int kTotal = kSc + (3 * 64 + 5 * 64 + 128 + 528) * 4;
   // final phase: DeltaNet / Gated: dX over V .. , q^ over the S0, dS buffers; KDA: its own map from 0
   static constexpr int fX = kV, fQ = kSD;
   static constexpr int gQS = 0, gKS = 64 * 132 * 4, gKE = 2 * gKS, gG = 3 * gKS, gA = 4 * gKS, gX = gA + 64 * LDA * 4, gD = gX + 64 * LDA * 4;
   static constexpr int gSeg = gD + 4 * 128 * 4;   // [16][128] scan scratch
-  static_assert(64 * LDA * 4 <= 4 * kSl && 64 * 136 * 4 <= 4 * kS1 && gSeg + 16 * 128 * 4 <= kSc && kTotal <= 232448, "shared memory");
+  static constexpr int kDot = KDA ? gSeg + 16 * 128 * 4 : kV + 64 * 136 * 4;   // final phase: q^ . dq^, k^ . dk^ per row, [2][4][64]
+  static_assert(64 * LDA * 4 <= 4 * kSl && 64 * 136 * 4 <= 4 * kS1 && kTotal <= 232448 &&
+                (KDA ? kDot + 2048 <= kSc : kDot + 2048 <= kSD && 2 * 64 * 136 * 2 <= 64 * 136 * 4), "shared memory");
 };
 
 template <bool KDA>
@@ -501,9 +503,13 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   float *sK = F(L::kK), *sKd = F(L::kKd), *sA = F(L::kA), *sT = F(L::kT);
   float *sV = F(L::kV), *sdO = F(L::kV + L::kSl), *sVn = F(L::kV + 2 * L::kSl), *sdR = F(L::kV + 3 * L::kSl);
   float* sBeta = F(L::kSc);
-  float *sEG = sBeta + 64, *sWd = sBeta + 128, *sGs = sBeta + 192, *sRk = sBeta + 256, *sRq = sBeta + 320;
-  float *sdB = sBeta + 384, *sdG = sBeta + 448, *sDq = sBeta + 512, *sDk = sBeta + 576;
-  float *sTS = sBeta + 640, *sEx = sBeta + 768, *sUn = sBeta + 896;   // <dS1, S0> per channel; KDA: sums for dG_L, block flags
+  float *sRk = sBeta + 64, *sRq = sBeta + 128;
+  // sums over a row's columns: one slot per quarter of the columns (sdB: and one for dR . V), added up by one thread at the
+  // end -- no atomics, so that equal inputs give equal bits
+  float *sdB = sBeta + 192, *sTS = sBeta + 512, *sU = sBeta + 640;   // dbeta [5][64]; <dS1, S0> per channel
+  float *sEG = sU, *sWd = sU + 64, *sGs = sU + 128, *sdG = sU + 192, *sXt = sU + 448;   // DeltaNet / Gated; dG [4][64], sums for dG_L [16]
+  float *sEx = sU, *sUn = sU + 512;                                                       // KDA: sums for dG_L [4][128], block flags
+  float *sDq = F(L::kDot), *sDk = sDq + 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
@@ -557,9 +563,9 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     }
     if (tid < 64) {
       sBeta[tid] = tid < rows ? p.beta[s_base + (t0 + tid) * s_tok] : 0.f;
-      sdB[tid] = sdG[tid] = sDq[tid] = sDk[tid] = 0.f;
     }
-    if (tid < 128) sTS[tid] = sEx[tid] = 0.f;
+    for (int i = tid; i < 320; i += kLoThreads) sdB[i] = 0.f;
+    if (tid < 128) sTS[tid] = 0.f;
     if (!KDA && warp == 15) {
       float lo = 0.f, hi = 0.f;
       if (p.variant == DR_GATED) {
@@ -697,7 +703,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       }
       acc += __shfl_xor_sync(0xffffffffu, acc, 1);
       acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      if ((tid & 3) == 0) sdB[vrow] += acc;
+      if ((tid & 3) == 0) sdB[256 + vrow] += acc;
       if (vrow < rows)
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dv) + v_base + (int64_t)(t0 + vrow) * v_tok + s * kVS + vcol) =
             make_uint4(mma::pack(x[0], x[1]), mma::pack(x[2], x[3]), mma::pack(x[4], x[5]), mma::pack(x[6], x[7]));
@@ -795,7 +801,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       float x = dbacc[hr];
       x += __shfl_xor_sync(0xffffffffu, x, 1);
       x += __shfl_xor_sync(0xffffffffu, x, 2);
-      if (t == 0) atomicAdd(&sdB[m0 + g + 8 * hr], x);
+      if (t == 0) sdB[64 * wc + m0 + g + 8 * hr] += x;
     }
   }
   // ---- q^ rows (KDA: the decayed forms of q^ and k^) ---------------------------------------------------------------------------------------
@@ -870,7 +876,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         ex0 += __shfl_xor_sync(0xffffffffu, ex0, o);
         ex1 += __shfl_xor_sync(0xffffffffu, ex1, o);
       }
-      if (g == 0) { atomicAdd(&sEx[c], ex0); atomicAdd(&sEx[c + 1], ex1); }
+      if (g == 0) *reinterpret_cast<float2*>(sEx + 128 * bi + c) = make_float2(ex0, ex1);
     }
     auto carry = [&](float (&d)[4][4], int blk) {   // refer the sums to the end of block blk
 #pragma unroll
@@ -929,6 +935,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       }
     }
     // the factors of the entries' own rows; dG
+    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       const int c = 32 * wc + 8 * nt + 2 * t;
@@ -973,11 +980,18 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
           dQ[nt][x] = dq;
           dKr[nt][x] = dkr + dkc;
         }
-        float sq = qh.x * dQ[nt][2 * hr] + qh.y * dQ[nt][2 * hr + 1], sk = kh.x * dKr[nt][2 * hr] + kh.y * dKr[nt][2 * hr + 1];
-        sq += __shfl_xor_sync(0xffffffffu, sq, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-        sk += __shfl_xor_sync(0xffffffffu, sk, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-        if (t == 0) { atomicAdd(&sDq[i], sq); atomicAdd(&sDk[i], sk); }
+        sq[hr] += qh.x * dQ[nt][2 * hr] + qh.y * dQ[nt][2 * hr + 1];
+        sk[hr] += kh.x * dKr[nt][2 * hr] + kh.y * dKr[nt][2 * hr + 1];
       }
+    }
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
+        sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
+      }
+      if (t == 0) { sDq[64 * wc + m0 + g + 8 * hr] = sq[hr]; sDk[64 * wc + m0 + g + 8 * hr] = sk[hr]; }
     }
   } else {
     const float eg[2] = {sEG[m0 + g], sEG[m0 + g + 8]}, el[2] = {sWd[m0 + g], sWd[m0 + g + 8]}, bt[2] = {sBeta[m0 + g], sBeta[m0 + g + 8]};
@@ -1046,16 +1060,16 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
         sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
       }
-      if (t == 0) { atomicAdd(&sdG[i], dgrow[hr]); atomicAdd(&sDq[i], sq[hr]); atomicAdd(&sDk[i], sk[hr]); }
+      if (t == 0) { sdG[64 * wc + i] = dgrow[hr]; sDq[64 * wc + i] = sq[hr]; sDk[64 * wc + i] = sk[hr]; }
     }
     extra = warp_sum(extra);
-    if (lane == 0) atomicAdd(&sdG[63], extra);
+    if (lane == 0) sXt[warp] = extra;
   }
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
     float db = dbrow[hr];
     db += __shfl_xor_sync(0xffffffffu, db, 1); db += __shfl_xor_sync(0xffffffffu, db, 2);
-    if (t == 0) atomicAdd(&sdB[m0 + g + 8 * hr], db);
+    if (t == 0) sdB[64 * wc + m0 + g + 8 * hr] += db;
   }
   __syncthreads();
   // ---- chain rule of the normalisation: y = s x / (|x| + eps), y^ = s x r:  dx = s r dy - y^ (y^ . dy) / (s |x|) ------------------------------------
@@ -1070,8 +1084,8 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     float fq = 0.f, fk = 0.f;
     if (p.l2norm) {
       const float nq = p.scale / mq - 1e-6f, nk = 1.f / mk - 1e-6f;   // |q|, |k|
-      fq = nq > 0.f ? sDq[i] / (p.scale * nq) : 0.f;
-      fk = nk > 0.f ? sDk[i] / nk : 0.f;
+      fq = nq > 0.f ? ((sDq[i] + sDq[64 + i]) + (sDq[128 + i] + sDq[192 + i])) / (p.scale * nq) : 0.f;
+      fk = nk > 0.f ? ((sDk[i] + sDk[64 + i]) + (sDk[128 + i] + sDk[192 + i])) / nk : 0.f;
     }
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
@@ -1108,12 +1122,12 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
             *reinterpret_cast<const uint4*>((which ? ok : oq) + r * 136 + c8);
     }
   }
-  if (tid < rows) p.dbeta[s_base + (t0 + tid) * s_tok] = sdB[tid];
+  if (tid < rows) p.dbeta[s_base + (t0 + tid) * s_tok] = (sdB[tid] + sdB[64 + tid]) + (sdB[128 + tid] + sdB[192 + tid]) + sdB[256 + tid];
   // ---- dg: reverse cumulative sum of dG inside the chunk ---------------------------------------------------------------------------------------
   if constexpr (KDA) {
     const int s = tid >> 7, c = tid & 127;   // 16-row segment, channel
     float acc = 0.f, loc[16];
-    if (s == 3) acc = sEx[c] + sTS[c] * ex2(sG[63 * 132 + c]);
+    if (s == 3) acc = (sEx[c] + sEx[128 + c]) + (sEx[256 + c] + sEx[384 + c]) + sTS[c] * ex2(sG[63 * 132 + c]);
 #pragma unroll
     for (int r = 15; r >= 0; --r) {
       acc += sDG[(16 * s + r) * 132 + c];
@@ -1128,8 +1142,9 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       if (16 * s + r < rows) p.dg[gk_base + (int64_t)(t0 + 16 * s + r) * gk_tok + c] = loc[r] + post;
   } else if (p.variant == DR_GATED && warp == 0) {
     float ts = sTS[lane] + sTS[lane + 32] + sTS[lane + 64] + sTS[lane + 96];
-    ts = warp_sum(ts) * expf(sGs[63]);
-    float lo = sdG[lane], hi = sdG[lane + 32] + (lane == 31 ? ts : 0.f);
+    ts = warp_sum(ts) * expf(sGs[63]) + warp_sum(lane < 16 ? sXt[lane] : 0.f);
+    float lo = (sdG[lane] + sdG[64 + lane]) + (sdG[128 + lane] + sdG[192 + lane]);
+    float hi = (sdG[lane + 32] + sdG[96 + lane]) + (sdG[160 + lane] + sdG[224 + lane]) + (lane == 31 ? ts : 0.f);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float a = __shfl_down_sync(0xffffffffu, lo, o), c = __shfl_down_sync(0xffffffffu, hi, o);
