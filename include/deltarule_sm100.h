@@ -57,7 +57,9 @@ typedef enum DrChunkPath {
   DR_PATH_TCGEN05 = 2, /* tcgen05/TMEM bf16-operand kernel (K=V=128, chunk 64, bf16 q,k,v) */
   DR_PATH_SPLIT = 3    /* two kernels: chunk-parallel intra-chunk pass + tcgen05 state pass over a caller
                           workspace (dr_workspace_bytes(desc, 0)); every variant, K=V=128, chunk 64, bf16
-                          q,k,v.  AUTO picks it for KDA when the workspace is given. */
+                          q,k,v.  AUTO picks it for KDA when the workspace is given. */,
+  DR_PATH_TRANSITION = 4 /* two kernels, every chunk's effect on the state computed chunk-parallel; K = V = 64 or 128, any
+                            storage types, caller workspace (dr_workspace_bytes(desc, 0)) */
 } DrChunkPath;
 
 /* Values the device status word can take (written by kernels, never trapped). */

@@ -29,7 +29,7 @@ _HEADERS = sorted(f.name for f in list((_PKG / "csrc").glob("*.cuh")) + list((_P
 DR_DELTA, DR_GATED, DR_KDA = 0, 1, 2
 DR_F32, DR_BF16 = 0, 1
 DR_LAYOUT_BHTD, DR_LAYOUT_BTHD = 0, 1
-DR_PATH_AUTO, DR_PATH_FP32, DR_PATH_TCGEN05, DR_PATH_SPLIT = 0, 1, 2, 3
+DR_PATH_AUTO, DR_PATH_FP32, DR_PATH_TCGEN05, DR_PATH_SPLIT, DR_PATH_TRANSITION = 0, 1, 2, 3, 4
 
 # bits of the device status word (DR_DEV_* in include/deltarule_sm100.h)
 DEVICE_STATUS_BITS = {1: "a bounded wait on an mbarrier ran out", 2: "an index check failed"}

@@ -52,7 +52,7 @@ int validate_common(const DrDesc* d, bool need_chunk) {
     // The reference raises ValueError when chunk_size % 16 != 0 for Gated DeltaNet and KDA
     // (gated_deltanet.py:318-321, kda.py:438-441); DeltaNet has no such rule.
     if (d->variant != DR_DELTA && d->chunk % 16) return DR_ERR_CHUNK;
-    if (d->path < DR_PATH_AUTO || d->path > DR_PATH_SPLIT) return DR_ERR_UNSUPPORTED;
+    if (d->path < DR_PATH_AUTO || d->path > DR_PATH_TRANSITION) return DR_ERR_UNSUPPORTED;
   }
   return DR_OK;
 }
@@ -122,9 +122,12 @@ int resolve_chunk_path(const DrDesc* d) {
 
 // AUTO without a tensor-core kernel: with scratch, whole chunks run in parallel (transition form); from two chunks on (one
 // chunk has no parallelism over the recurrence's), and up to 1 GB of scratch.
+bool trans_eligible(const DrDesc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
 int64_t trans_scratch(const DrDesc* d) {
-  if (resolve_chunk_path(d) != kPathRecurrence || d->K != d->V || (d->K != 64 && d->K != 128) || d->T <= 64) return 0;
+  if (!trans_eligible(d)) return 0;
   const int64_t need = dr::trans_workspace_bytes((int64_t)d->B * d->H, d->T, d->K);
+  if (d->path == DR_PATH_TRANSITION) return need;
+  if (resolve_chunk_path(d) != kPathRecurrence || d->T <= 64) return 0;
   return need <= (int64_t)1 << 30 ? need : 0;
 }
 
@@ -185,6 +188,7 @@ const char* dr_last_path(void) { return tl_path; }
 int64_t dr_workspace_bytes(const DrDesc* d, int op) {
   int s = validate_common(d, true);
   if (s != DR_OK) return s;
+  if (op == 0 && d->path == DR_PATH_TRANSITION) return trans_scratch(d);
   if (op == 0)
     return (resolve_chunk_path(d) == DR_PATH_SPLIT && split_eligible(d))
                ? dr::split_workspace_bytes((int64_t)d->B * d->H, d->T) : 0;
@@ -231,6 +235,11 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
     return check_cuda(dr::launch_chunk_fp32(p, st));
   }
   const int64_t scratch = trans_scratch(d);
+  if (path == DR_PATH_TRANSITION) {
+    if (!trans_eligible(d)) return DR_ERR_UNSUPPORTED;
+    if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
+    if (!workspace || (int64_t)workspace_bytes < scratch) return DR_ERR_WORKSPACE;
+  }
   if (scratch > 0 && workspace && aligned16(workspace) && (int64_t)workspace_bytes >= scratch) {
     tl_path = "chunk_transition";
     g_launches.fetch_add(2);

@@ -20,12 +20,12 @@ import torch
 
 from . import _lib
 from ._lib import (DR_BF16, DR_DELTA, DR_F32, DR_GATED, DR_KDA, DR_LAYOUT_BHTD, DR_LAYOUT_BTHD,
-                   DR_PATH_AUTO, DR_PATH_FP32, DR_PATH_TCGEN05, DR_PATH_SPLIT, DrDesc)
+                   DR_PATH_AUTO, DR_PATH_FP32, DR_PATH_TCGEN05, DR_PATH_SPLIT, DR_PATH_TRANSITION, DrDesc)
 
 Tensor = torch.Tensor
 _NATIVE = {torch.float32: DR_F32, torch.bfloat16: DR_BF16}
 _PATHS = {None: DR_PATH_AUTO, "auto": DR_PATH_AUTO, "fp32": DR_PATH_FP32, "tcgen05": DR_PATH_TCGEN05,
-          "split": DR_PATH_SPLIT}
+          "split": DR_PATH_SPLIT, "transition": DR_PATH_TRANSITION}
 
 # Kernel family used by the chunk entry point when a call does not say; tests set it to
 # force one family ("fp32" / "tcgen05").
