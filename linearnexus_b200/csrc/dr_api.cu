@@ -120,15 +120,24 @@ int resolve_chunk_path(const DrDesc* d) {
   return kPathRecurrence;
 }
 
-// AUTO without a tensor-core kernel: with scratch, whole chunks run in parallel (transition form); from two chunks on (one
-// chunk has no parallelism over the recurrence's), and up to 1 GB of scratch.
+// Shapes of the transition form, and its scratch where AUTO takes it (given that scratch); 0 elsewhere.
+//  * No tensor-core kernel for the storage types: in place of the token recurrence from two chunks on (with one chunk there is
+//    nothing to run in parallel).
+//  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.6 us per chunk, KDA's state
+//    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave and there are chunks
+//    enough to pay for the longer first pass (measured for 4, 8, 16 sequences: even at 5 chunks, 118 vs 90 us at 16 x 32
+//    chunks, 228 vs 80 us at 4 x 64; at 32 sequences the one-CTA kernels are ahead).  KDA switches from 17 chunks on: up to
+//    there its two-kernel form, what AUTO has always meant for it, is at most 15 us behind.
+// Both up to 1 GB of scratch.
 bool trans_eligible(const DrDesc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
 int64_t trans_scratch(const DrDesc* d) {
   if (!trans_eligible(d)) return 0;
-  const int64_t need = dr::trans_workspace_bytes((int64_t)d->B * d->H, d->T, d->K);
+  const int64_t units = (int64_t)d->B * d->H;
+  const int64_t need = dr::trans_workspace_bytes(units, d->T, d->K, split_eligible(d));
   if (d->path == DR_PATH_TRANSITION) return need;
-  if (resolve_chunk_path(d) != kPathRecurrence || d->T <= 64) return 0;
-  return need <= (int64_t)1 << 30 ? need : 0;
+  if (d->path != DR_PATH_AUTO || need > (int64_t)1 << 30) return 0;
+  if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d)) return d->T > 64 ? need : 0;
+  return units <= 18 && d->T > (d->variant == DR_KDA ? 16 : 5) * 64 ? need : 0;
 }
 
 bool fp32_chunk_eligible(const DrDesc* d) { return d->chunk <= 64 && d->K <= 128; }
@@ -194,8 +203,8 @@ int64_t dr_workspace_bytes(const DrDesc* d, int op) {
                ? dr::split_workspace_bytes((int64_t)d->B * d->H, d->T) : 0;
   if (op == 1) return dr::bwd_workspace_bytes(d);
   if (op == 2) {
-    const int64_t need = dr_workspace_bytes(d, 0);
-    return need != 0 ? need : trans_scratch(d);
+    const int64_t need = dr_workspace_bytes(d, 0), more = trans_scratch(d);
+    return need < 0 || need > more ? need : more;
   }
   return DR_ERR_UNSUPPORTED;
 }
@@ -210,6 +219,17 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
   const dr::FwdParams p = make_fwd(d, q, k, v, g, beta, h0, o, hT, status_dev);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int path = resolve_chunk_path(d);
+  const int64_t scratch = trans_scratch(d);
+  if (path == DR_PATH_TRANSITION) {
+    if (!trans_eligible(d)) return DR_ERR_UNSUPPORTED;
+    if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
+    if (!workspace || (int64_t)workspace_bytes < scratch) return DR_ERR_WORKSPACE;
+  }
+  if (scratch > 0 && workspace && aligned16(workspace) && (int64_t)workspace_bytes >= scratch) {
+    tl_path = "chunk_transition";
+    g_launches.fetch_add(2);
+    return check_cuda(dr::launch_chunk_trans(p, split_eligible(d), workspace, sm_count(), st));
+  }
   if (path == DR_PATH_SPLIT) {
     if (!split_eligible(d)) return DR_ERR_UNSUPPORTED;
     const int64_t need = dr::split_workspace_bytes((int64_t)d->B * d->H, d->T);
@@ -233,17 +253,6 @@ int dr_chunk_fwd(const DrDesc* d, const void* q, const void* k, const void* v, c
     tl_path = "chunk_fp32";
     g_launches.fetch_add(1);
     return check_cuda(dr::launch_chunk_fp32(p, st));
-  }
-  const int64_t scratch = trans_scratch(d);
-  if (path == DR_PATH_TRANSITION) {
-    if (!trans_eligible(d)) return DR_ERR_UNSUPPORTED;
-    if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
-    if (!workspace || (int64_t)workspace_bytes < scratch) return DR_ERR_WORKSPACE;
-  }
-  if (scratch > 0 && workspace && aligned16(workspace) && (int64_t)workspace_bytes >= scratch) {
-    tl_path = "chunk_transition";
-    g_launches.fetch_add(2);
-    return check_cuda(dr::launch_chunk_trans(p, workspace, sm_count(), st));
   }
   // AUTO without a tensor-core kernel for the shape, and DR_PATH_FP32 with chunks longer than 64 or K > 128
   tl_path = "recurrent";

@@ -17,4 +17,9 @@ cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, 
   return kda::launch_chunk_packed(p, seqs, workspace, stream);
 }
 
+int64_t trans_bf16_workspace_bytes(int64_t units, int T) { return kda::trans_workspace_bytes(units, T); }
+cudaError_t launch_chunk_trans_bf16(const FwdParams& p, void* workspace, int sms, cudaStream_t stream) {
+  return kda::launch_trans(p, workspace, sms, stream);
+}
+
 }  // namespace dr

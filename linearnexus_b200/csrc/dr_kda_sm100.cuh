@@ -26,6 +26,7 @@
 #pragma once
 
 #include "dr_chunk_sm100.cuh"
+#include "dr_mma.cuh"
 
 namespace dr {
 namespace kda {
@@ -131,10 +132,16 @@ struct IntraParams {
 struct IntraPackedParams : IntraParams {
   SeqTable seqs;
 };
+// The pass in transition form (see "few sequences" below): fragments instead of records.
+struct IntraTransParams : IntraParams {
+  uint4 *nf, *yf;     // [chunks][8 | 4 row tiles][8 k-steps][32 lanes]: A operands of m16n8k16
+  float4 *zf, *of;    // [chunks][8 | 4 row tiles][16 column tiles][32 lanes]: addends
+  float* el;          // [chunks][128] e^{G_L}
+};
 
 template <class Params>
 __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constant__ Params P) {
-  constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value;
+  constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value, kTrans = std::is_same<Params, IntraTransParams>::value;
   const FwdParams& p = P.p;
   extern __shared__ __align__(1024) uint8_t smem[];
   float* sG = reinterpret_cast<float*>(smem + IN_G);
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
     const int nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks;
     n = blockIdx.x % nchunks;
     b = unit / p.map.H; h = unit % p.map.H;
-    rec += ((int64_t)unit * nchunks + n) * WS_REC;
+    if constexpr (!kTrans) rec += ((int64_t)unit * nchunks + n) * WS_REC;
   }
   const int rows = min(kC, T - n * kC), t0 = tok0 + n * kC;
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
@@ -408,6 +415,142 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   __syncthreads();
   // ---- T = (I + diag(beta) A_kk)^-1 -----------------------------------------------------------------------------
   sm100::block_inverse_64(sAkk, sBeta, sT, tid);
+  if constexpr (kTrans) {
+    // ---- the chunk's effect on the state and on its own output, as fragments of trans_state_kernel ----------------------------
+    //   N = -Kd^T W, Z = Kd^T U, Y = Qg - A_qk W, A_qk U   with W = T diag(beta) k^ e^G, U = T diag(beta) V
+    // Tb = T diag(beta) -> bf16 over A_kk; A_qk masked in place; then (T and G dead) V over T, k^ e^G over G, Qg over q, Kd over k
+    __nv_bfloat16* sTb = sWst;                                              // [64][72]
+    __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(smem + IN_T);      // [64][136]
+    __nv_bfloat16* sKg = reinterpret_cast<__nv_bfloat16*>(smem + IN_G);     // [64][136]
+    uint4 vv[4], qg[4], kd[4], kg[4];
+    const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+      vv[it] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < rows) vv[it] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.v) + v_base + (t0 + row) * v_tok + col);
+    }
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const int piece = tid + kThreads * it, row = piece >> 3, col = (piece & 7) * 8;
+      float a[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? sT[row * LDT + col + e] * sBeta[col + e] : 0.f;
+      *reinterpret_cast<uint4*>(sTb + row * LDQ + col) = pack8(a);
+      if (col + 7 > row && (col >> 4) <= (row >> 4)) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (col + e > row) sAqk[row * LDQ + col + e] = __float2bfloat16_rn(0.f);
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+      const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col), uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
+      const uint32_t wq[4] = {uq.x, uq.y, uq.z, uq.w}, wk[4] = {uk.x, uk.y, uk.z, uk.w};
+      const float rq = sRq[row], rk = sRk[row];
+      float a[8], c[8], d[8];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 gg = *reinterpret_cast<const float2*>(sG + row * LDF + col + 2 * e), gl = *reinterpret_cast<const float2*>(sG + 63 * LDF + col + 2 * e);
+        const float2 qq = bf2(wq[e]), kk = bf2(wk[e]);
+        const float e0 = ex2(gg.x), e1 = ex2(gg.y);
+        a[2 * e] = qq.x * rq * e0; a[2 * e + 1] = qq.y * rq * e1;
+        c[2 * e] = kk.x * rk * ex2(gl.x - gg.x); c[2 * e + 1] = kk.y * rk * ex2(gl.y - gg.y);
+        d[2 * e] = kk.x * rk * e0; d[2 * e + 1] = kk.y * rk * e1;
+      }
+      qg[it] = pack8(a); kd[it] = pack8(c); kg[it] = pack8(d);
+    }
+    const int64_t chunk = blockIdx.x;
+    if (tid < kD) P.el[chunk * kD + tid] = ex2(sG[63 * LDF + tid]);
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+      *reinterpret_cast<uint4*>(sV + row * LDH + col) = vv[it];
+      *reinterpret_cast<uint4*>(sQ + row * LDH + col) = qg[it];
+      *reinterpret_cast<uint4*>(sK + row * LDH + col) = kd[it];
+      *reinterpret_cast<uint4*>(sKg + row * LDH + col) = kg[it];
+    }
+    __syncthreads();
+    const uint32_t aTb = tc::smem_u32(sTb), aV = tc::smem_u32(sV), aKg = tc::smem_u32(sKg), aKd = tc::smem_u32(sK), aAq = tc::smem_u32(sAqk);
+    // W^T, U^T of the warp's 16 channels / value columns (rows), columns = tokens; then as B operands (k = token)
+    uint32_t Wb[4][2][2], Ub[4][2][2];   // [16-token step][8-column half][k half]
+    {
+      float W[8][4], U[8][4];
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        W[nt][0] = W[nt][1] = W[nt][2] = W[nt][3] = 0.f;
+        U[nt][0] = U[nt][1] = U[nt][2] = U[nt][3] = 0.f;
+      }
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t aw[4], au[4];
+        mma::ldsm4t(aw, mma::frag_at(aKg, LDH, 16 * ks, 16 * warp, lane));
+        mma::ldsm4t(au, mma::frag_at(aV, LDH, 16 * ks, 16 * warp, lane));
+#pragma unroll
+        for (int n2 = 0; n2 < 4; ++n2) {
+          if (n2 >= ks) {
+            uint32_t bt[4];
+            mma::ldsm4(bt, mma::frag_b(aTb, LDQ, 16 * n2, 16 * ks, lane));
+            mma::bf16(W[2 * n2], aw, bt[0], bt[1]);
+            mma::bf16(W[2 * n2 + 1], aw, bt[2], bt[3]);
+            mma::bf16(U[2 * n2], au, bt[0], bt[1]);
+            mma::bf16(U[2 * n2 + 1], au, bt[2], bt[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+          for (int kh = 0; kh < 2; ++kh) {
+            Wb[ks][hf][kh] = mma::pack(W[2 * ks + kh][2 * hf], W[2 * ks + kh][2 * hf + 1]);
+            Ub[ks][hf][kh] = mma::pack(U[2 * ks + kh][2 * hf], U[2 * ks + kh][2 * hf + 1]);
+          }
+    }
+#pragma unroll 1
+    for (int mt = 0; mt < 12; ++mt) {   // rows of [Kd^T (8 tiles); A_qk (4 tiles)]
+      const bool st = mt < 8;
+      const int m = st ? mt : mt - 8;
+      float w[2][4], u[2][4];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) { w[hf][0] = w[hf][1] = w[hf][2] = w[hf][3] = 0.f; u[hf][0] = u[hf][1] = u[hf][2] = u[hf][3] = 0.f; }
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        if (st || ks <= m) {
+          uint32_t a[4];
+          if (st) mma::ldsm4t(a, mma::frag_at(aKd, LDH, 16 * ks, 16 * m, lane));
+          else mma::ldsm4(a, mma::frag_a(aAq, LDQ, 16 * m, 16 * ks, lane));
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            mma::bf16(w[hf], a, Wb[ks][hf][0], Wb[ks][hf][1]);
+            mma::bf16(u[hf], a, Ub[ks][hf][0], Ub[ks][hf][1]);
+          }
+        }
+      }
+      const int64_t at = (chunk * (st ? 8 : 4) + m) * 8 + warp;
+      if (st) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) { w[hf][0] = -w[hf][0]; w[hf][1] = -w[hf][1]; w[hf][2] = -w[hf][2]; w[hf][3] = -w[hf][3]; }
+      } else {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {
+            const float2 q2 = bf2(*reinterpret_cast<const uint32_t*>(sQ + (16 * m + g + 8 * hr) * LDH + 16 * warp + 8 * hf + 2 * t));
+            w[hf][2 * hr] = q2.x - w[hf][2 * hr];
+            w[hf][2 * hr + 1] = q2.y - w[hf][2 * hr + 1];
+          }
+      }
+      (st ? P.nf : P.yf)[at * 32 + lane] = make_uint4(mma::pack(w[0][0], w[0][1]), mma::pack(w[0][2], w[0][3]), mma::pack(w[1][0], w[1][1]), mma::pack(w[1][2], w[1][3]));
+      float4* dst = (st ? P.zf : P.of) + at * 64 + lane;
+      dst[0] = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
+      dst[32] = make_float4(u[1][0], u[1][1], u[1][2], u[1][3]);
+    }
+    return;
+  }
   // ---- record tiles: T diag(beta), A_qk, Qg = scale q^ e^G, Kd = k^ e^{G_L - G}, e^{G_L} ------------------------
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
@@ -819,6 +962,146 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
+}
+
+// ---- few sequences: the state pass in transition form ------------------------------------------------------------------------
+// The state kernel above has one CTA per sequence and ~2 us of dependent tensor-memory round trips per chunk, the fused kernel
+// ~3.7 us: with a handful of sequences most SMs idle.  Here a chunk's whole effect on the state is one product,
+//     S' = e^{G_L} S + N S + Z,    O = Y S + A_qk U,
+// with N, Z, Y, A_qk U from the intra pass, and the value columns are cut into slices of 8 NT per CTA.  Warps 0-7 keep 16 state
+// rows each in registers, their bf16 copy in shared memory is the B operand; warps 8-11 compute the output beside the chain.
+// Operands are bf16 where the other forwards have bf16 operands (N, Y and the copy of S), the state, Z and the sums fp32.
+constexpr int kTrThreads = 12 * 32;
+
+template <int NT>
+__global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid_constant__ IntraTransParams P) {
+  constexpr int VS = 8 * NT, LDS = VS + 8, SL = kD / VS;
+  const FwdParams& p = P.p;
+  __shared__ __align__(16) __nv_bfloat16 sS[2][kD * LDS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int unit = blockIdx.x / SL, v0 = (blockIdx.x % SL) * VS;
+  const int b = unit / p.map.H, h = unit % p.map.H, T = p.map.T, N = (T + kC - 1) / kC;
+  const int64_t chunk0 = (int64_t)unit * N;
+  const bool state = warp < 8;
+  const int mt = state ? warp : warp - 8, tiles = state ? 8 : 4, r0 = 16 * mt + g, r1 = r0 + 8;
+  const uint4* fa = (state ? P.nf : P.yf) + lane;
+  const float4* fc = (state ? P.zf : P.of) + (v0 / 8) * 32 + lane;
+  uint4 a[8];
+  float4 c[NT];
+  float S[NT][4], el0 = 0.f, el1 = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) a[ks] = fa[((chunk0 * tiles + mt) * 8 + ks) * 32];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) c[nt] = fc[((chunk0 * tiles + mt) * 16 + nt) * 32];
+  if (state) {
+    el0 = P.el[chunk0 * kD + r0]; el1 = P.el[chunk0 * kD + r1];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      float2 lo = make_float2(0.f, 0.f), hi = lo;
+      if (p.h0) {
+        lo = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t);
+        hi = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t);
+      }
+      S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
+    }
+  }
+  const int64_t o_tok = p.map.tok(kD), o_base = p.map.base(b, h, kD) + v0;
+  for (int n = 0; n < N; ++n) {
+    __nv_bfloat16* cS = sS[n & 1];
+    if (state) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        *reinterpret_cast<uint32_t*>(cS + r0 * LDS + 8 * nt + 2 * t) = mma::pack(S[nt][0], S[nt][1]);
+        *reinterpret_cast<uint32_t*>(cS + r1 * LDS + 8 * nt + 2 * t) = mma::pack(S[nt][2], S[nt][3]);
+      }
+    }
+    __syncthreads();
+    float d[NT][4], e[NT][4];   // two accumulators: shorter chains
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      d[nt][0] = c[nt].x; d[nt][1] = c[nt].y; d[nt][2] = c[nt].z; d[nt][3] = c[nt].w;
+      e[nt][0] = e[nt][1] = e[nt][2] = e[nt][3] = 0.f;
+    }
+    const int64_t cn = chunk0 + (n + 1 < N ? n + 1 : n);   // the next chunk's operands replace this one's as they are used
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) c[nt] = fc[((cn * tiles + mt) * 16 + nt) * 32];
+    const uint32_t base = tc::smem_u32(cS);
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const uint32_t ar[4] = {a[ks].x, a[ks].y, a[ks].z, a[ks].w};
+      a[ks] = fa[((cn * tiles + mt) * 8 + ks) * 32];
+#pragma unroll
+      for (int n2 = 0; n2 < NT / 2; ++n2) {
+        uint32_t bb[4];
+        mma::ldsm4t(bb, mma::frag_bt(base, LDS, 16 * ks, 16 * n2, lane));
+        mma::bf16((ks & 1) ? e[2 * n2] : d[2 * n2], ar, bb[0], bb[1]);
+        mma::bf16((ks & 1) ? e[2 * n2 + 1] : d[2 * n2 + 1], ar, bb[2], bb[3]);
+      }
+    }
+    if (state) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        S[nt][0] = el0 * S[nt][0] + (d[nt][0] + e[nt][0]); S[nt][1] = el0 * S[nt][1] + (d[nt][1] + e[nt][1]);
+        S[nt][2] = el1 * S[nt][2] + (d[nt][2] + e[nt][2]); S[nt][3] = el1 * S[nt][3] + (d[nt][3] + e[nt][3]);
+      }
+      el0 = P.el[cn * kD + r0]; el1 = P.el[cn * kD + r1];
+    } else {
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int tok = n * kC + r0 + 8 * hr;
+        if (tok < T) {
+          const int64_t at = o_base + (int64_t)tok * o_tok + 2 * t;
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const float x = d[nt][2 * hr] + e[nt][2 * hr], y = d[nt][2 * hr + 1] + e[nt][2 * hr + 1];
+            if (p.out_dt == DR_BF16) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.o) + at + 8 * nt) = mma::pack(x, y);
+            else *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.o) + at + 8 * nt) = make_float2(x, y);
+          }
+        }
+      }
+    }
+  }
+  if (state && p.hT) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t) = make_float2(S[nt][2], S[nt][3]);
+    }
+  }
+}
+
+// bytes per chunk: N, Y bf16; Z, A_qk U, e^{G_L} fp32
+constexpr int64_t kTrN = 128 * 128 * 2, kTrY = 64 * 128 * 2, kTrZ = 128 * 128 * 4, kTrO = 64 * 128 * 4, kTrE = 512;
+inline int64_t trans_workspace_bytes(int64_t units, int T) {
+  return units * ((T + kC - 1) / kC) * (kTrN + kTrY + kTrZ + kTrO + kTrE);
+}
+inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cudaStream_t stream) {
+  thread_local int attr_dev = -1;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (attr_dev != dev) {
+    e = cudaFuncSetAttribute(intra_kernel<IntraTransParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    if (e != cudaSuccess) return e;
+    attr_dev = dev;
+  }
+  const int64_t units = (int64_t)p.map.B * p.map.H, nc = units * ((p.map.T + kC - 1) / kC);
+  IntraTransParams P;
+  uint8_t* w = reinterpret_cast<uint8_t*>(workspace);
+  P.p = p;
+  P.ws = nullptr;
+  P.nf = reinterpret_cast<uint4*>(w); w += nc * kTrN;
+  P.yf = reinterpret_cast<uint4*>(w); w += nc * kTrY;
+  P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;
+  P.of = reinterpret_cast<float4*>(w); w += nc * kTrO;
+  P.el = reinterpret_cast<float*>(w);
+  intra_kernel<IntraTransParams><<<(unsigned)nc, kThreads, IN_TOTAL, stream>>>(P);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // 16 columns per CTA while the slices fit one wave: the chain's length is what counts
+  if (units * 8 <= sms) trans_state_kernel<2><<<(unsigned)(units * 8), kTrThreads, 0, stream>>>(P);
+  else trans_state_kernel<4><<<(unsigned)(units * 4), kTrThreads, 0, stream>>>(P);
+  return cudaGetLastError();
 }
 
 template <class IP, class SP>

@@ -15,9 +15,12 @@ int64_t split_workspace_bytes(int64_t units, int T);
 cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches);
 cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream);
 
-// forward in transition form (two kernels; K = V = 64 or 128, any storage types); the workspace holds trans_workspace_bytes
-int64_t trans_workspace_bytes(int64_t units, int T, int D);
-cudaError_t launch_chunk_trans(const FwdParams& p, void* workspace, int sms, cudaStream_t stream);
+// forward in transition form (two kernels; K = V = 64 or 128); bf16_tensor: the bf16-operand kernels (dr_fwd.cu; bf16 q, k, v,
+// K = V = 128, chunk 64), else float32 precision for any storage type
+int64_t trans_workspace_bytes(int64_t units, int T, int D, bool bf16_tensor);
+cudaError_t launch_chunk_trans(const FwdParams& p, bool bf16_tensor, void* workspace, int sms, cudaStream_t stream);
+int64_t trans_bf16_workspace_bytes(int64_t units, int T);
+cudaError_t launch_chunk_trans_bf16(const FwdParams& p, void* workspace, int sms, cudaStream_t stream);
 
 // backward (see dr_bwd.cuh)
 int64_t bwd_workspace_bytes(const DrDesc* d);
