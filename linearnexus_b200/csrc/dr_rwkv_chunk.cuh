@@ -1,0 +1,396 @@
+// RWKV-7 (diagonal plus low rank) and RWKV-6 scans, eight tokens per step of the state, on the warp-level tensor cores in
+// float32 precision (three tf32 products per pair, dr_tf32.cuh); K = 64, value columns in multiples of 64, bf16 or float32 storage.
+//
+// With W_i the product of the block's decays up to token i, h the state at its start and u_i = a_i^T h_{i-1}:
+//     u_i = (a_i W_{i-1})^T h + sum_{j<i} ak_ij v_j + ab_ij u_j        ak_ij = sum_c a_i (W_{i-1} / W_j) k_j,  ab: with b_j
+//     o_i = (q_i W_i)^T h     + sum_{j<=i} qk_ij v_j + qb_ij u_j        qk_ij = sum_c q_i (W_i / W_j) k_j,      qb: with b_j
+//     h'  = W_7 h + sum_j (W_7 / W_j k_j) v_j^T + (W_7 / W_j b_j) u_j^T
+// so U = T D_a + (T ak) V with T = (I - ab)^-1 [8 x 8].  RWKV-6 (o_i reads h_{i-1}, a bonus u q.k on the current token, no a, b) is
+// the same without U.
+//
+// Four warps keep the state transposed in accumulators (16 value columns x 64 keys each).  An accumulator is, register for
+// register, an A operand whose contraction runs over its columns: h feeds the dots, their result feeds T, U feeds the update,
+// and nothing of the state touches memory.  Three groups of four warps stage the blocks ahead, one block in three each (staging a
+// block is a chain of ~3.5 K cycles, the state's share ~1.5 K): raw rows from a ring of asynchronous copies, decay products, the
+// row vectors and the 8 x 8 coefficients.  Hand-overs are named barriers, arrived on by one side and waited for by the other.
+//
+// What bounds it: ~100 mma per warp and block of 8 cycles each (100 cycles per token).  The token recurrence it replaces here ran
+// at 540 cycles per token whatever its instruction count or prefetch depth: one dependent reduce-and-update chain per token, and
+// 260 shared-memory wavefronts per token to feed 160 multiply-adds per thread (a 16-byte load fills a quarter of a warp per
+// wavefront, broadcast or not).  A four-token form on the CUDA cores stayed at that roof (1.18 ms against 1.14).
+#pragma once
+
+#include "dr_linrec.cuh"
+#include "dr_mma.cuh"
+#include "dr_tcgen05.cuh"
+#include "dr_tf32.cuh"
+
+namespace dr {
+namespace rwkv {
+
+using mma::AFrag;
+using mma::BFrag;
+constexpr int kK = 64, kTB = 8, kGroups = 3, kRing = 3, kStages = 4, kThreads = 128 * (1 + kGroups), kCons = 128;
+constexpr int LDR = 72;    // row vectors [token][key], read as B operands along the key axis
+constexpr int LDH = 68;    // update vectors [token][key] and values [token][column], read across tokens
+
+template <int KIND, bool BF>
+struct Ring {
+  static constexpr int NV = KIND == LR_DPLR ? 5 : 3;            // q k w [a b]
+  static constexpr int ES = BF ? 2 : 4;
+  static constexpr int kVec = kTB * kK * ES;                    // bytes of one vector's block
+  static constexpr int kTasks = (NV + 1) * kVec / 512;          // warps' worth of 16-byte pieces (v last)
+  static constexpr int kSlot = (NV + 1) * kVec;
+};
+
+struct Stage {
+  float row[16][LDR];       // 0-7: q W (RWKV-6: q W_{i-1});  8-15: a W_{i-1}
+  float upd[16][LDH];       // 0-7: W_7 / W_j k;  8-15: W_7 / W_j b
+  float v[kTB][LDH];
+  float w[kK];              // W_7
+  float qk[64], qb[64], T[64], P[64];   // [i][j]; P = T ak
+};
+
+struct Scratch {            // of one staging group
+  float inv[16][LDR];       // k / W_j, b / W_j
+  float ab[64], ak[64];
+  int wide;
+};
+template <int KIND, bool BF>
+constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + kGroups * ((int)sizeof(Scratch) + kRing * Ring<KIND, BF>::kSlot) + 64; }
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+constexpr int kBarFull = 1, kBarEmpty = 1 + kStages, kBarGroup = 1 + 2 * kStages;
+
+template <int KIND, bool BF>
+__global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecParams p) {
+  using R = Ring<KIND, BF>;
+  constexpr bool LR = KIND == LR_DPLR;
+  constexpr int NV = R::NV;
+  extern __shared__ __align__(16) uint8_t smem[];
+  static_assert(sizeof(Stage) % 16 == 0, "stages stay aligned");
+  Stage* s_st = reinterpret_cast<Stage*>(smem);
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nvs = p.V / 64, unit = blockIdx.x / nvs, v0 = (blockIdx.x % nvs) * 64;
+  const int b = unit / p.H, h = unit % p.H, T = p.T, nblk = (T + kTB - 1) / kTB;
+
+  if (threadIdx.x >= kCons) {
+    // =========================== staging =========================================================================================
+    const int grp = (threadIdx.x - kCons) >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
+    constexpr int kGrpBytes = (sizeof(Scratch) + 15) / 16 * 16 + kRing * R::kSlot;
+    uint8_t* mine = smem + kStages * sizeof(Stage) + grp * kGrpBytes;
+    Scratch& X = *reinterpret_cast<Scratch*>(mine);
+    uint8_t* ring = mine + (sizeof(Scratch) + 15) / 16 * 16;
+    constexpr int kRounds = (R::kTasks + 3) / 4;
+    const uint8_t* src[kRounds];
+    int64_t step[kRounds];
+    int rtok[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int byte = (warp + 4 * r) * 512 + lane * 16, j = byte / R::kVec, off = byte % R::kVec;
+      const LrVec* vecs[5] = {&p.q, &p.k, &p.w, &p.a, &p.b};
+      const void* ptr = p.v.p;
+      int64_t st = p.v.st, at = p.v.at(b, h, 0) + v0;
+#pragma unroll
+      for (int jj = 0; jj < NV; ++jj)
+        if (jj == j) { ptr = vecs[jj]->p; st = vecs[jj]->st; at = vecs[jj]->at(b, h, 0); }
+      rtok[r] = off / (kK * R::ES);
+      src[r] = reinterpret_cast<const uint8_t*>(ptr) + (at + rtok[r] * st) * R::ES + off % (kK * R::ES);
+      step[r] = (int64_t)kTB * st * R::ES;
+    }
+    auto issue = [&](int blk) {   // blocks of this group: blk = grp, grp + kGroups, ...
+      if (blk * kTB < T) {
+        const uint32_t slot = tc::smem_u32(ring + (blk / kGroups % kRing) * R::kSlot) + (uint32_t)(warp * 512 + lane * 16);
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+          if (warp + 4 * r < R::kTasks) {
+            const bool ok = blk * kTB + rtok[r] < T;
+            tc::cp_async16(slot + 2048u * r, src[r] + (ok ? blk * step[r] : 0), ok);
+          }
+        }
+      }
+      tc::cp_async_commit();
+    };
+    auto sync128 = [&]() { bar_sync(kBarGroup + grp, 128); };
+    auto raw = [&](const uint8_t* slot, int j, int tok, int c) -> float {
+      const uint8_t* a = slot + j * R::kVec + (tok * kK + c) * R::ES;
+      return BF ? __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(a) << 16) : *reinterpret_cast<const float*>(a);
+    };
+    const int ch = tid & 63, role = tid >> 6;   // role 0: q rows and k vectors; role 1: a rows and b vectors (RWKV-6: values)
+    const float u_ch = !LR ? p.u[(int64_t)h * kK + ch] : 0.f;
+#pragma unroll
+    for (int i = 0; i < kRing; ++i) issue(grp + kGroups * i);
+    for (int blk = grp; blk < nblk; blk += kGroups) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
+      if (tid == 0) X.wide = 0;
+      if (blk >= kStages) bar_sync(kBarEmpty + blk % kStages, 256);   // the consumers have left this stage
+      sync128();   // every thread's pieces of this block have landed
+      const uint8_t* slot = ring + (blk / kGroups % kRing) * R::kSlot;
+      Stage& S = s_st[blk % kStages];
+      const int t0 = blk * kTB;
+      if (LR || role == 0) {
+        float w[8], y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float x = raw(slot, 2, i, ch);
+          w[i] = t0 + i < T ? (LR ? expf(x) : expf(-expf(x))) : 1.f;   // tokens past the end: decay 1, zero vectors
+        }
+        float W = 1.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float x;
+          if (LR) x = role == 0 ? raw(slot, 0, i, ch) * p.scale : raw(slot, 3, i, ch);
+          else x = t0 + i < T ? p.scale / (1.f + __expf(-raw(slot, 0, i, ch))) : 0.f;   // sigmoid(r) scale
+          if (LR && role == 0) W *= w[i];
+          S.row[8 * role + i][ch] = x * W;
+          if (!(LR && role == 0)) W *= w[i];
+          y[i] = raw(slot, LR && role == 1 ? 4 : 1, i, ch);
+        }
+        if (role == 0) {
+          S.w[ch] = W;
+          if (!(W >= 5.4e-20f)) X.wide = 1;   // 2^-64: too wide for the form with 1 / W_j below
+        }
+        float D = 1.f;
+#pragma unroll
+        for (int j = 7; j >= 0; --j) {
+          S.upd[8 * role + j][ch] = y[j] * D;
+          D *= w[j];
+        }
+        float I = 1.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          I *= __fdividef(1.f, w[j]);
+          X.inv[8 * role + j][ch] = y[j] * I;
+        }
+      }
+      // values (RWKV-6: by the threads without row work)
+      if (LR) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S.v[(tid >> 6) + 2 * e][ch] = raw(slot, NV, (tid >> 6) + 2 * e, ch);
+      } else if (role == 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) S.v[e][ch] = raw(slot, NV, e, ch);
+      }
+      sync128();
+      // ---- coefficients: rows q (and a) against k / W (warp 0) and b / W (warp 1) ----------------------------------------------------
+      if (X.wide) {   // too strong a decay: every pair with the decays in between multiplied up (four lanes per pair)
+        const int which = warp & 1;
+        if (LR || which == 0)
+          for (int e = (warp >> 1) * 32 + lane; e < 64 * 2 * 2; e += 64) {
+            const int half = e & 1, pair = (e >> 1) & 63, i = pair >> 3, j = pair & 7, isa = e >> 7;
+            float acc = 0.f;
+            if ((LR || !isa) && (isa || !LR ? j < i : j <= i) && t0 + i < T) {
+              for (int c = 32 * half; c < 32 * half + 32; ++c) {
+                float x = raw(slot, which ? 4 : 1, j, c);
+                const int hi = isa || !LR ? i - 1 : i;   // a reads the state before token i's decay; so does RWKV-6
+                for (int m = j + 1; m <= hi; ++m) { const float d = raw(slot, 2, m, c); x *= LR ? expf(d) : expf(-expf(d)); }
+                float q = raw(slot, isa ? 3 : 0, i, c);
+                if (!isa) q = LR ? q * p.scale : p.scale / (1.f + __expf(-q));
+                acc += q * x;
+              }
+            }
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            if (!half) (isa ? (which ? X.ab : X.ak) : (which ? S.qb : S.qk))[pair] = acc;
+          }
+      } else if (warp < (LR ? 2 : 1)) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          const float2 x0 = *reinterpret_cast<const float2*>(&S.row[g][8 * ks + 2 * t]);
+          const float2 x1 = LR ? *reinterpret_cast<const float2*>(&S.row[8 + g][8 * ks + 2 * t]) : make_float2(0.f, 0.f);
+          const float2 y = *reinterpret_cast<const float2*>(&X.inv[8 * warp + g][8 * ks + 2 * t]);
+          AFrag<true> a;
+          a.set(x0.x, x1.x, x0.y, x1.y);
+          BFrag<true> bb;
+          bb.set(y.x, y.y);
+          mma::fma<true>((ks & 1) ? d2 : d, a, bb);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int i = g, j = 2 * t + e;
+          const float q = d[e] + d2[e], a = d[2 + e] + d2[2 + e];
+          (warp ? S.qb : S.qk)[8 * i + j] = (LR ? j <= i : j < i) ? q : 0.f;
+          if (LR) (warp ? X.ab : X.ak)[8 * i + j] = j < i ? a : 0.f;
+        }
+      }
+      if (LR) {
+        sync128();
+        // T = (I - ab)^-1 by columns (eight lanes), P = T ak
+        if (warp == 0) {
+          if (lane < 8) {
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              x[i] = i == lane ? 1.f : 0.f;
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (j < i) x[i] += X.ab[8 * i + j] * x[j];
+              S.T[8 * i + lane] = x[i];
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int e = lane; e < 64; e += 32) {
+            float acc = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc += S.T[(e & ~7) + j] * X.ak[8 * j + (e & 7)];
+            S.P[e] = acc;
+          }
+        }
+      } else {
+        // the bonus on the current token: u q.k, eight sums over the channels (two warps' halves meet through X.ab)
+        if (role == 0) {
+          float x[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            x[i] = t0 + i < T ? p.scale / (1.f + __expf(-raw(slot, 0, i, ch))) * u_ch * raw(slot, 1, i, ch) : 0.f;
+#pragma unroll
+          for (int m = 4; m >= 1; m >>= 1) {
+            const bool up = lane & m;
+#pragma unroll
+            for (int i = 0; i < m; ++i) {
+              const float send = up ? x[i] : x[i + m], keep = up ? x[i + m] : x[i];
+              x[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+            }
+          }
+          x[0] += __shfl_xor_sync(0xffffffffu, x[0], 8);
+          x[0] += __shfl_xor_sync(0xffffffffu, x[0], 16);
+          if (lane < 8) X.ab[8 * warp + lane] = x[0];
+        }
+        sync128();
+        if (tid < 8) S.qk[9 * tid] = X.ab[tid] + X.ab[8 + tid];
+      }
+      bar_arrive(kBarFull + blk % kStages, 256);
+      sync128();           // the raw block has been read by every thread
+      issue(blk + kGroups * kRing);
+    }
+    return;
+  }
+
+  // =========================== the state: warp = 16 value columns ======================================================================
+  const int vb = 16 * (threadIdx.x >> 5);
+  float S[8][4];   // tile nt: columns vb + g, + 8 (rows), keys 8 nt + 2 t, + 1
+  const float* h0 = p.h0 ? p.h0 + (int64_t)unit * kK * p.V + v0 + vb + g : nullptr;
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[nt][e] = h0 ? h0[(int64_t)(8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] : 0.f;
+  const int64_t o_at = (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + v0 + vb + g;
+  for (int blk = 0; blk < nblk; ++blk) {
+    bar_sync(kBarFull + blk % kStages, 256);
+    const Stage& St = s_st[blk % kStages];
+    // dots of q (and a) with h, transposed: rows = columns of v, columns = tokens
+    float dq[2][4], da[2][4];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) { dq[x][0] = dq[x][1] = dq[x][2] = dq[x][3] = 0.f; da[x][0] = da[x][1] = da[x][2] = da[x][3] = 0.f; }
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      AFrag<true> a;
+      a.set(S[ks][0], S[ks][2], S[ks][1], S[ks][3]);
+      BFrag<true> bq;
+      const float2 y = *reinterpret_cast<const float2*>(&St.row[g][8 * ks + 2 * t]);
+      bq.set(y.x, y.y);
+      mma::fma<true>(dq[ks & 1], a, bq);
+      if constexpr (LR) {
+        const float2 z = *reinterpret_cast<const float2*>(&St.row[8 + g][8 * ks + 2 * t]);
+        BFrag<true> ba;
+        ba.set(z.x, z.y);
+        mma::fma<true>(da[ks & 1], a, ba);
+      }
+    }
+    // the decay of h: independent of the dots' results
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float2 w = *reinterpret_cast<const float2*>(&St.w[8 * nt + 2 * t]);
+      S[nt][0] *= w.x; S[nt][1] *= w.y; S[nt][2] *= w.x; S[nt][3] *= w.y;
+    }
+    AFrag<true> av;   // V^T: rows = columns of v, k = tokens (bf16 values are exact in one term)
+    av.set(St.v[2 * t][vb + g], St.v[2 * t][vb + g + 8], St.v[2 * t + 1][vb + g], St.v[2 * t + 1][vb + g + 8]);
+    auto mul_v = [&](float (&d)[4], const BFrag<true>& bb) {
+      if constexpr (BF) {
+        mma::tf32(d, av.h, bb.l);
+        mma::tf32(d, av.h, bb.h);
+      } else {
+        mma::fma<true>(d, av, bb);
+      }
+    };
+    auto small = [&](const float* m) {   // an 8 x 8 coefficient matrix [i][j] as B operand (k = j, n = i)
+      const float2 y = *reinterpret_cast<const float2*>(m + 8 * g + 2 * t);
+      BFrag<true> bb;
+      bb.set(y.x, y.y);
+      return bb;
+    };
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {   // h += V^T (W_7 / W_j k)
+      BFrag<true> bk;
+      bk.set(St.upd[2 * t][8 * nt + g], St.upd[2 * t + 1][8 * nt + g]);
+      mul_v(S[nt], bk);
+    }
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = dq[0][e] + dq[1][e];
+    mul_v(o, small(St.qk));
+    if constexpr (LR) {
+      float u[4] = {0.f, 0.f, 0.f, 0.f};
+      AFrag<true> aa;
+      aa.set(da[0][0] + da[1][0], da[0][2] + da[1][2], da[0][1] + da[1][1], da[0][3] + da[1][3]);
+      mul_v(u, small(St.P));
+      mma::fma<true>(u, aa, small(St.T));
+      AFrag<true> au;
+      au.set(u[0], u[2], u[1], u[3]);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {   // h += U^T (W_7 / W_j b)
+        BFrag<true> bb;
+        bb.set(St.upd[8 + 2 * t][8 * nt + g], St.upd[9 + 2 * t][8 * nt + g]);
+        mma::fma<true>(S[nt], au, bb);
+      }
+      mma::fma<true>(o, au, small(St.qb));
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int tok = blk * kTB + 2 * t + (e & 1);
+      if (tok < T) st_elem(p.o, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), BF ? DR_BF16 : DR_F32, o[e]);
+    }
+    if (blk + kStages < nblk) bar_arrive(kBarEmpty + blk % kStages, 256);
+  }
+  if (p.hT) {
+    float* hT = p.hT + (int64_t)unit * kK * p.V + v0 + vb + g;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) hT[(int64_t)(8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] = S[nt][e];
+  }
+}
+
+// 16-byte-aligned rows of K = 64 and whole 64-column slices; a decode step (one or two blocks) stays with the token kernel
+inline bool eligible(int kind, bool bf, const LinRecParams& p) {
+  const int ep = bf ? 8 : 4;
+  auto ok = [&](const LrVec& v) { return (reinterpret_cast<uintptr_t>(v.p) & 15) == 0 && v.sb % ep == 0 && v.sh % ep == 0 && v.st % ep == 0; };
+  return p.K == kK && p.V % 64 == 0 && p.T > kTB && p.s_v == 1 && ok(p.q) && ok(p.k) && ok(p.w) && ok(p.v) &&
+         (kind != LR_DPLR || (ok(p.a) && ok(p.b)));
+}
+
+template <int KIND, bool BF>
+inline cudaError_t launch_t(const LinRecParams& p, cudaStream_t stream) {
+  constexpr int bytes = smem_bytes<KIND, BF>();
+  auto kern = rwkv_chunk_kernel<KIND, BF>;
+  thread_local int attr_dev = -1;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (attr_dev != dev) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    attr_dev = dev;
+  }
+  kern<<<(unsigned)((int64_t)p.B * p.H * (p.V / 64)), kThreads, bytes, stream>>>(p);
+  return cudaGetLastError();
+}
+inline cudaError_t launch(int kind, bool bf, const LinRecParams& p, cudaStream_t stream) {
+  if (kind == LR_DPLR) return bf ? launch_t<LR_DPLR, true>(p, stream) : launch_t<LR_DPLR, false>(p, stream);
+  return bf ? launch_t<LR_RWKV6, true>(p, stream) : launch_t<LR_RWKV6, false>(p, stream);
+}
+
+}  // namespace rwkv
+}  // namespace dr

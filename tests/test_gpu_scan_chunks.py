@@ -31,3 +31,31 @@ def test_ssd_chunks(B, T, H, P, N, G):
                               chunk_size=64, **kw)
     _check(s, rs, 1e-5)
     _check(y, ry, 5e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,H,T,V,layout", [(1, 2, 9, 64, "bhtd"), (2, 3, 31, 128, "bthd"), (1, 2, 130, 64, "bhtd"), (1, 1, 203, 192, "bhtd")])
+def test_rwkv_blocks(dtype, B, H, T, V, layout):
+    """Four tokens per step of the state: tails of every length, several value slices, strong and vanishing decays."""
+    g = torch.Generator().manual_seed(T)
+    f = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).to(dtype)
+    kk = torch.nn.functional.normalize(torch.randn(B, H, T, 64, generator=g), dim=-1)
+    q, k, v = f(B, H, T, 64), f(B, H, T, 64, scale=0.5), f(B, H, T, V)
+    a, b = (-kk).to(dtype), (kk * torch.sigmoid(torch.randn(B, H, T, 64, generator=g))).to(dtype)
+    gk, u, h0 = -torch.exp(f(B, H, T, 64) - 1.0), torch.randn(H, 64, generator=g) * 0.5, torch.randn(B, H, 64, V, generator=g) * 0.1
+    gk[:, :, T // 2] = -60.0
+    gk[:, :, T // 3] = 0.0
+    gk = gk.to(dtype)
+    dev = lambda t: t.cuda() if layout == "bhtd" else t.transpose(1, 2).contiguous().cuda().transpose(1, 2)
+    d = lambda t: t.double()
+    tol = 5e-3 if dtype == torch.bfloat16 else 5e-6
+    o, s = L.dplr_delta_rule_recurrent(*(dev(t) for t in (q, k, v, a, b, gk)), scale=0.125, initial_state=h0.cuda())
+    ro, rs = R.dplr_delta_rule_recurrent(*(d(t) for t in (q, k, v, a, b, gk)), scale=0.125, initial_state=d(h0), compute_dtype=torch.float64)
+    _check(s, rs, 5e-6)
+    _check(o, ro, tol)
+    w = (-torch.randn(B, H, T, 64, generator=g).abs() - 0.5).to(dtype)
+    w[:, :, T // 2] = 5.0
+    o, s = L.rwkv6_recurrent(*(dev(t) for t in (q, k, v, w)), u.cuda(), scale=0.125, initial_state=h0.cuda())
+    ro, rs = R.rwkv6_recurrent(*(d(t) for t in (q, k, v, w, u)), scale=0.125, initial_state=d(h0), compute_dtype=torch.float64)
+    _check(s, rs, 5e-6)
+    _check(o, ro, tol)
