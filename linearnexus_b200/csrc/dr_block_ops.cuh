@@ -87,6 +87,7 @@ template <int DT> using ConvVec = Vec<DT>;
 
 template <int DT, int MW, bool EXACT>   // EXACT: the window is MW (compiled for 1..4); else any window up to MW
 __global__ void __launch_bounds__(128) short_conv_kernel(const ConvParams p) {
+  pdl_entry();
   using Q = ConvVec<DT>;
   using Raw = uint4;
   constexpr int N = Q::N, HW = MW - 1, ROWS = kConvSteps + HW;
@@ -164,11 +165,11 @@ inline cudaError_t launch_short_conv(const ConvParams& p, int dt, cudaStream_t s
   dim3 grid((cvecs + 31) / 32, (p.T + 4 * kConvSteps - 1) / (4 * kConvSteps), p.B);
 #define DR_CONV_CASE(DT)                                                                        \
   switch (p.W) {                                                                                \
-    case 1: short_conv_kernel<DT, 1, true><<<grid, 128, 0, stream>>>(p); break;                 \
-    case 2: short_conv_kernel<DT, 2, true><<<grid, 128, 0, stream>>>(p); break;                 \
-    case 3: short_conv_kernel<DT, 3, true><<<grid, 128, 0, stream>>>(p); break;                 \
-    case 4: short_conv_kernel<DT, 4, true><<<grid, 128, 0, stream>>>(p); break;                 \
-    default: short_conv_kernel<DT, kConvMaxW, false><<<grid, 128, 0, stream>>>(p); break;       \
+    case 1: return launch_pdl(short_conv_kernel<DT, 1, true>, grid, dim3(128), 0, stream, p);                        \
+    case 2: return launch_pdl(short_conv_kernel<DT, 2, true>, grid, dim3(128), 0, stream, p);                        \
+    case 3: return launch_pdl(short_conv_kernel<DT, 3, true>, grid, dim3(128), 0, stream, p);                        \
+    case 4: return launch_pdl(short_conv_kernel<DT, 4, true>, grid, dim3(128), 0, stream, p);                        \
+    default: return launch_pdl(short_conv_kernel<DT, kConvMaxW, false>, grid, dim3(128), 0, stream, p);              \
   }
   if (dt == DR_BF16) { DR_CONV_CASE(DR_BF16) } else { DR_CONV_CASE(DR_F32) }
 #undef DR_CONV_CASE
@@ -192,6 +193,7 @@ struct GateParams {
 };
 
 __global__ void __launch_bounds__(256) gate_act_kernel(const GateParams p) {
+  pdl_entry();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < p.n_g) {
     const int hk = (int)(i % ((int64_t)p.H * p.K));   // position inside a token: h * K + k
@@ -206,8 +208,7 @@ __global__ void __launch_bounds__(256) gate_act_kernel(const GateParams p) {
 
 inline cudaError_t launch_gate_act(const GateParams& p, cudaStream_t stream) {
   const int64_t n = p.n_g > p.n_beta ? p.n_g : p.n_beta;
-  gate_act_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(gate_act_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, p);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -248,6 +249,7 @@ struct NormParams {
 
 template <int ODT, int GDT, int YDT>
 __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const NormParams p) {
+  pdl_entry();
   constexpr int N = 4;   // every lane owns groups of 4 consecutive columns: 8- or 16-byte accesses
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // (b, t, h) flattened
@@ -318,6 +320,7 @@ constexpr int kNormRowsPerWarp = 4;
 
 template <int ODT, int GDT, int YDT>
 __global__ void __launch_bounds__(256) gated_rmsnorm_v128_kernel(const NormParams p) {
+  pdl_entry();
   constexpr int V = 128, P = kNormRowsPerWarp / 2;
   const int lane = threadIdx.x & 31, sub = lane >> 4, c = (lane & 15) * 8;
   const int64_t nrows = (int64_t)p.map.B * p.map.T * p.map.H;
@@ -381,9 +384,8 @@ inline cudaError_t launch_gated_rmsnorm(const NormParams& p, int odt, int gdt, i
   const unsigned grid128 = (unsigned)(want128 < (int64_t)sms * 8 ? want128 : (int64_t)sms * 8);
 #define DR_NORM_CASE(O, G, Y)                                                              \
   if (odt == O && gdt == G && ydt == Y) {                                                  \
-    if (p.V == 128) gated_rmsnorm_v128_kernel<O, G, Y><<<grid128, 256, 0, stream>>>(p);    \
-    else gated_rmsnorm_kernel<O, G, Y><<<grid, 256, 0, stream>>>(p);                       \
-    return cudaGetLastError();                                                             \
+    if (p.V == 128) return launch_pdl(gated_rmsnorm_v128_kernel<O, G, Y>, dim3(grid128), dim3(256), 0, stream, p);    \
+    return launch_pdl(gated_rmsnorm_kernel<O, G, Y>, dim3(grid), dim3(256), 0, stream, p);                       \
   }
   DR_NORM_CASE(DR_BF16, DR_BF16, DR_BF16)
   DR_NORM_CASE(DR_F32, DR_F32, DR_F32)

@@ -90,6 +90,7 @@ static_assert(2 * 64 * LDH * 2 >= 64 * 132 * 4 && 2 * (pre_smem<true>() + 1024) 
 
 template <bool KDA>
 __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
+  pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + PR_K);
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + PR_Q);
@@ -362,6 +363,7 @@ constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved,
 
 template <bool X3>
 __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
+  pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
   float* sS = reinterpret_cast<float*>(smem);          // [2][64 * LDP]
   float* sO = sS + 2 * 64 * LDP;                        // [2][32 * LDP]
@@ -498,6 +500,7 @@ template <bool KDA>
 __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   using L = LoSmem<KDA>;
   constexpr bool X3 = KDA;
+  pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
   auto F = [&](int off) { return reinterpret_cast<float*>(smem + off); };
   float *sK = F(L::kK), *sKd = F(L::kKd), *sA = F(L::kA), *sT = F(L::kT);
@@ -1202,8 +1205,7 @@ template <bool KDA>
 inline cudaError_t launch_pre_t(const Params& p, int64_t units, cudaStream_t stream) {
   const cudaError_t e = set_attributes<KDA>();
   if (e != cudaSuccess) return e;
-  pre_kernel<KDA><<<(unsigned)(units * p.N), kPreThreads, pre_smem<KDA>(), stream>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(pre_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kPreThreads), pre_smem<KDA>(), stream, p);
 }
 inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, const void* g, const float* beta, void* workspace,
                               cudaStream_t stream, int* launches) {
@@ -1217,11 +1219,9 @@ template <bool KDA>
 inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, cudaStream_t stream) {
   cudaError_t e = set_attributes<KDA>();
   if (e != cudaSuccess) return e;
-  state_kernel<KDA><<<(unsigned)(units * 4), kStThreads, kStSmem, stream>>>(p);
-  e = cudaGetLastError();
+  e = launch_pdl(state_kernel<KDA>, dim3((unsigned)(units * 4)), dim3(kStThreads), kStSmem, stream, p);
   if (e != cudaSuccess) return e;
-  local_kernel<KDA><<<(unsigned)(units * p.N), kLoThreads, LoSmem<KDA>::kTotal, stream>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(local_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kLoThreads), LoSmem<KDA>::kTotal, stream, p);
 }
 
 }  // namespace bwdc

@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
+  pdl_entry();
   const uint32_t tbase = ctl.tmem_base;
   const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
 
@@ -749,8 +750,7 @@ inline cudaError_t launch_chunk_kernel(Params& P, const FwdParams& p, int64_t un
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
-  kern<<<dim3((unsigned)units), dim3(kThreads), SM_TOTAL, stream>>>(P);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)units), dim3(kThreads), SM_TOTAL, stream, P);
 }
 
 inline cudaError_t launch_chunk(const FwdParams& p, cudaStream_t stream) {

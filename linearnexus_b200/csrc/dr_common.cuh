@@ -5,9 +5,35 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "deltarule_sm100.h"
 
 namespace dr {
+
+// Programmatic dependent launch.  A kernel of a layer's token step runs 2-4 us, of which the start (launch, first instruction,
+// first miss) is most: launch_pdl lets the grid start while its predecessor in the stream still runs, and every kernel launched
+// so calls pdl_entry() before it touches global memory: it waits there until the predecessor has completed and its writes are
+// visible, and lets its own successor start early in turn.  Nothing is read or written before the wait, so the order of effects
+// on the stream is what it was.
+__device__ __forceinline__ void pdl_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 // Addressing of one (batch, head) sequence inside a [B,H,T,D] or [B,T,H,D] tensor.
 // Element index of token t, feature d is  base(b,h,D) + t * tok(D) + d.

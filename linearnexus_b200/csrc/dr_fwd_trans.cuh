@@ -132,6 +132,7 @@ __device__ __forceinline__ void inverse_64(float* sT, const float* rs, int tid) 
 
 template <int D, bool KDA, bool X3>
 __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_kernel(const __grid_constant__ Params P) {
+  pdl_entry();
   using Z_ = Sizes<D>;
   constexpr int NTHR = Z_::NTHR, NW = Z_::NW, CT = Z_::CT, LD = Z_::LD;
   const FwdParams& p = P.p;
@@ -423,6 +424,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
 // Warps 0 .. D/16 - 1: state rows 16 w ..; four more warps: output rows 16 (w - D/16) ...  NT: 8-column tiles per CTA.
 template <int D, bool X3, int NT>
 __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const __grid_constant__ Params P) {
+  pdl_entry();
   constexpr int CT = D / 16, VS = 8 * NT, LDP = 2 * VS + 8;   // S in shared memory: row pairs interleaved [D / 2][VS][2]
   const FwdParams& p = P.p;
   __shared__ __align__(16) float sS[2][D / 2 * LDP];
@@ -553,15 +555,12 @@ inline cudaError_t launch_t(const FwdParams& p, void* workspace, int sms, cudaSt
   P.yf = reinterpret_cast<float4*>(f); f += nc * Z::fY;
   P.of = reinterpret_cast<float4*>(f); f += nc * Z::fO;
   P.el = f;
-  trans_pre_kernel<D, KDA, X3><<<(unsigned)nc, Z::NTHR, Z::smem(KDA), stream>>>(P);
-  e = cudaGetLastError();
+  e = launch_pdl(trans_pre_kernel<D, KDA, X3>, dim3((unsigned)nc), dim3(Z::NTHR), Z::smem(KDA), stream, P);
   if (e != cudaSuccess) return e;
   // narrow slices while they fit one wave: the chain's length is what counts, and every slice adds readers of N and Y
   if (units * (D / 16) <= sms)
-    trans_state_kernel<D, X3, 2><<<(unsigned)(units * (D / 16)), (D / 16 + 4) * 32, 0, stream>>>(P);
-  else
-    trans_state_kernel<D, X3, 4><<<(unsigned)(units * (D / 32)), (D / 16 + 4) * 32, 0, stream>>>(P);
-  return cudaGetLastError();
+    return launch_pdl(trans_state_kernel<D, X3, 2>, dim3((unsigned)(units * (D / 16))), dim3((D / 16 + 4) * 32), 0, stream, P);
+  return launch_pdl(trans_state_kernel<D, X3, 4>, dim3((unsigned)(units * (D / 32))), dim3((D / 16 + 4) * 32), 0, stream, P);
 }
 
 template <int D, bool X3>

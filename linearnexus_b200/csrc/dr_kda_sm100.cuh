@@ -143,6 +143,7 @@ template <class Params>
 __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constant__ Params P) {
   constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value, kTrans = std::is_same<Params, IntraTransParams>::value;
   const FwdParams& p = P.p;
+  pdl_entry();
   extern __shared__ __align__(1024) uint8_t smem[];
   float* sG = reinterpret_cast<float*>(smem + IN_G);
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + IN_K);
@@ -733,6 +734,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
+  pdl_entry();
   const uint32_t tbase = ctl.tmem_base;
   const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
   auto wait_bar = [&](uint64_t* bar, uint32_t parity) {
@@ -975,6 +977,7 @@ constexpr int kTrThreads = 12 * 32;
 
 template <int NT>
 __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid_constant__ IntraTransParams P) {
+  pdl_entry();
   constexpr int VS = 8 * NT, LDS = VS + 8, SL = kD / VS;
   const FwdParams& p = P.p;
   __shared__ __align__(16) __nv_bfloat16 sS[2][kD * LDS];
@@ -1095,13 +1098,11 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;
   P.of = reinterpret_cast<float4*>(w); w += nc * kTrO;
   P.el = reinterpret_cast<float*>(w);
-  intra_kernel<IntraTransParams><<<(unsigned)nc, kThreads, IN_TOTAL, stream>>>(P);
-  e = cudaGetLastError();
+  e = launch_pdl(intra_kernel<IntraTransParams>, dim3((unsigned)nc), dim3(kThreads), IN_TOTAL, stream, P);
   if (e != cudaSuccess) return e;
   // 16 columns per CTA while the slices fit one wave: the chain's length is what counts
-  if (units * 8 <= sms) trans_state_kernel<2><<<(unsigned)(units * 8), kTrThreads, 0, stream>>>(P);
-  else trans_state_kernel<4><<<(unsigned)(units * 4), kTrThreads, 0, stream>>>(P);
-  return cudaGetLastError();
+  if (units * 8 <= sms) return launch_pdl(trans_state_kernel<2>, dim3((unsigned)(units * 8)), dim3(kTrThreads), 0, stream, P);
+  return launch_pdl(trans_state_kernel<4>, dim3((unsigned)(units * 4)), dim3(kTrThreads), 0, stream, P);
 }
 
 template <class IP, class SP>
@@ -1121,12 +1122,10 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   S.p = p;
   S.ws = I.ws = reinterpret_cast<uint8_t*>(workspace);
   if (!sm100::make_panel_map(&S.tv, p.v, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
-  intra_kernel<IP><<<(unsigned)chunk_units, kThreads, IN_TOTAL, stream>>>(I);
-  e = cudaGetLastError();
+  e = launch_pdl(intra_kernel<IP>, dim3((unsigned)chunk_units), dim3(kThreads), IN_TOTAL, stream, I);
   if (e != cudaSuccess) return e;
   S.use_tma_out = p.o != nullptr && sm100::make_output_map(&S.to, p.o, p.map, p.out_dt == DR_BF16 ? 2 : 4);
-  state_kernel<SP><<<(unsigned)units, kStateThreads, ST_TOTAL, stream>>>(S);
-  return cudaGetLastError();
+  return launch_pdl(state_kernel<SP>, dim3((unsigned)units), dim3(kStateThreads), ST_TOTAL, stream, S);
 }
 
 inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches) {

@@ -65,6 +65,7 @@ constexpr int kBarFull = 1, kBarEmpty = 1 + kStages, kBarGroup = 1 + 2 * kStages
 
 template <int KIND, bool BF>
 __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecParams p) {
+  pdl_entry();
   using R = Ring<KIND, BF>;
   constexpr bool LR = KIND == LR_DPLR;
   constexpr int NV = R::NV;
@@ -384,8 +385,7 @@ inline cudaError_t launch_t(const LinRecParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
-  kern<<<(unsigned)((int64_t)p.B * p.H * (p.V / 64)), kThreads, bytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)((int64_t)p.B * p.H * (p.V / 64))), dim3(kThreads), bytes, stream, p);
 }
 inline cudaError_t launch(int kind, bool bf, const LinRecParams& p, cudaStream_t stream) {
   if (kind == LR_DPLR) return bf ? launch_t<LR_DPLR, true>(p, stream) : launch_t<LR_DPLR, false>(p, stream);

@@ -49,6 +49,7 @@ struct Smem {
 
 template <int N>
 __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecParams p, const int nseg) {
+  pdl_entry();
   using L = Smem<N>;
   constexpr int LDN = L::LDN, NT = N / 16, KS = N / 32;   // state tiles (8 columns) per warp, 16-column k-steps per warp
   extern __shared__ __align__(16) uint8_t smem[];
@@ -400,12 +401,14 @@ inline cudaError_t launch_n(const LinRecParams& p, int sms, cudaStream_t stream)
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = Smem<N>::kTotal;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = nseg;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see pdl_entry
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, p, nseg);
 }
 

@@ -38,6 +38,7 @@ constexpr int kStepThreads = 256;
 
 template <int ROWS>
 __global__ void __launch_bounds__(kStepThreads) step_kernel(const StepParams p) {
+  pdl_entry();
   extern __shared__ float smem[];
   const int K = p.K, V = p.V;
   float* s_q = smem;            // [K] normalised, scaled
@@ -204,12 +205,11 @@ inline cudaError_t launch_step(const StepParams& p, int64_t units, cudaStream_t 
   const size_t smem = step_smem_bytes(p.K, p.V);
   const dim3 grid((unsigned)units), block(kStepThreads);
   switch (step_rows(p.K, p.V)) {
-    case 4: step_kernel<4><<<grid, block, smem, stream>>>(p); break;
-    case 16: step_kernel<16><<<grid, block, smem, stream>>>(p); break;
-    case 32: step_kernel<32><<<grid, block, smem, stream>>>(p); break;
-    default: step_kernel<0><<<grid, block, smem, stream>>>(p); break;
+    case 4: return launch_pdl(step_kernel<4>, grid, block, smem, stream, p);
+    case 16: return launch_pdl(step_kernel<16>, grid, block, smem, stream, p);
+    case 32: return launch_pdl(step_kernel<32>, grid, block, smem, stream, p);
+    default: return launch_pdl(step_kernel<0>, grid, block, smem, stream, p);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace dr

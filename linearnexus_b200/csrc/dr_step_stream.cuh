@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_stream_kernel(const Step
   const int tid = threadIdx.x;
   const int vg = tid & 31, ks = tid >> 5;   // float4 column group, row group (rows ks, ks + 8, ...)
   const int64_t first = blockIdx.x, stride = gridDim.x;
-  if (first >= units) return;
+  if (first >= units) { pdl_entry(); return; }
   const int64_t nmine = (units - first + stride - 1) / stride;
 
   if (tid == 0) {
@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_stream_kernel(const Step
     s_abort = 0;
   }
   __syncthreads();
+  pdl_entry();
   auto issue_load = [&](int64_t i) {   // thread 0
     const uint32_t bar = tc::smem_u32(&full[i % kStreamStages]);
     tc::mbar_arrive_expect_tx(bar, kStreamStateBytes);
@@ -175,10 +176,16 @@ inline bool step_stream_eligible(const StepParams& p, int64_t units, int sms) {
 
 inline cudaError_t launch_step_stream(const StepParams& p, int64_t units, int sms, int32_t* status,
                                       cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(step_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+  thread_local int attr_dev = -1;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  step_stream_kernel<<<(unsigned)sms, kStepThreads, kStreamSmem, stream>>>(p, units, status);
-  return cudaGetLastError();
+  if (attr_dev != dev) {
+    e = cudaFuncSetAttribute(step_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+    if (e != cudaSuccess) return e;
+    attr_dev = dev;
+  }
+  return launch_pdl(step_stream_kernel, dim3((unsigned)sms), dim3(kStepThreads), kStreamSmem, stream, p, units, status);
 }
 
 }  // namespace dr
