@@ -216,20 +216,31 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
       *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kraw[i];
       *reinterpret_cast<float4*>(sG + c * LDF + 4 * lane) =
           make_float4(gv[i][0] * kLog2e, gv[i][1] * kLog2e, gv[i][2] * kLog2e, gv[i][3] * kLog2e);
-      float qmul = p.scale, kmul = 1.f;
-      if (p.l2norm) {
-        const float2 q0 = bf2(qraw[i].x), q1 = bf2(qraw[i].y), k0 = bf2(kraw[i].x), k1 = bf2(kraw[i].y);
-        const float nq = warp_sum(q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y);
-        const float nk = warp_sum(k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y);
-        qmul = p.scale / (sqrtf(nq) + 1e-6f);
-        kmul = 1.f / (sqrtf(nk) + 1e-6f);
-      }
-      if (lane == i) {
-        sBeta[c] = bt;
-        sRk[c] = kmul;
-        sRq[c] = qmul;
+    }
+    // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced (16 shuffles instead of
+    // 80), so that each lane takes one square root and one quotient (as every lane did for every row, a fifth of the pass)
+    float ss[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 q0 = bf2(qraw[i].x), q1 = bf2(qraw[i].y), k0 = bf2(kraw[i].x), k1 = bf2(kraw[i].y);
+      ss[i] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
+      ss[8 + i] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
+    }
+#pragma unroll
+    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        const bool up = lane & o;
+        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
+        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
+      const float top = lane < 16 ? p.scale : 1.f;
+      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+    }
+    if (lane < 8) sBeta[warp + 8 * lane] = bt;
   }
   __syncthreads();
   // ---- G = inclusive prefix sum of the log decay over the rows of the chunk, per channel ---------------------
@@ -557,13 +568,14 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   for (int it = 0; it < 2; ++it) {
     const int piece = tid + kThreads * it;
     int row, col;
-    piece64(piece, row, col);
-    float a[8];
+    piece64(piece, row, col);   // eight rows to a quarter warp: the 16-byte reads are free of bank conflicts
+    float a[8], bt[8];
+    *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sT + row * LDT + col);
+    *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sT + row * LDT + col + 4);
+    *reinterpret_cast<float4*>(bt) = *reinterpret_cast<const float4*>(sBeta + col);
+    *reinterpret_cast<float4*>(bt + 4) = *reinterpret_cast<const float4*>(sBeta + col + 4);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int j = col + e;
-      a[e] = j <= row ? sT[row * LDT + j] * sBeta[j] : 0.f;
-    }
+    for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? a[e] * bt[e] : 0.f;
     *reinterpret_cast<uint4*>(rec + WS_TB + piece * 16) = pack8(a);
     uint4 q = *reinterpret_cast<const uint4*>(sAqk + row * LDQ + col);
     uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
@@ -586,10 +598,14 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
     const uint32_t* wk = reinterpret_cast<const uint32_t*>(&uk);
     const float rq = sRq[row], rk = sRk[row];
     float a[8], c[8], kg[8];
+    float4 g4[2], l4[2];
+    g4[0] = *reinterpret_cast<const float4*>(sG + row * LDF + col);
+    g4[1] = *reinterpret_cast<const float4*>(sG + row * LDF + col + 4);
+    l4[0] = *reinterpret_cast<const float4*>(sG + 63 * LDF + col);
+    l4[1] = *reinterpret_cast<const float4*>(sG + 63 * LDF + col + 4);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float2 gg = *reinterpret_cast<const float2*>(sG + row * LDF + col + 2 * e);
-      const float2 gl = *reinterpret_cast<const float2*>(sG + 63 * LDF + col + 2 * e);
+      const float2 gg = reinterpret_cast<const float2*>(g4)[e], gl = reinterpret_cast<const float2*>(l4)[e];
       const float2 qq = bf2(wq[e]), kk = bf2(wk[e]);
       const float e0 = ex2(gg.x), e1 = ex2(gg.y);
       a[2 * e] = qq.x * rq * e0;
@@ -605,29 +621,37 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   }
   if (tid < kD) reinterpret_cast<float*>(rec + WS_EGL)[tid] = ex2(sG[63 * LDF + tid]);
   __syncthreads();
-  // ---- W = (T diag(beta)) (k^ e^G): 64x128x64 on mma.sync (tf32); warp = 16 rows x 64 channels ----------------------
-  // (A_kk is dead after the inverse: its array takes the bf16 staging tile of W; bf16 -> tf32 is exact)
+  // ---- W = (T diag(beta)) (k^ e^G): 64x128x64 on mma.sync (bf16); warp = 16 rows x 64 channels ----------------------
+  // T diag(beta) is fp32 in shared memory: two bf16 terms (16 bits, tf32 has 11), against the bf16 tile by ldmatrix; with tf32
+  // products the tile was read two bytes at a time.  Within eight tokens the contraction runs over (0 4 1 5 2 6 3 7), for which
+  // the reads of T are free of bank conflicts.
+  // (A_kk is dead after the inverse: its array takes the bf16 staging tile of W)
   {
     const int m0 = (warp >> 1) * 16, nb = (warp & 1) * 64;
     float d[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) { d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f; }
     const int r0 = m0 + g, r1 = r0 + 8;
-    for (int ks = 0; ks * 8 <= m0 + 15; ++ks) {
-      const int k0 = ks * 8 + t, k1 = k0 + 4;
-      const float s0 = sBeta[k0], s1 = sBeta[k1];
-      uint32_t a[4];
-      a[0] = sm100::to_tf32(k0 <= r0 ? sT[r0 * LDT + k0] * s0 : 0.f);
-      a[1] = sm100::to_tf32(k0 <= r1 ? sT[r1 * LDT + k0] * s0 : 0.f);
-      a[2] = sm100::to_tf32(k1 <= r0 ? sT[r0 * LDT + k1] * s1 : 0.f);
-      a[3] = sm100::to_tf32(k1 <= r1 ? sT[r1 * LDT + k1] * s1 : 0.f);
+    const uint32_t aB = tc::smem_u32(sQ) + 2u * (((lane & 8) + ((lane & 7) >> 1) + (lane & 1) * 4) * LDH + nb + (lane >> 4) * 8);
+    for (int kb = 0; kb <= m0; kb += 16) {
+      uint32_t hi[4], lo[4];
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        const int ch = nb + nt * 8 + g;
-        uint32_t bb[2];
-        bb[0] = (uint32_t)reinterpret_cast<const uint16_t*>(sQ)[k0 * LDH + ch] << 16;
-        bb[1] = (uint32_t)reinterpret_cast<const uint16_t*>(sQ)[k1 * LDH + ch] << 16;
-        sm100::mma_tf32(d[nt], a, bb);
+      for (int e = 0; e < 4; ++e) {   // e & 1: row half, e >> 1: k half
+        const int r = (e & 1) ? r1 : r0, k0 = kb + 8 * (e >> 1) + t, k1 = k0 + 4;
+        const float x = k0 <= r ? sT[r * LDT + k0] * sBeta[k0] : 0.f;
+        const float y = k1 <= r ? sT[r * LDT + k1] * sBeta[k1] : 0.f;
+        hi[e] = tc::pack_bf16(x, y);
+        const float2 h = bf2(hi[e]);
+        lo[e] = tc::pack_bf16(x - h.x, y - h.y);
+      }
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) {
+        uint32_t bb[4];
+        mma::ldsm4t(bb, aB + 2u * (kb * LDH + 16 * n2));
+        mma::bf16(d[2 * n2], hi, bb[0], bb[1]);
+        mma::bf16(d[2 * n2 + 1], hi, bb[2], bb[3]);
+        mma::bf16(d[2 * n2], lo, bb[0], bb[1]);
+        mma::bf16(d[2 * n2 + 1], lo, bb[2], bb[3]);
       }
     }
 #pragma unroll
