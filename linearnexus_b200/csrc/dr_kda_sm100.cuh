@@ -57,7 +57,7 @@ inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC -
 // (global loads, the serial prefix sum, the barriers between phases) hides behind the other's work.  The
 // inputs stay as raw bf16 with their l2-norm factors on the side, and the decayed bf16 operands of the
 // tensor-core products are formed in registers from them (no scaled copies in shared memory).
-constexpr int LDF = 132;   // row stride (floats) of G
+constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
 constexpr int IN_G = 0;                          // log2(e) G   fp32 [64][132]
@@ -92,6 +92,24 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+
+// packed pairs: one instruction per two products
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %2, %3, %1;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(0xbf800000bf800000ull));
+  return d;
+}
+__device__ __forceinline__ float2 ex2x2(float2 a) { return make_float2(ex2(a.x), ex2(a.y)); }
 
 // four consecutive elements starting at element index i (a multiple of 4)
 __device__ __forceinline__ void ld4(const void* p, int64_t i, int dt, float (&x)[4]) {
@@ -138,6 +156,24 @@ struct IntraTransParams : IntraParams {
   float4 *zf, *of;    // [chunks][8 | 4 row tiles][16 column tiles][32 lanes]: addends
   float* el;          // [chunks][128] e^{G_L}
 };
+
+// eight channels of one row: scale q^ e^G, k^ e^{G_L - G}, k^ e^G (G of the row and of the chunk's last row in log2 units)
+__device__ __forceinline__ void decayed_piece(const float* gr, const float* gl, uint4 q, uint4 k, float rq, float rk,
+                                              uint4& qg, uint4& kd, uint4& kg) {
+  float4 g4[2], l4[2];
+  g4[0] = *reinterpret_cast<const float4*>(gr); g4[1] = *reinterpret_cast<const float4*>(gr + 4);
+  l4[0] = *reinterpret_cast<const float4*>(gl); l4[1] = *reinterpret_cast<const float4*>(gl + 4);
+  const float2 q2 = make_float2(rq, rq), k2 = make_float2(rk, rk);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 gg = reinterpret_cast<const float2*>(g4)[e], ll = reinterpret_cast<const float2*>(l4)[e];
+    const float2 eg = ex2x2(gg), kk = mul2(bf2(reinterpret_cast<const uint32_t*>(&k)[e]), k2);
+    const float2 x = mul2(mul2(bf2(reinterpret_cast<const uint32_t*>(&q)[e]), q2), eg), y = mul2(kk, ex2x2(sub2(ll, gg))), z = mul2(kk, eg);
+    reinterpret_cast<uint32_t*>(&qg)[e] = tc::pack_bf16(x.x, x.y);
+    reinterpret_cast<uint32_t*>(&kd)[e] = tc::pack_bf16(y.x, y.y);
+    reinterpret_cast<uint32_t*>(&kg)[e] = tc::pack_bf16(z.x, z.y);
+  }
+}
 
 template <class Params>
 __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constant__ Params P) {
@@ -190,22 +226,37 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   {
     uint2 qraw[8], kraw[8];
     float gv[8][4];
+    {
+      const int64_t at = qk_base + (t0 + warp) * qk_tok + 4 * lane;
+      const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(p.q) + at;
+      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(p.k) + at;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = warp + 8 * i;
-      qraw[i] = make_uint2(0u, 0u); kraw[i] = make_uint2(0u, 0u);
-      gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = 0.f;
-      if (c < rows) {
-        const int64_t at = qk_base + (t0 + c) * qk_tok + 4 * lane;
-        qraw[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + at);
-        kraw[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at);
-        if (p.variant == DR_KDA) {
-          ld4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt, gv[i]);
-        } else if (p.variant == DR_GATED) {
-          const float gs = ld_elem(p.g, s_base + (t0 + c) * s_tok, p.g_dt);
-          gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = gs;
+      for (int i = 0; i < 8; ++i) {
+        qraw[i] = make_uint2(0u, 0u); kraw[i] = make_uint2(0u, 0u);
+        if (warp + 8 * i < rows) {
+          qraw[i] = *reinterpret_cast<const uint2*>(qp);
+          kraw[i] = *reinterpret_cast<const uint2*>(kp);
         }
+        qp += 8 * qk_tok; kp += 8 * qk_tok;
       }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = 0.f;
+    if (p.variant == DR_KDA) {   // one loop per storage type: no branch between the loads
+      int64_t at = gk_base + (t0 + warp) * gk_tok + 4 * lane;
+      if (p.g_dt == DR_BF16) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
+          if (warp + 8 * i < rows) ld4(p.g, at, DR_BF16, gv[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
+          if (warp + 8 * i < rows) ld4(p.g, at, DR_F32, gv[i]);
+      }
+    } else if (p.variant == DR_GATED) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (warp + 8 * i < rows) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = ld_elem(p.g, s_base + (t0 + warp + 8 * i) * s_tok, p.g_dt);
     }
     float bt = 0.f;
     if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
@@ -459,19 +510,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
     for (int it = 0; it < 4; ++it) {
       const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
       const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col), uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
-      const uint32_t wq[4] = {uq.x, uq.y, uq.z, uq.w}, wk[4] = {uk.x, uk.y, uk.z, uk.w};
-      const float rq = sRq[row], rk = sRk[row];
-      float a[8], c[8], d[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 gg = *reinterpret_cast<const float2*>(sG + row * LDF + col + 2 * e), gl = *reinterpret_cast<const float2*>(sG + 63 * LDF + col + 2 * e);
-        const float2 qq = bf2(wq[e]), kk = bf2(wk[e]);
-        const float e0 = ex2(gg.x), e1 = ex2(gg.y);
-        a[2 * e] = qq.x * rq * e0; a[2 * e + 1] = qq.y * rq * e1;
-        c[2 * e] = kk.x * rk * ex2(gl.x - gg.x); c[2 * e + 1] = kk.y * rk * ex2(gl.y - gg.y);
-        d[2 * e] = kk.x * rk * e0; d[2 * e + 1] = kk.y * rk * e1;
-      }
-      qg[it] = pack8(a); kd[it] = pack8(c); kg[it] = pack8(d);
+      decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], qg[it], kd[it], kg[it]);
     }
     const int64_t chunk = blockIdx.x;
     if (tid < kD) P.el[chunk * kD + tid] = ex2(sG[63 * LDF + tid]);
@@ -594,30 +633,11 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
     piece128(piece, row, col);
     const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col);
     const uint4 uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
-    const uint32_t* wq = reinterpret_cast<const uint32_t*>(&uq);
-    const uint32_t* wk = reinterpret_cast<const uint32_t*>(&uk);
-    const float rq = sRq[row], rk = sRk[row];
-    float a[8], c[8], kg[8];
-    float4 g4[2], l4[2];
-    g4[0] = *reinterpret_cast<const float4*>(sG + row * LDF + col);
-    g4[1] = *reinterpret_cast<const float4*>(sG + row * LDF + col + 4);
-    l4[0] = *reinterpret_cast<const float4*>(sG + 63 * LDF + col);
-    l4[1] = *reinterpret_cast<const float4*>(sG + 63 * LDF + col + 4);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 gg = reinterpret_cast<const float2*>(g4)[e], gl = reinterpret_cast<const float2*>(l4)[e];
-      const float2 qq = bf2(wq[e]), kk = bf2(wk[e]);
-      const float e0 = ex2(gg.x), e1 = ex2(gg.y);
-      a[2 * e] = qq.x * rq * e0;
-      a[2 * e + 1] = qq.y * rq * e1;
-      c[2 * e] = kk.x * rk * ex2(gl.x - gg.x);
-      c[2 * e + 1] = kk.y * rk * ex2(gl.y - gg.y);
-      kg[2 * e] = kk.x * rk * e0;
-      kg[2 * e + 1] = kk.y * rk * e1;
-    }
-    *reinterpret_cast<uint4*>(rec + WS_QG + piece * 16) = pack8(a);
-    *reinterpret_cast<uint4*>(rec + WS_KD + piece * 16) = pack8(c);
-    *reinterpret_cast<uint4*>(sQ + row * LDH + col) = pack8(kg);   // k^ e^G for the W product (q is dead)
+    uint4 a, c, kg;
+    decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], a, c, kg);
+    *reinterpret_cast<uint4*>(rec + WS_QG + piece * 16) = a;
+    *reinterpret_cast<uint4*>(rec + WS_KD + piece * 16) = c;
+    *reinterpret_cast<uint4*>(sQ + row * LDH + col) = kg;   // k^ e^G for the W product (q is dead)
   }
   if (tid < kD) reinterpret_cast<float*>(rec + WS_EGL)[tid] = ex2(sG[63 * LDF + tid]);
   __syncthreads();
