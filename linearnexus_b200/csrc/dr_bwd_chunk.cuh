@@ -492,8 +492,9 @@ struct LoSmem {
   static constexpr int gQS = 0, gKS = 64 * 132 * 4, gKE = 2 * gKS, gG = 3 * gKS, gA = 4 * gKS, gX = gA + 64 * LDA * 4, gD = gX + 64 * LDA * 4;
   static constexpr int gSeg = gD + 4 * 128 * 4;   // [16][128] scan scratch
   static constexpr int kDot = KDA ? gSeg + 16 * 128 * 4 : kV + 64 * 136 * 4;   // final phase: q^ . dq^, k^ . dk^ per row, [2][4][64]
+  static constexpr int gRaw = kDot + 2048;   // KDA: raw q and k rows, bf16 [2][64][136]
   static_assert(64 * LDA * 4 <= 4 * kSl && 64 * 136 * 4 <= 4 * kS1 && kTotal <= 232448 &&
-                (KDA ? kDot + 2048 <= kSc : kDot + 2048 <= kSD && 2 * 64 * 136 * 2 <= 64 * 136 * 4), "shared memory");
+                (KDA ? gRaw + 2 * 64 * LDH * 2 <= kSc : kDot + 2048 <= kSD && 2 * 64 * 136 * 2 <= 64 * 136 * 4), "shared memory");
 };
 
 template <bool KDA>
@@ -627,7 +628,53 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     if (s + 1 < kD / kVS) { issue_slice(s + 1); vr = load_v(s + 1); }
     // ---- R = beta V - beta (K^ e^G) S0,  dVn = A^T dO + Kd dS1 (eight columns per warp) ------------------------------------------
     const int n0 = 8 * wc;
-    {
+    if constexpr (KDA) {
+      // different left operands, each split into two terms: half of the warps take R, half dVn, sixteen columns each, so that
+      // a split serves two products (with both on every warp the splits were more than half of the instructions here)
+      const bool second = warp >= 8;
+      const int mr = 16 * ((warp & 7) >> 1), nc = 16 * (warp & 1);
+      const float *left = second ? sKd : sK, *right = second ? sdS : sS0;
+      float d[2][4];
+      zero4(d[0]); zero4(d[1]);
+#pragma unroll 4
+      for (int k0 = 0; k0 < kD; k0 += 8) {
+        const int k = k0 + t;
+        AFrag<true> a;
+        a.set(left[(mr + g) * 132 + k], left[(mr + g + 8) * 132 + k], left[(mr + g) * 132 + k + 4], left[(mr + g + 8) * 132 + k + 4]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          BFrag<true> bs;
+          bs.set(right[k * LDV + nc + 8 * nt + g], right[(k + 4) * LDV + nc + 8 * nt + g]);
+          fma<true>(d[nt], a, bs);
+        }
+      }
+      if (second) {
+        for (int k0 = mr; k0 < kC; k0 += 8) {
+          const int k = k0 + t;
+          AFrag<true> a;
+          a.set(sA[k * LDA + mr + g], sA[k * LDA + mr + g + 8], sA[(k + 4) * LDA + mr + g], sA[(k + 4) * LDA + mr + g + 8]);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            BFrag<false> bo;   // bf16 values: one term
+            bo.set(sdO[k * LDV + nc + 8 * nt + g], sdO[(k + 4) * LDV + nc + 8 * nt + g]);
+            mma::fma_b1(d[nt], a, bo);
+          }
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+          const int c = mr + g + 8 * hr, at = c * LDV + nc + 8 * nt + 2 * t;
+          if (second) {
+            *reinterpret_cast<float2*>(sdR + at) = make_float2(d[nt][2 * hr], d[nt][2 * hr + 1]);
+          } else {
+            const float2 x = ld2(sV + at);
+            const float bt = sBeta[c];
+            *reinterpret_cast<float2*>(sVn + at) = make_float2(bt * (x.x - d[nt][2 * hr]), bt * (x.y - d[nt][2 * hr + 1]));
+          }
+        }
+    } else {
       float r0[4], r1[4], d0[4], d1[4];
       zero4(r0); zero4(r1); zero4(d0); zero4(d1);
 #pragma unroll 4
@@ -641,12 +688,11 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
           bs.set(sS0[k * LDV + n0 + g], sS0[(k + 4) * LDV + n0 + g]);
           bd.set(sdS[k * LDV + n0 + g], sdS[(k + 4) * LDV + n0 + g]);
           fma<X3>(hf ? r1 : r0, a, bs);
-          if constexpr (KDA) a.set(sKd[(m0 + g) * 132 + k], sKd[(m0 + g + 8) * 132 + k], sKd[(m0 + g) * 132 + k + 4], sKd[(m0 + g + 8) * 132 + k + 4]);
           fma<X3>(hf ? d1 : d0, a, bd);
         }
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { r0[e] += r1[e]; d0[e] += d1[e]; if (!KDA) d0[e] *= sWd[m0 + g + 8 * (e >> 1)]; }
+      for (int e = 0; e < 4; ++e) { r0[e] += r1[e]; d0[e] += d1[e]; d0[e] *= sWd[m0 + g + 8 * (e >> 1)]; }
       for (int k0 = m0; k0 < kC; k0 += 8) {
         const int k = k0 + t;
         AFrag<X3> a;
@@ -659,7 +705,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       for (int hr = 0; hr < 2; ++hr) {
         const int c = m0 + g + 8 * hr, vv = n0 + 2 * t;
         const float2 x = ld2(sV + c * LDV + vv);
-        const float bt = sBeta[c], eg = KDA ? 1.f : sEG[c];
+        const float bt = sBeta[c], eg = sEG[c];
         *reinterpret_cast<float2*>(sVn + c * LDV + vv) = make_float2(bt * (x.x - eg * r0[2 * hr]), bt * (x.y - eg * r0[2 * hr + 1]));
         *reinterpret_cast<float2*>(sdR + c * LDV + vv) = make_float2(d0[2 * hr], d0[2 * hr + 1]);
       }
@@ -727,7 +773,8 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
 #pragma unroll
     for (int k0 = 0; k0 < kVS; k0 += 8) {
       const int k = k0 + 2 * t;
-      AFrag<X3> ao, ar, an;
+      AFrag<false> ao;   // bf16 values: one term in either precision
+      AFrag<X3> ar, an;
       {
         const float2 x0 = ld2(sdO + (m0 + g) * LDV + k), x1 = ld2(sdO + (m0 + g + 8) * LDV + k);
         ao.set(x0.x, x1.x, x0.y, x1.y);
@@ -742,7 +789,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
           const float2 y = ld2(sVn + (16 * wc + 8 * nt + g) * LDV + k);
           BFrag<X3> bv;
           bv.set(y.x, y.y);
-          fma<X3>(da[nt], ao, bv);
+          mma::fma_a1(da[nt], ao, bv);
           fma<X3>(dm[nt], ar, bv);
         }
       }
@@ -753,7 +800,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         BFrag<X3> bs, bd;
         bs.set(y.x, y.y);
         bd.set(z.x, z.y);
-        fma<X3>(dQ[nt], ao, bs);
+        mma::fma_a1(dQ[nt], ao, bs);
         fma<X3>(dKr[nt], ar, bs);
         fma<X3>(dKc[nt], an, bd);
       }
@@ -809,6 +856,8 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   }
   // ---- q^ rows (KDA: the decayed forms of q^ and k^) ---------------------------------------------------------------------------------------
   float* sQ = F(L::fQ);   // DeltaNet / Gated: [64][136]
+  __nv_bfloat16* sRaw = reinterpret_cast<__nv_bfloat16*>(smem + (KDA ? L::gRaw : 0));   // KDA
+  float* sDi = F(L::gSeg);   // KDA: 1 / total decay of each block (over the scan scratch)
   float *sQS = F(L::gQS), *sKS = F(L::gKS), *sKE = F(L::gKE), *sG = F(L::gG), *sD = F(L::gD);
   if constexpr (KDA) {
 #pragma unroll
@@ -821,6 +870,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       const int blk = tid >> 7, c = tid & 127;
       const float d = sG[(16 * blk + 15) * 132 + c] - (blk ? sG[(16 * blk - 1) * 132 + c] : 0.f);
       sD[blk * 128 + c] = ex2(d);
+      sDi[blk * 128 + c] = 1.f / ex2(d);
       if (!(d >= -64.f)) sUn[blk] = 1.f;
     }
   }
@@ -832,6 +882,8 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     const float m = p.l2norm ? p.scale / (nrm + 1e-6f) : p.scale;
     if (lane == 0) sRq[c] = m;
     if constexpr (KDA) {
+      *reinterpret_cast<uint2*>(sRaw + c * LDH + 4 * lane) = qr[i];
+      *reinterpret_cast<uint2*>(sRaw + (64 + c) * LDH + 4 * lane) = kr[i];
       const int blk = c >> 4;
       const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
       const float4 ge = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
@@ -906,7 +958,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         for (int nt = 0; nt < 4; ++nt) {
           const int c = 32 * wc + 8 * nt + g;
           float b0 = sKE[k * 132 + c], b1 = sKE[(k + 1) * 132 + c];
-          if (diag) { const float iv = 1.f / sD[bi * 128 + c]; b0 *= iv; b1 *= iv; }
+          if (diag) { const float iv = sDi[bi * 128 + c]; b0 *= iv; b1 *= iv; }
           BFrag<true> bk;
           bk.set(b0, b1);
           fma<true>(dQ[nt], aa, bk);
@@ -949,13 +1001,9 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       for (int hr = 0; hr < 2; ++hr) {
         const int i = m0 + g + 8 * hr;
         const float2 gi = ld2(sG + i * 132 + c);
-        float2 qh = make_float2(0.f, 0.f), kh = qh;
-        if (i < rows) {
-          const int64_t at = qk_base + (t0 + i) * qk_tok + c;
-          const uint32_t uq = *reinterpret_cast<const uint32_t*>(gq + at), uk = *reinterpret_cast<const uint32_t*>(gk + at);
-          qh = make_float2(mma::lo_f(uq) * sRq[i], mma::hi_f(uq) * sRq[i]);
-          kh = make_float2(mma::lo_f(uk) * sRk[i], mma::hi_f(uk) * sRk[i]);
-        }
+        const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
+        const float2 qh = make_float2(mma::lo_f(uq) * sRq[i], mma::hi_f(uq) * sRq[i]);
+        const float2 kh = make_float2(mma::lo_f(uk) * sRk[i], mma::hi_f(uk) * sRk[i]);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int x = 2 * hr + e;
@@ -1100,12 +1148,9 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       } else {
         float2 qh = make_float2(0.f, 0.f), kh = qh;
         if constexpr (KDA) {
-          if (i < rows) {
-            const int64_t at = qk_base + (t0 + i) * qk_tok + c;
-            const uint32_t uq = *reinterpret_cast<const uint32_t*>(gq + at), uk = *reinterpret_cast<const uint32_t*>(gk + at);
-            qh = make_float2(mma::lo_f(uq) * mq, mma::hi_f(uq) * mq);
-            kh = make_float2(mma::lo_f(uk) * mk, mma::hi_f(uk) * mk);
-          }
+          const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
+          qh = make_float2(mma::lo_f(uq) * mq, mma::hi_f(uq) * mq);
+          kh = make_float2(mma::lo_f(uk) * mk, mma::hi_f(uk) * mk);
         } else {
           qh = ld2(sQ + i * 136 + c); kh = ld2(sK + i * 132 + c);
         }

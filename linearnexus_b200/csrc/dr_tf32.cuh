@@ -55,6 +55,17 @@ __device__ __forceinline__ void fma(float (&d)[4], const AFrag<X3>& a, const BFr
   }
   tf32(d, a.h, b.h);
 }
+// products with one operand that is exact in a single term (a bf16 value)
+template <bool X3>
+__device__ __forceinline__ void fma_a1(float (&d)[4], const AFrag<false>& a, const BFrag<X3>& b) {
+  if constexpr (X3) tf32(d, a.h, b.l);
+  tf32(d, a.h, b.h);
+}
+template <bool X3>
+__device__ __forceinline__ void fma_b1(float (&d)[4], const AFrag<X3>& a, const BFrag<false>& b) {
+  if constexpr (X3) tf32(d, a.l, b.h);
+  tf32(d, a.h, b.h);
+}
 
 // In-place inclusive prefix sum over the 64 rows of sG [64][D + 4] per channel; NTHR threads, `seg`: scratch of
 // NTHR / (D / 4) rows of D floats.  Ends with a barrier.
