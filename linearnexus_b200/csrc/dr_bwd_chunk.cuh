@@ -633,14 +633,15 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       // a split serves two products (with both on every warp the splits were more than half of the instructions here)
       const bool second = warp >= 8;
       const int mr = 16 * ((warp & 7) >> 1), nc = 16 * (warp & 1);
-      const float *left = second ? sKd : sK, *right = second ? sdS : sS0;
+      const uint32_t left = mma::lda_at(tc::smem_u32(second ? sKd : sK), 132, mr, lane);
+      const float* right = second ? sdS : sS0;
       float d[2][4];
       zero4(d[0]); zero4(d[1]);
 #pragma unroll 4
       for (int k0 = 0; k0 < kD; k0 += 8) {
         const int k = k0 + t;
         AFrag<true> a;
-        a.set(left[(mr + g) * 132 + k], left[(mr + g + 8) * 132 + k], left[(mr + g) * 132 + k + 4], left[(mr + g + 8) * 132 + k + 4]);
+        mma::lda(a, left + 4u * k0);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           BFrag<true> bs;
@@ -675,6 +676,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
           }
         }
     } else {
+      const uint32_t aK = mma::lda_at(tc::smem_u32(sK), 132, m0, lane);
       float r0[4], r1[4], d0[4], d1[4];
       zero4(r0); zero4(r1); zero4(d0); zero4(d1);
 #pragma unroll 4
@@ -683,7 +685,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         for (int hf = 0; hf < 2; ++hf) {
           const int k = k0 + 8 * hf + t;
           AFrag<X3> a;
-          a.set(sK[(m0 + g) * 132 + k], sK[(m0 + g + 8) * 132 + k], sK[(m0 + g) * 132 + k + 4], sK[(m0 + g + 8) * 132 + k + 4]);
+          mma::lda(a, aK + 4u * (k0 + 8 * hf));
           BFrag<X3> bs, bd;
           bs.set(sS0[k * LDV + n0 + g], sS0[(k + 4) * LDV + n0 + g]);
           bd.set(sdS[k * LDV + n0 + g], sdS[(k + 4) * LDV + n0 + g]);
@@ -713,12 +715,13 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     __syncthreads();
     // ---- Vn = T R, dR = T^T dVn ------------------------------------------------------------------------------------------------------
     {
+      const uint32_t aT = mma::lda_at(tc::smem_u32(sT), LDT, m0, lane);
       float vn[4], dr[4];
       zero4(vn); zero4(dr);
       for (int k0 = 0; k0 < m0 + 16; k0 += 8) {
         const int k = k0 + t;
         AFrag<X3> a;
-        a.set(sT[(m0 + g) * LDT + k], sT[(m0 + g + 8) * LDT + k], sT[(m0 + g) * LDT + k + 4], sT[(m0 + g + 8) * LDT + k + 4]);
+        mma::lda(a, aT + 4u * k0);
         BFrag<X3> br;
         br.set(sVn[k * LDV + n0 + g], sVn[(k + 4) * LDV + n0 + g]);
         fma<X3>(vn, a, br);

@@ -55,6 +55,18 @@ __device__ __forceinline__ void fma(float (&d)[4], const AFrag<X3>& a, const BFr
   }
   tf32(d, a.h, b.h);
 }
+// A operand of 16 rows and 8 columns of a float32 array (row-major, row stride 4 mod 32 words: no bank conflicts) in one instruction:
+// ldmatrix moves pairs of 16-bit entries, i.e. whole words.  lda_at: the lane's address, to be advanced by columns.
+__device__ __forceinline__ uint32_t lda_at(uint32_t base, int ld, int r0, int lane) {
+  return base + 4u * (uint32_t)((r0 + (lane & 15)) * ld + (lane >> 4) * 4);
+}
+template <bool X3>
+__device__ __forceinline__ void lda(AFrag<X3>& a, uint32_t addr) {
+  uint32_t x[4];
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(addr) : "memory");
+  a.set(__uint_as_float(x[0]), __uint_as_float(x[1]), __uint_as_float(x[2]), __uint_as_float(x[3]));
+}
 // products with one operand that is exact in a single term (a bf16 value)
 template <bool X3>
 __device__ __forceinline__ void fma_a1(float (&d)[4], const AFrag<false>& a, const BFrag<X3>& b) {
