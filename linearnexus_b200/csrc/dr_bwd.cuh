@@ -1349,8 +1349,12 @@ inline cudaError_t bwd_side_stream(cudaStream_t* out) {
 
 // The checkpointing forward of the backward: state at the start of every chunk -> the head of the workspace.
 // With o / hT given it is also the forward a training step needs (dr_chunk_fwd_saving), so that step runs one
-// forward instead of two.  KDA at the tensor-core shape uses the two-kernel forward with its records parked in the
-// accumulator part of the workspace (262 KB per chunk there against 66 KB of records; the adjoint overwrites it).
+// forward instead of two.  KDA at the tensor-core shape uses the two-kernel forward with its records parked where
+// the adjoint will write dS of every chunk (66 KB each).
+// The pre-pass goes to the side stream BEHIND the forward kernel it overlaps with: that one is a chain over few CTAs, and the
+// pre-pass, whose CTAs fill the chip, would keep it waiting for an SM.  The two-kernel forward's own chunk-parallel pass fills
+// the chip as well, so there the fork lies between its kernels (KDA, B=2, T=4096, H=16: forward and pre-pass one after the
+// other took 590 us of a 1772 us step).
 // own_stream: the pre-pass may run on the library's side stream, forked from and joined to `stream` with events
 // (false for callers that must not create streams or events: the pre-pass then runs on `stream` before the forward).
 cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
@@ -1362,26 +1366,19 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
   auto pre = [&](cudaStream_t s) {
     return chunked ? bwdc::launch_pre(d, q, k, g, beta, workspace, s, launches) : launch_bwd_pre(d, q, k, g, beta, workspace, s, launches);
   };
-  if (chunked || bwd_tensor_core_path(d)) {
-    cudaStream_t side = nullptr;
-    cudaEvent_t forked = nullptr;
-    if (own_stream && bwd_side_stream(&side) == cudaSuccess &&
-        cudaEventCreateWithFlags(&forked, cudaEventDisableTiming) == cudaSuccess &&
-        cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess) {
-      cudaError_t ef = cudaEventRecord(forked, stream);
-      if (ef == cudaSuccess) ef = cudaStreamWaitEvent(side, forked, 0);
-      if (ef == cudaSuccess) ef = pre(side);
-      if (ef == cudaSuccess) ef = cudaEventRecord(joined, side);
-      cudaEventDestroy(forked);   // released once the work recorded in it has completed
-      if (ef != cudaSuccess) { cudaEventDestroy(joined); return ef; }
-    } else {
+  cudaStream_t side = nullptr;
+  cudaEvent_t forked = nullptr;
+  const bool want_pre = chunked || bwd_tensor_core_path(d);
+  if (want_pre) {
+    if (!(own_stream && bwd_side_stream(&side) == cudaSuccess &&
+          cudaEventCreateWithFlags(&forked, cudaEventDisableTiming) == cudaSuccess &&
+          cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess)) {
       if (forked) cudaEventDestroy(forked);
-      if (joined) { cudaEventDestroy(joined); joined = nullptr; }
+      forked = joined = nullptr;
       const cudaError_t ep = pre(stream);
       if (ep != cudaSuccess) return ep;
     }
   }
-  const int64_t N = (d->T + C - 1) / C, units = (int64_t)d->B * d->H;
   float* ckpt = reinterpret_cast<float*>(workspace);
   FwdParams f;
   f.q = q; f.k = k; f.v = v; f.g = g; f.beta = beta; f.h0 = h0; f.o = o; f.hT = hT; f.status = status;
@@ -1397,14 +1394,16 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
   const bool fused = tc_shape && (d->variant == DR_DELTA || (d->variant == DR_GATED && d->g_dtype == DR_F32)) &&
                      (!o || d->out_dtype == DR_BF16);
   const bool split = tc_shape && !fused && d->variant == DR_KDA;
-  cudaError_t e;
-  if (fused) {
+  cudaError_t e = cudaSuccess;
+  if (forked && !split) e = cudaEventRecord(forked, stream);
+  if (e != cudaSuccess) {
+  } else if (fused) {
     e = launch_chunk_fused(f, stream);
     ++*launches;
   } else if (split) {
     int n2 = 0;
     // its records lie where dS1 of every chunk will be written (bwdc::Params)
-    e = launch_chunk_split(f, bwdc::make_params(d, workspace).ds, stream, &n2);
+    e = launch_chunk_split(f, bwdc::make_params(d, workspace).ds, stream, &n2, forked);
     *launches += n2;
   } else {
     // every other shape: the token recurrence (the same function of the inputs as the chunk form, and on the CUDA
@@ -1412,10 +1411,13 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
     e = launch_recurrent(f, stream);
     ++*launches;
   }
-  if (joined) {   // what follows on `stream` waits for the pre-pass as well
-    const cudaError_t ej = cudaStreamWaitEvent(stream, joined, 0);
+  if (forked) {
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, forked, 0);
+    if (e == cudaSuccess) e = pre(side);
+    if (e == cudaSuccess) e = cudaEventRecord(joined, side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, joined, 0);   // what follows on `stream` waits for the pre-pass as well
+    cudaEventDestroy(forked);   // released once the work recorded in them has completed
     cudaEventDestroy(joined);
-    if (e == cudaSuccess) e = ej;
   }
   return e;
 }

@@ -17,9 +17,9 @@
 //
 // Per-channel decay cannot be folded into row/column factors of a plain K K^T product the way a scalar
 // decay can, and e^{-G} alone overflows for strong decay.  The chunk-local products therefore use 16-row
-// sub-blocks: an off-diagonal block (rows in sub-block bi, columns in an earlier sub-block) is the
-// bf16 tensor-core product of  x_i e^{G_i - G_n}  and  k_j e^{G_n - G_j}  with n the first row of bi, so
-// both exponents are <= 0; the four diagonal 16x16 blocks are summed exactly in fp32 on the CUDA cores.
+// sub-blocks: rows of sub-block bi against earlier columns are the bf16 tensor-core product of
+// x_i e^{G_i - G_n}  and  k_j e^{G_n - G_j}  with n the first row of bi, so both exponents are <= 0; the four diagonal
+// 16x16 blocks use the same form while their decay range stays below 2^64 and are summed exactly in fp32 otherwise.
 //
 // Shape: K = V = 128, chunk 64, bf16 q/k/v, g bf16 or fp32 ([.., K] for KDA; the scalar-decay and
 // decay-free variants are served too, by broadcasting), fp32 beta/state, bf16 or fp32 output.
@@ -57,6 +57,11 @@ inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC -
 // (global loads, the serial prefix sum, the barriers between phases) hides behind the other's work.  The
 // inputs stay as raw bf16 with their l2-norm factors on the side, and the decayed bf16 operands of the
 // tensor-core products are formed in registers from them (no scaled copies in shared memory).
+// What bounds it: latency of dependent phases at 16 warps per SM (issue slots 47 %, shared-memory pipe 55 %, tensor pipe 10 %
+// busy).  Of 24 K cycles per chunk (two chunks at a time) 6.1 K are the loads, 8.9 K the products and the inverse's start,
+// 7.4 K the record.  8192 chunks x 32 heads / 64: 930 -> 820 us with one quotient per row instead of one per lane, W as two bf16 terms
+// and 16-byte reads.  Forming the decayed rows once as bf16 tiles was slower (1.44 against 1.21 ms for the whole forward):
+// two passes over 16 rows per thread in registers cost more than the exponentials they save.
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
@@ -1150,7 +1155,8 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
 }
 
 template <class IP, class SP>
-inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace, int64_t chunk_units, int64_t units, cudaStream_t stream) {
+inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace, int64_t chunk_units, int64_t units, cudaStream_t stream,
+                               cudaEvent_t after_intra = nullptr) {
   thread_local int attr_dev = -1;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1168,16 +1174,17 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   if (!sm100::make_panel_map(&S.tv, p.v, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
   e = launch_pdl(intra_kernel<IP>, dim3((unsigned)chunk_units), dim3(kThreads), IN_TOTAL, stream, I);
   if (e != cudaSuccess) return e;
+  if (after_intra && (e = cudaEventRecord(after_intra, stream)) != cudaSuccess) return e;
   S.use_tma_out = p.o != nullptr && sm100::make_output_map(&S.to, p.o, p.map, p.out_dt == DR_BF16 ? 2 : 4);
   return launch_pdl(state_kernel<SP>, dim3((unsigned)units), dim3(kStateThreads), ST_TOTAL, stream, S);
 }
 
-inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches) {
+inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra) {
   IntraParams I;
   StateParams S;
   const int64_t units = (int64_t)p.map.B * p.map.H;
   *launches = 2;
-  return launch_pair(I, S, p, workspace, units * ((p.map.T + kC - 1) / kC), units, stream);
+  return launch_pair(I, S, p, workspace, units * ((p.map.T + kC - 1) / kC), units, stream, after_intra);
 }
 
 // Every sequence of `seqs` in one pair of launches; the workspace holds seqs.chunks records per head.

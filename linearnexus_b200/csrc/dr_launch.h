@@ -12,7 +12,8 @@ cudaError_t launch_chunk_fused(const FwdParams& p, cudaStream_t stream);
 cudaError_t launch_chunk_fused_packed(const FwdParams& p, const SeqTable& seqs, cudaStream_t stream);
 // two-kernel forward (any variant); the workspace holds split_workspace_bytes
 int64_t split_workspace_bytes(int64_t units, int T);
-cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches);
+// after_intra: recorded on `stream` between the two kernels (null: not)
+cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra = nullptr);
 cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream);
 
 // forward in transition form (two kernels; K = V = 64 or 128); bf16_tensor: the bf16-operand kernels (dr_fwd.cu; bf16 q, k, v,
