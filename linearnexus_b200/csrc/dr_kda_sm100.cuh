@@ -59,7 +59,7 @@ inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC -
 // tensor-core products are formed in registers from them (no scaled copies in shared memory).
 // What bounds it: latency of dependent phases at 16 warps per SM (issue slots 47 %, shared-memory pipe 55 %, tensor pipe 10 %
 // busy).  Of 24 K cycles per chunk (two chunks at a time) 6.1 K are the loads, 8.9 K the products and the inverse's start,
-// 7.4 K the record.  8192 chunks x 32 heads / 64: 930 -> 820 us with one quotient per row instead of one per lane, W as two bf16 terms
+// 7.4 K the record.  B=4 T=8192 H=32 (16384 chunks): 930 -> 820 us with one quotient per row instead of one per lane, W as two bf16 terms
 // and 16-byte reads.  Forming the decayed rows once as bf16 tiles was slower (1.44 against 1.21 ms for the whole forward):
 // two passes over 16 rows per thread in registers cost more than the exponentials they save.
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
