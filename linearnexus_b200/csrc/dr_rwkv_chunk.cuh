@@ -30,7 +30,8 @@ namespace rwkv {
 
 using mma::AFrag;
 using mma::BFrag;
-constexpr int kK = 64, kTB = 8, kGroups = 3, kRing = 3, kStages = 4, kThreads = 128 * (1 + kGroups), kCons = 128;
+constexpr int kK = 64, kTB = 8, kGroups = 2, kRing = 3, kStages = 4, kCons = 256, kThreads = kCons + 128 * kGroups;
+constexpr int kHand = kCons + 128;   // threads of a hand-over barrier: the consumers and one staging group
 constexpr int LDR = 72;    // row vectors [token][key], read as B operands along the key axis
 constexpr int LDH = 68;    // update vectors [token][key] and values [token][column], read across tokens
 
@@ -51,17 +52,27 @@ struct Stage {
   float qk[64], qb[64], T[64], P[64];   // [i][j]; P = T ak
 };
 
+using Exchange = float[2][4][2][2][32][4];   // [block parity][16 value columns][key half][q, a][lane][entry]: partial dots
+
 struct Scratch {            // of one staging group
   float inv[16][LDR];       // k / W_j, b / W_j
   float ab[64], ak[64];
   int wide;
 };
 template <int KIND, bool BF>
-constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + kGroups * ((int)sizeof(Scratch) + kRing * Ring<KIND, BF>::kSlot) + 64; }
+constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * ((int)sizeof(Scratch) + kRing * Ring<KIND, BF>::kSlot) + 64; }
 
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-constexpr int kBarFull = 1, kBarEmpty = 1 + kStages, kBarGroup = 1 + 2 * kStages;
+constexpr int kBarFull = 1, kBarEmpty = 1 + kStages, kBarGroup = 1 + 2 * kStages, kBarPair = kBarGroup + kGroups;
+static_assert(kBarPair + 4 <= 16, "named barriers");
+
+// a float32-precise product whose terms go to three accumulators (hi hi, lo hi, hi lo)
+__device__ __forceinline__ void fma3(float (&d)[3][4], const AFrag<true>& a, const BFrag<true>& b) {
+  mma::tf32(d[1], a.l, b.h);
+  mma::tf32(d[2], a.h, b.l);
+  mma::tf32(d[0], a.h, b.h);
+}
 
 template <int KIND, bool BF>
 __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecParams p) {
@@ -80,7 +91,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     // =========================== staging =========================================================================================
     const int grp = (threadIdx.x - kCons) >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
     constexpr int kGrpBytes = (sizeof(Scratch) + 15) / 16 * 16 + kRing * R::kSlot;
-    uint8_t* mine = smem + kStages * sizeof(Stage) + grp * kGrpBytes;
+    uint8_t* mine = smem + kStages * sizeof(Stage) + sizeof(Exchange) + grp * kGrpBytes;
     Scratch& X = *reinterpret_cast<Scratch*>(mine);
     uint8_t* ring = mine + (sizeof(Scratch) + 15) / 16 * 16;
     constexpr int kRounds = (R::kTasks + 3) / 4;
@@ -125,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     for (int blk = grp; blk < nblk; blk += kGroups) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
       if (tid == 0) X.wide = 0;
-      if (blk >= kStages) bar_sync(kBarEmpty + blk % kStages, 256);   // the consumers have left this stage
+      if (blk >= kStages) bar_sync(kBarEmpty + blk % kStages, kHand);   // the consumers have left this stage
       sync128();   // every thread's pieces of this block have landed
       const uint8_t* slot = ring + (blk / kGroups % kRing) * R::kSlot;
       Stage& S = s_st[blk % kStages];
@@ -262,48 +273,57 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
         sync128();
         if (tid < 8) S.qk[9 * tid] = X.ab[tid] + X.ab[8 + tid];
       }
-      bar_arrive(kBarFull + blk % kStages, 256);
+      bar_arrive(kBarFull + blk % kStages, kHand);
       sync128();           // the raw block has been read by every thread
       issue(blk + kGroups * kRing);
     }
     return;
   }
 
-  // =========================== the state: warp = 16 value columns ======================================================================
-  const int vb = 16 * (threadIdx.x >> 5);
-  float S[8][4];   // tile nt: columns vb + g, + 8 (rows), keys 8 nt + 2 t, + 1
+  // =========================== the state: warp = 16 value columns, 32 keys ==============================================================
+  const int cw = threadIdx.x >> 5, pair = cw & 3, half = cw >> 2, vb = 16 * pair, kb = 32 * half;
+  Exchange& ex = *reinterpret_cast<Exchange*>(smem + kStages * sizeof(Stage));
+  float S[4][4];   // tile nt: columns vb + g, + 8 (rows), keys kb + 8 nt + 2 t, + 1
   const float* h0 = p.h0 ? p.h0 + (int64_t)unit * kK * p.V + v0 + vb + g : nullptr;
 #pragma unroll
-  for (int nt = 0; nt < 8; ++nt)
+  for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) S[nt][e] = h0 ? h0[(int64_t)(8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] : 0.f;
+    for (int e = 0; e < 4; ++e) S[nt][e] = h0 ? h0[(int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] : 0.f;
   const int64_t o_at = (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + v0 + vb + g;
   for (int blk = 0; blk < nblk; ++blk) {
-    bar_sync(kBarFull + blk % kStages, 256);
+    bar_sync(kBarFull + blk % kStages, kHand);
     const Stage& St = s_st[blk % kStages];
-    // dots of q (and a) with h, transposed: rows = columns of v, columns = tokens
-    float dq[2][4], da[2][4];
+    const bool out = (blk & 1) == half;   // this warp's turn to form the block's output
+    // this half's part of the dots of q (and a) with h, transposed: rows = columns of v, columns = tokens.  The three terms of
+    // a float32 product go to accumulators of their own: four dependent products deep instead of twelve
+    float dq[3][4], da[3][4];
 #pragma unroll
-    for (int x = 0; x < 2; ++x) { dq[x][0] = dq[x][1] = dq[x][2] = dq[x][3] = 0.f; da[x][0] = da[x][1] = da[x][2] = da[x][3] = 0.f; }
+    for (int x = 0; x < 3; ++x) { dq[x][0] = dq[x][1] = dq[x][2] = dq[x][3] = 0.f; da[x][0] = da[x][1] = da[x][2] = da[x][3] = 0.f; }
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
+    for (int ks = 0; ks < 4; ++ks) {
       AFrag<true> a;
       a.set(S[ks][0], S[ks][2], S[ks][1], S[ks][3]);
       BFrag<true> bq;
-      const float2 y = *reinterpret_cast<const float2*>(&St.row[g][8 * ks + 2 * t]);
+      const float2 y = *reinterpret_cast<const float2*>(&St.row[g][kb + 8 * ks + 2 * t]);
       bq.set(y.x, y.y);
-      mma::fma<true>(dq[ks & 1], a, bq);
+      fma3(dq, a, bq);
       if constexpr (LR) {
-        const float2 z = *reinterpret_cast<const float2*>(&St.row[8 + g][8 * ks + 2 * t]);
+        const float2 z = *reinterpret_cast<const float2*>(&St.row[8 + g][kb + 8 * ks + 2 * t]);
         BFrag<true> ba;
         ba.set(z.x, z.y);
-        mma::fma<true>(da[ks & 1], a, ba);
+        fma3(da, a, ba);
       }
     }
-    // the decay of h: independent of the dots' results
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const float2 w = *reinterpret_cast<const float2*>(&St.w[8 * nt + 2 * t]);
+    for (int e = 0; e < 4; ++e) { dq[0][e] += dq[1][e] + dq[2][e]; da[0][e] += da[1][e] + da[2][e]; }
+    auto& mine = ex[blk & 1][pair][half];
+    const auto& other = ex[blk & 1][pair][half ^ 1];
+    *reinterpret_cast<float4*>(mine[0][lane]) = make_float4(dq[0][0], dq[0][1], dq[0][2], dq[0][3]);
+    if constexpr (LR) *reinterpret_cast<float4*>(mine[1][lane]) = make_float4(da[0][0], da[0][1], da[0][2], da[0][3]);
+    // decay of h and the values' update: independent of the dots
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const float2 w = *reinterpret_cast<const float2*>(&St.w[kb + 8 * nt + 2 * t]);
       S[nt][0] *= w.x; S[nt][1] *= w.y; S[nt][2] *= w.x; S[nt][3] *= w.y;
     }
     AFrag<true> av;   // V^T: rows = columns of v, k = tokens (bf16 values are exact in one term)
@@ -322,45 +342,52 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
       bb.set(y.x, y.y);
       return bb;
     };
+    float o[4] = {0.f, 0.f, 0.f, 0.f}, u[3][4];
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {   // h += V^T (W_7 / W_j k)
+    for (int x = 0; x < 3; ++x) u[x][0] = u[x][1] = u[x][2] = u[x][3] = 0.f;
+    if constexpr (LR) mul_v(u[0], small(St.P));
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {   // h += V^T (W_7 / W_j k)
       BFrag<true> bk;
-      bk.set(St.upd[2 * t][8 * nt + g], St.upd[2 * t + 1][8 * nt + g]);
+      bk.set(St.upd[2 * t][kb + 8 * nt + g], St.upd[2 * t + 1][kb + 8 * nt + g]);
       mul_v(S[nt], bk);
     }
-    float o[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = dq[0][e] + dq[1][e];
-    mul_v(o, small(St.qk));
+    if (out) mul_v(o, small(St.qk));
+    bar_sync(kBarPair + pair, 64);   // (two buffers: a warp is at most one block ahead of its partner)
+    if (out) {
+      const float4 x = *reinterpret_cast<const float4*>(other[0][lane]);
+      o[0] += dq[0][0] + x.x; o[1] += dq[0][1] + x.y; o[2] += dq[0][2] + x.z; o[3] += dq[0][3] + x.w;
+    }
     if constexpr (LR) {
-      float u[4] = {0.f, 0.f, 0.f, 0.f};
+      const float4 x = *reinterpret_cast<const float4*>(other[1][lane]);
       AFrag<true> aa;
-      aa.set(da[0][0] + da[1][0], da[0][2] + da[1][2], da[0][1] + da[1][1], da[0][3] + da[1][3]);
-      mul_v(u, small(St.P));
-      mma::fma<true>(u, aa, small(St.T));
+      aa.set(da[0][0] + x.x, da[0][2] + x.z, da[0][1] + x.y, da[0][3] + x.w);
+      fma3(u, aa, small(St.T));
       AFrag<true> au;
-      au.set(u[0], u[2], u[1], u[3]);
+      au.set(u[0][0] + (u[1][0] + u[2][0]), u[0][2] + (u[1][2] + u[2][2]), u[0][1] + (u[1][1] + u[2][1]), u[0][3] + (u[1][3] + u[2][3]));
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {   // h += U^T (W_7 / W_j b)
+      for (int nt = 0; nt < 4; ++nt) {   // h += U^T (W_7 / W_j b)
         BFrag<true> bb;
-        bb.set(St.upd[8 + 2 * t][8 * nt + g], St.upd[9 + 2 * t][8 * nt + g]);
+        bb.set(St.upd[8 + 2 * t][kb + 8 * nt + g], St.upd[9 + 2 * t][kb + 8 * nt + g]);
         mma::fma<true>(S[nt], au, bb);
       }
-      mma::fma<true>(o, au, small(St.qb));
+      if (out) mma::fma<true>(o, au, small(St.qb));
     }
+    if (blk + kStages < nblk) bar_arrive(kBarEmpty + blk % kStages, kHand);
+    if (out) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int tok = blk * kTB + 2 * t + (e & 1);
-      if (tok < T) st_elem(p.o, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), BF ? DR_BF16 : DR_F32, o[e]);
+      for (int e = 0; e < 4; ++e) {
+        const int tok = blk * kTB + 2 * t + (e & 1);
+        if (tok < T) st_elem(p.o, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), BF ? DR_BF16 : DR_F32, o[e]);
+      }
     }
-    if (blk + kStages < nblk) bar_arrive(kBarEmpty + blk % kStages, 256);
   }
   if (p.hT) {
     float* hT = p.hT + (int64_t)unit * kK * p.V + v0 + vb + g;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) hT[(int64_t)(8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] = S[nt][e];
+      for (int e = 0; e < 4; ++e) hT[(int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] = S[nt][e];
   }
 }
 
