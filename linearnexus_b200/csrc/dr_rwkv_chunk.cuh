@@ -8,13 +8,16 @@
 // so U = T D_a + (T ak) V with T = (I - ab)^-1 [8 x 8].  RWKV-6 (o_i reads h_{i-1}, a bonus u q.k on the current token, no a, b) is
 // the same without U.
 //
-// Four warps keep the state transposed in accumulators (16 value columns x 64 keys each).  An accumulator is, register for
-// register, an A operand whose contraction runs over its columns: h feeds the dots, their result feeds T, U feeds the update,
-// and nothing of the state touches memory.  Three groups of four warps stage the blocks ahead, one block in three each (staging a
-// block is a chain of ~3.5 K cycles, the state's share ~1.5 K): raw rows from a ring of asynchronous copies, decay products, the
-// row vectors and the 8 x 8 coefficients.  Hand-overs are named barriers, arrived on by one side and waited for by the other.
+// Eight warps keep the state transposed in accumulators (16 value columns x 32 keys each; the two warps of a column block
+// exchange their partial dots).  An accumulator is, register for register, an A operand whose contraction runs over its columns: h
+// feeds the dots, their result feeds T, U feeds the update, and nothing of the state touches memory.  Three groups of four warps
+// stage the blocks ahead, one block in three each: raw rows from a ring of asynchronous copies, decay products, the row vectors and
+// the 8 x 8 coefficients.  Hand-overs are named barriers, arrived on by one side and waited for by the other.
 //
-// What bounds it: ~100 mma per warp and block of 8 cycles each (100 cycles per token).  The token recurrence it replaces here ran
+// What bounds it: the chain of a block through the dots, U and the update, 2.6 K cycles with the schedulers 55 % and the tensor pipe 35 %
+// busy (B=8, T=4096, H=16: 868 us with four warps of 64 keys and products in source order, 820 with them free to move, 785
+// with eight warps, 761 with the B operands split once by the staging warps; two staging groups instead of three: 872).
+// The token recurrence it replaces here ran
 // at 540 cycles per token whatever its instruction count or prefetch depth: one dependent reduce-and-update chain per token, and
 // 260 shared-memory wavefronts per token to feed 160 multiply-adds per thread (a 16-byte load fills a quarter of a warp per
 // wavefront, broadcast or not).  A four-token form on the CUDA cores stayed at that roof (1.18 ms against 1.14).
@@ -30,10 +33,11 @@ namespace rwkv {
 
 using mma::AFrag;
 using mma::BFrag;
-constexpr int kK = 64, kTB = 8, kGroups = 2, kRing = 3, kStages = 4, kCons = 256, kThreads = kCons + 128 * kGroups;
+constexpr int kK = 64, kTB = 8, kGroups = 3, kRing = 3, kStages = 4, kCons = 256, kThreads = kCons + 128 * kGroups;
 constexpr int kHand = kCons + 128;   // threads of a hand-over barrier: the consumers and one staging group
 constexpr int LDR = 72;    // row vectors [token][key], read as B operands along the key axis
-constexpr int LDH = 68;    // update vectors [token][key] and values [token][column], read across tokens
+constexpr int LDU = 66;    // update vectors [token pair][key], read across tokens
+constexpr int LDH = 68;    // values [token][column], read across tokens
 
 template <int KIND, bool BF>
 struct Ring {
@@ -44,19 +48,40 @@ struct Ring {
   static constexpr int kSlot = (NV + 1) * kVec;
 };
 
+// What the consumers read as B operands is stored split into its two tf32 terms, once, by the staging warps (four warps of value
+// columns read each; splitting it there was a third of their instructions), in the order of a fragment: one 16-byte read each.
 struct Stage {
-  float row[16][LDR];       // 0-7: q W (RWKV-6: q W_{i-1});  8-15: a W_{i-1}
-  float upd[16][LDH];       // 0-7: W_7 / W_j k;  8-15: W_7 / W_j b
+  float2 row[16][LDR];      // (hi, lo); 0-7: q W (RWKV-6: q W_{i-1});  8-15: a W_{i-1}
+  float4 upd[8][LDU];       // token pairs (hi, hi, lo, lo); 0-3: W_7 / W_j k;  4-7: W_7 / W_j b
+  float4 qk[32], qb[32], T[32], P[32];   // [i][j / 2], (hi, hi, lo, lo) of j, j + 1; P = T ak
   float v[kTB][LDH];
   float w[kK];              // W_7
-  float qk[64], qb[64], T[64], P[64];   // [i][j]; P = T ak
 };
+__device__ __forceinline__ float2 split(float x) {
+  const float hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  return make_float2(hi, x - hi);
+}
+__device__ __forceinline__ float4 split2(float x, float y) {
+  const float2 a = split(x), b = split(y);
+  return make_float4(a.x, b.x, a.y, b.y);
+}
+__device__ __forceinline__ BFrag<true> frag(float4 x) {   // of a pair stored by split2
+  BFrag<true> b;
+  b.h[0] = __float_as_uint(x.x); b.h[1] = __float_as_uint(x.y);
+  b.l[0] = __float_as_uint(x.z); b.l[1] = __float_as_uint(x.w);
+  return b;
+}
+__device__ __forceinline__ void put(float4* m, int i, int j, float x) {   // one entry of an 8 x 8 coefficient matrix
+  const float2 a = split(x);
+  float* at = reinterpret_cast<float*>(m + 4 * i + (j >> 1)) + (j & 1);
+  at[0] = a.x; at[2] = a.y;
+}
 
 using Exchange = float[2][4][2][2][32][4];   // [block parity][16 value columns][key half][q, a][lane][entry]: partial dots
 
 struct Scratch {            // of one staging group
   float inv[16][LDR];       // k / W_j, b / W_j
-  float ab[64], ak[64];
+  float ab[64], ak[64], T[64];
   int wide;
 };
 template <int KIND, bool BF>
@@ -155,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
           if (LR) x = role == 0 ? raw(slot, 0, i, ch) * p.scale : raw(slot, 3, i, ch);
           else x = t0 + i < T ? p.scale / (1.f + __expf(-raw(slot, 0, i, ch))) : 0.f;   // sigmoid(r) scale
           if (LR && role == 0) W *= w[i];
-          S.row[8 * role + i][ch] = x * W;
+          S.row[8 * role + i][ch] = split(x * W);
           if (!(LR && role == 0)) W *= w[i];
           y[i] = raw(slot, LR && role == 1 ? 4 : 1, i, ch);
         }
@@ -165,9 +190,11 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
         }
         float D = 1.f;
 #pragma unroll
-        for (int j = 7; j >= 0; --j) {
-          S.upd[8 * role + j][ch] = y[j] * D;
+        for (int j = 7; j >= 0; j -= 2) {
+          const float hi = y[j] * D;
           D *= w[j];
+          S.upd[4 * role + (j >> 1)][ch] = split2(y[j - 1] * D, hi);
+          D *= w[j - 1];
         }
         float I = 1.f;
 #pragma unroll
@@ -203,28 +230,34 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
               }
             }
             acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            if (!half) (isa ? (which ? X.ab : X.ak) : (which ? S.qb : S.qk))[pair] = acc;
+            if (!half) {
+              if (isa) (which ? X.ab : X.ak)[pair] = acc;
+              else put(which ? S.qb : S.qk, i, j, acc);
+            }
           }
       } else if (warp < (LR ? 2 : 1)) {
         float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          const float2 x0 = *reinterpret_cast<const float2*>(&S.row[g][8 * ks + 2 * t]);
-          const float2 x1 = LR ? *reinterpret_cast<const float2*>(&S.row[8 + g][8 * ks + 2 * t]) : make_float2(0.f, 0.f);
+          const float4 x0 = *reinterpret_cast<const float4*>(&S.row[g][8 * ks + 2 * t]);
+          const float4 x1 = LR ? *reinterpret_cast<const float4*>(&S.row[8 + g][8 * ks + 2 * t]) : make_float4(0.f, 0.f, 0.f, 0.f);
           const float2 y = *reinterpret_cast<const float2*>(&X.inv[8 * warp + g][8 * ks + 2 * t]);
           AFrag<true> a;
-          a.set(x0.x, x1.x, x0.y, x1.y);
+          a.h[0] = __float_as_uint(x0.x); a.h[1] = __float_as_uint(x1.x); a.h[2] = __float_as_uint(x0.z); a.h[3] = __float_as_uint(x1.z);
+          a.l[0] = __float_as_uint(x0.y); a.l[1] = __float_as_uint(x1.y); a.l[2] = __float_as_uint(x0.w); a.l[3] = __float_as_uint(x1.w);
           BFrag<true> bb;
           bb.set(y.x, y.y);
           mma::fma<true>((ks & 1) ? d2 : d, a, bb);
         }
+        float q[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int i = g, j = 2 * t + e;
-          const float q = d[e] + d2[e], a = d[2 + e] + d2[2 + e];
-          (warp ? S.qb : S.qk)[8 * i + j] = (LR ? j <= i : j < i) ? q : 0.f;
+          const float a = d[2 + e] + d2[2 + e];
+          q[e] = (LR ? j <= i : j < i) ? d[e] + d2[e] : 0.f;
           if (LR) (warp ? X.ab : X.ak)[8 * i + j] = j < i ? a : 0.f;
         }
+        (warp ? S.qb : S.qk)[lane] = split2(q[0], q[1]);
       }
       if (LR) {
         sync128();
@@ -238,7 +271,8 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 #pragma unroll
               for (int j = 0; j < 8; ++j)
                 if (j < i) x[i] += X.ab[8 * i + j] * x[j];
-              S.T[8 * i + lane] = x[i];
+              X.T[8 * i + lane] = x[i];
+              put(S.T, i, lane, x[i]);
             }
           }
           __syncwarp();
@@ -246,8 +280,8 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
           for (int e = lane; e < 64; e += 32) {
             float acc = 0.f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc += S.T[(e & ~7) + j] * X.ak[8 * j + (e & 7)];
-            S.P[e] = acc;
+            for (int j = 0; j < 8; ++j) acc += X.T[(e & ~7) + j] * X.ak[8 * j + (e & 7)];
+            put(S.P, e >> 3, e & 7, acc);
           }
         }
       } else {
@@ -271,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
           if (lane < 8) X.ab[8 * warp + lane] = x[0];
         }
         sync128();
-        if (tid < 8) S.qk[9 * tid] = X.ab[tid] + X.ab[8 + tid];
+        if (tid < 8) put(S.qk, tid, tid, X.ab[tid] + X.ab[8 + tid]);
       }
       bar_arrive(kBarFull + blk % kStages, kHand);
       sync128();           // the raw block has been read by every thread
@@ -303,16 +337,12 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     for (int ks = 0; ks < 4; ++ks) {
       AFrag<true> a;
       a.set(S[ks][0], S[ks][2], S[ks][1], S[ks][3]);
-      BFrag<true> bq;
-      const float2 y = *reinterpret_cast<const float2*>(&St.row[g][kb + 8 * ks + 2 * t]);
-      bq.set(y.x, y.y);
-      fma3(dq, a, bq);
-      if constexpr (LR) {
-        const float2 z = *reinterpret_cast<const float2*>(&St.row[8 + g][kb + 8 * ks + 2 * t]);
-        BFrag<true> ba;
-        ba.set(z.x, z.y);
-        fma3(da, a, ba);
-      }
+      auto row = [&](int r) {   // two keys, each (hi, lo)
+        const float4 y = *reinterpret_cast<const float4*>(&St.row[r][kb + 8 * ks + 2 * t]);
+        return frag(make_float4(y.x, y.z, y.y, y.w));
+      };
+      fma3(dq, a, row(g));
+      if constexpr (LR) fma3(da, a, row(8 + g));
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) { dq[0][e] += dq[1][e] + dq[2][e]; da[0][e] += da[1][e] + da[2][e]; }
@@ -336,21 +366,14 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
         mma::fma<true>(d, av, bb);
       }
     };
-    auto small = [&](const float* m) {   // an 8 x 8 coefficient matrix [i][j] as B operand (k = j, n = i)
-      const float2 y = *reinterpret_cast<const float2*>(m + 8 * g + 2 * t);
-      BFrag<true> bb;
-      bb.set(y.x, y.y);
-      return bb;
-    };
+    auto small = [&](const float4* m) { return frag(m[lane]); };   // an 8 x 8 coefficient matrix [i][j] as B operand (k = j, n = i)
     float o[4] = {0.f, 0.f, 0.f, 0.f}, u[3][4];
 #pragma unroll
     for (int x = 0; x < 3; ++x) u[x][0] = u[x][1] = u[x][2] = u[x][3] = 0.f;
     if constexpr (LR) mul_v(u[0], small(St.P));
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {   // h += V^T (W_7 / W_j k)
-      BFrag<true> bk;
-      bk.set(St.upd[2 * t][kb + 8 * nt + g], St.upd[2 * t + 1][kb + 8 * nt + g]);
-      mul_v(S[nt], bk);
+      mul_v(S[nt], frag(St.upd[t][kb + 8 * nt + g]));
     }
     if (out) mul_v(o, small(St.qk));
     bar_sync(kBarPair + pair, 64);   // (two buffers: a warp is at most one block ahead of its partner)
@@ -367,9 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
       au.set(u[0][0] + (u[1][0] + u[2][0]), u[0][2] + (u[1][2] + u[2][2]), u[0][1] + (u[1][1] + u[2][1]), u[0][3] + (u[1][3] + u[2][3]));
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {   // h += U^T (W_7 / W_j b)
-        BFrag<true> bb;
-        bb.set(St.upd[8 + 2 * t][kb + 8 * nt + g], St.upd[9 + 2 * t][kb + 8 * nt + g]);
-        mma::fma<true>(S[nt], au, bb);
+        mma::fma<true>(S[nt], au, frag(St.upd[4 + t][kb + 8 * nt + g]));
       }
       if (out) mma::fma<true>(o, au, small(St.qb));
     }
