@@ -358,15 +358,18 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
 // state_kernel: eight warps, warp w owns channel rows 16 w .. 16 w + 15 of dS [128][32]
 // =====================================================================================================================
 constexpr int kStThreads = 256;
-constexpr int kStSmem = 2 * 96 * 72 * 4;
 constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved, [rows / 2][32 columns][2], 72 floats per pair
+// X3: dS as its two terms, [rows / 2][32 columns][hi, hi, lo, lo]: split once by the warp that owns it, not by the eight that read it
+template <bool X3> constexpr int ld_ds = X3 ? 136 : LDP;
+template <bool X3> constexpr int st_smem = 2 * (64 * ld_ds<X3> + 32 * LDP) * 4;
 
 template <bool X3>
 __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
   pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
-  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * LDP]
-  float* sO = sS + 2 * 64 * LDP;                        // [2][32 * LDP]
+  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * LDS_]
+  constexpr int LDS_ = ld_ds<X3>;
+  float* sO = sS + 2 * 64 * LDS_;                       // [2][32 * LDP]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int unit = blockIdx.x >> 2, v0 = (blockIdx.x & 3) * kVS;
   const int b = unit / p.map.H, h = unit % p.map.H;
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
   }
   uint4 dor = load_do(p.N - 1);
   for (int n = p.N - 1; n >= 0; --n) {
-    float* cS = sS + (n & 1) * 64 * LDP;
+    float* cS = sS + (n & 1) * 64 * LDS_;
     float* cO = sO + (n & 1) * 32 * LDP;
     // dS1 of this chunk: to memory, and to the other warps
     float* out = p.ds + (chunk0 + n) * (kD * kD) + v0;
@@ -410,10 +413,22 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
       const int c = 8 * nt + 2 * t;
       *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
       *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
-      float* w0 = cS + (r0 >> 1) * LDP + 2 * c + (r0 & 1);
-      float* w1 = cS + (r1 >> 1) * LDP + 2 * c + (r1 & 1);
-      w0[0] = S[nt][0]; w0[2] = S[nt][1];
-      w1[0] = S[nt][2]; w1[2] = S[nt][3];
+      if constexpr (X3) {   // the lanes of a row pair swap: the even row's takes column c of both rows, the odd row's c + 1
+        const bool odd = g & 1;
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+          const float got = __shfl_xor_sync(0xffffffffu, odd ? S[nt][2 * hr] : S[nt][2 * hr + 1], 4);
+          const float x = odd ? got : S[nt][2 * hr], y = odd ? S[nt][2 * hr + 1] : got;   // even row, odd row
+          BFrag<true> f;
+          f.set(x, y);
+          *reinterpret_cast<uint4*>(cS + ((hr ? r1 : r0) >> 1) * LDS_ + 4 * (c + odd)) = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
+        }
+      } else {
+        float* w0 = cS + (r0 >> 1) * LDP + 2 * c + (r0 & 1);
+        float* w1 = cS + (r1 >> 1) * LDP + 2 * c + (r1 & 1);
+        w0[0] = S[nt][0]; w0[2] = S[nt][1];
+        w1[0] = S[nt][2]; w1[2] = S[nt][3];
+      }
     }
     {
       const uint32_t w[4] = {dor.x, dor.y, dor.z, dor.w};
@@ -438,9 +453,9 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const float2 y = ld2(cO + (4 * ks + t) * LDP + 2 * (8 * nt + g));
-        BFrag<X3> bo;
+        BFrag<false> bo;   // bf16 values: one term in either precision
         bo.set(y.x, y.y);
-        fma<X3>(Z[nt], a, bo);
+        mma::fma_b1(Z[nt], a, bo);
       }
     }
 #pragma unroll
@@ -450,9 +465,14 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
       nf[ks] = __ldcs(p.nf + ((cn * 8 + warp) * 16 + ks) * 32 + lane);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
         BFrag<X3> bs;
-        bs.set(y.x, y.y);
+        if constexpr (X3) {
+          const uint4 y = *reinterpret_cast<const uint4*>(cS + (4 * ks + t) * LDS_ + 4 * (8 * nt + g));
+          bs.h[0] = y.x; bs.h[1] = y.y; bs.l[0] = y.z; bs.l[1] = y.w;
+        } else {
+          const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
+          bs.set(y.x, y.y);
+        }
         if (ks & 1) fma<X3>(Z[nt], a, bs); else fma<X3>(S[nt], a, bs);
       }
     }
@@ -1245,7 +1265,7 @@ inline cudaError_t set_attributes() {
   if (e != cudaSuccess || attr_dev == dev) return e;
   e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem<KDA>::kTotal);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(state_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(state_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem<KDA>);
   if (e == cudaSuccess) attr_dev = dev;
   return e;
 }
@@ -1267,7 +1287,7 @@ template <bool KDA>
 inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, cudaStream_t stream) {
   cudaError_t e = set_attributes<KDA>();
   if (e != cudaSuccess) return e;
-  e = launch_pdl(state_kernel<KDA>, dim3((unsigned)(units * 4)), dim3(kStThreads), kStSmem, stream, p);
+  e = launch_pdl(state_kernel<KDA>, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem<KDA>, stream, p);
   if (e != cudaSuccess) return e;
   return launch_pdl(local_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kLoThreads), LoSmem<KDA>::kTotal, stream, p);
 }
