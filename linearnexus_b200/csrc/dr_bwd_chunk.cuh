@@ -84,9 +84,11 @@ constexpr int kPreThreads = 256;
 constexpr int LDH = 136;   // row stride (bf16) of the raw k, q rows
 constexpr int PR_K = 0, PR_Q = PR_K + 64 * LDH * 2, PR_X = PR_Q + 64 * LDH * 2, PR_A = PR_X + 64 * LDT * 4;
 constexpr int PR_SC = PR_A + 64 * 72 * 4;     // beta, rk, rq, G, fw, fd (64 each)
-constexpr int PR_G = PR_SC + 6 * 64 * 4;      // KDA: log2(e) G [64][132]; Kd [64][132] later takes the place of k, q
-template <bool KDA> constexpr int pre_smem() { return KDA ? PR_G + 64 * 132 * 4 : PR_G; }
-static_assert(2 * 64 * LDH * 2 >= 64 * 132 * 4 && 2 * (pre_smem<true>() + 1024) <= 233472, "two CTAs per SM");
+constexpr int LDG = 136;   // row stride of G: pairs of eight rows are read without bank conflicts
+constexpr int LDK = 130;   // row stride (16-byte entries) of the split Kd
+constexpr int PR_G = PR_SC + 6 * 64 * 4;      // KDA: log2(e) G [64][136]; Kd as token pairs [32][130] (hi, hi, lo, lo) later over k, q, X, A
+template <bool KDA> constexpr int pre_smem() { return KDA ? PR_G + 64 * LDG * 4 : PR_G; }
+static_assert(PR_SC >= 32 * LDK * 16 && 2 * (pre_smem<true>() + 1024) <= 233472, "two CTAs per SM");
 
 template <bool KDA>
 __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + PR_K);
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + PR_Q);
-  float* sKd = reinterpret_cast<float*>(smem + PR_K);
+  uint4* sKd = reinterpret_cast<uint4*>(smem + PR_K);
   float* sX = reinterpret_cast<float*>(smem + PR_X);
   float* sA = reinterpret_cast<float*>(smem + PR_A);
   float* sBeta = reinterpret_cast<float*>(smem + PR_SC);
@@ -135,16 +137,33 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       const int c = warp + 8 * i;
       *reinterpret_cast<uint2*>(sQ + c * LDH + 4 * lane) = qr[i];
       *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kr[i];
-      if constexpr (KDA) *reinterpret_cast<float4*>(sG + c * 132 + 4 * lane) = gr[i];
-      float qmul = p.scale, kmul = 1.f;
-      if (p.l2norm) {
-        const float q0 = mma::lo_f(qr[i].x), q1 = mma::hi_f(qr[i].x), q2 = mma::lo_f(qr[i].y), q3 = mma::hi_f(qr[i].y);
-        const float k0 = mma::lo_f(kr[i].x), k1 = mma::hi_f(kr[i].x), k2 = mma::lo_f(kr[i].y), k3 = mma::hi_f(kr[i].y);
-        qmul = p.scale / (sqrtf(warp_sum(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3)) + 1e-6f);
-        kmul = 1.f / (sqrtf(warp_sum(k0 * k0 + k1 * k1 + k2 * k2 + k3 * k3)) + 1e-6f);
-      }
-      if (lane == i) { sBeta[c] = bt; sRk[c] = kmul; sRq[c] = qmul; }
+      if constexpr (KDA) *reinterpret_cast<float4*>(sG + c * LDG + 4 * lane) = gr[i];
     }
+    // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced, so that each lane takes one
+    // square root and one quotient
+    float ss[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float q0 = mma::lo_f(qr[i].x), q1 = mma::hi_f(qr[i].x), q2 = mma::lo_f(qr[i].y), q3 = mma::hi_f(qr[i].y);
+      const float k0 = mma::lo_f(kr[i].x), k1 = mma::hi_f(kr[i].x), k2 = mma::lo_f(kr[i].y), k3 = mma::hi_f(kr[i].y);
+      ss[i] = q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3;
+      ss[8 + i] = k0 * k0 + k1 * k1 + k2 * k2 + k3 * k3;
+    }
+#pragma unroll
+    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        const bool up = lane & o;
+        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
+        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
+      const float top = lane < 16 ? p.scale : 1.f;
+      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+    }
+    if (lane < 8) sBeta[warp + 8 * lane] = bt;
     if (!KDA && warp == 0) {
       mma::scan_scalars(g_lo, g_hi, lane);
       sGs[lane] = g_lo; sGs[lane + 32] = g_hi;
@@ -152,8 +171,8 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   }
   __syncthreads();
   if constexpr (KDA) {
-    mma::scan_channels<kPreThreads, kD>(sG, sX, tid);
-    if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * 132 + tid]);
+    mma::scan_channels<kPreThreads, kD, LDG>(sG, sX, tid);
+    if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * LDG + tid]);
     if (tid < 64) { sFw[tid] = sBeta[tid] * sRk[tid]; }
   } else {
     const float gl = sGs[63];
@@ -165,33 +184,61 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   }
   // ---- X = tril(K^K^^T.E, -1), A = tril(Q^K^^T.E): 20 tiles of 16 x 8 at or below the diagonal dealt to the warps ----------
   auto unsafe = [&](int blk) -> bool {   // KDA, warp-uniform: the decay inside the block exceeds 2^64 in some channel
-    const float4 ga = *reinterpret_cast<const float4*>(sG + 16 * blk * 132 + 4 * lane);
-    const float4 gb = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
+    const float4 ga = *reinterpret_cast<const float4*>(sG + 16 * blk * LDG + 4 * lane);
+    const float4 gb = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * LDG + 4 * lane);
     return __any_sync(0xffffffffu, !(fmaxf(fmaxf(ga.x - gb.x, ga.y - gb.y), fmaxf(ga.z - gb.z, ga.w - gb.w)) <= 64.f));
   };
+  if constexpr (KDA) {
+    // eight warp tasks (16-row block; 8-column tiles)  3;0-2  3;3-5  3;6-7  2;0-2  2;3-5  1;0-1  1;2-3  0;0-1: the decayed rows are formed
+    // once for a task's tiles; the contraction runs over pairs of neighbouring channels
+    const int mt = warp < 3 ? 3 : warp < 5 ? 2 : warp < 7 ? 1 : 0;
+    const int nt0 = warp < 3 ? 3 * warp : warp < 5 ? 3 * (warp - 3) : warp < 7 ? 2 * (warp - 5) : 0;
+    const int ntn = (warp == 2 || warp >= 5) ? 2 : 3;
+    const bool skip = unsafe(mt);   // the diagonal block is done exactly below
+    const int r0 = 16 * mt + g, r1 = r0 + 8, nrow = 16 * mt;
+    float dk[3][4], dq[3][4];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) { zero4(dk[x]); zero4(dq[x]); }
+#pragma unroll 2
+    for (int ks = 0; ks < 16; ++ks) {
+      const int c = 8 * ks + 2 * t;
+      const float2 gn = ld2(sG + nrow * LDG + c), ga = ld2(sG + r0 * LDG + c), gb = ld2(sG + r1 * LDG + c);
+      const float e00 = ex2(ga.x - gn.x), e01 = ex2(ga.y - gn.y), e10 = ex2(gb.x - gn.x), e11 = ex2(gb.y - gn.y);
+      const uint32_t k0 = *reinterpret_cast<const uint32_t*>(sK + r0 * LDH + c), k1 = *reinterpret_cast<const uint32_t*>(sK + r1 * LDH + c);
+      const uint32_t q0 = *reinterpret_cast<const uint32_t*>(sQ + r0 * LDH + c), q1 = *reinterpret_cast<const uint32_t*>(sQ + r1 * LDH + c);
+      AFrag<true> ak, aq;
+      ak.set(mma::lo_f(k0) * e00, mma::lo_f(k1) * e10, mma::hi_f(k0) * e01, mma::hi_f(k1) * e11);
+      aq.set(mma::lo_f(q0) * e00, mma::lo_f(q1) * e10, mma::hi_f(q0) * e01, mma::hi_f(q1) * e11);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        if (x < ntn && !(skip && nt0 + x >= 2 * mt)) {
+          const int j = 8 * (nt0 + x) + g;
+          const float2 gj = ld2(sG + j * LDG + c);
+          const uint32_t kj = *reinterpret_cast<const uint32_t*>(sK + j * LDH + c);
+          BFrag<true> bk;
+          bk.set(mma::lo_f(kj) * ex2(gn.x - gj.x), mma::hi_f(kj) * ex2(gn.y - gj.y));
+          fma<true>(dk[x], ak, bk);
+          fma<true>(dq[x], aq, bk);
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      if (x < ntn && !(skip && nt0 + x >= 2 * mt)) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 16 * mt + g + 8 * (e >> 1), j = 8 * (nt0 + x) + 2 * t + (e & 1);
+          sX[i * LDT + j] = j < i ? dk[x][e] * sRk[j] * sRk[i] : 0.f;
+          sA[i * 72 + j] = j <= i ? dq[x][e] * sRk[j] * sRq[i] : 0.f;
+        }
+      }
+    }
+  } else {
 #pragma unroll 1
-  for (int tile = warp; tile < 20; tile += kPreThreads / 32) {
+  for (int tile = warp; tile < 20; tile += kPreThreads / 32) {   // raw bf16 rows: exact products
     const int mt = tile < 2 ? 0 : tile < 6 ? 1 : tile < 12 ? 2 : 3, nt = tile - mt * (mt + 1);
     float dk[4], dq[4];
     zero4(dk); zero4(dq);
-    if constexpr (KDA) {
-      if (nt >= 2 * mt && unsafe(mt)) continue;   // done exactly below
-      const int r0 = 16 * mt + g, r1 = r0 + 8, j = 8 * nt + g, nrow = 16 * mt;
-#pragma unroll 2
-      for (int ks = 0; ks < 16; ++ks) {
-        const int c0 = 8 * ks + t, c1 = c0 + 4;
-        const float n0 = sG[nrow * 132 + c0], n1 = sG[nrow * 132 + c1];
-        const float e00 = ex2(sG[r0 * 132 + c0] - n0), e10 = ex2(sG[r1 * 132 + c0] - n0);
-        const float e01 = ex2(sG[r0 * 132 + c1] - n1), e11 = ex2(sG[r1 * 132 + c1] - n1);
-        AFrag<true> ak, aq;
-        ak.set(bf(sK + r0 * LDH + c0) * e00, bf(sK + r1 * LDH + c0) * e10, bf(sK + r0 * LDH + c1) * e01, bf(sK + r1 * LDH + c1) * e11);
-        aq.set(bf(sQ + r0 * LDH + c0) * e00, bf(sQ + r1 * LDH + c0) * e10, bf(sQ + r0 * LDH + c1) * e01, bf(sQ + r1 * LDH + c1) * e11);
-        BFrag<true> bk;
-        bk.set(bf(sK + j * LDH + c0) * ex2(n0 - sG[j * 132 + c0]), bf(sK + j * LDH + c1) * ex2(n1 - sG[j * 132 + c1]));
-        fma<true>(dk, ak, bk);
-        fma<true>(dq, aq, bk);
-      }
-    } else {   // raw bf16 rows: exact products
       const uint32_t aK = tc::smem_u32(sK), aQ = tc::smem_u32(sQ);
 #pragma unroll
       for (int k2 = 0; k2 < 4; ++k2) {
@@ -206,14 +253,14 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         mma::bf16(dk, a1, bb[2], bb[3]);
         mma::bf16(dq, q1, bb[2], bb[3]);
       }
-    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = 16 * mt + g + 8 * (e >> 1), j = 8 * nt + 2 * t + (e & 1);
-      const float f = KDA ? sRk[j] : sRk[j] * __expf(fminf(sGs[i] - sGs[j], 0.f));
+      const float f = sRk[j] * __expf(fminf(sGs[i] - sGs[j], 0.f));
       sX[i * LDT + j] = j < i ? dk[e] * f * sRk[i] : 0.f;
       sA[i * 72 + j] = j <= i ? dq[e] * f * sRq[i] : 0.f;
     }
+  }
   }
   if constexpr (KDA) {   // diagonal blocks with too wide a decay range: exactly, one entry per thread
     for (int blk = 0; blk < 4; ++blk) {
@@ -222,7 +269,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       float ak = 0.f, aq = 0.f;
       if (j <= i)
         for (int c = 0; c < kD; ++c) {
-          const float w = bf(sK + j * LDH + c) * ex2(fminf(sG[i * 132 + c] - sG[j * 132 + c], 0.f));
+          const float w = bf(sK + j * LDH + c) * ex2(fminf(sG[i * LDG + c] - sG[j * LDG + c], 0.f));
           ak += bf(sK + i * LDH + c) * w;
           aq += bf(sQ + i * LDH + c) * w;
         }
@@ -264,8 +311,8 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
     const int j0 = 8 * ks + t, j1 = j0 + 4;
     float a0 = bf(sK + j0 * LDH + ch0), a1 = bf(sK + j0 * LDH + ch1), a2 = bf(sK + j1 * LDH + ch0), a3 = bf(sK + j1 * LDH + ch1);
     if constexpr (KDA) {
-      a0 *= ex2(sG[j0 * 132 + ch0]); a1 *= ex2(sG[j0 * 132 + ch1]);
-      a2 *= ex2(sG[j1 * 132 + ch0]); a3 *= ex2(sG[j1 * 132 + ch1]);
+      a0 *= ex2(sG[j0 * LDG + ch0]); a1 *= ex2(sG[j0 * LDG + ch1]);
+      a2 *= ex2(sG[j1 * LDG + ch0]); a3 *= ex2(sG[j1 * LDG + ch1]);
     }
     AFrag<X3> a;
     a.set(a0, a1, a2, a3);
@@ -288,7 +335,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int ch = e < 2 ? ch0 : ch1, i = 8 * nt + 2 * t + (e & 1);
-        Y[nt][e] = bf(sQ + i * LDH + ch) * sRq[i] * (KDA ? ex2(sG[i * 132 + ch]) : expf(sGs[i]));
+        Y[nt][e] = bf(sQ + i * LDH + ch) * sRq[i] * (KDA ? ex2(sG[i * LDG + ch]) : expf(sGs[i]));
       }
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
@@ -311,20 +358,25 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   }
   // ---- N = -W^T Kd -> fragments -----------------------------------------------------------------------------------------------
   if constexpr (KDA) {
-    float4 kd[8];
-    const float4 gl = *reinterpret_cast<const float4*>(sG + 63 * 132 + 4 * lane);
+    // lane = channels lane, lane + 32, ..; warp = token pairs warp, warp + 8, ..; split into the two terms once
+    uint4 kd[4][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = warp + 8 * i;
-      const uint2 u = *reinterpret_cast<const uint2*>(sK + c * LDH + 4 * lane);
-      const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
-      const float r = sRk[c];
-      kd[i] = make_float4(mma::lo_f(u.x) * r * ex2(gl.x - gg.x), mma::hi_f(u.x) * r * ex2(gl.y - gg.y),
-                          mma::lo_f(u.y) * r * ex2(gl.z - gg.z), mma::hi_f(u.y) * r * ex2(gl.w - gg.w));
+    for (int x = 0; x < 4; ++x) {
+      const int c = lane + 32 * x;
+      const float gl = sG[63 * LDG + c];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 2 * (warp + 8 * i);
+        BFrag<true> f;
+        f.set(bf(sK + r * LDH + c) * sRk[r] * ex2(gl - sG[r * LDG + c]), bf(sK + (r + 1) * LDH + c) * sRk[r + 1] * ex2(gl - sG[(r + 1) * LDG + c]));
+        kd[i][x] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
+      }
     }
-    __syncthreads();   // every read of k and q is done
+    __syncthreads();   // every read of k, q, X and A is done
 #pragma unroll
-    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(sKd + (warp + 8 * i) * 132 + 4 * lane) = kd[i];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) sKd[(warp + 8 * i) * LDK + lane + 32 * x] = kd[i][x];
     __syncthreads();
   }
 #pragma unroll 1
@@ -342,8 +394,12 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       for (int nt = 0; nt < 8; ++nt) {
         const int c = 64 * half + 8 * nt + g;
         BFrag<X3> bk;
-        if constexpr (KDA) bk.set(sKd[i0 * 132 + c], sKd[(i0 + 1) * 132 + c]);
-        else bk.set(bf(sK + i0 * LDH + c), bf(sK + (i0 + 1) * LDH + c));
+        if constexpr (KDA) {
+          const uint4 y = sKd[(4 * ks + t) * LDK + c];
+          bk.h[0] = y.x; bk.h[1] = y.y; bk.l[0] = y.z; bk.l[1] = y.w;
+        } else {
+          bk.set(bf(sK + i0 * LDH + c), bf(sK + (i0 + 1) * LDH + c));
+        }
         fma<X3>(d[nt], a, bk);
       }
     }

@@ -79,11 +79,11 @@ __device__ __forceinline__ void fma_b1(float (&d)[4], const AFrag<X3>& a, const 
   tf32(d, a.h, b.h);
 }
 
-// In-place inclusive prefix sum over the 64 rows of sG [64][D + 4] per channel; NTHR threads, `seg`: scratch of
+// In-place inclusive prefix sum over the 64 rows of sG [64][LD] per channel; NTHR threads, `seg`: scratch of
 // NTHR / (D / 4) rows of D floats.  Ends with a barrier.
-template <int NTHR, int D>
+template <int NTHR, int D, int LD = D + 4>
 __device__ __forceinline__ void scan_channels(float* sG, float* seg, int tid) {
-  constexpr int LD = D + 4, NSEG = NTHR / (D / 4), R = 64 / NSEG;   // rows per segment
+  constexpr int NSEG = NTHR / (D / 4), R = 64 / NSEG;   // rows per segment
   const int s = tid / (D / 4), c4 = 4 * (tid % (D / 4));
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), loc[R];
 #pragma unroll
