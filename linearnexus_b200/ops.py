@@ -318,7 +318,9 @@ _VARIANTS = {"delta": DR_DELTA, "gated": DR_GATED, "kda": DR_KDA}
 
 
 def _train_prep(variant, q, k, v, g, beta, initial_state, scale, chunk_size, use_qk_l2norm, out_dtype=None):
-    """Common argument handling of the backward-related entry points ([B,H,T,D] contiguous copies)."""
+    """Common argument handling of the backward-related entry points.  Token-major views are read in place, as the forward
+    does (copying them cost up to a quarter of a training step, in the forward and again in the backward); anything else
+    becomes [B,H,T,D] contiguous copies."""
     var = _VARIANTS[variant]
     B, Hq, T, K = q.shape
     H, V = v.shape[1], v.shape[-1]   # Hq < H: grouped value attention (dq, dk come back summed over each group)
@@ -331,11 +333,10 @@ def _train_prep(variant, q, k, v, g, beta, initial_state, scale, chunk_size, use
         beta = beta.squeeze(-1)
     dev = q.device
     common = torch.float32 if any(t.dtype not in _NATIVE for t in (q, k, v)) or len({q.dtype, k.dtype, v.dtype}) > 1 else q.dtype
-    qn, kn, vn = (t.to(common).contiguous() for t in (q, k, v))
-    gn = None if g is None else _native(g).contiguous()
-    bn = beta.to(torch.float32).contiguous()
+    layout, (qn, kn, vn, gn, bn) = _layout([q.to(common), k.to(common), v.to(common), None if g is None else _native(g),
+                                            beta.to(torch.float32)])
     h0 = _state(initial_state, B, H, K, V, dev)
-    d = _desc(var, DR_LAYOUT_BHTD, B, H, T, K, V, chunk_size, qn, gn, common if out_dtype is None else out_dtype,
+    d = _desc(var, layout, B, H, T, K, V, chunk_size, qn, gn, common if out_dtype is None else out_dtype,
               use_qk_l2norm, scale)
     d.qk_heads = Hq
     lib = _lib.load()
@@ -358,7 +359,7 @@ def chunk_forward_saving(variant, q, k, v, g, beta, initial_state=None, scale=No
     d, lib, need, (qn, kn, vn, gn, bn, h0), (B, H, T, K, V, dev, common) = _train_prep(
         variant, q, k, v, g, beta, initial_state, scale, chunk_size, use_qk_l2norm, native_out)
     ws = torch.empty(need, dtype=torch.uint8, device=dev)
-    o = torch.empty((B, H, T, V), dtype=native_out, device=dev)
+    o = torch.empty_like(vn, dtype=native_out)   # (keeps a token-major layout)
     hT = torch.empty((B, H, K, V), dtype=torch.float32, device=dev)
     with torch.cuda.device(dev):
         st = lib.dr_chunk_fwd_saving(ctypes.byref(d), _ptr(qn), _ptr(kn), _ptr(vn), _ptr(gn), _ptr(bn), _ptr(h0),
@@ -378,14 +379,18 @@ def chunk_backward(variant, q, k, v, g, beta, d_o, initial_state=None, d_final_s
     _require_cuda(q, k, v, g, beta, d_o, initial_state, d_final_state)
     d, lib, need, (qn, kn, vn, gn, bn, h0), (B, H, T, K, V, dev, common) = _train_prep(
         variant, q, k, v, g, beta, initial_state, scale, chunk_size, use_qk_l2norm)
-    don = d_o.to(common).contiguous()
+    don = d_o.to(common)
+    if d.layout == DR_LAYOUT_BTHD:
+        don = don.transpose(1, 2).contiguous().transpose(1, 2)
+    else:
+        don = don.contiguous()
     dhT = _state(d_final_state, B, H, K, V, dev)
     if saved is not None and (saved.numel() < need or saved.device != dev or saved.dtype != torch.uint8):
         raise ValueError("saved must be the workspace returned by chunk_forward_saving for the same shapes")
     ws = torch.empty(need, dtype=torch.uint8, device=dev) if saved is None else saved
     dq, dk, dv = torch.empty_like(qn), torch.empty_like(kn), torch.empty_like(vn)
-    dbeta = torch.empty((B, H, T), dtype=torch.float32, device=dev)
-    dg = None if g is None else torch.empty(gn.shape, dtype=torch.float32, device=dev)
+    dbeta = torch.empty_like(bn)
+    dg = None if g is None else torch.empty_like(gn, dtype=torch.float32)
     dh0 = torch.empty((B, H, K, V), dtype=torch.float32, device=dev)
     with torch.cuda.device(dev):
         if saved is None:
@@ -424,6 +429,7 @@ class _ChunkFn(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, g if g is not None else q.new_empty(0), beta,
                               initial_state if initial_state is not None else q.new_empty(0))
         ctx.saved_ws = saved
+        ctx.set_materialize_grads(False)   # no zeros for a final state that the loss does not read
         ctx.meta = (variant, scale, chunk_size, l2norm, g is not None, initial_state is not None)
         return o, hT
 
@@ -436,6 +442,8 @@ class _ChunkFn(torch.autograd.Function):
                 f"the backward kernels cover chunk_size <= 64 and K <= 128 (K % 16 == 0 for 'kda'); got chunk_size="
                 f"{chunk_size}, K={q.shape[-1]}.  The forward of this shape is available (this call ran it).")
         saved, ctx.saved_ws = ctx.saved_ws, None   # consumed: a second backward recomputes
+        if d_o is None:
+            d_o = torch.zeros_like(v)
         gr = chunk_backward(variant, q, k, v, g if has_g else None, beta, d_o, h0 if has_h0 else None, d_hT,
                             scale=scale, chunk_size=chunk_size, use_qk_l2norm=l2norm, saved=saved)
         dg = gr["dg"].to(g.dtype) if has_g else None
