@@ -43,6 +43,8 @@ struct Api {
   decltype(&dr_dplr_recurrent) dplr_recurrent;
   decltype(&dr_rwkv6_recurrent) rwkv6_recurrent;
   decltype(&dr_ssd_scan) ssd_scan;
+  decltype(&dr_chunk_fwd_saving) chunk_fwd_saving;
+  decltype(&dr_chunk_bwd_saved) chunk_bwd_saved;
 } api;
 bool g_open = false;
 
@@ -269,6 +271,109 @@ PyObject* py_sequence(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     if (st < 0) return PyLong_FromLong(st);
     return pair(o, hT);
+  });
+}
+
+// What the two halves of a training step share: the inputs and their descriptor.
+struct Training {
+  Call c;
+  const at::Tensor *q, *k, *v, *g, *beta;
+  int64_t B, Hq, T, K, H, V;
+  int dt, layout;
+  DrDesc d;
+  // a: variant, q, k, v, g, beta; out < 0: the inputs' storage type
+  Training(PyObject* const* a, PyObject* scale_arg, PyObject* chunk, PyObject* l2norm, int out) {
+    const int variant = (int)as_int(a[0]);
+    q = &c.req(a[1]); k = &c.req(a[2]); v = &c.req(a[3]); g = c.opt(a[4]); beta = &c.req(a[5]);
+    need(q->dim() == 4 && v->dim() == 4 && k->sizes().equals(q->sizes()));
+    B = q->size(0); Hq = q->size(1); T = q->size(2); K = q->size(3); H = v->size(1); V = v->size(3);
+    need(v->size(0) == B && v->size(2) == T && Hq > 0 && H % Hq == 0 && is_shape(*beta, {B, H, T}) && beta->scalar_type() == at::kFloat);
+    dt = qkv_dtype(*q, *k, *v);
+    need((g != nullptr) == (variant != DR_DELTA));
+    int g_dt = DR_F32;
+    if (g) {
+      need(variant == DR_GATED ? is_shape(*g, {B, H, T}) : is_shape(*g, {B, H, T, K}));
+      g_dt = dtype_code(*g);
+    }
+    layout = common_layout({q, k, v, g, beta});
+    need(layout == DR_LAYOUT_BHTD || (Hq > 1 && T > 1));
+    const double scale = scale_arg == Py_None ? 1.0 / std::sqrt((double)K) : as_double(scale_arg);
+    d = make_desc(variant, layout, B, H, T, K, V, as_int(chunk), dt, g_dt, out < 0 ? dt : out, l2norm == Py_True, scale, 0, Hq);
+    need(!PyErr_Occurred());
+  }
+  bool laid_out(const at::Tensor& t) const { return layout == DR_LAYOUT_BHTD ? t.is_contiguous() : is_bthd_view(t); }
+  at::Tensor like(const at::Tensor& t, at::ScalarType st) const { return c.empty_strided(t.sizes(), t.strides(), st); }
+};
+
+// train_fwd(variant, q, k, v, g, beta, h0, scale, chunk, l2norm, out_dtype) -> (o, hT, workspace) | status | None
+PyObject* py_train_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n == 11);
+    const long out = as_int(a[10]);
+    need(out >= 0 && out <= DR_BF16);
+    Training t(a, a[7], a[8], a[9], (int)out);
+    const at::Tensor* h0 = t.c.opt(a[6]);
+    if (h0) { need(is_shape(*h0, {t.B, t.H, t.K, t.V})); need_f32(h0); }
+    const int64_t ws_bytes = api.workspace_bytes(&t.d, 1);
+    if (ws_bytes < 0) return PyLong_FromLong((long)ws_bytes);
+    const at::Tensor ws = t.c.empty({ws_bytes}, at::kByte);
+    const at::Tensor o = sequence_out(t.c, t.layout, t.B, t.H, t.T, t.V, scalar_type((int)out));
+    const at::Tensor hT = t.c.empty({t.B, t.H, t.K, t.V}, at::kFloat);
+    void* stream = t.c.stream();
+    int st;
+    {
+      Unlocked u;
+      st = api.chunk_fwd_saving(&t.d, ptr(*t.q), ptr(*t.k), ptr(*t.v), ptr(t.g), fptr(t.beta), fptr(h0), o.mutable_data_ptr(), fmut(hT),
+                                ws.mutable_data_ptr(), (size_t)ws_bytes, t.c.status(), stream);
+    }
+    if (st < 0) return PyLong_FromLong(st);
+    PyObject* r = PyTuple_New(3);
+    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(o));
+    PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(hT));
+    PyTuple_SET_ITEM(r, 2, THPVariable_Wrap(ws));
+    return r;
+  });
+}
+
+// train_bwd(variant, q, k, v, g, beta, d_o, d_hT, scale, chunk, l2norm, workspace) -> (dq, dk, dv, dg, dbeta, dh0) | status | None
+PyObject* py_train_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n == 12);
+    Training t(a, a[8], a[9], a[10], -1);
+    const at::Tensor &given = t.c.req(a[6]), &ws = t.c.req(a[11]);
+    const at::Tensor* d_hT = t.c.opt(a[7]);
+    need(is_shape(given, {t.B, t.H, t.T, t.V}) && t.laid_out(given));
+    if (d_hT) { need(is_shape(*d_hT, {t.B, t.H, t.K, t.V})); need_f32(d_hT); }
+    const int64_t ws_bytes = api.workspace_bytes(&t.d, 1);
+    if (ws_bytes < 0) return PyLong_FromLong((long)ws_bytes);
+    need(ws.scalar_type() == at::kByte && ws.is_contiguous() && ws.numel() >= ws_bytes);
+    const at::Tensor d_o = given.to(t.q->scalar_type());   // (keeps the layout; KDA's output is float32)
+    const at::Tensor dq = t.like(*t.q, t.q->scalar_type()), dk = t.like(*t.k, t.q->scalar_type()), dv = t.like(*t.v, t.q->scalar_type());
+    const at::Tensor dbeta = t.like(*t.beta, at::kFloat), dh0 = t.c.empty({t.B, t.H, t.K, t.V}, at::kFloat);
+    at::Tensor dg;
+    if (t.g) dg = t.like(*t.g, at::kFloat);
+    void* stream = t.c.stream();
+    int st;
+    {
+      Unlocked u;
+      st = api.chunk_bwd_saved(&t.d, ptr(*t.q), ptr(*t.k), ptr(*t.v), ptr(t.g), fptr(t.beta), ptr(d_o), fptr(d_hT), dq.mutable_data_ptr(),
+                               dk.mutable_data_ptr(), dv.mutable_data_ptr(), fmut(dbeta), t.g ? fmut(dg) : nullptr, fmut(dh0),
+                               ws.mutable_data_ptr(), (size_t)ws.numel(), t.c.status(), stream);
+    }
+    if (st < 0) return PyLong_FromLong(st);
+    PyObject* r = PyTuple_New(6);
+    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(dq));
+    PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(dk));
+    PyTuple_SET_ITEM(r, 2, THPVariable_Wrap(dv));
+    if (t.g) {
+      PyTuple_SET_ITEM(r, 3, THPVariable_Wrap(dg));
+    } else {
+      Py_INCREF(Py_None);
+      PyTuple_SET_ITEM(r, 3, Py_None);
+    }
+    PyTuple_SET_ITEM(r, 4, THPVariable_Wrap(dbeta));
+    PyTuple_SET_ITEM(r, 5, THPVariable_Wrap(dh0));
+    return r;
   });
 }
 
@@ -537,6 +642,8 @@ PyObject* py_open(PyObject*, PyObject* arg) {
   DR_SYM(dplr_recurrent, "dr_dplr_recurrent")
   DR_SYM(rwkv6_recurrent, "dr_rwkv6_recurrent")
   DR_SYM(ssd_scan, "dr_ssd_scan")
+  DR_SYM(chunk_fwd_saving, "dr_chunk_fwd_saving")
+  DR_SYM(chunk_bwd_saved, "dr_chunk_bwd_saved")
 #undef DR_SYM
   g_open = true;
   Py_RETURN_NONE;
@@ -555,7 +662,7 @@ PyObject* py_set_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define DR_FN(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"open", py_open, METH_O, nullptr}, DR_FN(set_status), DR_FN(step), DR_FN(sequence), DR_FN(packed), DR_FN(conv), DR_FN(gates),
-    DR_FN(norm), DR_FN(scan), DR_FN(ssd), {nullptr, nullptr, 0, nullptr}};
+    DR_FN(norm), DR_FN(scan), DR_FN(ssd), DR_FN(train_fwd), DR_FN(train_bwd), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

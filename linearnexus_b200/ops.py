@@ -352,9 +352,14 @@ def chunk_forward_saving(variant, q, k, v, g, beta, initial_state=None, scale=No
     """The chunkwise forward of a training step: returns ``(o, final_state, saved)`` where ``saved`` is the
     backward workspace holding the state at the start of every chunk; pass it to ``chunk_backward(..., saved=)``
     so that the backward does not recompute the forward."""
-    _require_cuda(q, k, v, g, beta, initial_state)
     if out_dtype is None:
         out_dtype = torch.float32 if variant == "kda" else q.dtype
+    if variant in _VARIANTS:
+        r = _native_calls().train_fwd(_VARIANTS[variant], q, k, v, g, beta, initial_state, scale, chunk_size, bool(use_qk_l2norm),
+                                      _NATIVE.get(out_dtype, -1))
+        if r.__class__ is tuple:
+            return r
+    _require_cuda(q, k, v, g, beta, initial_state)
     native_out = out_dtype if out_dtype in _NATIVE else torch.float32
     d, lib, need, (qn, kn, vn, gn, bn, h0), (B, H, T, K, V, dev, common) = _train_prep(
         variant, q, k, v, g, beta, initial_state, scale, chunk_size, use_qk_l2norm, native_out)
@@ -376,6 +381,11 @@ def chunk_backward(variant, q, k, v, g, beta, d_o, initial_state=None, d_final_s
     dbeta float32 [B,H,T]; dg float32 [like g] (None for "delta"); dh0 float32 [B,H,K,V].
     ``saved``: the third result of ``chunk_forward_saving`` on the same inputs (skips the forward recomputation;
     the buffer is consumed)."""
+    if saved is not None and variant in _VARIANTS:
+        r = _native_calls().train_bwd(_VARIANTS[variant], q, k, v, g, beta, d_o, d_final_state, scale, chunk_size,
+                                      bool(use_qk_l2norm), saved)
+        if r.__class__ is tuple:
+            return dict(zip(("dq", "dk", "dv", "dg", "dbeta", "dh0"), r))
     _require_cuda(q, k, v, g, beta, d_o, initial_state, d_final_state)
     d, lib, need, (qn, kn, vn, gn, bn, h0), (B, H, T, K, V, dev, common) = _train_prep(
         variant, q, k, v, g, beta, initial_state, scale, chunk_size, use_qk_l2norm)
