@@ -127,7 +127,8 @@ int resolve_chunk_path(const DrDesc* d) {
 //    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave and there are chunks
 //    enough to pay for the longer first pass (measured for 4, 8, 16 sequences: even at 5 chunks, 118 vs 90 us at 16 x 32
 //    chunks, 228 vs 80 us at 4 x 64; at 32 sequences the one-CTA kernels are ahead).  KDA switches from 17 chunks on: up to
-//    there its two-kernel form, what AUTO has always meant for it, is at most 15 us behind.
+//    there its two-kernel form, what AUTO has always meant for it, is at most 15 us behind.  Past 32 chunks the two-kernel form
+//    overtakes it earlier (both first passes fill the chip then; 16 x 128 chunks: 340 against 357 us, 8 x 128: 292 against 267).
 // Both up to 1 GB of scratch.
 bool trans_eligible(const DrDesc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
 int64_t trans_scratch(const DrDesc* d) {
@@ -137,7 +138,8 @@ int64_t trans_scratch(const DrDesc* d) {
   if (d->path == DR_PATH_TRANSITION) return need;
   if (d->path != DR_PATH_AUTO || need > (int64_t)1 << 30) return 0;
   if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d)) return d->T > 64 ? need : 0;
-  return units <= 18 && d->T > (d->variant == DR_KDA ? 16 : 5) * 64 ? need : 0;
+  const bool kda = d->variant == DR_KDA;
+  return units <= (kda && d->T > 32 * 64 ? 12 : 18) && d->T > (kda ? 16 : 5) * 64 ? need : 0;
 }
 
 bool fp32_chunk_eligible(const DrDesc* d) { return d->chunk <= 64 && d->K <= 128; }
