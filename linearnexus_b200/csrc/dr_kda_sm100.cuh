@@ -98,6 +98,8 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   return d;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // packed pairs: one instruction per two products
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   float2 d;
@@ -151,6 +153,7 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
 struct IntraParams {
   FwdParams p;
   uint8_t* ws;
+  int resident;   // CTAs that run at a time
 };
 struct IntraPackedParams : IntraParams {
   SeqTable seqs;
@@ -272,6 +275,22 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
       *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kraw[i];
       *reinterpret_cast<float4*>(sG + c * LDF + 4 * lane) =
           make_float4(gv[i][0] * kLog2e, gv[i][1] * kLog2e, gv[i][2] * kLog2e, gv[i][3] * kLog2e);
+    }
+    if constexpr (!kPacked && !kTrans) {
+      // the rows of the chunk that follows in this CTA's place, into L2 (thread = a quarter of a row): 1090 -> 1081 us at B=4 T=8192 H=32
+      const int64_t nb = (int64_t)blockIdx.x + P.resident;
+      if (nb < gridDim.x) {
+        const int nchunks = (T + kC - 1) / kC, u2 = (int)(nb / nchunks), tok = ((int)nb - u2 * nchunks) * kC + (tid >> 2);
+        if (tok < T) {
+          const int b2 = u2 / p.map.H, h2 = u2 - b2 * p.map.H;
+          prefetch_l2(reinterpret_cast<const __nv_bfloat16*>((tid & 2) ? p.k : p.q) + p.map.base_qk(b2, h2, kD) + (int64_t)tok * qk_tok + (tid & 1) * 64);
+          if (p.variant == DR_KDA) {
+            const int64_t at = p.map.base(b2, h2, kD) + (int64_t)tok * gk_tok + (tid & 3) * 32;
+            if (p.g_dt == DR_F32) prefetch_l2(reinterpret_cast<const float*>(p.g) + at);
+            else if (!(tid & 1)) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.g) + at);
+          }
+        }
+      }
     }
     // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced (16 shuffles instead of
     // 80), so that each lane takes one square root and one quotient (as every lane did for every row, a fifth of the pass)
@@ -1157,11 +1176,13 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
 template <class IP, class SP>
 inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace, int64_t chunk_units, int64_t units, cudaStream_t stream,
                                cudaEvent_t after_intra = nullptr) {
-  thread_local int attr_dev = -1;
+  thread_local int attr_dev = -1, sms = 0;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (attr_dev != dev) {
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(intra_kernel<IP>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(state_kernel<SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_TOTAL);
@@ -1171,6 +1192,7 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   I.p = p;
   S.p = p;
   S.ws = I.ws = reinterpret_cast<uint8_t*>(workspace);
+  I.resident = 2 * sms;
   if (!sm100::make_panel_map(&S.tv, p.v, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
   e = launch_pdl(intra_kernel<IP>, dim3((unsigned)chunk_units), dim3(kThreads), IN_TOTAL, stream, I);
   if (e != cudaSuccess) return e;
