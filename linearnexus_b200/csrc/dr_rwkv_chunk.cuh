@@ -16,7 +16,8 @@
 //
 // What bounds it: the chain of a block through the dots, U and the update, 2.6 K cycles with the schedulers 55 % and the tensor pipe 35 %
 // busy (B=8, T=4096, H=16: 868 us with four warps of 64 keys and products in source order, 820 with them free to move, 785
-// with eight warps, 761 with the B operands split once by the staging warps; two staging groups instead of three: 872).
+// with eight warps, 761 with the B operands split once by the staging warps; two staging groups instead of three: 872; 690 with
+// running products in blocks of too strong a decay).
 // The token recurrence it replaces here ran
 // at 540 cycles per token whatever its instruction count or prefetch depth: one dependent reduce-and-update chain per token, and
 // 260 shared-memory wavefronts per token to feed 160 multiply-adds per thread (a 16-byte load fills a quarter of a warp per
@@ -213,28 +214,46 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
       }
       sync128();
       // ---- coefficients: rows q (and a) against k / W (warp 0) and b / W (warp 1) ----------------------------------------------------
-      if (X.wide) {   // too strong a decay: every pair with the decays in between multiplied up (four lanes per pair)
-        const int which = warp & 1;
-        if (LR || which == 0)
-          for (int e = (warp >> 1) * 32 + lane; e < 64 * 2 * 2; e += 64) {
-            const int half = e & 1, pair = (e >> 1) & 63, i = pair >> 3, j = pair & 7, isa = e >> 7;
-            float acc = 0.f;
-            if ((LR || !isa) && (isa || !LR ? j < i : j <= i) && t0 + i < T) {
-              for (int c = 32 * half; c < 32 * half + 32; ++c) {
-                float x = raw(slot, which ? 4 : 1, j, c);
-                const int hi = isa || !LR ? i - 1 : i;   // a reads the state before token i's decay; so does RWKV-6
-                for (int m = j + 1; m <= hi; ++m) { const float d = raw(slot, 2, m, c); x *= LR ? expf(d) : expf(-expf(d)); }
-                float q = raw(slot, isa ? 3 : 0, i, c);
-                if (!isa) q = LR ? q * p.scale : p.scale / (1.f + __expf(-q));
-                acc += q * x;
-              }
-            }
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            if (!half) {
-              if (isa) (which ? X.ab : X.ak)[pair] = acc;
-              else put(which ? S.qb : S.qk, i, j, acc);
+      if (X.wide) {
+        // too strong a decay: the decays between two tokens multiplied up.  Four lanes per (row kind, vector kind, j), sixteen channels
+        // each, the product running over i (with every pair on its own, and its exponentials, such a block took 35 us)
+        if (role == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {   // the decays take the place of k / W_j, which is not used
+            const float x = raw(slot, 2, i, ch);
+            X.inv[i][ch] = t0 + i < T ? (LR ? expf(x) : expf(-expf(x))) : 1.f;
+          }
+        }
+        sync128();
+        const int item = tid >> 2, isa = item >> 4, which = (item >> 3) & 1, j = item & 7;
+        if (LR || item < 8) {
+          const bool incl = LR && !isa;   // q reads the state after token i's decay; a (and RWKV-6) the one before
+          float acc[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+          for (int c = tid & 3; c < kK; c += 4) {
+            float x = raw(slot, which ? 4 : 1, j, c);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float w = i > j ? X.inv[i][c] : 1.f;
+              if (incl) x *= w;
+              float q = raw(slot, isa ? 3 : 0, i, c);
+              if (!isa) q = LR ? q * p.scale : p.scale / (1.f + __expf(-q));
+              acc[i] += q * x;
+              if (!incl) x *= w;
             }
           }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 1);
+            acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 2);
+            if ((tid & 3) == 0) {
+              const float v = (incl ? i >= j : i > j) && t0 + i < T ? acc[i] : 0.f;
+              if (isa) (which ? X.ab : X.ak)[8 * i + j] = v;
+              else put(which ? S.qb : S.qk, i, j, v);
+            }
+          }
+        }
       } else if (warp < (LR ? 2 : 1)) {
         float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -413,7 +432,10 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 }
 
 // 16-byte-aligned rows of K = 64 and whole 64-column slices; a decode step (one or two blocks) stays with the token kernel
-inline bool eligible(int kind, bool bf, const LinRecParams& p) {
+// RWKV-6 has no reduction on its token chain, and with more sequences than SMs the token recurrence, whose CTAs share an SM, stays
+// level or ahead (256 sequences: 747 against 759 us at T = 2048, 194 against 198 at 512); RWKV-7 gains there, too (887 against 754).
+inline bool eligible(int kind, bool bf, const LinRecParams& p, int sms) {
+  if (kind != LR_DPLR && (int64_t)p.B * p.H * (p.V / 64) > sms) return false;
   const int ep = bf ? 8 : 4;
   auto ok = [&](const LrVec& v) { return (reinterpret_cast<uintptr_t>(v.p) & 15) == 0 && v.sb % ep == 0 && v.sh % ep == 0 && v.st % ep == 0; };
   return p.K == kK && p.V % 64 == 0 && p.T > kTB && p.s_v == 1 && ok(p.q) && ok(p.k) && ok(p.w) && ok(p.v) &&
