@@ -122,7 +122,8 @@ int resolve_chunk_path(const DrDesc* d) {
 
 // Shapes of the transition form, and its scratch where AUTO takes it (given that scratch); 0 elsewhere.
 //  * No tensor-core kernel for the storage types: in place of the token recurrence from two chunks on (with one chunk there is
-//    nothing to run in parallel).
+//    nothing to run in parallel).  DeltaNet's recurrence, without a decay per token, stays ahead up to half of the second
+//    chunk at K = V = 128 (32 sequences, T = 65: 34 against 44 us; T = 130: 57 against 49).
 //  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.6 us per chunk, KDA's state
 //    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave and there are chunks
 //    enough to pay for the longer first pass (measured for 4, 8, 16 sequences: even at 5 chunks, 118 vs 90 us at 16 x 32
@@ -137,7 +138,8 @@ int64_t trans_scratch(const DrDesc* d) {
   const int64_t need = dr::trans_workspace_bytes(units, d->T, d->K, split_eligible(d));
   if (d->path == DR_PATH_TRANSITION) return need;
   if (d->path != DR_PATH_AUTO || need > (int64_t)1 << 30) return 0;
-  if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d)) return d->T > 64 ? need : 0;
+  if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d))
+    return d->T > (d->variant == DR_DELTA && d->K == 128 ? 96 : 64) ? need : 0;
   const bool kda = d->variant == DR_KDA;
   return units <= (kda && d->T > 32 * 64 ? 12 : 18) && d->T > (kda ? 16 : 5) * 64 ? need : 0;
 }
