@@ -12,7 +12,8 @@
 // exchange their partial dots).  An accumulator is, register for register, an A operand whose contraction runs over its columns: h
 // feeds the dots, their result feeds T, U feeds the update, and nothing of the state touches memory.  Three groups of four warps
 // stage the blocks ahead, one block in three each: raw rows from a ring of asynchronous copies, decay products, the row vectors and
-// the 8 x 8 coefficients.  Hand-overs are named barriers, arrived on by one side and waited for by the other.
+// the 8 x 8 coefficients.  A filled stage is handed over by a named barrier, arrived on by its group and waited for by the state's
+// warps; an emptied one by an mbarrier (see kEmptyTries).
 //
 // What bounds it: the chain of a block through the dots, U and the update, 2.6 K cycles with the schedulers 55 % and the tensor pipe 35 %
 // busy (B=8, T=4096, H=16: 868 us with four warps of 64 keys and products in source order, 820 with them free to move, 785
@@ -26,6 +27,7 @@
 
 #include "dr_linrec.cuh"
 #include "dr_mma.cuh"
+#include "dr_sm100_common.cuh"
 #include "dr_tcgen05.cuh"
 #include "dr_tf32.cuh"
 
@@ -86,12 +88,21 @@ struct Scratch {            // of one staging group
   int wide;
 };
 template <int KIND, bool BF>
-constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * ((int)sizeof(Scratch) + kRing * Ring<KIND, BF>::kSlot) + 64; }
+constexpr int group_bytes() { return ((int)sizeof(Scratch) + 15) / 16 * 16 + kRing * Ring<KIND, BF>::kSlot; }
+template <int KIND, bool BF>
+constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * group_bytes<KIND, BF>() + kStages * 8; }
+static_assert(smem_bytes<LR_DPLR, false>() <= 232448, "227 KB per CTA");
 
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-constexpr int kBarFull = 1, kBarEmpty = 1 + kStages, kBarGroup = 1 + 2 * kStages, kBarPair = kBarGroup + kGroups;
+constexpr int kBarFull = 1, kBarGroup = 1 + kStages, kBarPair = kBarGroup + kGroups;
 static_assert(kBarPair + 4 <= 16, "named barriers");
+// A stage passes from group to group (kStages is no multiple of kGroups), so "the consumers have left stage s for the n-th time" is
+// phase n of an mbarrier: a named barrier has no phases, and two groups would meet on it in either order.  The group of block blk
+// waits for phase blk / kStages - 1.  It cannot be a phase behind (phase blk / kStages needs blk staged first), nor a phase ahead:
+// its last block, blk - kGroups, was staged after every warp had left blk - kGroups - kStages, so after it had arrived for the phase
+// before.
+constexpr uint32_t kEmptyTries = 1u << 20;   // and about a second of clock
 
 // a float32-precise product whose terms go to three accumulators (hi hi, lo hi, hi lo)
 __device__ __forceinline__ void fma3(float (&d)[3][4], const AFrag<true>& a, const BFrag<true>& b) {
@@ -112,12 +123,17 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nvs = p.V / 64, unit = blockIdx.x / nvs, v0 = (blockIdx.x % nvs) * 64;
   const int b = unit / p.H, h = unit % p.H, T = p.T, nblk = (T + kTB - 1) / kTB;
+  const uint32_t empty = tc::smem_u32(smem + smem_bytes<KIND, BF>() - kStages * 8);   // one mbarrier per stage
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) tc::mbar_init(empty + 8 * i, kCons / 32);
+    tc::fence_mbar_init();
+  }
+  __syncthreads();
 
   if (threadIdx.x >= kCons) {
     // =========================== staging =========================================================================================
     const int grp = (threadIdx.x - kCons) >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
-    constexpr int kGrpBytes = (sizeof(Scratch) + 15) / 16 * 16 + kRing * R::kSlot;
-    uint8_t* mine = smem + kStages * sizeof(Stage) + sizeof(Exchange) + grp * kGrpBytes;
+    uint8_t* mine = smem + kStages * sizeof(Stage) + sizeof(Exchange) + grp * group_bytes<KIND, BF>();
     Scratch& X = *reinterpret_cast<Scratch*>(mine);
     uint8_t* ring = mine + (sizeof(Scratch) + 15) / 16 * 16;
     constexpr int kRounds = (R::kTasks + 3) / 4;
@@ -161,8 +177,12 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     for (int i = 0; i < kRing; ++i) issue(grp + kGroups * i);
     for (int blk = grp; blk < nblk; blk += kGroups) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
-      if (tid == 0) X.wide = 0;
-      if (blk >= kStages) bar_sync(kBarEmpty + blk % kStages, kHand);   // the consumers have left this stage
+      if (tid == 0) {
+        X.wide = 0;
+        if (blk >= kStages &&   // the consumers have left this stage
+            !tc::mbar_wait_compact(empty + 8 * (blk % kStages), (blk / kStages - 1) & 1, kEmptyTries) && p.status)
+          atomicOr(p.status, DR_DEV_TIMEOUT);
+      }
       sync128();   // every thread's pieces of this block have landed
       const uint8_t* slot = ring + (blk / kGroups % kRing) * R::kSlot;
       Stage& S = s_st[blk % kStages];
@@ -413,7 +433,8 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
       }
       if (out) mma::fma<true>(o, au, small(St.qb));
     }
-    if (blk + kStages < nblk) bar_arrive(kBarEmpty + blk % kStages, kHand);
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive(empty + 8 * (blk % kStages));
     if (out) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
