@@ -16,12 +16,14 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdint>
+#include <exception>
 #include <vector>
 
 #include "deltarule_sm100.h"
@@ -162,7 +164,8 @@ DrDesc make_desc(int variant, int layout, int64_t B, int64_t H, int64_t T, int64
   return d;
 }
 
-// Runs `f` (which returns a new reference) and turns "not the plain case" into None, C++ errors into Python ones.
+// Runs `f` (which returns a new reference) and turns "not the plain case" into None, C++ errors into the Python exceptions that
+// torch's own functions raise for them (an allocation that does not fit: torch.OutOfMemoryError, which callers catch).
 template <class F>
 PyObject* guarded(F f) {
   try {
@@ -172,8 +175,8 @@ PyObject* guarded(F f) {
   } catch (const NotPlain&) {
     if (PyErr_Occurred()) PyErr_Clear();   // an argument of another type: the Python path reports it
     Py_RETURN_NONE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
 }
