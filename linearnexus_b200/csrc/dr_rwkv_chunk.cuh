@@ -88,10 +88,12 @@ struct Scratch {            // of one staging group
   int wide;
 };
 template <int KIND, bool BF>
-constexpr int group_bytes() { return ((int)sizeof(Scratch) + 15) / 16 * 16 + kRing * Ring<KIND, BF>::kSlot; }
+constexpr int kGroupBytes = ((int)sizeof(Scratch) + 15) / 16 * 16 + kRing * Ring<KIND, BF>::kSlot;
+template <int KIND, bool BF>   // then one mbarrier per stage
+constexpr int kEmptyAt = kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * kGroupBytes<KIND, BF>;
 template <int KIND, bool BF>
-constexpr int smem_bytes() { return kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * group_bytes<KIND, BF>() + kStages * 8; }
-static_assert(smem_bytes<LR_DPLR, false>() <= 232448, "227 KB per CTA");
+constexpr int kSmemBytes = kEmptyAt<KIND, BF> + kStages * 8;
+static_assert(kEmptyAt<LR_DPLR, false> % 8 == 0 && kSmemBytes<LR_DPLR, false> <= 232448, "227 KB per CTA");
 
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
@@ -102,6 +104,9 @@ static_assert(kBarPair + 4 <= 16, "named barriers");
 // waits for phase blk / kStages - 1.  It cannot be a phase behind (phase blk / kStages needs blk staged first), nor a phase ahead:
 // its last block, blk - kGroups, was staged after every warp had left blk - kGroups - kStages, so after it had arrived for the phase
 // before.
+// Measured against the named barriers it replaces (which could be passed out of order): RWKV-7 B=8, T=4096, H=16 685 -> 681 us, B=1,
+// T=2048, H=8 345 -> 342; RWKV-6 B=4, T=2048, H=16 380 -> 386.  Every thread of the group waits: one waiting for the others took
+// 2.2 % more.  Three stages, each of one group, with named barriers: 710, 356, 430.
 constexpr uint32_t kEmptyTries = 1u << 20;   // and about a second of clock
 
 // a float32-precise product whose terms go to three accumulators (hi hi, lo hi, hi lo)
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nvs = p.V / 64, unit = blockIdx.x / nvs, v0 = (blockIdx.x % nvs) * 64;
   const int b = unit / p.H, h = unit % p.H, T = p.T, nblk = (T + kTB - 1) / kTB;
-  const uint32_t empty = tc::smem_u32(smem + smem_bytes<KIND, BF>() - kStages * 8);   // one mbarrier per stage
+  const uint32_t empty = tc::smem_u32(smem + kEmptyAt<KIND, BF>);
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) tc::mbar_init(empty + 8 * i, kCons / 32);
     tc::fence_mbar_init();
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
   if (threadIdx.x >= kCons) {
     // =========================== staging =========================================================================================
     const int grp = (threadIdx.x - kCons) >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
-    uint8_t* mine = smem + kStages * sizeof(Stage) + sizeof(Exchange) + grp * group_bytes<KIND, BF>();
+    uint8_t* mine = smem + kStages * sizeof(Stage) + sizeof(Exchange) + grp * kGroupBytes<KIND, BF>;
     Scratch& X = *reinterpret_cast<Scratch*>(mine);
     uint8_t* ring = mine + (sizeof(Scratch) + 15) / 16 * 16;
     constexpr int kRounds = (R::kTasks + 3) / 4;
@@ -177,12 +182,10 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     for (int i = 0; i < kRing; ++i) issue(grp + kGroups * i);
     for (int blk = grp; blk < nblk; blk += kGroups) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
-      if (tid == 0) {
-        X.wide = 0;
-        if (blk >= kStages &&   // the consumers have left this stage
-            !tc::mbar_wait_compact(empty + 8 * (blk % kStages), (blk / kStages - 1) & 1, kEmptyTries) && p.status)
-          atomicOr(p.status, DR_DEV_TIMEOUT);
-      }
+      if (tid == 0) X.wide = 0;
+      if (blk >= kStages &&   // the consumers have left this stage
+          !tc::mbar_wait_compact(empty + 8 * (blk % kStages), (blk / kStages - 1) & 1, kEmptyTries) && p.status)
+        atomicOr(p.status, DR_DEV_TIMEOUT);
       sync128();   // every thread's pieces of this block have landed
       const uint8_t* slot = ring + (blk / kGroups % kRing) * R::kSlot;
       Stage& S = s_st[blk % kStages];
@@ -465,7 +468,7 @@ inline bool eligible(int kind, bool bf, const LinRecParams& p, int sms) {
 
 template <int KIND, bool BF>
 inline cudaError_t launch_t(const LinRecParams& p, cudaStream_t stream) {
-  constexpr int bytes = smem_bytes<KIND, BF>();
+  constexpr int bytes = kSmemBytes<KIND, BF>;
   auto kern = rwkv_chunk_kernel<KIND, BF>;
   thread_local int attr_dev = -1;
   int dev = -1;
