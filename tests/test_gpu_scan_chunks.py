@@ -59,3 +59,25 @@ def test_rwkv_blocks(dtype, B, H, T, V, layout):
     ro, rs = R.rwkv6_recurrent(*(d(t) for t in (q, k, v, w, u)), scale=0.125, initial_state=d(h0), compute_dtype=torch.float64)
     _check(s, rs, 5e-6)
     _check(o, ro, tol)
+
+
+@pytest.mark.parametrize("B,T,H,N,first,A", [(1, 64, 2, 128, 32, -16.0), (1, 200, 2, 64, 1, -16.0), (2, 130, 80, 128, 20, -4.0),
+                                             (1, 1100, 2, 128, 32, -16.0), (1, 200, 2, 64, 5, -1.0e6)])
+def test_ssd_reset_then_accumulate(B, T, H, N, first, A):
+    """A strong decay in the first tokens of every chunk (the state is dropped), weak ones behind it: the chunk form has to keep the
+    weak decays to float32 precision, as the token recurrence does.  Bound: dt' = softplus(dt) in float32 is within 3e-7 of 64 bits
+    and enters a weight as factor and as exponent (|A dt'| <= 0.32 a token, e-folding after a few), the sums and products add a few
+    2^-24 each; 1.5e-6 of the state's largest entry.  A float32 running sum over the chunk misses it by two orders."""
+    g = torch.Generator().manual_seed(T)
+    f = lambda *s, scale=1.0: torch.randn(*s, generator=g) * scale
+    bf = lambda t: t.bfloat16()
+    x, Bm, Cm, D = bf(f(B, T, H, 64)), bf(f(B, T, 1, N, scale=0.5)), bf(f(B, T, 1, N, scale=0.5)), f(H)
+    weak = min(0.02, 0.32 / -A)
+    dt = torch.where((torch.arange(T) % 64 < first)[None, :, None], torch.tensor(5.0), torch.tensor(weak).expm1().log()).expand(B, T, H)
+    dt = (dt + f(B, T, H, scale=0.01)).contiguous()
+    Ah, h0 = torch.full((H,), A), f(B, H, 64, N)
+    c, d = (lambda t: t.cuda()), (lambda t: t.double())
+    y, s = L.ssd_chunk_scan(c(x), c(dt), c(Ah), c(Bm), c(Cm), c(D), ssm_state=c(h0))
+    ry, rs = R.ssd_token_recurrence(d(x), d(dt), d(Ah), d(Bm), d(Cm), d(D), ssm_state=d(h0))
+    _check(s, rs, 1.5e-6)
+    _check(y, ry, 5e-3)
