@@ -31,6 +31,7 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
+constexpr int64_t kPackedScratch = (int64_t)1 << 30;   // varlen.PACKED_SCRATCH
 int32_t* g_status[kMaxDevices] = {nullptr};   // device status words, registered by the Python side
 
 struct Api {
@@ -422,10 +423,13 @@ PyObject* py_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const double scale = a[8] == Py_None ? 1.0 / std::sqrt((double)K) : as_double(a[8]);
     const DrDesc d = make_desc(variant, DR_LAYOUT_BTHD, 1, H, longest, K, V, as_int(a[9]), dt, g_dt, (int)out, a[10] == Py_True, scale, 0, Hq);
     need(!PyErr_Occurred());
-    DrDesc dw = d;   // room for every sequence's chunks at once (one launch over all of them)
+    // scratch for every sequence's chunks at once (one launch over all of them) up to kPackedScratch, past that in several launches;
+    // the longest sequence's in any case
+    DrDesc dw = d;
     dw.T = (int32_t)std::min<int64_t>(total + 64 * (int64_t)n_seqs, INT32_MAX);
-    const int64_t ws_bytes = api.workspace_bytes(&dw, 0);
-    if (ws_bytes < 0) return PyLong_FromLong((long)ws_bytes);
+    const int64_t all = api.workspace_bytes(&dw, 0);
+    if (all < 0) return PyLong_FromLong((long)all);
+    const int64_t ws_bytes = std::min(all, std::max(api.workspace_bytes(&d, 0), kPackedScratch));
     at::Tensor ws;
     if (ws_bytes > 0) ws = c.empty({ws_bytes}, at::kByte);
     const at::Tensor o = c.empty({total, H, V}, scalar_type((int)out));

@@ -47,6 +47,10 @@ def pad(x_flat: Tensor, indices: Tensor, batch: int, seq: int) -> Tensor:
     return out.reshape((batch, seq) + tuple(x_flat.shape[1:]))
 
 
+# Most scratch a packed forward asks for, unless its longest sequence alone needs more: a batch whose chunks do not fit goes in
+# several launches.
+PACKED_SCRATCH = 1 << 30
+
 _VAR = {"delta": DR_DELTA, "gated": DR_GATED, "kda": DR_KDA}
 
 
@@ -117,9 +121,12 @@ def chunkwise_varlen(variant: str, q: Tensor, k: Tensor, v: Tensor, g: Optional[
     d = ops._desc(_VAR[variant], DR_LAYOUT_BTHD, 1, H, longest, K, V, chunk_size, qn, gn, native_out, use_qk_l2norm, scale)
     d.qk_heads = Hq
     lib = _lib.load()
-    d.T = total + 64 * n   # room for every sequence's chunks at once (one launch over all of them)
+    longest_need = int(lib.dr_workspace_bytes(ctypes.byref(d), 0))
+    d.T = min(total + 64 * n, 2**31 - 1)   # every sequence's chunks at once: one launch over all of them
     need = int(lib.dr_workspace_bytes(ctypes.byref(d), 0))
     d.T = longest
+    if need > 0:
+        need = min(need, max(longest_need, PACKED_SCRATCH))
     if need == -7:
         raise ValueError(f"chunk_size (BT={chunk_size}) must be divisible by BC=16.")
     _lib.check(need if need < 0 else 0, "dr_workspace_bytes")

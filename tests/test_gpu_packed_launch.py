@@ -43,3 +43,31 @@ def test_packed_launch(variant, lens, poison):
         ro, rs = _alone(variant, x, cu[i], cu[i + 1], h0[i:i + 1])
         assert torch.equal(o[cu[i]:cu[i + 1]], ro) and torch.equal(s[i], rs), i
         assert torch.isfinite(ro.float()).all()
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_scratch_of_a_packed_batch_is_bounded(native):
+    """14 sequences whose records would take 1.16 GB: at most 1 GiB is asked for, the batch goes in two launches, and the results are
+    those of its halves (which fit) bit for bit."""
+    n, T, H = 14, 4000, 16
+    g = torch.Generator(device="cuda").manual_seed(0)
+    f = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k, v = (f(n * T, H, 128).bfloat16() for _ in range(3))
+    d = -f(n * T, H, 128).abs().mul_(0.05).bfloat16()
+    beta = torch.sigmoid(f(n * T, H))
+    if not native:   # another storage type of beta goes the Python way
+        beta = beta.bfloat16()
+    L.check_device_status()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    run = lambda a, b: L.chunkwise_varlen("kda", *(t[a * T:b * T] for t in (q, k, v, d, beta)), [i * T for i in range(b - a + 1)], out_dtype=torch.bfloat16)
+    o, s = run(0, n)
+    asked = torch.cuda.max_memory_allocated() - before
+    results = o.numel() * 2 + s.numel() * 4 + (0 if native else beta.numel() * 4)
+    assert asked <= results + (1 << 30) + (8 << 20)
+    h = n // 2
+    for a, b in ((0, h), (h, n)):
+        ro, rs = run(a, b)
+        assert torch.equal(o[a * T:b * T], ro) and torch.equal(s[a:b], rs)
+    L.check_device_status()
