@@ -77,6 +77,10 @@ __device__ __forceinline__ bool in_bounds(int32_t* status, int64_t i, int64_t n)
 #else
 __device__ __forceinline__ bool in_bounds(int32_t*, int64_t, int64_t) { return true; }
 #endif
+// the same for `len` entries from i on (one vector access)
+__device__ __forceinline__ bool in_bounds_run(int32_t* status, int64_t i, int len, int64_t n) {
+  return in_bounds(status, i, n) && in_bounds(status, i + len - 1, n);
+}
 
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll

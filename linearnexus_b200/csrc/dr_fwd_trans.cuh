@@ -147,6 +147,9 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
   const int64_t qk_base = p.map.base_qk(b, h, D), qk_tok = p.map.tok_qk(D), vg_base = p.map.base(b, h, D), vg_tok = p.map.tok(D);
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1), chunk = (int64_t)unit * P.N + n;
 
+  // index check of an entry of a scratch array that holds `per` floats a chunk
+  auto scratch = [&](int64_t i, int width, int64_t per) { return in_bounds(p.status, i, (int64_t)p.map.B * p.map.H * P.N * (per / width)); };
+
   // ---- q^, k^ (normalised, scaled), v, decay, beta ---------------------------------------------------------------------------
   {
     constexpr int LPR = D / 4, RPP = NTHR / LPR, PASSES = 64 / RPP;   // lanes per row, rows per pass
@@ -157,19 +160,21 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
       const int c = r0 + RPP * i;
       qv[i] = kv[i] = vv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (KDA) gv[i] = qv[i];
-      if (c < rows) {
-        qv[i] = load4(p.q, qk_base + (t0 + c) * qk_tok + c4, p.qkv_dt);
-        kv[i] = load4(p.k, qk_base + (t0 + c) * qk_tok + c4, p.qkv_dt);
-        vv[i] = load4(p.v, vg_base + (t0 + c) * vg_tok + c4, p.qkv_dt);
-        if constexpr (KDA) gv[i] = load4(p.g, vg_base + (t0 + c) * vg_tok + c4, p.g_dt);
+      const int64_t qk_at = qk_base + (t0 + c) * qk_tok + c4, vg_at = vg_base + (t0 + c) * vg_tok + c4;
+      if (c < rows && in_bounds_run(p.status, qk_at, 4, p.n_qk) && in_bounds_run(p.status, vg_at, 4, p.n_v)) {
+        qv[i] = load4(p.q, qk_at, p.qkv_dt);
+        kv[i] = load4(p.k, qk_at, p.qkv_dt);
+        vv[i] = load4(p.v, vg_at, p.qkv_dt);
+        if constexpr (KDA) gv[i] = load4(p.g, vg_at, p.g_dt);   // (K = V: as many entries as v)
       }
     }
-    if (tid < 64) sBeta[tid] = tid < rows ? p.beta[s_base + (t0 + tid) * s_tok] : 0.f;
+    auto token = [&](int r) { return r < rows && in_bounds(p.status, s_base + (t0 + r) * s_tok, p.n_tok); };
+    if (tid < 64) sBeta[tid] = token(tid) ? p.beta[s_base + (t0 + tid) * s_tok] : 0.f;
     if (!KDA && warp == NW - 1) {
       float lo = 0.f, hi = 0.f;
       if (p.variant == DR_GATED) {
-        if (lane < rows) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
-        if (lane + 32 < rows) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
+        if (token(lane)) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
+        if (token(lane + 32)) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
       }
       // sums inside the 16-row blocks (two blocks per 32 lanes), up to a row and over its rest
       float plo = lo, phi = hi, slo = lo, shi = hi;
@@ -246,8 +251,8 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
     sBef[blk * D + c] = bef;
     sAft[blk * D + c] = aft;
     __syncthreads();
-    if (tid < D) P.el[chunk * D + tid] = sBef[3 * D + tid] * sD[3 * D + tid];
-  } else if (tid < D) {
+    if (tid < D && scratch(chunk * D + tid, 1, Z_::fE)) P.el[chunk * D + tid] = sBef[3 * D + tid] * sD[3 * D + tid];
+  } else if (tid < D && scratch(chunk * D + tid, 1, Z_::fE)) {
     P.el[chunk * D + tid] = sEG[63];
   }
   // ---- X = tril(K^K^^T.E, -1), A = tril(Q^K^^T.E) ----------------------------------------------------------------------------------
@@ -297,13 +302,20 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
       if (!unsafe(blk) || tid >= 256) continue;
       const int i = 16 * blk + (tid >> 4), j = 16 * blk + (tid & 15);
       float ak = 0.f, aq = 0.f;
+      auto qk = [&](const void* x, int r, int c) {
+        const int64_t at = qk_base + (t0 + r) * qk_tok + c;
+        return in_bounds(p.status, at, p.n_qk) ? ld_elem(x, at, p.qkv_dt) : 0.f;
+      };
       if (j <= i && i < rows)
         for (int c = 0; c < D; ++c) {
           float x = 0.f;   // the decay of tokens j + 1 .. i, from the inputs
-          for (int m = j + 1; m <= i; ++m) x += ld_elem(p.g, vg_base + (t0 + m) * vg_tok + c, p.g_dt);
-          const float w = ld_elem(p.k, qk_base + (t0 + j) * qk_tok + c, p.qkv_dt) * sRk[j] * expf(x);
-          ak += ld_elem(p.k, qk_base + (t0 + i) * qk_tok + c, p.qkv_dt) * w;
-          aq += ld_elem(p.q, qk_base + (t0 + i) * qk_tok + c, p.qkv_dt) * w;
+          for (int m = j + 1; m <= i; ++m) {
+            const int64_t at = vg_base + (t0 + m) * vg_tok + c;
+            if (in_bounds(p.status, at, p.n_gk)) x += ld_elem(p.g, at, p.g_dt);
+          }
+          const float w = qk(p.k, j, c) * sRk[j] * expf(x);
+          ak += qk(p.k, i, c) * w;
+          aq += qk(p.q, i, c) * w;
         }
       ak *= sRk[i];
       aq *= sRq[i];
@@ -388,6 +400,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
     const int64_t at = ((chunk * CT + mt) * (2 * CT) + 2 * own) * 32 + lane;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
+      if (!scratch(at + 32 * hf, 4, Z_::fN)) continue;
       P.nf[at + 32 * hf] = make_float4(-w[hf][0], -w[hf][2], -w[hf][1], -w[hf][3]);
       P.zf[at + 32 * hf] = make_float4(u[hf][0], u[hf][1], u[hf][2], u[hf][3]);
     }
@@ -415,6 +428,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
         const int i = 16 * mt + g + 8 * (e >> 1), c = 16 * own + 8 * hf + 2 * t + (e & 1);
         y[e] = sQ[i * LD + c] * (KDA ? sBef[mt * D + c] : sEG[i]) - w[hf][e];
       }
+      if (!scratch(at + 32 * hf, 4, Z_::fY)) continue;
       P.yf[at + 32 * hf] = make_float4(y[0], y[2], y[1], y[3]);
       P.of[at + 32 * hf] = make_float4(u[hf][0], u[hf][1], u[hf][2], u[hf][3]);
     }
@@ -441,20 +455,25 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
   const int tiles = state ? CT : 4;
   float4 a[D / 8], c[NT];
   float S[NT][4], el0 = 0.f, el1 = 0.f;
-  auto at_a = [&](int64_t ch, int ks) { return ((ch * tiles + mt) * (D / 8) + ks) * 32 + lane; };
-  auto at_c = [&](int64_t ch, int nt) { return ((ch * tiles + mt) * (D / 8) + v0 / 8 + nt) * 32 + lane; };
+  // entry `i` of a scratch array; both halves of the warps read arrays of tiles * (D / 8) * 32 entries a chunk
+  const int64_t entries = (int64_t)p.map.B * p.map.H * P.N * tiles * (D / 8) * 32;
+  auto get = [&](const float4* f, int64_t i) { return in_bounds(p.status, i, entries) ? f[i] : make_float4(0.f, 0.f, 0.f, 0.f); };
+  auto get_a = [&](int64_t ch, int ks) { return get(fa, ((ch * tiles + mt) * (D / 8) + ks) * 32 + lane); };
+  auto get_c = [&](int64_t ch, int nt) { return get(fc, ((ch * tiles + mt) * (D / 8) + v0 / 8 + nt) * 32 + lane); };
+  auto get_el = [&](int64_t ch, int r) { return in_bounds(p.status, ch * D + r, (int64_t)p.map.B * p.map.H * P.N * D) ? P.el[ch * D + r] : 0.f; };
+  auto s_at = [&](int r, int nt) { return ((int64_t)unit * D + r) * D + v0 + 8 * nt + 2 * t; };
 #pragma unroll
-  for (int ks = 0; ks < D / 8; ++ks) a[ks] = fa[at_a(chunk0, ks)];
+  for (int ks = 0; ks < D / 8; ++ks) a[ks] = get_a(chunk0, ks);
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) c[nt] = fc[at_c(chunk0, nt)];
+  for (int nt = 0; nt < NT; ++nt) c[nt] = get_c(chunk0, nt);
   if (state) {
-    el0 = P.el[chunk0 * D + r0]; el1 = P.el[chunk0 * D + r1];
+    el0 = get_el(chunk0, r0); el1 = get_el(chunk0, r1);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       float2 lo = make_float2(0.f, 0.f), hi = lo;
-      if (p.h0) {
-        lo = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * D + r0) * D + v0 + 8 * nt + 2 * t);
-        hi = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * D + r1) * D + v0 + 8 * nt + 2 * t);
+      if (p.h0 && in_bounds_run(p.status, s_at(r0, nt), 2, p.n_state) && in_bounds_run(p.status, s_at(r1, nt), 2, p.n_state)) {
+        lo = *reinterpret_cast<const float2*>(p.h0 + s_at(r0, nt));
+        hi = *reinterpret_cast<const float2*>(p.h0 + s_at(r1, nt));
       }
       S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
     }
@@ -481,12 +500,12 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
     }
     const int64_t cn = chunk0 + (n + 1 < P.N ? n + 1 : n);   // the next chunk's operands replace this one's as they are used
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) c[nt] = fc[at_c(cn, nt)];
+    for (int nt = 0; nt < NT; ++nt) c[nt] = get_c(cn, nt);
 #pragma unroll
     for (int ks = 0; ks < D / 8; ++ks) {
       AFrag<X3> fr;
       fr.set(a[ks].x, a[ks].y, a[ks].z, a[ks].w);
-      a[ks] = fa[at_a(cn, ks)];
+      a[ks] = get_a(cn, ks);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
@@ -501,7 +520,7 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
         S[nt][0] = el0 * S[nt][0] + (d[nt][0] + e[nt][0]); S[nt][1] = el0 * S[nt][1] + (d[nt][1] + e[nt][1]);
         S[nt][2] = el1 * S[nt][2] + (d[nt][2] + e[nt][2]); S[nt][3] = el1 * S[nt][3] + (d[nt][3] + e[nt][3]);
       }
-      el0 = P.el[cn * D + r0]; el1 = P.el[cn * D + r1];
+      el0 = get_el(cn, r0); el1 = get_el(cn, r1);
     } else {
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
@@ -511,6 +530,7 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             const float x = d[nt][2 * hr] + e[nt][2 * hr], y = d[nt][2 * hr + 1] + e[nt][2 * hr + 1];
+            if (!in_bounds_run(p.status, at + 8 * nt, 2, p.n_v)) continue;
             if (p.out_dt == DR_BF16)
               *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.o) + at + 8 * nt) = mma::pack(x, y);
             else
@@ -523,8 +543,9 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
   if (state && p.hT) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * D + r0) * D + v0 + 8 * nt + 2 * t) = make_float2(S[nt][0], S[nt][1]);
-      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * D + r1) * D + v0 + 8 * nt + 2 * t) = make_float2(S[nt][2], S[nt][3]);
+      if (!in_bounds_run(p.status, s_at(r0, nt), 2, p.n_state) || !in_bounds_run(p.status, s_at(r1, nt), 2, p.n_state)) continue;
+      *reinterpret_cast<float2*>(p.hT + s_at(r0, nt)) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(p.hT + s_at(r1, nt)) = make_float2(S[nt][2], S[nt][3]);
     }
   }
 }

@@ -1060,6 +1060,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
   uint4 a[8];
   float4 c[NT];
   float S[NT][4], el0 = 0.f, el1 = 0.f;
+  auto s_at = [&](int r, int nt) { return ((int64_t)unit * kD + r) * kD + v0 + 8 * nt + 2 * t; };
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) a[ks] = fa[((chunk0 * tiles + mt) * 8 + ks) * 32];
 #pragma unroll
@@ -1069,9 +1070,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       float2 lo = make_float2(0.f, 0.f), hi = lo;
-      if (p.h0) {
-        lo = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t);
-        hi = *reinterpret_cast<const float2*>(p.h0 + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t);
+      if (p.h0 && in_bounds_run(p.status, s_at(r0, nt), 2, p.n_state) && in_bounds_run(p.status, s_at(r1, nt), 2, p.n_state)) {
+        lo = *reinterpret_cast<const float2*>(p.h0 + s_at(r0, nt));
+        hi = *reinterpret_cast<const float2*>(p.h0 + s_at(r1, nt));
       }
       S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
     }
@@ -1125,6 +1126,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             const float x = d[nt][2 * hr] + e[nt][2 * hr], y = d[nt][2 * hr + 1] + e[nt][2 * hr + 1];
+            if (!in_bounds_run(p.status, at + 8 * nt, 2, p.n_v)) continue;
             if (p.out_dt == DR_BF16) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.o) + at + 8 * nt) = mma::pack(x, y);
             else *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.o) + at + 8 * nt) = make_float2(x, y);
           }
@@ -1135,8 +1137,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
   if (state && p.hT) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t) = make_float2(S[nt][0], S[nt][1]);
-      *reinterpret_cast<float2*>(p.hT + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t) = make_float2(S[nt][2], S[nt][3]);
+      if (!in_bounds_run(p.status, s_at(r0, nt), 2, p.n_state) || !in_bounds_run(p.status, s_at(r1, nt), 2, p.n_state)) continue;
+      *reinterpret_cast<float2*>(p.hT + s_at(r0, nt)) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(p.hT + s_at(r1, nt)) = make_float2(S[nt][2], S[nt][3]);
     }
   }
 }

@@ -143,20 +143,22 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
     uint8_t* ring = mine + (sizeof(Scratch) + 15) / 16 * 16;
     constexpr int kRounds = (R::kTasks + 3) / 4;
     const uint8_t* src[kRounds];
-    int64_t step[kRounds];
+    int64_t step[kRounds], at0[kRounds], size[kRounds];   // (the last two: index checks of the debug build)
     int rtok[kRounds];
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
       const int byte = (warp + 4 * r) * 512 + lane * 16, j = byte / R::kVec, off = byte % R::kVec;
       const LrVec* vecs[5] = {&p.q, &p.k, &p.w, &p.a, &p.b};
       const void* ptr = p.v.p;
-      int64_t st = p.v.st, at = p.v.at(b, h, 0) + v0;
+      int64_t st = p.v.st, at = p.v.at(b, h, 0) + v0, n = p.v.n;
 #pragma unroll
       for (int jj = 0; jj < NV; ++jj)
-        if (jj == j) { ptr = vecs[jj]->p; st = vecs[jj]->st; at = vecs[jj]->at(b, h, 0); }
+        if (jj == j) { ptr = vecs[jj]->p; st = vecs[jj]->st; at = vecs[jj]->at(b, h, 0); n = vecs[jj]->n; }
       rtok[r] = off / (kK * R::ES);
       src[r] = reinterpret_cast<const uint8_t*>(ptr) + (at + rtok[r] * st) * R::ES + off % (kK * R::ES);
       step[r] = (int64_t)kTB * st * R::ES;
+      at0[r] = at + rtok[r] * st + off % (kK * R::ES) / R::ES;
+      size[r] = n;
     }
     auto issue = [&](int blk) {   // blocks of this group: blk = grp, grp + kGroups, ...
       if (blk * kTB < T) {
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
           if (warp + 4 * r < R::kTasks) {
-            const bool ok = blk * kTB + rtok[r] < T;
+            const bool ok = blk * kTB + rtok[r] < T && in_bounds_run(p.status, at0[r] + blk * (step[r] / R::ES), 16 / R::ES, size[r]);
             tc::cp_async16(slot + 2048u * r, src[r] + (ok ? blk * step[r] : 0), ok);
           }
         }
@@ -364,7 +366,10 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) S[nt][e] = h0 ? h0[(int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] : 0.f;
+    for (int e = 0; e < 4; ++e) {
+      const int64_t at = (int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1);
+      S[nt][e] = h0 && in_bounds(p.status, (h0 - p.h0) + at, p.n_state) ? h0[at] : 0.f;
+    }
   const int64_t o_at = (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + v0 + vb + g;
   for (int blk = 0; blk < nblk; ++blk) {
     bar_sync(kBarFull + blk % kStages, kHand);
@@ -442,7 +447,8 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int tok = blk * kTB + 2 * t + (e & 1);
-        if (tok < T) st_elem(p.o, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), BF ? DR_BF16 : DR_F32, o[e]);
+        if (tok < T && in_bounds(p.status, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), p.n_o))
+          st_elem(p.o, o_at + (int64_t)tok * p.o_st + 8 * (e >> 1), BF ? DR_BF16 : DR_F32, o[e]);
       }
     }
   }
@@ -451,7 +457,10 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) hT[(int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1)] = S[nt][e];
+      for (int e = 0; e < 4; ++e) {
+        const int64_t at = (int64_t)(kb + 8 * nt + 2 * t + (e & 1)) * p.V + 8 * (e >> 1);
+        if (in_bounds(p.status, (hT - p.hT) + at, p.n_state)) hT[at] = S[nt][e];
+      }
   }
 }
 

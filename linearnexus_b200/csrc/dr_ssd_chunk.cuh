@@ -72,11 +72,13 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
   const int b = unit / p.H, h = unit % p.H, T = p.T;
   const int nchunks = (T + kC - 1) / kC, per = (nchunks + nseg - 1) / nseg;
   const int c_lo = min(seg * per, nchunks), c_hi = min(c_lo + per, nchunks);
-  const __nv_bfloat16* gC = reinterpret_cast<const __nv_bfloat16*>(p.q.p) + p.q.at(b, h, 0);
-  const __nv_bfloat16* gB = reinterpret_cast<const __nv_bfloat16*>(p.k.p) + p.k.at(b, h, 0);
-  const __nv_bfloat16* gx = reinterpret_cast<const __nv_bfloat16*>(p.v.p) + p.v.at(b, h, 0) + slice * kP;
-  __nv_bfloat16* gy = reinterpret_cast<__nv_bfloat16*>(p.o) + b * p.o_sb + h * p.o_sh + slice * kP;
-  const float* gdt = reinterpret_cast<const float*>(p.dt.p) + p.dt.at(b, h, 0);
+  const int64_t c_at = p.q.at(b, h, 0), b_at = p.k.at(b, h, 0), x_at = p.v.at(b, h, 0) + slice * kP, dt_at = p.dt.at(b, h, 0);
+  const int64_t y_at = b * p.o_sb + h * p.o_sh + slice * kP;
+  const __nv_bfloat16* gC = reinterpret_cast<const __nv_bfloat16*>(p.q.p) + c_at;
+  const __nv_bfloat16* gB = reinterpret_cast<const __nv_bfloat16*>(p.k.p) + b_at;
+  const __nv_bfloat16* gx = reinterpret_cast<const __nv_bfloat16*>(p.v.p) + x_at;
+  __nv_bfloat16* gy = reinterpret_cast<__nv_bfloat16*>(p.o) + y_at;
+  const float* gdt = reinterpret_cast<const float*>(p.dt.p) + dt_at;
   const float A_h = p.A[h], D_h = p.D[h], bias_h = p.dt_bias ? p.dt_bias[h] : 0.f;
   const uint32_t sbase = tc::smem_u32(smem);
 
@@ -88,14 +90,16 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
     for (int nt = 0; nt < NT; ++nt) S[nt][0] = S[nt][1] = S[nt][2] = S[nt][3] = 0.f;
   };
   zero_state();
-  if (p.h0 && seg == 0) {
+  auto load_h0 = [&]() {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
+      if (!in_bounds_run(p.status, s_unit + 8 * nt, 2, p.n_state) || !in_bounds_run(p.status, s_unit + 8 * N + 8 * nt, 2, p.n_state)) continue;
       const float2 lo = *reinterpret_cast<const float2*>(p.h0 + s_unit + 8 * nt);
       const float2 hi = *reinterpret_cast<const float2*>(p.h0 + s_unit + 8 * N + 8 * nt);
       S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
     }
-  }
+  };
+  if (p.h0 && seg == 0) load_h0();
 
   auto tile_B = [&](int st) { return sbase + L::kB + st * L::kStage; };
   auto tile_C = [&](int st) { return sbase + L::kB + st * L::kStage + L::kTileN; };
@@ -108,13 +112,16 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
     for (int i = tid; i < kC * (N / 8); i += kThreads) {
       const int r = i / (N / 8), q = (i % (N / 8)) * 8;
       const int64_t row = t0 + (r < rows ? r : 0);
-      tc::cp_async16(tile_B(st) + 2u * (r * LDN + q), gB + row * p.k.st + q, r < rows);
-      if (full) tc::cp_async16(tile_C(st) + 2u * (r * LDN + q), gC + row * p.q.st + q, r < rows);
+      tc::cp_async16(tile_B(st) + 2u * (r * LDN + q), gB + row * p.k.st + q,
+                     r < rows && in_bounds_run(p.status, b_at + row * p.k.st + q, 8, p.k.n));
+      if (full) tc::cp_async16(tile_C(st) + 2u * (r * LDN + q), gC + row * p.q.st + q,
+                               r < rows && in_bounds_run(p.status, c_at + row * p.q.st + q, 8, p.q.n));
     }
 #pragma unroll
     for (int i = tid; i < kC * (kP / 8); i += kThreads) {
       const int r = i / (kP / 8), q = (i % (kP / 8)) * 8;
-      tc::cp_async16(tile_X(st) + 2u * (r * LDX + q), gx + (int64_t)(t0 + (r < rows ? r : 0)) * p.v.st + q, r < rows);
+      const int64_t at = (int64_t)(t0 + (r < rows ? r : 0)) * p.v.st + q;
+      tc::cp_async16(tile_X(st) + 2u * (r * LDX + q), gx + at, r < rows && in_bounds_run(p.status, x_at + at, 8, p.v.n));
     }
     tc::cp_async_commit();
   };
@@ -123,8 +130,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
   auto fetch_dt = [&](int c) {
     if (warp == 0) {
       const int t0 = c * kC + lane;
-      dt_lo = t0 < T ? gdt[(int64_t)t0 * p.dt.st] : 0.f;
-      dt_hi = t0 + 32 < T ? gdt[(int64_t)(t0 + 32) * p.dt.st] : 0.f;
+      const int64_t at = (int64_t)t0 * p.dt.st, at32 = (int64_t)(t0 + 32) * p.dt.st;
+      dt_lo = t0 < T && in_bounds(p.status, dt_at + at, p.dt.n) ? gdt[at] : 0.f;
+      dt_hi = t0 + 32 < T && in_bounds(p.status, dt_at + at32, p.dt.n) ? gdt[at32] : 0.f;
     }
   };
   auto scan_dt = [&](int c, int st) {
@@ -230,14 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
       }
     } else {
       zero_state();
-      if (p.h0) {
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          const float2 lo = *reinterpret_cast<const float2*>(p.h0 + s_unit + 8 * nt);
-          const float2 hi = *reinterpret_cast<const float2*>(p.h0 + s_unit + 8 * N + 8 * nt);
-          S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
-        }
-      }
+      if (p.h0) load_h0();
     }
     cluster.sync();   // the others have read this CTA's copy (and p.hT may alias p.h0)
   }
@@ -375,13 +376,14 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
 #pragma unroll
     for (int i = tid; i < kC * (kP / 8); i += kThreads) {
       const int r = i / (kP / 8), q = (i % (kP / 8)) * 8;
-      if (t0 + r < T)
+      if (t0 + r < T && in_bounds_run(p.status, y_at + (int64_t)(t0 + r) * p.o_st + q, 8, p.n_o))
         *reinterpret_cast<uint4*>(gy + (int64_t)(t0 + r) * p.o_st + q) = *reinterpret_cast<const uint4*>(sYo + r * LDX + q);
     }
   }
   if (p.hT && seg == nseg - 1) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
+      if (!in_bounds_run(p.status, s_unit + 8 * nt, 2, p.n_state) || !in_bounds_run(p.status, s_unit + 8 * N + 8 * nt, 2, p.n_state)) continue;
       *reinterpret_cast<float2*>(p.hT + s_unit + 8 * nt) = make_float2(S[nt][0], S[nt][1]);
       *reinterpret_cast<float2*>(p.hT + s_unit + 8 * N + 8 * nt) = make_float2(S[nt][2], S[nt][3]);
     }

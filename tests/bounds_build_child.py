@@ -49,6 +49,31 @@ def main(out_path):
         y, s = L.ssd_chunk_scan(rn(2, T, 4, 24), rn(2, T, 4), -rn(4).abs(), rn(2, T, 2, 20), rn(2, T, 2, 20), rn(4), n_groups=2,
                                 ssm_state=rn(2, 4, 24, 20) * 0.1, dt_bias=rn(4))
         out[f"o{n}"], out[f"s{n}"] = y.cpu().numpy(), s.cpu().numpy(); n += 1
+    # the chunk forms of the scans at their tiles' edges, and of a few long sequences
+    for dt in (torch.bfloat16, torch.float32):
+        for (T, H, V) in ((9, 2, 64), (67, 3, 128), (130, 1, 192)):
+            q, k, a, b = ((rn(2, H, T, 64) * 0.3).to(dt) for _ in range(4))
+            v, gk = rn(2, H, T, V).to(dt), -rn(2, H, T, 64).abs().to(dt)
+            gk[:, :, T // 2] = -70.0
+            h0 = rn(2, H, 64, V) * 0.1
+            for view in (lambda x: x, lambda x: x.transpose(1, 2).contiguous().transpose(1, 2)):
+                o, s = L.dplr_delta_rule_recurrent(*(view(x) for x in (q, k, v, a, b, gk)), initial_state=h0)
+                out[f"o{n}"], out[f"s{n}"] = o.float().cpu().numpy(), s.cpu().numpy(); n += 1
+                o, s = L.rwkv6_recurrent(*(view(x) for x in (q, k, v, gk)), rn(H, 64), initial_state=h0)
+                out[f"o{n}"], out[f"s{n}"] = o.float().cpu().numpy(), s.cpu().numpy(); n += 1
+    for (B, T, H, P, N, G) in ((1, 32, 2, 64, 64, 1), (2, 67, 4, 128, 128, 2), (1, 577, 1, 64, 64, 1), (1, 1100, 2, 64, 128, 1)):
+        y, s = L.ssd_chunk_scan(rn(B, T, H, P).bfloat16(), rn(B, T, H), -rn(H).abs(), rn(B, T, G, N).bfloat16(), rn(B, T, G, N).bfloat16(), rn(H),
+                                n_groups=G, ssm_state=rn(B, H, P, N) * 0.1, dt_bias=rn(H))
+        out[f"o{n}"], out[f"s{n}"] = y.float().cpu().numpy(), s.cpu().numpy(); n += 1
+    for variant, d, dt, T in (("gated", 128, torch.bfloat16, 391), ("kda", 128, torch.bfloat16, 1100), ("kda", 128, torch.float32, 130),
+                              ("kda", 64, torch.bfloat16, 130), ("delta", 128, torch.float32, 200)):
+        c = cu(make_rows(variant, 0, 1, 2, T, d, d, seed=T, io_dtype=dt, h0_std=0.1))
+        if variant == "kda":
+            c["g"][:, :, T // 2] = -70.0   # a block that is summed entry by entry
+        fn = {"delta": L.delta_rule_chunkwise, "gated": L.gated_delta_rule_chunkwise, "kda": L.kda_chunkwise}[variant]
+        o, s = fn(*(c[x] for x in ("q", "k", "v", "g", "beta") if c[x] is not None), initial_state=c["h0"])
+        assert _lib.last_path() == "chunk_transition"
+        out[f"o{n}"], out[f"s{n}"] = o.float().cpu().numpy(), s.cpu().numpy(); n += 1
     torch.cuda.synchronize()
     try:
         L.check_device_status()
