@@ -10,7 +10,9 @@
 //                       chain, the output product beside it in warps of its own
 //
 // Decays are sums over a 16-row block up to a row, sums over its rest, and block totals, each summed by itself: a difference
-// of long cumulative sums would lose what the recurrence keeps when a strong decay came earlier in the chunk.  Per-channel
+// of long cumulative sums would lose what the recurrence keeps when a strong decay came earlier in the chunk.  Inside a block the
+// scalar decays are differences all the same, so those sums are taken in 64 bits and kept as a float32 pair (eight tokens of -80, then
+// eight of -0.02 a block: outputs off by 3.2e-5 with float32 sums, 6.5e-7 so).  Per-channel
 // decays are folded into the rows once: q e^{prefix}, k e^{prefix}, k e^{suffix}; products between blocks carry the totals of
 // the blocks in between.  A block whose decay exceeds 2^64 in some channel is summed entry by entry.
 //
@@ -32,13 +34,16 @@ using mma::BFrag;
 constexpr int kC = 64;
 constexpr int LDX = 72;
 constexpr float kLog2e = 1.4426950408889634f;
+// A token's scalar log decay is cut off here: float32 has only zeros left for what crosses it, and -infinity (a hard reset) would
+// leave infinity minus infinity between the tokens behind it.
+constexpr float kDecayFloor = -200.f;
 
 template <int D>
 struct Sizes {
   static constexpr int NTHR = D == 128 ? 512 : 256, NW = NTHR / 32, CT = D / 16, LD = D + 4;
   static constexpr int kK = 0, kQ = kK + 64 * LD * 4, kV = kQ + 64 * LD * 4, kX = kV + 64 * LD * 4, kA = kX + 64 * LDX * 4;
-  static constexpr int kSc = kA + 64 * LDX * 4;   // beta, prefix, suffix, e^G, e^{G_L - G}, norm factors of q and k (64 each), flags
-  static constexpr int kD = kSc + 8 * 64 * 4;     // KDA: per block and channel: its total decay, the decay before it, after it
+  static constexpr int kSc = kA + 64 * LDX * 4;   // beta, prefix, suffix, e^G, e^{G_L - G}, norm factors of q and k, flags, rest of the prefix (64 each)
+  static constexpr int kD = kSc + 9 * 64 * 4;     // KDA: per block and channel: its total decay, the decay before it, after it
   static constexpr int kE = kD + 3 * 4 * D * 4;   // KDA: k e^{suffix} [64][LD]
   static constexpr int smem(bool kda) { return kda ? kE + 64 * LD * 4 : kD; }
   // floats per chunk: N, Z, Y, A U, e^{G_L}
@@ -139,7 +144,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
   extern __shared__ __align__(16) uint8_t smem[];
   auto F = [&](int off) { return reinterpret_cast<float*>(smem + off); };
   float *sK = F(Z_::kK), *sQ = F(Z_::kQ), *sV = F(Z_::kV), *sX = F(Z_::kX), *sA = F(Z_::kA), *sBeta = F(Z_::kSc);
-  float *sPre = sBeta + 64, *sSuf = sBeta + 128, *sEG = sBeta + 192, *sWd = sBeta + 256, *sRq = sBeta + 320, *sRk = sBeta + 384, *sUn = sBeta + 448;
+  float *sPre = sBeta + 64, *sSuf = sBeta + 128, *sEG = sBeta + 192, *sWd = sBeta + 256, *sRq = sBeta + 320, *sRk = sBeta + 384, *sUn = sBeta + 448, *sPreLo = sBeta + 512;
   float *sD = F(Z_::kD), *sBef = sD + 4 * D, *sAft = sD + 8 * D, *sE = F(Z_::kE);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int unit = blockIdx.x / P.N, n = blockIdx.x % P.N;
@@ -176,15 +181,20 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
         if (token(lane)) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
         if (token(lane + 32)) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
       }
+      if (lo < kDecayFloor) lo = kDecayFloor;
+      if (hi < kDecayFloor) hi = kDecayFloor;
       // sums inside the 16-row blocks (two blocks per 32 lanes), up to a row and over its rest
-      float plo = lo, phi = hi, slo = lo, shi = hi;
+      double dlo = lo, dhi = hi;
+      float slo = lo, shi = hi;
 #pragma unroll
       for (int o = 1; o < 16; o <<= 1) {
-        const float a = __shfl_up_sync(0xffffffffu, plo, o), c = __shfl_up_sync(0xffffffffu, phi, o);
+        const double a = __shfl_up_sync(0xffffffffu, dlo, o), c = __shfl_up_sync(0xffffffffu, dhi, o);
         const float d = __shfl_down_sync(0xffffffffu, slo, o), e = __shfl_down_sync(0xffffffffu, shi, o);
-        if ((lane & 15) >= o) { plo += a; phi += c; }
+        if ((lane & 15) >= o) { dlo += a; dhi += c; }
         if ((lane & 15) + o < 16) { slo += d; shi += e; }
       }
+      const float plo = (float)dlo, phi = (float)dhi;
+      sPreLo[lane] = (float)(dlo - plo); sPreLo[lane + 32] = (float)(dhi - phi);
       const float xlo = __shfl_down_sync(0xffffffffu, slo, 1), xhi = __shfl_down_sync(0xffffffffu, shi, 1);   // exclusive
       slo = (lane & 15) == 15 ? 0.f : xlo; shi = (lane & 15) == 15 ? 0.f : xhi;
       const float t0_ = __shfl_sync(0xffffffffu, plo, 15), t1_ = __shfl_sync(0xffffffffu, plo, 31), t2_ = __shfl_sync(0xffffffffu, phi, 15),
@@ -289,7 +299,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
       float f = 1.f;
       if constexpr (!KDA) {
         const int bj = nt >> 1;
-        float x = bj == mt ? sPre[i] - sPre[jj] : sPre[i] + sSuf[jj];
+        float x = bj == mt ? (sPre[i] - sPre[jj]) + (sPreLo[i] - sPreLo[jj]) : sPre[i] + sSuf[jj];
         for (int y = bj + 1; y < mt; ++y) x += sUn[8 + y];
         f = expf(fminf(x, 0.f));
       }
