@@ -12,7 +12,8 @@
 // Decays are sums over a 16-row block up to a row, sums over its rest, and block totals, each summed by itself: a difference
 // of long cumulative sums would lose what the recurrence keeps when a strong decay came earlier in the chunk.  Inside a block the
 // scalar decays are differences all the same, so those sums are taken in 64 bits and kept as a float32 pair (eight tokens of -80, then
-// eight of -0.02 a block: outputs off by 3.2e-5 with float32 sums, 6.5e-7 so).  Per-channel
+// eight of -0.02 a block: outputs off by 3.2e-5 with float32 sums, 6.5e-7 so); per-channel ones
+// carry the rounding of their float32 sums along (one token of -40 a block: 5.3e-6 without, 6.4e-7 with).  Per-channel
 // decays are folded into the rows once: q e^{prefix}, k e^{prefix}, k e^{suffix}; products between blocks carry the totals of
 // the blocks in between.  A block whose decay exceeds 2^64 in some channel is summed entry by entry.
 //
@@ -236,23 +237,33 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
     static_assert(NTHR == 4 * D, "one thread per block and channel");
     const int blk = tid / D, c = tid % D;
     if (tid < 4) sUn[tid] = 0.f;
-    float gr[16], suf = 0.f;
+    float gr[16], suf = 0.f, rest = 0.f;
+    auto add = [](float& sum, float& rest, float x) {   // sum + rest += x without a rounding of the sum
+      const float s = sum + x, y = s - sum;
+      rest += (sum - (s - y)) + (x - y);
+      sum = s;
+    };
+    auto factor = [](float sum, float rest) {   // 2^(sum + rest)
+      const float f = ex2(sum);
+      return f > 0.f ? fmaf(f, rest * 0.69314718f, f) : f;
+    };
 #pragma unroll
     for (int r = 0; r < 16; ++r) gr[r] = sE[(16 * blk + r) * LD + c];
 #pragma unroll
     for (int r = 15; r >= 0; --r) {
-      sE[(16 * blk + r) * LD + c] = sK[(16 * blk + r) * LD + c] * ex2(suf);
-      suf += gr[r];
+      sE[(16 * blk + r) * LD + c] = sK[(16 * blk + r) * LD + c] * factor(suf, rest);
+      add(suf, rest, gr[r]);
     }
+    sD[blk * D + c] = factor(suf, rest);
     float pre = 0.f;
+    rest = 0.f;
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      pre += gr[r];
-      const float f = ex2(pre);
+      add(pre, rest, gr[r]);
+      const float f = factor(pre, rest);
       sK[(16 * blk + r) * LD + c] *= f;
       sQ[(16 * blk + r) * LD + c] *= f;
     }
-    sD[blk * D + c] = ex2(suf);
     __syncthreads();
     if (!(suf >= -64.f)) sUn[blk] = 1.f;
     float bef = 1.f, aft = 1.f;

@@ -100,13 +100,16 @@ def test_per_channel_backward_with_strong_decay(T):
         assert torch.isfinite(got[name]).all() and _err(got[name], ref[name].double()) <= 2e-2, name
 
 
-@pytest.mark.parametrize("D,tokens,decay", [(64, 8, -80.0), (128, 8, -80.0), (64, 1, -1.0e5), (128, 3, float("-inf"))])
-def test_transition_form_reset_inside_a_block(D, tokens, decay):
-    """Scalar decays that drop the state at the head of every 16-row block: the weak decays behind them keep float32 precision (the
+@pytest.mark.parametrize("variant,D,tokens,decay", [("gated", 64, 8, -80.0), ("gated", 128, 8, -80.0), ("gated", 64, 1, -1.0e5),
+                                                    ("gated", 128, 3, float("-inf")), ("kda", 64, 1, -40.0), ("kda", 128, 1, -40.0),
+                                                    ("kda", 64, 2, float("-inf"))])
+def test_transition_form_reset_inside_a_block(variant, D, tokens, decay):
+    """Decays that drop the state at the head of every 16-row block: the weak decays behind them keep float32 precision (the
     bound is that of the other float32 cases), and an infinite log decay is a reset, not a NaN."""
-    i = O.make_inputs("gated", 1, 2, 200, D, D, seed=3, io_dtype=torch.float32, h0_std=0.1)
-    i["g"] = torch.where(torch.arange(200) % 16 < tokens, decay, -0.02).expand(1, 2, 200).contiguous()
-    o, s = _run("gated", {k: t.cuda() for k, t in i.items()})
+    i = O.make_inputs(variant, 1, 2, 200, D, D, seed=3, io_dtype=torch.float32, h0_std=0.1)
+    g = torch.where(torch.arange(200) % 16 < tokens, decay, -0.02)
+    i["g"] = (g.expand(1, 2, 200) if variant == "gated" else g[:, None].expand(1, 2, 200, D)).contiguous()
+    o, s = _run(variant, {k: t.cuda() for k, t in i.items()})
     assert _lib.last_path() == "chunk_transition"
-    ro, rs = _truth("gated", i)
+    ro, rs = _truth(variant, i)
     assert _err(o, ro) <= 5e-6 and _err(s, rs) <= 5e-6
