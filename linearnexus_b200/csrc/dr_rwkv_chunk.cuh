@@ -464,11 +464,16 @@ __global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecPar
   }
 }
 
-// 16-byte-aligned rows of K = 64 and whole 64-column slices; a decode step (one or two blocks) stays with the token kernel
-// RWKV-6 has no reduction on its token chain, and with more sequences than SMs the token recurrence, whose CTAs share an SM, stays
-// level or ahead (256 sequences: 747 against 759 us at T = 2048, 194 against 198 at 512); RWKV-7 gains there, too (887 against 754).
+// 16-byte-aligned rows of K = 64 and whole 64-column slices; a decode step (one block) stays with the token kernel.  While every slice
+// has an SM the blocks win from the second on (8 to 144 slices: 7.2 against 9.4 us at T = 9, 8.1 against 10.7 at 16, 17 against 25
+// at 64).  This kernel fills an SM, the token recurrence's CTAs share one: in several waves the blocks win late, at about 20 tokens per
+// wave (two waves: 17.8 against 16.8 us at T = 24, 24.3 against 27.0 at 48; three: 37.6 against 35.2 at 48, 76.6 against 80.4 at 128;
+// seven: 105 against 95 at 64, 180 against 178 at 128, 622 against 670 at 512).
+// RWKV-6 has no reduction on its token chain, and the token recurrence stays level or ahead in several waves (256 slices: 747
+// against 759 us at T = 2048, 194 against 198 at 512).
 inline bool eligible(int kind, bool bf, const LinRecParams& p, int sms) {
-  if (kind != LR_DPLR && (int64_t)p.B * p.H * (p.V / 64) > sms) return false;
+  const int64_t waves = sms > 0 ? ((int64_t)p.B * p.H * (p.V / 64) + sms - 1) / sms : 1;
+  if (waves > 1 && (kind != LR_DPLR || p.T < 20 * waves)) return false;
   const int ep = bf ? 8 : 4;
   auto ok = [&](const LrVec& v) { return (reinterpret_cast<uintptr_t>(v.p) & 15) == 0 && v.sb % ep == 0 && v.sh % ep == 0 && v.st % ep == 0; };
   return p.K == kK && p.V % 64 == 0 && p.T > kTB && p.s_v == 1 && ok(p.q) && ok(p.k) && ok(p.w) && ok(p.v) &&

@@ -81,3 +81,16 @@ def test_ssd_reset_then_accumulate(B, T, H, N, first, A):
     ry, rs = R.ssd_token_recurrence(d(x), d(dt), d(Ah), d(Bm), d(Cm), d(D), ssm_state=d(h0))
     _check(s, rs, 1.5e-6)
     _check(y, ry, 5e-3)
+
+
+@pytest.mark.parametrize("T", [9, 39, 40, 41])
+def test_rwkv_more_sequences_than_sms(T):
+    """Two waves of slices, on both sides of the line between the token recurrence and the blocks (20 tokens a wave)."""
+    g = torch.Generator().manual_seed(T)
+    f = lambda *s: torch.randn(*s, generator=g)
+    kk = torch.nn.functional.normalize(f(1, 150, T, 64), dim=-1)
+    x = (f(1, 150, T, 64), f(1, 150, T, 64) * 0.5, f(1, 150, T, 64), -kk, kk * torch.sigmoid(f(1, 150, T, 64)), -torch.exp(f(1, 150, T, 64) - 1.0))
+    o, s = L.dplr_delta_rule_recurrent(*(t.cuda() for t in x), scale=0.125)
+    ro, rs = R.dplr_delta_rule_recurrent(*(t.double() for t in x), scale=0.125, compute_dtype=torch.float64)
+    _check(o, ro, 5e-6)
+    _check(s, rs, 5e-6)
