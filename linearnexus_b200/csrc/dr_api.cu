@@ -121,16 +121,33 @@ int resolve_chunk_path(const DrDesc* d) {
 }
 
 // Shapes of the transition form, and its scratch where AUTO takes it (given that scratch); 0 elsewhere.
-//  * No tensor-core kernel for the storage types: in place of the token recurrence from two chunks on (with one chunk there is
-//    nothing to run in parallel).  DeltaNet's recurrence, without a decay per token, stays ahead up to half of the second
-//    chunk at K = V = 128 (32 sequences, T = 65: 34 against 44 us; T = 130: 57 against 49).
+//  * No tensor-core kernel for the storage types: in place of the token recurrence from two chunks on, where it is the faster one
+//    (recurrence_ahead).  The line at 64 tokens is not the crossover: with a decay per token and few sequences that lies at about 32
+//    (d = 64, 4 sequences: 41 against 22 us at T = 64, 23 against 22 at 32; d = 128: 56 against 36, 31 against 36).  DeltaNet's
+//    recurrence, without one, stays ahead up to half of the second chunk at K = V = 128 (32 sequences, T = 65: 33 against 43 us;
+//    T = 96 level).
 //  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.6 us per chunk, KDA's state
-//    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave and there are chunks
-//    enough to pay for the longer first pass (measured for 4, 8, 16 sequences: even at 5 chunks, 118 vs 90 us at 16 x 32
-//    chunks, 228 vs 80 us at 4 x 64; at 32 sequences the one-CTA kernels are ahead).  KDA switches from 17 chunks on: up to
-//    there its two-kernel form, what AUTO has always meant for it, is at most 15 us behind.  Past 32 chunks the two-kernel form
-//    overtakes it earlier (both first passes fill the chip then; 16 x 128 chunks: 340 against 357 us, 8 x 128: 292 against 267).
+//    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave (kTransUnits) and there
+//    are chunks enough to pay for the longer first pass (scalar decay: 30.8 against 30.3 us at 18 sequences x 7 chunks, 22.4
+//    against 30 at 4 or 8; 118 against 90 at 16 x 32, 228 against 80 at 4 x 64; at 32 sequences the one-CTA kernels are ahead).
+//    KDA switches from 17 chunks on; the two-kernel form it has up to there is behind from 10 chunks on for 18 sequences (50 against
+//    41 us at 16 chunks) and from 3 on for 4 (44 against 29).  Past 32 chunks the two-kernel form overtakes earlier (both first
+//    passes fill the chip then; 16 x 128 chunks: 340 against 357 us, 8 x 128: 292 against 267).
 // Both up to 1 GB of scratch.
+constexpr int kTransUnits = 148 / 8;
+// Whether the token recurrence beats the transition form from two chunks on, in microseconds measured for 4 to 512 sequences and 65 to
+// 1000 tokens.  The transition form's work grows with the chunks of all sequences, whole ones, while the recurrence is bound by its
+// chain until its CTAs fill the chip.  So the recurrence wins for many short sequences (d = 128, 128 sequences, T = 65: 72 against
+// 110 us gated, 45 against 107 DeltaNet; d = 64, 512 sequences: 109 against 134), and for DeltaNet at d = 128 from 128 sequences on
+// at any length (624 against 762 us at T = 1000).
+bool recurrence_ahead(const DrDesc* d) {
+  struct Cost { float fixed, chunk, token, unit_token; };   // transition: fixed + chunk * chunks; recurrence: per token, per sequence and token
+  static constexpr Cost cost[2][3] = {{{10.f, 0.11f, 0.37f, 0.00162f}, {10.f, 0.11f, 0.66f, 0.0027f}, {10.f, 0.138f, 0.68f, 0.0029f}},
+                                      {{20.f, 0.36f, 0.42f, 0.0047f}, {20.f, 0.36f, 0.93f, 0.0070f}, {20.f, 0.41f, 1.05f, 0.0076f}}};
+  const Cost& c = cost[d->K == 128][d->variant];
+  const float units = (float)d->B * (float)d->H, chunks = units * (float)((d->T + 63) / 64);
+  return 6.f + (float)d->T * std::max(c.token, units * c.unit_token) < c.fixed + chunks * c.chunk;
+}
 bool trans_eligible(const DrDesc* d) { return d->K == d->V && (d->K == 64 || d->K == 128); }
 int64_t trans_scratch(const DrDesc* d) {
   if (!trans_eligible(d)) return 0;
@@ -139,9 +156,9 @@ int64_t trans_scratch(const DrDesc* d) {
   if (d->path == DR_PATH_TRANSITION) return need;
   if (d->path != DR_PATH_AUTO || need > (int64_t)1 << 30) return 0;
   if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d))
-    return d->T > (d->variant == DR_DELTA && d->K == 128 ? 96 : 64) ? need : 0;
+    return d->T > (d->variant == DR_DELTA && d->K == 128 ? 96 : 64) && !recurrence_ahead(d) ? need : 0;
   const bool kda = d->variant == DR_KDA;
-  return units <= (kda && d->T > 32 * 64 ? 12 : 18) && d->T > (kda ? 16 : 5) * 64 ? need : 0;
+  return units <= (kda && d->T > 32 * 64 ? 12 : kTransUnits) && d->T > (kda ? 16 : 5) * 64 ? need : 0;
 }
 
 bool fp32_chunk_eligible(const DrDesc* d) { return d->chunk <= 64 && d->K <= 128; }

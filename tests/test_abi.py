@@ -142,6 +142,26 @@ def test_forward_workspace_sizes_need_no_gpu():
     assert need(_lib.DR_KDA, None, qkv=torch.empty(0)) == 0        # fp32 inputs stay on the exact kernel
 
 
+def test_float32_chunk_calls_take_the_faster_form():
+    """dr_workspace_bytes(desc, 2) of float32 chunk calls: scratch where AUTO takes the transition form, none where the token recurrence
+    is ahead (short inputs; many sequences)."""
+    import ctypes
+    import torch
+    from linearnexus_b200 import ops
+    lib = _lib.load()
+    f = torch.empty(0)
+    def transition(variant, D, units, T):
+        d = ops._desc(variant, _lib.DR_LAYOUT_BHTD, units, 1, T, D, D, 64, f, f, torch.float32, True, 0.1, None)
+        return int(lib.dr_workspace_bytes(ctypes.byref(d), 2)) > 0
+    D_, G_, K_ = _lib.DR_DELTA, _lib.DR_GATED, _lib.DR_KDA
+    for case in ((G_, 64, 8, 65), (G_, 64, 128, 65), (G_, 128, 64, 65), (G_, 128, 128, 300), (K_, 64, 512, 300), (K_, 128, 64, 130),
+                 (D_, 64, 8, 512), (D_, 64, 128, 130), (D_, 128, 32, 97), (D_, 128, 64, 1000)):
+        assert transition(*case), case
+    for case in ((G_, 64, 8, 64), (D_, 128, 32, 96), (G_, 64, 512, 65), (G_, 128, 128, 65), (G_, 128, 512, 130), (K_, 64, 512, 65),
+                 (K_, 128, 128, 130), (D_, 64, 512, 1000), (D_, 128, 128, 1000), (D_, 128, 64, 130)):
+        assert not transition(*case), case
+
+
 def test_grouped_head_count_is_validated_on_the_host():
     """DrDesc.qk_heads: 0 or a divisor of H; anything else is a shape error before any launch."""
     import ctypes
