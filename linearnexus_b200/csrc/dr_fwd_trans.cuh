@@ -30,8 +30,9 @@
 namespace dr {
 namespace trans {
 
-using mma::AFrag;
-using mma::BFrag;
+// operands in two tf32 terms: three products per pair, float32 precision
+using AFrag = mma::AFrag<true>;
+using BFrag = mma::BFrag<true>;
 constexpr int kC = 64;
 constexpr int LDX = 72;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -71,7 +72,7 @@ __device__ __forceinline__ float4 load4(const void* base, int64_t at, int dt) {
 
 // T = (I + diag(rs) A)^-1 in place for a strictly lower-triangular 64 x 64 A (row stride LDX): 8 x 8 diagonal blocks by
 // substitution, then three merge levels T_10 = -T_11 (diag(rs) A_10) T_00.  Above the diagonal: scratch.
-template <bool X3, int NW>
+template <int NW>
 __device__ __forceinline__ void inverse_64(float* sT, const float* rs, int tid) {
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   if (tid < 64) {
@@ -108,8 +109,8 @@ __device__ __forceinline__ void inverse_64(float* sT, const float* rs, int tid) 
         zero4(d);
 #pragma unroll 1
         for (int k = t; k < bs; k += 8) {
-          AFrag<X3> a;
-          BFrag<X3> b;
+          AFrag a;
+          BFrag b;
           if (step == 0) {   // diag(rs) A_10 T_00 -> the mirrored block (rows c0 .., columns r0 ..)
             a.set(m0 < bs ? sT[(r0 + m0) * LDX + c0 + k] : 0.f, m1 < bs ? sT[(r0 + m1) * LDX + c0 + k] : 0.f,
                   m0 < bs ? sT[(r0 + m0) * LDX + c0 + k + 4] : 0.f, m1 < bs ? sT[(r0 + m1) * LDX + c0 + k + 4] : 0.f);
@@ -119,7 +120,7 @@ __device__ __forceinline__ void inverse_64(float* sT, const float* rs, int tid) 
                   m0 < bs && k + 4 <= m0 ? sT[(r0 + m0) * LDX + r0 + k + 4] : 0.f, m1 < bs && k + 4 <= m1 ? sT[(r0 + m1) * LDX + r0 + k + 4] : 0.f);
             b.set(sT[(c0 + k) * LDX + r0 + n], sT[(c0 + k + 4) * LDX + r0 + n]);
           }
-          mma::fma<X3>(d, a, b);
+          mma::fma<true>(d, a, b);
         }
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
@@ -136,7 +137,7 @@ __device__ __forceinline__ void inverse_64(float* sT, const float* rs, int tid) 
   }
 }
 
-template <int D, bool KDA, bool X3>
+template <int D, bool KDA>
 __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_kernel(const __grid_constant__ Params P) {
   pdl_entry();
   using Z_ = Sizes<D>;
@@ -296,13 +297,13 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
         if (bj == mt) { f0 = 1.f / sD[mt * D + c0]; f1 = 1.f / sD[mt * D + c1]; }
         for (int x = bj + 1; x < mt; ++x) { f0 *= sD[x * D + c0]; f1 *= sD[x * D + c1]; }
       }
-      AFrag<X3> ak, aq;
+      AFrag ak, aq;
       ak.set(sK[r0 * LD + c0], sK[r1 * LD + c0], sK[r0 * LD + c1], sK[r1 * LD + c1]);
       aq.set(sQ[r0 * LD + c0], sQ[r1 * LD + c0], sQ[r0 * LD + c1], sQ[r1 * LD + c1]);
-      BFrag<X3> bk;
+      BFrag bk;
       bk.set(kj[j * LD + c0] * f0, kj[j * LD + c1] * f1);
-      mma::fma<X3>(dk, ak, bk);
-      mma::fma<X3>(dq, aq, bk);
+      mma::fma<true>(dk, ak, bk);
+      mma::fma<true>(dq, aq, bk);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
     }
   }
   __syncthreads();
-  inverse_64<X3, NW>(sX, sBeta, tid);   // ends with a barrier
+  inverse_64<NW>(sX, sBeta, tid);   // ends with a barrier
   // ---- W^T and U^T of the warp's 16 channels / value columns (two warps share them): rows = columns of W / U, columns = tokens ---------
   const int own = warp % CT, part = warp / CT, ch0 = 16 * own + g, ch1 = ch0 + 8;
   float W[8][4], U[8][4];
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
       w00 = w01 = b0 * sEG[j0];
       w10 = w11 = b1 * sEG[j1];
     }
-    AFrag<X3> aw, au;
+    AFrag aw, au;
     aw.set(sK[j0 * LD + ch0] * w00, sK[j0 * LD + ch1] * w01, sK[j1 * LD + ch0] * w10, sK[j1 * LD + ch1] * w11);
     au.set(sV[j0 * LD + ch0] * b0, sV[j0 * LD + ch1] * b0, sV[j1 * LD + ch0] * b1, sV[j1 * LD + ch1] * b1);
 #pragma unroll
@@ -371,10 +372,10 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
       if (nt >= ks) {
         const int i = 8 * nt + g;
         const float2 x = ld2(sX + i * LDX + j0);
-        BFrag<X3> bt;
+        BFrag bt;
         bt.set(j0 <= i ? x.x : 0.f, j1 <= i ? x.y : 0.f);
-        mma::fma<X3>(W[nt], aw, bt);
-        mma::fma<X3>(U[nt], au, bt);
+        mma::fma<true>(W[nt], aw, bt);
+        mma::fma<true>(U[nt], au, bt);
       }
     }
   }
@@ -397,14 +398,14 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
   }
   __syncthreads();
   // ---- [Kd^T; A] [W | U]: an accumulator of W^T or U^T is, register for register, the B operand of its columns ----------------------------
-  auto products = [&](float (&w)[2][4], float (&u)[2][4], int ks, const AFrag<X3>& a) {
+  auto products = [&](float (&w)[2][4], float (&u)[2][4], int ks, const AFrag& a) {
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-      BFrag<X3> bw, bu;
+      BFrag bw, bu;
       bw.set(W[ks][2 * hf], W[ks][2 * hf + 1]);
       bu.set(U[ks][2 * hf], U[ks][2 * hf + 1]);
-      mma::fma<X3>(w[hf], a, bw);
-      mma::fma<X3>(u[hf], a, bu);
+      mma::fma<true>(w[hf], a, bw);
+      mma::fma<true>(u[hf], a, bu);
     }
   };
 #pragma unroll 1
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const float* k0 = sK + (8 * ks + 2 * t) * LD + 16 * mt + g;
-      AFrag<X3> a;
+      AFrag a;
       a.set(k0[0], k0[8], k0[LD], k0[LD + 8]);
       products(w, u, ks, a);
     }
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
     for (int ks = 0; ks < 8; ++ks) {
       if (ks <= 2 * mt + 1) {
         const float2 x0 = ld2(sA + (16 * mt + g) * LDX + 8 * ks + 2 * t), x1 = ld2(sA + (16 * mt + g + 8) * LDX + 8 * ks + 2 * t);
-        AFrag<X3> a;
+        AFrag a;
         a.set(x0.x, x1.x, x0.y, x1.y);
         products(w, u, ks, a);
       }
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(Sizes<D>::NTHR, D == 64 ? 2 : 1) trans_pre_ker
 }
 
 // Warps 0 .. D/16 - 1: state rows 16 w ..; four more warps: output rows 16 (w - D/16) ...  NT: 8-column tiles per CTA.
-template <int D, bool X3, int NT>
+template <int D, int NT>
 __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const __grid_constant__ Params P) {
   pdl_entry();
   constexpr int CT = D / 16, VS = 8 * NT, LDP = 2 * VS + 8;   // S in shared memory: row pairs interleaved [D / 2][VS][2]
@@ -524,15 +525,15 @@ __global__ void __launch_bounds__((D / 16 + 4) * 32, 1) trans_state_kernel(const
     for (int nt = 0; nt < NT; ++nt) c[nt] = get_c(cn, nt);
 #pragma unroll
     for (int ks = 0; ks < D / 8; ++ks) {
-      AFrag<X3> fr;
+      AFrag fr;
       fr.set(a[ks].x, a[ks].y, a[ks].z, a[ks].w);
       a[ks] = get_a(cn, ks);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
-        BFrag<X3> bs;
+        BFrag bs;
         bs.set(y.x, y.y);
-        if (ks & 1) mma::fma<X3>(e[nt], fr, bs); else mma::fma<X3>(d[nt], fr, bs);
+        if (ks & 1) mma::fma<true>(e[nt], fr, bs); else mma::fma<true>(d[nt], fr, bs);
       }
     }
     if (state) {
@@ -575,7 +576,7 @@ inline int64_t workspace_bytes(int64_t units, int T, int D) {
   return units * ((T + kC - 1) / kC) * 4 * (D == 128 ? Sizes<128>::kFloats : Sizes<64>::kFloats);
 }
 
-template <int D, bool KDA, bool X3>
+template <int D, bool KDA>
 inline cudaError_t launch_t(const FwdParams& p, void* workspace, int sms, cudaStream_t stream) {
   using Z = Sizes<D>;
   thread_local int attr_dev = -1;
@@ -583,7 +584,7 @@ inline cudaError_t launch_t(const FwdParams& p, void* workspace, int sms, cudaSt
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (attr_dev != dev) {
-    e = cudaFuncSetAttribute(trans_pre_kernel<D, KDA, X3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z::smem(KDA));
+    e = cudaFuncSetAttribute(trans_pre_kernel<D, KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z::smem(KDA));
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
@@ -597,17 +598,17 @@ inline cudaError_t launch_t(const FwdParams& p, void* workspace, int sms, cudaSt
   P.yf = reinterpret_cast<float4*>(f); f += nc * Z::fY;
   P.of = reinterpret_cast<float4*>(f); f += nc * Z::fO;
   P.el = f;
-  e = launch_pdl(trans_pre_kernel<D, KDA, X3>, dim3((unsigned)nc), dim3(Z::NTHR), Z::smem(KDA), stream, P);
+  e = launch_pdl(trans_pre_kernel<D, KDA>, dim3((unsigned)nc), dim3(Z::NTHR), Z::smem(KDA), stream, P);
   if (e != cudaSuccess) return e;
   // narrow slices while they fit one wave: the chain's length is what counts, and every slice adds readers of N and Y
   if (units * (D / 16) <= sms)
-    return launch_pdl(trans_state_kernel<D, X3, 2>, dim3((unsigned)(units * (D / 16))), dim3((D / 16 + 4) * 32), 0, stream, P);
-  return launch_pdl(trans_state_kernel<D, X3, 4>, dim3((unsigned)(units * (D / 32))), dim3((D / 16 + 4) * 32), 0, stream, P);
+    return launch_pdl(trans_state_kernel<D, 2>, dim3((unsigned)(units * (D / 16))), dim3((D / 16 + 4) * 32), 0, stream, P);
+  return launch_pdl(trans_state_kernel<D, 4>, dim3((unsigned)(units * (D / 32))), dim3((D / 16 + 4) * 32), 0, stream, P);
 }
 
-template <int D, bool X3>
+template <int D>
 inline cudaError_t launch_d(const FwdParams& p, void* workspace, int sms, cudaStream_t stream) {
-  return p.variant == DR_KDA ? launch_t<D, true, X3>(p, workspace, sms, stream) : launch_t<D, false, X3>(p, workspace, sms, stream);
+  return p.variant == DR_KDA ? launch_t<D, true>(p, workspace, sms, stream) : launch_t<D, false>(p, workspace, sms, stream);
 }
 
 }  // namespace trans

@@ -65,7 +65,7 @@ inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC -
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
-constexpr int IN_G = 0;                          // log2(e) G   fp32 [64][132]
+constexpr int IN_G = 0;                          // log2(e) G   fp32 [64][136]
 constexpr int IN_K = IN_G + 64 * LDF * 4;        // raw k       bf16 [64][136]
 constexpr int IN_Q = IN_K + 64 * LDH * 2;        // raw q       bf16 [64][136]
 constexpr int IN_AKK = IN_Q + 64 * LDH * 2;      // A_kk fp32 [64][68]; later the W staging tile bf16 [64][136]
@@ -159,7 +159,8 @@ struct IntraPackedParams : IntraParams {
   SeqTable seqs;
 };
 // The pass in transition form (see "few sequences" below): fragments instead of records.
-struct IntraTransParams : IntraParams {
+struct IntraTransParams {
+  FwdParams p;
   uint4 *nf, *yf;     // [chunks][8 | 4 row tiles][8 k-steps][32 lanes]: A operands of m16n8k16
   float4 *zf, *of;    // [chunks][8 | 4 row tiles][16 column tiles][32 lanes]: addends
   float* el;          // [chunks][128] e^{G_L}
@@ -203,7 +204,8 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   int T = p.map.T, n, b, h, tok0 = 0;
-  uint8_t* rec = P.ws;
+  uint8_t* rec = nullptr;
+  if constexpr (!kTrans) rec = P.ws;
   if constexpr (kPacked) {
     h = blockIdx.x / P.seqs.chunks;
     const int c = blockIdx.x % P.seqs.chunks;
@@ -1163,7 +1165,6 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   IntraTransParams P;
   uint8_t* w = reinterpret_cast<uint8_t*>(workspace);
   P.p = p;
-  P.ws = nullptr;
   P.nf = reinterpret_cast<uint4*>(w); w += nc * kTrN;
   P.yf = reinterpret_cast<uint4*>(w); w += nc * kTrY;
   P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;

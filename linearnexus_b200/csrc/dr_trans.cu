@@ -9,7 +9,7 @@ int64_t trans_workspace_bytes(int64_t units, int T, int D, bool bf16_tensor) {
 }
 cudaError_t launch_chunk_trans(const FwdParams& p, bool bf16_tensor, void* workspace, int sms, cudaStream_t stream) {
   if (bf16_tensor) return launch_chunk_trans_bf16(p, workspace, sms, stream);
-  return p.K == 64 ? trans::launch_d<64, true>(p, workspace, sms, stream) : trans::launch_d<128, true>(p, workspace, sms, stream);
+  return p.K == 64 ? trans::launch_d<64>(p, workspace, sms, stream) : trans::launch_d<128>(p, workspace, sms, stream);
 }
 
 }  // namespace dr
