@@ -12,7 +12,8 @@
 // selective reset: A dt of -80 a token) a float32 sum has lost the small decays of the tokens behind it.  So G is summed in
 // 64 bits and kept as a float32 pair, and a difference is formed part by part: its error is that of the difference itself.  Reset of
 // 32 tokens at A dt = -80, then 0.32 a token: the state is off by 2.6e-7 of its largest entry (T = 64; 1.2e-7 at T = 1100), 8.3e-5
-// with float32 sums; the token recurrence by 9e-8.  At B=8, T=4096, H=16, N=128 this takes 334 us, float32 sums 322.
+// with float32 sums; the token recurrence by 9e-8.  B=8, T=4096, H=16, N=128:
+// 319 us (334 with the scan behind the state update on a warp with three tiles of P; float32 sums there: 322).
 //
 // One CTA of eight warps per (batch, head, 64 value rows).  Warp w keeps S rows 16 (w & 3).. and state columns of half
 // w >> 2 in accumulator registers for the whole sequence: an m16n8 accumulator of S is, register for register, the B
@@ -39,6 +40,7 @@ namespace ssd {
 
 constexpr int kC = 64, kP = 64, kThreads = 256;
 constexpr int LDX = kP + 8;    // row stride of the x, P and y tiles (bf16)
+constexpr int kScanWarp = 5;       // takes dt to the scalars; one of the warps with two tiles of P (0-3 have three)
 constexpr int kScalars = 5 * kC;   // per-token scalars of a stage
 // A token's log decay is cut off here: what crosses the token is 0 in float32 either way (the decays of a head have one sign),
 // and the sums stay finite and within the pair's 48 bits.
@@ -125,10 +127,10 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
     }
     tc::cp_async_commit();
   };
-  // dt of the next chunk (warp 0, two tokens per lane), then its scan: G, e^G, dt, dt e^{G_L - G}
+  // dt of the next chunk (one warp, two tokens per lane), then its scan: G, e^G, dt, dt e^{G_L - G}
   float dt_lo = 0.f, dt_hi = 0.f;
   auto fetch_dt = [&](int c) {
-    if (warp == 0) {
+    if (warp == kScanWarp) {
       const int t0 = c * kC + lane;
       const int64_t at = (int64_t)t0 * p.dt.st, at32 = (int64_t)(t0 + 32) * p.dt.st;
       dt_lo = t0 < T && in_bounds(p.status, dt_at + at, p.dt.n) ? gdt[at] : 0.f;
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
     }
   };
   auto scan_dt = [&](int c, int st) {
-    if (warp == 0) {
+    if (warp == kScanWarp) {
       const int t0 = c * kC + lane;
       float* sc = scalars(st);
       const float d0 = t0 < T ? fminf(fmaxf(softplus_f(dt_lo + bias_h), p.dt_lo), p.dt_hi) : 0.f;
@@ -321,6 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
 #pragma unroll
       for (int r = 0; r < 2; ++r) { y[mt][r][0] *= e0; y[mt][r][1] *= e0; y[mt][r][2] *= e1; y[mt][r][3] *= e1; }
     }
+    if (c + 1 < c_hi) scan_dt(c + 1, st ^ 1);   // (the last reader of that stage's scalars was the previous chunk's state update)
     __syncthreads();   // P is complete
     // ---- + P x: the 16-token blocks 0 and 3 by one half of the warps, 1 and 2 by the other (five products each) --------
 #pragma unroll
@@ -371,7 +374,6 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
       }
     }
     state_update(st);
-    if (c + 1 < c_hi) scan_dt(c + 1, st ^ 1);
     __syncthreads();   // the output rows are complete
 #pragma unroll
     for (int i = tid; i < kC * (kP / 8); i += kThreads) {
