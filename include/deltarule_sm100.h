@@ -127,7 +127,8 @@ const char* dr_last_path(void);
  * given less returns DR_ERR_WORKSPACE (there is no silent downgrade to a slower kernel: ask for
  * DR_PATH_FP32 to run without scratch).
  * op=2: scratch with which dr_chunk_fwd is at its fastest -- at least the op=0 figure; shapes that AUTO runs on the token
- * recurrence without scratch (float32 storage with K = V = 64 or 128, more than one chunk) run chunk-parallel with it.
+ * recurrence without scratch (float32 storage with K = V = 64 or 128, more than one chunk) run chunk-parallel with it where
+ * that is the faster form, and few long bf16 sequences at K = V = 128 as well.
  * op=1 returns DR_ERR_UNSUPPORTED for shapes the backward does not cover: chunk > 64, K > 128,
  * or DR_KDA with K % 16 != 0 (the forward entry points accept those shapes). */
 int64_t dr_workspace_bytes(const DrDesc* desc, int op);
@@ -154,8 +155,9 @@ int dr_chunk_fwd(const DrDesc* desc, const void* q, const void* k, const void* v
  * h0, hT: float32 [n_seqs, H, K, V] or null.  desc: B and T are ignored (B = 1 and T = each sequence's length are
  * filled in per sequence), layout must be DR_LAYOUT_BTHD.  Every sequence starts from its own initial state and
  * is cut into chunks from its own first token, so no chunk straddles a boundary; the result equals the
- * reference op run on each sequence alone.  One launch sequence per sequence on `stream`, no copies; workspace as
- * for dr_chunk_fwd sized for the longest sequence (dr_workspace_bytes with T = that length, B = 1).
+ * reference op run on each sequence alone.  At the tensor-core shape one launch (KDA: two) over all sequences the workspace
+ * holds, else one launch per sequence, on `stream`, no copies.  Workspace: at least what dr_chunk_fwd needs for the longest sequence
+ * (dr_workspace_bytes(desc, 0) with T = that length, B = 1); with more, up to T = total_T + 64 n_seqs, fewer launches.
  */
 int dr_chunk_fwd_varlen(const DrDesc* desc, const void* q, const void* k, const void* v, const void* g,
                         const float* beta, const int32_t* cu_seqlens_host, int32_t n_seqs, const float* h0, void* o,
@@ -196,7 +198,7 @@ int dr_step(const DrDesc* desc, const void* q, const void* k, const void* v, con
  * dr_chunk_bwd_saved, which is dr_chunk_bwd without the recomputation.  Under jax this is the fwd / bwd pair of a
  * jax.custom_vjp around the three *_chunkwise functions, the workspace being the residual.
  * desc->path is ignored (the forward kernel is chosen by shape as in dr_chunk_bwd); out_dtype as in dr_chunk_fwd.
- * For bf16 DeltaNet / Gated DeltaNet the saving forward also leaves the adjoint's chunk-parallel pre-pass results in
+ * For bf16 DeltaNet / Gated DeltaNet, and KDA at K = V = 128, the saving forward also leaves the adjoint's chunk-parallel pre-pass in
  * the workspace; that kernel runs beside the forward on a non-blocking side stream the library creates once per
  * device, forked from and joined to `stream` with events (stream order as seen by the caller is unchanged).
  */

@@ -18,7 +18,7 @@
 // What bounds it: the chain of a block through the dots, U and the update, 2.6 K cycles with the schedulers 55 % and the tensor pipe 35 %
 // busy (B=8, T=4096, H=16: 868 us with four warps of 64 keys and products in source order, 820 with them free to move, 785
 // with eight warps, 761 with the B operands split once by the staging warps; two staging groups instead of three: 872; 690 with
-// running products in blocks of too strong a decay).
+// running products in blocks of too strong a decay; 681 with the stages handed back by mbarriers).
 // The token recurrence it replaces here ran
 // at 540 cycles per token whatever its instruction count or prefetch depth: one dependent reduce-and-update chain per token, and
 // 260 shared-memory wavefronts per token to feed 160 multiply-adds per thread (a 16-byte load fills a quarter of a warp per

@@ -1,9 +1,9 @@
 """The other matrix-state scans of LinearNexus over the sm_100a C ABI: RWKV-7 DPLR, RWKV-6, Mamba-2 SSD.
 
 Names, argument order, keyword defaults, shapes and output dtypes follow the LinearNexus functions cited per
-function (paths relative to the LinearNexus tree); arrays are torch CUDA tensors.  All three run the token
-recurrence with the float32 state in registers (``csrc/dr_linrec.cuh``); a chunked tensor-core form exists for the
-delta-rule family only.  There is no CPU path.
+function (paths relative to the LinearNexus tree); arrays are torch CUDA tensors.  At the models' shapes they run in chunk
+form on the tensor cores in float32 precision (``csrc/dr_rwkv_chunk.cuh``, ``csrc/dr_ssd_chunk.cuh``), elsewhere as the token
+recurrence with the float32 state in registers (``csrc/dr_linrec.cuh``).  There is no CPU path.
 """
 from __future__ import annotations
 

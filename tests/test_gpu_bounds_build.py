@@ -1,6 +1,7 @@
 """The debug build with index checks (-DDR_BOUNDS_CHECK) on tiny, ragged and odd shapes: T in {1, 63, 64, 65, 130},
 d in {64, 128} and a size that is a multiple of nothing, every variant, fp32 and bf16, through the recurrence, the AUTO
-chunk path and the fp32 chunk kernel, plus the RWKV / SSD scans.  No index may leave its array (status word clean),
+chunk path and the fp32 chunk kernel, plus the RWKV / SSD scans (odd sizes, and the tile edges of their chunk forms) and the
+transition forms.  No index may leave its array (status word clean),
 and the outputs must equal the release build's bit for bit: the checks change nothing but what they skip.  The release
 run is repeated as well: the same launch twice has to give the same bits (a race would not)."""
 import os

@@ -36,7 +36,7 @@ def test_ssd_chunks(B, T, H, P, N, G):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,H,T,V,layout", [(1, 2, 9, 64, "bhtd"), (2, 3, 31, 128, "bthd"), (1, 2, 130, 64, "bhtd"), (1, 1, 203, 192, "bhtd")])
 def test_rwkv_blocks(dtype, B, H, T, V, layout):
-    """Four tokens per step of the state: tails of every length, several value slices, strong and vanishing decays."""
+    """Eight tokens per step of the state: tails of every length, several value slices, strong and vanishing decays."""
     g = torch.Generator().manual_seed(T)
     f = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).to(dtype)
     kk = torch.nn.functional.normalize(torch.randn(B, H, T, 64, generator=g), dim=-1)

@@ -93,8 +93,8 @@ def test_tcgen05_is_default_for_headline_shape():
 @pytest.mark.parametrize("variant", ["gated", "delta"])
 @pytest.mark.parametrize("T", [100, 320])
 def test_tcgen05_without_tma_inputs(variant, T):
-    """Inputs the tensor maps cannot describe -- [B,T,H,D] storage (rows of a sequence not contiguous) or a
-    length that is not a multiple of 8 -- take the per-thread copy path of the same kernel: same results."""
+    """[B,T,H,D] storage (rows of a sequence not contiguous) and lengths that are no multiple of 8 or of a chunk: other tensor maps,
+    the same tiles, so the same results bit for bit."""
     inp = O.make_inputs(variant, 2, 3, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
     o, hT = _run(variant, inp, "tcgen05")
     ro, rS = _truth(variant, inp)
@@ -109,8 +109,6 @@ def test_tcgen05_without_tma_inputs(variant, T):
                                                initial_state=cu["h0"], chunk_size=64, path="tcgen05")
     assert _lib.last_path() == "chunk_tcgen05"
     assert o2.transpose(1, 2).is_contiguous()
-    # the two load paths feed identical tiles to identical products
-    if T % 8 == 0:
-        assert _rel(o2, ro) <= BF16_TOL and _rel(hT2, rS) <= BF16_TOL
-    else:
-        assert torch.equal(o2, o) and torch.equal(hT2, hT)
+    # both storages feed identical tiles to identical products
+    assert _rel(o2, ro) <= BF16_TOL and _rel(hT2, rS) <= BF16_TOL
+    assert torch.equal(o2, o) and torch.equal(hT2, hT)
