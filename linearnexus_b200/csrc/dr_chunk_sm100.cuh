@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(16) Ctl ctl;   // its float arrays are read with 16-byte loads
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int grp = warp >> 2;             // 0 PA, 1 PB, 2 CA, 3 CB
   const int gt = tid & (kGrp - 1);       // thread index inside its group = tensor-memory lane it owns
   const int wq = warp & 3;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
     issue_kq(0);
     clear_tail(0);
     if (warp == 0) { tc::cp_async_wait_all(); __syncwarp(); scan_stage(0); }
-    if (gt == 64) issue_d1(0);
+    if (wq == 2 && tc::elect_one()) issue_d1(0);
     if (nchunks > 1) issue_kq(1);   // the copies run two chunks ahead of the masks (see the end of the loop body)
     uint32_t phP = 0;
     for (int n = 0; n < nchunks; ++n) {
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       // what the NEXT chunk needs from this group, behind the hand-over
       if (n + 1 < nchunks) {
         clear_tail(n + 1);
-        if (gt == 64) issue_d1(n + 1);       // completes behind PB's inverse of this chunk
+        if (wq == 2 && tc::elect_one()) issue_d1(n + 1);       // completes behind PB's inverse of this chunk
         if (warp == 0) { tc::cp_async_wait_all(); __syncwarp(); scan_stage(n + 1); }
       }
       // chunk n-2 has left the consumer: its ring tile and its scalar and rq slots, (n+2) % 4, are free.  The copies of
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       }
       group_sync128(3);
       // ---- (3) V_new^T = U^T - S^T W^T --------------------------------------------------------------------
-      if (gt == 0) {
+      if (wq == 0 && tc::elect_one()) {
         wait_bar(&ctl.wrdy, n & 1);          // W tile written by CB
         wait_bar(&ctl.barUW, n & 1);         // U^T complete
         tc::tc_fence_after();
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       tc::tc_fence_before();
       group_sync128(3);
       // ---- (5) S^T += (decayed V_new^T) K^ ;  (4) Do = V_new^T A_qk^T -------------------------------------------
-      if (gt == 0) {
+      if (wq == 0 && tc::elect_one()) {
         tc::tc_fence_after();
         const uint64_t kd0 = tc::smem_desc_sw128(aQK, QK_PANEL, 1024);  // K^ MN-major
 #pragma unroll
@@ -568,8 +568,8 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
     // The group's three products per chunk are issued by threads of three different warps (a product blocks its issuing
     // thread for 330-540 cycles, and the warps meet again at the group's next barrier): W^T by thread 0, U^T and the V
     // copy by thread 32, Dq by thread 64.  Each commits to its own barrier.
-    constexpr int kUThread = 32, kDqThread = 64;
-    // V rows of chunk m -> tile (thread kUThread)
+    constexpr int kUWarp = 1, kDqWarp = 2;
+    // V rows of chunk m -> tile (warp kUWarp)
     auto issue_v = [&](int m) {
       const uint32_t bar = tc::smem_u32(&ctl.vb), dst = tc::smem_u32(sV);
       tc::mbar_arrive_expect_tx(bar, 2 * V_PANEL);
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
         if (c0 == kC - 16) {
           tc::tc_fence_before();
           group_sync128(4);      // Dq and this stage's accumulator are in registers, in every thread
-          if (next >= 0 && gt == kDqThread) issue_dq(next);
+          if (next >= 0 && wq == kDqWarp && tc::elect_one()) issue_dq(next);
         }
         if (go) {
           // phases kept apart by hand: 8 packed pairs, then 8 exchanges, then 8 stores
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       }
     };
 
-    if (gt == kUThread) issue_v(0);
+    if (wq == kUWarp && tc::elect_one()) issue_v(0);
     for (int n = 0; n < nchunks; ++n) {
       const int s = n & 1;
       const uint32_t aQK = tc::smem_u32(smem + SM_QKR + (n % kRing) * QK_TILE);
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       wait_bar(&ctl.full[n % 3], (n / 3) & 1);
       tc::tc_fence_after();
       // ---- (2a) W^T = K^T Tw^T -> this stage's accumulator, idle until U^T is issued into it ---------------
-      if (gt == 0) {
+      if (wq == 0 && tc::elect_one()) {
         const uint64_t kd0 = tc::smem_desc_sw128(aQK, QK_PANEL, 1024);   // K MN-major, 16 chunk rows per step
         const uint64_t twd0 = tc::smem_desc(aXB + XB_TW, 128, A_RBS);
 #pragma unroll 1
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       // ---- (2b) U^T = V^T Tb^T -> the same accumulator ---------------------------------------------------
       if constexpr (kPacked) {
         const int rowsn = T - n * kC;
-        if (rowsn < kC && wq == kUThread / 32) {   // see clear_tail
+        if (rowsn < kC && wq == kUWarp) {   // see clear_tail
           wait_bar(&ctl.vb, n & 1);
           for (int i = lane; i < (kC - rowsn) * 16; i += 32)
             *reinterpret_cast<uint4*>(sV + (i & 8) / 8 * V_PANEL + (rowsn + (i >> 4)) * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
           __syncwarp();
         }
       }
-      if (gt == kUThread) {
+      if (wq == kUWarp && tc::elect_one()) {
         tc::tc_fence_after();
         wait_bar(&ctl.vb, n & 1);
         tc::tc_fence_after();
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
         wait_bar(&ctl.barDq, (n - 1) & 1);
         tc::tc_fence_after();
         out_epilogue(n - 1, n);
-      } else if (gt == kDqThread) {
+      } else if (wq == kDqWarp && tc::elect_one()) {
         issue_dq(0);
       }
     }

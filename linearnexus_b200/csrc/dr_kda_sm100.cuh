@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   const FwdParams& p = P.p;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) StateCtl ctl;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int hs = (tid >> 7) & 1, l128 = tid & 127;
   int T = p.map.T, unit = blockIdx.x, tok0 = 0;
   int b = unit / p.map.H;
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
 
   if (warp == 8) {
     // =========================== ISSUING WARP (one thread) ======================================================
-    if (tid == kThreads) {
+    if (tc::elect_one()) {
       // the record of chunk m -> buffer m & 1, the V rows straight from the input
       auto issue_load = [&](int m) {
         const uint32_t bar = tc::smem_u32(&ctl.full[m & 1]);
