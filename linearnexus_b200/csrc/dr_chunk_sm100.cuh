@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       wait_bar(&ctl.kq[m % kRing], (m / kRing) & 1);
       tc::tc_fence_after();
       const uint64_t ad0 = tc::smem_desc_sw128(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE), 16, 1024);
-#pragma unroll 1
+#pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
         const uint64_t ad = desc_adv(ad0, (ks >> 2) * QK_PANEL + (ks & 3) * 32);
         tc::mma_ss(tbase + TM_D1, ad, ad, id_n64, ks > 0);
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       wait_bar(&ctl.sbrdy, m & 1);
       tc::tc_fence_after();
       const uint64_t qd0 = tc::smem_desc_sw128(tc::smem_u32(smem + SM_QKR + (m % kRing) * QK_TILE) + QK_PANEL / 2, 16, 1024);   // rows 64..127
-#pragma unroll 1
+#pragma unroll
       for (int ks = 0; ks < 8; ++ks)
         tc::mma_ts(tbase + TM_DQ, tbase + TM_SB + ks * 8, desc_adv(qd0, (ks >> 2) * QK_PANEL + (ks & 3) * 32), id_n64, ks > 0);
       tc::mma_commit(tc::smem_u32(&ctl.barDq));
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
       if (wq == 0 && tc::elect_one()) {
         const uint64_t kd0 = tc::smem_desc_sw128(aQK, QK_PANEL, 1024);   // K MN-major, 16 chunk rows per step
         const uint64_t twd0 = tc::smem_desc(aXB + XB_TW, 128, A_RBS);
-#pragma unroll 1
+#pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(kd0, ks * 2048), desc_adv(twd0, ks * 256), id_n64_amn, ks > 0);
         tc::mma_commit(tc::smem_u32(&ctl.barW));
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
         tc::tc_fence_after();
         const uint64_t vd0 = tc::smem_desc_sw128(tc::smem_u32(sV), V_PANEL, 1024);
         const uint64_t tbd0 = tc::smem_desc(aXB + XB_TB, 128, A_RBS);
-#pragma unroll 1
+#pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           tc::mma_ss(tbase + TM_DU + 64 * s, desc_adv(vd0, ks * 2048), desc_adv(tbd0, ks * 256), id_n64_amn, ks > 0);
         tc::mma_commit(tc::smem_u32(&ctl.barUW));
