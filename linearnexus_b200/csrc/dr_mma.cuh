@@ -63,5 +63,17 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& p1, uint32_t&
   p3 = pack(x, y);
 }
 
+// The same by truncation: 8 + 8 + 8 bits, so the three terms add up to the float exactly (rounding needs the terms' signs for
+// that); eleven instructions either way, these without a conversion.  Infinities come out as inf, NaN, NaN.
+__device__ __forceinline__ void split3_exact(float x, float y, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+  uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+  p1 = __byte_perm(a, b, 0x7632);
+  x -= __uint_as_float(a & 0xffff0000u); y -= __uint_as_float(b & 0xffff0000u);
+  a = __float_as_uint(x); b = __float_as_uint(y);
+  p2 = __byte_perm(a, b, 0x7632);
+  x -= __uint_as_float(a & 0xffff0000u); y -= __uint_as_float(b & 0xffff0000u);
+  p3 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+
 }  // namespace mma
 }  // namespace dr
