@@ -8,7 +8,7 @@
 //     y  = e^{G_i} Y1 + Y2 + D x;  S^T <- e^{G_L} S^T + D
 // The state stays in the registers of the group that owns it (thread = state column n, 64 values) and only its terms go through
 // shared memory, so no product waits for another chunk's product: the chain is one multiply-add per entry and the split, and the
-// step follows the sum of the tensor work (3.1 K cycles) or the longest group, whichever is longer.
+// step follows the sum of the tensor work (4.5 K cycles) or the longest group, whichever is longer.
 //
 // 20 warps, one CTA per (batch, head, 64 value columns):
 //   0-7    G -> P; warp = rows of a quarter (warp & 3) and half of the columns (warp >> 2)
@@ -20,8 +20,10 @@
 // B, C, the terms of S and of xs have one tile each, x three (it is read again for the outputs, whose rows are staged over it),
 // the scalars two.  A product that accumulates onto one of another shape waits for it: only products of equal shape are ordered.
 //
-// What bounds it: B=8, T=4096, H=16, N=128: 318 us in the mma.sync form (tensor pipe 41 % of 1024 multiply-adds per clock and SM;
-// tcgen05 takes 4096).  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
+// What bounds it: B=8, T=4096, H=16, N=128: 133 us, 318 in the mma.sync form (tensor pipe 41 % of 1024 multiply-adds per clock and SM;
+// tcgen05 takes 4096).  A chunk takes 7.5 K cycles: tensor pipe 59 %, issue slots 52 %, and the warps' first stall after their
+// hand-overs is the instruction fetch, so the loops are kept rolled (150 KB of code: 215 us, 100 KB: 162, 72 KB: 140).  Twenty-four
+// warps with the outputs on their own (setmaxnreg for the state's group): 137.  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
 //
 // Infinities and NaN in x: P is 0 above the diagonal, but 0 x inf is NaN, and a whole chunk is one product.  Such an entry is
 // taken out of the tile of Y2 (it stays in xs, so the state gets it) and the outputs of its column from its token on become NaN.
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       const float w = scalars(it)[SC_W + lt];
       uint8_t *tile = x_tile(it), *dst = smem + L::kXt;
       __nv_bfloat162 inf = __floats2bfloat162_rn(0.f, 0.f);   // 0 x every entry: NaN if one is not finite
-#pragma unroll 2
+#pragma unroll 1
       for (int c = 0; c < 8; ++c) {
         const uint32_t at = piece_at(lt, c);
         const uint4 u = *reinterpret_cast<const uint4*>(tile + at);
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       __syncwarp();
       const int t0 = chunk_of(it) * kC + 32 * wq + (lane >> 3);   // the warp's own 32 rows leave as whole rows
       int64_t at = (int64_t)t0 * p.o_st + 8 * (lane & 7);
-#pragma unroll 4
+#pragma unroll 2
       for (int r = 0; r < 8; ++r) {
         if (t0 + 4 * r < T && in_bounds_run(p.status, y_at + at, 8, p.n_o))
           *reinterpret_cast<uint4*>(gy + at) = *reinterpret_cast<const uint4*>(tile + piece_at(32 * wq + 4 * r + (lane >> 3), lane & 7));
@@ -607,8 +609,13 @@ inline cudaError_t launch_n(const LinRecParams& p, int sms, cudaStream_t stream)
   }
   const int64_t ctas = (int64_t)p.B * p.H * (p.V / kP);
   const int nchunks = (p.T + kC - 1) / kC;
+  // Segments: a step of the first pass costs half of a full one, and every segment reads all earlier ends.  Four from four chunks on (8 heads,
+  // T=400: 19.7 us, 21.0 with two, 32.5 in the mma.sync form; T=300 with two segments 19.8, whole 15.3); eight only from 32 chunks
+  // on and for at most eight clusters (T=4000: 46 against 54 us with four; sixteen clusters of eight run in two waves: 16 heads, T=2000: 67
+  // against 37).
   int nseg = 1;
-  while (nseg < 8 && ctas * nseg * 2 <= sms && nchunks >= 4 * nseg) nseg *= 2;
+  while (nseg < 4 && ctas * nseg * 2 <= sms && nchunks >= 4) nseg *= 2;
+  if (nseg == 4 && ctas <= 8 && nchunks >= 32) nseg = 8;
   Params P;
   P.p = p;
   P.nseg = nseg;
@@ -629,6 +636,14 @@ inline cudaError_t launch_n(const LinRecParams& p, int sms, cudaStream_t stream)
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, P);
+}
+
+// What ssd::eligible takes, but for a single 64-token chunk (8 heads, T=64: 9.6 us here, 8.5 there; 256 heads 20.7 / 16.3) and for
+// half-size states in so few chunks that the chain of this form is longer (N=64, 8 heads, T=600: 23.8 / 21.4; T=1000: 23.9 / 21.9;
+// T=400: 19.7 / 32).
+inline bool ahead(const LinRecParams& p, int sms) {
+  const int64_t ctas = (int64_t)p.B * p.H * (p.V / kP);
+  return p.T > 64 && !(p.K == 64 && p.T > 512 && p.T <= 1024 && ctas * 4 <= sms) && sm100::encode_tiled_fn() != nullptr;
 }
 
 inline cudaError_t launch(const LinRecParams& p, int sms, cudaStream_t stream) {

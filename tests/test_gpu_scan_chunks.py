@@ -16,7 +16,11 @@ def _check(got, ref, tol):
 
 
 @pytest.mark.parametrize("B,T,H,P,N,G", [(1, 32, 2, 64, 64, 1), (1, 63, 2, 64, 128, 2), (2, 65, 4, 128, 128, 2), (1, 200, 2, 64, 128, 1),
-                                         (1, 577, 1, 64, 64, 1), (1, 1100, 2, 64, 128, 1), (3, 129, 50, 64, 64, 5)])
+                                         (1, 577, 1, 64, 64, 1), (1, 1100, 2, 64, 128, 1), (3, 129, 50, 64, 64, 5),
+                                         # tcgen05 form: one chunk, a whole one, one token more; four and eight segments, empty ones among
+                                         # them; more CTAs than SMs; three value slices
+                                         (1, 127, 2, 64, 64, 1), (2, 128, 2, 64, 128, 1), (1, 513, 3, 192, 128, 1), (1, 641, 2, 64, 128, 2),
+                                         (1, 4100, 1, 64, 64, 1), (5, 257, 32, 64, 128, 1)])
 def test_ssd_chunks(B, T, H, P, N, G):
     g = torch.Generator().manual_seed(T)
     f = lambda *s, scale=1.0: torch.randn(*s, generator=g) * scale
@@ -31,6 +35,24 @@ def test_ssd_chunks(B, T, H, P, N, G):
                               chunk_size=64, **kw)
     _check(s, rs, 1e-5)
     _check(y, ry, 5e-3)
+
+
+@pytest.mark.parametrize("N", [64, 128])
+def test_ssd_non_finite_input(N):
+    """An infinity or NaN in x reaches the outputs of its own column from its token on, and the state, and nothing before it."""
+    g = torch.Generator().manual_seed(N)
+    f = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).cuda()
+    x, dt, A, D = f(1, 300, 2, 64).bfloat16(), f(1, 300, 2), -torch.exp(f(2)), f(2)
+    Bm, Cm = f(1, 300, 1, N, scale=0.5).bfloat16(), f(1, 300, 1, N, scale=0.5).bfloat16()
+    y0, s0 = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    x[0, 70, 1, 5], x[0, 200, 1, 6] = float("inf"), float("nan")
+    y, s = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    bad = torch.zeros_like(y, dtype=torch.bool)
+    bad[0, 70:, 1, 5] = bad[0, 200:, 1, 6] = True
+    assert torch.equal(torch.isfinite(y.float()), ~bad) and torch.equal(y[~bad], y0[~bad])
+    gone = torch.zeros_like(s, dtype=torch.bool)
+    gone[0, 1, 5:7] = True
+    assert torch.equal(torch.isfinite(s), ~gone) and torch.equal(s[~gone], s0[~gone])
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
