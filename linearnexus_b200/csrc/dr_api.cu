@@ -508,7 +508,6 @@ int dr_chunk_bwd_saved(const DrDesc* d, const void* q, const void* k, const void
                        const float* beta, const void* d_o, const float* d_hT, void* dq, void* dk, void* dv,
                        float* dbeta, float* dg, float* dh0, void* workspace, size_t workspace_bytes,
                        int32_t* status_dev, void* stream) {
-  (void)status_dev;   // the adjoint kernels have no bounded waits: nothing can be reported here
   int s = validate_common(d, true);
   if (s != DR_OK) return s;
   if (!q || !k || !v || !beta || !d_o || !dq || !dk || !dv || !dbeta) return DR_ERR_NULL;
@@ -522,7 +521,7 @@ int dr_chunk_bwd_saved(const DrDesc* d, const void* q, const void* k, const void
   if ((int64_t)workspace_bytes < need || !workspace) return DR_ERR_WORKSPACE;
   tl_path = "bwd_saved";
   int launches = 0;
-  cudaError_t e = dr::launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace,
+  cudaError_t e = dr::launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace, status_dev,
                                          reinterpret_cast<cudaStream_t>(stream), &launches);
   g_launches.fetch_add(launches);
   return check_cuda(e);

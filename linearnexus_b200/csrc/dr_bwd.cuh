@@ -1425,14 +1425,14 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
 cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                                       const float* beta, const void* d_o, const float* d_hT, void* dq, void* dk,
                                       void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
-                                      cudaStream_t stream, int* launches) {
+                                      int32_t* status, cudaStream_t stream, int* launches) {
   const int C = d->chunk, K = d->K, V = d->V;
   if (bwdc::eligible(d)) {
     bwdc::Params p = bwdc::make_params(d, workspace);
     p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta; p.d_o = d_o; p.d_hT = d_hT;
     p.dq = dq; p.dk = dk; p.dv = dv; p.dbeta = dbeta; p.dg = dg; p.dh0 = dh0;
     const int64_t units = (int64_t)d->B * d->H;
-    cudaError_t e = d->variant == DR_KDA ? bwdc::launch_adjoint_t<true>(p, units, stream) : bwdc::launch_adjoint_t<false>(p, units, stream);
+    cudaError_t e = d->variant == DR_KDA ? bwdc::launch_adjoint_t<true>(p, units, status, stream) : bwdc::launch_adjoint_t<false>(p, units, status, stream);
     *launches += 2;
     if (e != cudaSuccess || p.map.Hq == p.map.H) return e;
     // grouped q/k heads: the heads' dq^, dk^ summed over each group, then the chain rule
@@ -1509,11 +1509,10 @@ cudaError_t launch_bwd(const DrDesc* d, const void* q, const void* k, const void
                               const float* beta, const float* h0, const void* d_o, const float* d_hT, void* dq,
                               void* dk, void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
                               int32_t* status, cudaStream_t stream, int* launches, bool own_stream) {
-  // only the forward has bounded waits that can report; the adjoint kernels synchronise with block barriers
   cudaError_t e = launch_bwd_forward(d, q, k, v, g, beta, h0, nullptr, nullptr, workspace, status, stream, launches,
                                      own_stream);
   if (e != cudaSuccess) return e;
-  return launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace, stream, launches);
+  return launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace, status, stream, launches);
 }
 
 }  // namespace dr

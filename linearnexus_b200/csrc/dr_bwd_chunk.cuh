@@ -5,10 +5,12 @@
 //     dS0 = e^{G_L} dS1 + N dS1 + Y^T dO
 // one [128 x 128] product per chunk and nothing else on the chain.  Three kernels:
 //
-//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as the A fragments of
-//                 mma.sync in the order the lanes of state_kernel load them (16 bytes per lane, no shared memory).
-//   state_kernel  one CTA per (sequence, 32 value columns) walks the chunks backwards; dS stays in accumulator
-//                 registers, its copy in shared memory is the B operand; stores dS1 of every chunk.
+//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles or as the A
+//                 fragments of mma.sync in the order the lanes of state_kernel load them (16 bytes per lane, no shared memory).
+//   chain_kernel  (scalar decays) one CTA per (sequence, 64 value columns) walks the chunks backwards on tcgen05, dS in registers;
+//                 stores dS1 of every chunk.  N and Y as two bf16 terms.
+//   state_kernel  (per-channel decays) the same on mma.sync, one CTA per (sequence, 32 value columns); dS stays in accumulator
+//                 registers, its copy in shared memory is the B operand.
 //   local_kernel  one CTA per chunk, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1
 //                 and the chunk's inputs, looping over four value slices with the sums over v in registers; then the
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
@@ -41,8 +43,8 @@ struct Params {
   const void* q; const void* k; const void* v; const void* g; const float* beta; const void* d_o; const float* d_hT;
   void* dq; void* dk; void* dv; float* dbeta; float* dg; float* dh0;
   const float* ckpt;    // [units][N][128][128] state at the start of every chunk
-  float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]
-  float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]
+  float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]; scalar decays: kNTile bytes per chunk
+  float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]; scalar decays: kYTile
   float* xat;           // [units][N][3][64][64] X, A, T
   float* ds;            // [units][N][128][128] dS1
   float* el;            // [units][N][128] e^{G_L}
@@ -62,9 +64,18 @@ using mma::AFrag;
 using mma::BFrag;
 using mma::fma;
 __device__ __forceinline__ void zero4(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
-// value as the product will see it, rounded to nearest instead of cut (single-product operands that are stored)
-template <bool X3>
-__device__ __forceinline__ float stored(float x) { return X3 ? x : __uint_as_float(sm100::to_tf32(x)); }
+// Operands of chain_kernel in memory: N [128][128] and Y^T [128][64] as two bf16 terms each, tiles of 8 x 8 core matrices.
+constexpr int kNTile = 2 * 128 * 128 * 2, kYTile = 2 * 128 * 64 * 2, kYRbs = 8 * 128;
+// an m16n8 accumulator (rows r, r + 8; two neighbouring columns) -> its two terms, `next` bytes to the rows 8 further on and `lo`
+// bytes to the second term; a warp writes 128 contiguous bytes per store
+__device__ __forceinline__ void store_terms(uint8_t* dst, int next, int lo, const float (&d)[4]) {
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+    const uint32_t h = mma::pack(d[2 * hr], d[2 * hr + 1]);
+    *reinterpret_cast<uint32_t*>(dst + hr * next) = h;
+    *reinterpret_cast<uint32_t*>(dst + hr * next + lo) = mma::pack(d[2 * hr] - mma::lo_f(h), d[2 * hr + 1] - mma::hi_f(h));
+  }
+}
 
 // four channels of the log decay in log2 units
 __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
@@ -351,10 +362,15 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         }
       }
     }
-    float4* dst = p.yf + (chunk * 8 + warp) * 8 * 32 + lane;
+    if constexpr (KDA) {
+      float4* dst = p.yf + (chunk * 8 + warp) * 8 * 32 + lane;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-      dst[nt * 32] = make_float4(stored<X3>(Y[nt][0]), stored<X3>(Y[nt][2]), stored<X3>(Y[nt][1]), stored<X3>(Y[nt][3]));
+      for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(Y[nt][0], Y[nt][2], Y[nt][1], Y[nt][3]);
+    } else {
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + chunk * kYTile + 2 * warp * kYRbs + g * 16 + 4 * t;
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
+    }
   }
   // ---- N = -W^T Kd -> fragments -----------------------------------------------------------------------------------------------
   if constexpr (KDA) {
@@ -403,29 +419,32 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         fma<X3>(d[nt], a, bk);
       }
     }
-    float4* dst = p.nf + ((chunk * 8 + warp) * 16 + 8 * half) * 32 + lane;
+    if constexpr (KDA) {
+      float4* dst = p.nf + ((chunk * 8 + warp) * 16 + 8 * half) * 32 + lane;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-      dst[nt * 32] = make_float4(stored<X3>(d[nt][0]), stored<X3>(d[nt][2]), stored<X3>(d[nt][1]), stored<X3>(d[nt][3]));
+      for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(d[nt][0], d[nt][2], d[nt][1], d[nt][3]);
+    } else {
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.nf) + chunk * kNTile + 2 * warp * sm100::RBS + 8 * half * 128 + g * 16 + 4 * t;
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
+    }
   }
 }
 
 // =====================================================================================================================
-// state_kernel: eight warps, warp w owns channel rows 16 w .. 16 w + 15 of dS [128][32]
+// state_kernel: the state pass for per-channel decays; eight warps, warp w owns channel rows 16 w .. 16 w + 15 of dS [128][32]
 // =====================================================================================================================
 constexpr int kStThreads = 256;
 constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved, [rows / 2][32 columns][2], 72 floats per pair
-// X3: dS as its two terms, [rows / 2][32 columns][hi, hi, lo, lo]: split once by the warp that owns it, not by the eight that read it
-template <bool X3> constexpr int ld_ds = X3 ? 136 : LDP;
-template <bool X3> constexpr int st_smem = 2 * (64 * ld_ds<X3> + 32 * LDP) * 4;
+// dS as its two terms, [rows / 2][32 columns][hi, hi, lo, lo]: split once by the warp that owns it, not by the eight that read it
+constexpr int kLdS = 136;
+constexpr int st_smem = 2 * (64 * kLdS + 32 * LDP) * 4;
 
-template <bool X3>
-__global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
+static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
   pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
-  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * LDS_]
-  constexpr int LDS_ = ld_ds<X3>;
-  float* sO = sS + 2 * 64 * LDS_;                       // [2][32 * LDP]
+  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * kLdS]
+  float* sO = sS + 2 * 64 * kLdS;                       // [2][32 * LDP]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int unit = blockIdx.x >> 2, v0 = (blockIdx.x & 3) * kVS;
   const int b = unit / p.map.H, h = unit % p.map.H;
@@ -460,7 +479,7 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
   }
   uint4 dor = load_do(p.N - 1);
   for (int n = p.N - 1; n >= 0; --n) {
-    float* cS = sS + (n & 1) * 64 * LDS_;
+    float* cS = sS + (n & 1) * 64 * kLdS;
     float* cO = sO + (n & 1) * 32 * LDP;
     // dS1 of this chunk: to memory, and to the other warps
     float* out = p.ds + (chunk0 + n) * (kD * kD) + v0;
@@ -469,21 +488,15 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
       const int c = 8 * nt + 2 * t;
       *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
       *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
-      if constexpr (X3) {   // the lanes of a row pair swap: the even row's takes column c of both rows, the odd row's c + 1
-        const bool odd = g & 1;
+      // the lanes of a row pair swap: the even row's takes column c of both rows, the odd row's c + 1
+      const bool odd = g & 1;
 #pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          const float got = __shfl_xor_sync(0xffffffffu, odd ? S[nt][2 * hr] : S[nt][2 * hr + 1], 4);
-          const float x = odd ? got : S[nt][2 * hr], y = odd ? S[nt][2 * hr + 1] : got;   // even row, odd row
-          BFrag<true> f;
-          f.set(x, y);
-          *reinterpret_cast<uint4*>(cS + ((hr ? r1 : r0) >> 1) * LDS_ + 4 * (c + odd)) = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
-        }
-      } else {
-        float* w0 = cS + (r0 >> 1) * LDP + 2 * c + (r0 & 1);
-        float* w1 = cS + (r1 >> 1) * LDP + 2 * c + (r1 & 1);
-        w0[0] = S[nt][0]; w0[2] = S[nt][1];
-        w1[0] = S[nt][2]; w1[2] = S[nt][3];
+      for (int hr = 0; hr < 2; ++hr) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? S[nt][2 * hr] : S[nt][2 * hr + 1], 4);
+        const float x = odd ? got : S[nt][2 * hr], y = odd ? S[nt][2 * hr + 1] : got;   // even row, odd row
+        BFrag<true> f;
+        f.set(x, y);
+        *reinterpret_cast<uint4*>(cS + ((hr ? r1 : r0) >> 1) * kLdS + 4 * (c + odd)) = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
       }
     }
     {
@@ -503,7 +516,7 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
     for (int nt = 0; nt < 4; ++nt) zero4(Z[nt]);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      AFrag<X3> a;
+      AFrag<true> a;
       a.set(yf[ks].x, yf[ks].y, yf[ks].z, yf[ks].w);
       yf[ks] = __ldcs(p.yf + ((cn * 8 + warp) * 8 + ks) * 32 + lane);
 #pragma unroll
@@ -516,20 +529,15 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
     }
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
-      AFrag<X3> a;
+      AFrag<true> a;
       a.set(nf[ks].x, nf[ks].y, nf[ks].z, nf[ks].w);
       nf[ks] = __ldcs(p.nf + ((cn * 8 + warp) * 16 + ks) * 32 + lane);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        BFrag<X3> bs;
-        if constexpr (X3) {
-          const uint4 y = *reinterpret_cast<const uint4*>(cS + (4 * ks + t) * LDS_ + 4 * (8 * nt + g));
-          bs.h[0] = y.x; bs.h[1] = y.y; bs.l[0] = y.z; bs.l[1] = y.w;
-        } else {
-          const float2 y = ld2(cS + (4 * ks + t) * LDP + 2 * (8 * nt + g));
-          bs.set(y.x, y.y);
-        }
-        if (ks & 1) fma<X3>(Z[nt], a, bs); else fma<X3>(S[nt], a, bs);
+        BFrag<true> bs;
+        const uint4 y = *reinterpret_cast<const uint4*>(cS + (4 * ks + t) * kLdS + 4 * (8 * nt + g));
+        bs.h[0] = y.x; bs.h[1] = y.y; bs.l[0] = y.z; bs.l[1] = y.w;
+        if (ks & 1) fma<true>(Z[nt], a, bs); else fma<true>(S[nt], a, bs);
       }
     }
 #pragma unroll
@@ -546,6 +554,197 @@ __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
       *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
     }
   }
+}
+
+// =====================================================================================================================
+// chain_kernel: the state pass for scalar decays on tcgen05, one CTA per (sequence, 64 value columns)
+//
+// dS stays in registers (thread = channel row, 32 columns); its two bf16 terms are the B operand, N and Y^T arrive by bulk copies as
+// the A operands, two terms each: three products N dS and two Y^T dO per 16 channels or tokens, 16 bits of every operand where
+// one tf32 product had 11.  Y^T dO of a chunk is issued while the chunk before it is still on its way through the registers, into
+// the other accumulator.  The chain per chunk: terms of dS -> 24 products -> multiply-add.
+//
+// What bounds it: B=2, T=4096, H=16 (64 CTAs): 105 us, 158 as mma.sync tf32 products over 128 CTAs (every warp read all of dS: shared
+// memory 62 %); gradient of the initial state against float64 3.2e-4 -> 2.4e-4.  The products of a chunk take 1.2 K cycles, its 100 KB of
+// operands 1.8 K at 55 bytes a clock.  Asking for the operands five chunks ahead in L2: 12 us slower.
+// =====================================================================================================================
+constexpr int kChThreads = 288, kChCols = 64;   // eight worker warps and one that issues
+// N hi twice, N lo, Y^T and d_o twice, the terms of dS, staging of its rows
+constexpr int kNTerm = kNTile / 2, kOTile = 64 * 128;
+constexpr int CH_H = 0, CH_L = CH_H + 2 * kNTerm, CH_Y = CH_L + kNTerm, CH_O = CH_Y + 2 * kYTile, CH_S = CH_O + 2 * kOTile, CH_G = CH_S + 2 * 128 * 128, CH_TOTAL = CH_G + 8 * 2048;
+static_assert(CH_O % 1024 == 0 && CH_S % 1024 == 0 && CH_TOTAL <= 232448 - 1024, "shared memory");
+struct alignas(64) ChainParams {
+  CUtensorMap to;   // panels of d_o (see sm100::make_panel_map)
+  Params p;
+  int32_t* status;
+};
+
+static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __grid_constant__ ChainParams P) {
+  const Params& p = P.p;
+  // a name of its own: declarations of one name in a namespace share the first one's alignment
+  extern __shared__ __align__(1024) uint8_t chain_smem[];
+  uint8_t* const smem = chain_smem;
+  __shared__ __align__(8) struct {
+    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y, bar_d;
+    uint32_t tmem_base;
+    int abort;
+  } ctl;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int unit = blockIdx.x / (kD / kChCols), v0 = blockIdx.x % (kD / kChCols) * kChCols;
+  const int b = unit / p.map.H, h = unit % p.map.H;
+  if (warp == 0) {
+    tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), 128);
+    tc::tmem_relinquish();
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(tc::smem_u32(&ctl.full_h[i]), 1);
+      tc::mbar_init(tc::smem_u32(&ctl.full_y[i]), 1);
+    }
+    tc::mbar_init(tc::smem_u32(&ctl.full_l), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.rdy), 256);
+    tc::mbar_init(tc::smem_u32(&ctl.bar_y), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.bar_d), 1);
+    tc::fence_mbar_init();
+    ctl.abort = 0;
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  pdl_entry();
+  const uint32_t tbase = ctl.tmem_base, sbase = tc::smem_u32(smem);
+  auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
+    const uint32_t at = tc::smem_u32(&bar);
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp >> 3);
+  };
+  const int64_t chunk0 = (int64_t)unit * p.N;
+  if (warp == 8) {
+    if (tc::elect_one()) {
+      auto n_at = [&](int it) { return reinterpret_cast<const uint8_t*>(p.nf) + (chunk0 + p.N - 1 - it) * kNTile; };
+      auto y_at = [&](int it) { return reinterpret_cast<const uint8_t*>(p.yf) + (chunk0 + p.N - 1 - it) * kYTile; };
+      auto load_term = [&](uint64_t& full, uint32_t dst, const uint8_t* src) {
+        const uint32_t bar = tc::smem_u32(&full);
+        tc::mbar_arrive_expect_tx(bar, kNTerm);
+        tc::bulk_g2s(dst, src, kNTerm, bar);
+      };
+      auto load_h = [&](int it) { load_term(ctl.full_h[it & 1], sbase + CH_H + (it & 1) * kNTerm, n_at(it)); };
+      auto load_l = [&](int it) { load_term(ctl.full_l, sbase + CH_L, n_at(it) + kNTerm); };
+      auto load_y = [&](int it) {
+        const uint32_t bar = tc::smem_u32(&ctl.full_y[it & 1]);
+        tc::mbar_arrive_expect_tx(bar, kYTile + kOTile);
+        tc::tma_load_4d(sbase + CH_O + (it & 1) * kOTile, &P.to, v0, h, (p.N - 1 - it) * kC, b, bar);
+        tc::bulk_g2s(sbase + CH_Y + (it & 1) * kYTile, y_at(it), kYTile, bar);
+      };
+      load_y(0);
+      load_h(0);
+      load_l(0);
+      if (p.N > 1) { load_y(1); load_h(1); }
+      constexpr uint32_t id = tc::idesc_bf16(128, 64, 0, 1);
+      auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
+      const uint64_t sd = tc::smem_desc_sw128(sbase + CH_S, 128 * 128, 1024), ld = tc::smem_desc(sbase + CH_L, 128, sm100::RBS);
+#pragma unroll 1
+      for (int it = 0; it < p.N; ++it) {
+        const uint32_t acc = tbase + (it & 1) * 64;   // (read for chunk it - 2 before its successor's dS was ready)
+        const uint64_t yd = tc::smem_desc(sbase + CH_Y + (it & 1) * kYTile, 128, kYRbs);
+        const uint64_t od = tc::smem_desc_sw128(sbase + CH_O + (it & 1) * kOTile, 128 * 128, 1024);
+        const uint64_t hd = tc::smem_desc(sbase + CH_H + (it & 1) * kNTerm, 128, sm100::RBS);
+        wait_bar(ctl.full_y[it & 1], (it >> 1) & 1);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          tc::mma_ss(acc, adv(yd, ks * 256), adv(od, ks * 2048), id, ks > 0);
+          tc::mma_ss(acc, adv(yd, kYTile / 2 + ks * 256), adv(od, ks * 2048), id, 1);
+        }
+        tc::mma_commit(tc::smem_u32(&ctl.bar_y));
+        wait_bar(ctl.full_h[it & 1], (it >> 1) & 1);
+        wait_bar(ctl.rdy, it & 1);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, ks * 2048), id, 1);
+          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, 128 * 128 + ks * 2048), id, 1);
+        }
+        wait_bar(ctl.full_l, it & 1);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
+        tc::mma_commit(tc::smem_u32(&ctl.bar_d));
+        wait_bar(ctl.bar_y, it & 1);   // Y^T and d_o have been read
+        if (it + 2 < p.N) load_y(it + 2);
+        wait_bar(ctl.bar_d, it & 1);   // N has been read
+        if (it + 1 < p.N) load_l(it + 1);
+        if (it + 2 < p.N) load_h(it + 2);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int row = 32 * (warp & 3) + lane, hc = warp >> 2;   // this thread's channel and half of the columns
+    const uint32_t lane_addr = (uint32_t)(32 * (warp & 3)) << 16;
+    const int64_t at = (int64_t)row * kD + v0 + 32 * hc;
+    uint8_t* stage = smem + CH_G + warp * 2048;
+    float S[32];
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) {   // (d_hT and dh0 need not be aligned to more than eight bytes)
+      const float2 x = p.d_hT ? ld2(p.d_hT + (int64_t)unit * kD * kD + at + c) : make_float2(0.f, 0.f);
+      S[c] = x.x; S[c + 1] = x.y;
+    }
+#pragma unroll 1
+    for (int it = 0; it < p.N; ++it) {
+      const int64_t chunk = chunk0 + p.N - 1 - it;
+      const float el = p.el[chunk * 128 + row];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = S[8 * c + 2 * e], y = S[8 * c + 2 * e + 1];
+          hi[e] = mma::pack(x, y);
+          lo[e] = mma::pack(x - mma::lo_f(hi[e]), y - mma::hi_f(hi[e]));
+        }
+        uint8_t* dst = smem + CH_S + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(dst + 128 * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      tc::fence_async_smem();
+      sm100::mbar_arrive(tc::smem_u32(&ctl.rdy));
+      // dS1 of this chunk -> memory, sixteen rows at a time through the warp's 2 KB: whole 128-byte lines (a thread's own row in 16-byte
+      // pieces made the write the longest part of a chunk)
+      float* ds = p.ds + chunk * (kD * kD) + (int64_t)(32 * (warp & 3)) * kD + v0 + 32 * hc;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int r0 = lane & 15;
+        if ((lane >> 4) == hf) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            *reinterpret_cast<float4*>(stage + r0 * 128 + ((q ^ (r0 & 7)) << 4)) = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = 4 * i + (lane >> 3), q = lane & 7;
+          *reinterpret_cast<float4*>(ds + (int64_t)(16 * hf + r) * kD + 4 * q) = *reinterpret_cast<const float4*>(stage + r * 128 + ((q ^ (r & 7)) << 4));
+        }
+        __syncwarp();
+      }
+      wait_bar(ctl.bar_d, it & 1);
+      tc::tc_fence_after();
+      uint32_t d[32];
+      tc::tmem_ld32(tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
+      tc::tc_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 32; ++c) S[c] = S[c] * el + __uint_as_float(d[c]);
+      tc::tc_fence_before();
+    }
+    if (p.dh0) {
+      float* out = p.dh0 + (int64_t)unit * kD * kD + at;
+#pragma unroll
+      for (int c = 0; c < 32; c += 2) *reinterpret_cast<float2*>(out + c) = make_float2(S[c], S[c + 1]);
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tbase, 128);
+  if (tid == 0) sm100::report_wait(P.status, ctl.abort);
 }
 
 // =====================================================================================================================
@@ -1321,7 +1520,9 @@ inline cudaError_t set_attributes() {
   if (e != cudaSuccess || attr_dev == dev) return e;
   e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem<KDA>::kTotal);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(state_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem<KDA>);
+  if (e == cudaSuccess)
+    e = KDA ? cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem)
+            : cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
   if (e == cudaSuccess) attr_dev = dev;
   return e;
 }
@@ -1340,10 +1541,18 @@ inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, con
   return d->variant == DR_KDA ? launch_pre_t<true>(p, units, stream) : launch_pre_t<false>(p, units, stream);
 }
 template <bool KDA>
-inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, cudaStream_t stream) {
+inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* status, cudaStream_t stream) {
   cudaError_t e = set_attributes<KDA>();
   if (e != cudaSuccess) return e;
-  e = launch_pdl(state_kernel<KDA>, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem<KDA>, stream, p);
+  if constexpr (KDA) {
+    e = launch_pdl(state_kernel, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem, stream, p);
+  } else {
+    ChainParams c;
+    c.p = p;
+    c.status = status;
+    if (!sm100::make_panel_map(&c.to, p.d_o, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
+    e = launch_pdl(chain_kernel, dim3((unsigned)(units * (kD / kChCols))), dim3(kChThreads), CH_TOTAL, stream, c);
+  }
   if (e != cudaSuccess) return e;
   return launch_pdl(local_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kLoThreads), LoSmem<KDA>::kTotal, stream, p);
 }

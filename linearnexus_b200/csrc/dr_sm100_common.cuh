@@ -42,6 +42,30 @@ static __device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int
   atomicOr(status, DR_DEV_TIMEOUT);
 }
 
+// The same in line, for kernels with few sites or with many live registers (a call costs its site more code than the loop): the place
+// goes to the abort flag, which the kernel's last thread hands to the status word with report_wait.
+__device__ __forceinline__ int wait_record(uint32_t bar_offset, uint32_t grp) {
+  const uint32_t num = bar_offset / 8u < 63u ? bar_offset / 8u : 63u;
+  return DR_DEV_TIMEOUT | (int)((num | (grp << 6)) << 8);
+}
+__device__ __forceinline__ void wait_inline(uint32_t bar, uint32_t parity, int* abort_flag, uint32_t bar_offset, uint32_t grp) {
+  if (tc::mbar_try(bar, parity)) return;
+  const uint32_t start = (uint32_t)clock();
+  while (!tc::mbar_try(bar, parity)) {
+    volatile int* gave_up = abort_flag;
+    if (*gave_up) return;
+    if ((uint32_t)clock() - start > 2000000000u) {
+      *gave_up = wait_record(bar_offset, grp);
+      return;
+    }
+  }
+}
+__device__ __forceinline__ void report_wait(int32_t* status, int record) {
+  if (!record || !status) return;
+  atomicCAS(status, 0, record);
+  atomicOr(status, DR_DEV_TIMEOUT);
+}
+
 // Test kernel of the record above: one thread waits, with this very routine and its full bound (about a second of SM
 // clock), on an mbarrier that nothing arrives on.  The status word gets DR_DEV_TIMEOUT and the site given here; a second
 // wait of the same CTA returns at once (abort flag) and leaves the record alone.  The kernel returns normally.

@@ -131,19 +131,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
   tc::tc_fence_after();
   pdl_entry();
   const uint32_t tbase = ctl.tmem_base, lane_addr = (uint32_t)(wq * 32) << 16, sbase = tc::smem_u32(smem);
-  // Bounded (about a second of SM clock); once one has run out the others return at once.  In line: a call costs its site more code.
   auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
     const uint32_t at = tc::smem_u32(&bar);
-    if (tc::mbar_try(at, parity)) return;
-    const uint32_t start = (uint32_t)clock();
-    while (!tc::mbar_try(at, parity)) {
-      volatile int* gave_up = &ctl.abort;
-      if (*gave_up) return;
-      if ((uint32_t)clock() - start > 2000000000u) {
-        *gave_up = DR_DEV_TIMEOUT | ((at - tc::smem_u32(&ctl)) / 8 | (warp < 8 ? 0 : warp < 12 ? 1 : warp < 16 ? 2 : 3) << 6) << 8;
-        return;
-      }
-    }
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp < 8 ? 0 : warp < 12 ? 1 : warp < 16 ? 2 : 3);
   };
   auto arrive = [&](uint64_t& bar) { sm100::mbar_arrive(tc::smem_u32(&bar)); };
   auto scalars = [&](int it) { return reinterpret_cast<float*>(smem + L::kSc) + (it % kXs) * kScalars * kC; };
@@ -578,10 +568,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tbase, 512);
-  if (tid == 0 && ctl.abort && p.status) {   // as wait_more records it
-    atomicCAS(p.status, 0, ctl.abort);
-    atomicOr(p.status, DR_DEV_TIMEOUT);
-  }
+  if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
 // Rows of 64 columns of 128 tokens of a [B][T][heads][cols] array (any strides), 128-byte swizzle; tokens past T arrive as zeros.
