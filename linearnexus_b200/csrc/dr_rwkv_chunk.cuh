@@ -11,7 +11,7 @@
 // Eight warps keep the state transposed in accumulators (16 value columns x 32 keys each; the two warps of a column block
 // exchange their partial dots).  An accumulator is, register for register, an A operand whose contraction runs over its columns: h
 // feeds the dots, their result feeds T, U feeds the update, and nothing of the state touches memory.  Three groups of four warps
-// stage the blocks ahead, one block in three each: raw rows from a ring of asynchronous copies, decay products, the row vectors and
+// (RWKV-6: four) stage the blocks ahead in turn: raw rows from a ring of asynchronous copies, decay products, the row vectors and
 // the 8 x 8 coefficients.  A filled stage is handed over by a named barrier, arrived on by its group and waited for by the state's
 // warps; an emptied one by an mbarrier (see kEmptyTries).
 //
@@ -36,7 +36,11 @@ namespace rwkv {
 
 using mma::AFrag;
 using mma::BFrag;
-constexpr int kK = 64, kTB = 8, kGroups = 3, kRing = 3, kStages = 4, kCons = 256, kThreads = kCons + 128 * kGroups;
+constexpr int kK = 64, kTB = 8, kGroups = 3, kRing = 3, kStages = 4, kCons = 256;
+// Staging groups.  RWKV-6 has less of a chain per block (no U), so there a fourth pays: B=8, T=4096, H=16 764 -> 718 us, B=2, T=500 97.9 ->
+// 92.7; RWKV-7 681 -> 692.  float32 rows leave room for three.
+template <int KIND, bool BF> constexpr int groups_of = KIND == LR_RWKV6 && BF ? 4 : kGroups;
+template <int KIND, bool BF> constexpr int threads_of = kCons + 128 * groups_of<KIND, BF>;
 constexpr int kHand = kCons + 128;   // threads of a hand-over barrier: the consumers and one staging group
 constexpr int LDR = 72;    // row vectors [token][key], read as B operands along the key axis
 constexpr int LDU = 66;    // update vectors [token pair][key], read across tokens
@@ -90,16 +94,16 @@ struct Scratch {            // of one staging group
 template <int KIND, bool BF>
 constexpr int kGroupBytes = ((int)sizeof(Scratch) + 15) / 16 * 16 + kRing * Ring<KIND, BF>::kSlot;
 template <int KIND, bool BF>   // then one mbarrier per stage
-constexpr int kEmptyAt = kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + kGroups * kGroupBytes<KIND, BF>;
+constexpr int kEmptyAt = kStages * (int)sizeof(Stage) + (int)sizeof(Exchange) + groups_of<KIND, BF> * kGroupBytes<KIND, BF>;
 template <int KIND, bool BF>
 constexpr int kSmemBytes = kEmptyAt<KIND, BF> + kStages * 8;
-static_assert(kEmptyAt<LR_DPLR, false> % 8 == 0 && kSmemBytes<LR_DPLR, false> <= 232448, "227 KB per CTA");
+static_assert(kEmptyAt<LR_DPLR, false> % 8 == 0 && kEmptyAt<LR_RWKV6, true> % 8 == 0 && kSmemBytes<LR_DPLR, false> <= 232448 && kSmemBytes<LR_RWKV6, true> <= 232448, "227 KB per CTA");
 
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-constexpr int kBarFull = 1, kBarGroup = 1 + kStages, kBarPair = kBarGroup + kGroups;
+constexpr int kBarFull = 1, kBarGroup = 1 + kStages, kBarPair = kBarGroup + groups_of<LR_RWKV6, true>;
 static_assert(kBarPair + 4 <= 16, "named barriers");
-// A stage passes from group to group (kStages is no multiple of kGroups), so "the consumers have left stage s for the n-th time" is
+// With three groups a stage passes from group to group (kStages is no multiple of kGroups), so "the consumers have left stage s for the n-th time" is
 // phase n of an mbarrier: a named barrier has no phases, and two groups would meet on it in either order.  The group of block blk
 // waits for phase blk / kStages - 1.  It cannot be a phase behind (phase blk / kStages needs blk staged first), nor a phase ahead:
 // its last block, blk - kGroups, was staged after every warp had left blk - kGroups - kStages, so after it had arrived for the phase
@@ -117,10 +121,11 @@ __device__ __forceinline__ void fma3(float (&d)[3][4], const AFrag<true>& a, con
 }
 
 template <int KIND, bool BF>
-__global__ void __launch_bounds__(kThreads, 1) rwkv_chunk_kernel(const LinRecParams p) {
+__global__ void __launch_bounds__(threads_of<KIND, BF>, 1) rwkv_chunk_kernel(const LinRecParams p) {
   pdl_entry();
   using R = Ring<KIND, BF>;
   constexpr bool LR = KIND == LR_DPLR;
+  constexpr int kGroups = groups_of<KIND, BF>;
   constexpr int NV = R::NV;
   extern __shared__ __align__(16) uint8_t smem[];
   static_assert(sizeof(Stage) % 16 == 0, "stages stay aligned");
@@ -493,7 +498,7 @@ inline cudaError_t launch_t(const LinRecParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
-  return launch_pdl(kern, dim3((unsigned)((int64_t)p.B * p.H * (p.V / 64))), dim3(kThreads), bytes, stream, p);
+  return launch_pdl(kern, dim3((unsigned)((int64_t)p.B * p.H * (p.V / 64))), dim3(threads_of<KIND, BF>), bytes, stream, p);
 }
 inline cudaError_t launch(int kind, bool bf, const LinRecParams& p, cudaStream_t stream) {
   if (kind == LR_DPLR) return bf ? launch_t<LR_DPLR, true>(p, stream) : launch_t<LR_DPLR, false>(p, stream);

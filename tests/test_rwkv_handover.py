@@ -62,7 +62,8 @@ def test_rwkv_stage_handover_in_every_order():
         assert explore(groups, stages, "bar_sync(kBarEmpty" not in SRC, nblk) is None
 
 
-@pytest.mark.parametrize("groups,stages,phases,sound", [(3, 4, False, False), (3, 3, False, True), (3, 4, True, True), (3, 6, False, True)])
+@pytest.mark.parametrize("groups,stages,phases,sound", [(3, 4, False, False), (3, 3, False, True), (3, 4, True, True), (3, 6, False, True),
+                                                            (4, 4, True, True)])
 def test_exploration_tells_sound_from_unsound(groups, stages, phases, sound):
     """Without phases a stage has to belong to one group (stages a multiple of the groups)."""
     assert (explore(groups, stages, phases, 20) is None) == sound
