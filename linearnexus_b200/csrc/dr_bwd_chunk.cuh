@@ -438,7 +438,7 @@ constexpr int kStThreads = 256;
 constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved, [rows / 2][32 columns][2], 72 floats per pair
 // dS as its two terms, [rows / 2][32 columns][hi, hi, lo, lo]: split once by the warp that owns it, not by the eight that read it
 constexpr int kLdS = 136;
-constexpr int st_smem = 2 * (64 * kLdS + 32 * LDP) * 4;
+constexpr int st_rows = 2 * (64 * kLdS + 32 * LDP) * 4, st_smem = st_rows + 8 * 2048;
 
 static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
   pdl_entry();
@@ -446,6 +446,7 @@ static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Param
   float* sS = reinterpret_cast<float*>(smem);          // [2][64 * kLdS]
   float* sO = sS + 2 * 64 * kLdS;                       // [2][32 * LDP]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  uint8_t* stage = smem + st_rows + warp * 2048;
   const int unit = blockIdx.x >> 2, v0 = (blockIdx.x & 3) * kVS;
   const int b = unit / p.map.H, h = unit % p.map.H;
   const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
@@ -481,13 +482,13 @@ static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Param
   for (int n = p.N - 1; n >= 0; --n) {
     float* cS = sS + (n & 1) * 64 * kLdS;
     float* cO = sO + (n & 1) * 32 * LDP;
-    // dS1 of this chunk: to memory, and to the other warps
-    float* out = p.ds + (chunk0 + n) * (kD * kD) + v0;
+    // dS1 of this chunk: to memory (sixteen rows through the warp's 2 KB, as whole 128-byte lines), and to the other warps
+    float* out = p.ds + (chunk0 + n) * (kD * kD) + (int64_t)(16 * warp) * kD + v0;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       const int c = 8 * nt + 2 * t;
-      *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
-      *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
+      *reinterpret_cast<float2*>(stage + g * 128 + (((2 * nt + (t >> 1)) ^ g) << 4) + 8 * (t & 1)) = make_float2(S[nt][0], S[nt][1]);
+      *reinterpret_cast<float2*>(stage + (g + 8) * 128 + (((2 * nt + (t >> 1)) ^ g) << 4) + 8 * (t & 1)) = make_float2(S[nt][2], S[nt][3]);
       // the lanes of a row pair swap: the even row's takes column c of both rows, the odd row's c + 1
       const bool odd = g & 1;
 #pragma unroll
@@ -508,6 +509,12 @@ static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Param
     const int64_t cn = chunk0 + (n > 0 ? n - 1 : 0);   // the next chunk's operands replace this one's as they are used
     dor = load_do(n - 1);
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = 4 * i + (lane >> 3), q = lane & 7;
+      *reinterpret_cast<float4*>(out + (int64_t)r * kD + 4 * q) = *reinterpret_cast<const float4*>(stage + r * 128 + ((q ^ (r & 7)) << 4));
+    }
+    __syncwarp();
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) { S[nt][0] *= el0; S[nt][1] *= el0; S[nt][2] *= el1; S[nt][3] *= el1; }
     el0 = p.el[cn * 128 + r0]; el1 = p.el[cn * 128 + r1];
