@@ -23,7 +23,8 @@
 // What bounds it: B=8, T=4096, H=16, N=128: 133 us, 318 in the mma.sync form (tensor pipe 41 % of 1024 multiply-adds per clock and SM;
 // tcgen05 takes 4096).  A chunk takes 7.5 K cycles: tensor pipe 59 %, issue slots 52 %, and the warps' first stall after their
 // hand-overs is the instruction fetch, so the loops are kept rolled (150 KB of code: 215 us, 100 KB: 162, 72 KB: 140).  Twenty-four
-// warps with the outputs on their own (setmaxnreg for the state's group): 137.  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
+// warps with the outputs on their own (setmaxnreg for the state's group): 137; xs by the warps with the least of P: 136; the issue loops
+// unrolled by four: 142.  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
 //
 // Infinities and NaN in x: P is 0 above the diagonal, but 0 x inf is NaN, and a whole chunk is one product.  Such an entry is
 // taken out of the tile of Y2 (it stays in xs, so the state gets it) and the outputs of its column from its token on become NaN.
