@@ -18,7 +18,7 @@
 //   17     copies B, C, x (one thread, TMA, 128-byte swizzle; tokens past the end arrive as zeros)
 //   18, 19 dt -> scalars of a chunk
 // B, C, the terms of S and of xs have one tile each, x three (it is read again for the outputs, whose rows are staged over it),
-// the scalars two.  A product that accumulates onto one of another shape waits for it: only products of equal shape are ordered.
+// the scalars three stages.  A product that accumulates onto one of another shape waits for it: only products of equal shape are ordered.
 //
 // What bounds it: B=8, T=4096, H=16, N=128: 133 us, 318 in the mma.sync form (tensor pipe 41 % of 1024 multiply-adds per clock and SM;
 // tcgen05 takes 4096).  A chunk takes 7.5 K cycles: tensor pipe 59 %, issue slots 52 %, and the warps' first stall after their
