@@ -1043,32 +1043,102 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
 // with N, Z, Y, A_qk U from the intra pass, and the value columns are cut into slices of 8 NT per CTA.  Warps 0-7 keep 16 state
 // rows each in registers, their bf16 copy in shared memory is the B operand; warps 8-11 compute the output beside the chain.
 // Operands are bf16 where the other forwards have bf16 operands (N, Y and the copy of S), the state, Z and the sums fp32.
-constexpr int kTrThreads = 12 * 32;
-
+//
+// STAGED: a chunk's operands (60 KB with 16 columns) arrive by bulk copies of a thirteenth warp, two or three chunks ahead, and each lane
+// reads its fragments from shared memory as they lie, one chunk ahead.  Loaded from memory one chunk ahead, they were what the chain of
+// many CTAs waited for (1.2 us a chunk, first stall the loads; 8 sequences, T=4096, whole forward: 129 -> 101 us; 16, T=1777: a layer 103 ->
+// 96), while with six sequences or fewer memory answers within a chunk and the copy is a detour (four, T=3000: 60.6 against 64.0;
+// six, T=2000: 49.6 against 52.5).
+constexpr int kTrWorkers = 12 * 32;
+template <bool STAGED> constexpr int kTrThreads = kTrWorkers + (STAGED ? 32 : 0);
 template <int NT>
-__global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid_constant__ IntraTransParams P) {
-  pdl_entry();
-  constexpr int VS = 8 * NT, LDS = VS + 8, SL = kD / VS;
+struct TrSmem {
+  static constexpr int kStages = NT == 2 ? 3 : 2;
+  static constexpr int kN = 0, kY = kN + 128 * 128 * 2, kZ = kY + 64 * 128 * 2, kO = kZ + 8 * NT * 512, kE = kO + 4 * NT * 512;
+  static constexpr int kStage = kE + 512, kTotal = kStages * kStage;
+};
+
+template <int NT, bool STAGED>
+__global__ void __launch_bounds__(kTrThreads<STAGED>, 1) trans_state_kernel(const __grid_constant__ IntraTransParams P) {
+  using L = TrSmem<NT>;
+  constexpr int VS = 8 * NT, LDS = VS + 8, SL = kD / VS, ST = L::kStages;
   const FwdParams& p = P.p;
+  extern __shared__ __align__(128) uint8_t trans_smem[];   // a name of its own: see chain_kernel
   __shared__ __align__(16) __nv_bfloat16 sS[2][kD * LDS];
+  __shared__ __align__(8) struct { uint64_t full[ST], empty[ST]; int abort; } ctl;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  if constexpr (STAGED) {
+    if (tid == 0) {
+      for (int i = 0; i < ST; ++i) {
+        tc::mbar_init(tc::smem_u32(&ctl.full[i]), 1);
+        tc::mbar_init(tc::smem_u32(&ctl.empty[i]), kTrWorkers / 32);
+      }
+      tc::fence_mbar_init();
+      ctl.abort = 0;
+    }
+    __syncthreads();
+  }
+  pdl_entry();
+  auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
+    const uint32_t at = tc::smem_u32(&bar);
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp == 12);
+  };
   const int unit = blockIdx.x / SL, v0 = (blockIdx.x % SL) * VS;
   const int b = unit / p.map.H, h = unit % p.map.H, T = p.map.T, N = (T + kC - 1) / kC;
   const int64_t chunk0 = (int64_t)unit * N;
   const bool state = warp < 8;
-  const int mt = state ? warp : warp - 8, tiles = state ? 8 : 4, r0 = 16 * mt + g, r1 = r0 + 8;
-  const uint4* fa = (state ? P.nf : P.yf) + lane;
-  const float4* fc = (state ? P.zf : P.of) + (v0 / 8) * 32 + lane;
+  const int mt = state ? warp : warp - 8, r0 = 16 * mt + g, r1 = r0 + 8;
+  if (STAGED && warp == 12) {
+    // copies of a chunk: lane 0 N, 1 Y, 2 e^{G_L}, 3-10 the row tiles of Z, 11-14 those of A_qk U
+    for (int n = 0; n < N; ++n) {
+      const int st = n % ST;
+      if (n >= ST) wait_bar(ctl.empty[st], (n / ST - 1) & 1);
+      const uint32_t bar = tc::smem_u32(&ctl.full[st]), dst = tc::smem_u32(trans_smem) + st * L::kStage;
+      if (lane == 0) tc::mbar_arrive_expect_tx(bar, L::kStage);
+      __syncwarp();
+      const int64_t c = chunk0 + n;
+      if (lane == 0) tc::bulk_g2s(dst + L::kN, P.nf + c * 8 * 8 * 32, 128 * 128 * 2, bar);
+      if (lane == 1) tc::bulk_g2s(dst + L::kY, P.yf + c * 4 * 8 * 32, 64 * 128 * 2, bar);
+      if (lane == 2) tc::bulk_g2s(dst + L::kE, P.el + c * kD, 512, bar);
+      if (lane >= 3 && lane < 11) tc::bulk_g2s(dst + L::kZ + (lane - 3) * NT * 512, P.zf + ((c * 8 + lane - 3) * 16 + v0 / 8) * 32, NT * 512, bar);
+      if (lane >= 11 && lane < 15) tc::bulk_g2s(dst + L::kO + (lane - 11) * NT * 512, P.of + ((c * 4 + lane - 11) * 16 + v0 / 8) * 32, NT * 512, bar);
+    }
+    return;
+  }
   uint4 a[8];
   float4 c[NT];
   float S[NT][4], el0 = 0.f, el1 = 0.f;
+  // this lane's fragments of chunk n
+  struct Source { const uint4* a; const float4* c; const float* el; };
+  auto source = [&](int n) {
+    if constexpr (STAGED) {
+      const uint8_t* stage = trans_smem + n % ST * L::kStage;
+      return Source{reinterpret_cast<const uint4*>(stage + (state ? L::kN : L::kY)) + mt * 8 * 32 + lane,
+                    reinterpret_cast<const float4*>(stage + (state ? L::kZ : L::kO)) + mt * NT * 32 + lane, reinterpret_cast<const float*>(stage + L::kE)};
+    } else {
+      const int64_t at = (chunk0 + n) * (state ? 8 : 4) + mt;
+      return Source{(state ? P.nf : P.yf) + at * 8 * 32 + lane, (state ? P.zf : P.of) + (at * 16 + v0 / 8) * 32 + lane, P.el + (chunk0 + n) * kD};
+    }
+  };
+  auto arrived = [&](int n) { if constexpr (STAGED) wait_bar(ctl.full[n % ST], (n / ST) & 1); };
+  auto done = [&](int n) {   // the warp has read its part of the stage
+    if constexpr (STAGED) {
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(tc::smem_u32(&ctl.empty[n % ST]));
+    }
+  };
   auto s_at = [&](int r, int nt) { return ((int64_t)unit * kD + r) * kD + v0 + 8 * nt + 2 * t; };
+  {
+    arrived(0);
+    const Source f = source(0);
 #pragma unroll
-  for (int ks = 0; ks < 8; ++ks) a[ks] = fa[((chunk0 * tiles + mt) * 8 + ks) * 32];
+    for (int ks = 0; ks < 8; ++ks) a[ks] = f.a[ks * 32];
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) c[nt] = fc[((chunk0 * tiles + mt) * 16 + nt) * 32];
+    for (int nt = 0; nt < NT; ++nt) c[nt] = f.c[nt * 32];
+    if (state) { el0 = f.el[r0]; el1 = f.el[r1]; }
+    done(0);
+  }
   if (state) {
-    el0 = P.el[chunk0 * kD + r0]; el1 = P.el[chunk0 * kD + r1];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       float2 lo = make_float2(0.f, 0.f), hi = lo;
@@ -1089,21 +1159,25 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
         *reinterpret_cast<uint32_t*>(cS + r1 * LDS + 8 * nt + 2 * t) = mma::pack(S[nt][2], S[nt][3]);
       }
     }
-    __syncthreads();
+    if constexpr (STAGED) asm volatile("bar.sync 1, %0;" ::"n"(kTrWorkers) : "memory");
+    else __syncthreads();
     float d[NT][4], e[NT][4];   // two accumulators: shorter chains
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       d[nt][0] = c[nt].x; d[nt][1] = c[nt].y; d[nt][2] = c[nt].z; d[nt][3] = c[nt].w;
       e[nt][0] = e[nt][1] = e[nt][2] = e[nt][3] = 0.f;
     }
-    const int64_t cn = chunk0 + (n + 1 < N ? n + 1 : n);   // the next chunk's operands replace this one's as they are used
+    // the next chunk's fragments replace this one's as they are used
+    const bool more = n + 1 < N;
+    if (more) arrived(n + 1);
+    const Source f = source(more ? n + 1 : n);
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) c[nt] = fc[((cn * tiles + mt) * 16 + nt) * 32];
+    for (int nt = 0; nt < NT; ++nt) c[nt] = f.c[nt * 32];
     const uint32_t base = tc::smem_u32(cS);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const uint32_t ar[4] = {a[ks].x, a[ks].y, a[ks].z, a[ks].w};
-      a[ks] = fa[((cn * tiles + mt) * 8 + ks) * 32];
+      a[ks] = f.a[ks * 32];
 #pragma unroll
       for (int n2 = 0; n2 < NT / 2; ++n2) {
         uint32_t bb[4];
@@ -1112,13 +1186,16 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
         mma::bf16((ks & 1) ? e[2 * n2 + 1] : d[2 * n2 + 1], ar, bb[2], bb[3]);
       }
     }
+    float x0 = 0.f, x1 = 0.f;
+    if (STAGED && state) { x0 = f.el[r0]; x1 = f.el[r1]; }
+    if (more) done(n + 1);
     if (state) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         S[nt][0] = el0 * S[nt][0] + (d[nt][0] + e[nt][0]); S[nt][1] = el0 * S[nt][1] + (d[nt][1] + e[nt][1]);
         S[nt][2] = el1 * S[nt][2] + (d[nt][2] + e[nt][2]); S[nt][3] = el1 * S[nt][3] + (d[nt][3] + e[nt][3]);
       }
-      el0 = P.el[cn * kD + r0]; el1 = P.el[cn * kD + r1];
+      el0 = STAGED ? x0 : f.el[r0]; el1 = STAGED ? x1 : f.el[r1];
     } else {
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
@@ -1144,6 +1221,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) trans_state_kernel(const __grid
       *reinterpret_cast<float2*>(p.hT + s_at(r1, nt)) = make_float2(S[nt][2], S[nt][3]);
     }
   }
+  if constexpr (STAGED) {
+    if (tid == 0) sm100::report_wait(p.status, ctl.abort);
+  }
 }
 
 // bytes per chunk: N, Y bf16; Z, A_qk U, e^{G_L} fp32
@@ -1158,6 +1238,8 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   if (e != cudaSuccess) return e;
   if (attr_dev != dev) {
     e = cudaFuncSetAttribute(intra_kernel<IntraTransParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<2>::kTotal);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<4>::kTotal);
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
@@ -1173,8 +1255,9 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   e = launch_pdl(intra_kernel<IntraTransParams>, dim3((unsigned)nc), dim3(kThreads), IN_TOTAL, stream, P);
   if (e != cudaSuccess) return e;
   // 16 columns per CTA while the slices fit one wave: the chain's length is what counts
-  if (units * 8 <= sms) return launch_pdl(trans_state_kernel<2>, dim3((unsigned)(units * 8)), dim3(kTrThreads), 0, stream, P);
-  return launch_pdl(trans_state_kernel<4>, dim3((unsigned)(units * 4)), dim3(kTrThreads), 0, stream, P);
+  if (units <= 6) return launch_pdl(trans_state_kernel<2, false>, dim3((unsigned)(units * 8)), dim3(kTrThreads<false>), 0, stream, P);   // see the kernel
+  if (units * 8 <= sms) return launch_pdl(trans_state_kernel<2, true>, dim3((unsigned)(units * 8)), dim3(kTrThreads<true>), TrSmem<2>::kTotal, stream, P);
+  return launch_pdl(trans_state_kernel<4, true>, dim3((unsigned)(units * 4)), dim3(kTrThreads<true>), TrSmem<4>::kTotal, stream, P);
 }
 
 template <class IP, class SP>
