@@ -2,7 +2,8 @@
 
 Names, argument order, keyword defaults, shapes and output dtypes follow the LinearNexus functions cited per
 function (paths relative to the LinearNexus tree); arrays are torch CUDA tensors.  At the models' shapes they run in chunk
-form on the tensor cores in float32 precision (``csrc/dr_rwkv_chunk.cuh``, ``csrc/dr_ssd_chunk.cuh``), elsewhere as the token
+form on the tensor cores in float32 precision (``csrc/dr_rwkv_chunk.cuh``, ``csrc/dr_ssd_sm100.cuh``,
+``csrc/dr_ssd_chunk.cuh``), elsewhere as the token
 recurrence with the float32 state in registers (``csrc/dr_linrec.cuh``).  There is no CPU path.
 """
 from __future__ import annotations

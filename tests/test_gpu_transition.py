@@ -64,7 +64,8 @@ def test_transition_form_bf16_storage():
 
 
 @pytest.mark.parametrize("variant", ["delta", "gated", "kda"])
-@pytest.mark.parametrize("B,H,Hq,T,layout", [(1, 2, 2, 64, "bhtd"), (1, 4, 2, 321, "bthd"), (2, 4, 4, 450, "bhtd"), (1, 20, 10, 200, "bthd")])
+@pytest.mark.parametrize("B,H,Hq,T,layout", [(1, 2, 2, 64, "bhtd"), (1, 4, 2, 321, "bthd"), (2, 4, 4, 450, "bhtd"), (1, 20, 10, 200, "bthd"),
+                                              (1, 7, 7, 64, "bhtd"), (1, 7, 7, 150, "bthd")])
 def test_transition_form_bf16_tensor_shape(variant, B, H, Hq, T, layout):
     i = O.make_inputs(variant, B, H, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
     i["q"], i["k"] = i["q"][:, :Hq].contiguous(), i["k"][:, :Hq].contiguous()
