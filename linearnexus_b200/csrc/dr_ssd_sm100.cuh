@@ -49,6 +49,8 @@ constexpr int kXs = 3;                  // x tiles, and scalars of a chunk, in f
 // per chunk and token j: G as a float32 pair (log2 units), dt, e^G, dt e^{G_L - G}; dt e^{G_r - G_j} for r = 32, 64, 96 (j < r)
 constexpr int kScalars = 8, SC_G = 0, SC_R = kC, SC_DT = 2 * kC, SC_EG = 3 * kC, SC_W = 4 * kC, SC_H = 5 * kC;
 
+constexpr int kBadRow = kP + 4;         // per column, then one word for the whole chunk
+
 // tensor-memory columns
 constexpr uint32_t TM_G = 0;      // G, then P: per 16 tokens j the hi and mid terms (8 + 8 columns)   128
 constexpr uint32_t TM_PL = 128;   // lo terms of P                                                     64
@@ -64,15 +66,15 @@ struct Smem {
   static constexpr int kXt = kX + kXs * kPanel;         // terms of xs
   static constexpr int kSt = kXt + 3 * kPanel;          // terms of S^T; a segment's end state [64][128] fp32 between the passes
   static constexpr int kSc = kSt + 3 * kPanel;          // kXs stages of kScalars arrays
-  static constexpr int kBad = kSc + kXs * kScalars * kC * 4;     // two stages of: first token with a non-finite x, per column
-  static constexpr int kTotal = kBad + 2 * kP * 4;
+  static constexpr int kBad = kSc + kXs * kScalars * kC * 4;     // kXs stages of kBadRow words, see bad_of
+  static constexpr int kTotal = kBad + kXs * kBadRow * 4;
 };
 
 struct Ctl {
   uint64_t fullB, fullC, fullX[kXs], scal[kXs], xs, d_read[kXs], x_free[kXs], s_rdy, y_read, p_rdy[4];
   uint64_t barDa, barD, barG, barY1a, barY1, barY;
   uint32_t tmem_base;
-  int abort, bad[2];
+  int abort;
   float seg_decay;
 };
 
@@ -120,10 +122,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
     init(ctl.xs, 128); init(ctl.s_rdy, 128);
     init(ctl.barDa, 1); init(ctl.barD, 1); init(ctl.barG, 1); init(ctl.barY1a, 1); init(ctl.barY1, 1); init(ctl.barY, 1);
     tc::fence_mbar_init();
-    ctl.abort = ctl.bad[0] = ctl.bad[1] = 0;
+    ctl.abort = 0;
   }
-  int* const sBad = reinterpret_cast<int*>(smem + L::kBad);
-  if (tid < 2 * kP) sBad[tid] = kC;
+  if (tid < kXs * kBadRow) reinterpret_cast<uint32_t*>(smem + L::kBad)[tid] = 0u;
   if (N == 64)
     for (int i = tid; i < kPanel / 16; i += kThreads) *reinterpret_cast<uint4*>(smem + L::kB + kPanel + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
   tc::fence_async_smem();
@@ -294,6 +295,11 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
     __nv_bfloat16* gy = reinterpret_cast<__nv_bfloat16*>(p.o) + y_at;
     const float D_h = p.D[h];
     auto x_tile = [&](int it) { return smem + L::kX + (it % kXs) * kPanel; };
+    // Which columns of step `it` have a non-finite x, and from which token on: per column the largest bad_key of such a token (a word of
+    // an earlier step is smaller than every key of this one, so nothing is reset), then one word for the whole chunk.  A stage is
+    // written again three steps on, once the tile is: every thread has read it by then (x_free).
+    auto bad_of = [&](int it) { return reinterpret_cast<uint32_t*>(smem + L::kBad) + (it % kXs) * kBadRow; };
+    auto bad_key = [&](int it, int token) { return (uint32_t)(it + 1) * kC + (kC - 1 - token); };
     auto make_xs = [&](int it) {
       if (it == n1) boundary();
       wait_bar(ctl.scal[it % kXs], (it / kXs) & 1);
@@ -324,10 +330,10 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
           uint16_t* x = reinterpret_cast<uint16_t*>(tile + piece_at(lt, q >> 3)) + (q & 7);
           if ((*x & 0x7f80) == 0x7f80) {
             *x = 0;
-            atomicMin(sBad + (it & 1) * kP + q, lt);
+            atomicMax(bad_of(it) + q, bad_key(it, lt));
           }
         }
-        ctl.bad[it & 1] = 1;
+        bad_of(it)[kP] = bad_key(it, kC - 1);
       }
       tc::fence_async_smem();
       arrive(ctl.xs);
@@ -338,7 +344,8 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       tc::tc_fence_after();
       const float eg = scalars(it)[SC_EG + lt];
       uint8_t* tile = x_tile(it);
-      const bool bad = ctl.bad[it & 1] != 0;
+      const uint32_t* bad_at = bad_of(it);
+      const bool bad = bad_at[kP] == bad_key(it, kC - 1);
 #pragma unroll 1
       for (int c0 = 0; c0 < kP; c0 += 16) {
         uint32_t y1[16], y1b[16], y2[16];
@@ -362,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
           if (bad) {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-              if (lt >= sBad[(it & 1) * kP + c0 + 8 * c + e]) v[e >> 1] |= 0x7fffu << (16 * (e & 1));
+              if (bad_at[c0 + 8 * c + e] >= bad_key(it, lt)) v[e >> 1] |= 0x7fffu << (16 * (e & 1));
           }
           *reinterpret_cast<uint4*>(tile + at) = u;
         }
@@ -380,12 +387,6 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       }
       tc::fence_async_smem();
       arrive(ctl.x_free[it % kXs]);
-      if (bad) {   // (the flag is one value for the whole group)
-        sm100::group_sync128(1);
-        if (lt < kP) sBad[(it & 1) * kP + lt] = kC;
-        if (lt == 0) ctl.bad[it & 1] = 0;
-        sm100::group_sync128(1);
-      }
     };
 #pragma unroll 1
     for (int it = 0; it <= steps; ++it) {   // the outputs one step behind

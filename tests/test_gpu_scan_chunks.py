@@ -55,6 +55,27 @@ def test_ssd_non_finite_input(N):
     assert torch.equal(torch.isfinite(s), ~gone) and torch.equal(s[~gone], s0[~gone])
 
 
+@pytest.mark.parametrize("B,T,H,N", [(1, 4100, 2, 128), (1, 1100, 4, 128), (1, 1100, 4, 64), (2, 1000, 45, 128)])
+def test_ssd_non_finite_input_in_every_chunk(B, T, H, N):
+    """One non-finite x in each chunk of every segment (eight, four, four and one of them), each in a column of its own: a chunk's notes
+    must not be taken for those of a neighbour that uses the same stage."""
+    g = torch.Generator().manual_seed(T + N)
+    f = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).cuda()
+    x, dt, A, D = f(B, T, H, 64).bfloat16(), f(B, T, H), -torch.exp(f(H)), f(H)
+    Bm, Cm = f(B, T, 1, N, scale=0.5).bfloat16(), f(B, T, 1, N, scale=0.5).bfloat16()
+    y0, s0 = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    bad, gone = torch.zeros_like(y0, dtype=torch.bool), torch.zeros_like(s0, dtype=torch.bool)
+    for c in range(0, T, 128):
+        n = c // 128
+        t, h, q = min(T - 1, c + 37 * n % 128), n % H, (5 * n + 3) % 64
+        x[:, t, h, q] = (float("inf"), float("nan"), -float("inf"))[n % 3]
+        bad[:, t:, h, q] = True
+        gone[:, h, q] = True
+    y, s = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    assert torch.equal(torch.isfinite(y.float()), ~bad) and torch.equal(y[~bad], y0[~bad])
+    assert torch.equal(torch.isfinite(s), ~gone) and torch.equal(s[~gone], s0[~gone])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,H,T,V,layout", [(1, 2, 9, 64, "bhtd"), (2, 3, 31, 128, "bthd"), (1, 2, 130, 64, "bhtd"), (1, 1, 203, 192, "bhtd")])
 def test_rwkv_blocks(dtype, B, H, T, V, layout):
