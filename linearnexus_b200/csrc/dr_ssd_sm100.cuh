@@ -70,6 +70,24 @@ struct Smem {
   static constexpr int kTotal = kBad + kXs * kBadRow * 4;
 };
 
+// 2^{(a + b) - (c + d)} of two float32 pairs, to about one unit in the last place: the difference is taken whole (what a - c loses joins
+// the rests), and e^{f ln 2}, |f| <= 1/2, is its Taylor series to f^7 (the next term is below 6e-9).  Underflows gradually, as exp2f does.
+__device__ __forceinline__ float exp2_diff(float a, float b, float c, float d) {
+  const float s = a - c, t = s - a;
+  const float rest = ((a - (s - t)) - (c + t)) + (b - d);   // (two-sum)
+  const float x = fminf(fmaxf(s, -252.f), 254.f), n = rintf(x), f = (x - n) + rest;
+  float p = 1.5252734e-5f;   // (ln 2)^k / k!
+  p = fmaf(p, f, 1.5403530e-4f);
+  p = fmaf(p, f, 1.3333558e-3f);
+  p = fmaf(p, f, 9.6181291e-3f);
+  p = fmaf(p, f, 5.5504109e-2f);
+  p = fmaf(p, f, 2.4022651e-1f);
+  p = fmaf(p, f, 6.9314718e-1f);
+  p = fmaf(p, f, 1.f);
+  const int e = (int)n, half = e / 2;
+  return p * __int_as_float((127 + half) << 23) * __int_as_float((127 + e - half) << 23);
+}
+
 struct Ctl {
   uint64_t fullB, fullC, fullX[kXs], scal[kXs], xs, d_read[kXs], x_free[kXs], s_rdy, y_read, p_rdy[4];
   uint64_t barDa, barD, barG, barY1a, barY1, barY;
@@ -156,8 +174,11 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       wait_bar(ctl.barG, m & 1);
       tc::tc_fence_after();
       const float Gi = sc[SC_G + lt], ri = sc[SC_R + lt];
-      // left of the warp's 32 x 32 diagonal block the decay is a product of two: to its first row r, and from there
-      const float fi = tc::fast_exp2((Gi - sc[SC_G + 32 * wq]) + (ri - sc[SC_R + 32 * wq]));
+      // Left of the warp's 32 x 32 diagonal block the decay is a product of two: to its first row r, and from there.  Both factors are
+      // exact to about one unit in the last place, since the rounding of a long difference would cost more than the product does:
+      // rms error of a weight between the halves of a chunk 4.0e-8 (decays of 2^-0.2 a token) and 4.1e-8 (2^-1); as one exponential
+      // of the rounded difference 1.8e-7 and 9.8e-7, as the mma.sync form has it across its chunks 9e-8 and 3.9e-7.
+      const float fi = exp2_diff(Gi, ri, sc[SC_G + 32 * wq], sc[SC_R + 32 * wq]);
       const float* sH = sc + SC_H + (wq - 1) * kC;
 #pragma unroll 1
       for (int kb = 0; kb < 4; ++kb) {
@@ -182,11 +203,21 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const float4 G = *reinterpret_cast<const float4*>(sc + SC_G + j0 + 4 * q), r2 = *reinterpret_cast<const float4*>(sc + SC_R + j0 + 4 * q);
+              f[4 * q] = (Gi - G.x) + (ri - r2.x); f[4 * q + 1] = (Gi - G.y) + (ri - r2.y);
+              f[4 * q + 2] = (Gi - G.z) + (ri - r2.z); f[4 * q + 3] = (Gi - G.w) + (ri - r2.w);
+            }
+            // the fast form drops what lies below the normal range; the sums run one way, so the first column has the smallest
+            if (__any_sync(0xffffffffu, f[0] < -125.f)) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) f[e] = exp2f(f[e]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) f[e] = tc::fast_exp2(f[e]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
               const float4 d = *reinterpret_cast<const float4*>(sc + SC_DT + j0 + 4 * q);
-              f[4 * q] = tc::fast_exp2((Gi - G.x) + (ri - r2.x)) * d.x;
-              f[4 * q + 1] = tc::fast_exp2((Gi - G.y) + (ri - r2.y)) * d.y;
-              f[4 * q + 2] = tc::fast_exp2((Gi - G.z) + (ri - r2.z)) * d.z;
-              f[4 * q + 3] = tc::fast_exp2((Gi - G.w) + (ri - r2.w)) * d.w;
+              f[4 * q] *= d.x; f[4 * q + 1] *= d.y; f[4 * q + 2] *= d.z; f[4 * q + 3] *= d.w;
             }
             tc::tc_wait_ld();
 #pragma unroll
@@ -558,9 +589,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
         const float x = GL - G;   // the sums of a head run one way: what is lost here is (GL - x) - G
         sc[SC_EG + j] = exp2f(G) * (1.f + kLn2 * R);
         sc[SC_W + j] = d * exp2f(x) * (1.f + kLn2 * (((GL - x) - G) + (RL - R)));
-#pragma unroll
-        for (int q = 1; q < 4; ++q)
-          sc[SC_H + (q - 1) * kC + j] = r < q ? d * tc::fast_exp2((sc[SC_G + 32 * q] - G) + (sc[SC_R + 32 * q] - R)) : 0.f;
+#pragma unroll 1
+        for (int q = it < n1 ? 4 : r + 1; q < 4; ++q)   // (P alone needs them)
+          sc[SC_H + (q - 1) * kC + j] = d * exp2_diff(sc[SC_G + 32 * q], sc[SC_R + 32 * q], G, R);
       }
       __syncwarp();
       if (lane == 0) arrive(ctl.scal[it % kXs]);

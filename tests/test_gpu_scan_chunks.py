@@ -1,6 +1,8 @@
 """The chunk forms of the state scans (bf16 storage) at the edges of their tiles: ragged ends, the smallest length they
 take, several value slices, grouped B and C, and the segmented (cluster) launch.  float32 state within 1e-4 and outputs
 within one bf16 rounding of the float64 recurrence."""
+import math
+
 import pytest
 import torch
 
@@ -124,6 +126,63 @@ def test_ssd_reset_then_accumulate(B, T, H, N, first, A):
     ry, rs = R.ssd_token_recurrence(d(x), d(dt), d(Ah), d(Bm), d(Cm), d(D), ssm_state=d(h0))
     _check(s, rs, 1.5e-6)
     _check(y, ry, 5e-3)
+
+
+@pytest.mark.parametrize("first,second", [((2, 64), (0, 62)), ((66, 128), (64, 126)), ((70, 128), (0, 64))])
+@pytest.mark.parametrize("most", [0.02, 0.2, 1.0])
+def test_ssd_decay_weights_inside_a_chunk(first, second, most):
+    """The weight of token j in the output of token i, e^{G_i - G_j} dt_j, to float32 precision: in every head two tokens whose weighted
+    inputs cancel but for what float32 leaves of the second one's factor, so that the output is the error.  Tokens i from one
+    half of a chunk of 128, j and k from the same or the other half; decays of up to ``most`` powers of two a token.
+
+    Expected of each of the two weights, as relative variance.  Tokens of one 32-row block: one exponential of the rounded difference d
+    (log2 units; two sums, each uniform over one unit in the last place of d, times ln 2; the exponential itself 6.0e-8 rms, measured
+    over [-120, 0]) and two products (uniform, 2^-24 at most).  Other tokens: two factors of about one unit in the last place
+    (2.6e-8 rms each) and three products.  512 heads: the rms over that expectation scatters by 3 %; bound five times that."""
+    g = torch.Generator().manual_seed(first[0] + 1000 * second[1])
+    Bt, H, T, N = 64, 8, 128, 128
+    A = -(torch.rand(H, generator=g) * 0.9 + 0.1) * most * 4 * math.log(2)      # dt = 1/4
+    x, Bm, Cm = torch.zeros(Bt, T, H, 64), torch.zeros(Bt, T, H, N), torch.zeros(Bt, T, H, N)
+    pick = lambda r: torch.randint(*r, (Bt, H), generator=g)
+    i, j, k = pick(first), pick(second), pick(second)
+    j, k = torch.minimum(j, i - 1), torch.minimum(k, i - 1)
+    k = torch.where(k == j, torch.where(j > 0, j - 1, j + 1), k)
+    b, h = torch.arange(Bt)[:, None].expand(Bt, H), torch.arange(H)[None].expand(Bt, H)
+    log_w = (A * 0.25).double()[None]
+    wj, wk = torch.exp(log_w * (i - j)), torch.exp(log_w * (i - k))
+    factor = -(wj / wk).float()
+    hi = factor.bfloat16().float()
+    mid = (factor - hi).bfloat16().float()
+    lo = (factor - hi - mid).bfloat16().float()      # three bf16 terms are the float32 number
+    Cm[b, i, h, 0] = Cm[b, i, h, 1] = Cm[b, i, h, 2] = 1
+    Bm[b, j, h, 0] = 1
+    Bm[b, k, h, 0], Bm[b, k, h, 1], Bm[b, k, h, 2] = hi, mid, lo
+    x[b, j, h] = x[b, k, h] = 1
+    c = lambda t: t.cuda()
+    y, _ = L.ssd_chunk_scan(c(x).bfloat16(), c(torch.zeros(Bt, T, H)), c(A), c(Bm).bfloat16(), c(Cm).bfloat16(), c(torch.zeros(H)),
+                            n_groups=H, dt_limit=(0.25, 0.25))
+    err = (y.double().cpu()[b, i, h, 0] / 0.25 - (wj + (hi.double() + mid + lo) * wk)) / wj
+    var = torch.zeros_like(err)
+    for col in (j, k):
+        d = (log_w * (i - col)).abs() / math.log(2)
+        ulp = torch.exp2(torch.floor(torch.log2(d)) - 23)
+        near = 2 * (ulp * math.log(2)) ** 2 / 12 + 6.0e-8 ** 2 + 2 * 2.0 ** -48 / 3
+        var += torch.where(i // 32 == col // 32, near, torch.full_like(d, 2 * 2.6e-8 ** 2 + 3 * 2.0 ** -48 / 3))
+    use = (i >= 2) & (k < i) & (k != j)
+    assert (err ** 2 / var)[use].mean().sqrt().item() <= 1.15
+
+
+@pytest.mark.parametrize("apart", [1, 40])
+def test_ssd_weights_below_the_normal_range(apart):
+    """A weight of 2^-130 between two tokens of a chunk still counts (as in the token recurrence): the input times 2^120 is 2^-10."""
+    T, j = 128, 20
+    x, Bm, Cm = torch.zeros(1, T, 1, 64), torch.zeros(1, T, 1, 128), torch.zeros(1, T, 1, 128)
+    A = torch.tensor([-4 * 130 / apart * math.log(2)])
+    x[0, j], Bm[0, j, 0, 0], Cm[0, j + apart, 0, 0] = 1, 2.0 ** 60, 2.0 ** 60
+    c = lambda t: t.cuda()
+    y, _ = L.ssd_chunk_scan(c(x).bfloat16(), c(torch.zeros(1, T, 1)), c(A), c(Bm).bfloat16(), c(Cm).bfloat16(), c(torch.zeros(1)), dt_limit=(0.25, 0.25))
+    want = 0.25 * math.exp(A.double().item() * 0.25 * apart) * 2.0 ** 120
+    assert (y[0, j + apart].double().cpu() / want - 1).abs().max().item() <= 5e-3
 
 
 @pytest.mark.parametrize("T", [9, 39, 40, 41])
