@@ -26,6 +26,9 @@
 // distributed shared memory (S is linear in its start: S_end = decay S_start + S_local), then each runs its segment in
 // full from its true start.  That costs 1.4x the work and divides the chain by the cluster size.
 //
+// Infinities and NaN in x: P is 0 above the diagonal, but 0 x inf is NaN, and sixteen tokens enter one product.  Such an entry is taken
+// out of the operand of P x (the state gets it), and the outputs of its column from its token on become NaN.
+//
 // What bounds it: 1940 mma per chunk and head (N = 128) of 8 cycles each per scheduler, 3.9 K cycles; the token
 // recurrence needs 3 K V FMAs per token = 64 x 192 cycles and ran at 64 x 900.
 #pragma once
@@ -58,7 +61,8 @@ struct Smem {
   static constexpr int kSt = kY + kC * 68 * 4;              // this segment's end state fp32 [64][N] (clusters)
   static constexpr int kSc = kSt + kP * N * 4;              // per stage: G[64], e^G[64], dt[64], dt e^{G_L - G}[64], rest of G[64]
   static constexpr int kDec = kSc + 2 * kScalars * 4;       // this segment's decay
-  static constexpr int kTotal = kDec + 16;
+  static constexpr int kBad = kDec + 16;                     // see bad_key; one word per value column, one for the whole chunk
+  static constexpr int kTotal = kBad + (kP + 4) * 4;
 };
 
 template <int N>
@@ -246,6 +250,12 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
     cluster.sync();   // the others have read this CTA's copy (and p.hT may alias p.h0)
   }
 
+  // Non-finite x of a chunk: per column the largest bad_key of such a token.  A word of an earlier chunk is smaller than every key of
+  // this one; words are written behind the barrier at "P is complete" and read behind the next.
+  uint32_t* sBad = reinterpret_cast<uint32_t*>(smem + L::kBad);
+  auto bad_key = [&](int c, int token) { return (uint32_t)(c + 1) * kC + (kC - 1 - token); };
+  if (tid <= kP) sBad[tid] = 0u;   // (the first barrier of the loop lies before the first use)
+
   const uint32_t sPm = sbase + L::kPm;
   float* sY = reinterpret_cast<float*>(smem + L::kY);
   __nv_bfloat16* sYo = reinterpret_cast<__nv_bfloat16*>(smem + L::kPm);   // output rows: the P tiles are dead by then
@@ -332,6 +342,21 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
       const int kt = nh ? 1 + kk : 3 * kk;
       uint32_t xb[4];
       mma::ldsm4t(xb, mma::frag_bt(tile_X(st), LDX, 16 * kt, p0, lane));
+      __nv_bfloat162 inf = __floats2bfloat162_rn(0.f, 0.f);   // 0 x every entry: NaN if one is not finite
+#pragma unroll
+      for (int r = 0; r < 4; ++r) inf = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&xb[r]), __floats2bfloat162_rn(0.f, 0.f), inf);
+      if (__hisnan(inf.x) || __hisnan(inf.y)) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {   // entry: token 16 kt + 2t + (e & 1) + 8 (e >> 1 & 1), column p0 + g + 8 (e >> 2)
+          const uint32_t half = (e & 1) ? 0xffff0000u : 0xffffu, exp = half & 0x7f807f80u;
+          if ((xb[e >> 1] & exp) == exp) {
+            xb[e >> 1] &= ~half;
+            atomicMax(sBad + p0 + g + 8 * (e >> 2), bad_key(c, 16 * kt + 2 * t + (e & 1) + 8 * ((e >> 1) & 1)));
+          }
+        }
+        sBad[kP] = bad_key(c, kC - 1);
+      }
+      __syncwarp();
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt) {
         if (mt >= kt) {
@@ -358,6 +383,7 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
       }
     }
     __syncthreads();   // partials written; every warp is done with P
+    const bool bad = sBad[kP] == bad_key(c, kC - 1);
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
 #pragma unroll
@@ -369,8 +395,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_chunk_kernel(const LinRecPara
           const int i = 16 * mt + g + 8 * hr, cc = p0 + 8 * r + 2 * t;
           const float2 o = *reinterpret_cast<const float2*>(sY + i * 68 + cc);
           const uint32_t xx = *reinterpret_cast<const uint32_t*>(smem + L::kB + st * L::kStage + 2 * L::kTileN + 2 * (i * LDX + cc));
-          *reinterpret_cast<uint32_t*>(sYo + i * LDX + cc) =
-              mma::pack(v[2 * hr] + o.x + D_h * mma::lo_f(xx), v[2 * hr + 1] + o.y + D_h * mma::hi_f(xx));
+          uint32_t out = mma::pack(v[2 * hr] + o.x + D_h * mma::lo_f(xx), v[2 * hr + 1] + o.y + D_h * mma::hi_f(xx));
+          if (bad) out |= (sBad[cc] >= bad_key(c, i) ? 0x7fffu : 0u) | (sBad[cc + 1] >= bad_key(c, i) ? 0x7fff0000u : 0u);
+          *reinterpret_cast<uint32_t*>(sYo + i * LDX + cc) = out;
         }
       }
     }

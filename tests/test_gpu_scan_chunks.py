@@ -57,6 +57,26 @@ def test_ssd_non_finite_input(N):
     assert torch.equal(torch.isfinite(s), ~gone) and torch.equal(s[~gone], s0[~gone])
 
 
+@pytest.mark.parametrize("T,N", [(32, 128), (64, 64), (64, 128), (1000, 64)])
+def test_ssd_non_finite_input_in_short_sequences(T, N):
+    """The same in the mma.sync form: nothing before the token, and not the rest of its sixteen-token block either."""
+    g = torch.Generator().manual_seed(T + N)
+    f = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).cuda()
+    x, dt, A, D = f(1, T, 2, 64).bfloat16(), f(1, T, 2), -torch.exp(f(2)), f(2)
+    Bm, Cm = f(1, T, 1, N, scale=0.5).bfloat16(), f(1, T, 1, N, scale=0.5).bfloat16()
+    y0, s0 = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    bad, gone = torch.zeros_like(y0, dtype=torch.bool), torch.zeros_like(s0, dtype=torch.bool)
+    for n, t in enumerate(range(15, T, 53)):
+        h, q = n % 2, (11 * n + 3) % 64
+        x[0, t, h, q] = (float("inf"), float("nan"), -float("inf"))[n % 3]
+        bad[0, t:, h, q] = True
+        gone[0, h, q] = True
+    x[0, T - 1, 0, 63], bad[0, T - 1, 0, 63], gone[0, 0, 63] = float("nan"), True, True
+    y, s = L.ssd_chunk_scan(x, dt, A, Bm, Cm, D)
+    assert torch.equal(torch.isfinite(y.float()), ~bad) and torch.equal(y[~bad], y0[~bad])
+    assert torch.equal(torch.isfinite(s), ~gone) and torch.equal(s[~gone], s0[~gone])
+
+
 @pytest.mark.parametrize("B,T,H,N", [(1, 4100, 2, 128), (1, 1100, 4, 128), (1, 1100, 4, 64), (2, 1000, 45, 128)])
 def test_ssd_non_finite_input_in_every_chunk(B, T, H, N):
     """One non-finite x in each chunk of every segment (eight, four, four and one of them), each in a column of its own: a chunk's notes
