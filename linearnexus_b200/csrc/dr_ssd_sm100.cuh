@@ -171,8 +171,6 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       const int m = it - n1;
       const float* sc = scalars(it);
       wait_bar(ctl.scal[it % kXs], (it / kXs) & 1);
-      wait_bar(ctl.barG, m & 1);
-      tc::tc_fence_after();
       const float Gi = sc[SC_G + lt], ri = sc[SC_R + lt];
       // Left of the warp's 32 x 32 diagonal block the decay is a product of two: to its first row r, and from there.  Both factors are
       // exact to about one unit in the last place, since the rounding of a long difference would cost more than the product does:
@@ -180,6 +178,8 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
       // of the rounded difference 1.8e-7 and 9.8e-7, as the mma.sync form has it across its chunks 9e-8 and 3.9e-7.
       const float fi = exp2_diff(Gi, ri, sc[SC_G + 32 * wq], sc[SC_R + 32 * wq]);
       const float* sH = sc + SC_H + (wq - 1) * kC;
+      wait_bar(ctl.barG, m & 1);
+      tc::tc_fence_after();
 #pragma unroll 1
       for (int kb = 0; kb < 4; ++kb) {
         const int j0 = 64 * jh + 16 * kb;
