@@ -9,7 +9,7 @@
 namespace dr {
 
 cudaError_t launch_linrec(int kind, bool io_bf16, const LinRecParams& p, int sms, cudaStream_t stream) {
-  if (kind == LR_SSD && io_bf16 && ssd::eligible(p)) return ssdu::ahead(p, sms) ? ssdu::launch(p, sms, stream) : ssd::launch(p, sms, stream);
+  if (kind == LR_SSD && io_bf16 && ssd::eligible(p)) return ssdu::ahead(p) ? ssdu::launch(p, stream) : ssd::launch(p, sms, stream);
   if (kind != LR_SSD && rwkv::eligible(kind, io_bf16, p, sms)) return rwkv::launch(kind, io_bf16, p, stream);
   return launch_linrec_tokens(kind, io_bf16, p, stream);
 }

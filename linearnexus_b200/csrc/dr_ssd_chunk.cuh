@@ -1,5 +1,5 @@
-// Mamba-2 SSD scan in chunk form on the warp-level tensor cores, bf16 storage, float32-exact products.  One chunk, and short
-// sequences of half-size states; the rest runs on tcgen05 (dr_ssd_sm100.cuh, ssdu::ahead).
+// Mamba-2 SSD scan in chunk form on the warp-level tensor cores, bf16 storage, float32-exact products.  One chunk, and few
+// sequences of medium length with half-size states; the rest runs on tcgen05 (dr_ssd_sm100.cuh, ssdu::ahead).
 //
 // With a_t = A dt_t, G the running sum of a over a 64-token chunk and S [P][N] the state at its start:
 //     P_ij = (C_i . B_j) e^{G_i - G_j} dt_j   (j <= i)

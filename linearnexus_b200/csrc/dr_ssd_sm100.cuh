@@ -615,27 +615,51 @@ inline bool make_map(CUtensorMap* m, const LrVec& v, int cols, int B, int heads,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// How many clusters of 2, 4 and 8 CTAs run at once (B200: 74, 33, 15, as the SMs of a GPC divide), once per host thread and device.
+struct ClusterFit { int dev = -1, n[4] = {0, 0, 0, 0}; };
 template <int N>
-inline cudaError_t launch_n(const LinRecParams& p, int sms, cudaStream_t stream) {
-  auto kern = ssd_sm100_kernel<N>;
-  thread_local int attr_dev = -1;
+inline cudaError_t cluster_fit(const ClusterFit** out) {
+  thread_local ClusterFit fit;
+  *out = &fit;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (attr_dev != dev) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<N>::kTotal);
-    if (e != cudaSuccess) return e;
-    attr_dev = dev;
+  if (e != cudaSuccess || fit.dev == dev) return e;
+  e = cudaFuncSetAttribute(ssd_sm100_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<N>::kTotal);
+  for (int i = 1; i < 4 && e == cudaSuccess; ++i) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1u << i);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = Smem<N>::kTotal;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << i;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaOccupancyMaxActiveClusters(&fit.n[i], ssd_sm100_kernel<N>, &cfg);
   }
+  if (e == cudaSuccess) fit.dev = dev;
+  return e;
+}
+
+template <int N>
+inline cudaError_t launch_n(const LinRecParams& p, cudaStream_t stream) {
+  auto kern = ssd_sm100_kernel<N>;
+  const ClusterFit* fit;
+  const cudaError_t e = cluster_fit<N>(&fit);
+  if (e != cudaSuccess) return e;
   const int64_t ctas = (int64_t)p.B * p.H * (p.V / kP);
   const int nchunks = (p.T + kC - 1) / kC;
-  // Segments: a step of the first pass costs half of a full one, and every segment reads all earlier ends.  Four from four chunks on (8 heads,
-  // T=400: 19.7 us, 21.0 with two, 32.5 in the mma.sync form; T=300 with two segments 19.8, whole 15.3); eight only from 32 chunks
-  // on and for at most eight clusters (T=4000: 46 against 54 us with four; sixteen clusters of eight run in two waves: 16 heads, T=2000: 67
-  // against 37).
+  // Segments: a step of the first pass costs half of a full one, and every segment reads all earlier ends; clusters that do not all run
+  // at once cost a second wave (N = 128, T=400 in fours: 33 CTAs 20.8 us, 34 of them 37.8; 20.8 whole).  Us at N = 128, chunks:
+  //   8 CTAs    4: 19.8 whole, 19.1 in fours, 31.5 in eights   5: 23.3, 24.4, 31.6   7: 30.6, 24.5, 31.8   8: 34.1, 24.6, 31.9
+  //             16: 62.3, 35.7, 37.1   20: 41.6 in fours, 42.7 in eights   22: 47.2, 42.9   32: 57.8, 48.2   (6, 28 CTAs: 28.2, 26.2)
+  //   74 CTAs   4: 20.6 whole, 22.7 in pairs   7: 31.5, 34.3   8: 35.0, 34.3   9: 38.6, 40.3   12: 49.2, 46.2   16: 63.5, 58.0
+  // N = 64 is up to 8 % below, with the same crossings (four chunks whole: 18.0, in fours 18.5).
   int nseg = 1;
-  while (nseg < 4 && ctas * nseg * 2 <= sms && nchunks >= 4) nseg *= 2;
-  if (nseg == 4 && ctas <= 8 && nchunks >= 32) nseg = 8;
+  if (nchunks > 20 && ctas <= fit->n[3]) nseg = 8;
+  else if ((nchunks == 4 || nchunks > 5) && ctas <= fit->n[2]) nseg = 4;
+  else if (nchunks >= 8 && ctas <= fit->n[1]) nseg = 2;
   Params P;
   P.p = p;
   P.nseg = nseg;
@@ -658,16 +682,22 @@ inline cudaError_t launch_n(const LinRecParams& p, int sms, cudaStream_t stream)
   return cudaLaunchKernelEx(&cfg, kern, P);
 }
 
-// What ssd::eligible takes, but for a single 64-token chunk (8 heads, T=64: 9.6 us here, 8.5 there; 256 heads 20.7 / 16.3) and for
-// half-size states in so few chunks that the chain of this form is longer (N=64, 8 heads, T=600: 23.8 / 21.4; T=1000: 23.9 / 21.9;
-// T=400: 19.7 / 32).
-inline bool ahead(const LinRecParams& p, int sms) {
-  const int64_t ctas = (int64_t)p.B * p.H * (p.V / kP);
-  return p.T > 64 && !(p.K == 64 && p.T > 512 && p.T <= 1024 && ctas * 4 <= sms) && sm100::encode_tiled_fn() != nullptr;
+// What ssd::eligible takes, but for
+//  * a single 64-token chunk (8 heads, T=64: 9.6 us here, 8.5 there; 256 heads 20.7 / 16.3);
+//  * half-size states in few sequences where the other form's segments, of half the chunk and less fixed cost, come out ahead while
+//    they all run at once: four of them for 513 to 768 tokens (N = 64, 28 CTAs, T = 513 / 640 / 768: 22.5 / 22.8 / 25.2 here, 21.9 /
+//    22.0 / 22.2 there; T = 800, 16 CTAs: 23.8 / 26.5), eight for 961 to 2560 (8 CTAs, T = 960 / 961 / 1300 / 2048 / 2560 / 2816: 23.5 /
+//    23.5 / 28.7 / 34.0 / 39.3 / 41.2 here, 26.4 / 21.6 / 26.3 / 32.0 / 37.1 / 41.8 there; 16 CTAs, T = 1024: 23.9 / 38.1).
+inline bool ahead(const LinRecParams& p) {
+  if (p.T <= 64 || !sm100::encode_tiled_fn()) return false;
+  const bool four = p.T > 512 && p.T <= 768, eight = p.T > 960 && p.T <= 2560;
+  if (p.K != 64 || !(four || eight)) return true;
+  const ClusterFit* fit;
+  return cluster_fit<64>(&fit) != cudaSuccess || (int64_t)p.B * p.H * (p.V / kP) > fit->n[four ? 2 : 3];
 }
 
-inline cudaError_t launch(const LinRecParams& p, int sms, cudaStream_t stream) {
-  return p.K == 64 ? launch_n<64>(p, sms, stream) : launch_n<128>(p, sms, stream);
+inline cudaError_t launch(const LinRecParams& p, cudaStream_t stream) {
+  return p.K == 64 ? launch_n<64>(p, stream) : launch_n<128>(p, stream);
 }
 
 }  // namespace ssdu

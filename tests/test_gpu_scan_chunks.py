@@ -22,7 +22,12 @@ def _check(got, ref, tol):
                                          # tcgen05 form: one chunk, a whole one, one token more; four and eight segments, empty ones among
                                          # them; more CTAs than SMs; three value slices
                                          (1, 127, 2, 64, 64, 1), (2, 128, 2, 64, 128, 1), (1, 513, 3, 192, 128, 1), (1, 641, 2, 64, 128, 2),
-                                         (1, 4100, 1, 64, 64, 1), (5, 257, 32, 64, 128, 1)])
+                                         (1, 4100, 1, 64, 64, 1), (5, 257, 32, 64, 128, 1),
+                                         # both sides of the lines between whole sequences, two, four and eight segments (15, 33 and 74
+                                         # clusters at once), and of those to the mma.sync form at N = 64
+                                         (1, 641, 33, 64, 128, 1), (1, 700, 34, 64, 128, 1), (1, 900, 37, 128, 128, 1), (1, 900, 25, 192, 64, 1),
+                                         (1, 2561, 15, 64, 128, 1), (1, 2600, 16, 64, 64, 1), (1, 768, 33, 64, 64, 1), (1, 769, 4, 64, 64, 1), (1, 960, 4, 64, 64, 1), (1, 961, 15, 64, 64, 1),
+                                         (1, 961, 16, 64, 64, 1), (1, 2560, 5, 192, 64, 1), (1, 2561, 3, 64, 64, 1)])
 def test_ssd_chunks(B, T, H, P, N, G):
     g = torch.Generator().manual_seed(T)
     f = lambda *s, scale=1.0: torch.randn(*s, generator=g) * scale
