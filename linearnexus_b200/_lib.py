@@ -36,7 +36,7 @@ DEVICE_STATUS_BITS = {1: "a bounded wait on an mbarrier ran out", 2: "an index c
 
 
 def device_status_site(word: int):
-    """(barrier number, warp group) of the first wait that gave up in a tcgen05 kernel, from bits 8..15 of the device
+    """(barrier number, warp group) of the recorded wait that gave up in a tcgen05 kernel, from bits 8..15 of the device
     status word (DR_DEV_SITE in include/deltarule_sm100.h); None when the word carries no timeout."""
     if not word & 1:
         return None

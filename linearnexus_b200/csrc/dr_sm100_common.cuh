@@ -28,7 +28,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 
 // The rest of a wait whose first try_wait came back empty, kept out of line (the kernel's speed follows its code size).
 // Bounded; when the bound runs out every later wait of the CTA returns at once (abort flag), DR_DEV_TIMEOUT is set, and
-// the first such wait of the launch leaves its place in bits 8..15 of the status word (bits 8..13: the barrier's number
+// the first such wait to get there leaves its place in bits 8..15 of the status word (bits 8..13: the barrier's number
 // in the control block, 63 for one behind the float arrays; bits 14..15: the warp group).
 static __device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int32_t* status, int* abort_flag, uint32_t bar_offset,
                                        uint32_t grp) {
@@ -43,7 +43,9 @@ static __device__ __noinline__ void wait_more(uint32_t bar, uint32_t parity, int
 }
 
 // The same in line, for kernels with few sites or with many live registers (a call costs its site more code than the loop): the place
-// goes to the abort flag, which the kernel's last thread hands to the status word with report_wait.
+// goes to the abort flag, which one thread hands to the status word at the kernel's end with report_wait: the place of a wait that found
+// no other's record (of several that run out within the same few cycles, the last to store; a compare-and-swap at the sites costs
+// the Mamba-2 scan 4 %), in the first CTA to end.
 __device__ __forceinline__ int wait_record(uint32_t bar_offset, uint32_t grp) {
   const uint32_t num = bar_offset / 8u < 63u ? bar_offset / 8u : 63u;
   return DR_DEV_TIMEOUT | (int)((num | (grp << 6)) << 8);
