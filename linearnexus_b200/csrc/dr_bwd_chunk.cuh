@@ -625,6 +625,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
     sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp >> 3);
   };
   const int64_t chunk0 = (int64_t)unit * p.N;
+  const int steps = p.dh0 ? p.N : p.N - 1;   // the product of the first chunk gives the initial state's gradient alone
   if (warp == 8) {
     if (tc::elect_one()) {
       auto n_at = [&](int it) { return reinterpret_cast<const uint8_t*>(p.nf) + (chunk0 + p.N - 1 - it) * kNTile; };
@@ -642,15 +643,13 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         tc::tma_load_4d(sbase + CH_O + (it & 1) * kOTile, &P.to, v0, h, (p.N - 1 - it) * kC, b, bar);
         tc::bulk_g2s(sbase + CH_Y + (it & 1) * kYTile, y_at(it), kYTile, bar);
       };
-      load_y(0);
-      load_h(0);
-      load_l(0);
-      if (p.N > 1) { load_y(1); load_h(1); }
+      if (steps > 0) { load_y(0); load_h(0); load_l(0); }
+      if (steps > 1) { load_y(1); load_h(1); }
       constexpr uint32_t id = tc::idesc_bf16(128, 64, 0, 1);
       auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
       const uint64_t sd = tc::smem_desc_sw128(sbase + CH_S, 128 * 128, 1024), ld = tc::smem_desc(sbase + CH_L, 128, sm100::RBS);
 #pragma unroll 1
-      for (int it = 0; it < p.N; ++it) {
+      for (int it = 0; it < steps; ++it) {
         const uint32_t acc = tbase + (it & 1) * 64;   // (read for chunk it - 2 before its successor's dS was ready)
         const uint64_t yd = tc::smem_desc(sbase + CH_Y + (it & 1) * kYTile, 128, kYRbs);
         const uint64_t od = tc::smem_desc_sw128(sbase + CH_O + (it & 1) * kOTile, 128 * 128, 1024);
@@ -677,10 +676,10 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
         tc::mma_commit(tc::smem_u32(&ctl.bar_d));
         wait_bar(ctl.bar_y, it & 1);   // Y^T and d_o have been read
-        if (it + 2 < p.N) load_y(it + 2);
+        if (it + 2 < steps) load_y(it + 2);
         wait_bar(ctl.bar_d, it & 1);   // N has been read
-        if (it + 1 < p.N) load_l(it + 1);
-        if (it + 2 < p.N) load_h(it + 2);
+        if (it + 1 < steps) load_l(it + 1);
+        if (it + 2 < steps) load_h(it + 2);
       }
     }
     __syncwarp();
@@ -699,21 +698,23 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
     for (int it = 0; it < p.N; ++it) {
       const int64_t chunk = chunk0 + p.N - 1 - it;
       const float el = p.el[chunk * 128 + row];
+      if (it < steps) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t hi[4], lo[4];
+        for (int c = 0; c < 4; ++c) {
+          uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float x = S[8 * c + 2 * e], y = S[8 * c + 2 * e + 1];
-          hi[e] = mma::pack(x, y);
-          lo[e] = mma::pack(x - mma::lo_f(hi[e]), y - mma::hi_f(hi[e]));
+          for (int e = 0; e < 4; ++e) {
+            const float x = S[8 * c + 2 * e], y = S[8 * c + 2 * e + 1];
+            hi[e] = mma::pack(x, y);
+            lo[e] = mma::pack(x - mma::lo_f(hi[e]), y - mma::hi_f(hi[e]));
+          }
+          uint8_t* dst = smem + CH_S + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
+          *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(dst + 128 * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
-        uint8_t* dst = smem + CH_S + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
-        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(dst + 128 * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        tc::fence_async_smem();
+        sm100::mbar_arrive(tc::smem_u32(&ctl.rdy));
       }
-      tc::fence_async_smem();
-      sm100::mbar_arrive(tc::smem_u32(&ctl.rdy));
       // dS1 of this chunk -> memory, sixteen rows at a time through the warp's 2 KB: whole 128-byte lines (a thread's own row in 16-byte
       // pieces made the write the longest part of a chunk)
       float* ds = p.ds + chunk * (kD * kD) + (int64_t)(32 * (warp & 3)) * kD + v0 + 32 * hc;
@@ -733,6 +734,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         }
         __syncwarp();
       }
+      if (it == steps) break;
       wait_bar(ctl.bar_d, it & 1);
       tc::tc_fence_after();
       uint32_t d[32];

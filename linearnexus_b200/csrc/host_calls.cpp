@@ -339,11 +339,12 @@ PyObject* py_train_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// train_bwd(variant, q, k, v, g, beta, d_o, d_hT, scale, chunk, l2norm, workspace) -> (dq, dk, dv, dg, dbeta, dh0) | status | None
+// train_bwd(variant, q, k, v, g, beta, d_o, d_hT, scale, chunk, l2norm, workspace, want_dh0) -> (dq, dk, dv, dg, dbeta, dh0 | None) | status | None
 PyObject* py_train_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n == 12);
+    need(n == 13);
     Training t(a, a[8], a[9], a[10], -1);
+    const bool want_dh0 = a[12] == Py_True;
     const at::Tensor &given = t.c.req(a[6]), &ws = t.c.req(a[11]);
     const at::Tensor* d_hT = t.c.opt(a[7]);
     need(is_shape(given, {t.B, t.H, t.T, t.V}) && t.laid_out(given));
@@ -353,15 +354,16 @@ PyObject* py_train_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need(ws.scalar_type() == at::kByte && ws.is_contiguous() && ws.numel() >= ws_bytes);
     const at::Tensor d_o = given.to(t.q->scalar_type());   // (keeps the layout; KDA's output is float32)
     const at::Tensor dq = t.like(*t.q, t.q->scalar_type()), dk = t.like(*t.k, t.q->scalar_type()), dv = t.like(*t.v, t.q->scalar_type());
-    const at::Tensor dbeta = t.like(*t.beta, at::kFloat), dh0 = t.c.empty({t.B, t.H, t.K, t.V}, at::kFloat);
-    at::Tensor dg;
+    const at::Tensor dbeta = t.like(*t.beta, at::kFloat);
+    at::Tensor dg, dh0;
     if (t.g) dg = t.like(*t.g, at::kFloat);
+    if (want_dh0) dh0 = t.c.empty({t.B, t.H, t.K, t.V}, at::kFloat);
     void* stream = t.c.stream();
     int st;
     {
       Unlocked u;
       st = api.chunk_bwd_saved(&t.d, ptr(*t.q), ptr(*t.k), ptr(*t.v), ptr(t.g), fptr(t.beta), ptr(d_o), fptr(d_hT), dq.mutable_data_ptr(),
-                               dk.mutable_data_ptr(), dv.mutable_data_ptr(), fmut(dbeta), t.g ? fmut(dg) : nullptr, fmut(dh0),
+                               dk.mutable_data_ptr(), dv.mutable_data_ptr(), fmut(dbeta), t.g ? fmut(dg) : nullptr, want_dh0 ? fmut(dh0) : nullptr,
                                ws.mutable_data_ptr(), (size_t)ws.numel(), t.c.status(), stream);
     }
     if (st < 0) return PyLong_FromLong(st);
@@ -369,14 +371,14 @@ PyObject* py_train_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(dq));
     PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(dk));
     PyTuple_SET_ITEM(r, 2, THPVariable_Wrap(dv));
-    if (t.g) {
-      PyTuple_SET_ITEM(r, 3, THPVariable_Wrap(dg));
-    } else {
+    auto wrapped = [](bool there, const at::Tensor& x) -> PyObject* {
+      if (there) return THPVariable_Wrap(x);
       Py_INCREF(Py_None);
-      PyTuple_SET_ITEM(r, 3, Py_None);
-    }
+      return Py_None;
+    };
+    PyTuple_SET_ITEM(r, 3, wrapped(t.g != nullptr, dg));
     PyTuple_SET_ITEM(r, 4, THPVariable_Wrap(dbeta));
-    PyTuple_SET_ITEM(r, 5, THPVariable_Wrap(dh0));
+    PyTuple_SET_ITEM(r, 5, wrapped(want_dh0, dh0));
     return r;
   });
 }

@@ -374,7 +374,7 @@ def chunk_forward_saving(variant, q, k, v, g, beta, initial_state=None, scale=No
 
 
 def chunk_backward(variant, q, k, v, g, beta, d_o, initial_state=None, d_final_state=None, scale=None,
-                   chunk_size=64, use_qk_l2norm=True, saved=None):
+                   chunk_size=64, use_qk_l2norm=True, saved=None, _want_dh0=True):
     """Gradients of sum(o * d_o) + sum(final_state * d_final_state) for ``variant`` in
     {"delta", "gated", "kda"}.  Returns a dict: dq, dk [like q: with grouped q/k heads, summed over each
     group's value heads], dv [like v] in the q/k/v dtype;
@@ -383,7 +383,7 @@ def chunk_backward(variant, q, k, v, g, beta, d_o, initial_state=None, d_final_s
     the buffer is consumed)."""
     if saved is not None and variant in _VARIANTS:
         r = _native_calls().train_bwd(_VARIANTS[variant], q, k, v, g, beta, d_o, d_final_state, scale, chunk_size,
-                                      bool(use_qk_l2norm), saved)
+                                      bool(use_qk_l2norm), saved, _want_dh0)
         if r.__class__ is tuple:
             return dict(zip(("dq", "dk", "dv", "dg", "dbeta", "dh0"), r))
     _require_cuda(q, k, v, g, beta, d_o, initial_state, d_final_state)
@@ -401,7 +401,7 @@ def chunk_backward(variant, q, k, v, g, beta, d_o, initial_state=None, d_final_s
     dq, dk, dv = torch.empty_like(qn), torch.empty_like(kn), torch.empty_like(vn)
     dbeta = torch.empty_like(bn)
     dg = None if g is None else torch.empty_like(gn, dtype=torch.float32)
-    dh0 = torch.empty((B, H, K, V), dtype=torch.float32, device=dev)
+    dh0 = torch.empty((B, H, K, V), dtype=torch.float32, device=dev) if _want_dh0 else None
     with torch.cuda.device(dev):
         if saved is None:
             st = lib.dr_chunk_bwd(ctypes.byref(d), _ptr(qn), _ptr(kn), _ptr(vn), _ptr(gn), _ptr(bn), _ptr(h0), _ptr(don),
@@ -454,11 +454,12 @@ class _ChunkFn(torch.autograd.Function):
         saved, ctx.saved_ws = ctx.saved_ws, None   # consumed: a second backward recomputes
         if d_o is None:
             d_o = torch.zeros_like(v)
+        want_dh0 = has_h0 and ctx.needs_input_grad[6]
         gr = chunk_backward(variant, q, k, v, g if has_g else None, beta, d_o, h0 if has_h0 else None, d_hT,
-                            scale=scale, chunk_size=chunk_size, use_qk_l2norm=l2norm, saved=saved)
+                            scale=scale, chunk_size=chunk_size, use_qk_l2norm=l2norm, saved=saved, _want_dh0=want_dh0)
         dg = gr["dg"].to(g.dtype) if has_g else None
         return (None, gr["dq"], gr["dk"], gr["dv"], dg, gr["dbeta"].reshape(beta.shape).to(beta.dtype),
-                gr["dh0"].to(h0.dtype) if has_h0 else None, None, None, None, None, None)
+                gr["dh0"].to(h0.dtype) if want_dh0 else None, None, None, None, None, None)
 
 
 def _wants_grad(*ts):

@@ -175,3 +175,26 @@ def test_forward_of_grad_inputs_runs_for_shapes_the_backward_does_not_cover():
     assert torch.equal(o, o2) and torch.equal(hT, hT2)
     with pytest.raises(NotImplementedError, match="chunk_size <= 64"):
         o.sum().backward()
+
+
+@pytest.mark.parametrize("variant", ["delta", "gated", "kda"])
+@pytest.mark.parametrize("T", [17, 64, 65, 150, 320])
+def test_gradients_without_the_initial_states(variant, T):
+    """A training step without an initial state does not ask for its gradient: every other gradient stays the same, bit for bit."""
+    inp = O.make_inputs(variant, 1, 3, T, 128, 128, seed=T, io_dtype=torch.bfloat16)
+    cu = {k: None if t is None else t.cuda() for k, t in inp.items()}
+    args = (variant, cu["q"], cu["k"], cu["v"], cu["g"], cu["beta"])
+    d_o = torch.randn(1, 3, T, 128, generator=torch.Generator().manual_seed(T)).cuda()
+    d_hT = torch.randn(1, 3, 128, 128, generator=torch.Generator().manual_seed(T + 1)).cuda()
+    for last in (None, d_hT):
+        whole = ops.chunk_backward(*args, d_o, None, last, saved=ops.chunk_forward_saving(*args)[2])
+        part = ops.chunk_backward(*args, d_o, None, last, saved=ops.chunk_forward_saving(*args)[2], _want_dh0=False)
+        assert part.pop("dh0") is None and whole.pop("dh0") is not None
+        for name, x in whole.items():
+            assert x is part[name] is None or torch.equal(x, part[name]), name
+    leaves = [None if t is None else t.clone().requires_grad_() for t in args[1:]]
+    h0 = torch.zeros(1, 3, 128, 128, device="cuda")   # given, but no gradient wanted
+    f = {"delta": lambda: L.delta_rule_chunkwise(leaves[0], leaves[1], leaves[2], leaves[4], h0),
+         "gated": lambda: L.gated_delta_rule_chunkwise(*leaves, initial_state=h0), "kda": lambda: L.kda_chunkwise(*leaves, initial_state=h0)}[variant]
+    f()[0].sum().backward()
+    assert h0.grad is None and all(t is None or torch.isfinite(t.grad).all() for t in leaves)
