@@ -126,13 +126,15 @@ int resolve_chunk_path(const DrDesc* d) {
 //    (d = 64, 4 sequences: 41 against 22 us at T = 64, 23 against 22 at 32; d = 128: 56 against 36, 31 against 36).  DeltaNet's
 //    recurrence, without one, stays ahead up to half of the second chunk at K = V = 128 (32 sequences, T = 65: 33 against 43 us;
 //    T = 96 level).
-//  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.6 us per chunk, KDA's state
-//    pass 2.1); slices of the value axis with 0.75 us per chunk win while sequences x 8 slices fit one wave (kTransUnits) and there
-//    are chunks enough to pay for the longer first pass (scalar decay: 30.8 against 30.3 us at 18 sequences x 7 chunks, 22.4
-//    against 30 at 4 or 8; 118 against 90 at 16 x 32, 228 against 80 at 4 x 64; at 32 sequences the one-CTA kernels are ahead).
-//    KDA switches from 17 chunks on; the two-kernel form it has up to there is behind from 10 chunks on for 18 sequences (50 against
-//    41 us at 16 chunks) and from 3 on for 4 (44 against 29).  Past 32 chunks the two-kernel form overtakes earlier (both first
-//    passes fill the chip then; 16 x 128 chunks: 340 against 357 us, 8 x 128: 292 against 267).
+//  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.5 us per chunk, KDA's state
+//    pass 2.1); slices of the value axis, 0.95 us per chunk past six sequences and 0.75 below, win while sequences x 8 slices fit one
+//    wave (kTransUnits) and there are chunks enough to pay for the longer first pass.  Us, this form against the other, sequences x
+//    chunks, scalar decay: 8 x 6 22.8 / 25.4, 18 x 6 29.6 / 25.7, 18 x 8 31.4 / 32.6, 18 x 16 38.9 / 60.1, 16 x 32 74.7 / 115, 4 x 64
+//    82 / 223, 18 x 128 276 / 443; KDA, from 17 chunks on: 18 x 17 51.4 / 53.6, 4 x 32 46.8 / 63.3, 12 x 128 228 / 288.
+//    The lines lie where they were drawn for a slower state pass; the crossings now: for scalar decay from 10 sequences on at eight
+//    chunks, and from 20 to 26 sequences this form is ahead from about 12 chunks on (20 x 32: 97 / 115, 24 x 32: 106 / 115, 28 x 32:
+//    118 / 115); KDA at 3 chunks for 4 sequences (18.1 / 18.9) and 8 for 18, and past 32 chunks up to 18 sequences as well (14 x 40:
+//    82 / 99, 18 x 128: 277 / 326), while 6 x 128 is level (252 / 246).
 // Both up to 1 GB of scratch.
 constexpr int kTransUnits = 148 / 8;
 // Whether the token recurrence beats the transition form from two chunks on, in microseconds measured for 4 to 512 sequences and 65 to

@@ -20,8 +20,9 @@
 // The one-CTA-per-sequence-slice adjoint it replaces here walked all of a chunk's work in sequence (B=2, T=4096, H=16:
 // 1.26 ms; with per-channel decay 12 ms on the CUDA cores) and stored four fp32 copies of dq^, dk^.
 //
-// Products are mma.sync tf32 with fp32 operands.  DeltaNet / Gated DeltaNet: one product (operands cut to tf32, as the
-// adjoint they replace).  KDA: three products per pair (x = hi + lo; see dr_tf32.cuh), i.e. float32 precision, as the
+// Products are mma.sync tf32 with fp32 operands, but for chain_kernel's (tcgen05, two bf16 terms per operand, 16 bits).  DeltaNet / Gated
+// DeltaNet: one product (operands cut to tf32, as the adjoint they replace).  KDA: three products per pair (x = hi + lo; see
+// dr_tf32.cuh), i.e. float32 precision, as the
 // CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
 // referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
 // decay range exceeds 2^64 is summed exactly.
@@ -573,7 +574,13 @@ static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Param
 //
 // What bounds it: B=2, T=4096, H=16 (64 CTAs): 105 us, 158 as mma.sync tf32 products over 128 CTAs (every warp read all of dS: shared
 // memory 62 %); gradient of the initial state against float64 3.2e-4 -> 2.4e-4.  The products of a chunk take 1.2 K cycles, its 100 KB of
-// operands 1.8 K at 55 bytes a clock.  Asking for the operands five chunks ahead in L2: 12 us slower.
+// operands 1.8 K at 55 bytes a clock.  Asking for the operands five chunks ahead in L2: 12 us slower.  Counters (16 sequences, 64
+// chunks): 2.75 K cycles and 1.95 K warp instructions per chunk, tensor pipe 37 %, issue slots 18 %.
+//
+// Taken at every size.  The backward's kernels against those with the mma.sync pass, 16 sequences of one, two and three chunks: 35.2 ->
+// 37.2 us, 37.5 -> 38.6, 39.4 -> 40.0, initial state's gradient included (asking for the tensor map earlier or leaving out N dS
+// while dS is zero does not change that).  Forward and backward together, 1 to 256 sequences: 1 to 9 % faster at five chunks, 4 to
+// 13 % at 16, 6 to 14 % at 64; from 48 sequences on ahead or level at every length.
 // =====================================================================================================================
 constexpr int kChThreads = 288, kChCols = 64;   // eight worker warps and one that issues
 // N hi twice, N lo, Y^T and d_o twice, the terms of dS, staging of its rows

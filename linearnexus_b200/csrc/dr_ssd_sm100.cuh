@@ -1,4 +1,5 @@
-// Mamba-2 SSD scan in chunk form on tcgen05, bf16 storage, float32-exact products.  Formulas: header of dr_ssd_chunk.cuh,
+// Mamba-2 SSD scan in chunk form on tcgen05, bf16 storage, float32 operands of the products as three bf16 terms (24 bits), decay
+// factors to float32 precision (measured in the tests: test_ssd_decay_weights_inside_a_chunk).  Formulas: header of dr_ssd_chunk.cuh,
 // with chunks of 128 tokens; per chunk, with S^T [N][P] the state at its start,
 //     G  = C B^T                                      128 x 128 x N   both from shared memory
 //     P  = tril(G e^{G_i - G_j} dt_j), three bf16 terms over G in tensor memory (the third beside it)
@@ -8,7 +9,8 @@
 //     y  = e^{G_i} Y1 + Y2 + D x;  S^T <- e^{G_L} S^T + D
 // The state stays in the registers of the group that owns it (thread = state column n, 64 values) and only its terms go through
 // shared memory, so no product waits for another chunk's product: the chain is one multiply-add per entry and the split, and the
-// step follows the sum of the tensor work (4.5 K cycles) or the longest group, whichever is longer.
+// step follows the sum of the tensor work (N = 128: 48 products of N = 64 at 49 cycles or 33 and 24 of N = 128 at 65, 3.1 K cycles), the
+// waits between them, or the longest group, whichever is longer.
 //
 // 20 warps, one CTA per (batch, head, 64 value columns):
 //   0-7    G -> P; warp = rows of a quarter (warp & 3) and half of the columns (warp >> 2)
@@ -20,11 +22,12 @@
 // B, C, the terms of S and of xs have one tile each, x three (it is read again for the outputs, whose rows are staged over it),
 // the scalars three stages.  A product that accumulates onto one of another shape waits for it: only products of equal shape are ordered.
 //
-// What bounds it: B=8, T=4096, H=16, N=128: 133 us, 318 in the mma.sync form (tensor pipe 41 % of 1024 multiply-adds per clock and SM;
-// tcgen05 takes 4096).  A chunk takes 7.5 K cycles: tensor pipe 59 %, issue slots 52 %, and the warps' first stall after their
-// hand-overs is the instruction fetch, so the loops are kept rolled (150 KB of code: 215 us, 100 KB: 162, 72 KB: 140).  Twenty-four
-// warps with the outputs on their own (setmaxnreg for the state's group): 137; xs by the warps with the least of P: 136; the issue loops
-// unrolled by four: 142.  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
+// What bounds it: B=8, T=4096, H=16, N=128: 133 to 137 us on different boxes, 318 in the mma.sync form (tensor pipe 41 % of 1024
+// multiply-adds per clock and SM; tcgen05 takes 4096).  A chunk takes 7.1 K cycles: tensor pipe 40 %, issue slots 53 %, 15.0 K warp
+// instructions; per instruction issued a warp waits 4.0 cycles on hand-overs and tensor memory and 0.8 on the instruction fetch, so
+// the loops are kept rolled (75 KB of code; 150 KB: 215 us, 100 KB: 162).  Twenty-four warps with the outputs on their own
+// (setmaxnreg for the state's group): 137, 133 without; xs by the warps with the least of P: 136; the issue loops unrolled by four:
+// 142.  Segments over a cluster for few sequences, decay sums in 64 bits and their cut-off: as there.
 //
 // Infinities and NaN in x: P is 0 above the diagonal, but 0 x inf is NaN, and a whole chunk is one product.  Such an entry is
 // taken out of the tile of Y2 (it stays in xs, so the state gets it) and the outputs of its column from its token on become NaN.
@@ -605,6 +608,8 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
 }
 
 // Rows of 64 columns of 128 tokens of a [B][T][heads][cols] array (any strides), 128-byte swizzle; tokens past T arrive as zeros.
+// Encoded anew for each call, 0.05 us each on the host (measured), less than looking one up by its strides would save.  What
+// ssd::eligible takes can be encoded: base and strides are multiples of 16 bytes, and the strides of an array in memory stay below 2^40.
 inline bool make_map(CUtensorMap* m, const LrVec& v, int cols, int B, int heads, int T) {
   sm100::EncodeTiledFn encode = sm100::encode_tiled_fn();
   if (!encode) return false;

@@ -194,10 +194,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn_major, 
 
 // ---- MMA issue (one thread) -------------------------------------------------------------------
 // One lane of a whole warp.  The products of a kernel are issued under this predicate and not under a comparison of the thread
-// index: a branch taken by elect.sync is known to hold one thread, so the descriptors go to uniform registers directly, where
-// a compare costs a loop over the active lanes around every instruction.  Measured (one issuing thread per SM, M = 128):
-// A from tensor memory, N = 32 / 64: 17 / 33 cycles per instruction under elect.sync, 46 under a compare in a tight loop and
-// 70 to 126 in less regular code; A from shared memory, N = 64: 49 either way in the tight loop (bound by shared memory).
+// index.  Measured (one issuing thread per SM, M = 128): A from tensor memory, N = 32 / 64: 17 / 33 cycles per instruction under
+// elect.sync, 46 under a compare in a tight loop and 70 to 126 in less regular code; A from shared memory, N = 64: 49 either way
+// in the tight loop (bound by shared memory).
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one)::"memory");
