@@ -11,19 +11,18 @@
 //                 stores dS1 of every chunk.  N and Y as two bf16 terms.
 //   state_kernel  (per-channel decays) the same on mma.sync, one CTA per (sequence, 32 value columns); dS stays in accumulator
 //                 registers, its copy in shared memory is the B operand.
-//   local_kernel  one CTA per chunk, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1
-//                 and the chunk's inputs, looping over four value slices with the sums over v in registers; then the
+//   the local pass, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1 and the chunk's inputs; then the
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
 //                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
-//                 finalize kernel).
+//                 finalize kernel).  Scalar decays: local_sm100_kernel (dr_bwd_local_sm100.cuh), persistent, on tcgen05.  Per-channel
+//                 decays: local_kernel, one CTA per chunk, looping over four value slices with the sums over v in registers.
 //
 // The one-CTA-per-sequence-slice adjoint it replaces here walked all of a chunk's work in sequence (B=2, T=4096, H=16:
 // 1.26 ms; with per-channel decay 12 ms on the CUDA cores) and stored four fp32 copies of dq^, dk^.
 //
-// Products are mma.sync tf32 with fp32 operands, but for chain_kernel's (tcgen05, two bf16 terms per operand, 16 bits).  DeltaNet / Gated
-// DeltaNet: one product (operands cut to tf32, as the adjoint they replace).  KDA: three products per pair (x = hi + lo; see
-// dr_tf32.cuh), i.e. float32 precision, as the
-// CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
+// DeltaNet / Gated DeltaNet: products on tcgen05 with two bf16 terms per float32 operand (16 bits); in pre_kernel mma.sync bf16 for the exact
+// ones of X and A and one tf32 product for W, Y and N.  KDA: mma.sync, three tf32 products per pair (x = hi + lo; see dr_tf32.cuh), i.e.
+// float32 precision, as the CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
 // referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
 // decay range exceeds 2^64 is summed exactly.
 #pragma once
@@ -46,9 +45,10 @@ struct Params {
   const float* ckpt;    // [units][N][128][128] state at the start of every chunk
   float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]; scalar decays: kNTile bytes per chunk
   float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]; scalar decays: kYTile
-  float* xat;           // [units][N][3][64][64] X, A, T
+  float* xat;           // [units][N][3][64][64] X, A, T; scalar decays: A and T as two bf16 terms, the tiles of local_sm100_kernel
   float* ds;            // [units][N][128][128] dS1
   float* el;            // [units][N][128] e^{G_L}
+  float* norms;         // scalar decays: [units][N][2][64] norm factors of k and q
   float* part;          // grouped heads: dq^ [units][N*64][128], then dk^ (over nf)
   SeqMap map;
   int N, variant, g_dt, l2norm;
@@ -78,6 +78,11 @@ __device__ __forceinline__ void store_terms(uint8_t* dst, int next, int lo, cons
   }
 }
 
+// two floats as two packed bf16 terms
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = mma::pack(x, y);
+  lo = mma::pack(x - mma::lo_f(hi), y - mma::hi_f(hi));
+}
 // four channels of the log decay in log2 units
 __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   float4 x;
@@ -295,13 +300,35 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   for (int i = tid; i < 64 * 16; i += kPreThreads) {
     const int r = i >> 4, c4 = (i & 15) * 4;
     if ((c4 >> 4) <= (r >> 4)) {
-      *reinterpret_cast<float4*>(xat + r * 64 + c4) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
-      *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
+      // (scalar decays: columns in fours, so that a warp of the reader takes 32 rows of four at once)
+      *reinterpret_cast<float4*>(xat + (KDA ? r * 64 + c4 : c4 * 64 + 4 * r)) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      if constexpr (KDA) *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
     }
+  }
+  // scalar decays: A, T as core matrices of 8 x 8, the blocks of eight rows next to each other; high terms, then low ones
+  auto put_tile = [&](const float* src, int ld, float* dst) {
+#pragma unroll
+    for (int x = 0; x < 512 / kPreThreads; ++x) {
+      const int i = tid + kPreThreads * x, r = 8 * ((i >> 3) & 7) + (i & 7), c = 8 * (i >> 6);
+      if ((c >> 4) > (r >> 4)) continue;
+      uint32_t h[4], l[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 y = ld2(src + r * ld + c + 2 * e);
+        split2(c + 2 * e <= r ? y.x : 0.f, c + 2 * e + 1 <= r ? y.y : 0.f, h[e], l[e]);
+      }
+      reinterpret_cast<uint4*>(dst)[i] = make_uint4(h[0], h[1], h[2], h[3]);
+      reinterpret_cast<uint4*>(dst)[512 + i] = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+  };
+  if constexpr (!KDA) {
+    put_tile(sA, 72, xat + 4096);
+    if (tid < 128) p.norms[chunk * 128 + tid] = (tid < 64 ? sRk : sRq - 64)[tid];
   }
   __syncthreads();
   sm100::block_inverse_64(sX, sBeta, sX, tid);   // ends with a barrier
-  for (int i = tid; i < 64 * 16; i += kPreThreads) {
+  if constexpr (!KDA) put_tile(sX, LDT, xat + 8192);
+  for (int i = tid; KDA && i < 64 * 16; i += kPreThreads) {
     const int r = i >> 4, c4 = (i & 15) * 4;
     if ((c4 >> 4) <= (r >> 4)) {
       float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
@@ -769,29 +796,24 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
 constexpr int kLoThreads = 512;
 constexpr int LDV = 40;    // row stride of the value-slice arrays
 constexpr int LDA = 72;    // of A, dA, dX
-// phase 1 (bytes): k^ (KDA: k^ e^G and k^ e^{G_L - G}), A, T, then V, dO, Vn, dR [64][40] and two buffers of S0, dS [128][40]
-template <bool KDA>
+// phase 1 (bytes): k^ e^G and k^ e^{G_L - G}, A, T, then V, dO, Vn, dR [64][40] and two buffers of S0, dS [128][40]
 struct LoSmem {
   static constexpr int kK = 0, kKd = kK + 64 * 132 * 4;
-  static constexpr int kA = kKd + (KDA ? 64 * 132 * 4 : 0), kT = kA + 64 * LDA * 4;
+  static constexpr int kA = kKd + 64 * 132 * 4, kT = kA + 64 * LDA * 4;
   static constexpr int kV = kT + 64 * LDT * 4, kSl = 64 * LDV * 4;   // V, dO, Vn, dR
   static constexpr int kSD = kV + 4 * kSl, kS1 = 128 * LDV * 4;        // [2][S0, dS]
   static constexpr int kSc = kSD + 4 * kS1;
   static constexpr int kTotal = kSc + (3 * 64 + 5 * 64 + 128 + 528) * 4;
-  // final phase: DeltaNet / Gated: dX over V .. , q^ over the S0, dS buffers; KDA: its own map from 0
-  static constexpr int fX = kV, fQ = kSD;
+  // final phase: a map of its own from 0
   static constexpr int gQS = 0, gKS = 64 * 132 * 4, gKE = 2 * gKS, gG = 3 * gKS, gA = 4 * gKS, gX = gA + 64 * LDA * 4, gD = gX + 64 * LDA * 4;
   static constexpr int gSeg = gD + 4 * 128 * 4;   // [16][128] scan scratch
-  static constexpr int kDot = KDA ? gSeg + 16 * 128 * 4 : kV + 64 * 136 * 4;   // final phase: q^ . dq^, k^ . dk^ per row, [2][4][64]
-  static constexpr int gRaw = kDot + 2048;   // KDA: raw q and k rows, bf16 [2][64][136]
-  static_assert(64 * LDA * 4 <= 4 * kSl && 64 * 136 * 4 <= 4 * kS1 && kTotal <= 232448 &&
-                (KDA ? gRaw + 2 * 64 * LDH * 2 <= kSc : kDot + 2048 <= kSD && 2 * 64 * 136 * 2 <= 64 * 136 * 4), "shared memory");
+  static constexpr int kDot = gSeg + 16 * 128 * 4;   // final phase: q^ . dq^, k^ . dk^ per row, [2][4][64]
+  static constexpr int gRaw = kDot + 2048;   // raw q and k rows, bf16 [2][64][136]
+  static_assert(kTotal <= 232448 && gRaw + 2 * 64 * LDH * 2 <= kSc, "shared memory");
 };
 
-template <bool KDA>
-__global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
-  using L = LoSmem<KDA>;
-  constexpr bool X3 = KDA;
+static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
+  using L = LoSmem;
   pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
   auto F = [&](int off) { return reinterpret_cast<float*>(smem + off); };
@@ -802,8 +824,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   // sums over a row's columns: one slot per quarter of the columns (sdB: and one for dR . V), added up by one thread at the
   // end -- no atomics, so that equal inputs give equal bits
   float *sdB = sBeta + 192, *sTS = sBeta + 512, *sU = sBeta + 640;   // dbeta [5][64]; <dS1, S0> per channel
-  float *sEG = sU, *sWd = sU + 64, *sGs = sU + 128, *sdG = sU + 192, *sXt = sU + 448;   // DeltaNet / Gated; dG [4][64], sums for dG_L [16]
-  float *sEx = sU, *sUn = sU + 512;                                                       // KDA: sums for dG_L [4][128], block flags
+  float *sEx = sU, *sUn = sU + 512;   // sums for dG_L [4][128], block flags
   float *sDq = F(L::kDot), *sDk = sDq + 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
@@ -853,7 +874,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < rows) {
         kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
-        if constexpr (KDA) gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
+        gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
       }
     }
     if (tid < 64) {
@@ -861,25 +882,11 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     }
     for (int i = tid; i < 320; i += kLoThreads) sdB[i] = 0.f;
     if (tid < 128) sTS[tid] = 0.f;
-    if (!KDA && warp == 15) {
-      float lo = 0.f, hi = 0.f;
-      if (p.variant == DR_GATED) {
-        if (lane < rows) lo = ld_elem(p.g, s_base + (t0 + lane) * s_tok, p.g_dt);
-        if (lane + 32 < rows) hi = ld_elem(p.g, s_base + (t0 + lane + 32) * s_tok, p.g_dt);
-      }
-      mma::scan_scalars(lo, hi, lane);
-      const float gl = __shfl_sync(0xffffffffu, hi, 31);
-      sGs[lane] = lo; sGs[lane + 32] = hi;
-      sEG[lane] = expf(lo); sEG[lane + 32] = expf(hi);
-      sWd[lane] = expf(fminf(gl - lo, 0.f)); sWd[lane + 32] = expf(fminf(gl - hi, 0.f));
-    }
-    float* sG = F(L::kSD + 2 * L::kS1);   // KDA: the second slice buffer, not yet in use (behind it: scan scratch)
-    if constexpr (KDA) {
+    float* sG = F(L::kSD + 2 * L::kS1);   // the second slice buffer, not yet in use (behind it: scan scratch)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
-      __syncthreads();
-      mma::scan_channels<kLoThreads, kD>(sG, sVn, tid);   // scratch 8 KB
-    }
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
+    __syncthreads();
+    mma::scan_channels<kLoThreads, kD>(sG, sVn, tid);   // scratch 8 KB
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int c = warp + 16 * i;
@@ -887,15 +894,11 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       const float nrm = p.l2norm ? sqrtf(warp_sum(k0 * k0 + k1 * k1 + k2 * k2 + k3 * k3)) : 0.f;
       const float m = p.l2norm ? 1.f / (nrm + 1e-6f) : 1.f;
       if (lane == 0) sRk[c] = m;
-      if constexpr (KDA) {
-        const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane), gl = *reinterpret_cast<const float4*>(sG + 63 * 132 + 4 * lane);
-        *reinterpret_cast<float4*>(sK + c * 132 + 4 * lane) =
-            make_float4(k0 * m * ex2(gg.x), k1 * m * ex2(gg.y), k2 * m * ex2(gg.z), k3 * m * ex2(gg.w));
-        *reinterpret_cast<float4*>(sKd + c * 132 + 4 * lane) =
-            make_float4(k0 * m * ex2(gl.x - gg.x), k1 * m * ex2(gl.y - gg.y), k2 * m * ex2(gl.z - gg.z), k3 * m * ex2(gl.w - gg.w));
-      } else {
-        *reinterpret_cast<float4*>(sK + c * 132 + 4 * lane) = make_float4(k0 * m, k1 * m, k2 * m, k3 * m);
-      }
+      const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane), gl = *reinterpret_cast<const float4*>(sG + 63 * 132 + 4 * lane);
+      *reinterpret_cast<float4*>(sK + c * 132 + 4 * lane) =
+          make_float4(k0 * m * ex2(gg.x), k1 * m * ex2(gg.y), k2 * m * ex2(gg.z), k3 * m * ex2(gg.w));
+      *reinterpret_cast<float4*>(sKd + c * 132 + 4 * lane) =
+          make_float4(k0 * m * ex2(gl.x - gg.x), k1 * m * ex2(gl.y - gg.y), k2 * m * ex2(gl.z - gg.z), k3 * m * ex2(gl.w - gg.w));
     }
   }
   float dQ[4][4], dKr[4][4], dKc[4][4], da[2][4], dm[2][4];   // dQg, dKg (negated), dKt; dA, dR Vn^T
@@ -919,90 +922,52 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     if (s + 1 < kD / kVS) { issue_slice(s + 1); vr = load_v(s + 1); }
     // ---- R = beta V - beta (K^ e^G) S0,  dVn = A^T dO + Kd dS1 (eight columns per warp) ------------------------------------------
     const int n0 = 8 * wc;
-    if constexpr (KDA) {
-      // different left operands, each split into two terms: half of the warps take R, half dVn, sixteen columns each, so that
-      // a split serves two products (with both on every warp the splits were more than half of the instructions here)
-      const bool second = warp >= 8;
-      const int mr = 16 * ((warp & 7) >> 1), nc = 16 * (warp & 1);
-      const uint32_t left = mma::lda_at(tc::smem_u32(second ? sKd : sK), 132, mr, lane);
-      const float* right = second ? sdS : sS0;
-      float d[2][4];
-      zero4(d[0]); zero4(d[1]);
+    // different left operands, each split into two terms: half of the warps take R, half dVn, sixteen columns each, so that
+    // a split serves two products (with both on every warp the splits were more than half of the instructions here)
+    const bool second = warp >= 8;
+    const int mr = 16 * ((warp & 7) >> 1), nc = 16 * (warp & 1);
+    const uint32_t left = mma::lda_at(tc::smem_u32(second ? sKd : sK), 132, mr, lane);
+    const float* right = second ? sdS : sS0;
+    float d[2][4];
+    zero4(d[0]); zero4(d[1]);
 #pragma unroll 4
-      for (int k0 = 0; k0 < kD; k0 += 8) {
-        const int k = k0 + t;
-        AFrag<true> a;
-        mma::lda(a, left + 4u * k0);
+    for (int k0 = 0; k0 < kD; k0 += 8) {
+      const int k = k0 + t;
+      AFrag<true> a;
+      mma::lda(a, left + 4u * k0);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          BFrag<true> bs;
-          bs.set(right[k * LDV + nc + 8 * nt + g], right[(k + 4) * LDV + nc + 8 * nt + g]);
-          fma<true>(d[nt], a, bs);
-        }
-      }
-      if (second) {
-        for (int k0 = mr; k0 < kC; k0 += 8) {
-          const int k = k0 + t;
-          AFrag<true> a;
-          a.set(sA[k * LDA + mr + g], sA[k * LDA + mr + g + 8], sA[(k + 4) * LDA + mr + g], sA[(k + 4) * LDA + mr + g + 8]);
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            BFrag<false> bo;   // bf16 values: one term
-            bo.set(sdO[k * LDV + nc + 8 * nt + g], sdO[(k + 4) * LDV + nc + 8 * nt + g]);
-            mma::fma_b1(d[nt], a, bo);
-          }
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          const int c = mr + g + 8 * hr, at = c * LDV + nc + 8 * nt + 2 * t;
-          if (second) {
-            *reinterpret_cast<float2*>(sdR + at) = make_float2(d[nt][2 * hr], d[nt][2 * hr + 1]);
-          } else {
-            const float2 x = ld2(sV + at);
-            const float bt = sBeta[c];
-            *reinterpret_cast<float2*>(sVn + at) = make_float2(bt * (x.x - d[nt][2 * hr]), bt * (x.y - d[nt][2 * hr + 1]));
-          }
-        }
-    } else {
-      const uint32_t aK = mma::lda_at(tc::smem_u32(sK), 132, m0, lane);
-      float r0[4], r1[4], d0[4], d1[4];
-      zero4(r0); zero4(r1); zero4(d0); zero4(d1);
-#pragma unroll 4
-      for (int k0 = 0; k0 < kD; k0 += 16) {
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int k = k0 + 8 * hf + t;
-          AFrag<X3> a;
-          mma::lda(a, aK + 4u * (k0 + 8 * hf));
-          BFrag<X3> bs, bd;
-          bs.set(sS0[k * LDV + n0 + g], sS0[(k + 4) * LDV + n0 + g]);
-          bd.set(sdS[k * LDV + n0 + g], sdS[(k + 4) * LDV + n0 + g]);
-          fma<X3>(hf ? r1 : r0, a, bs);
-          fma<X3>(hf ? d1 : d0, a, bd);
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { r0[e] += r1[e]; d0[e] += d1[e]; d0[e] *= sWd[m0 + g + 8 * (e >> 1)]; }
-      for (int k0 = m0; k0 < kC; k0 += 8) {
-        const int k = k0 + t;
-        AFrag<X3> a;
-        a.set(sA[k * LDA + m0 + g], sA[k * LDA + m0 + g + 8], sA[(k + 4) * LDA + m0 + g], sA[(k + 4) * LDA + m0 + g + 8]);
-        BFrag<X3> bo;
-        bo.set(sdO[k * LDV + n0 + g], sdO[(k + 4) * LDV + n0 + g]);
-        fma<X3>(d0, a, bo);
-      }
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int c = m0 + g + 8 * hr, vv = n0 + 2 * t;
-        const float2 x = ld2(sV + c * LDV + vv);
-        const float bt = sBeta[c], eg = sEG[c];
-        *reinterpret_cast<float2*>(sVn + c * LDV + vv) = make_float2(bt * (x.x - eg * r0[2 * hr]), bt * (x.y - eg * r0[2 * hr + 1]));
-        *reinterpret_cast<float2*>(sdR + c * LDV + vv) = make_float2(d0[2 * hr], d0[2 * hr + 1]);
+      for (int nt = 0; nt < 2; ++nt) {
+        BFrag<true> bs;
+        bs.set(right[k * LDV + nc + 8 * nt + g], right[(k + 4) * LDV + nc + 8 * nt + g]);
+        fma<true>(d[nt], a, bs);
       }
     }
+    if (second) {
+      for (int k0 = mr; k0 < kC; k0 += 8) {
+        const int k = k0 + t;
+        AFrag<true> a;
+        a.set(sA[k * LDA + mr + g], sA[k * LDA + mr + g + 8], sA[(k + 4) * LDA + mr + g], sA[(k + 4) * LDA + mr + g + 8]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          BFrag<false> bo;   // bf16 values: one term
+          bo.set(sdO[k * LDV + nc + 8 * nt + g], sdO[(k + 4) * LDV + nc + 8 * nt + g]);
+          mma::fma_b1(d[nt], a, bo);
+        }
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int c = mr + g + 8 * hr, at = c * LDV + nc + 8 * nt + 2 * t;
+        if (second) {
+          *reinterpret_cast<float2*>(sdR + at) = make_float2(d[nt][2 * hr], d[nt][2 * hr + 1]);
+        } else {
+          const float2 x = ld2(sV + at);
+          const float bt = sBeta[c];
+          *reinterpret_cast<float2*>(sVn + at) = make_float2(bt * (x.x - d[nt][2 * hr]), bt * (x.y - d[nt][2 * hr + 1]));
+        }
+      }
     __syncthreads();
     // ---- Vn = T R, dR = T^T dVn ------------------------------------------------------------------------------------------------------
     {
@@ -1011,19 +976,19 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       zero4(vn); zero4(dr);
       for (int k0 = 0; k0 < m0 + 16; k0 += 8) {
         const int k = k0 + t;
-        AFrag<X3> a;
+        AFrag<true> a;
         mma::lda(a, aT + 4u * k0);
-        BFrag<X3> br;
+        BFrag<true> br;
         br.set(sVn[k * LDV + n0 + g], sVn[(k + 4) * LDV + n0 + g]);
-        fma<X3>(vn, a, br);
+        fma<true>(vn, a, br);
       }
       for (int k0 = m0; k0 < kC; k0 += 8) {
         const int k = k0 + t;
-        AFrag<X3> a;
+        AFrag<true> a;
         a.set(sT[k * LDT + m0 + g], sT[k * LDT + m0 + g + 8], sT[(k + 4) * LDT + m0 + g], sT[(k + 4) * LDT + m0 + g + 8]);
-        BFrag<X3> bd;
+        BFrag<true> bd;
         bd.set(sdR[k * LDV + n0 + g], sdR[(k + 4) * LDV + n0 + g]);
-        fma<X3>(dr, a, bd);
+        fma<true>(dr, a, bd);
       }
       __syncthreads();
 #pragma unroll
@@ -1068,7 +1033,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     for (int k0 = 0; k0 < kVS; k0 += 8) {
       const int k = k0 + 2 * t;
       AFrag<false> ao;   // bf16 values: one term in either precision
-      AFrag<X3> ar, an;
+      AFrag<true> ar, an;
       {
         const float2 x0 = ld2(sdO + (m0 + g) * LDV + k), x1 = ld2(sdO + (m0 + g + 8) * LDV + k);
         ao.set(x0.x, x1.x, x0.y, x1.y);
@@ -1081,22 +1046,22 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float2 y = ld2(sVn + (16 * wc + 8 * nt + g) * LDV + k);
-          BFrag<X3> bv;
+          BFrag<true> bv;
           bv.set(y.x, y.y);
           mma::fma_a1(da[nt], ao, bv);
-          fma<X3>(dm[nt], ar, bv);
+          fma<true>(dm[nt], ar, bv);
         }
       }
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const int ch = 32 * wc + 8 * nt + g;
         const float2 y = ld2(sS0 + ch * LDV + k), z = ld2(sdS + ch * LDV + k);
-        BFrag<X3> bs, bd;
+        BFrag<true> bs, bd;
         bs.set(y.x, y.y);
         bd.set(z.x, z.y);
         mma::fma_a1(dQ[nt], ao, bs);
-        fma<X3>(dKr[nt], ar, bs);
-        fma<X3>(dKc[nt], an, bd);
+        fma<true>(dKr[nt], ar, bs);
+        fma<true>(dKc[nt], an, bd);
       }
     }
   }
@@ -1104,21 +1069,18 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   uint2 qr[4], kr[4];
   float4 gr[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {   // the chunk's q (KDA: and k, g) rows once more, in flight behind the next lines
+  for (int i = 0; i < 4; ++i) {   // the chunk's q, k, g rows once more, in flight behind the next lines
     const int c = warp + 16 * i;
     qr[i] = kr[i] = make_uint2(0u, 0u);
     gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < rows) {
       qr[i] = *reinterpret_cast<const uint2*>(gq + qk_base + (t0 + c) * qk_tok + 4 * lane);
-      if constexpr (KDA) {
-        kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
-        gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
-      }
+      kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
+      gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
     }
   }
   __syncthreads();   // phase 1 is over: its arrays may be written
-  float* fA = KDA ? F(L::gA) : sA;
-  float* fX = KDA ? F(L::gX) : F(L::fX);
+  float *fA = F(L::gA), *fX = F(L::gX);
   {
     float dbacc[2] = {0.f, 0.f};
 #pragma unroll
@@ -1131,7 +1093,7 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         float av[2], xv[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const float ee = (j + e <= i) ? (KDA ? 1.f : __expf(fminf(sGs[i] - sGs[j + e], 0.f))) : 0.f;
+          const float ee = (j + e <= i) ? 1.f : 0.f;
           const float dmv = -dm[nt][2 * hr + e];
           dbacc[hr] += dmv * (e ? xx.y : xx.x);   // X carries its decay factor
           av[e] = da[nt][2 * hr + e] * ee;
@@ -1148,25 +1110,22 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
       if (t == 0) sdB[64 * wc + m0 + g + 8 * hr] += x;
     }
   }
-  // ---- q^ rows (KDA: the decayed forms of q^ and k^) ---------------------------------------------------------------------------------------
-  float* sQ = F(L::fQ);   // DeltaNet / Gated: [64][136]
-  __nv_bfloat16* sRaw = reinterpret_cast<__nv_bfloat16*>(smem + (KDA ? L::gRaw : 0));   // KDA
-  float* sDi = F(L::gSeg);   // KDA: 1 / total decay of each block (over the scan scratch)
+  // ---- the decayed forms of q^ and k^ ---------------------------------------------------------------------------------------
+  __nv_bfloat16* sRaw = reinterpret_cast<__nv_bfloat16*>(smem + L::gRaw);
+  float* sDi = F(L::gSeg);   // 1 / total decay of each block (over the scan scratch)
   float *sQS = F(L::gQS), *sKS = F(L::gKS), *sKE = F(L::gKE), *sG = F(L::gG), *sD = F(L::gD);
-  if constexpr (KDA) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
-    __syncthreads();
-    mma::scan_channels<kLoThreads, kD>(sG, F(L::gSeg), tid);
-    if (tid < 4) sUn[tid] = 0.f;
-    __syncthreads();
-    {   // total decay of each 16-row block; flag blocks whose range is too wide for the product form
-      const int blk = tid >> 7, c = tid & 127;
-      const float d = sG[(16 * blk + 15) * 132 + c] - (blk ? sG[(16 * blk - 1) * 132 + c] : 0.f);
-      sD[blk * 128 + c] = ex2(d);
-      sDi[blk * 128 + c] = 1.f / ex2(d);
-      if (!(d >= -64.f)) sUn[blk] = 1.f;
-    }
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(sG + (warp + 16 * i) * 132 + 4 * lane) = gr[i];
+  __syncthreads();
+  mma::scan_channels<kLoThreads, kD>(sG, F(L::gSeg), tid);
+  if (tid < 4) sUn[tid] = 0.f;
+  __syncthreads();
+  {   // total decay of each 16-row block; flag blocks whose range is too wide for the product form
+    const int blk = tid >> 7, c = tid & 127;
+    const float d = sG[(16 * blk + 15) * 132 + c] - (blk ? sG[(16 * blk - 1) * 132 + c] : 0.f);
+    sD[blk * 128 + c] = ex2(d);
+    sDi[blk * 128 + c] = 1.f / ex2(d);
+    if (!(d >= -64.f)) sUn[blk] = 1.f;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -1175,186 +1134,70 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
     const float nrm = p.l2norm ? sqrtf(warp_sum(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3)) : 0.f;
     const float m = p.l2norm ? p.scale / (nrm + 1e-6f) : p.scale;
     if (lane == 0) sRq[c] = m;
-    if constexpr (KDA) {
-      *reinterpret_cast<uint2*>(sRaw + c * LDH + 4 * lane) = qr[i];
-      *reinterpret_cast<uint2*>(sRaw + (64 + c) * LDH + 4 * lane) = kr[i];
-      const int blk = c >> 4;
-      const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
-      const float4 ge = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
-      float4 gn = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (blk) gn = *reinterpret_cast<const float4*>(sG + (16 * blk - 1) * 132 + 4 * lane);
-      const float mk = sRk[c];
-      const float k0 = mma::lo_f(kr[i].x) * mk, k1 = mma::hi_f(kr[i].x) * mk, k2 = mma::lo_f(kr[i].y) * mk, k3 = mma::hi_f(kr[i].y) * mk;
-      const float e0 = ex2(gg.x - gn.x), e1 = ex2(gg.y - gn.y), e2 = ex2(gg.z - gn.z), e3 = ex2(gg.w - gn.w);
-      *reinterpret_cast<float4*>(sQS + c * 132 + 4 * lane) = make_float4(q0 * m * e0, q1 * m * e1, q2 * m * e2, q3 * m * e3);
-      *reinterpret_cast<float4*>(sKS + c * 132 + 4 * lane) = make_float4(k0 * e0, k1 * e1, k2 * e2, k3 * e3);
-      *reinterpret_cast<float4*>(sKE + c * 132 + 4 * lane) =
-          make_float4(k0 * ex2(ge.x - gg.x), k1 * ex2(ge.y - gg.y), k2 * ex2(ge.z - gg.z), k3 * ex2(ge.w - gg.w));
-    } else {
-      *reinterpret_cast<float4*>(sQ + c * 136 + 4 * lane) = make_float4(q0 * m, q1 * m, q2 * m, q3 * m);
-    }
+    *reinterpret_cast<uint2*>(sRaw + c * LDH + 4 * lane) = qr[i];
+    *reinterpret_cast<uint2*>(sRaw + (64 + c) * LDH + 4 * lane) = kr[i];
+    const int blk = c >> 4;
+    const float4 gg = *reinterpret_cast<const float4*>(sG + c * 132 + 4 * lane);
+    const float4 ge = *reinterpret_cast<const float4*>(sG + (16 * blk + 15) * 132 + 4 * lane);
+    float4 gn = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (blk) gn = *reinterpret_cast<const float4*>(sG + (16 * blk - 1) * 132 + 4 * lane);
+    const float mk = sRk[c];
+    const float k0 = mma::lo_f(kr[i].x) * mk, k1 = mma::hi_f(kr[i].x) * mk, k2 = mma::lo_f(kr[i].y) * mk, k3 = mma::hi_f(kr[i].y) * mk;
+    const float e0 = ex2(gg.x - gn.x), e1 = ex2(gg.y - gn.y), e2 = ex2(gg.z - gn.z), e3 = ex2(gg.w - gn.w);
+    *reinterpret_cast<float4*>(sQS + c * 132 + 4 * lane) = make_float4(q0 * m * e0, q1 * m * e1, q2 * m * e2, q3 * m * e3);
+    *reinterpret_cast<float4*>(sKS + c * 132 + 4 * lane) = make_float4(k0 * e0, k1 * e1, k2 * e2, k3 * e3);
+    *reinterpret_cast<float4*>(sKE + c * 132 + 4 * lane) =
+        make_float4(k0 * ex2(ge.x - gg.x), k1 * ex2(ge.y - gg.y), k2 * ex2(ge.z - gg.z), k3 * ex2(ge.w - gg.w));
   }
   __syncthreads();
   // ---- dQ^ = dQg e^G + (dA.E) K^ ; dK^ rows and columns (four channel tiles per warp: 32 wc ..) -------------------------------------------------
-  float dbrow[2] = {0.f, 0.f}, extra = 0.f;
-  float Dg[KDA ? 4 : 1][4];   // KDA: dG of this lane's entries
-  if constexpr (KDA) {
-    const int bi = warp >> 2;
-    const bool exact = sUn[bi] != 0.f;
-    // dbeta: -dKg . k^ e^G; dG_L: dKt . k^ e^{G_L - G}
+  float dbrow[2] = {0.f, 0.f};
+  float Dg[4][4];   // dG of this lane's entries
+  const int bi = warp >> 2;
+  const bool exact = sUn[bi] != 0.f;
+  // dbeta: -dKg . k^ e^G; dG_L: dKt . k^ e^{G_L - G}
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = 32 * wc + 8 * nt + 2 * t;
-      float2 en = make_float2(1.f, 1.f);   // decay before the block, and from its end to the chunk's
-      if (bi) { const float2 x = ld2(sG + (16 * bi - 1) * 132 + c); en = make_float2(ex2(x.x), ex2(x.y)); }
-      const float2 gl = ld2(sG + 63 * 132 + c), ge = ld2(sG + (16 * bi + 15) * 132 + c);
-      const float2 ee = make_float2(ex2(gl.x - ge.x), ex2(gl.y - ge.y));
-      float ex0 = 0.f, ex1 = 0.f;
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int i = m0 + g + 8 * hr;
-        const float2 ks = ld2(sKS + i * 132 + c), ke = ld2(sKE + i * 132 + c);
-        dbrow[hr] -= dKr[nt][2 * hr] * ks.x * en.x + dKr[nt][2 * hr + 1] * ks.y * en.y;
-        ex0 += dKc[nt][2 * hr] * ke.x * ee.x;
-        ex1 += dKc[nt][2 * hr + 1] * ke.y * ee.y;
-        dKr[nt][2 * hr] *= -sBeta[i];
-        dKr[nt][2 * hr + 1] *= -sBeta[i];
-      }
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        ex0 += __shfl_xor_sync(0xffffffffu, ex0, o);
-        ex1 += __shfl_xor_sync(0xffffffffu, ex1, o);
-      }
-      if (g == 0) *reinterpret_cast<float2*>(sEx + 128 * bi + c) = make_float2(ex0, ex1);
-    }
-    auto carry = [&](float (&d)[4][4], int blk) {   // refer the sums to the end of block blk
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const float2 x = ld2(sD + blk * 128 + 32 * wc + 8 * nt + 2 * t);
-        d[nt][0] *= x.x; d[nt][1] *= x.y; d[nt][2] *= x.x; d[nt][3] *= x.y;
-      }
-    };
-    // rows: sums over the columns of earlier blocks, each block's decay carried on the way; then the diagonal block
-#pragma unroll 1
-    for (int bj = 0; bj <= bi; ++bj) {
-      const bool diag = bj == bi;
-      if (diag && exact) break;
-      if (!diag) { carry(dQ, bj); carry(dKr, bj); }
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int k = 16 * bj + 8 * hf + 2 * t;
-        AFrag<true> aa, ax;
-        const float2 x0 = ld2(fA + (m0 + g) * LDA + k), x1 = ld2(fA + (m0 + g + 8) * LDA + k);
-        aa.set(x0.x, x1.x, x0.y, x1.y);
-        const float2 y0 = ld2(fX + (m0 + g) * LDA + k), y1 = ld2(fX + (m0 + g + 8) * LDA + k);
-        ax.set(y0.x, y1.x, y0.y, y1.y);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const int c = 32 * wc + 8 * nt + g;
-          float b0 = sKE[k * 132 + c], b1 = sKE[(k + 1) * 132 + c];
-          if (diag) { const float iv = sDi[bi * 128 + c]; b0 *= iv; b1 *= iv; }
-          BFrag<true> bk;
-          bk.set(b0, b1);
-          fma<true>(dQ[nt], aa, bk);
-          fma<true>(dKr[nt], ax, bk);
-        }
-      }
-    }
-    // columns: the rows of later blocks, last first; then the diagonal block, referred to the block's start
-#pragma unroll 1
-    for (int bj = 3; bj >= bi; --bj) {
-      const bool diag = bj == bi;
-      if (diag && exact) break;
-      carry(dKc, bj);
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int k = 16 * bj + 8 * hf + t;
-        AFrag<true> aa, ax;
-        aa.set(fA[k * LDA + m0 + g], fA[k * LDA + m0 + g + 8], fA[(k + 4) * LDA + m0 + g], fA[(k + 4) * LDA + m0 + g + 8]);
-        ax.set(fX[k * LDA + m0 + g], fX[k * LDA + m0 + g + 8], fX[(k + 4) * LDA + m0 + g], fX[(k + 4) * LDA + m0 + g + 8]);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const int c = 32 * wc + 8 * nt + g;
-          BFrag<true> bq, bk;
-          bq.set(sQS[k * 132 + c], sQS[(k + 4) * 132 + c]);
-          bk.set(sKS[k * 132 + c], sKS[(k + 4) * 132 + c]);
-          fma<true>(dKc[nt], aa, bq);
-          fma<true>(dKc[nt], ax, bk);
-        }
-      }
-    }
-    // the factors of the entries' own rows; dG
-    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = 32 * wc + 8 * nt + 2 * t;
-      float2 gn = make_float2(0.f, 0.f);
-      if (bi) gn = ld2(sG + (16 * bi - 1) * 132 + c);
-      const float2 ge = ld2(sG + (16 * bi + 15) * 132 + c);
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int i = m0 + g + 8 * hr;
-        const float2 gi = ld2(sG + i * 132 + c);
-        const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
-        const float2 qh = make_float2(mma::lo_f(uq) * sRq[i], mma::hi_f(uq) * sRq[i]);
-        const float2 kh = make_float2(mma::lo_f(uk) * sRk[i], mma::hi_f(uk) * sRk[i]);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int x = 2 * hr + e;
-          const float Gi = e ? gi.y : gi.x, Gn = e ? gn.y : gn.x, Ge = e ? ge.y : ge.x;
-          const float fr = ex2(Gi - Gn), fc = ex2((exact ? Ge : Gn) - Gi);
-          float dq = dQ[nt][x] * fr, dkr = dKr[nt][x] * fr, dkc = dKc[nt][x] * fc;
-          if (exact) {   // the diagonal block entry by entry
-            for (int j = m0; j < m0 + 16; ++j) {
-              const float Gj = sG[j * 132 + c + e];
-              if (j >= rows) break;
-              const int64_t at = qk_base + (t0 + j) * qk_tok + c + e;
-              const float kj = bf(gk + at) * sRk[j], qj = bf(gq + at) * sRq[j];
-              if (j <= i) {
-                const float w = ex2(Gi - Gj) * kj;
-                dq += fA[i * LDA + j] * w;
-                dkr += fX[i * LDA + j] * w;
-              }
-              if (j >= i) {
-                const float w = ex2(Gj - Gi);
-                dkc += w * (fA[j * LDA + i] * qj + fX[j * LDA + i] * kj);
-              }
-            }
-          }
-          Dg[nt][x] = (e ? qh.y : qh.x) * dq + (e ? kh.y : kh.x) * (dkr - dkc);
-          dQ[nt][x] = dq;
-          dKr[nt][x] = dkr + dkc;
-        }
-        sq[hr] += qh.x * dQ[nt][2 * hr] + qh.y * dQ[nt][2 * hr + 1];
-        sk[hr] += kh.x * dKr[nt][2 * hr] + kh.y * dKr[nt][2 * hr + 1];
-      }
-    }
+  for (int nt = 0; nt < 4; ++nt) {
+    const int c = 32 * wc + 8 * nt + 2 * t;
+    float2 en = make_float2(1.f, 1.f);   // decay before the block, and from its end to the chunk's
+    if (bi) { const float2 x = ld2(sG + (16 * bi - 1) * 132 + c); en = make_float2(ex2(x.x), ex2(x.y)); }
+    const float2 gl = ld2(sG + 63 * 132 + c), ge = ld2(sG + (16 * bi + 15) * 132 + c);
+    const float2 ee = make_float2(ex2(gl.x - ge.x), ex2(gl.y - ge.y));
+    float ex0 = 0.f, ex1 = 0.f;
 #pragma unroll
     for (int hr = 0; hr < 2; ++hr) {
-#pragma unroll
-      for (int o = 1; o < 4; o <<= 1) {
-        sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
-        sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
-      }
-      if (t == 0) { sDq[64 * wc + m0 + g + 8 * hr] = sq[hr]; sDk[64 * wc + m0 + g + 8 * hr] = sk[hr]; }
+      const int i = m0 + g + 8 * hr;
+      const float2 ks = ld2(sKS + i * 132 + c), ke = ld2(sKE + i * 132 + c);
+      dbrow[hr] -= dKr[nt][2 * hr] * ks.x * en.x + dKr[nt][2 * hr + 1] * ks.y * en.y;
+      ex0 += dKc[nt][2 * hr] * ke.x * ee.x;
+      ex1 += dKc[nt][2 * hr + 1] * ke.y * ee.y;
+      dKr[nt][2 * hr] *= -sBeta[i];
+      dKr[nt][2 * hr + 1] *= -sBeta[i];
     }
-  } else {
-    const float eg[2] = {sEG[m0 + g], sEG[m0 + g + 8]}, el[2] = {sWd[m0 + g], sWd[m0 + g + 8]}, bt[2] = {sBeta[m0 + g], sBeta[m0 + g + 8]};
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int o = 4; o < 32; o <<= 1) {
+      ex0 += __shfl_xor_sync(0xffffffffu, ex0, o);
+      ex1 += __shfl_xor_sync(0xffffffffu, ex1, o);
+    }
+    if (g == 0) *reinterpret_cast<float2*>(sEx + 128 * bi + c) = make_float2(ex0, ex1);
+  }
+  auto carry = [&](float (&d)[4][4], int blk) {   // refer the sums to the end of block blk
 #pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const float2 kh = ld2(sK + (m0 + g + 8 * hr) * 132 + 32 * wc + 8 * nt + 2 * t);
-        const int e = 2 * hr;
-        dbrow[hr] -= (dKr[nt][e] * kh.x + dKr[nt][e + 1] * kh.y) * eg[hr];
-        extra += (dKc[nt][e] * kh.x + dKc[nt][e + 1] * kh.y) * el[hr];
-        dQ[nt][e] *= eg[hr]; dQ[nt][e + 1] *= eg[hr];
-        dKr[nt][e] *= -bt[hr] * eg[hr]; dKr[nt][e + 1] *= -bt[hr] * eg[hr];
-        dKc[nt][e] *= el[hr]; dKc[nt][e + 1] *= el[hr];
-      }
-    for (int k0 = 0; k0 < m0 + 16; k0 += 8) {
-      const int k = k0 + 2 * t;
-      AFrag<X3> aa, ax;
+    for (int nt = 0; nt < 4; ++nt) {
+      const float2 x = ld2(sD + blk * 128 + 32 * wc + 8 * nt + 2 * t);
+      d[nt][0] *= x.x; d[nt][1] *= x.y; d[nt][2] *= x.x; d[nt][3] *= x.y;
+    }
+  };
+  // rows: sums over the columns of earlier blocks, each block's decay carried on the way; then the diagonal block
+#pragma unroll 1
+  for (int bj = 0; bj <= bi; ++bj) {
+    const bool diag = bj == bi;
+    if (diag && exact) break;
+    if (!diag) { carry(dQ, bj); carry(dKr, bj); }
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int k = 16 * bj + 8 * hf + 2 * t;
+      AFrag<true> aa, ax;
       const float2 x0 = ld2(fA + (m0 + g) * LDA + k), x1 = ld2(fA + (m0 + g + 8) * LDA + k);
       aa.set(x0.x, x1.x, x0.y, x1.y);
       const float2 y0 = ld2(fX + (m0 + g) * LDA + k), y1 = ld2(fX + (m0 + g + 8) * LDA + k);
@@ -1362,53 +1205,92 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const int c = 32 * wc + 8 * nt + g;
-        BFrag<X3> bk;
-        bk.set(sK[k * 132 + c], sK[(k + 1) * 132 + c]);
-        fma<X3>(dQ[nt], aa, bk);
-        fma<X3>(dKr[nt], ax, bk);
+        float b0 = sKE[k * 132 + c], b1 = sKE[(k + 1) * 132 + c];
+        if (diag) { const float iv = sDi[bi * 128 + c]; b0 *= iv; b1 *= iv; }
+        BFrag<true> bk;
+        bk.set(b0, b1);
+        fma<true>(dQ[nt], aa, bk);
+        fma<true>(dKr[nt], ax, bk);
       }
     }
-    for (int k0 = m0; k0 < kC; k0 += 8) {
-      const int k = k0 + t;
-      AFrag<X3> aa, ax;
+  }
+  // columns: the rows of later blocks, last first; then the diagonal block, referred to the block's start
+#pragma unroll 1
+  for (int bj = 3; bj >= bi; --bj) {
+    const bool diag = bj == bi;
+    if (diag && exact) break;
+    carry(dKc, bj);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int k = 16 * bj + 8 * hf + t;
+      AFrag<true> aa, ax;
       aa.set(fA[k * LDA + m0 + g], fA[k * LDA + m0 + g + 8], fA[(k + 4) * LDA + m0 + g], fA[(k + 4) * LDA + m0 + g + 8]);
       ax.set(fX[k * LDA + m0 + g], fX[k * LDA + m0 + g + 8], fX[(k + 4) * LDA + m0 + g], fX[(k + 4) * LDA + m0 + g + 8]);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
         const int c = 32 * wc + 8 * nt + g;
-        BFrag<X3> bq, bk;
-        bq.set(sQ[k * 136 + c], sQ[(k + 4) * 136 + c]);
-        bk.set(sK[k * 132 + c], sK[(k + 4) * 132 + c]);
-        fma<X3>(dKc[nt], aa, bq);
-        fma<X3>(dKc[nt], ax, bk);
+        BFrag<true> bq, bk;
+        bq.set(sQS[k * 132 + c], sQS[(k + 4) * 132 + c]);
+        bk.set(sKS[k * 132 + c], sKS[(k + 4) * 132 + c]);
+        fma<true>(dKc[nt], aa, bq);
+        fma<true>(dKc[nt], ax, bk);
       }
     }
-    float dgrow[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
+  }
+  // the factors of the entries' own rows; dG
+  float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int i = m0 + g + 8 * hr, c = 32 * wc + 8 * nt + 2 * t, e = 2 * hr;
-        const float2 qh = ld2(sQ + i * 136 + c), kh = ld2(sK + i * 132 + c);
-        const float a = qh.x * dQ[nt][e] + qh.y * dQ[nt][e + 1];
-        const float kr_ = kh.x * dKr[nt][e] + kh.y * dKr[nt][e + 1], kc_ = kh.x * dKc[nt][e] + kh.y * dKc[nt][e + 1];
-        sq[hr] += a; sk[hr] += kr_ + kc_;
-        dgrow[hr] += a + kr_ - kc_;
-        dKr[nt][e] += dKc[nt][e]; dKr[nt][e + 1] += dKc[nt][e + 1];
-      }
+  for (int nt = 0; nt < 4; ++nt) {
+    const int c = 32 * wc + 8 * nt + 2 * t;
+    float2 gn = make_float2(0.f, 0.f);
+    if (bi) gn = ld2(sG + (16 * bi - 1) * 132 + c);
+    const float2 ge = ld2(sG + (16 * bi + 15) * 132 + c);
 #pragma unroll
     for (int hr = 0; hr < 2; ++hr) {
       const int i = m0 + g + 8 * hr;
+      const float2 gi = ld2(sG + i * 132 + c);
+      const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
+      const float2 qh = make_float2(mma::lo_f(uq) * sRq[i], mma::hi_f(uq) * sRq[i]);
+      const float2 kh = make_float2(mma::lo_f(uk) * sRk[i], mma::hi_f(uk) * sRk[i]);
 #pragma unroll
-      for (int o = 1; o < 4; o <<= 1) {
-        dgrow[hr] += __shfl_xor_sync(0xffffffffu, dgrow[hr], o);
-        sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
-        sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
+      for (int e = 0; e < 2; ++e) {
+        const int x = 2 * hr + e;
+        const float Gi = e ? gi.y : gi.x, Gn = e ? gn.y : gn.x, Ge = e ? ge.y : ge.x;
+        const float fr = ex2(Gi - Gn), fc = ex2((exact ? Ge : Gn) - Gi);
+        float dq = dQ[nt][x] * fr, dkr = dKr[nt][x] * fr, dkc = dKc[nt][x] * fc;
+        if (exact) {   // the diagonal block entry by entry
+          for (int j = m0; j < m0 + 16; ++j) {
+            const float Gj = sG[j * 132 + c + e];
+            if (j >= rows) break;
+            const int64_t at = qk_base + (t0 + j) * qk_tok + c + e;
+            const float kj = bf(gk + at) * sRk[j], qj = bf(gq + at) * sRq[j];
+            if (j <= i) {
+              const float w = ex2(Gi - Gj) * kj;
+              dq += fA[i * LDA + j] * w;
+              dkr += fX[i * LDA + j] * w;
+            }
+            if (j >= i) {
+              const float w = ex2(Gj - Gi);
+              dkc += w * (fA[j * LDA + i] * qj + fX[j * LDA + i] * kj);
+            }
+          }
+        }
+        Dg[nt][x] = (e ? qh.y : qh.x) * dq + (e ? kh.y : kh.x) * (dkr - dkc);
+        dQ[nt][x] = dq;
+        dKr[nt][x] = dkr + dkc;
       }
-      if (t == 0) { sdG[64 * wc + i] = dgrow[hr]; sDq[64 * wc + i] = sq[hr]; sDk[64 * wc + i] = sk[hr]; }
+      sq[hr] += qh.x * dQ[nt][2 * hr] + qh.y * dQ[nt][2 * hr + 1];
+      sk[hr] += kh.x * dKr[nt][2 * hr] + kh.y * dKr[nt][2 * hr + 1];
     }
-    extra = warp_sum(extra);
-    if (lane == 0) sXt[warp] = extra;
+  }
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      sq[hr] += __shfl_xor_sync(0xffffffffu, sq[hr], o);
+      sk[hr] += __shfl_xor_sync(0xffffffffu, sk[hr], o);
+    }
+    if (t == 0) { sDq[64 * wc + m0 + g + 8 * hr] = sq[hr]; sDk[64 * wc + m0 + g + 8 * hr] = sk[hr]; }
   }
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
@@ -1419,9 +1301,9 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   __syncthreads();
   // ---- chain rule of the normalisation: y = s x / (|x| + eps), y^ = s x r:  dx = s r dy - y^ (y^ . dy) / (s |x|) ------------------------------------
   const bool grouped = p.map.Hq != p.map.H;
-  __nv_bfloat16* oq = reinterpret_cast<__nv_bfloat16*>(KDA ? smem + L::gKS : smem + L::fX);   // staging [64][136] bf16, twice
+  __nv_bfloat16* oq = reinterpret_cast<__nv_bfloat16*>(smem + L::gKS);   // staging [64][136] bf16, twice
   __nv_bfloat16* ok = oq + 64 * 136;
-  float* sDG = F(L::gQS);   // KDA: dG [64][132]
+  float* sDG = F(L::gQS);   // dG [64][132]
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
     const int i = m0 + g + 8 * hr;
@@ -1441,17 +1323,13 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
         *reinterpret_cast<float2*>(p.part + (int64_t)gridDim.x * (kC * kD) + at) = make_float2(dKr[nt][e], dKr[nt][e + 1]);
       } else {
         float2 qh = make_float2(0.f, 0.f), kh = qh;
-        if constexpr (KDA) {
-          const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
-          qh = make_float2(mma::lo_f(uq) * mq, mma::hi_f(uq) * mq);
-          kh = make_float2(mma::lo_f(uk) * mk, mma::hi_f(uk) * mk);
-        } else {
-          qh = ld2(sQ + i * 136 + c); kh = ld2(sK + i * 132 + c);
-        }
+        const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
+        qh = make_float2(mma::lo_f(uq) * mq, mma::hi_f(uq) * mq);
+        kh = make_float2(mma::lo_f(uk) * mk, mma::hi_f(uk) * mk);
         *reinterpret_cast<uint32_t*>(oq + i * 136 + c) = mma::pack(mq * dQ[nt][e] - qh.x * fq, mq * dQ[nt][e + 1] - qh.y * fq);
         *reinterpret_cast<uint32_t*>(ok + i * 136 + c) = mma::pack(mk * dKr[nt][e] - kh.x * fk, mk * dKr[nt][e + 1] - kh.y * fk);
       }
-      if constexpr (KDA) *reinterpret_cast<float2*>(sDG + i * 132 + c) = make_float2(Dg[nt][e], Dg[nt][e + 1]);
+      *reinterpret_cast<float2*>(sDG + i * 132 + c) = make_float2(Dg[nt][e], Dg[nt][e + 1]);
     }
   }
   __syncthreads();
@@ -1466,38 +1344,30 @@ __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
   }
   if (tid < rows) p.dbeta[s_base + (t0 + tid) * s_tok] = (sdB[tid] + sdB[64 + tid]) + (sdB[128 + tid] + sdB[192 + tid]) + sdB[256 + tid];
   // ---- dg: reverse cumulative sum of dG inside the chunk ---------------------------------------------------------------------------------------
-  if constexpr (KDA) {
-    const int s = tid >> 7, c = tid & 127;   // 16-row segment, channel
-    float acc = 0.f, loc[16];
-    if (s == 3) acc = (sEx[c] + sEx[128 + c]) + (sEx[256 + c] + sEx[384 + c]) + sTS[c] * ex2(sG[63 * 132 + c]);
+  const int s = tid >> 7, c = tid & 127;   // 16-row segment, channel
+  float acc = 0.f, loc[16];
+  if (s == 3) acc = (sEx[c] + sEx[128 + c]) + (sEx[256 + c] + sEx[384 + c]) + sTS[c] * ex2(sG[63 * 132 + c]);
 #pragma unroll
-    for (int r = 15; r >= 0; --r) {
-      acc += sDG[(16 * s + r) * 132 + c];
-      loc[r] = acc;
-    }
-    sD[s * 128 + c] = acc;
-    __syncthreads();
-    float post = 0.f;
-    for (int s2 = s + 1; s2 < 4; ++s2) post += sD[s2 * 128 + c];
-#pragma unroll
-    for (int r = 0; r < 16; ++r)
-      if (16 * s + r < rows) p.dg[gk_base + (int64_t)(t0 + 16 * s + r) * gk_tok + c] = loc[r] + post;
-  } else if (p.variant == DR_GATED && warp == 0) {
-    float ts = sTS[lane] + sTS[lane + 32] + sTS[lane + 64] + sTS[lane + 96];
-    ts = warp_sum(ts) * expf(sGs[63]) + warp_sum(lane < 16 ? sXt[lane] : 0.f);
-    float lo = (sdG[lane] + sdG[64 + lane]) + (sdG[128 + lane] + sdG[192 + lane]);
-    float hi = (sdG[lane + 32] + sdG[96 + lane]) + (sdG[160 + lane] + sdG[224 + lane]) + (lane == 31 ? ts : 0.f);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float a = __shfl_down_sync(0xffffffffu, lo, o), c = __shfl_down_sync(0xffffffffu, hi, o);
-      if (lane + o < 32) { lo += a; hi += c; }
-    }
-    lo += __shfl_sync(0xffffffffu, hi, 0);
-    if (lane < rows) p.dg[s_base + (t0 + lane) * s_tok] = lo;
-    if (lane + 32 < rows) p.dg[s_base + (t0 + lane + 32) * s_tok] = hi;
+  for (int r = 15; r >= 0; --r) {
+    acc += sDG[(16 * s + r) * 132 + c];
+    loc[r] = acc;
   }
+  sD[s * 128 + c] = acc;
+  __syncthreads();
+  float post = 0.f;
+  for (int s2 = s + 1; s2 < 4; ++s2) post += sD[s2 * 128 + c];
+#pragma unroll
+  for (int r = 0; r < 16; ++r)
+    if (16 * s + r < rows) p.dg[gk_base + (int64_t)(t0 + 16 * s + r) * gk_tok + c] = loc[r] + post;
 }
 
+}  // namespace bwdc
+}  // namespace dr
+
+#include "dr_bwd_local_sm100.cuh"
+
+namespace dr {
+namespace bwdc {
 // =====================================================================================================================
 // host side
 // =====================================================================================================================
@@ -1505,7 +1375,7 @@ inline bool eligible(const DrDesc* d) {
   return d->K == kD && d->V == kD && d->chunk == kC && d->qkv_dtype == DR_BF16;
 }
 // floats per chunk: checkpoint, N (later the grouped heads' dq^, dk^), Y, X A T, dS1 (first the records of the two-kernel
-// forward: 66048 bytes), e^{G_L}
+// forward: 66048 bytes; scalar decays: and the norm factors), e^{G_L}
 constexpr int64_t kCkpt = 16384, kNf = 16384, kYf = 8192, kXat = 3 * 4096, kDs = 16512, kEl = 128;
 constexpr int64_t kFloats = kCkpt + kNf + kYf + kXat + kDs + kEl;
 inline int64_t workspace_bytes(const DrDesc* d) {
@@ -1521,7 +1391,7 @@ inline Params make_params(const DrDesc* d, void* workspace) {
   p.nf = reinterpret_cast<float4*>(f); p.part = f; f += nc * kNf;
   p.yf = reinterpret_cast<float4*>(f); f += nc * kYf;
   p.xat = f; f += nc * kXat;
-  p.ds = f; f += nc * kDs;
+  p.ds = f; p.norms = f + nc * kCkpt; f += nc * kDs;
   p.el = f;
   p.map.B = d->B; p.map.H = d->H; p.map.T = d->T; p.map.bthd = d->layout == DR_LAYOUT_BTHD;
   p.map.Hq = d->qk_heads > 0 ? d->qk_heads : d->H;
@@ -1529,17 +1399,22 @@ inline Params make_params(const DrDesc* d, void* workspace) {
   return p;
 }
 template <bool KDA>
-inline cudaError_t set_attributes() {
-  thread_local int attr_dev = -1;
+inline cudaError_t set_attributes(int* sms = nullptr) {
+  thread_local int attr_dev = -1, count = 0;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || attr_dev == dev) return e;
-  e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem<KDA>::kTotal);
-  if (e == cudaSuccess)
-    e = KDA ? cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem)
-            : cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
-  if (e == cudaSuccess) attr_dev = dev;
+  if (e == cudaSuccess && attr_dev != dev) {
+    e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
+    if (e == cudaSuccess)
+      e = KDA ? cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal)
+              : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
+    if (e == cudaSuccess)
+      e = KDA ? cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem)
+              : cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) attr_dev = dev;
+  }
+  if (sms) *sms = count;
   return e;
 }
 template <bool KDA>
@@ -1558,19 +1433,32 @@ inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, con
 }
 template <bool KDA>
 inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* status, cudaStream_t stream) {
-  cudaError_t e = set_attributes<KDA>();
+  int sms = 0;
+  cudaError_t e = set_attributes<KDA>(&sms);
   if (e != cudaSuccess) return e;
+  const int64_t chunks = units * p.N;
   if constexpr (KDA) {
     e = launch_pdl(state_kernel, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem, stream, p);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(local_kernel, dim3((unsigned)chunks), dim3(kLoThreads), LoSmem::kTotal, stream, p);
   } else {
     ChainParams c;
     c.p = p;
     c.status = status;
     if (!sm100::make_panel_map(&c.to, p.d_o, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
     e = launch_pdl(chain_kernel, dim3((unsigned)(units * (kD / kChCols))), dim3(kChThreads), CH_TOTAL, stream, c);
+    if (e != cudaSuccess) return e;
+    LocalParams lp;
+    lp.p = p; lp.chunks = (int)chunks; lp.status = status;
+    lp.n_tok = units * p.map.T; lp.n_part = 2 * chunks * (kC * kD);
+    const SeqMap& m = p.map;
+    auto panels = [&](CUtensorMap* t, const void* base, int heads) { return sm100::make_panel_map(t, base, m.B, heads, m.T, m.bthd != 0); };
+    lp.to = c.to;
+    if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
+        !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
+      return cudaErrorInvalidValue;
+    return launch_pdl(local_sm100_kernel, dim3((unsigned)(chunks < sms ? chunks : sms)), dim3(kLtThreads), LT_TOTAL, stream, lp);
   }
-  if (e != cudaSuccess) return e;
-  return launch_pdl(local_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kLoThreads), LoSmem<KDA>::kTotal, stream, p);
 }
 
 }  // namespace bwdc

@@ -198,3 +198,43 @@ def test_gradients_without_the_initial_states(variant, T):
          "gated": lambda: L.gated_delta_rule_chunkwise(*leaves, initial_state=h0), "kda": lambda: L.kda_chunkwise(*leaves, initial_state=h0)}[variant]
     f()[0].sum().backward()
     assert h0.grad is None and all(t is None or torch.isfinite(t.grad).all() for t in leaves)
+
+
+@pytest.mark.parametrize("variant,B,Hq,H,T,bthd,strong", [
+    ("gated", 1, 1, 1, 1, False, False), ("delta", 1, 2, 2, 63, True, False), ("gated", 1, 1, 2, 64, False, True),
+    ("gated", 2, 1, 3, 65, True, False), ("delta", 1, 1, 2, 129, False, False), ("gated", 1, 2, 2, 200, True, True),
+    ("gated", 3, 2, 2, 1665, False, False)])   # the last: 162 chunks, more than one per CTA
+def test_local_pass_on_tcgen05(variant, B, Hq, H, T, bthd, strong):
+    """Ragged chunks, one token, grouped q/k heads, both storages, a second chunk per persistent CTA, decays of e^-30 a token, against
+    float64.  bf16 outputs round at 2^-9 (2-norm 1.7e-3); operands of the forward's checkpoints are bf16 too, in all 1e-2 of the largest."""
+    inp = O.make_inputs(variant, B, H, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
+    if variant == "delta":
+        inp["k"] = torch.nn.functional.normalize(inp["k"].float(), dim=-1).bfloat16()
+    if strong:
+        inp["g"][:, :, ::5] = -30.0
+    q, k = inp["q"][:, :Hq], inp["k"][:, :Hq]
+    gen = torch.Generator().manual_seed(T + 1)
+    do, dhT = torch.randn(B, H, T, 128, generator=gen).bfloat16(), torch.randn(B, H, 128, 128, generator=gen) * 0.1
+    def cu(x):
+        if x is None:
+            return None
+        return x.transpose(1, 2).contiguous().cuda().transpose(1, 2) if bthd else x.contiguous().cuda()
+    l2 = variant != "delta"
+    args = (variant, cu(q), cu(k), cu(inp["v"]), cu(inp["g"]), cu(inp["beta"]), cu(do))
+    run = lambda: ops.chunk_backward(*args, initial_state=inp["h0"].cuda(), d_final_state=dhT.cuda(), chunk_size=64, use_qk_l2norm=l2)
+    got, again = run(), run()
+    L.check_device_status()
+    rep = lambda x: x.double().repeat_interleave(H // Hq, 1)
+    d = lambda x: None if x is None else x.double()
+    ref = O.delta_rule_grads(variant, rep(q), rep(k), d(inp["v"]), d(inp["g"]), d(inp["beta"]), d(inp["h0"]), d(do), d(dhT),
+                             use_qk_l2norm=l2)
+    for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):
+        want = ref[name]
+        if want is None:
+            assert got[name] is None
+            continue
+        if name in ("dq", "dk"):
+            want = want.view(B, Hq, H // Hq, T, 128).sum(2)
+        assert torch.equal(got[name], again[name]), name
+        err = (got[name].double().cpu() - want).norm() / want.norm()
+        assert err <= 1e-2, (name, err)
