@@ -1,10 +1,10 @@
 // Chunkwise forward with PER-CHANNEL decay (KDA) for Blackwell, as two kernels:
 //
-//   (1) intra_kernel   one CTA per (sequence, chunk), all chunks in parallel: everything that does not
+//   (1) intra_kernel   all chunks in parallel, persistent CTAs: everything that does not
 //                      depend on the running state.  Cumulative log decay G, the decayed chunk-local
 //                      products A_kk, A_qk, the unit-lower inverse T = (I + diag(beta) A_kk)^-1 and the
 //                      bf16 operand tiles of the state pass, written to a workspace record per chunk in
-//                      exactly the 8x8 core-matrix order the tensor cores read, so that the state kernel
+//                      exactly the swizzled order the tensor cores read, so that the state kernel
 //                      fetches each tile with ONE 1-d bulk copy (no tensor map).
 //   (2) state_kernel   one CTA per sequence walks the chunks; the fp32 state lives transposed in tensor
 //                      memory (lane = value column) and every product is a tcgen05.mma:
@@ -16,7 +16,8 @@
 //                      with W = T diag(beta) (k^ e^G), Qg = scale q^ e^G, Kd = k^ e^{G_L - G}.
 //
 // Per-channel decay cannot be folded into row/column factors of a plain K K^T product the way a scalar
-// decay can, and e^{-G} alone overflows for strong decay.  The chunk-local products therefore use 16-row
+// decay can, and e^{-G} alone overflows for strong decay.  A chunk that decays by at most 2^64 takes one product of decayed rows (see
+// intra_kernel); for the others, and in the transition form, the chunk-local products use 16-row
 // sub-blocks: rows of sub-block bi against earlier columns are the bf16 tensor-core product of
 // x_i e^{G_i - G_n}  and  k_j e^{G_n - G_j}  with n the first row of bi, so both exponents are <= 0; the four diagonal
 // 16x16 blocks use the same form while their decay range stays below 2^64 and are summed exactly in fp32 otherwise.
@@ -24,6 +25,8 @@
 // Shape: K = V = 128, chunk 64, bf16 q/k/v, g bf16 or fp32 ([.., K] for KDA; the scalar-decay and
 // decay-free variants are served too, by broadcasting), fp32 beta/state, bf16 or fp32 output.
 #pragma once
+
+#include <algorithm>
 
 #include "dr_chunk_sm100.cuh"
 #include "dr_mma.cuh"
@@ -38,8 +41,8 @@ using sm100::A_RBS;
 constexpr int kC = 64, kD = 128;
 constexpr int kThreads = 256;
 
-// workspace record of one chunk (bytes); every tile in 8x8 core-matrix order
-constexpr int WS_W = 0;                    // W   [64][128] bf16
+// workspace record of one chunk (bytes); tiles in the 128-byte swizzle, panels of 64 columns one after the other
+constexpr int WS_W = 0;                    // W^T [128][64] bf16
 constexpr int WS_QG = WS_W + 16384;        // Qg  [64][128] bf16
 constexpr int WS_KD = WS_QG + 16384;       // Kd  [64][128] bf16
 constexpr int WS_TB = WS_KD + 16384;       // T diag(beta) [64][64] bf16
@@ -52,16 +55,11 @@ constexpr int WS_ASKED = 82432;
 static_assert(WS_REC <= WS_ASKED, "records fit what callers provide");
 inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC - 1) / kC) * (int64_t)WS_ASKED; }
 
-// ---- intra-chunk kernel ------------------------------------------------------------------------------------
+// ---- the general products and the transition form's pass ----------------------------------------------------------
 // Shared memory is kept under half an SM's worth so that two CTAs are resident and one chunk's latency
 // (global loads, the serial prefix sum, the barriers between phases) hides behind the other's work.  The
 // inputs stay as raw bf16 with their l2-norm factors on the side, and the decayed bf16 operands of the
 // tensor-core products are formed in registers from them (no scaled copies in shared memory).
-// What bounds it: latency of dependent phases at 16 warps per SM (issue slots 47 %, shared-memory pipe 55 %, tensor pipe 10 %
-// busy).  Of 24 K cycles per chunk (two chunks at a time) 6.1 K are the loads, 8.9 K the products and the inverse's start,
-// 7.4 K the record.  B=4 T=8192 H=32 (16384 chunks): 930 -> 820 us with one quotient per row instead of one per lane, W as two bf16 terms
-// and 16-byte reads.  Forming the decayed rows once as bf16 tiles was slower (1.44 against 1.21 ms for the whole forward):
-// two passes over 16 rows per thread in registers cost more than the exponentials they save.
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
@@ -151,9 +149,10 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
 // Kernel parameters of the intra pass; a packed batch adds the table of its sequences (p then describes the packed
 // arrays: B = 1, T = all tokens, token-major).
 struct IntraParams {
+  CUtensorMap tq, tk, tg;   // panels of q and k; g as boxes of 64 rows
   FwdParams p;
   uint8_t* ws;
-  int resident;   // CTAs that run at a time
+  int chunks, use_tma;
 };
 struct IntraPackedParams : IntraParams {
   SeqTable seqs;
@@ -184,168 +183,11 @@ __device__ __forceinline__ void decayed_piece(const float* gr, const float* gl, 
   }
 }
 
-template <class Params>
-__global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constant__ Params P) {
-  constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value, kTrans = std::is_same<Params, IntraTransParams>::value;
-  const FwdParams& p = P.p;
-  pdl_entry();
-  extern __shared__ __align__(1024) uint8_t smem[];
-  float* sG = reinterpret_cast<float*>(smem + IN_G);
-  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + IN_K);
-  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + IN_Q);
-  float* sAkk = reinterpret_cast<float*>(smem + IN_AKK);
-  __nv_bfloat16* sWst = reinterpret_cast<__nv_bfloat16*>(smem + IN_AKK);
-  float* sT = reinterpret_cast<float*>(smem + IN_T);
-  __nv_bfloat16* sAqk = reinterpret_cast<__nv_bfloat16*>(smem + IN_AQK);
-  float* sBeta = reinterpret_cast<float*>(smem + IN_BETA);
-  float* sRk = sBeta + 64;
-  float* sRq = sBeta + 128;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  int T = p.map.T, n, b, h, tok0 = 0;
-  uint8_t* rec = nullptr;
-  if constexpr (!kTrans) rec = P.ws;
-  if constexpr (kPacked) {
-    h = blockIdx.x / P.seqs.chunks;
-    const int c = blockIdx.x % P.seqs.chunks;
-    int lo = 0, hi = P.seqs.n - 1;   // the last sequence that starts at or before chunk c
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (P.seqs.first[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    n = c - P.seqs.first[lo];
-    T = P.seqs.len[lo];
-    tok0 = P.seqs.start[lo];
-    b = 0;
-    rec += ((int64_t)P.seqs.first[lo] * p.map.H + (int64_t)h * ((T + kC - 1) / kC) + n) * WS_REC;
-  } else {
-    const int nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks;
-    n = blockIdx.x % nchunks;
-    b = unit / p.map.H; h = unit % p.map.H;
-    if constexpr (!kTrans) rec += ((int64_t)unit * nchunks + n) * WS_REC;
-  }
-  const int rows = min(kC, T - n * kC), t0 = tok0 + n * kC;
-  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
-  const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);         // per-channel decay: per value head
-  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  constexpr float kLog2e = 1.4426950408889634f;
-
-  // ---- load: raw k, q rows, their norm factors, the log decay (in log2 units); lane = four channels ---------
-  // (all global loads of the warp's eight rows are issued before the first is used)
-  {
-    uint2 qraw[8], kraw[8];
-    float gv[8][4];
-    {
-      const int64_t at = qk_base + (t0 + warp) * qk_tok + 4 * lane;
-      const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(p.q) + at;
-      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(p.k) + at;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        qraw[i] = make_uint2(0u, 0u); kraw[i] = make_uint2(0u, 0u);
-        if (warp + 8 * i < rows) {
-          qraw[i] = *reinterpret_cast<const uint2*>(qp);
-          kraw[i] = *reinterpret_cast<const uint2*>(kp);
-        }
-        qp += 8 * qk_tok; kp += 8 * qk_tok;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = 0.f;
-    if (p.variant == DR_KDA) {   // one loop per storage type: no branch between the loads
-      int64_t at = gk_base + (t0 + warp) * gk_tok + 4 * lane;
-      if (p.g_dt == DR_BF16) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
-          if (warp + 8 * i < rows) ld4(p.g, at, DR_BF16, gv[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
-          if (warp + 8 * i < rows) ld4(p.g, at, DR_F32, gv[i]);
-      }
-    } else if (p.variant == DR_GATED) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (warp + 8 * i < rows) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = ld_elem(p.g, s_base + (t0 + warp + 8 * i) * s_tok, p.g_dt);
-    }
-    float bt = 0.f;
-    if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = warp + 8 * i;
-      *reinterpret_cast<uint2*>(sQ + c * LDH + 4 * lane) = qraw[i];
-      *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kraw[i];
-      *reinterpret_cast<float4*>(sG + c * LDF + 4 * lane) =
-          make_float4(gv[i][0] * kLog2e, gv[i][1] * kLog2e, gv[i][2] * kLog2e, gv[i][3] * kLog2e);
-    }
-    if constexpr (!kPacked && !kTrans) {
-      // the rows of the chunk that follows in this CTA's place, into L2 (thread = a quarter of a row): 1090 -> 1081 us at B=4 T=8192 H=32
-      const int64_t nb = (int64_t)blockIdx.x + P.resident;
-      if (nb < gridDim.x) {
-        const int nchunks = (T + kC - 1) / kC, u2 = (int)(nb / nchunks), tok = ((int)nb - u2 * nchunks) * kC + (tid >> 2);
-        if (tok < T) {
-          const int b2 = u2 / p.map.H, h2 = u2 - b2 * p.map.H;
-          prefetch_l2(reinterpret_cast<const __nv_bfloat16*>((tid & 2) ? p.k : p.q) + p.map.base_qk(b2, h2, kD) + (int64_t)tok * qk_tok + (tid & 1) * 64);
-          if (p.variant == DR_KDA) {
-            const int64_t at = p.map.base(b2, h2, kD) + (int64_t)tok * gk_tok + (tid & 3) * 32;
-            if (p.g_dt == DR_F32) prefetch_l2(reinterpret_cast<const float*>(p.g) + at);
-            else if (!(tid & 1)) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.g) + at);
-          }
-        }
-      }
-    }
-    // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced (16 shuffles instead of
-    // 80), so that each lane takes one square root and one quotient (as every lane did for every row, a fifth of the pass)
-    float ss[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float2 q0 = bf2(qraw[i].x), q1 = bf2(qraw[i].y), k0 = bf2(kraw[i].x), k1 = bf2(kraw[i].y);
-      ss[i] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
-      ss[8 + i] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
-    }
-#pragma unroll
-    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
-#pragma unroll
-      for (int i = 0; i < m; ++i) {
-        const bool up = lane & o;
-        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
-        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    }
-    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
-    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
-      const float top = lane < 16 ? p.scale : 1.f;
-      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
-    }
-    if (lane < 8) sBeta[warp + 8 * lane] = bt;
-  }
-  __syncthreads();
-  // ---- G = inclusive prefix sum of the log decay over the rows of the chunk, per channel ---------------------
-  // thread = (8-row segment, four channels): local scan, then the totals of the earlier segments are added;
-  // the segment totals live in the first rows of the (still unused) T array
-  {
-    const int seg = tid >> 5, c4 = 4 * (tid & 31);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 loc[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const float4 x = *reinterpret_cast<const float4*>(sG + (8 * seg + r) * LDF + c4);
-      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
-      loc[r] = acc;
-    }
-    *reinterpret_cast<float4*>(sT + seg * 128 + c4) = acc;
-    __syncthreads();
-    float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s2 = 0; s2 < seg; ++s2) {
-      const float4 x = *reinterpret_cast<const float4*>(sT + s2 * 128 + c4);
-      pre.x += x.x; pre.y += x.y; pre.z += x.z; pre.w += x.w;
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      *reinterpret_cast<float4*>(sG + (8 * seg + r) * LDF + c4) =
-          make_float4(loc[r].x + pre.x, loc[r].y + pre.y, loc[r].z + pre.z, loc[r].w + pre.w);
-    __syncthreads();
-  }
+// The chunk-local products for any decay: A_kk (below the diagonal) and A_qk (bf16; above the diagonal of its 16-row blocks scratch) from G
+// and the raw rows.  256 threads (named barrier 1); G, rows and norm factors in shared memory behind a barrier; ends with one.
+__device__ __forceinline__ void general_products(const float* sG, const __nv_bfloat16* sK, const __nv_bfloat16* sQ, float* sAkk, float* sT,
+                                                 __nv_bfloat16* sAqk, const float* sRk, const float* sRq, int tid) {
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   // ---- chunk-local products on mma.sync (bf16) -------------------------------------------------------------------
   // Rows of sub-block bi against the columns of blocks 0..bi; operands  x_i e^{G_i - G_n}  and  k_j e^{G_n - G_j}
   // (n = first row of bi) are formed in registers; the k and q rows share their decay factors and the column
@@ -430,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
   // Two warps per block, 64 channels each, two channels per lane; the 16 rows of k and the per-row decay
   // d_r = e^{G_r - G_{r-1}} stay in registers, so e^{G_i - G_j} is a running product (no exponentials per pair).
   // Partial sums of the two channel halves meet in a scratch array (the T array, not yet in use).
-  __syncthreads();   // the tensor-core tasks have written their (possibly non-finite) entries of these blocks
+  sm100::group_sync(1);   // the tensor-core tasks have written their (possibly non-finite) entries of these blocks
   if (block_unsafe(warp >> 1)) {
     const int blk = warp >> 1, half = warp & 1, ch0 = 64 * half + 2 * lane;
     float2 kr[16], dd[16];
@@ -489,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
         }
       }
     }
-    asm volatile("bar.sync %0, 64;" ::"r"(2 + blk) : "memory");   // the two warps of this block
+    asm volatile("bar.sync %0, 64;" ::"r"(8 + blk) : "memory");   // the two warps of this block
     const float* p0 = sT + blk * 512;
     const float* p1 = sT + (4 + blk) * 512;
     for (int e = lane; e < 256; e += 32) {
@@ -501,219 +343,730 @@ __global__ void __launch_bounds__(kThreads, 2) intra_kernel(const __grid_constan
       }
     }
   }
-  __syncthreads();
-  // ---- T = (I + diag(beta) A_kk)^-1 -----------------------------------------------------------------------------
-  sm100::block_inverse_64(sAkk, sBeta, sT, tid);
-  if constexpr (kTrans) {
-    // ---- the chunk's effect on the state and on its own output, as fragments of trans_state_kernel ----------------------------
-    //   N = -Kd^T W, Z = Kd^T U, Y = Qg - A_qk W, A_qk U   with W = T diag(beta) k^ e^G, U = T diag(beta) V
-    // Tb = T diag(beta) -> bf16 over A_kk; A_qk masked in place; then (T and G dead) V over T, k^ e^G over G, Qg over q, Kd over k
-    __nv_bfloat16* sTb = sWst;                                              // [64][72]
-    __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(smem + IN_T);      // [64][136]
-    __nv_bfloat16* sKg = reinterpret_cast<__nv_bfloat16*>(smem + IN_G);     // [64][136]
-    uint4 vv[4], qg[4], kd[4], kg[4];
-    const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-      vv[it] = make_uint4(0u, 0u, 0u, 0u);
-      if (row < rows) vv[it] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.v) + v_base + (t0 + row) * v_tok + col);
-    }
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const int piece = tid + kThreads * it, row = piece >> 3, col = (piece & 7) * 8;
-      float a[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? sT[row * LDT + col + e] * sBeta[col + e] : 0.f;
-      *reinterpret_cast<uint4*>(sTb + row * LDQ + col) = pack8(a);
-      if (col + 7 > row && (col >> 4) <= (row >> 4)) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (col + e > row) sAqk[row * LDQ + col + e] = __float2bfloat16_rn(0.f);
-      }
-    }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-      const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col), uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
-      decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], qg[it], kd[it], kg[it]);
-    }
-    const int64_t chunk = blockIdx.x;
-    if (tid < kD) P.el[chunk * kD + tid] = ex2(sG[63 * LDF + tid]);
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-      *reinterpret_cast<uint4*>(sV + row * LDH + col) = vv[it];
-      *reinterpret_cast<uint4*>(sQ + row * LDH + col) = qg[it];
-      *reinterpret_cast<uint4*>(sK + row * LDH + col) = kd[it];
-      *reinterpret_cast<uint4*>(sKg + row * LDH + col) = kg[it];
-    }
-    __syncthreads();
-    const uint32_t aTb = tc::smem_u32(sTb), aV = tc::smem_u32(sV), aKg = tc::smem_u32(sKg), aKd = tc::smem_u32(sK), aAq = tc::smem_u32(sAqk);
-    // W^T, U^T of the warp's 16 channels / value columns (rows), columns = tokens; then as B operands (k = token)
-    uint32_t Wb[4][2][2], Ub[4][2][2];   // [16-token step][8-column half][k half]
+  sm100::group_sync(1);
+}
+static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const __grid_constant__ IntraTransParams P) {
+  const FwdParams& p = P.p;
+  pdl_entry();
+  extern __shared__ __align__(1024) uint8_t smem[];
+  float* sG = reinterpret_cast<float*>(smem + IN_G);
+  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + IN_K);
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + IN_Q);
+  float* sAkk = reinterpret_cast<float*>(smem + IN_AKK);
+  __nv_bfloat16* sWst = reinterpret_cast<__nv_bfloat16*>(smem + IN_AKK);
+  float* sT = reinterpret_cast<float*>(smem + IN_T);
+  __nv_bfloat16* sAqk = reinterpret_cast<__nv_bfloat16*>(smem + IN_AQK);
+  float* sBeta = reinterpret_cast<float*>(smem + IN_BETA);
+  float* sRk = sBeta + 64;
+  float* sRq = sBeta + 128;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int T = p.map.T, nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks, n = blockIdx.x % nchunks;
+  const int b = unit / p.map.H, h = unit % p.map.H, rows = min(kC, T - n * kC), t0 = n * kC;
+  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
+  const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);         // per-channel decay: per value head
+  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
+  constexpr float kLog2e = 1.4426950408889634f;
+
+  // ---- load: raw k, q rows, their norm factors, the log decay (in log2 units); lane = four channels ---------
+  // (all global loads of the warp's eight rows are issued before the first is used)
+  {
+    uint2 qraw[8], kraw[8];
+    float gv[8][4];
     {
-      float W[8][4], U[8][4];
+      const int64_t at = qk_base + (t0 + warp) * qk_tok + 4 * lane;
+      const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(p.q) + at;
+      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(p.k) + at;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        W[nt][0] = W[nt][1] = W[nt][2] = W[nt][3] = 0.f;
-        U[nt][0] = U[nt][1] = U[nt][2] = U[nt][3] = 0.f;
-      }
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        uint32_t aw[4], au[4];
-        mma::ldsm4t(aw, mma::frag_at(aKg, LDH, 16 * ks, 16 * warp, lane));
-        mma::ldsm4t(au, mma::frag_at(aV, LDH, 16 * ks, 16 * warp, lane));
-#pragma unroll
-        for (int n2 = 0; n2 < 4; ++n2) {
-          if (n2 >= ks) {
-            uint32_t bt[4];
-            mma::ldsm4(bt, mma::frag_b(aTb, LDQ, 16 * n2, 16 * ks, lane));
-            mma::bf16(W[2 * n2], aw, bt[0], bt[1]);
-            mma::bf16(W[2 * n2 + 1], aw, bt[2], bt[3]);
-            mma::bf16(U[2 * n2], au, bt[0], bt[1]);
-            mma::bf16(U[2 * n2 + 1], au, bt[2], bt[3]);
-          }
+      for (int i = 0; i < 8; ++i) {
+        qraw[i] = make_uint2(0u, 0u); kraw[i] = make_uint2(0u, 0u);
+        if (warp + 8 * i < rows) {
+          qraw[i] = *reinterpret_cast<const uint2*>(qp);
+          kraw[i] = *reinterpret_cast<const uint2*>(kp);
         }
+        qp += 8 * qk_tok; kp += 8 * qk_tok;
       }
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-          for (int kh = 0; kh < 2; ++kh) {
-            Wb[ks][hf][kh] = mma::pack(W[2 * ks + kh][2 * hf], W[2 * ks + kh][2 * hf + 1]);
-            Ub[ks][hf][kh] = mma::pack(U[2 * ks + kh][2 * hf], U[2 * ks + kh][2 * hf + 1]);
-          }
     }
-#pragma unroll 1
-    for (int mt = 0; mt < 12; ++mt) {   // rows of [Kd^T (8 tiles); A_qk (4 tiles)]
-      const bool st = mt < 8;
-      const int m = st ? mt : mt - 8;
-      float w[2][4], u[2][4];
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) { w[hf][0] = w[hf][1] = w[hf][2] = w[hf][3] = 0.f; u[hf][0] = u[hf][1] = u[hf][2] = u[hf][3] = 0.f; }
+    for (int i = 0; i < 8; ++i) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = 0.f;
+    if (p.variant == DR_KDA) {   // one loop per storage type: no branch between the loads
+      int64_t at = gk_base + (t0 + warp) * gk_tok + 4 * lane;
+      if (p.g_dt == DR_BF16) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        if (st || ks <= m) {
-          uint32_t a[4];
-          if (st) mma::ldsm4t(a, mma::frag_at(aKd, LDH, 16 * ks, 16 * m, lane));
-          else mma::ldsm4(a, mma::frag_a(aAq, LDQ, 16 * m, 16 * ks, lane));
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            mma::bf16(w[hf], a, Wb[ks][hf][0], Wb[ks][hf][1]);
-            mma::bf16(u[hf], a, Ub[ks][hf][0], Ub[ks][hf][1]);
-          }
-        }
-      }
-      const int64_t at = (chunk * (st ? 8 : 4) + m) * 8 + warp;
-      if (st) {
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) { w[hf][0] = -w[hf][0]; w[hf][1] = -w[hf][1]; w[hf][2] = -w[hf][2]; w[hf][3] = -w[hf][3]; }
+        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
+          if (warp + 8 * i < rows) ld4(p.g, at, DR_BF16, gv[i]);
       } else {
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-          for (int hr = 0; hr < 2; ++hr) {
-            const float2 q2 = bf2(*reinterpret_cast<const uint32_t*>(sQ + (16 * m + g + 8 * hr) * LDH + 16 * warp + 8 * hf + 2 * t));
-            w[hf][2 * hr] = q2.x - w[hf][2 * hr];
-            w[hf][2 * hr + 1] = q2.y - w[hf][2 * hr + 1];
-          }
+        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
+          if (warp + 8 * i < rows) ld4(p.g, at, DR_F32, gv[i]);
       }
-      (st ? P.nf : P.yf)[at * 32 + lane] = make_uint4(mma::pack(w[0][0], w[0][1]), mma::pack(w[0][2], w[0][3]), mma::pack(w[1][0], w[1][1]), mma::pack(w[1][2], w[1][3]));
-      float4* dst = (st ? P.zf : P.of) + at * 64 + lane;
-      dst[0] = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
-      dst[32] = make_float4(u[1][0], u[1][1], u[1][2], u[1][3]);
+    } else if (p.variant == DR_GATED) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (warp + 8 * i < rows) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = ld_elem(p.g, s_base + (t0 + warp + 8 * i) * s_tok, p.g_dt);
     }
-    return;
+    float bt = 0.f;
+    if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = warp + 8 * i;
+      *reinterpret_cast<uint2*>(sQ + c * LDH + 4 * lane) = qraw[i];
+      *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kraw[i];
+      *reinterpret_cast<float4*>(sG + c * LDF + 4 * lane) =
+          make_float4(gv[i][0] * kLog2e, gv[i][1] * kLog2e, gv[i][2] * kLog2e, gv[i][3] * kLog2e);
+    }
+    // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced (16 shuffles instead of
+    // 80), so that each lane takes one square root and one quotient (as every lane did for every row, a fifth of the pass)
+    float ss[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 q0 = bf2(qraw[i].x), q1 = bf2(qraw[i].y), k0 = bf2(kraw[i].x), k1 = bf2(kraw[i].y);
+      ss[i] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
+      ss[8 + i] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
+    }
+#pragma unroll
+    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        const bool up = lane & o;
+        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
+        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
+      const float top = lane < 16 ? p.scale : 1.f;
+      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+    }
+    if (lane < 8) sBeta[warp + 8 * lane] = bt;
   }
-  // ---- record tiles: T diag(beta), A_qk, Qg = scale q^ e^G, Kd = k^ e^{G_L - G}, e^{G_L} ------------------------
+  __syncthreads();
+  // ---- G = inclusive prefix sum of the log decay over the rows of the chunk, per channel ---------------------
+  // thread = (8-row segment, four channels): local scan, then the totals of the earlier segments are added;
+  // the segment totals live in the first rows of the (still unused) T array
+  {
+    const int seg = tid >> 5, c4 = 4 * (tid & 31);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 loc[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float4 x = *reinterpret_cast<const float4*>(sG + (8 * seg + r) * LDF + c4);
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+      loc[r] = acc;
+    }
+    *reinterpret_cast<float4*>(sT + seg * 128 + c4) = acc;
+    __syncthreads();
+    float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s2 = 0; s2 < seg; ++s2) {
+      const float4 x = *reinterpret_cast<const float4*>(sT + s2 * 128 + c4);
+      pre.x += x.x; pre.y += x.y; pre.z += x.z; pre.w += x.w;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      *reinterpret_cast<float4*>(sG + (8 * seg + r) * LDF + c4) =
+          make_float4(loc[r].x + pre.x, loc[r].y + pre.y, loc[r].z + pre.z, loc[r].w + pre.w);
+    __syncthreads();
+  }
+  general_products(sG, sK, sQ, sAkk, sT, sAqk, sRk, sRq, tid);
+  // ---- T = (I + diag(beta) A_kk)^-1 -----------------------------------------------------------------------------
+  sm100::block_inverse_64(sAkk, sBeta, sT, tid);
+  // ---- the chunk's effect on the state and on its own output, as fragments of trans_state_kernel ----------------------------
+  //   N = -Kd^T W, Z = Kd^T U, Y = Qg - A_qk W, A_qk U   with W = T diag(beta) k^ e^G, U = T diag(beta) V
+  // Tb = T diag(beta) -> bf16 over A_kk; A_qk masked in place; then (T and G dead) V over T, k^ e^G over G, Qg over q, Kd over k
+  __nv_bfloat16* sTb = sWst;                                              // [64][72]
+  __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(smem + IN_T);      // [64][136]
+  __nv_bfloat16* sKg = reinterpret_cast<__nv_bfloat16*>(smem + IN_G);     // [64][136]
+  uint4 vv[4], qg[4], kd[4], kg[4];
+  const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+    vv[it] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows) vv[it] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.v) + v_base + (t0 + row) * v_tok + col);
+  }
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
-    const int piece = tid + kThreads * it;
-    int row, col;
-    piece64(piece, row, col);   // eight rows to a quarter warp: the 16-byte reads are free of bank conflicts
-    float a[8], bt[8];
-    *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sT + row * LDT + col);
-    *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sT + row * LDT + col + 4);
-    *reinterpret_cast<float4*>(bt) = *reinterpret_cast<const float4*>(sBeta + col);
-    *reinterpret_cast<float4*>(bt + 4) = *reinterpret_cast<const float4*>(sBeta + col + 4);
+    const int piece = tid + kThreads * it, row = piece >> 3, col = (piece & 7) * 8;
+    float a[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? a[e] * bt[e] : 0.f;
-    *reinterpret_cast<uint4*>(rec + WS_TB + piece * 16) = pack8(a);
-    uint4 q = *reinterpret_cast<const uint4*>(sAqk + row * LDQ + col);
-    uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
+    for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? sT[row * LDT + col + e] * sBeta[col + e] : 0.f;
+    *reinterpret_cast<uint4*>(sTb + row * LDQ + col) = pack8(a);
+    if (col + 7 > row && (col >> 4) <= (row >> 4)) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {   // keep j <= row
-      const int j = col + 2 * e;
-      if (j > row) qw[e] = 0u;
-      else if (j + 1 > row) qw[e] &= 0x0000ffffu;
+      for (int e = 0; e < 8; ++e)
+        if (col + e > row) sAqk[row * LDQ + col + e] = __float2bfloat16_rn(0.f);
     }
-    *reinterpret_cast<uint4*>(rec + WS_AQK + piece * 16) = q;
   }
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
-    const int piece = tid + kThreads * it;
-    int row, col;
-    piece128(piece, row, col);
-    const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col);
-    const uint4 uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
-    uint4 a, c, kg;
-    decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], a, c, kg);
-    *reinterpret_cast<uint4*>(rec + WS_QG + piece * 16) = a;
-    *reinterpret_cast<uint4*>(rec + WS_KD + piece * 16) = c;
-    *reinterpret_cast<uint4*>(sQ + row * LDH + col) = kg;   // k^ e^G for the W product (q is dead)
+    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+    const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col), uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
+    decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], qg[it], kd[it], kg[it]);
   }
-  if (tid < kD) reinterpret_cast<float*>(rec + WS_EGL)[tid] = ex2(sG[63 * LDF + tid]);
+  const int64_t chunk = blockIdx.x;
+  if (tid < kD) P.el[chunk * kD + tid] = ex2(sG[63 * LDF + tid]);
   __syncthreads();
-  // ---- W = (T diag(beta)) (k^ e^G): 64x128x64 on mma.sync (bf16); warp = 16 rows x 64 channels ----------------------
-  // T diag(beta) is fp32 in shared memory: two bf16 terms (16 bits, tf32 has 11), against the bf16 tile by ldmatrix; with tf32
-  // products the tile was read two bytes at a time.  Within eight tokens the contraction runs over (0 4 1 5 2 6 3 7), for which
-  // the reads of T are free of bank conflicts.
-  // (A_kk is dead after the inverse: its array takes the bf16 staging tile of W)
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
+    *reinterpret_cast<uint4*>(sV + row * LDH + col) = vv[it];
+    *reinterpret_cast<uint4*>(sQ + row * LDH + col) = qg[it];
+    *reinterpret_cast<uint4*>(sK + row * LDH + col) = kd[it];
+    *reinterpret_cast<uint4*>(sKg + row * LDH + col) = kg[it];
+  }
+  __syncthreads();
+  const uint32_t aTb = tc::smem_u32(sTb), aV = tc::smem_u32(sV), aKg = tc::smem_u32(sKg), aKd = tc::smem_u32(sK), aAq = tc::smem_u32(sAqk);
+  // W^T, U^T of the warp's 16 channels / value columns (rows), columns = tokens; then as B operands (k = token)
+  uint32_t Wb[4][2][2], Ub[4][2][2];   // [16-token step][8-column half][k half]
   {
-    const int m0 = (warp >> 1) * 16, nb = (warp & 1) * 64;
-    float d[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) { d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f; }
-    const int r0 = m0 + g, r1 = r0 + 8;
-    const uint32_t aB = tc::smem_u32(sQ) + 2u * (((lane & 8) + ((lane & 7) >> 1) + (lane & 1) * 4) * LDH + nb + (lane >> 4) * 8);
-    for (int kb = 0; kb <= m0; kb += 16) {
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {   // e & 1: row half, e >> 1: k half
-        const int r = (e & 1) ? r1 : r0, k0 = kb + 8 * (e >> 1) + t, k1 = k0 + 4;
-        const float x = k0 <= r ? sT[r * LDT + k0] * sBeta[k0] : 0.f;
-        const float y = k1 <= r ? sT[r * LDT + k1] * sBeta[k1] : 0.f;
-        hi[e] = tc::pack_bf16(x, y);
-        const float2 h = bf2(hi[e]);
-        lo[e] = tc::pack_bf16(x - h.x, y - h.y);
-      }
-#pragma unroll
-      for (int n2 = 0; n2 < 4; ++n2) {
-        uint32_t bb[4];
-        mma::ldsm4t(bb, aB + 2u * (kb * LDH + 16 * n2));
-        mma::bf16(d[2 * n2], hi, bb[0], bb[1]);
-        mma::bf16(d[2 * n2 + 1], hi, bb[2], bb[3]);
-        mma::bf16(d[2 * n2], lo, bb[0], bb[1]);
-        mma::bf16(d[2 * n2 + 1], lo, bb[2], bb[3]);
-      }
-    }
+    float W[8][4], U[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      *reinterpret_cast<uint32_t*>(sWst + r0 * LDH + nb + nt * 8 + 2 * t) = tc::pack_bf16(d[nt][0], d[nt][1]);
-      *reinterpret_cast<uint32_t*>(sWst + r1 * LDH + nb + nt * 8 + 2 * t) = tc::pack_bf16(d[nt][2], d[nt][3]);
+      W[nt][0] = W[nt][1] = W[nt][2] = W[nt][3] = 0.f;
+      U[nt][0] = U[nt][1] = U[nt][2] = U[nt][3] = 0.f;
+    }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t aw[4], au[4];
+      mma::ldsm4t(aw, mma::frag_at(aKg, LDH, 16 * ks, 16 * warp, lane));
+      mma::ldsm4t(au, mma::frag_at(aV, LDH, 16 * ks, 16 * warp, lane));
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) {
+        if (n2 >= ks) {
+          uint32_t bt[4];
+          mma::ldsm4(bt, mma::frag_b(aTb, LDQ, 16 * n2, 16 * ks, lane));
+          mma::bf16(W[2 * n2], aw, bt[0], bt[1]);
+          mma::bf16(W[2 * n2 + 1], aw, bt[2], bt[3]);
+          mma::bf16(U[2 * n2], au, bt[0], bt[1]);
+          mma::bf16(U[2 * n2 + 1], au, bt[2], bt[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh) {
+          Wb[ks][hf][kh] = mma::pack(W[2 * ks + kh][2 * hf], W[2 * ks + kh][2 * hf + 1]);
+          Ub[ks][hf][kh] = mma::pack(U[2 * ks + kh][2 * hf], U[2 * ks + kh][2 * hf + 1]);
+        }
+  }
+#pragma unroll 1
+  for (int mt = 0; mt < 12; ++mt) {   // rows of [Kd^T (8 tiles); A_qk (4 tiles)]
+    const bool st = mt < 8;
+    const int m = st ? mt : mt - 8;
+    float w[2][4], u[2][4];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) { w[hf][0] = w[hf][1] = w[hf][2] = w[hf][3] = 0.f; u[hf][0] = u[hf][1] = u[hf][2] = u[hf][3] = 0.f; }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      if (st || ks <= m) {
+        uint32_t a[4];
+        if (st) mma::ldsm4t(a, mma::frag_at(aKd, LDH, 16 * ks, 16 * m, lane));
+        else mma::ldsm4(a, mma::frag_a(aAq, LDQ, 16 * m, 16 * ks, lane));
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          mma::bf16(w[hf], a, Wb[ks][hf][0], Wb[ks][hf][1]);
+          mma::bf16(u[hf], a, Ub[ks][hf][0], Ub[ks][hf][1]);
+        }
+      }
+    }
+    const int64_t at = (chunk * (st ? 8 : 4) + m) * 8 + warp;
+    if (st) {
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) { w[hf][0] = -w[hf][0]; w[hf][1] = -w[hf][1]; w[hf][2] = -w[hf][2]; w[hf][3] = -w[hf][3]; }
+    } else {
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+          const float2 q2 = bf2(*reinterpret_cast<const uint32_t*>(sQ + (16 * m + g + 8 * hr) * LDH + 16 * warp + 8 * hf + 2 * t));
+          w[hf][2 * hr] = q2.x - w[hf][2 * hr];
+          w[hf][2 * hr + 1] = q2.y - w[hf][2 * hr + 1];
+        }
+    }
+    (st ? P.nf : P.yf)[at * 32 + lane] = make_uint4(mma::pack(w[0][0], w[0][1]), mma::pack(w[0][2], w[0][3]), mma::pack(w[1][0], w[1][1]), mma::pack(w[1][2], w[1][3]));
+    float4* dst = (st ? P.zf : P.of) + at * 64 + lane;
+    dst[0] = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
+    dst[32] = make_float4(u[1][0], u[1][1], u[1][2], u[1][3]);
+  }
+}
+
+// ---- intra-chunk kernel, records ------------------------------------------------------------------------------------------------
+// Two persistent CTAs per SM: eight warps that work, one that issues copies and products.  A worker warp owns eight rows of the chunk, a lane
+// four channels of them, from the prefix sums to the tiles.
+//
+// With G summed from the chunk's start, e^{G_i - G_j} = e^{G_i} e^{-G_j}: while no channel decays by more than 2^64 over the chunk, the
+// factors fit bf16's exponents, and both chunk-local products are one tcgen05 product, [k^ e^G; q^ e^G] (k^ e^{-G})^T, of tiles
+// of which the record and W need the first two anyway.  An entry above the diagonal may be as large as 2^64 |k|^2; none is used.
+// Chunks with a wider range (never with trained gates, but legal input) take general_products, which refers the decays to 16-row blocks.
+//
+// Rows arrive by TMA a chunk ahead: k and q into the tiles that their decayed forms are written over, q where q^ e^G of the chunk
+// before has left for its record, k where Kd has.  So Kd takes k^ e^G's place of the chunk before and the two change places every
+// chunk.  Tiles are in the 128-byte swizzle, rows of 128 bytes, panels of 64 columns (W^T: [128 channels][64 tokens], one panel); they go to
+// the record by bulk copies.
+//
+// What bounds it: B=4 T=8192 H=32 (16384 chunks): 820 us with the general products for every chunk and rows loaded by the warps -> 448, the whole
+// forward 1076 -> 723; 2.1 GB of rows and records are 327 us at the copy rate.  16.5 K cycles per chunk, two chunks at a time (24 K): 1.2 K
+// waiting for rows, 2.0 K prefix sums and norms, 2.0 K tiles, 1.4 K for the product, 3.8 K inverse, 0.9 K for W^T; issue slots 51 %.  With loads by
+// the warps into registers a chunk ahead they wait 6 K cycles for room in what the tiles leave of the L1 (690 us).  Fewer instructions in the
+// prefix sums and norms (packed adds, one barrier with a vote) made it 2 to 7 % slower.  Output error against float64 (2-norm, 64 heads,
+// T=500): 4.3e-3 -> 3.8e-3, one rounding per operand instead of two; T=1: 2.7e-3 -> 3.0e-3, where the general form's factors are 1.
+constexpr int kIntraThreads = kThreads + 32;
+constexpr int IS_A = 0, IS_Q = 8192, IS_B = 16384, IS_PANEL = 24576;   // k^ e^G | q^ e^G | Kd of 64 channels, then of the other 64; A and B by turns
+constexpr int IS_G = 2 * IS_PANEL;         // log decay as it arrives [64][128]
+constexpr int IS_AQK = IS_G + 32768;
+constexpr int IS_TOT = IS_AQK + 8192;      // decay of each eight rows [8][128]
+constexpr int IS_X = 96256;                // k^ e^{-G}, then A_kk and its inverse [64][68] fp32, then T diag(beta), two terms
+constexpr int IS_BETA = IS_X + 64 * LDT * 4;
+struct IntraCtl {
+  float beta[64], rk[64], rq[64];
+  uint64_t bar[2], full, free;
+  uint32_t tmem_base;
+  int wide, abort;
+};
+constexpr int IS_TOTAL = IS_BETA + sizeof(IntraCtl);
+// the arrays of the general products: A_kk where the inverse expects it
+constexpr int IG_K = 64 * LDF * 4, IG_Q = IG_K + 64 * LDH * 2, IG_T = IG_Q + 64 * LDH * 2, IG_AQK = IG_T + 64 * LDT * 4;
+static_assert(IS_TOT + 4096 <= IS_X && IS_X % 1024 == 0 && IG_AQK + 64 * LDQ * 2 <= IS_X, "shared memory");
+static_assert(2 * (IS_TOTAL + 1024) <= 233472, "two CTAs per SM");
+
+static __device__ __noinline__ void general_products_call(uint8_t* smem, int tid) {   // the rare way
+  const IntraCtl& ctl = *reinterpret_cast<const IntraCtl*>(smem + IS_BETA);
+  general_products(reinterpret_cast<const float*>(smem), reinterpret_cast<const __nv_bfloat16*>(smem + IG_K),
+                   reinterpret_cast<const __nv_bfloat16*>(smem + IG_Q), reinterpret_cast<float*>(smem + IS_X), reinterpret_cast<float*>(smem + IG_T),
+                   reinterpret_cast<__nv_bfloat16*>(smem + IG_AQK), ctl.rk, ctl.rq, tid);
+}
+
+template <class Params>
+__global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_constant__ Params P) {
+  constexpr bool kPacked = std::is_same<Params, IntraPackedParams>::value;
+  const FwdParams& p = P.p;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  IntraCtl& ctl = *reinterpret_cast<IntraCtl*>(smem + IS_BETA);
+  float* sX = reinterpret_cast<float*>(smem + IS_X);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  if (warp == 8) {
+    tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), 128);
+    tc::tmem_relinquish();
+  }
+  if (tid == 0) {
+    tc::mbar_init(tc::smem_u32(&ctl.bar[0]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.bar[1]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.full), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.free), 1);
+    tc::fence_mbar_init();
+    ctl.abort = 0;
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  pdl_entry();
+  const uint32_t tb = ctl.tmem_base, sb = tc::smem_u32(smem);
+  auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
+    const uint32_t at = tc::smem_u32(&bar);
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp == 8);
+  };
+  // chunk number -> batch, head, first token, rows of it that exist, number of its record
+  struct At { int b, h, tok, rows; int64_t rec; };
+  auto place = [&](int c) -> At {
+    At x;
+    if constexpr (kPacked) {   // heads outermost in the grid, innermost but one in the records
+      x.b = 0;
+      x.h = c / P.seqs.chunks;
+      c -= x.h * P.seqs.chunks;
+      int lo = 0, hi = P.seqs.n - 1;   // the last sequence that starts at or before chunk c
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (P.seqs.first[mid] <= c) lo = mid; else hi = mid - 1;
+      }
+      const int n = c - P.seqs.first[lo], T = P.seqs.len[lo];
+      x.tok = P.seqs.start[lo] + n * kC;
+      x.rows = min(kC, T - n * kC);
+      x.rec = (int64_t)P.seqs.first[lo] * p.map.H + (int64_t)x.h * ((T + kC - 1) / kC) + n;
+    } else {
+      const int nchunks = (p.map.T + kC - 1) / kC, unit = c / nchunks, n = c - unit * nchunks;
+      x.b = unit / p.map.H; x.h = unit - x.b * p.map.H;
+      x.tok = n * kC;
+      x.rows = min(kC, p.map.T - n * kC);
+      x.rec = c;
+    }
+    return x;
+  };
+
+  if (warp == 8) {
+    // =========================== ISSUING WARP (one thread) ==================================================================
+    auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
+    auto load_g = [&](const At& x) {
+      const uint32_t bar = tc::smem_u32(&ctl.full), bytes = p.g_dt == DR_BF16 ? 16384 : 32768;
+      tc::mbar_arrive_expect_tx(bar, 32768 + bytes);
+      tc::tma_load_4d(sb + IS_G, &P.tg, 0, x.tok, x.h, x.b, bar);
+    };
+    auto load_qk = [&](const At& x, int k_at) {
+      const uint32_t bar = tc::smem_u32(&ctl.full);
+      const int hq = p.map.hq(x.h);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        tc::tma_load_4d(sb + e * IS_PANEL + k_at, &P.tk, 64 * e, hq, x.tok, x.b, bar);
+        tc::tma_load_4d(sb + e * IS_PANEL + IS_Q, &P.tq, 64 * e, hq, x.tok, x.b, bar);
+      }
+    };
+    if (P.use_tma && tc::elect_one()) {
+      const At x = place(blockIdx.x);
+      load_g(x);
+      load_qk(x, IS_A);
+    }
+    __syncwarp();
+    uint32_t ph = 0, ph0 = 0;   // ph: chunks so far; also which of the two places has k^ e^G
+#pragma unroll 1
+    for (int c = blockIdx.x; c < P.chunks; c += gridDim.x, ph ^= 1) {
+      const At x = place(c);
+      uint8_t* rec = P.ws + x.rec * WS_REC;
+      const int next = c + gridDim.x;
+      const uint32_t kg = ph ? IS_B : IS_A, kd = ph ? IS_A : IS_B;
+      asm volatile("bar.sync 2, 288;" ::: "memory");
+      tc::tc_fence_after();
+      const bool wide = ctl.wide;
+      if (tc::elect_one()) {
+        if (!wide) {   // rows: k^ e^G, q^ e^G or the other way round
+          const uint64_t ad = tc::smem_desc_sw128(sb + (ph ? IS_Q : IS_A), 128, 1024), bd = tc::smem_desc_sw128(sb + IS_X, 128, 1024);
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            tc::mma_ss(tb, adv(ad, (ks >> 2) * IS_PANEL + (ks & 3) * 32), adv(bd, (ks >> 2) * 8192 + (ks & 3) * 32), tc::idesc_bf16(128, 64, 0, 0), ks > 0);
+          tc::mma_commit(tc::smem_u32(&ctl.bar[0]));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          tc::bulk_s2g(rec + WS_KD + 8192 * e, sb + e * IS_PANEL + kd, 8192);
+          tc::bulk_s2g(rec + WS_QG + 8192 * e, sb + e * IS_PANEL + IS_Q, 8192);
+        }
+        if (wide) tc::bulk_s2g(rec + WS_AQK, sb + IS_AQK, 8192);
+        tc::bulk_commit();
+        if (P.use_tma && next < P.chunks) {
+          const At y = place(next);
+          load_g(y);
+          if (!wide) wait_bar(ctl.bar[0], ph0);
+          tc::bulk_wait_read_all();
+          load_qk(y, kd);
+        }
+      }
+      __syncwarp();
+      if (!wide) {
+        ph0 ^= 1;
+        asm volatile("bar.sync 3, 288;" ::: "memory");
+        if (tc::elect_one()) tc::bulk_s2g(rec + WS_AQK, sb + IS_AQK, 8192);
+        __syncwarp();
+      }
+      asm volatile("bar.sync 4, 288;" ::: "memory");
+      tc::tc_fence_after();
+      if (tc::elect_one()) {
+        // W^T = (k^ e^G)^T (T diag(beta))^T: sixteen tokens at a time, N = the rows that they reach
+        const uint64_t ad = tc::smem_desc_sw128(sb + kg, IS_PANEL, 1024), bd = tc::smem_desc_sw128(sb + IS_X, 128, 1024);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const uint32_t id = tc::idesc_bf16(128, 64 - 16 * ks, 1, 0);
+          tc::mma_ss(tb + 64 + 16 * ks, adv(ad, ks * 2048), adv(bd, ks * (2048 + 32)), id, ks > 0);
+          tc::mma_ss(tb + 64 + 16 * ks, adv(ad, ks * 2048), adv(bd, 8192 + ks * (2048 + 32)), id, 1);
+        }
+        tc::mma_commit(tc::smem_u32(&ctl.bar[1]));
+        tc::bulk_s2g(rec + WS_TB, sb + IS_X, 8192);
+      }
+      __syncwarp();
+      asm volatile("bar.sync 5, 288;" ::: "memory");
+      if (tc::elect_one()) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) tc::bulk_s2g(rec + WS_W + 8192 * e, sb + e * IS_PANEL + kg, 8192);
+        tc::bulk_commit();
+        tc::bulk_wait_read_all();
+        sm100::mbar_arrive(tc::smem_u32(&ctl.free));   // everything but the next chunk's rows may be written over
+      }
+      __syncwarp();
+    }
+    tc::bulk_wait_all();
+  } else {
+    // =========================== WORKERS ====================================================================================
+    auto sync = []() { sm100::group_sync(1); };
+    auto hand_over = [](int id) {
+      tc::fence_async_smem();
+      tc::tc_fence_before();
+      asm volatile("bar.arrive %0, 288;" ::"r"(id) : "memory");
+    };
+    constexpr float kLog2e = 1.4426950408889634f;
+    uint32_t ph = 0, ph0 = 0;
+#pragma unroll 1
+    for (int c = blockIdx.x; c < P.chunks; c += gridDim.x, ph ^= 1) {
+      const int kg = ph ? IS_B : IS_A, kd = ph ? IS_A : IS_B;
+      // byte of this lane's four channels in row 8 warp + r of a panel: + 128 r, piece ^ r
+      const int piece = (lane & 15) >> 1, own = (lane >> 4) * IS_PANEL + warp * 1024 + (lane & 1) * 8;
+      auto entry = [&](int base, int r) { return reinterpret_cast<uint2*>(smem + base + own + r * 128 + ((piece ^ r) << 4)); };
+      // ---- the warp's rows, prefix sums over them, norm factors ------------------------------------------------------------------------
+      float4 G[8];
+      {
+        const At x = place(c);
+        const int rows = x.rows - 8 * warp, tok = x.tok + 8 * warp;
+        const int64_t s_tok = p.map.tok(1), s_at = p.map.base(x.b, x.h, 1) + tok * s_tok;
+        const float bt = lane < 8 && lane < rows ? p.beta[s_at + lane * s_tok] : 0.f;
+        if (P.use_tma) {
+          wait_bar(ctl.full, ph);
+          if (p.g_dt == DR_BF16) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              const uint2 u = *reinterpret_cast<const uint2*>(smem + IS_G + (8 * warp + r) * 256 + lane * 8);
+              const float2 y = bf2(u.x), z = bf2(u.y);
+              G[r] = make_float4(y.x, y.y, z.x, z.y);
+            }
+          } else {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) G[r] = *reinterpret_cast<const float4*>(smem + IS_G + (8 * warp + r) * 512 + lane * 16);
+          }
+          if (kPacked && rows < 8) {   // rows of the next sequence
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+              if (r >= rows) { *entry(IS_Q, r) = *entry(kg, r) = make_uint2(0u, 0u); G[r] = make_float4(0.f, 0.f, 0.f, 0.f); }
+          }
+        } else {   // arrays that TMA does not take, and one decay per token
+          wait_bar(ctl.free, ph ^ 1);
+          const int64_t st = p.map.tok_qk(kD), gst = p.map.tok(kD);
+          const int64_t at = p.map.base_qk(x.b, x.h, kD) + tok * st + 4 * lane, g_at = p.map.base(x.b, x.h, kD) + tok * gst + 4 * lane;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            uint2 q = make_uint2(0u, 0u), k = q;
+            float y[4] = {0.f, 0.f, 0.f, 0.f};
+            if (r < rows) {
+              q = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + at + r * st);
+              k = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at + r * st);
+              if (p.variant == DR_KDA) ld4(p.g, g_at + r * gst, p.g_dt, y);
+              else if (p.variant == DR_GATED) y[0] = y[1] = y[2] = y[3] = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
+            }
+            G[r] = make_float4(y[0], y[1], y[2], y[3]);
+            *entry(IS_Q, r) = q;
+            *entry(kg, r) = k;
+          }
+        }
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          acc.x += G[r].x * kLog2e; acc.y += G[r].y * kLog2e; acc.z += G[r].z * kLog2e; acc.w += G[r].w * kLog2e;
+          G[r] = acc;
+        }
+        *reinterpret_cast<float4*>(smem + IS_TOT + warp * 512 + lane * 16) = acc;
+        // the sums are scattered over the lanes as they are reduced (16 shuffles), so that each lane takes one square root and one quotient
+        float ss[16];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const uint2 q = *entry(IS_Q, r), k = *entry(kg, r);
+          const float2 q0 = bf2(q.x), q1 = bf2(q.y), k0 = bf2(k.x), k1 = bf2(k.y);
+          ss[r] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
+          ss[8 + r] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
+        }
+#pragma unroll
+        for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
+#pragma unroll
+          for (int i = 0; i < m; ++i) {
+            const bool up = lane & o;
+            const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
+            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        }
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+        if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
+          const float top = lane < 16 ? p.scale : 1.f;
+          (lane < 16 ? ctl.rq : ctl.rk)[8 * warp + ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+        }
+        if (lane < 8) ctl.beta[8 * warp + lane] = bt;
+        if (warp == 0) {   // (the record's tail; its address is not worth keeping)
+          sync();
+          float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
+            run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
+          }
+          *reinterpret_cast<float4*>(P.ws + x.rec * WS_REC + WS_EGL + 16 * lane) = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
+        } else {
+          sync();
+        }
+      }
+      bool wide;   // the same in every warp: each sees all channels
+      float4 el;   // e^{G_L}
+      {
+        float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
+        float most = 0.f;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          if (s == warp) pre = run;
+          const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
+          run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
+          most = fmaxf(most, fmaxf(fmaxf(fabsf(run.x), fabsf(run.y)), fmaxf(fabsf(run.z), fabsf(run.w))));
+        }
+        const float all = (run.x + run.y) + (run.z + run.w);   // NaN if any sum was
+        wide = __any_sync(0xffffffffu, !(most <= 64.f && all == all));
+        el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
+#pragma unroll
+        for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
+      }
+      if (tid == 0) ctl.wide = wide;
+      wait_bar(ctl.free, ph ^ 1);   // the chunk before has left
+      if (!wide) {
+        // ---- the tiles ------------------------------------------------------------------------------------------------------------------
+        const float2 el0 = make_float2(el.x, el.y), el1 = make_float2(el.z, el.w);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float2 g0 = make_float2(G[r].x, G[r].y), g1 = make_float2(G[r].z, G[r].w);
+          const float2 e0 = ex2x2(g0), e1 = ex2x2(g1), i0 = make_float2(ex2(-g0.x), ex2(-g0.y)), i1 = make_float2(ex2(-g1.x), ex2(-g1.y));
+          const float fk = ctl.rk[8 * warp + r], fq = ctl.rq[8 * warp + r];
+          const float2 rk = make_float2(fk, fk), rq = make_float2(fq, fq);
+          const uint2 q = *entry(IS_Q, r), k = *entry(kg, r);
+          const float2 k0 = mul2(bf2(k.x), rk), k1 = mul2(bf2(k.y), rk);
+          const float2 x0 = mul2(k0, i0), x1 = mul2(k1, i1);
+          const float2 a0 = mul2(k0, e0), a1 = mul2(k1, e1), b0 = mul2(mul2(bf2(q.x), rq), e0), b1 = mul2(mul2(bf2(q.y), rq), e1);
+          const float2 d0 = mul2(x0, el0), d1 = mul2(x1, el1);
+          *entry(kg, r) = make_uint2(tc::pack_bf16(a0.x, a0.y), tc::pack_bf16(a1.x, a1.y));
+          *entry(IS_Q, r) = make_uint2(tc::pack_bf16(b0.x, b0.y), tc::pack_bf16(b1.x, b1.y));
+          *entry(kd, r) = make_uint2(tc::pack_bf16(d0.x, d0.y), tc::pack_bf16(d1.x, d1.y));
+          *reinterpret_cast<uint2*>(smem + IS_X + (lane >> 4) * 8192 + warp * 1024 + (lane & 1) * 8 + r * 128 + ((piece ^ r) << 4)) =
+              make_uint2(tc::pack_bf16(x0.x, x0.y), tc::pack_bf16(x1.x, x1.y));
+        }
+      } else {
+        // ---- any decay: through the arrays of the general products ---------------------------------------------------------------------------
+        uint2 q[8], k[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          q[r] = *entry(IS_Q, r);
+          k[r] = *entry(kg, r);
+        }
+        sync();   // every warp has its rows and the decays
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int row = 8 * warp + r;
+          *reinterpret_cast<float4*>(smem + (row * LDF + 4 * lane) * 4) = G[r];
+          *reinterpret_cast<uint2*>(smem + IG_K + (row * LDH + 4 * lane) * 2) = k[r];
+          *reinterpret_cast<uint2*>(smem + IG_Q + (row * LDH + 4 * lane) * 2) = q[r];
+        }
+        sync();
+        general_products_call(smem, tid);
+        uint4 tq[4], td[4], tk[4], aq[2];
+        const float* sG = reinterpret_cast<const float*>(smem);
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int i = tid + kThreads * it, row = i >> 4, col = (i & 15) * 8;
+          decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, *reinterpret_cast<const uint4*>(smem + IG_Q + (row * LDH + col) * 2),
+                        *reinterpret_cast<const uint4*>(smem + IG_K + (row * LDH + col) * 2), ctl.rq[row], ctl.rk[row], tq[it], td[it], tk[it]);
+        }
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+          const int i = tid + kThreads * it, row = i >> 3, col = (i & 7) * 8;
+          aq[it] = *reinterpret_cast<const uint4*>(smem + IG_AQK + (row * LDQ + col) * 2);
+          uint32_t* w = reinterpret_cast<uint32_t*>(&aq[it]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {   // keep j <= row
+            const int j = col + 2 * e;
+            if (j > row) w[e] = 0u;
+            else if (j + 1 > row) w[e] &= 0x0000ffffu;
+          }
+        }
+        sync();
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int i = tid + kThreads * it, row = i >> 4, col = (i & 15) * 8, off = (col >> 6) * IS_PANEL + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4);
+          *reinterpret_cast<uint4*>(smem + kg + off) = tk[it];
+          *reinterpret_cast<uint4*>(smem + IS_Q + off) = tq[it];
+          *reinterpret_cast<uint4*>(smem + kd + off) = td[it];
+        }
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+          const int i = tid + kThreads * it, row = i >> 3, col = (i & 7) * 8;
+          *reinterpret_cast<uint4*>(smem + IS_AQK + row * 128 + (((col >> 3) ^ (row & 7)) << 4)) = aq[it];
+        }
+      }
+      hand_over(2);
+      const int row = 32 * (warp & 3) + lane, hf = warp >> 2;   // this thread's row of the products, half of their columns
+      const uint32_t ta = tb + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * hf;
+      if (!wide) {
+        // ---- A_kk, A_qk (rows 0 .. 63 and 64 .., by turns) ------------------------------------------------------------------------------------
+        wait_bar(ctl.bar[0], ph0);
+        ph0 ^= 1;
+        tc::tc_fence_after();
+        uint32_t x[32];
+        tc::tmem_ld32(ta, x);
+        tc::tc_wait_ld();
+        const int i = row & 63, last = i - 32 * hf;
+        if ((uint32_t)(row >> 6) == ph) {   // over k^ e^{-G}, which has been read; what is above the diagonal is not used
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            *reinterpret_cast<uint4*>(sX + i * LDT + 32 * hf + 4 * e) = make_uint4(x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint32_t w[4];
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+              const int j = 8 * e + 2 * f;
+              w[f] = tc::pack_bf16(j <= last ? __uint_as_float(x[j]) : 0.f, j + 1 <= last ? __uint_as_float(x[j + 1]) : 0.f);
+            }
+            *reinterpret_cast<uint4*>(smem + IS_AQK + i * 128 + (((4 * hf + e) ^ (i & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        hand_over(3);
+        sync();
+      }
+      // ---- T = (I + diag(beta) A_kk)^-1 in place, then T diag(beta) as two terms ---------------------------------------------------------------
+      sm100::block_inverse_64(sX, ctl.beta, sX, tid);
+      {
+        uint4 hi[2], lo[2];
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+          int r, col;
+          piece64(tid + kThreads * it, r, col);   // eight rows to a quarter warp: the 16-byte reads are free of bank conflicts
+          float a[8], bb[8];
+          *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sX + r * LDT + col);
+          *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sX + r * LDT + col + 4);
+          *reinterpret_cast<float4*>(bb) = *reinterpret_cast<const float4*>(ctl.beta + col);
+          *reinterpret_cast<float4*>(bb + 4) = *reinterpret_cast<const float4*>(ctl.beta + col + 4);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = col + 2 * e <= r ? a[2 * e] * bb[2 * e] : 0.f, y = col + 2 * e + 1 <= r ? a[2 * e + 1] * bb[2 * e + 1] : 0.f;
+            const uint32_t u = tc::pack_bf16(x, y);
+            const float2 f = bf2(u);
+            reinterpret_cast<uint32_t*>(&hi[it])[e] = u;
+            reinterpret_cast<uint32_t*>(&lo[it])[e] = tc::pack_bf16(x - f.x, y - f.y);
+          }
+        }
+        sync();
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+          int r, col;
+          piece64(tid + kThreads * it, r, col);
+          const int off = r * 128 + (((col >> 3) ^ (r & 7)) << 4);
+          *reinterpret_cast<uint4*>(smem + IS_X + off) = hi[it];
+          *reinterpret_cast<uint4*>(smem + IS_X + 8192 + off) = lo[it];
+        }
+      }
+      hand_over(4);
+      // ---- W^T, over k^ e^G ------------------------------------------------------------------------------------------------------------------
+      wait_bar(ctl.bar[1], ph);
+      tc::tc_fence_after();
+      {
+        uint32_t x[32];
+        tc::tmem_ld32(ta + 64, x);
+        tc::tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint32_t w[4];
+#pragma unroll
+          for (int f = 0; f < 4; ++f) w[f] = tc::pack_bf16(__uint_as_float(x[8 * e + 2 * f]), __uint_as_float(x[8 * e + 2 * f + 1]));
+          *reinterpret_cast<uint4*>(smem + kg + (row >> 6) * IS_PANEL + (row & 63) * 128 + (((4 * hf + e) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      hand_over(5);
     }
   }
+  tc::tc_fence_before();
   __syncthreads();
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int piece = tid + kThreads * it;
-    int row, col;
-    piece128(piece, row, col);
-    *reinterpret_cast<uint4*>(rec + WS_W + piece * 16) = *reinterpret_cast<const uint4*>(sWst + row * LDH + col);
-  }
+  if (warp == 8) tc::tmem_dealloc(tb, 128);
+  if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
 // ---- state kernel ----------------------------------------------------------------------------------------------
@@ -727,11 +1080,13 @@ constexpr uint32_t TM_COLS = 512;
 // shared memory: two record buffers, two V tiles (two swizzled panels of 64 columns each, straight from the input by
 // TMA), then the fp32 output staging tile [64][128]
 constexpr int V_PANEL = 64 * 128, V_TILE = 2 * V_PANEL;
-constexpr int ST_V = 2 * WS_REC;
+constexpr int ST_REC = (WS_REC + 1023) / 1024 * 1024;
+constexpr int ST_V = 2 * ST_REC;
 constexpr int ST_O = ST_V + 2 * V_TILE;
 static_assert(ST_V % 1024 == 0, "swizzled tiles");
 constexpr int ST_TOTAL = ST_O + 64 * 128 * 4;
 
+static_assert(sizeof(IntraPackedParams) <= 4096, "kernel parameters");
 struct StateCtl {
   uint64_t full[2], go1, go2, go3, bar1, bar2;
   uint32_t tmem_base;
@@ -822,7 +1177,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
       auto issue_load = [&](int m) {
         const uint32_t bar = tc::smem_u32(&ctl.full[m & 1]);
         tc::mbar_arrive_expect_tx(bar, WS_REC + V_TILE);
-        const uint32_t dst = tc::smem_u32(smem + (m & 1) * WS_REC), dv = tc::smem_u32(smem + ST_V + (m & 1) * V_TILE);
+        const uint32_t dst = tc::smem_u32(smem + (m & 1) * ST_REC), dv = tc::smem_u32(smem + ST_V + (m & 1) * V_TILE);
         const uint8_t* src = recs + (int64_t)m * WS_REC;
         tc::tma_load_4d(dv, &P.tv, 0, h, tok0 + m * kC, b, bar);
         tc::tma_load_4d(dv + V_PANEL, &P.tv, 64, h, tok0 + m * kC, b, bar);
@@ -834,11 +1189,11 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
       if (nchunks > 1) issue_load(1);
       const uint32_t id_n64 = tc::idesc_bf16(128, 64, 0, 0);
       const uint32_t id_n64_amn = tc::idesc_bf16(128, 64, 1, 0);
-      const uint32_t id_n64_neg = id_n64 | (1u << 13);
+      const uint32_t id_n64_neg = tc::idesc_bf16(128, 64, 0, 1) | (1u << 13);
       const uint32_t id_n128_bmn = tc::idesc_bf16(128, 128, 0, 1);
       for (int n = 0; n < nchunks; ++n) {
         const int s = n & 1;
-        const uint8_t* st = smem + s * WS_REC;
+        const uint8_t* st = smem + s * ST_REC;
         const uint32_t aW = tc::smem_u32(st + WS_W), aQg = tc::smem_u32(st + WS_QG), aKd = tc::smem_u32(st + WS_KD);
         const uint32_t aV = tc::smem_u32(smem + ST_V + s * V_TILE), aTb = tc::smem_u32(st + WS_TB), aAqk = tc::smem_u32(st + WS_AQK);
         wait_bar(&ctl.full[s], (n >> 1) & 1);
@@ -848,14 +1203,14 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
           const uint64_t ad = tc::smem_desc_sw128(aV + ks * 2048, V_PANEL, 1024);   // MN-major, 16 chunk rows per step
-          const uint64_t bd = tc::smem_desc(aTb + ks * 256, 128, A_RBS);
+          const uint64_t bd = tc::smem_desc_sw128(aTb + ks * 32, 128, 1024);
           tc::mma_ss(tbase + TM_DU + 64 * s, ad, bd, id_n64_amn, ks > 0);
         }
         wait_bar(&ctl.go1, n & 1);
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {   // Vn^T = U^T - S^T W^T
-          const uint64_t bd = tc::smem_desc(aW + ks * 256, 128, RBS);
+          const uint64_t bd = tc::smem_desc_sw128(aW + ks * 2048, 16384, 1024);   // MN-major
           tc::mma_ts(tbase + TM_DU + 64 * s, tbase + TM_SB + ks * 8, bd, id_n64_neg, 1);
         }
         tc::mma_commit(tc::smem_u32(&ctl.bar1));
@@ -863,19 +1218,19 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {   // Dq = S^T Qg^T
-          const uint64_t bd = tc::smem_desc(aQg + ks * 256, 128, RBS);
+          const uint64_t bd = tc::smem_desc_sw128(aQg + (ks >> 2) * 8192 + (ks & 3) * 32, 128, 1024);
           tc::mma_ts(tbase + TM_DQ, tbase + TM_SB + ks * 8, bd, id_n64, ks > 0);
         }
         wait_bar(&ctl.go3, n & 1);
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {   // S^T += Vn^T Kd   (Kd MN-major)
-          const uint64_t bd = tc::smem_desc(aKd + ks * 2 * RBS, RBS, 128);
+          const uint64_t bd = tc::smem_desc_sw128(aKd + ks * 2048, 8192, 1024);
           tc::mma_ts(tbase + TM_S, tbase + TM_VA + ks * 8, bd, id_n128_bmn, 1);
         }
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {   // Do = Vn^T A_qk^T
-          const uint64_t bd = tc::smem_desc(aAqk + ks * 256, 128, A_RBS);
+          const uint64_t bd = tc::smem_desc_sw128(aAqk + ks * 32, 128, 1024);
           tc::mma_ts(tbase + TM_DU + 64 * s, tbase + TM_VA + ks * 8, bd, id_n64, ks > 0);
         }
         tc::mma_commit(tc::smem_u32(&ctl.bar2));
@@ -958,7 +1313,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
 
     for (int n = 0; n < nchunks; ++n) {
       const int s = n & 1;
-      const float* sEGL = reinterpret_cast<const float*>(smem + s * WS_REC + WS_EGL);
+      const float* sEGL = reinterpret_cast<const float*>(smem + s * ST_REC + WS_EGL);
       wait_bar(&ctl.full[s], (n >> 1) & 1);
       if (n > 0) {
         wait_bar(&ctl.bar2, (n - 1) & 1);   // the previous chunk's state update and Do have completed
@@ -1237,7 +1592,7 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (attr_dev != dev) {
-    e = cudaFuncSetAttribute(intra_kernel<IntraTransParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    e = cudaFuncSetAttribute(intra_trans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<2>::kTotal);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<4>::kTotal);
     if (e != cudaSuccess) return e;
@@ -1252,7 +1607,7 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;
   P.of = reinterpret_cast<float4*>(w); w += nc * kTrO;
   P.el = reinterpret_cast<float*>(w);
-  e = launch_pdl(intra_kernel<IntraTransParams>, dim3((unsigned)nc), dim3(kThreads), IN_TOTAL, stream, P);
+  e = launch_pdl(intra_trans_kernel, dim3((unsigned)nc), dim3(kThreads), IN_TOTAL, stream, P);
   if (e != cudaSuccess) return e;
   // 16 columns per CTA while the slices fit one wave: the chain's length is what counts
   if (units <= 6) return launch_pdl(trans_state_kernel<2, false>, dim3((unsigned)(units * 8)), dim3(kTrThreads<false>), 0, stream, P);   // see the kernel
@@ -1270,7 +1625,7 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   if (attr_dev != dev) {
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(intra_kernel<IP>, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    e = cudaFuncSetAttribute(intra_kernel<IP>, cudaFuncAttributeMaxDynamicSharedMemorySize, IS_TOTAL);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(state_kernel<SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_TOTAL);
     if (e != cudaSuccess) return e;
@@ -1279,9 +1634,12 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   I.p = p;
   S.p = p;
   S.ws = I.ws = reinterpret_cast<uint8_t*>(workspace);
-  I.resident = 2 * sms;
+  I.chunks = (int)chunk_units;
+  I.use_tma = p.variant == DR_KDA && sm100::make_panel_map(&I.tq, p.q, p.map.B, p.map.Hq, p.map.T, p.map.bthd != 0) &&
+              sm100::make_panel_map(&I.tk, p.k, p.map.B, p.map.Hq, p.map.T, p.map.bthd != 0) &&
+              sm100::make_output_map(&I.tg, const_cast<void*>(p.g), p.map, p.g_dt == DR_BF16 ? 2 : 4);
   if (!sm100::make_panel_map(&S.tv, p.v, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
-  e = launch_pdl(intra_kernel<IP>, dim3((unsigned)chunk_units), dim3(kThreads), IN_TOTAL, stream, I);
+  e = launch_pdl(intra_kernel<IP>, dim3((unsigned)std::min<int64_t>(chunk_units, 2 * sms)), dim3(kIntraThreads), IS_TOTAL, stream, I);
   if (e != cudaSuccess) return e;
   if (after_intra && (e = cudaEventRecord(after_intra, stream)) != cudaSuccess) return e;
   S.use_tma_out = p.o != nullptr && sm100::make_output_map(&S.to, p.o, p.map, p.out_dt == DR_BF16 ? 2 : 4);

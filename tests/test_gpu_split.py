@@ -76,6 +76,20 @@ def test_kda_split_strong_decay(decay):
     assert _rel(o, ro) <= BF16_TOL and _rel(hT, rS) <= BF16_TOL
 
 
+@pytest.mark.parametrize("nats", [44.3, 44.4])
+def test_kda_narrow_and_wide_chunks(nats):
+    """Chunks whose decay stays below 2^64 (44.36 nats) take one product, the others the 16-row form; a positive log decay
+    takes the second, too.  400 chunks: a CTA works on several, of both kinds, one after the other."""
+    H, T = 100, 250
+    inp = O.make_inputs("kda", 1, H, T, 128, 128, seed=11, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["g"][:, 1::3, 64:192, 5] = -nats / 64
+    inp["g"][:, 2::3, 130, 7] = 0.05
+    inp["g"][:, ::7, 200, 9] = -1e4
+    o, hT = _run("kda", inp, "split")
+    ro, rS = _truth("kda", inp)
+    assert _rel(o, ro) <= BF16_TOL and _rel(hT, rS) <= BF16_TOL
+
+
 def test_kda_split_bf16_output_and_bthd():
     inp = O.make_inputs("kda", 2, 3, 130, 128, 128, seed=9, io_dtype=torch.bfloat16, h0_std=0.02)
     ro, rS = _truth("kda", inp)
