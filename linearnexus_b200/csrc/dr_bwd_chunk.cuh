@@ -15,17 +15,20 @@
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
 //                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
 //                 finalize kernel).  Scalar decays: local_sm100_kernel (dr_bwd_local_sm100.cuh), persistent, on tcgen05.  Per-channel
-//                 decays: local_kernel, one CTA per chunk, looping over four value slices with the sums over v in registers.
+//                 decays: local_sm100_kda_kernel (dr_bwd_local_kda.cuh), likewise, for chunks that decay by at most 2^16, and for the others
+//                 local_kernel, looping over four value slices with the sums over v in registers.
 //
 // The one-CTA-per-sequence-slice adjoint it replaces here walked all of a chunk's work in sequence (B=2, T=4096, H=16:
 // 1.26 ms; with per-channel decay 12 ms on the CUDA cores) and stored four fp32 copies of dq^, dk^.
 //
 // DeltaNet / Gated DeltaNet: products on tcgen05 with two bf16 terms per float32 operand (16 bits); in pre_kernel mma.sync bf16 for the exact
-// ones of X and A and one tf32 product for W, Y and N.  KDA: mma.sync, three tf32 products per pair (x = hi + lo; see dr_tf32.cuh), i.e.
-// float32 precision, as the CUDA-core adjoint it replaces.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
+// ones of X and A and one tf32 product for W, Y and N.  KDA: three tf32 products per pair (x = hi + lo; see dr_tf32.cuh) on mma.sync, i.e.
+// float32 precision, as the CUDA-core adjoint it replaces, or three fp16 products of scaled operands on tcgen05.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
 // referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
 // decay range exceeds 2^64 is summed exactly.
 #pragma once
+
+#include <cuda_fp16.h>
 
 #include "dr_common.cuh"
 #include "dr_mma.cuh"
@@ -45,7 +48,7 @@ struct Params {
   const float* ckpt;    // [units][N][128][128] state at the start of every chunk
   float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]; scalar decays: kNTile bytes per chunk
   float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]; scalar decays: kYTile
-  float* xat;           // [units][N][3][64][64] X, A, T; scalar decays: A and T as two bf16 terms, the tiles of local_sm100_kernel
+  float* xat;           // [units][N][3][64][64] X, A, T; scalar decays: A and T as two bf16 terms, the tiles of local_sm100_kernel; KDA: see kXWide
   float* ds;            // [units][N][128][128] dS1
   float* el;            // [units][N][128] e^{G_L}
   float* norms;         // scalar decays: [units][N][2][64] norm factors of k and q
@@ -94,6 +97,52 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   }
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
+// Per-channel decays: what pre_kernel leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
+// whether the chunk is local_kernel's (a channel decays by more than 2^16, or a decay is positive) or local_sm100_kda_kernel's, and for
+// the latter the largest entries (bounds) of A, T, k^ and q^, in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
+// in fours, A and T as two fp16 terms in tiles.
+constexpr float kWideKda = 16.f;   // log2 units
+constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096, kXTop = 2097;
+enum { kTopA, kTopT, kTopK, kTopQ, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
+
+// the power of two that brings `top` to 2^13 .. 2^14 (none for zero and infinity); its inverse
+__device__ __forceinline__ float lift(uint32_t top) {
+  const uint32_t e = top >> 23;
+  return top == 0u || e == 255u ? 1.f : __uint_as_float(min(267u - e, 253u) << 23);
+}
+__device__ __forceinline__ float drop(uint32_t top) { return __uint_as_float((254u << 23) - __float_as_uint(lift(top))); }
+__device__ __forceinline__ uint32_t pack_h(float x, float y) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+  return r;
+}
+// two floats as two packed fp16 terms
+__device__ __forceinline__ void split2h(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = pack_h(x, y);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = pack_h(x - f.x, y - f.y);
+}
+// The chunks blockIdx.x, + gridDim.x, .. of one kind; warp-uniform, one read per 32 of them.
+template <bool WIDE>
+struct ChunkList {
+  int base;
+  uint32_t mask;
+  __device__ __forceinline__ ChunkList(const float* xat, int chunks, int lane) : base(blockIdx.x) { fetch(xat, chunks, lane); }
+  __device__ __forceinline__ void fetch(const float* xat, int chunks, int lane) {
+    const int64_t c = base + (int64_t)lane * gridDim.x;
+    mask = __ballot_sync(0xffffffffu, c < chunks && (__ldcg(xat + c * (3 * 64 * 64) + kXWide) != 0.f) == WIDE);
+  }
+  __device__ __forceinline__ int next(const float* xat, int chunks, int lane) {   // `chunks` behind the last
+    while (mask == 0u) {
+      if ((int64_t)base + 32 * gridDim.x >= chunks) return chunks;
+      base += 32 * gridDim.x;
+      fetch(xat, chunks, lane);
+    }
+    const int i = __ffs(mask) - 1;
+    mask &= mask - 1;
+    return base + i * (int)gridDim.x;
+  }
+};
 // =====================================================================================================================
 // pre_kernel
 // =====================================================================================================================
@@ -127,6 +176,10 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
   const int64_t chunk = (int64_t)unit * p.N + n;
 
+  bool wide = false;
+  float bound = 0.f, topA = 0.f;   // of a row of q^ or k^; of A
+  __shared__ uint32_t sTop[4];
+  if (KDA && tid < 4) sTop[tid] = 0u;
   // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
   {
     uint2 qr[8], kr[8];
@@ -142,6 +195,12 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         kr[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at);
         if constexpr (KDA) gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
       }
+    }
+    if constexpr (KDA) {
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(fmaxf(gr[i].x, gr[i].y), fmaxf(gr[i].z, gr[i].w)));
+      wide = m > 0.f;
     }
     float bt = 0.f, g_lo = 0.f, g_hi = 0.f;
     if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
@@ -177,8 +236,9 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
     }
     ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
     if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
-      const float top = lane < 16 ? p.scale : 1.f;
-      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+      const float top = lane < 16 ? p.scale : 1.f, nrm = sqrtf(ss[0]), m = p.l2norm ? top / (nrm + 1e-6f) : top;
+      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = m;
+      bound = fabsf(m * nrm);
     }
     if (lane < 8) sBeta[warp + 8 * lane] = bt;
     if (!KDA && warp == 0) {
@@ -189,7 +249,13 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   __syncthreads();
   if constexpr (KDA) {
     mma::scan_channels<kPreThreads, kD, LDG>(sG, sX, tid);
-    if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * LDG + tid]);
+    if (tid < 128) {
+      p.el[chunk * 128 + tid] = ex2(sG[63 * LDG + tid]);
+      wide |= !(sG[63 * LDG + tid] >= -kWideKda);
+      p.xat[chunk * (3 * 64 * 64) + kXNorms + (tid >> 5) * kXNormRow + lane] = (tid < 64 ? sRk : sRq - 64)[tid];
+    }
+    atomicMax(&sTop[kTopQ], __reduce_max_sync(0xffffffffu, lane < 16 ? __float_as_uint(bound) : 0u));
+    atomicMax(&sTop[kTopK], __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : __float_as_uint(bound)));
     if (tid < 64) { sFw[tid] = sBeta[tid] * sRk[tid]; }
   } else {
     const float gl = sGs[63];
@@ -246,10 +312,13 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         for (int e = 0; e < 4; ++e) {
           const int i = 16 * mt + g + 8 * (e >> 1), j = 8 * (nt0 + x) + 2 * t + (e & 1);
           sX[i * LDT + j] = j < i ? dk[x][e] * sRk[j] * sRk[i] : 0.f;
-          sA[i * 72 + j] = j <= i ? dq[x][e] * sRk[j] * sRq[i] : 0.f;
+          const float y = j <= i ? dq[x][e] * sRk[j] * sRq[i] : 0.f;
+          sA[i * 72 + j] = y;
+          topA = fmaxf(topA, fabsf(y));
         }
       }
     }
+    atomicMax(&sTop[kTopA], __reduce_max_sync(0xffffffffu, __float_as_uint(topA)));
   } else {
 #pragma unroll 1
   for (int tile = warp; tile < 20; tile += kPreThreads / 32) {   // raw bf16 rows: exact products
@@ -294,19 +363,20 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       sA[i * 72 + j] = j <= i ? aq * sRq[i] * sRk[j] : 0.f;
     }
   }
-  __syncthreads();
+  wide = __syncthreads_or(wide);
   // ---- X, A -> global (16 x 16 blocks at or below the diagonal), then T in place of X ----------------------------------------
   float* xat = p.xat + chunk * (3 * 64 * 64);
+  const bool as_rows = KDA && wide;
   for (int i = tid; i < 64 * 16; i += kPreThreads) {
     const int r = i >> 4, c4 = (i & 15) * 4;
     if ((c4 >> 4) <= (r >> 4)) {
-      // (scalar decays: columns in fours, so that a warp of the reader takes 32 rows of four at once)
-      *reinterpret_cast<float4*>(xat + (KDA ? r * 64 + c4 : c4 * 64 + 4 * r)) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
-      if constexpr (KDA) *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
+      // (columns in fours, so that a warp of the reader takes 32 rows of four at once)
+      *reinterpret_cast<float4*>(xat + (as_rows ? r * 64 + c4 : c4 * 64 + 4 * r)) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      if (as_rows) *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
     }
   }
-  // scalar decays: A, T as core matrices of 8 x 8, the blocks of eight rows next to each other; high terms, then low ones
-  auto put_tile = [&](const float* src, int ld, float* dst) {
+  // A, T as core matrices of 8 x 8, the blocks of eight rows next to each other; high terms, then low ones; of `s` times the entries as fp16 for KDA
+  auto put_tile = [&](const float* src, int ld, float* dst, float s) {
 #pragma unroll
     for (int x = 0; x < 512 / kPreThreads; ++x) {
       const int i = tid + kPreThreads * x, r = 8 * ((i >> 3) & 7) + (i & 7), c = 8 * (i >> 6);
@@ -314,30 +384,42 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       uint32_t h[4], l[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 y = ld2(src + r * ld + c + 2 * e);
-        split2(c + 2 * e <= r ? y.x : 0.f, c + 2 * e + 1 <= r ? y.y : 0.f, h[e], l[e]);
+        float2 y = ld2(src + r * ld + c + 2 * e);
+        if (c + 2 * e > r) y.x = 0.f;
+        if (c + 2 * e + 1 > r) y.y = 0.f;
+        if constexpr (KDA) split2h(s * y.x, s * y.y, h[e], l[e]); else split2(y.x, y.y, h[e], l[e]);
       }
       reinterpret_cast<uint4*>(dst)[i] = make_uint4(h[0], h[1], h[2], h[3]);
       reinterpret_cast<uint4*>(dst)[512 + i] = make_uint4(l[0], l[1], l[2], l[3]);
     }
   };
-  if constexpr (!KDA) {
-    put_tile(sA, 72, xat + 4096);
-    if (tid < 128) p.norms[chunk * 128 + tid] = (tid < 64 ? sRk : sRq - 64)[tid];
-  }
+  if (!as_rows) put_tile(sA, 72, xat + 4096, KDA ? lift(sTop[kTopA]) : 1.f);
+  if (!KDA && tid < 128) p.norms[chunk * 128 + tid] = (tid < 64 ? sRk : sRq - 64)[tid];
   __syncthreads();
   sm100::block_inverse_64(sX, sBeta, sX, tid);   // ends with a barrier
-  if constexpr (!KDA) put_tile(sX, LDT, xat + 8192);
-  for (int i = tid; KDA && i < 64 * 16; i += kPreThreads) {
-    const int r = i >> 4, c4 = (i & 15) * 4;
-    if ((c4 >> 4) <= (r >> 4)) {
-      float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
-      if (c4 + 0 > r) v.x = 0.f;
-      if (c4 + 1 > r) v.y = 0.f;
-      if (c4 + 2 > r) v.z = 0.f;
-      if (c4 + 3 > r) v.w = 0.f;
-      *reinterpret_cast<float4*>(xat + 8192 + r * 64 + c4) = v;
+  if constexpr (KDA) {
+    float m = 0.f;
+    for (int i = tid; i < 64 * 16; i += kPreThreads) {
+      const int r = i >> 4, c4 = (i & 15) * 4;
+      if ((c4 >> 4) <= (r >> 4)) {
+        float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+        if (c4 + 0 > r) v.x = 0.f;
+        if (c4 + 1 > r) v.y = 0.f;
+        if (c4 + 2 > r) v.z = 0.f;
+        if (c4 + 3 > r) v.w = 0.f;
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        if (wide) *reinterpret_cast<float4*>(xat + 8192 + r * 64 + c4) = v;
+      }
     }
+    if (!wide) {
+      atomicMax(&sTop[kTopT], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+      __syncthreads();
+      if (tid < 4) xat[kXTop + tid] = __uint_as_float(sTop[tid]);
+      put_tile(sX, LDT, xat + 8192, lift(sTop[kTopT]));
+    }
+    if (tid == 0) xat[kXWide] = wide ? 1.f : 0.f;
+  } else {
+    put_tile(sX, LDT, xat + 8192, 1.f);
   }
   // ---- W^T: rows = the warp's 16 channels, columns = tokens; W = T diag(beta) K^ e^G ----------------------------------------
   constexpr bool X3 = KDA;
@@ -812,7 +894,7 @@ struct LoSmem {
   static_assert(kTotal <= 232448 && gRaw + 2 * 64 * LDH * 2 <= kSc, "shared memory");
 };
 
-static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p) {
+static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Params p, const int chunks) {
   using L = LoSmem;
   pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
@@ -827,7 +909,11 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
   float *sEx = sU, *sUn = sU + 512;   // sums for dG_L [4][128], block flags
   float *sDq = F(L::kDot), *sDk = sDq + 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
+  ChunkList<true> list(p.xat, chunks, lane);
+#pragma unroll 1
+  for (int at_chunk = list.next(p.xat, chunks, lane); at_chunk < chunks; at_chunk = list.next(p.xat, chunks, lane)) {
+  __syncthreads();   // the chunk before is done with shared memory
+  const int unit = at_chunk / p.N, n = at_chunk % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
   const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);
@@ -1320,7 +1406,7 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
       if (grouped) {
         const int64_t at = (chunk * kC + i) * kD + c;
         *reinterpret_cast<float2*>(p.part + at) = make_float2(dQ[nt][e], dQ[nt][e + 1]);
-        *reinterpret_cast<float2*>(p.part + (int64_t)gridDim.x * (kC * kD) + at) = make_float2(dKr[nt][e], dKr[nt][e + 1]);
+        *reinterpret_cast<float2*>(p.part + (int64_t)chunks * (kC * kD) + at) = make_float2(dKr[nt][e], dKr[nt][e + 1]);
       } else {
         float2 qh = make_float2(0.f, 0.f), kh = qh;
         const uint32_t uq = *reinterpret_cast<const uint32_t*>(sRaw + i * LDH + c), uk = *reinterpret_cast<const uint32_t*>(sRaw + (64 + i) * LDH + c);
@@ -1359,12 +1445,14 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
 #pragma unroll
   for (int r = 0; r < 16; ++r)
     if (16 * s + r < rows) p.dg[gk_base + (int64_t)(t0 + 16 * s + r) * gk_tok + c] = loc[r] + post;
+  }
 }
 
 }  // namespace bwdc
 }  // namespace dr
 
 #include "dr_bwd_local_sm100.cuh"
+#include "dr_bwd_local_kda.cuh"
 
 namespace dr {
 namespace bwdc {
@@ -1406,8 +1494,9 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
   if (e == cudaSuccess && attr_dev != dev) {
     e = cudaFuncSetAttribute(pre_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem<KDA>());
     if (e == cudaSuccess)
-      e = KDA ? cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal)
+      e = KDA ? cudaFuncSetAttribute(local_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_TOTAL)
               : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
+    if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal);
     if (e == cudaSuccess)
       e = KDA ? cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem)
               : cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
@@ -1437,27 +1526,34 @@ inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* sta
   cudaError_t e = set_attributes<KDA>(&sms);
   if (e != cudaSuccess) return e;
   const int64_t chunks = units * p.N;
+  const dim3 grid((unsigned)(chunks < sms ? chunks : sms));
+  LocalParams lp;
+  lp.p = p; lp.chunks = (int)chunks; lp.status = status;
+  lp.n_tok = units * p.map.T; lp.n_part = 2 * chunks * (kC * kD);
+  const SeqMap& m = p.map;
+  auto panels = [&](CUtensorMap* t, const void* base, int heads) { return sm100::make_panel_map(t, base, m.B, heads, m.T, m.bthd != 0); };
+  if (!panels(&lp.to, p.d_o, m.H)) return cudaErrorInvalidValue;
   if constexpr (KDA) {
     e = launch_pdl(state_kernel, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem, stream, p);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(local_kernel, dim3((unsigned)chunks), dim3(kLoThreads), LoSmem::kTotal, stream, p);
   } else {
     ChainParams c;
     c.p = p;
     c.status = status;
-    if (!sm100::make_panel_map(&c.to, p.d_o, p.map.B, p.map.H, p.map.T, p.map.bthd != 0)) return cudaErrorInvalidValue;
+    c.to = lp.to;
     e = launch_pdl(chain_kernel, dim3((unsigned)(units * (kD / kChCols))), dim3(kChThreads), CH_TOTAL, stream, c);
-    if (e != cudaSuccess) return e;
-    LocalParams lp;
-    lp.p = p; lp.chunks = (int)chunks; lp.status = status;
-    lp.n_tok = units * p.map.T; lp.n_part = 2 * chunks * (kC * kD);
-    const SeqMap& m = p.map;
-    auto panels = [&](CUtensorMap* t, const void* base, int heads) { return sm100::make_panel_map(t, base, m.B, heads, m.T, m.bthd != 0); };
-    lp.to = c.to;
-    if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
-        !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
+  }
+  if (e != cudaSuccess) return e;
+  if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
+      !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
+    return cudaErrorInvalidValue;
+  if constexpr (KDA) {
+    if (!sm100::make_output_map(&lp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
       return cudaErrorInvalidValue;
-    return launch_pdl(local_sm100_kernel, dim3((unsigned)(chunks < sms ? chunks : sms)), dim3(kLtThreads), LT_TOTAL, stream, lp);
+    e = launch_pdl(local_sm100_kda_kernel, grid, dim3(kLtThreads), LK_TOTAL, stream, lp);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
+  } else {
+    return launch_pdl(local_sm100_kernel, grid, dim3(kLtThreads), LT_TOTAL, stream, lp);
   }
 }
 

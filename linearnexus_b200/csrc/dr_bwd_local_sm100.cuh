@@ -50,6 +50,7 @@ constexpr int LT_TOTAL = LT_CTL + sizeof(LtCtl);
 static_assert(LT_TOTAL <= 232448, "shared memory");
 struct alignas(64) LocalParams {
   CUtensorMap tq, tk, tv, to, tdq, tdk, tdv;   // panels of 64 columns (see sm100::make_panel_map)
+  CUtensorMap tg;   // per-channel decays: boxes of 64 rows
   Params p;
   int chunks;
   int32_t* status;

@@ -284,7 +284,7 @@ struct MapKey {
   bool operator==(const MapKey& o) const { return base == o.base && a == o.a && b == o.b && c == o.c && kind == o.kind; }
 };
 struct MapCache {
-  static constexpr int kSlots = 32;
+  static constexpr int kSlots = 64;   // a KDA training step looks up thirteen, of buffers that may alternate
   std::mutex mu;
   MapKey key[kSlots];
   CUtensorMap map[kSlots];

@@ -238,3 +238,37 @@ def test_local_pass_on_tcgen05(variant, B, Hq, H, T, bthd, strong):
         assert torch.equal(got[name], again[name]), name
         err = (got[name].double().cpu() - want).norm() / want.norm()
         assert err <= 1e-2, (name, err)
+
+
+@pytest.mark.parametrize("B,Hq,H,T,bthd,l2,decay", [
+    (1, 1, 1, 1, False, True, None), (1, 2, 2, 63, True, True, None), (1, 1, 2, 64, False, False, None), (2, 1, 3, 65, True, True, None),
+    (1, 2, 2, 129, False, True, 11.0), (1, 2, 2, 129, False, True, 11.2), (1, 1, 2, 200, True, True, 30.0), (1, 2, 2, 130, False, False, -0.5),
+    (3, 2, 2, 1665, False, True, 40.0)])   # the last: 162 chunks, more than one per CTA
+def test_kda_local_passes(B, Hq, H, T, bthd, l2, decay):
+    """KDA: chunks that decay by at most 2^16 (11.09 nats) in every channel take the tcgen05 kernel, the others -- and those with a positive
+    log decay -- the one with 16-row blocks; ragged chunks, grouped q/k heads, both storages, rows that are not normalised.  Against float64;
+    bf16 outputs round at 2^-9 (2-norm 1.7e-3), operands of the forward's checkpoints are bf16 too, in all 1e-2 of the largest."""
+    inp = O.make_inputs("kda", B, H, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
+    if not l2:
+        inp["k"] = (1.5 * torch.nn.functional.normalize(inp["k"].float(), dim=-1)).bfloat16()
+        inp["beta"] = inp["beta"] * 0.5
+    if decay is not None:   # one channel of the second chunk (of every other chunk of the long one)
+        for t0 in range(64, T, 128):
+            inp["g"][:, -1, t0:t0 + 64, 17] = -decay / 64
+    q, k = inp["q"][:, :Hq], inp["k"][:, :Hq]
+    gen = torch.Generator().manual_seed(T + 1)
+    do, dhT = torch.randn(B, H, T, 128, generator=gen).bfloat16(), torch.randn(B, H, 128, 128, generator=gen) * 0.1
+    def cu(x):
+        return x.transpose(1, 2).contiguous().cuda().transpose(1, 2) if bthd else x.contiguous().cuda()
+    args = ("kda", cu(q), cu(k), cu(inp["v"]), cu(inp["g"]), cu(inp["beta"]), cu(do))
+    run = lambda: ops.chunk_backward(*args, initial_state=inp["h0"].cuda(), d_final_state=dhT.cuda(), chunk_size=64, use_qk_l2norm=l2)
+    got, again = run(), run()
+    L.check_device_status()
+    rep = lambda x: x.double().repeat_interleave(H // Hq, 1)
+    ref = O.delta_rule_grads("kda", rep(q), rep(k), inp["v"].double(), inp["g"].double(), inp["beta"].double(), inp["h0"].double(), do.double(),
+                             dhT.double(), use_qk_l2norm=l2)
+    for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):
+        want = ref[name].view(B, Hq, H // Hq, T, 128).sum(2) if name in ("dq", "dk") else ref[name]
+        assert torch.equal(got[name], again[name]), name
+        err = (got[name].double().cpu() - want).norm() / want.norm()
+        assert err <= 1e-2, (name, err)
