@@ -5,12 +5,9 @@
 //     dS0 = e^{G_L} dS1 + N dS1 + Y^T dO
 // one [128 x 128] product per chunk and nothing else on the chain.  Three kernels:
 //
-//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles or as the A
-//                 fragments of mma.sync in the order the lanes of state_kernel load them (16 bytes per lane, no shared memory).
-//   chain_kernel  (scalar decays) one CTA per (sequence, 64 value columns) walks the chunks backwards on tcgen05, dS in registers;
-//                 stores dS1 of every chunk.  N and Y as two bf16 terms.
-//   state_kernel  (per-channel decays) the same on mma.sync, one CTA per (sequence, 32 value columns); dS stays in accumulator
-//                 registers, its copy in shared memory is the B operand.
+//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles.
+//   chain_kernel  one CTA per (sequence, 64 value columns) walks the chunks backwards on tcgen05, dS in registers; stores dS1 of every
+//                 chunk.  N and Y as two bf16 terms; per-channel decays: two fp16 terms of scaled operands.
 //   the local pass, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1 and the chunk's inputs; then the
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
 //                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
@@ -46,8 +43,8 @@ struct Params {
   const void* q; const void* k; const void* v; const void* g; const float* beta; const void* d_o; const float* d_hT;
   void* dq; void* dk; void* dv; float* dbeta; float* dg; float* dh0;
   const float* ckpt;    // [units][N][128][128] state at the start of every chunk
-  float4* nf;           // [units][N][8 row tiles][16 k-steps][32 lanes]; scalar decays: kNTile bytes per chunk
-  float4* yf;           // [units][N][8 row tiles][8 k-steps][32 lanes]; scalar decays: kYTile
+  float4* nf;           // [units][N] kNTile bytes
+  float4* yf;           // [units][N] kYTile bytes
   float* xat;           // [units][N][3][64][64] X, A, T; scalar decays: A and T as two bf16 terms, the tiles of local_sm100_kernel; KDA: see kXWide
   float* ds;            // [units][N][128][128] dS1
   float* el;            // [units][N][128] e^{G_L}
@@ -98,12 +95,12 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
 // Per-channel decays: what pre_kernel leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
-// whether the chunk is local_kernel's (a channel decays by more than 2^16, or a decay is positive) or local_sm100_kda_kernel's, and for
-// the latter the largest entries (bounds) of A, T, k^ and q^, in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
+// whether the chunk is local_kernel's (a channel decays by more than 2^16, or a decay is positive) or local_sm100_kda_kernel's, and
+// the largest entries (A, T for the latter only; Y) or bounds of them (k^, q^, N), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
 // in fours, A and T as two fp16 terms in tiles.
 constexpr float kWideKda = 16.f;   // log2 units
 constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096, kXTop = 2097;
-enum { kTopA, kTopT, kTopK, kTopQ, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
+enum { kTopA, kTopT, kTopK, kTopQ, kTopN, kTopY, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
 
 // the power of two that brings `top` to 2^13 .. 2^14 (none for zero and infinity); its inverse
 __device__ __forceinline__ float lift(uint32_t top) {
@@ -121,6 +118,20 @@ __device__ __forceinline__ void split2h(float x, float y, uint32_t& hi, uint32_t
   hi = pack_h(x, y);
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = pack_h(x - f.x, y - f.y);
+}
+// store_terms for fp16 terms of `s` times the entries
+__device__ __forceinline__ void store_terms_h(uint8_t* dst, int next, int lo, const float (&d)[4], float s) {
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+    uint32_t h, l;
+    split2h(s * d[2 * hr], s * d[2 * hr + 1], h, l);
+    *reinterpret_cast<uint32_t*>(dst + hr * next) = h;
+    *reinterpret_cast<uint32_t*>(dst + hr * next + lo) = l;
+  }
+}
+// Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation.
+__host__ __device__ constexpr uint32_t idesc_fp16(int M, int N, int a_mn_major, int b_mn_major) {
+  return tc::idesc_bf16(M, N, a_mn_major, b_mn_major) & ~((1u << 7) | (1u << 10));
 }
 // The chunks blockIdx.x, + gridDim.x, .. of one kind; warp-uniform, one read per 32 of them.
 template <bool WIDE>
@@ -178,8 +189,8 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
 
   bool wide = false;
   float bound = 0.f, topA = 0.f;   // of a row of q^ or k^; of A
-  __shared__ uint32_t sTop[4];
-  if (KDA && tid < 4) sTop[tid] = 0u;
+  __shared__ uint32_t sTop[7];     // in the order of kTop (N: of W), then of Kd
+  if (KDA && tid < 7) sTop[tid] = 0u;
   // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
   {
     uint2 qr[8], kr[8];
@@ -414,10 +425,15 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
     if (!wide) {
       atomicMax(&sTop[kTopT], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
       __syncthreads();
-      if (tid < 4) xat[kXTop + tid] = __uint_as_float(sTop[tid]);
+      if (tid == 0) xat[kXTop + kTopT] = __uint_as_float(sTop[kTopT]);
       put_tile(sX, LDT, xat + 8192, lift(sTop[kTopT]));
     }
-    if (tid == 0) xat[kXWide] = wide ? 1.f : 0.f;
+    if (tid == 0) {
+      xat[kXWide] = wide ? 1.f : 0.f;
+      xat[kXTop + kTopA] = __uint_as_float(sTop[kTopA]);
+      xat[kXTop + kTopK] = __uint_as_float(sTop[kTopK]);
+      xat[kXTop + kTopQ] = __uint_as_float(sTop[kTopQ]);
+    }
   } else {
     put_tile(sX, LDT, xat + 8192, 1.f);
   }
@@ -448,7 +464,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       }
     }
   }
-  // ---- Y^T = (Q^ e^G)^T - W^T A^T -> fragments of the state kernel (an accumulator is a fragment with its columns as k) --------
+  // ---- Y^T = (Q^ e^G)^T - W^T A^T -> tiles (an accumulator is a fragment with its columns as k) ---------------------------------------
   {
     float Y[8][4];
 #pragma unroll
@@ -473,19 +489,28 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       }
     }
     if constexpr (KDA) {
-      float4* dst = p.yf + (chunk * 8 + warp) * 8 * 32 + lane;
+      float m = 0.f, w = 0.f;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(Y[nt][0], Y[nt][2], Y[nt][1], Y[nt][3]);
-    } else {
-      uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + chunk * kYTile + 2 * warp * kYRbs + g * 16 + 4 * t;
+      for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
+        for (int e = 0; e < 4; ++e) { m = fmaxf(m, fabsf(Y[nt][e])); w = fmaxf(w, fabsf(W[nt][e])); }
+      atomicMax(&sTop[kTopY], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+      atomicMax(&sTop[kTopN], __reduce_max_sync(0xffffffffu, __float_as_uint(w)));
+      __syncthreads();
+      if (tid == 0) xat[kXTop + kTopY] = __uint_as_float(sTop[kTopY]);
+    }
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + chunk * kYTile + 2 * warp * kYRbs + g * 16 + 4 * t;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      if constexpr (KDA) store_terms_h(dst + nt * 128, kYRbs, kYTile / 2, Y[nt], lift(sTop[kTopY])); else store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
     }
   }
-  // ---- N = -W^T Kd -> fragments -----------------------------------------------------------------------------------------------
+  uint32_t topN = 0u;
+  // ---- N = -W^T Kd -> tiles -----------------------------------------------------------------------------------------------
   if constexpr (KDA) {
     // lane = channels lane, lane + 32, ..; warp = token pairs warp, warp + 8, ..; split into the two terms once
     uint4 kd[4][4];
+    float m = 0.f;
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const int c = lane + 32 * x;
@@ -494,16 +519,22 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       for (int i = 0; i < 4; ++i) {
         const int r = 2 * (warp + 8 * i);
         BFrag<true> f;
-        f.set(bf(sK + r * LDH + c) * sRk[r] * ex2(gl - sG[r * LDG + c]), bf(sK + (r + 1) * LDH + c) * sRk[r + 1] * ex2(gl - sG[(r + 1) * LDG + c]));
+        const float y0 = bf(sK + r * LDH + c) * sRk[r] * ex2(gl - sG[r * LDG + c]), y1 = bf(sK + (r + 1) * LDH + c) * sRk[r + 1] * ex2(gl - sG[(r + 1) * LDG + c]);
+        f.set(y0, y1);
+        m = fmaxf(m, fmaxf(fabsf(y0), fabsf(y1)));
         kd[i][x] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
       }
     }
+    atomicMax(&sTop[6], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     __syncthreads();   // every read of k, q, X and A is done
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int x = 0; x < 4; ++x) sKd[(warp + 8 * i) * LDK + lane + 32 * x] = kd[i][x];
     __syncthreads();
+    // |N| <= 64 |W| |Kd|: loose by some 2^7 of the 2^18 that the terms have to spare
+    topN = __float_as_uint(64.f * __uint_as_float(sTop[kTopN]) * __uint_as_float(sTop[6]));
+    if (tid == 0) xat[kXTop + kTopN] = __uint_as_float(topN);
   }
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
@@ -529,152 +560,16 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         fma<X3>(d[nt], a, bk);
       }
     }
-    if constexpr (KDA) {
-      float4* dst = p.nf + ((chunk * 8 + warp) * 16 + 8 * half) * 32 + lane;
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.nf) + chunk * kNTile + 2 * warp * sm100::RBS + 8 * half * 128 + g * 16 + 4 * t;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(d[nt][0], d[nt][2], d[nt][1], d[nt][3]);
-    } else {
-      uint8_t* dst = reinterpret_cast<uint8_t*>(p.nf) + chunk * kNTile + 2 * warp * sm100::RBS + 8 * half * 128 + g * 16 + 4 * t;
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
+    for (int nt = 0; nt < 8; ++nt) {
+      if constexpr (KDA) store_terms_h(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt], lift(topN)); else store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
     }
   }
 }
 
 // =====================================================================================================================
-// state_kernel: the state pass for per-channel decays; eight warps, warp w owns channel rows 16 w .. 16 w + 15 of dS [128][32]
-// =====================================================================================================================
-constexpr int kStThreads = 256;
-constexpr int LDP = 72;    // dS and dO in shared memory: row pairs interleaved, [rows / 2][32 columns][2], 72 floats per pair
-// dS as its two terms, [rows / 2][32 columns][hi, hi, lo, lo]: split once by the warp that owns it, not by the eight that read it
-constexpr int kLdS = 136;
-constexpr int st_rows = 2 * (64 * kLdS + 32 * LDP) * 4, st_smem = st_rows + 8 * 2048;
-
-static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Params p) {
-  pdl_entry();
-  extern __shared__ __align__(16) uint8_t smem[];
-  float* sS = reinterpret_cast<float*>(smem);          // [2][64 * kLdS]
-  float* sO = sS + 2 * 64 * kLdS;                       // [2][32 * LDP]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  uint8_t* stage = smem + st_rows + warp * 2048;
-  const int unit = blockIdx.x >> 2, v0 = (blockIdx.x & 3) * kVS;
-  const int b = unit / p.map.H, h = unit % p.map.H;
-  const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
-  const int r0 = 16 * warp + g, r1 = r0 + 8;
-  float S[4][4];   // tile nt: rows r0, r1; columns 8 nt + 2t, + 1
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt) {
-    float2 lo = make_float2(0.f, 0.f), hi = lo;
-    if (p.d_hT) {
-      lo = *reinterpret_cast<const float2*>(p.d_hT + ((int64_t)unit * kD + r0) * kD + v0 + 8 * nt + 2 * t);
-      hi = *reinterpret_cast<const float2*>(p.d_hT + ((int64_t)unit * kD + r1) * kD + v0 + 8 * nt + 2 * t);
-    }
-    S[nt][0] = lo.x; S[nt][1] = lo.y; S[nt][2] = hi.x; S[nt][3] = hi.y;
-  }
-  const int orow = tid >> 2, ocol = (tid & 3) * 8;   // this thread's eight columns of dO
-  auto load_do = [&](int n) -> uint4 {
-    const int tok = n * kC + orow;
-    if (n < 0 || tok >= p.map.T) return make_uint4(0u, 0u, 0u, 0u);
-    return *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_o) + v_base + (int64_t)tok * v_tok + v0 + ocol);
-  };
-  const int64_t chunk0 = (int64_t)unit * p.N;
-  float4 nf[16], yf[8];
-  float el0, el1;
-  {
-    const int64_t c = chunk0 + p.N - 1;
-#pragma unroll
-    for (int ks = 0; ks < 16; ++ks) nf[ks] = __ldcs(p.nf + ((c * 8 + warp) * 16 + ks) * 32 + lane);
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) yf[ks] = __ldcs(p.yf + ((c * 8 + warp) * 8 + ks) * 32 + lane);
-    el0 = p.el[c * 128 + r0]; el1 = p.el[c * 128 + r1];
-  }
-  uint4 dor = load_do(p.N - 1);
-  for (int n = p.N - 1; n >= 0; --n) {
-    float* cS = sS + (n & 1) * 64 * kLdS;
-    float* cO = sO + (n & 1) * 32 * LDP;
-    // dS1 of this chunk: to memory (sixteen rows through the warp's 2 KB, as whole 128-byte lines), and to the other warps
-    float* out = p.ds + (chunk0 + n) * (kD * kD) + (int64_t)(16 * warp) * kD + v0;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = 8 * nt + 2 * t;
-      *reinterpret_cast<float2*>(stage + g * 128 + (((2 * nt + (t >> 1)) ^ g) << 4) + 8 * (t & 1)) = make_float2(S[nt][0], S[nt][1]);
-      *reinterpret_cast<float2*>(stage + (g + 8) * 128 + (((2 * nt + (t >> 1)) ^ g) << 4) + 8 * (t & 1)) = make_float2(S[nt][2], S[nt][3]);
-      // the lanes of a row pair swap: the even row's takes column c of both rows, the odd row's c + 1
-      const bool odd = g & 1;
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? S[nt][2 * hr] : S[nt][2 * hr + 1], 4);
-        const float x = odd ? got : S[nt][2 * hr], y = odd ? S[nt][2 * hr + 1] : got;   // even row, odd row
-        BFrag<true> f;
-        f.set(x, y);
-        *reinterpret_cast<uint4*>(cS + ((hr ? r1 : r0) >> 1) * kLdS + 4 * (c + odd)) = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
-      }
-    }
-    {
-      const uint32_t w[4] = {dor.x, dor.y, dor.z, dor.w};
-      float* o = cO + (orow >> 1) * LDP + 2 * ocol + (orow & 1);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { o[4 * e] = mma::lo_f(w[e]); o[4 * e + 2] = mma::hi_f(w[e]); }
-    }
-    const int64_t cn = chunk0 + (n > 0 ? n - 1 : 0);   // the next chunk's operands replace this one's as they are used
-    dor = load_do(n - 1);
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 4 * i + (lane >> 3), q = lane & 7;
-      *reinterpret_cast<float4*>(out + (int64_t)r * kD + 4 * q) = *reinterpret_cast<const float4*>(stage + r * 128 + ((q ^ (r & 7)) << 4));
-    }
-    __syncwarp();
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) { S[nt][0] *= el0; S[nt][1] *= el0; S[nt][2] *= el1; S[nt][3] *= el1; }
-    el0 = p.el[cn * 128 + r0]; el1 = p.el[cn * 128 + r1];
-    float Z[4][4];   // second accumulator: shorter chains
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) zero4(Z[nt]);
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      AFrag<true> a;
-      a.set(yf[ks].x, yf[ks].y, yf[ks].z, yf[ks].w);
-      yf[ks] = __ldcs(p.yf + ((cn * 8 + warp) * 8 + ks) * 32 + lane);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const float2 y = ld2(cO + (4 * ks + t) * LDP + 2 * (8 * nt + g));
-        BFrag<false> bo;   // bf16 values: one term in either precision
-        bo.set(y.x, y.y);
-        mma::fma_b1(Z[nt], a, bo);
-      }
-    }
-#pragma unroll
-    for (int ks = 0; ks < 16; ++ks) {
-      AFrag<true> a;
-      a.set(nf[ks].x, nf[ks].y, nf[ks].z, nf[ks].w);
-      nf[ks] = __ldcs(p.nf + ((cn * 8 + warp) * 16 + ks) * 32 + lane);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        BFrag<true> bs;
-        const uint4 y = *reinterpret_cast<const uint4*>(cS + (4 * ks + t) * kLdS + 4 * (8 * nt + g));
-        bs.h[0] = y.x; bs.h[1] = y.y; bs.l[0] = y.z; bs.l[1] = y.w;
-        if (ks & 1) fma<true>(Z[nt], a, bs); else fma<true>(S[nt], a, bs);
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) S[nt][e] += Z[nt][e];
-  }
-  if (p.dh0) {
-    float* out = p.dh0 + (int64_t)unit * kD * kD + v0;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = 8 * nt + 2 * t;
-      *reinterpret_cast<float2*>(out + (int64_t)r0 * kD + c) = make_float2(S[nt][0], S[nt][1]);
-      *reinterpret_cast<float2*>(out + (int64_t)r1 * kD + c) = make_float2(S[nt][2], S[nt][3]);
-    }
-  }
-}
-
-// =====================================================================================================================
-// chain_kernel: the state pass for scalar decays on tcgen05, one CTA per (sequence, 64 value columns)
+// chain_kernel: the state pass on tcgen05, one CTA per (sequence, 64 value columns)
 //
 // dS stays in registers (thread = channel row, 32 columns); its two bf16 terms are the B operand, N and Y^T arrive by bulk copies as
 // the A operands, two terms each: three products N dS and two Y^T dO per 16 channels or tokens, 16 bits of every operand where
@@ -691,7 +586,11 @@ static __global__ void __launch_bounds__(kStThreads, 1) state_kernel(const Param
 // while dS is zero does not change that).  Forward and backward together, 1 to 256 sequences: 1 to 9 % faster at five chunks, 4 to
 // 13 % at 16, 6 to 14 % at 64; from 48 sequences on ahead or level at every length.
 // =====================================================================================================================
+// Per-channel decays: two fp16 terms of operands whose largest entry is brought to 2^13 and above (22 bits; pre_kernel gives the bounds of N and Y),
+// the two products with accumulators of their own; four more warps find the power of two for d_o and turn it into fp16 where it lies.
 constexpr int kChThreads = 288, kChCols = 64;   // eight worker warps and one that issues
+constexpr int kChWarpsKda = 4;
+template <bool KDA> constexpr int ch_threads() { return kChThreads + (KDA ? 32 * kChWarpsKda : 0); }
 // N hi twice, N lo, Y^T and d_o twice, the terms of dS, staging of its rows
 constexpr int kNTerm = kNTile / 2, kOTile = 64 * 128;
 constexpr int CH_H = 0, CH_L = CH_H + 2 * kNTerm, CH_Y = CH_L + kNTerm, CH_O = CH_Y + 2 * kYTile, CH_S = CH_O + 2 * kOTile, CH_G = CH_S + 2 * 128 * 128, CH_TOTAL = CH_G + 8 * 2048;
@@ -702,25 +601,30 @@ struct alignas(64) ChainParams {
   int32_t* status;
 };
 
-static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __grid_constant__ ChainParams P) {
+template <bool KDA>
+__global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __grid_constant__ ChainParams P) {
   const Params& p = P.p;
   // a name of its own: declarations of one name in a namespace share the first one's alignment
   extern __shared__ __align__(1024) uint8_t chain_smem[];
   uint8_t* const smem = chain_smem;
   __shared__ __align__(8) struct {
-    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y, bar_d;
+    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y, bar_d, full_o[2];
     uint32_t tmem_base;
     int abort;
+    uint32_t top_s[4], top_o[8];   // largest entries of dS and d_o, by turns
   } ctl;
+  constexpr uint32_t kTmem = KDA ? 256 : 128, kTmemN = 128;   // (KDA: N dS behind the two accumulators of Y^T d_o)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int unit = blockIdx.x / (kD / kChCols), v0 = blockIdx.x % (kD / kChCols) * kChCols;
   const int b = unit / p.map.H, h = unit % p.map.H;
   if (warp == 0) {
-    tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), 128);
+    tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), kTmem);
     tc::tmem_relinquish();
   }
+  if (tid < 8) ctl.top_s[tid & 3] = ctl.top_o[tid] = 0u;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(tc::smem_u32(&ctl.full_o[i]), 32 * kChWarpsKda);
       tc::mbar_init(tc::smem_u32(&ctl.full_h[i]), 1);
       tc::mbar_init(tc::smem_u32(&ctl.full_y[i]), 1);
     }
@@ -738,7 +642,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
   const uint32_t tbase = ctl.tmem_base, sbase = tc::smem_u32(smem);
   auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
     const uint32_t at = tc::smem_u32(&bar);
-    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp >> 3);
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), min(warp >> 3, 1));
   };
   const int64_t chunk0 = (int64_t)unit * p.N;
   const int steps = p.dh0 ? p.N : p.N - 1;   // the product of the first chunk gives the initial state's gradient alone
@@ -761,7 +665,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
       };
       if (steps > 0) { load_y(0); load_h(0); load_l(0); }
       if (steps > 1) { load_y(1); load_h(1); }
-      constexpr uint32_t id = tc::idesc_bf16(128, 64, 0, 1);
+      constexpr uint32_t id = KDA ? idesc_fp16(128, 64, 0, 1) : tc::idesc_bf16(128, 64, 0, 1);
       auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
       const uint64_t sd = tc::smem_desc_sw128(sbase + CH_S, 128 * 128, 1024), ld = tc::smem_desc(sbase + CH_L, 128, sm100::RBS);
 #pragma unroll 1
@@ -771,6 +675,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         const uint64_t od = tc::smem_desc_sw128(sbase + CH_O + (it & 1) * kOTile, 128 * 128, 1024);
         const uint64_t hd = tc::smem_desc(sbase + CH_H + (it & 1) * kNTerm, 128, sm100::RBS);
         wait_bar(ctl.full_y[it & 1], (it >> 1) & 1);
+        if constexpr (KDA) wait_bar(ctl.full_o[it & 1], (it >> 1) & 1);
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
@@ -781,15 +686,16 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         wait_bar(ctl.full_h[it & 1], (it >> 1) & 1);
         wait_bar(ctl.rdy, it & 1);
         tc::tc_fence_after();
+        const uint32_t acc_n = KDA ? tbase + kTmemN : acc;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, ks * 2048), id, 1);
-          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, 128 * 128 + ks * 2048), id, 1);
+          tc::mma_ss(acc_n, adv(hd, ks * 256), adv(sd, ks * 2048), id, !KDA || ks > 0);
+          tc::mma_ss(acc_n, adv(hd, ks * 256), adv(sd, 128 * 128 + ks * 2048), id, 1);
         }
         wait_bar(ctl.full_l, it & 1);
         tc::tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
+        for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc_n, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
         tc::mma_commit(tc::smem_u32(&ctl.bar_d));
         wait_bar(ctl.bar_y, it & 1);   // Y^T and d_o have been read
         if (it + 2 < steps) load_y(it + 2);
@@ -799,6 +705,37 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
       }
     }
     __syncwarp();
+  } else if (KDA && warp > 8) {
+    // d_o, two threads to a token: its largest entry, then fp16 in place
+    const int at = (tid - kChThreads) * 64;
+#pragma unroll 1
+    for (int it = 0; it < steps; ++it) {
+      uint4* tile = reinterpret_cast<uint4*>(smem + CH_O + (it & 1) * kOTile + at);
+      wait_bar(ctl.full_y[it & 1], (it >> 1) & 1);
+      uint4 x[4];
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = tile[(i + (lane >> 1)) & 3];   // (pieces skewed by the token: no bank conflicts)
+        const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m = fmaxf(m, fmaxf(fabsf(mma::lo_f(w[e])), fabsf(mma::hi_f(w[e]))));
+      }
+      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+      if (lane == 0) atomicMax(&ctl.top_o[it & 7], top);
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      if (tid == kChThreads) ctl.top_o[(it + 4) & 7] = 0u;   // (the workers are past its last use: this tile came after chunk it - 2's product)
+      const float s = lift(ctl.top_o[it & 7]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = pack_h(s * mma::lo_f(w[e]), s * mma::hi_f(w[e]));
+        tile[(i + (lane >> 1)) & 3] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      tc::fence_async_smem();
+      sm100::mbar_arrive(tc::smem_u32(&ctl.full_o[it & 1]));
+    }
   } else {
     const int row = 32 * (warp & 3) + lane, hc = warp >> 2;   // this thread's channel and half of the columns
     const uint32_t lane_addr = (uint32_t)(32 * (warp & 3)) << 16;
@@ -814,6 +751,22 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
     for (int it = 0; it < p.N; ++it) {
       const int64_t chunk = chunk0 + p.N - 1 - it;
       const float el = p.el[chunk * 128 + row];
+      float s = 1.f, fn = 1.f, fy = 1.f;
+      if (KDA && it < steps) {
+        const float* xat = p.xat + chunk * (3 * 64 * 64) + kXTop;
+        fn = drop(__float_as_uint(__ldcg(xat + kTopN)));
+        fy = drop(__float_as_uint(__ldcg(xat + kTopY)));
+        float m = 0.f;
+#pragma unroll
+        for (int c = 0; c < 32; ++c) m = fmaxf(m, fabsf(S[c]));
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if (lane == 0) atomicMax(&ctl.top_s[it & 3], top);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (tid == 0) ctl.top_s[(it + 2) & 3] = 0u;
+        const uint32_t all = ctl.top_s[it & 3];
+        s = lift(all);
+        fn = fminf(fn * drop(all), 3.4e38f);
+      }
       if (it < steps) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -821,8 +774,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float x = S[8 * c + 2 * e], y = S[8 * c + 2 * e + 1];
-            hi[e] = mma::pack(x, y);
-            lo[e] = mma::pack(x - mma::lo_f(hi[e]), y - mma::hi_f(hi[e]));
+            if constexpr (KDA) split2h(s * x, s * y, hi[e], lo[e]); else split2(x, y, hi[e], lo[e]);
           }
           uint8_t* dst = smem + CH_S + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -851,13 +803,22 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
         __syncwarp();
       }
       if (it == steps) break;
+      uint32_t d[32];
+      if constexpr (KDA) {   // Y^T d_o is long done
+        wait_bar(ctl.bar_y, it & 1);
+        tc::tc_fence_after();
+        tc::tmem_ld32(tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
+        tc::tc_wait_ld();
+        fy = fminf(fy * drop(ctl.top_o[it & 7]), 3.4e38f);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) S[c] = S[c] * el + __uint_as_float(d[c]) * fy;
+      }
       wait_bar(ctl.bar_d, it & 1);
       tc::tc_fence_after();
-      uint32_t d[32];
-      tc::tmem_ld32(tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
+      tc::tmem_ld32(KDA ? tbase + lane_addr + kTmemN + 32 * hc : tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
       tc::tc_wait_ld();
 #pragma unroll
-      for (int c = 0; c < 32; ++c) S[c] = S[c] * el + __uint_as_float(d[c]);
+      for (int c = 0; c < 32; ++c) S[c] = KDA ? S[c] + __uint_as_float(d[c]) * fn : S[c] * el + __uint_as_float(d[c]);
       tc::tc_fence_before();
     }
     if (p.dh0) {
@@ -868,7 +829,7 @@ static __global__ void __launch_bounds__(kChThreads, 1) chain_kernel(const __gri
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, 128);
+  if (warp == 0) tc::tmem_dealloc(tbase, kTmem);
   if (tid == 0) sm100::report_wait(P.status, ctl.abort);
 }
 
@@ -1498,8 +1459,7 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
               : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal);
     if (e == cudaSuccess)
-      e = KDA ? cudaFuncSetAttribute(state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, st_smem)
-              : cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
+      e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) attr_dev = dev;
   }
@@ -1533,15 +1493,11 @@ inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* sta
   const SeqMap& m = p.map;
   auto panels = [&](CUtensorMap* t, const void* base, int heads) { return sm100::make_panel_map(t, base, m.B, heads, m.T, m.bthd != 0); };
   if (!panels(&lp.to, p.d_o, m.H)) return cudaErrorInvalidValue;
-  if constexpr (KDA) {
-    e = launch_pdl(state_kernel, dim3((unsigned)(units * 4)), dim3(kStThreads), st_smem, stream, p);
-  } else {
-    ChainParams c;
-    c.p = p;
-    c.status = status;
-    c.to = lp.to;
-    e = launch_pdl(chain_kernel, dim3((unsigned)(units * (kD / kChCols))), dim3(kChThreads), CH_TOTAL, stream, c);
-  }
+  ChainParams c;
+  c.p = p;
+  c.status = status;
+  c.to = lp.to;
+  e = launch_pdl(chain_kernel<KDA>, dim3((unsigned)(units * (kD / kChCols))), dim3(ch_threads<KDA>()), CH_TOTAL, stream, c);
   if (e != cudaSuccess) return e;
   if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
       !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))

@@ -53,10 +53,6 @@ struct LkCtl {
 };
 constexpr int LK_TOTAL = LK_CTL + sizeof(LkCtl);
 static_assert(LK_TOTAL <= 232448 && LK_CTL % 16 == 0 && offsetof(LkCtl, beta) % 16 == 0 && offsetof(LkSums, f) % 16 == 0, "shared memory");
-// Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation.
-__host__ __device__ constexpr uint32_t idesc_fp16(int M, int N, int a_mn_major, int b_mn_major) {
-  return tc::idesc_bf16(M, N, a_mn_major, b_mn_major) & ~((1u << 7) | (1u << 10));
-}
 static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(const __grid_constant__ LocalParams P) {
   const Params& p = P.p;
   extern __shared__ __align__(1024) uint8_t lk_smem[];
