@@ -1364,7 +1364,7 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
   cudaEvent_t joined = nullptr;
   const bool chunked = bwdc::eligible(d);
   auto pre = [&](cudaStream_t s) {
-    return chunked ? bwdc::launch_pre(d, q, k, g, beta, workspace, s, launches) : launch_bwd_pre(d, q, k, g, beta, workspace, s, launches);
+    return chunked ? bwdc::launch_pre(d, q, k, g, beta, workspace, status, s, s != stream, launches) : launch_bwd_pre(d, q, k, g, beta, workspace, s, launches);
   };
   cudaStream_t side = nullptr;
   cudaEvent_t forked = nullptr;

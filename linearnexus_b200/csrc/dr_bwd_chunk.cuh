@@ -5,7 +5,8 @@
 //     dS0 = e^{G_L} dS1 + N dS1 + Y^T dO
 // one [128 x 128] product per chunk and nothing else on the chain.  Three kernels:
 //
-//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles.
+//   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles.  Per-channel decays:
+//                 pre_sm100_kda_kernel (dr_bwd_pre_kda.cuh), persistent, on tcgen05, and pre_kernel for the chunks that it leaves.
 //   chain_kernel  one CTA per (sequence, 64 value columns) walks the chunks backwards on tcgen05, dS in registers; stores dS1 of every
 //                 chunk.  N and Y as two bf16 terms; per-channel decays: two fp16 terms of scaled operands.
 //   the local pass, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1 and the chunk's inputs; then the
@@ -94,9 +95,9 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   }
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
-// Per-channel decays: what pre_kernel leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
-// whether the chunk is local_kernel's (a channel decays by more than 2^16, or a decay is positive) or local_sm100_kda_kernel's, and
-// the largest entries (A, T for the latter only; Y) or bounds of them (k^, q^, N), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
+// Per-channel decays: what the pre-pass leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
+// whether the chunk is pre_kernel's and local_kernel's (a channel decays by more than 2^16, or a decay is positive) or pre_sm100_kda_kernel's and
+// local_sm100_kda_kernel's, and the largest entries (A, T) or bounds of them (k^, q^, N, Y), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
 // in fours, A and T as two fp16 terms in tiles.
 constexpr float kWideKda = 16.f;   // log2 units
 constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096, kXTop = 2097;
@@ -138,7 +139,10 @@ template <bool WIDE>
 struct ChunkList {
   int base;
   uint32_t mask;
-  __device__ __forceinline__ ChunkList(const float* xat, int chunks, int lane) : base(blockIdx.x) { fetch(xat, chunks, lane); }
+  __device__ __forceinline__ void start(const float* xat, int chunks, int lane) {
+    base = blockIdx.x;
+    fetch(xat, chunks, lane);
+  }
   __device__ __forceinline__ void fetch(const float* xat, int chunks, int lane) {
     const int64_t c = base + (int64_t)lane * gridDim.x;
     mask = __ballot_sync(0xffffffffu, c < chunks && (__ldcg(xat + c * (3 * 64 * 64) + kXWide) != 0.f) == WIDE);
@@ -168,7 +172,7 @@ template <bool KDA> constexpr int pre_smem() { return KDA ? PR_G + 64 * LDG * 4 
 static_assert(PR_SC >= 32 * LDK * 16 && 2 * (pre_smem<true>() + 1024) <= 233472, "two CTAs per SM");
 
 template <bool KDA>
-__global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
+__global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, const int chunks) {
   pdl_entry();
   extern __shared__ __align__(16) uint8_t smem[];
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + PR_K);
@@ -180,17 +184,21 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   float *sRk = sBeta + 64, *sRq = sBeta + 128, *sGs = sBeta + 192, *sFw = sBeta + 256, *sFd = sBeta + 320;
   float* sG = reinterpret_cast<float*>(smem + PR_G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int unit = blockIdx.x / p.N, n = blockIdx.x % p.N;
+  __shared__ uint32_t sTop[3];     // largest entries of Y, W and Kd
+  ChunkList<true> list;
+  if constexpr (KDA) list.start(p.xat, chunks, lane);
+#pragma unroll 1
+  for (int c = KDA ? list.next(p.xat, chunks, lane) : blockIdx.x; c < chunks; c = KDA ? list.next(p.xat, chunks, lane) : chunks) {
+  const int64_t chunk = c;
+  const int unit = c / p.N, n = c % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
   const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  const int64_t chunk = (int64_t)unit * p.N + n;
-
-  bool wide = false;
-  float bound = 0.f, topA = 0.f;   // of a row of q^ or k^; of A
-  __shared__ uint32_t sTop[7];     // in the order of kTop (N: of W), then of Kd
-  if (KDA && tid < 7) sTop[tid] = 0u;
+  if constexpr (KDA) {
+    __syncthreads();   // the chunk before is done with shared memory
+    if (tid < 3) sTop[tid] = 0u;
+  }
   // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
   {
     uint2 qr[8], kr[8];
@@ -206,12 +214,6 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         kr[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at);
         if constexpr (KDA) gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
       }
-    }
-    if constexpr (KDA) {
-      float m = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(fmaxf(gr[i].x, gr[i].y), fmaxf(gr[i].z, gr[i].w)));
-      wide = m > 0.f;
     }
     float bt = 0.f, g_lo = 0.f, g_hi = 0.f;
     if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
@@ -247,9 +249,8 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
     }
     ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
     if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
-      const float top = lane < 16 ? p.scale : 1.f, nrm = sqrtf(ss[0]), m = p.l2norm ? top / (nrm + 1e-6f) : top;
-      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = m;
-      bound = fabsf(m * nrm);
+      const float top = lane < 16 ? p.scale : 1.f;
+      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
     }
     if (lane < 8) sBeta[warp + 8 * lane] = bt;
     if (!KDA && warp == 0) {
@@ -260,13 +261,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
   __syncthreads();
   if constexpr (KDA) {
     mma::scan_channels<kPreThreads, kD, LDG>(sG, sX, tid);
-    if (tid < 128) {
-      p.el[chunk * 128 + tid] = ex2(sG[63 * LDG + tid]);
-      wide |= !(sG[63 * LDG + tid] >= -kWideKda);
-      p.xat[chunk * (3 * 64 * 64) + kXNorms + (tid >> 5) * kXNormRow + lane] = (tid < 64 ? sRk : sRq - 64)[tid];
-    }
-    atomicMax(&sTop[kTopQ], __reduce_max_sync(0xffffffffu, lane < 16 ? __float_as_uint(bound) : 0u));
-    atomicMax(&sTop[kTopK], __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : __float_as_uint(bound)));
+    if (tid < 128) p.el[chunk * 128 + tid] = ex2(sG[63 * LDG + tid]);
     if (tid < 64) { sFw[tid] = sBeta[tid] * sRk[tid]; }
   } else {
     const float gl = sGs[63];
@@ -323,13 +318,10 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         for (int e = 0; e < 4; ++e) {
           const int i = 16 * mt + g + 8 * (e >> 1), j = 8 * (nt0 + x) + 2 * t + (e & 1);
           sX[i * LDT + j] = j < i ? dk[x][e] * sRk[j] * sRk[i] : 0.f;
-          const float y = j <= i ? dq[x][e] * sRk[j] * sRq[i] : 0.f;
-          sA[i * 72 + j] = y;
-          topA = fmaxf(topA, fabsf(y));
+          sA[i * 72 + j] = j <= i ? dq[x][e] * sRk[j] * sRq[i] : 0.f;
         }
       }
     }
-    atomicMax(&sTop[kTopA], __reduce_max_sync(0xffffffffu, __float_as_uint(topA)));
   } else {
 #pragma unroll 1
   for (int tile = warp; tile < 20; tile += kPreThreads / 32) {   // raw bf16 rows: exact products
@@ -374,20 +366,19 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       sA[i * 72 + j] = j <= i ? aq * sRq[i] * sRk[j] : 0.f;
     }
   }
-  wide = __syncthreads_or(wide);
+  __syncthreads();
   // ---- X, A -> global (16 x 16 blocks at or below the diagonal), then T in place of X ----------------------------------------
   float* xat = p.xat + chunk * (3 * 64 * 64);
-  const bool as_rows = KDA && wide;
   for (int i = tid; i < 64 * 16; i += kPreThreads) {
     const int r = i >> 4, c4 = (i & 15) * 4;
     if ((c4 >> 4) <= (r >> 4)) {
-      // (columns in fours, so that a warp of the reader takes 32 rows of four at once)
-      *reinterpret_cast<float4*>(xat + (as_rows ? r * 64 + c4 : c4 * 64 + 4 * r)) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
-      if (as_rows) *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
+      // (scalar decays: columns in fours, so that a warp of the reader takes 32 rows of four at once)
+      *reinterpret_cast<float4*>(xat + (KDA ? r * 64 + c4 : c4 * 64 + 4 * r)) = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      if constexpr (KDA) *reinterpret_cast<float4*>(xat + 4096 + r * 64 + c4) = *reinterpret_cast<const float4*>(sA + r * 72 + c4);
     }
   }
-  // A, T as core matrices of 8 x 8, the blocks of eight rows next to each other; high terms, then low ones; of `s` times the entries as fp16 for KDA
-  auto put_tile = [&](const float* src, int ld, float* dst, float s) {
+  // scalar decays: A, T as core matrices of 8 x 8, the blocks of eight rows next to each other; high terms, then low ones
+  auto put_tile = [&](const float* src, int ld, float* dst) {
 #pragma unroll
     for (int x = 0; x < 512 / kPreThreads; ++x) {
       const int i = tid + kPreThreads * x, r = 8 * ((i >> 3) & 7) + (i & 7), c = 8 * (i >> 6);
@@ -395,47 +386,30 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       uint32_t h[4], l[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        float2 y = ld2(src + r * ld + c + 2 * e);
-        if (c + 2 * e > r) y.x = 0.f;
-        if (c + 2 * e + 1 > r) y.y = 0.f;
-        if constexpr (KDA) split2h(s * y.x, s * y.y, h[e], l[e]); else split2(y.x, y.y, h[e], l[e]);
+        const float2 y = ld2(src + r * ld + c + 2 * e);
+        split2(c + 2 * e <= r ? y.x : 0.f, c + 2 * e + 1 <= r ? y.y : 0.f, h[e], l[e]);
       }
       reinterpret_cast<uint4*>(dst)[i] = make_uint4(h[0], h[1], h[2], h[3]);
       reinterpret_cast<uint4*>(dst)[512 + i] = make_uint4(l[0], l[1], l[2], l[3]);
     }
   };
-  if (!as_rows) put_tile(sA, 72, xat + 4096, KDA ? lift(sTop[kTopA]) : 1.f);
-  if (!KDA && tid < 128) p.norms[chunk * 128 + tid] = (tid < 64 ? sRk : sRq - 64)[tid];
+  if constexpr (!KDA) {
+    put_tile(sA, 72, xat + 4096);
+    if (tid < 128) p.norms[chunk * 128 + tid] = (tid < 64 ? sRk : sRq - 64)[tid];
+  }
   __syncthreads();
   sm100::block_inverse_64(sX, sBeta, sX, tid);   // ends with a barrier
-  if constexpr (KDA) {
-    float m = 0.f;
-    for (int i = tid; i < 64 * 16; i += kPreThreads) {
-      const int r = i >> 4, c4 = (i & 15) * 4;
-      if ((c4 >> 4) <= (r >> 4)) {
-        float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
-        if (c4 + 0 > r) v.x = 0.f;
-        if (c4 + 1 > r) v.y = 0.f;
-        if (c4 + 2 > r) v.z = 0.f;
-        if (c4 + 3 > r) v.w = 0.f;
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        if (wide) *reinterpret_cast<float4*>(xat + 8192 + r * 64 + c4) = v;
-      }
+  if constexpr (!KDA) put_tile(sX, LDT, xat + 8192);
+  for (int i = tid; KDA && i < 64 * 16; i += kPreThreads) {
+    const int r = i >> 4, c4 = (i & 15) * 4;
+    if ((c4 >> 4) <= (r >> 4)) {
+      float4 v = *reinterpret_cast<const float4*>(sX + r * LDT + c4);
+      if (c4 + 0 > r) v.x = 0.f;
+      if (c4 + 1 > r) v.y = 0.f;
+      if (c4 + 2 > r) v.z = 0.f;
+      if (c4 + 3 > r) v.w = 0.f;
+      *reinterpret_cast<float4*>(xat + 8192 + r * 64 + c4) = v;
     }
-    if (!wide) {
-      atomicMax(&sTop[kTopT], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-      __syncthreads();
-      if (tid == 0) xat[kXTop + kTopT] = __uint_as_float(sTop[kTopT]);
-      put_tile(sX, LDT, xat + 8192, lift(sTop[kTopT]));
-    }
-    if (tid == 0) {
-      xat[kXWide] = wide ? 1.f : 0.f;
-      xat[kXTop + kTopA] = __uint_as_float(sTop[kTopA]);
-      xat[kXTop + kTopK] = __uint_as_float(sTop[kTopK]);
-      xat[kXTop + kTopQ] = __uint_as_float(sTop[kTopQ]);
-    }
-  } else {
-    put_tile(sX, LDT, xat + 8192, 1.f);
   }
   // ---- W^T: rows = the warp's 16 channels, columns = tokens; W = T diag(beta) K^ e^G ----------------------------------------
   constexpr bool X3 = KDA;
@@ -494,15 +468,15 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) { m = fmaxf(m, fabsf(Y[nt][e])); w = fmaxf(w, fabsf(W[nt][e])); }
-      atomicMax(&sTop[kTopY], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-      atomicMax(&sTop[kTopN], __reduce_max_sync(0xffffffffu, __float_as_uint(w)));
+      atomicMax(&sTop[0], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+      atomicMax(&sTop[1], __reduce_max_sync(0xffffffffu, __float_as_uint(w)));
       __syncthreads();
-      if (tid == 0) xat[kXTop + kTopY] = __uint_as_float(sTop[kTopY]);
+      if (tid == 0) xat[kXTop + kTopY] = __uint_as_float(sTop[0]);
     }
     uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + chunk * kYTile + 2 * warp * kYRbs + g * 16 + 4 * t;
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      if constexpr (KDA) store_terms_h(dst + nt * 128, kYRbs, kYTile / 2, Y[nt], lift(sTop[kTopY])); else store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
+      if constexpr (KDA) store_terms_h(dst + nt * 128, kYRbs, kYTile / 2, Y[nt], lift(sTop[0])); else store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
     }
   }
   uint32_t topN = 0u;
@@ -525,7 +499,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
         kd[i][x] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
       }
     }
-    atomicMax(&sTop[6], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    atomicMax(&sTop[2], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     __syncthreads();   // every read of k, q, X and A is done
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -533,7 +507,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
       for (int x = 0; x < 4; ++x) sKd[(warp + 8 * i) * LDK + lane + 32 * x] = kd[i][x];
     __syncthreads();
     // |N| <= 64 |W| |Kd|: loose by some 2^7 of the 2^18 that the terms have to spare
-    topN = __float_as_uint(64.f * __uint_as_float(sTop[kTopN]) * __uint_as_float(sTop[6]));
+    topN = __float_as_uint(64.f * __uint_as_float(sTop[1]) * __uint_as_float(sTop[2]));
     if (tid == 0) xat[kXTop + kTopN] = __uint_as_float(topN);
   }
 #pragma unroll 1
@@ -565,6 +539,7 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p) {
     for (int nt = 0; nt < 8; ++nt) {
       if constexpr (KDA) store_terms_h(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt], lift(topN)); else store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
     }
+  }
   }
 }
 
@@ -870,7 +845,8 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
   float *sEx = sU, *sUn = sU + 512;   // sums for dG_L [4][128], block flags
   float *sDq = F(L::kDot), *sDk = sDq + 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  ChunkList<true> list(p.xat, chunks, lane);
+  ChunkList<true> list;
+  list.start(p.xat, chunks, lane);
 #pragma unroll 1
   for (int at_chunk = list.next(p.xat, chunks, lane); at_chunk < chunks; at_chunk = list.next(p.xat, chunks, lane)) {
   __syncthreads();   // the chunk before is done with shared memory
@@ -1414,6 +1390,7 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
 
 #include "dr_bwd_local_sm100.cuh"
 #include "dr_bwd_local_kda.cuh"
+#include "dr_bwd_pre_kda.cuh"
 
 namespace dr {
 namespace bwdc {
@@ -1458,6 +1435,7 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
       e = KDA ? cudaFuncSetAttribute(local_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_TOTAL)
               : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal);
+    if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(pre_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_TOTAL);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
@@ -1467,18 +1445,35 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
   return e;
 }
 template <bool KDA>
-inline cudaError_t launch_pre_t(const Params& p, int64_t units, cudaStream_t stream) {
-  const cudaError_t e = set_attributes<KDA>();
+inline cudaError_t launch_pre_t(const Params& p, int64_t units, int32_t* status, cudaStream_t stream, bool beside, int* launches) {
+  int sms = 0;
+  cudaError_t e = set_attributes<KDA>(&sms);
   if (e != cudaSuccess) return e;
-  return launch_pdl(pre_kernel<KDA>, dim3((unsigned)(units * p.N)), dim3(kPreThreads), pre_smem<KDA>(), stream, p);
+  const int64_t chunks = units * p.N;
+  if constexpr (KDA) {
+    PreParams pp;
+    pp.p = p; pp.chunks = (int)chunks; pp.status = status;
+    const SeqMap& m = p.map;
+    if (!sm100::make_panel_map(&pp.tq, p.q, m.B, m.Hq, m.T, m.bthd != 0) || !sm100::make_panel_map(&pp.tk, p.k, m.B, m.Hq, m.T, m.bthd != 0) ||
+        !sm100::make_output_map(&pp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
+      return cudaErrorInvalidValue;
+    ++*launches;
+    // Beside the forward's state pass, whose CTAs keep an SM each for 2.65 us a chunk (this kernel: 10.4 us), its own CTAs keep off those SMs while
+    // there are few of them: those that wait for one would do their share of the chunks behind it.  32 sequences of 64 chunks: 185 us on
+    // 116 SMs, by the same figures 170 + 144 on all of them; level at about 59 sequences.
+    const int64_t free = beside && 5 * units <= 2 * sms ? sms - units : sms;
+    e = launch_pdl(pre_sm100_kda_kernel, dim3((unsigned)(chunks < free ? chunks : free)), dim3(kLtThreads), PK_TOTAL, stream, pp);
+    if (e != cudaSuccess) return e;
+  }
+  ++*launches;
+  return launch_pdl(pre_kernel<KDA>, dim3((unsigned)(!KDA || chunks < 2 * sms ? chunks : 2 * sms)), dim3(kPreThreads), pre_smem<KDA>(), stream, p, (int)chunks);
 }
 inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, const void* g, const float* beta, void* workspace,
-                              cudaStream_t stream, int* launches) {
+                              int32_t* status, cudaStream_t stream, bool beside, int* launches) {
   Params p = make_params(d, workspace);
   p.q = q; p.k = k; p.g = g; p.beta = beta;
-  ++*launches;
   const int64_t units = (int64_t)d->B * d->H;
-  return d->variant == DR_KDA ? launch_pre_t<true>(p, units, stream) : launch_pre_t<false>(p, units, stream);
+  return d->variant == DR_KDA ? launch_pre_t<true>(p, units, status, stream, beside, launches) : launch_pre_t<false>(p, units, status, stream, beside, launches);
 }
 template <bool KDA>
 inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* status, cudaStream_t stream) {
