@@ -1433,7 +1433,7 @@ cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, co
     p.dq = dq; p.dk = dk; p.dv = dv; p.dbeta = dbeta; p.dg = dg; p.dh0 = dh0;
     const int64_t units = (int64_t)d->B * d->H;
     cudaError_t e = d->variant == DR_KDA ? bwdc::launch_adjoint_t<true>(p, units, status, stream) : bwdc::launch_adjoint_t<false>(p, units, status, stream);
-    *launches += d->variant == DR_KDA ? 3 : 2;
+    *launches += d->variant == DR_KDA && !p.few ? 3 : 2;
     if (e != cudaSuccess || p.map.Hq == p.map.H) return e;
     // grouped q/k heads: the heads' dq^, dk^ summed over each group, then the chain rule
     BwdFinalParams fp{};

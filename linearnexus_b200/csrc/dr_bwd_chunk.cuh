@@ -53,6 +53,7 @@ struct Params {
   float* part;          // grouped heads: dq^ [units][N*64][128], then dk^ (over nf)
   SeqMap map;
   int N, variant, g_dt, l2norm;
+  int few;              // KDA: pre_kernel and local_kernel take every chunk (see kFewKda)
   float scale;
 };
 
@@ -139,25 +140,29 @@ template <bool WIDE>
 struct ChunkList {
   int base;
   uint32_t mask;
-  __device__ __forceinline__ void start(const float* xat, int chunks, int lane) {
+  __device__ __forceinline__ void start(const Params& p, int chunks, int lane) {
     base = blockIdx.x;
-    fetch(xat, chunks, lane);
+    fetch(p, chunks, lane);
   }
-  __device__ __forceinline__ void fetch(const float* xat, int chunks, int lane) {
+  __device__ __forceinline__ void fetch(const Params& p, int chunks, int lane) {
     const int64_t c = base + (int64_t)lane * gridDim.x;
-    mask = __ballot_sync(0xffffffffu, c < chunks && (__ldcg(xat + c * (3 * 64 * 64) + kXWide) != 0.f) == WIDE);
+    mask = __ballot_sync(0xffffffffu, c < chunks && ((WIDE && p.few) || (__ldcg(p.xat + c * (3 * 64 * 64) + kXWide) != 0.f) == WIDE));
   }
-  __device__ __forceinline__ int next(const float* xat, int chunks, int lane) {   // `chunks` behind the last
+  __device__ __forceinline__ int next(const Params& p, int chunks, int lane) {   // `chunks` behind the last
     while (mask == 0u) {
       if ((int64_t)base + 32 * gridDim.x >= chunks) return chunks;
       base += 32 * gridDim.x;
-      fetch(xat, chunks, lane);
+      fetch(p, chunks, lane);
     }
     const int i = __ffs(mask) - 1;
     mask &= mask - 1;
     return base + i * (int)gridDim.x;
   }
 };
+// Few chunks, in short sequences: a training step is bound by the host, and the two launches that look for wide chunks cost more than the kernels on
+// tcgen05 give; every chunk is then treated as a wide one.  Whole step, so / as wide and narrow chunks: 20 chunks in 4 sequences 132 / 139 us, 40 in 4
+// 134 / 140, 80 in 16 133 / 138; 64 in 4 152 / 139, 128 in 8 159 / 139.
+constexpr int kFewKda = 80, kFewLength = 10;
 // =====================================================================================================================
 // pre_kernel
 // =====================================================================================================================
@@ -186,9 +191,9 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   __shared__ uint32_t sTop[3];     // largest entries of Y, W and Kd
   ChunkList<true> list;
-  if constexpr (KDA) list.start(p.xat, chunks, lane);
+  if constexpr (KDA) list.start(p, chunks, lane);
 #pragma unroll 1
-  for (int c = KDA ? list.next(p.xat, chunks, lane) : blockIdx.x; c < chunks; c = KDA ? list.next(p.xat, chunks, lane) : chunks) {
+  for (int c = KDA ? list.next(p, chunks, lane) : blockIdx.x; c < chunks; c = KDA ? list.next(p, chunks, lane) : chunks) {
   const int64_t chunk = c;
   const int unit = c / p.N, n = c % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
@@ -846,9 +851,9 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
   float *sDq = F(L::kDot), *sDk = sDq + 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   ChunkList<true> list;
-  list.start(p.xat, chunks, lane);
+  list.start(p, chunks, lane);
 #pragma unroll 1
-  for (int at_chunk = list.next(p.xat, chunks, lane); at_chunk < chunks; at_chunk = list.next(p.xat, chunks, lane)) {
+  for (int at_chunk = list.next(p, chunks, lane); at_chunk < chunks; at_chunk = list.next(p, chunks, lane)) {
   __syncthreads();   // the chunk before is done with shared memory
   const int unit = at_chunk / p.N, n = at_chunk % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
@@ -1412,6 +1417,7 @@ inline Params make_params(const DrDesc* d, void* workspace) {
   Params p{};
   p.N = (d->T + kC - 1) / kC;
   const int64_t nc = (int64_t)d->B * d->H * p.N;
+  p.few = nc <= kFewKda && p.N <= kFewLength;
   float* f = reinterpret_cast<float*>(workspace);
   p.ckpt = f; f += nc * kCkpt;
   p.nf = reinterpret_cast<float4*>(f); p.part = f; f += nc * kNf;
@@ -1450,7 +1456,7 @@ inline cudaError_t launch_pre_t(const Params& p, int64_t units, int32_t* status,
   cudaError_t e = set_attributes<KDA>(&sms);
   if (e != cudaSuccess) return e;
   const int64_t chunks = units * p.N;
-  if constexpr (KDA) {
+  if (KDA && !p.few) {
     PreParams pp;
     pp.p = p; pp.chunks = (int)chunks; pp.status = status;
     const SeqMap& m = p.map;
@@ -1498,6 +1504,7 @@ inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* sta
       !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
     return cudaErrorInvalidValue;
   if constexpr (KDA) {
+    if (p.few) return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
     if (!sm100::make_output_map(&lp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
       return cudaErrorInvalidValue;
     e = launch_pdl(local_sm100_kda_kernel, grid, dim3(kLtThreads), LK_TOTAL, stream, lp);

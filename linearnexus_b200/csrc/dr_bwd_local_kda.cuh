@@ -92,7 +92,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
   constexpr uint32_t tKS = 0, tKD = 64, tAO = 128, tQ1 = 192, tR = 256, tV = 320, tVn = 384, tdR = 448;
   constexpr uint32_t tKr1 = 0, tKc1 = 64, tA = 128, tM = 256, tQ2 = 128, tKr2 = 256, tKc2 = 320, tKc3 = 384;
   ChunkList<false> list;
-  list.start(p.xat, P.chunks, lane);
+  list.start(p, P.chunks, lane);
 
   if (warp == 16) {
     // (only the low word changes: the address field does not carry into the other)
@@ -150,7 +150,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
       if (lane < 4) ctl.top[turn][lane] = __float_as_uint(tops);
       __syncwarp();
     };
-    int c = list.next(p.xat, P.chunks, lane);
+    int c = list.next(p, P.chunks, lane);
     if (c < P.chunks) {
       load_vectors(c);
       store_vectors(0);
@@ -168,7 +168,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
 #pragma unroll 1
     for (int next; c < P.chunks; c = next, ph ^= 1) {
       asm volatile("" : "+r"(sb), "+r"(tb));   // the descriptors are formed for each chunk: kept over the loop they would be spilled
-      next = list.next(p.xat, P.chunks, lane);
+      next = list.next(p, P.chunks, lane);
       asm volatile("bar.sync 7, 544;" ::: "memory");
       tc::tc_fence_after();
       constexpr uint32_t hi_lo[3] = {0, 1, 0}, lo_hi[3] = {0, 0, 1};   // terms of A and of B in the three products
@@ -354,7 +354,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
   } else {
     uint32_t ph = 0;
 #pragma unroll 1
-    for (int c = list.next(p.xat, P.chunks, lane); c < P.chunks; c = list.next(p.xat, P.chunks, lane), ph ^= 1) {
+    for (int c = list.next(p, P.chunks, lane); c < P.chunks; c = list.next(p, P.chunks, lane), ph ^= 1) {
       // (what follows from the thread's place is formed for each chunk: kept over the loop it would be spilled, and there is no L1 to speak of)
       int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       asm volatile("" : "+r"(warp), "+r"(lane));

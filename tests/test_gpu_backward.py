@@ -241,12 +241,13 @@ def test_local_pass_on_tcgen05(variant, B, Hq, H, T, bthd, strong):
 
 
 @pytest.mark.parametrize("B,Hq,H,T,bthd,l2,decay", [
-    (1, 1, 1, 1, False, True, None), (1, 2, 2, 63, True, True, None), (1, 1, 2, 64, False, False, None), (2, 1, 3, 65, True, True, None),
-    (1, 2, 2, 129, False, True, 11.0), (1, 2, 2, 129, False, True, 11.2), (1, 1, 2, 200, True, True, 30.0), (1, 2, 2, 130, False, False, -0.5),
+    (1, 1, 1, 1, False, True, None), (2, 1, 3, 65, True, True, None), (1, 2, 2, 130, False, False, -0.5), (1, 1, 2, 640, True, True, 30.0),
+    (81, 1, 1, 1, False, True, None), (41, 1, 1, 65, True, True, 11.0), (1, 1, 2, 641, False, False, None), (1, 2, 2, 703, False, True, 11.0),
+    (1, 2, 2, 704, True, True, 11.2), (1, 1, 2, 800, True, True, 30.0), (1, 2, 2, 730, False, False, -0.5),
     (3, 2, 2, 1665, False, True, 40.0)])   # the last: 162 chunks, more than one per CTA
 def test_kda_local_passes(B, Hq, H, T, bthd, l2, decay):
-    """KDA: chunks that decay by at most 2^16 (11.09 nats) in every channel take the tcgen05 kernel, the others -- and those with a positive
-    log decay -- the one with 16-row blocks; ragged chunks, grouped q/k heads, both storages, rows that are not normalised.  Against float64;
+    """KDA: chunks that decay by at most 2^16 (11.09 nats) in every channel take the tcgen05 kernels, the others -- those with a positive
+    log decay, and all of at most 80 in sequences of at most ten -- the ones with 16-row blocks; ragged chunks, grouped q/k heads, both storages, rows that are not normalised.  Against float64;
     bf16 outputs round at 2^-9 (2-norm 1.7e-3), operands of the forward's checkpoints are bf16 too, in all 1e-2 of the largest."""
     inp = O.make_inputs("kda", B, H, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
     if not l2:
