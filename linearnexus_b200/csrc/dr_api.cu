@@ -129,12 +129,11 @@ int resolve_chunk_path(const DrDesc* d) {
 //  * bf16 at the tensor-core shape: few sequences leave most SMs idle under one CTA per sequence (3.5 us per chunk, KDA's state
 //    pass 2.1); slices of the value axis, 0.95 us per chunk past six sequences and 0.75 below, win while sequences x 8 slices fit one
 //    wave (kTransUnits) and there are chunks enough to pay for the longer first pass.  Us, this form against the other, sequences x
-//    chunks, scalar decay: 8 x 6 22.8 / 25.4, 18 x 6 29.6 / 25.7, 18 x 8 31.4 / 32.6, 18 x 16 38.9 / 60.1, 16 x 32 74.7 / 115, 4 x 64
-//    82 / 223, 18 x 128 276 / 443; KDA, from 17 chunks on: 18 x 17 51.4 / 53.6, 4 x 32 46.8 / 63.3, 12 x 128 228 / 288.
-//    The lines lie where they were drawn for a slower state pass; the crossings now: for scalar decay from 10 sequences on at eight
-//    chunks, and from 20 to 26 sequences this form is ahead from about 12 chunks on (20 x 32: 97 / 115, 24 x 32: 106 / 115, 28 x 32:
-//    118 / 115); KDA at 3 chunks for 4 sequences (18.1 / 18.9) and 8 for 18, and past 32 chunks up to 18 sequences as well (14 x 40:
-//    82 / 99, 18 x 128: 277 / 326), while 6 x 128 is level (252 / 246).
+//    chunks, scalar decay: 8 x 5 18 / 22, 18 x 5 23 / 23, 18 x 8 26 / 33, 18 x 16 34 / 61, 16 x 32 63 / 116, 4 x 64 79 / 225, 18 x 128
+//    227 / 444; KDA: 4 x 32 43 / 61, 16 x 32 66 / 73, 18 x 32 66 / 76, 12 x 128 197 / 253, 18 x 128 233 / 272.
+//    The lines lie where they were drawn for a slower first pass; the crossings now: for scalar decay this form is ahead up to 37
+//    sequences from 8 chunks on (32 x 8 29 / 33, 32 x 64 187 / 226), but its outputs are less exact there (3.9e-3 against 3.4e-3); KDA at
+//    5 chunks for 8 sequences (18 / 19) and 12 for 18 (31 / 33).
 // Both up to 1 GB of scratch.
 constexpr int kTransUnits = 148 / 8;
 // Whether the token recurrence beats the transition form from two chunks on, in microseconds measured for 4 to 512 sequences and 65 to
@@ -160,7 +159,7 @@ int64_t trans_scratch(const DrDesc* d) {
   if (resolve_chunk_path(d) == kPathRecurrence && !split_eligible(d))
     return d->T > (d->variant == DR_DELTA && d->K == 128 ? 96 : 64) && !recurrence_ahead(d) ? need : 0;
   const bool kda = d->variant == DR_KDA;
-  return units <= (kda && d->T > 32 * 64 ? 12 : kTransUnits) && d->T > (kda ? 16 : 5) * 64 ? need : 0;
+  return units <= kTransUnits && d->T > (kda ? 16 : 5) * 64 ? need : 0;
 }
 
 bool fp32_chunk_eligible(const DrDesc* d) { return d->chunk <= 64 && d->K <= 128; }

@@ -63,17 +63,6 @@ inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC -
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
-constexpr int IN_G = 0;                          // log2(e) G   fp32 [64][136]
-constexpr int IN_K = IN_G + 64 * LDF * 4;        // raw k       bf16 [64][136]
-constexpr int IN_Q = IN_K + 64 * LDH * 2;        // raw q       bf16 [64][136]
-constexpr int IN_AKK = IN_Q + 64 * LDH * 2;      // A_kk fp32 [64][68]; later the W staging tile bf16 [64][136]
-constexpr int IN_T = IN_AKK + 64 * LDT * 4;      // T    fp32 [64][68]
-constexpr int IN_AQK = IN_T + 64 * LDT * 4;      // A_qk bf16 [64][72]
-constexpr int IN_BETA = IN_AQK + 64 * LDQ * 2;   // beta[64], rk[64], rq[64]
-constexpr int IN_TOTAL = IN_BETA + 3 * 64 * 4;
-static_assert(64 * LDT * 4 == 64 * LDH * 2, "the W staging tile reuses the A_kk array");
-static_assert(2 * (IN_TOTAL + 1024) <= 233472, "two CTAs per SM");
-
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -159,6 +148,7 @@ struct IntraPackedParams : IntraParams {
 };
 // The pass in transition form (see "few sequences" below): fragments instead of records.
 struct IntraTransParams {
+  CUtensorMap tq, tk, tv, tg;   // panels of q, k and v; g as boxes of 64 rows
   FwdParams p;
   uint4 *nf, *yf;     // [chunks][8 | 4 row tiles][8 k-steps][32 lanes]: A operands of m16n8k16
   float4 *zf, *of;    // [chunks][8 | 4 row tiles][16 column tiles][32 lanes]: addends
@@ -345,255 +335,6 @@ __device__ __forceinline__ void general_products(const float* sG, const __nv_bfl
   }
   sm100::group_sync(1);
 }
-static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const __grid_constant__ IntraTransParams P) {
-  const FwdParams& p = P.p;
-  pdl_entry();
-  extern __shared__ __align__(1024) uint8_t smem[];
-  float* sG = reinterpret_cast<float*>(smem + IN_G);
-  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + IN_K);
-  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + IN_Q);
-  float* sAkk = reinterpret_cast<float*>(smem + IN_AKK);
-  __nv_bfloat16* sWst = reinterpret_cast<__nv_bfloat16*>(smem + IN_AKK);
-  float* sT = reinterpret_cast<float*>(smem + IN_T);
-  __nv_bfloat16* sAqk = reinterpret_cast<__nv_bfloat16*>(smem + IN_AQK);
-  float* sBeta = reinterpret_cast<float*>(smem + IN_BETA);
-  float* sRk = sBeta + 64;
-  float* sRq = sBeta + 128;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int T = p.map.T, nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks, n = blockIdx.x % nchunks;
-  const int b = unit / p.map.H, h = unit % p.map.H, rows = min(kC, T - n * kC), t0 = n * kC;
-  const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);   // q, k (possibly fewer heads)
-  const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);         // per-channel decay: per value head
-  const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  constexpr float kLog2e = 1.4426950408889634f;
-
-  // ---- load: raw k, q rows, their norm factors, the log decay (in log2 units); lane = four channels ---------
-  // (all global loads of the warp's eight rows are issued before the first is used)
-  {
-    uint2 qraw[8], kraw[8];
-    float gv[8][4];
-    {
-      const int64_t at = qk_base + (t0 + warp) * qk_tok + 4 * lane;
-      const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(p.q) + at;
-      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(p.k) + at;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        qraw[i] = make_uint2(0u, 0u); kraw[i] = make_uint2(0u, 0u);
-        if (warp + 8 * i < rows) {
-          qraw[i] = *reinterpret_cast<const uint2*>(qp);
-          kraw[i] = *reinterpret_cast<const uint2*>(kp);
-        }
-        qp += 8 * qk_tok; kp += 8 * qk_tok;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = 0.f;
-    if (p.variant == DR_KDA) {   // one loop per storage type: no branch between the loads
-      int64_t at = gk_base + (t0 + warp) * gk_tok + 4 * lane;
-      if (p.g_dt == DR_BF16) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
-          if (warp + 8 * i < rows) ld4(p.g, at, DR_BF16, gv[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i, at += 8 * gk_tok)
-          if (warp + 8 * i < rows) ld4(p.g, at, DR_F32, gv[i]);
-      }
-    } else if (p.variant == DR_GATED) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (warp + 8 * i < rows) gv[i][0] = gv[i][1] = gv[i][2] = gv[i][3] = ld_elem(p.g, s_base + (t0 + warp + 8 * i) * s_tok, p.g_dt);
-    }
-    float bt = 0.f;
-    if (lane < 8 && warp + 8 * lane < rows) bt = p.beta[s_base + (t0 + warp + 8 * lane) * s_tok];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = warp + 8 * i;
-      *reinterpret_cast<uint2*>(sQ + c * LDH + 4 * lane) = qraw[i];
-      *reinterpret_cast<uint2*>(sK + c * LDH + 4 * lane) = kraw[i];
-      *reinterpret_cast<float4*>(sG + c * LDF + 4 * lane) =
-          make_float4(gv[i][0] * kLog2e, gv[i][1] * kLog2e, gv[i][2] * kLog2e, gv[i][3] * kLog2e);
-    }
-    // norm factors of the warp's 16 rows: the sums are scattered over the lanes as they are reduced (16 shuffles instead of
-    // 80), so that each lane takes one square root and one quotient (as every lane did for every row, a fifth of the pass)
-    float ss[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float2 q0 = bf2(qraw[i].x), q1 = bf2(qraw[i].y), k0 = bf2(kraw[i].x), k1 = bf2(kraw[i].y);
-      ss[i] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
-      ss[8 + i] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
-    }
-#pragma unroll
-    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
-#pragma unroll
-      for (int i = 0; i < m; ++i) {
-        const bool up = lane & o;
-        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
-        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    }
-    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
-    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
-      const float top = lane < 16 ? p.scale : 1.f;
-      (lane < 16 ? sRq : sRk)[warp + 8 * ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
-    }
-    if (lane < 8) sBeta[warp + 8 * lane] = bt;
-  }
-  __syncthreads();
-  // ---- G = inclusive prefix sum of the log decay over the rows of the chunk, per channel ---------------------
-  // thread = (8-row segment, four channels): local scan, then the totals of the earlier segments are added;
-  // the segment totals live in the first rows of the (still unused) T array
-  {
-    const int seg = tid >> 5, c4 = 4 * (tid & 31);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 loc[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const float4 x = *reinterpret_cast<const float4*>(sG + (8 * seg + r) * LDF + c4);
-      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
-      loc[r] = acc;
-    }
-    *reinterpret_cast<float4*>(sT + seg * 128 + c4) = acc;
-    __syncthreads();
-    float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s2 = 0; s2 < seg; ++s2) {
-      const float4 x = *reinterpret_cast<const float4*>(sT + s2 * 128 + c4);
-      pre.x += x.x; pre.y += x.y; pre.z += x.z; pre.w += x.w;
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      *reinterpret_cast<float4*>(sG + (8 * seg + r) * LDF + c4) =
-          make_float4(loc[r].x + pre.x, loc[r].y + pre.y, loc[r].z + pre.z, loc[r].w + pre.w);
-    __syncthreads();
-  }
-  general_products(sG, sK, sQ, sAkk, sT, sAqk, sRk, sRq, tid);
-  // ---- T = (I + diag(beta) A_kk)^-1 -----------------------------------------------------------------------------
-  sm100::block_inverse_64(sAkk, sBeta, sT, tid);
-  // ---- the chunk's effect on the state and on its own output, as fragments of trans_state_kernel ----------------------------
-  //   N = -Kd^T W, Z = Kd^T U, Y = Qg - A_qk W, A_qk U   with W = T diag(beta) k^ e^G, U = T diag(beta) V
-  // Tb = T diag(beta) -> bf16 over A_kk; A_qk masked in place; then (T and G dead) V over T, k^ e^G over G, Qg over q, Kd over k
-  __nv_bfloat16* sTb = sWst;                                              // [64][72]
-  __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(smem + IN_T);      // [64][136]
-  __nv_bfloat16* sKg = reinterpret_cast<__nv_bfloat16*>(smem + IN_G);     // [64][136]
-  uint4 vv[4], qg[4], kd[4], kg[4];
-  const int64_t v_base = p.map.base(b, h, kD), v_tok = p.map.tok(kD);
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-    vv[it] = make_uint4(0u, 0u, 0u, 0u);
-    if (row < rows) vv[it] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.v) + v_base + (t0 + row) * v_tok + col);
-  }
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int piece = tid + kThreads * it, row = piece >> 3, col = (piece & 7) * 8;
-    float a[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = col + e <= row ? sT[row * LDT + col + e] * sBeta[col + e] : 0.f;
-    *reinterpret_cast<uint4*>(sTb + row * LDQ + col) = pack8(a);
-    if (col + 7 > row && (col >> 4) <= (row >> 4)) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (col + e > row) sAqk[row * LDQ + col + e] = __float2bfloat16_rn(0.f);
-    }
-  }
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-    const uint4 uq = *reinterpret_cast<const uint4*>(sQ + row * LDH + col), uk = *reinterpret_cast<const uint4*>(sK + row * LDH + col);
-    decayed_piece(sG + row * LDF + col, sG + 63 * LDF + col, uq, uk, sRq[row], sRk[row], qg[it], kd[it], kg[it]);
-  }
-  const int64_t chunk = blockIdx.x;
-  if (tid < kD) P.el[chunk * kD + tid] = ex2(sG[63 * LDF + tid]);
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int piece = tid + kThreads * it, row = piece >> 4, col = (piece & 15) * 8;
-    *reinterpret_cast<uint4*>(sV + row * LDH + col) = vv[it];
-    *reinterpret_cast<uint4*>(sQ + row * LDH + col) = qg[it];
-    *reinterpret_cast<uint4*>(sK + row * LDH + col) = kd[it];
-    *reinterpret_cast<uint4*>(sKg + row * LDH + col) = kg[it];
-  }
-  __syncthreads();
-  const uint32_t aTb = tc::smem_u32(sTb), aV = tc::smem_u32(sV), aKg = tc::smem_u32(sKg), aKd = tc::smem_u32(sK), aAq = tc::smem_u32(sAqk);
-  // W^T, U^T of the warp's 16 channels / value columns (rows), columns = tokens; then as B operands (k = token)
-  uint32_t Wb[4][2][2], Ub[4][2][2];   // [16-token step][8-column half][k half]
-  {
-    float W[8][4], U[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      W[nt][0] = W[nt][1] = W[nt][2] = W[nt][3] = 0.f;
-      U[nt][0] = U[nt][1] = U[nt][2] = U[nt][3] = 0.f;
-    }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      uint32_t aw[4], au[4];
-      mma::ldsm4t(aw, mma::frag_at(aKg, LDH, 16 * ks, 16 * warp, lane));
-      mma::ldsm4t(au, mma::frag_at(aV, LDH, 16 * ks, 16 * warp, lane));
-#pragma unroll
-      for (int n2 = 0; n2 < 4; ++n2) {
-        if (n2 >= ks) {
-          uint32_t bt[4];
-          mma::ldsm4(bt, mma::frag_b(aTb, LDQ, 16 * n2, 16 * ks, lane));
-          mma::bf16(W[2 * n2], aw, bt[0], bt[1]);
-          mma::bf16(W[2 * n2 + 1], aw, bt[2], bt[3]);
-          mma::bf16(U[2 * n2], au, bt[0], bt[1]);
-          mma::bf16(U[2 * n2 + 1], au, bt[2], bt[3]);
-        }
-      }
-    }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh) {
-          Wb[ks][hf][kh] = mma::pack(W[2 * ks + kh][2 * hf], W[2 * ks + kh][2 * hf + 1]);
-          Ub[ks][hf][kh] = mma::pack(U[2 * ks + kh][2 * hf], U[2 * ks + kh][2 * hf + 1]);
-        }
-  }
-#pragma unroll 1
-  for (int mt = 0; mt < 12; ++mt) {   // rows of [Kd^T (8 tiles); A_qk (4 tiles)]
-    const bool st = mt < 8;
-    const int m = st ? mt : mt - 8;
-    float w[2][4], u[2][4];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) { w[hf][0] = w[hf][1] = w[hf][2] = w[hf][3] = 0.f; u[hf][0] = u[hf][1] = u[hf][2] = u[hf][3] = 0.f; }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      if (st || ks <= m) {
-        uint32_t a[4];
-        if (st) mma::ldsm4t(a, mma::frag_at(aKd, LDH, 16 * ks, 16 * m, lane));
-        else mma::ldsm4(a, mma::frag_a(aAq, LDQ, 16 * m, 16 * ks, lane));
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          mma::bf16(w[hf], a, Wb[ks][hf][0], Wb[ks][hf][1]);
-          mma::bf16(u[hf], a, Ub[ks][hf][0], Ub[ks][hf][1]);
-        }
-      }
-    }
-    const int64_t at = (chunk * (st ? 8 : 4) + m) * 8 + warp;
-    if (st) {
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) { w[hf][0] = -w[hf][0]; w[hf][1] = -w[hf][1]; w[hf][2] = -w[hf][2]; w[hf][3] = -w[hf][3]; }
-    } else {
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          const float2 q2 = bf2(*reinterpret_cast<const uint32_t*>(sQ + (16 * m + g + 8 * hr) * LDH + 16 * warp + 8 * hf + 2 * t));
-          w[hf][2 * hr] = q2.x - w[hf][2 * hr];
-          w[hf][2 * hr + 1] = q2.y - w[hf][2 * hr + 1];
-        }
-    }
-    (st ? P.nf : P.yf)[at * 32 + lane] = make_uint4(mma::pack(w[0][0], w[0][1]), mma::pack(w[0][2], w[0][3]), mma::pack(w[1][0], w[1][1]), mma::pack(w[1][2], w[1][3]));
-    float4* dst = (st ? P.zf : P.of) + at * 64 + lane;
-    dst[0] = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
-    dst[32] = make_float4(u[1][0], u[1][1], u[1][2], u[1][3]);
-  }
-}
-
 // ---- intra-chunk kernel, records ------------------------------------------------------------------------------------------------
 // Two persistent CTAs per SM: eight warps that work, one that issues copies and products.  A worker warp owns eight rows of the chunk, a lane
 // four channels of them, from the prefix sums to the tiles.
@@ -633,11 +374,10 @@ constexpr int IG_K = 64 * LDF * 4, IG_Q = IG_K + 64 * LDH * 2, IG_T = IG_Q + 64 
 static_assert(IS_TOT + 4096 <= IS_X && IS_X % 1024 == 0 && IG_AQK + 64 * LDQ * 2 <= IS_X, "shared memory");
 static_assert(2 * (IS_TOTAL + 1024) <= 233472, "two CTAs per SM");
 
-static __device__ __noinline__ void general_products_call(uint8_t* smem, int tid) {   // the rare way
-  const IntraCtl& ctl = *reinterpret_cast<const IntraCtl*>(smem + IS_BETA);
+static __device__ __noinline__ void general_products_call(uint8_t* smem, const float* rk, const float* rq, int tid) {   // the rare way
   general_products(reinterpret_cast<const float*>(smem), reinterpret_cast<const __nv_bfloat16*>(smem + IG_K),
                    reinterpret_cast<const __nv_bfloat16*>(smem + IG_Q), reinterpret_cast<float*>(smem + IS_X), reinterpret_cast<float*>(smem + IG_T),
-                   reinterpret_cast<__nv_bfloat16*>(smem + IG_AQK), ctl.rk, ctl.rq, tid);
+                   reinterpret_cast<__nv_bfloat16*>(smem + IG_AQK), rk, rq, tid);
 }
 
 template <class Params>
@@ -946,7 +686,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           *reinterpret_cast<uint2*>(smem + IG_Q + (row * LDH + 4 * lane) * 2) = q[r];
         }
         sync();
-        general_products_call(smem, tid);
+        general_products_call(smem, ctl.rk, ctl.rq, tid);
         uint4 tq[4], td[4], tk[4], aq[2];
         const float* sG = reinterpret_cast<const float*>(smem);
 #pragma unroll
@@ -1066,6 +806,429 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 8) tc::tmem_dealloc(tb, 128);
+  if (tid == 0) sm100::report_wait(p.status, ctl.abort);
+}
+
+// ---- intra-chunk kernel, transition form ------------------------------------------------------------------------------------------
+// The chunk's effect on the state and on its own output, as fragments of trans_state_kernel:
+//   N = -Kd^T W, Z = Kd^T U, Y = Qg - A_qk W, A_qk U   with W = T diag(beta) k^ e^G, U = T diag(beta) V
+// One CTA of eight warps per chunk, two per SM; up to T as intra_kernel, with one place for each tile.  The four products have bf16 operands as
+// in the other forwards; their accumulators are read in the shape of mma.sync's, which is what the fragments are, so nothing passes through
+// shared memory on its way out.  A_qk's products have M = 128 rows, of which the lower 64 are V's bits and nobody reads them.
+//
+// What bounds it: B=1, T=1777, H=16 (448 chunks, one and a half waves): 48 us with the general products and everything on mma.sync -> 32.5, the
+// layer around it 95 -> 82; the phases of a chunk follow each other, two chunks to an SM.  Errors against float64 (2-norm, output / state, T=1024, H=4):
+// Gated 4.7e-3 / 3.0e-3 -> 3.9e-3 / 2.4e-3, KDA (T=1100) 4.4e-3 / 3.0e-3 -> 3.5e-3 / 2.5e-3: one rounding per decayed operand instead of two,
+// and T diag(beta) as two terms.
+constexpr int IT_KG = 0, IT_QG = 16384, IT_AQK = 32768, IT_V = IT_AQK + 8192, IT_TOT = IT_V + 16384;   // k^ e^G, later U^T; ..; V
+constexpr int IT_KD = IS_X - 16384;        // Kd; the log decay arrives over Kd and X
+struct TransCtl {
+  float beta[64], rk[64], rq[64];
+  uint64_t bar[4], full, full_v;
+  uint32_t tmem_base;
+  int abort;
+};
+constexpr int IT_TOTAL = IS_BETA + sizeof(TransCtl);
+static_assert(IT_TOT + 4096 <= IT_KD && IT_KD % 1024 == 0 && IT_V % 1024 == 0 && 2 * (IT_TOTAL + 1024) <= 233472, "two CTAs per SM");
+
+static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const __grid_constant__ IntraTransParams P) {
+  const FwdParams& p = P.p;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  TransCtl& ctl = *reinterpret_cast<TransCtl*>(smem + IS_BETA);
+  float* sX = reinterpret_cast<float*>(smem + IS_X);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int T = p.map.T, nchunks = (T + kC - 1) / kC, unit = blockIdx.x / nchunks, t0 = (blockIdx.x - unit * nchunks) * kC;
+  const int b = unit / p.map.H, h = unit - b * p.map.H, rows = min(kC, T - t0) - 8 * warp;   // rows of this warp (may be none)
+  const int64_t chunk = blockIdx.x;
+  if (warp == 0) {
+    tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), 256);
+    tc::tmem_relinquish();
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 4; ++i) tc::mbar_init(tc::smem_u32(&ctl.bar[i]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.full), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.full_v), 1);
+    tc::fence_mbar_init();
+    ctl.abort = 0;
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  pdl_entry();
+  const uint32_t tb = ctl.tmem_base, sb = tc::smem_u32(smem);
+  auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
+    const uint32_t at = tc::smem_u32(&bar);
+    sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), 0);
+  };
+  auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
+  auto tiles_sync = [&]() {
+    tc::fence_async_smem();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+  };
+  auto load_v = [&]() {
+    const uint32_t bar = tc::smem_u32(&ctl.full_v);
+    tc::mbar_arrive_expect_tx(bar, 16384);
+    tc::tma_load_4d(sb + IT_V, &P.tv, 0, h, t0, b, bar);
+    tc::tma_load_4d(sb + IT_V + 8192, &P.tv, 64, h, t0, b, bar);
+  };
+  if (tid == 0) {
+    const uint32_t bar = tc::smem_u32(&ctl.full);
+    const int hq = p.map.hq(h);
+    tc::mbar_arrive_expect_tx(bar, 32768 + (p.variant == DR_KDA ? (p.g_dt == DR_BF16 ? 16384 : 32768) : 0));
+    if (p.variant == DR_KDA) tc::tma_load_4d(sb + IT_KD, &P.tg, 0, t0, h, b, bar);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      tc::tma_load_4d(sb + IT_KG + 8192 * e, &P.tk, 64 * e, hq, t0, b, bar);
+      tc::tma_load_4d(sb + IT_QG + 8192 * e, &P.tq, 64 * e, hq, t0, b, bar);
+    }
+    load_v();
+  }
+  constexpr float kLog2e = 1.4426950408889634f;
+  // byte of this lane's four channels in row 8 warp + r of a panel: + 128 r, piece ^ r
+  const int piece = (lane & 15) >> 1, own = (lane >> 4) * 8192 + warp * 1024 + (lane & 1) * 8;
+  auto entry = [&](int base, int r) { return reinterpret_cast<uint2*>(smem + base + own + r * 128 + ((piece ^ r) << 4)); };
+  // ---- the warp's rows, prefix sums over them, norm factors ----------------------------------------------------------------------------
+  float4 G[8];
+  {
+    const int64_t s_tok = p.map.tok(1), s_at = p.map.base(b, h, 1) + (t0 + 8 * warp) * s_tok;
+    const float bt = lane < 8 && lane < rows ? p.beta[s_at + lane * s_tok] : 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      float x = 0.f;
+      if (p.variant == DR_GATED && r < rows) x = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
+      G[r] = make_float4(x, x, x, x);
+    }
+    wait_bar(ctl.full, 0);
+    if (p.variant == DR_KDA) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        if (p.g_dt == DR_BF16) {
+          const uint2 u = *reinterpret_cast<const uint2*>(smem + IT_KD + (8 * warp + r) * 256 + lane * 8);
+          const float2 y = bf2(u.x), z = bf2(u.y);
+          G[r] = make_float4(y.x, y.y, z.x, z.y);
+        } else {
+          G[r] = *reinterpret_cast<const float4*>(smem + IT_KD + (8 * warp + r) * 512 + lane * 16);
+        }
+      }
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      acc.x += G[r].x * kLog2e; acc.y += G[r].y * kLog2e; acc.z += G[r].z * kLog2e; acc.w += G[r].w * kLog2e;
+      G[r] = acc;
+    }
+    *reinterpret_cast<float4*>(smem + IT_TOT + warp * 512 + lane * 16) = acc;
+    // the sums are scattered over the lanes as they are reduced (16 shuffles), so that each lane takes one square root and one quotient
+    float ss[16];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint2 q = *entry(IT_QG, r), k = *entry(IT_KG, r);
+      const float2 q0 = bf2(q.x), q1 = bf2(q.y), k0 = bf2(k.x), k1 = bf2(k.y);
+      ss[r] = q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
+      ss[8 + r] = k0.x * k0.x + k0.y * k0.y + k1.x * k1.x + k1.y * k1.y;
+    }
+#pragma unroll
+    for (int o = 16, m = 8; o > 1; o >>= 1, m >>= 1) {
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        const bool up = lane & o;
+        const float send = up ? ss[i] : ss[i + m], keep = up ? ss[i + m] : ss[i];
+        ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    if (!(lane & 1)) {   // lanes 0, 2 .. 14: q rows, 16 .. 30: k rows
+      const float top = lane < 16 ? p.scale : 1.f;
+      (lane < 16 ? ctl.rq : ctl.rk)[8 * warp + ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
+    }
+    if (lane < 8) ctl.beta[8 * warp + lane] = bt;
+  }
+  __syncthreads();   // the log decay, where Kd and k^ e^{-G} go, has been read, too
+  bool wide;   // the same in every warp: each sees all channels
+  float4 el;   // e^{G_L}
+  {
+    float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
+    float most = 0.f;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      if (s == warp) pre = run;
+      const float4 y = *reinterpret_cast<const float4*>(smem + IT_TOT + s * 512 + lane * 16);
+      run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
+      most = fmaxf(most, fmaxf(fmaxf(fabsf(run.x), fabsf(run.y)), fmaxf(fabsf(run.z), fabsf(run.w))));
+    }
+    const float all = (run.x + run.y) + (run.z + run.w);   // NaN if any sum was
+    wide = __any_sync(0xffffffffu, !(most <= 64.f && all == all));
+    el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
+    if (warp == 0) *reinterpret_cast<float4*>(P.el + chunk * kD + 4 * lane) = el;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
+  }
+  const int row = 32 * (warp & 3) + lane, hf = warp >> 2;   // this thread's row of a product, half of its columns
+  const uint32_t ta = tb + ((uint32_t)(32 * (warp & 3)) << 16);
+  if (!wide) {
+    // ---- the tiles; A_kk, A_qk -------------------------------------------------------------------------------------------------------------
+    const float2 el0 = make_float2(el.x, el.y), el1 = make_float2(el.z, el.w);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float2 g0 = make_float2(G[r].x, G[r].y), g1 = make_float2(G[r].z, G[r].w);
+      const float2 e0 = ex2x2(g0), e1 = ex2x2(g1), i0 = make_float2(ex2(-g0.x), ex2(-g0.y)), i1 = make_float2(ex2(-g1.x), ex2(-g1.y));
+      const float fk = ctl.rk[8 * warp + r], fq = ctl.rq[8 * warp + r];
+      const float2 rk = make_float2(fk, fk), rq = make_float2(fq, fq);
+      const uint2 q = *entry(IT_QG, r), k = *entry(IT_KG, r);
+      const float2 k0 = mul2(bf2(k.x), rk), k1 = mul2(bf2(k.y), rk);
+      const float2 x0 = mul2(k0, i0), x1 = mul2(k1, i1);
+      const float2 a0 = mul2(k0, e0), a1 = mul2(k1, e1), b0 = mul2(mul2(bf2(q.x), rq), e0), b1 = mul2(mul2(bf2(q.y), rq), e1);
+      const float2 d0 = mul2(x0, el0), d1 = mul2(x1, el1);
+      *entry(IT_KG, r) = make_uint2(tc::pack_bf16(a0.x, a0.y), tc::pack_bf16(a1.x, a1.y));
+      *entry(IT_QG, r) = make_uint2(tc::pack_bf16(b0.x, b0.y), tc::pack_bf16(b1.x, b1.y));
+      *entry(IT_KD, r) = make_uint2(tc::pack_bf16(d0.x, d0.y), tc::pack_bf16(d1.x, d1.y));
+      *entry(IS_X, r) = make_uint2(tc::pack_bf16(x0.x, x0.y), tc::pack_bf16(x1.x, x1.y));
+    }
+    tiles_sync();
+    if (warp == 0) {
+      if (tc::elect_one()) {
+        const uint64_t kg = tc::smem_desc_sw128(sb + IT_KG, 128, 1024), qg = tc::smem_desc_sw128(sb + IT_QG, 128, 1024), bd = tc::smem_desc_sw128(sb + IS_X, 128, 1024);
+        // rows 64 .. of the first product and of the second are the tile that follows, and not read
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          tc::mma_ss(tb, adv(kg, (ks >> 2) * 8192 + (ks & 3) * 32), adv(bd, (ks >> 2) * 8192 + (ks & 3) * 32), tc::idesc_bf16(128, 64, 0, 0), ks > 0);
+          tc::mma_ss(tb + 64, adv(qg, (ks >> 2) * 8192 + (ks & 3) * 32), adv(bd, (ks >> 2) * 8192 + (ks & 3) * 32), tc::idesc_bf16(128, 64, 0, 0), ks > 0);
+        }
+        tc::mma_commit(tc::smem_u32(&ctl.bar[0]));
+      }
+      __syncwarp();
+    }
+    wait_bar(ctl.bar[0], 0);
+    tc::tc_fence_after();
+    if (row < 64) {   // what is above the diagonal of A_kk is not used
+      uint32_t x[32];
+      tc::tmem_ld32(ta + 32 * hf, x);
+      tc::tc_wait_ld();
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        *reinterpret_cast<uint4*>(sX + row * LDT + 32 * hf + 4 * e) = make_uint4(x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
+      tc::tmem_ld32(ta + 64 + 32 * hf, x);
+      tc::tc_wait_ld();
+      const int last = row - 32 * hf;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint32_t w[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const int j = 8 * e + 2 * f;
+          w[f] = tc::pack_bf16(j <= last ? __uint_as_float(x[j]) : 0.f, j + 1 <= last ? __uint_as_float(x[j + 1]) : 0.f);
+        }
+        *reinterpret_cast<uint4*>(smem + IT_AQK + row * 128 + (((4 * hf + e) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  } else {
+    // ---- any decay: through the arrays of the general products, over V, which arrives once more ------------------------------------------------
+    uint2 q[8], k[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      q[r] = *entry(IT_QG, r);
+      k[r] = *entry(IT_KG, r);
+    }
+    wait_bar(ctl.full_v, 0);
+    __syncthreads();   // every warp has its rows and the decays
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int i = 8 * warp + r;
+      *reinterpret_cast<float4*>(smem + (i * LDF + 4 * lane) * 4) = G[r];
+      *reinterpret_cast<uint2*>(smem + IG_K + (i * LDH + 4 * lane) * 2) = k[r];
+      *reinterpret_cast<uint2*>(smem + IG_Q + (i * LDH + 4 * lane) * 2) = q[r];
+    }
+    __syncthreads();
+    general_products_call(smem, ctl.rk, ctl.rq, tid);
+    uint4 tq[4], td[4], tk[4], aq[2];
+    const float* sG = reinterpret_cast<const float*>(smem);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int i = tid + kThreads * it, r = i >> 4, col = (i & 15) * 8;
+      decayed_piece(sG + r * LDF + col, sG + 63 * LDF + col, *reinterpret_cast<const uint4*>(smem + IG_Q + (r * LDH + col) * 2),
+                    *reinterpret_cast<const uint4*>(smem + IG_K + (r * LDH + col) * 2), ctl.rq[r], ctl.rk[r], tq[it], td[it], tk[it]);
+    }
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const int i = tid + kThreads * it, r = i >> 3, col = (i & 7) * 8;
+      aq[it] = *reinterpret_cast<const uint4*>(smem + IG_AQK + (r * LDQ + col) * 2);
+      uint32_t* w = reinterpret_cast<uint32_t*>(&aq[it]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {   // keep j <= r
+        const int j = col + 2 * e;
+        if (j > r) w[e] = 0u;
+        else if (j + 1 > r) w[e] &= 0x0000ffffu;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int i = tid + kThreads * it, r = i >> 4, col = (i & 15) * 8, off = (col >> 6) * 8192 + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4);
+      *reinterpret_cast<uint4*>(smem + IT_KG + off) = tk[it];
+      *reinterpret_cast<uint4*>(smem + IT_QG + off) = tq[it];
+      *reinterpret_cast<uint4*>(smem + IT_KD + off) = td[it];
+    }
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const int i = tid + kThreads * it, r = i >> 3, col = (i & 7) * 8;
+      *reinterpret_cast<uint4*>(smem + IT_AQK + r * 128 + (((col >> 3) ^ (r & 7)) << 4)) = aq[it];
+    }
+    tiles_sync();
+    if (tid == 0) load_v();
+  }
+  __syncthreads();
+  // ---- T = (I + diag(beta) A_kk)^-1 in place, then T diag(beta) as two terms -----------------------------------------------------------------
+  sm100::block_inverse_64(sX, ctl.beta, sX, tid);
+  {
+    uint4 hi[2], lo[2];
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      int r, col;
+      piece64(tid + kThreads * it, r, col);   // eight rows to a quarter warp: the 16-byte reads are free of bank conflicts
+      float a[8], bb[8];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sX + r * LDT + col);
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sX + r * LDT + col + 4);
+      *reinterpret_cast<float4*>(bb) = *reinterpret_cast<const float4*>(ctl.beta + col);
+      *reinterpret_cast<float4*>(bb + 4) = *reinterpret_cast<const float4*>(ctl.beta + col + 4);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = col + 2 * e <= r ? a[2 * e] * bb[2 * e] : 0.f, y = col + 2 * e + 1 <= r ? a[2 * e + 1] * bb[2 * e + 1] : 0.f;
+        const uint32_t u = tc::pack_bf16(x, y);
+        const float2 f = bf2(u);
+        reinterpret_cast<uint32_t*>(&hi[it])[e] = u;
+        reinterpret_cast<uint32_t*>(&lo[it])[e] = tc::pack_bf16(x - f.x, y - f.y);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      int r, col;
+      piece64(tid + kThreads * it, r, col);
+      const int off = r * 128 + (((col >> 3) ^ (r & 7)) << 4);
+      *reinterpret_cast<uint4*>(smem + IS_X + off) = hi[it];
+      *reinterpret_cast<uint4*>(smem + IS_X + 8192 + off) = lo[it];
+    }
+  }
+  tiles_sync();
+  // ---- W^T, U^T: sixteen tokens at a time, N = the rows that they reach; then as tiles [128 channels][64 tokens] ----------------------------------
+  wait_bar(ctl.full_v, wide);
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      const uint64_t kg = tc::smem_desc_sw128(sb + IT_KG, 8192, 1024), vd = tc::smem_desc_sw128(sb + IT_V, 8192, 1024), bd = tc::smem_desc_sw128(sb + IS_X, 128, 1024);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        const uint32_t id = tc::idesc_bf16(128, 64 - 16 * ks, 1, 0);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          tc::mma_ss(tb + 16 * ks, adv(kg, ks * 2048), adv(bd, 8192 * x + ks * (2048 + 32)), id, ks + x > 0);
+          tc::mma_ss(tb + 64 + 16 * ks, adv(vd, ks * 2048), adv(bd, 8192 * x + ks * (2048 + 32)), id, ks + x > 0);
+        }
+      }
+      tc::mma_commit(tc::smem_u32(&ctl.bar[1]));
+    }
+    __syncwarp();
+  }
+  wait_bar(ctl.bar[1], 0);
+  tc::tc_fence_after();
+#pragma unroll
+  for (int y = 0; y < 2; ++y) {
+    uint32_t x[32];
+    tc::tmem_ld32(ta + 64 * y + 32 * hf, x);
+    tc::tc_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint32_t w[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) w[f] = tc::pack_bf16(__uint_as_float(x[8 * e + 2 * f]), __uint_as_float(x[8 * e + 2 * f + 1]));
+      *reinterpret_cast<uint4*>(smem + (y ? IT_KG : IS_X) + row * 128 + (((4 * hf + e) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  tiles_sync();
+  const int g = lane >> 2, t = lane & 3;
+  const uint64_t wd = tc::smem_desc_sw128(sb + IS_X, 128, 1024), ud = tc::smem_desc_sw128(sb + IT_KG, 128, 1024);
+  // ---- N, Z -> fragments ---------------------------------------------------------------------------------------------------------------------
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      const uint64_t kd = tc::smem_desc_sw128(sb + IT_KD, 8192, 1024);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tb, adv(kd, ks * 2048), adv(wd, ks * 32), tc::idesc_bf16(128, 128, 1, 0), ks > 0);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tb + 128, adv(kd, ks * 2048), adv(ud, ks * 32), tc::idesc_bf16(128, 128, 1, 0), ks > 0);
+      tc::mma_commit(tc::smem_u32(&ctl.bar[2]));
+    }
+    __syncwarp();
+  }
+  wait_bar(ctl.bar[2], 0);
+  tc::tc_fence_after();
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {   // sixteen rows at a time, 64 columns
+    const int mt = 2 * (warp & 3) + m;
+    uint32_t x[32];
+    tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 64 * hf, x);
+    tc::tc_wait_ld();
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = mma::pack(-__uint_as_float(x[8 * ks + 2 * e]), -__uint_as_float(x[8 * ks + 2 * e + 1]));
+      P.nf[((chunk * 8 + mt) * 8 + 4 * hf + ks) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 128 + 64 * hf, x);
+    tc::tc_wait_ld();
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+      P.zf[((chunk * 8 + mt) * 16 + 8 * hf + nt) * 32 + lane] =
+          make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  // ---- Y = Qg - A_qk W, A_qk U -> fragments -------------------------------------------------------------------------------------------------------
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      const uint64_t ad = tc::smem_desc_sw128(sb + IT_AQK, 128, 1024);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tb, adv(ad, ks * 32), adv(wd, ks * 32), tc::idesc_bf16(128, 128, 0, 0), ks > 0);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tb + 128, adv(ad, ks * 32), adv(ud, ks * 32), tc::idesc_bf16(128, 128, 0, 0), ks > 0);
+      tc::mma_commit(tc::smem_u32(&ctl.bar[3]));
+    }
+    __syncwarp();
+  }
+  wait_bar(ctl.bar[3], 0);
+  tc::tc_fence_after();
+  if ((warp & 3) < 2) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int mt = 2 * (warp & 3) + m;
+      uint32_t x[32];
+      tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 64 * hf, x);
+      tc::tc_wait_ld();
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {   // e & 1: row half, e >> 1: column half
+          const int r = 16 * mt + g + 8 * (e & 1);   // (r & 7 is g)
+          const float2 q = bf2(*reinterpret_cast<const uint32_t*>(smem + IT_QG + hf * 8192 + r * 128 + (((2 * ks + (e >> 1)) ^ g) << 4) + 4 * t));
+          const int i = 8 * ks + 4 * (e >> 1) + 2 * (e & 1);
+          w[e] = mma::pack(q.x - __uint_as_float(x[i]), q.y - __uint_as_float(x[i + 1]));
+        }
+        P.yf[((chunk * 4 + mt) * 8 + 4 * hf + ks) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 128 + 64 * hf, x);
+      tc::tc_wait_ld();
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+        P.of[((chunk * 4 + mt) * 16 + 8 * hf + nt) * 32 + lane] =
+            make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tb, 256);
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
@@ -1592,7 +1755,7 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (attr_dev != dev) {
-    e = cudaFuncSetAttribute(intra_trans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_TOTAL);
+    e = cudaFuncSetAttribute(intra_trans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IT_TOTAL);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<2>::kTotal);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(trans_state_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrSmem<4>::kTotal);
     if (e != cudaSuccess) return e;
@@ -1607,7 +1770,12 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;
   P.of = reinterpret_cast<float4*>(w); w += nc * kTrO;
   P.el = reinterpret_cast<float*>(w);
-  e = launch_pdl(intra_trans_kernel, dim3((unsigned)nc), dim3(kThreads), IN_TOTAL, stream, P);
+  const SeqMap& m = p.map;
+  if (!sm100::make_panel_map(&P.tq, p.q, m.B, m.Hq, m.T, m.bthd != 0) || !sm100::make_panel_map(&P.tk, p.k, m.B, m.Hq, m.T, m.bthd != 0) ||
+      !sm100::make_panel_map(&P.tv, p.v, m.B, m.H, m.T, m.bthd != 0) ||
+      (p.variant == DR_KDA && !sm100::make_output_map(&P.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4)))
+    return cudaErrorInvalidValue;
+  e = launch_pdl(intra_trans_kernel, dim3((unsigned)nc), dim3(kThreads), IT_TOTAL, stream, P);
   if (e != cudaSuccess) return e;
   // 16 columns per CTA while the slices fit one wave: the chain's length is what counts
   if (units <= 6) return launch_pdl(trans_state_kernel<2, false>, dim3((unsigned)(units * 8)), dim3(kTrThreads<false>), 0, stream, P);   // see the kernel

@@ -114,3 +114,22 @@ def test_transition_form_reset_inside_a_block(variant, D, tokens, decay):
     assert _lib.last_path() == "chunk_transition"
     ro, rs = _truth(variant, i)
     assert _err(o, ro) <= 5e-6 and _err(s, rs) <= 5e-6
+
+
+@pytest.mark.parametrize("variant,T", [("kda", 1100), ("gated", 400)])
+def test_transition_form_bf16_wide_chunks(variant, T):
+    """bf16: chunks that decay by more than 2^64 in some channel take the 16-row form, the others one product; a positive log decay too.  bf16
+    operands and float32 sums: 2e-2 of the largest value, the budget of the other bf16 forwards."""
+    inp = O.make_inputs(variant, 1, 3, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
+    g = inp["g"]
+    for h, x in enumerate((-44.3 / 64, -44.4 / 64, -300.0)):
+        (g[:, h, 64:128, 5] if variant == "kda" else g[:, h, 64:128])[...] = x
+    (g[:, 1, 200, 7] if variant == "kda" else g[:, 1, 200])[...] = 0.05
+    cu = {k: (None if v is None else v.cuda()) for k, v in inp.items()}
+    op, ref = (L.kda_chunkwise, O.kda_recurrent) if variant == "kda" else (L.gated_delta_rule_chunkwise, O.gated_delta_rule_recurrent)
+    o, hT = op(cu["q"], cu["k"], cu["v"], cu["g"], cu["beta"], initial_state=cu["h0"], chunk_size=64)
+    assert _lib.last_path() == "chunk_transition"
+    L.check_device_status()
+    ro, rS = ref(*(inp[x].double() for x in ("q", "k", "v", "g", "beta")), initial_state=inp["h0"].double(), compute_dtype=torch.float64)
+    for got, want in ((o, ro), (hT, rS)):
+        assert (got.double().cpu() - want).abs().max() <= 2e-2 * want.abs().max()
