@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
   extern __shared__ __align__(1024) uint8_t chain_smem[];
   uint8_t* const smem = chain_smem;
   __shared__ __align__(8) struct {
-    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y, bar_d, full_o[2];
+    // (Y^T d_o of a chunk may be done before the slowest worker asks for the chunk before's, hence two barriers by turns; tests/test_chain_handover.py)
+    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y[2], bar_d, full_o[2];
     uint32_t tmem_base;
     int abort;
     uint32_t top_s[4], top_o[8];   // largest entries of dS and d_o, by turns
@@ -610,7 +611,8 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
     }
     tc::mbar_init(tc::smem_u32(&ctl.full_l), 1);
     tc::mbar_init(tc::smem_u32(&ctl.rdy), 256);
-    tc::mbar_init(tc::smem_u32(&ctl.bar_y), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.bar_y[0]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.bar_y[1]), 1);
     tc::mbar_init(tc::smem_u32(&ctl.bar_d), 1);
     tc::fence_mbar_init();
     ctl.abort = 0;
@@ -662,7 +664,7 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
           tc::mma_ss(acc, adv(yd, ks * 256), adv(od, ks * 2048), id, ks > 0);
           tc::mma_ss(acc, adv(yd, kYTile / 2 + ks * 256), adv(od, ks * 2048), id, 1);
         }
-        tc::mma_commit(tc::smem_u32(&ctl.bar_y));
+        tc::mma_commit(tc::smem_u32(&ctl.bar_y[it & 1]));
         wait_bar(ctl.full_h[it & 1], (it >> 1) & 1);
         wait_bar(ctl.rdy, it & 1);
         tc::tc_fence_after();
@@ -677,7 +679,7 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc_n, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
         tc::mma_commit(tc::smem_u32(&ctl.bar_d));
-        wait_bar(ctl.bar_y, it & 1);   // Y^T and d_o have been read
+        wait_bar(ctl.bar_y[it & 1], (it >> 1) & 1);   // Y^T and d_o have been read
         if (it + 2 < steps) load_y(it + 2);
         wait_bar(ctl.bar_d, it & 1);   // N has been read
         if (it + 1 < steps) load_l(it + 1);
@@ -785,7 +787,7 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
       if (it == steps) break;
       uint32_t d[32];
       if constexpr (KDA) {   // Y^T d_o is long done
-        wait_bar(ctl.bar_y, it & 1);
+        wait_bar(ctl.bar_y[it & 1], (it >> 1) & 1);
         tc::tc_fence_after();
         tc::tmem_ld32(tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
         tc::tc_wait_ld();

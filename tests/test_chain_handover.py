@@ -1,0 +1,65 @@
+"""The barriers of the backward's serial pass (chain_kernel) between the warp that issues products, the tensor pipe and the workers, explored on the
+CPU over every order in which they can proceed.  How many barriers announce Y^T d_o is read from the kernel's source.
+
+The property: nobody passes a wait before its phase is complete, and nobody waits for a phase that the barrier has left behind (a wait by parity then
+returns only with the next one of that parity, which may never come)."""
+import re
+from pathlib import Path
+
+SRC = (Path(__file__).resolve().parents[1] / "linearnexus_b200" / "csrc" / "dr_bwd_chunk.cuh").read_text()
+
+
+def explore(slots, chunks, workers=2):
+    """None, or a text that says what goes wrong.  A state: the issuer's step, products issued and completed (alternately Y^T d_o and N dS), the step of
+    every worker.  Steps per chunk, issuer: issue Y^T d_o; wait for all workers, issue N dS; wait for the one; wait for the other.  Worker:
+    announce dS; wait for Y^T d_o; wait for N dS."""
+    def passes(done, n):   # a wait for phase n by parity, `done` phases complete: None when it passes too early
+        if done & 1 == n & 1:
+            return False
+        return True if done > n else None
+    start = (0, 0, 0, (0,) * workers)
+    seen, todo = {start}, [start]
+    while todo:
+        issuer, issued, completed, work = todo.pop()
+        y_done, d_done = (completed + 1) // 2, completed // 2
+        on = lambda n: (y_done - n % slots + slots - 1) // slots   # phases complete of the barrier that chunk n's Y^T d_o arrives on
+        out = []
+        if completed < issued:
+            out.append((issuer, issued, completed + 1, work))
+        it, step = divmod(issuer, 4)
+        if it < chunks:
+            if step == 0:
+                out.append((issuer + 1, issued + 1, completed, work))
+            elif step == 1:
+                if all(w > 3 * it for w in work):
+                    out.append((issuer + 1, issued + 1, completed, work))
+            else:
+                ok = passes(on(it), it // slots) if step == 2 else passes(d_done, it)
+                if ok is None:
+                    return f"the issuer passes its wait in chunk {it} too early"
+                if ok:
+                    out.append((issuer + 1, issued, completed, work))
+        for i, w in enumerate(work):
+            it, step = divmod(w, 3)
+            if it >= chunks:
+                continue
+            ok = True if step == 0 else passes(on(it), it // slots) if step == 1 else passes(d_done, it)
+            if ok is None:
+                return f"a worker passes its wait in chunk {it} too early"
+            if ok:
+                out.append((issuer, issued, completed, work[:i] + (w + 1,) + work[i + 1:]))
+        if not out and (issuer < 4 * chunks or any(w < 3 * chunks for w in work)):
+            return f"nothing can proceed: issuer in chunk {issuer // 4}, workers in {[w // 3 for w in work]}"
+        for s in out:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return None
+
+
+def test_chain_handover_in_every_order():
+    slots = int(re.search(r"bar_y\[(\d)\], bar_d", SRC).group(1))
+    waits = re.findall(r"wait_bar\(ctl\.bar_y\[it & 1\], \(it >> 1\) & 1\)", SRC)
+    assert slots == 2 and len(waits) == 2 and "mma_commit(tc::smem_u32(&ctl.bar_y[it & 1]))" in SRC
+    assert explore(slots, 7) is None
+    assert "nothing can proceed" in explore(1, 7)   # one barrier: a worker that is late by a product waits for good
