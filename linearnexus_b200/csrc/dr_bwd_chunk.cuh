@@ -1443,6 +1443,9 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
       e = KDA ? cudaFuncSetAttribute(local_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_TOTAL)
               : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal);
+    cudaFuncAttributes at{};
+    if (KDA && e == cudaSuccess) e = cudaFuncGetAttributes(&at, local_sm100_kda_kernel);
+    if (KDA && e == cudaSuccess && at.numRegs != kLkRegs) e = cudaErrorInvalidConfiguration;   // its register split counts on them
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(pre_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_TOTAL);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
@@ -1460,7 +1463,7 @@ inline cudaError_t launch_pre_t(const Params& p, int64_t units, int32_t* status,
   const int64_t chunks = units * p.N;
   if (KDA && !p.few) {
     PreParams pp;
-    pp.p = p; pp.chunks = (int)chunks; pp.status = status;
+    pp.p = p; pp.chunks = (int)chunks; pp.status = status; pp.n_tok = units * p.map.T;
     const SeqMap& m = p.map;
     if (!sm100::make_panel_map(&pp.tq, p.q, m.B, m.Hq, m.T, m.bthd != 0) || !sm100::make_panel_map(&pp.tk, p.k, m.B, m.Hq, m.T, m.bthd != 0) ||
         !sm100::make_output_map(&pp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
@@ -1509,7 +1512,7 @@ inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* sta
     if (p.few) return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
     if (!sm100::make_output_map(&lp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
       return cudaErrorInvalidValue;
-    e = launch_pdl(local_sm100_kda_kernel, grid, dim3(kLtThreads), LK_TOTAL, stream, lp);
+    e = launch_pdl(local_sm100_kda_kernel, grid, dim3(kLkThreads), LK_TOTAL, stream, lp);
     if (e != cudaSuccess) return e;
     return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
   } else {

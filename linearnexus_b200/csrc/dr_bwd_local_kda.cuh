@@ -18,7 +18,7 @@
 // A thread of an epilogue owns one channel and sixteen tokens, and so does the one that forms Kg, Kd and Qg: G stays in its registers.  The
 // three are formed twice, before the products of 1 and of 4: beside the states (128 KB) there is no room to keep them.
 //
-// What bounds it: B=2, T=4096, H=16 (2048 chunks, 14 per CTA): 342 us, 49 K cycles per chunk, where local_kernel takes 882 us (three tf32 products on
+// What bounds it: B=2, T=4096, H=16 (2048 chunks, 14 per CTA): 330 us, 48 K cycles per chunk, where local_kernel takes 882 us (three tf32 products on
 // mma.sync, 119 K); the training step 1490 -> 966 us, 265 -> 197 at B=1, T=1000.  Issue slots 34 %, tensor pipe 16 %: the element-wise work between the
 // products, 4.2 K instructions per warp, and the barriers around the largest entries.  Almost nothing is left for an L1, so what is not in
 // shared memory costs an L2 access: with g, q, X, A and T by loads of the warps 71 K cycles, with everything the compiler would keep over the
@@ -53,7 +53,11 @@ struct LkCtl {
 };
 constexpr int LK_TOTAL = LK_CTL + sizeof(LkCtl);
 static_assert(LK_TOTAL <= 232448 && LK_CTL % 16 == 0 && offsetof(LkCtl, beta) % 16 == 0 && offsetof(LkSums, f) % 16 == 0, "shared memory");
-static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(const __grid_constant__ LocalParams P) {
+// Registers: 640 threads of 96 (the fifth warp group is the issuing warp and three that leave); the workers take 104, the issuing group keeps 64, which
+// adds up to what the block was launched with (launch_adjoint_t asks for 96).  With 544 threads and 96 each 1.4 % slower, spills 308 bytes against 136.
+constexpr int kLkThreads = 640, kLkRegs = 96, kLkWorkerRegs = 104, kLkIssueRegs = 64;
+static_assert(512 * kLkWorkerRegs + 128 * kLkIssueRegs <= kLkThreads * kLkRegs, "the split waits for good otherwise");
+static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(const __grid_constant__ LocalParams P) {
   const Params& p = P.p;
   extern __shared__ __align__(1024) uint8_t lk_smem[];
   uint8_t* const smem = lk_smem;
@@ -94,7 +98,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
   ChunkList<false> list;
   list.start(p, P.chunks, lane);
 
-  if (warp == 16) {
+  if (warp >= 16) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLkIssueRegs));
+    if (warp == 16) {
     // (only the low word changes: the address field does not carry into the other)
     auto adv = [](uint64_t d, uint32_t bytes) { return (d & 0xffffffff00000000ull) | ((uint32_t)d + (bytes >> 4)); };
     auto commit = [&](int i) { tc::mma_commit(tc::smem_u32(&ctl.bar[i])); };
@@ -351,7 +357,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kda_kernel(c
       }
       __syncwarp();
     }
+    }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kLkWorkerRegs));
     uint32_t ph = 0;
 #pragma unroll 1
     for (int c = list.next(p, P.chunks, lane); c < P.chunks; c = list.next(p, P.chunks, lane), ph ^= 1) {

@@ -42,6 +42,7 @@ struct alignas(64) PreParams {
   Params p;
   int chunks;
   int32_t* status;
+  int64_t n_tok;   // entries of the arrays with one number per token (index checks of the debug build)
 };
 
 static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(const __grid_constant__ PreParams P) {
@@ -84,8 +85,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
     auto load = [&](int c, uint32_t turn) {
       const int unit = c / p.N, b = unit / p.map.H, h = unit % p.map.H, hq = p.map.hq(h), t0 = (c % p.N) * kC, rows = min(kC, p.map.T - t0);
       const int64_t at = p.map.base(b, h, 1) + (int64_t)t0 * p.map.tok(1), tok = p.map.tok(1);
-      ctl.beta[turn][lane] = lane < rows ? p.beta[at + lane * tok] : 0.f;
-      ctl.beta[turn][lane + 32] = lane + 32 < rows ? p.beta[at + (lane + 32) * tok] : 0.f;
+      auto in = [&](int i) { return i < rows && in_bounds(P.status, at + i * tok, P.n_tok); };
+      ctl.beta[turn][lane] = in(lane) ? p.beta[at + lane * tok] : 0.f;
+      ctl.beta[turn][lane + 32] = in(lane + 32) ? p.beta[at + (lane + 32) * tok] : 0.f;
       __syncwarp();   // (before the barrier is armed: who waits for it sees them)
       if (tc::elect_one()) {
         const uint32_t bar = tc::smem_u32(&ctl.full);
