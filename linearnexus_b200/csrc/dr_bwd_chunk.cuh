@@ -8,7 +8,7 @@
 //   pre_kernel    one CTA per chunk, beside the forward (q, k, g, beta only): X, A, T, and N, Y as chain_kernel's tiles.  Per-channel decays:
 //                 pre_sm100_kda_kernel (dr_bwd_pre_kda.cuh), persistent, on tcgen05, and pre_kernel for the chunks that it leaves.
 //   chain_kernel  one CTA per (sequence, 64 value columns) walks the chunks backwards on tcgen05, dS in registers; stores dS1 of every
-//                 chunk.  N and Y as two bf16 terms; per-channel decays: two fp16 terms of scaled operands.
+//                 chunk.  N and Y as two bf16 terms; per-channel decays: three.
 //   the local pass, all chunks in parallel: everything else, from S0 (the forward's checkpoint), dS1 and the chunk's inputs; then the
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
 //                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
@@ -98,11 +98,11 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
 }
 // Per-channel decays: what the pre-pass leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
 // whether the chunk is pre_kernel's and local_kernel's (a channel decays by more than 2^16, or a decay is positive) or pre_sm100_kda_kernel's and
-// local_sm100_kda_kernel's, and the largest entries (A, T) or bounds of them (k^, q^, N, Y), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
+// local_sm100_kda_kernel's, and the largest entries (A, T) or bounds of them (k^, q^), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
 // in fours, A and T as two fp16 terms in tiles.
 constexpr float kWideKda = 16.f;   // log2 units
 constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096, kXTop = 2097;
-enum { kTopA, kTopT, kTopK, kTopQ, kTopN, kTopY, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
+enum { kTopA, kTopT, kTopK, kTopQ, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
 
 // the power of two that brings `top` to 2^13 .. 2^14 (none for zero and infinity); its inverse
 __device__ __forceinline__ float lift(uint32_t top) {
@@ -121,15 +121,14 @@ __device__ __forceinline__ void split2h(float x, float y, uint32_t& hi, uint32_t
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = pack_h(x - f.x, y - f.y);
 }
-// store_terms for fp16 terms of `s` times the entries
-__device__ __forceinline__ void store_terms_h(uint8_t* dst, int next, int lo, const float (&d)[4], float s) {
+// Per-channel decays: Y^T and the two halves of N's columns in float32, [128 rows][64 columns] each: eight columns of a row are a unit, eight rows'
+// units of the same columns follow each other; the first four columns of all units, then the others.  An m16n8 accumulator (lane g, t) of column
+// tile nt, rows r0 + g and eight further on.
+constexpr int kHalf4 = 128 * 64 / 4;   // float4 of one such array
+__device__ __forceinline__ void store_f32(float4* dst, int r0, int nt, int g, int t, const float (&d)[4]) {
 #pragma unroll
-  for (int hr = 0; hr < 2; ++hr) {
-    uint32_t h, l;
-    split2h(s * d[2 * hr], s * d[2 * hr + 1], h, l);
-    *reinterpret_cast<uint32_t*>(dst + hr * next) = h;
-    *reinterpret_cast<uint32_t*>(dst + hr * next + lo) = l;
-  }
+  for (int hr = 0; hr < 2; ++hr)
+    reinterpret_cast<float2*>(dst + (t >> 1) * (kHalf4 / 2) + ((r0 >> 3) + hr) * 64 + nt * 8 + g)[t & 1] = make_float2(d[2 * hr], d[2 * hr + 1]);
 }
 // Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation.
 __host__ __device__ constexpr uint32_t idesc_fp16(int M, int N, int a_mn_major, int b_mn_major) {
@@ -189,7 +188,6 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
   float *sRk = sBeta + 64, *sRq = sBeta + 128, *sGs = sBeta + 192, *sFw = sBeta + 256, *sFd = sBeta + 320;
   float* sG = reinterpret_cast<float*>(smem + PR_G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  __shared__ uint32_t sTop[3];     // largest entries of Y, W and Kd
   ChunkList<true> list;
   if constexpr (KDA) list.start(p, chunks, lane);
 #pragma unroll 1
@@ -202,7 +200,6 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
   if constexpr (KDA) {
     __syncthreads();   // the chunk before is done with shared memory
-    if (tid < 3) sTop[tid] = 0u;
   }
   // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
   {
@@ -467,29 +464,17 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
         }
       }
     }
-    if constexpr (KDA) {
-      float m = 0.f, w = 0.f;
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { m = fmaxf(m, fabsf(Y[nt][e])); w = fmaxf(w, fabsf(W[nt][e])); }
-      atomicMax(&sTop[0], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-      atomicMax(&sTop[1], __reduce_max_sync(0xffffffffu, __float_as_uint(w)));
-      __syncthreads();
-      if (tid == 0) xat[kXTop + kTopY] = __uint_as_float(sTop[0]);
-    }
     uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + chunk * kYTile + 2 * warp * kYRbs + g * 16 + 4 * t;
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      if constexpr (KDA) store_terms_h(dst + nt * 128, kYRbs, kYTile / 2, Y[nt], lift(sTop[0])); else store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
+      if constexpr (KDA) store_f32(p.yf + chunk * kHalf4, 16 * warp, nt, g, t, Y[nt]);
+      else store_terms(dst + nt * 128, kYRbs, kYTile / 2, Y[nt]);
     }
   }
-  uint32_t topN = 0u;
   // ---- N = -W^T Kd -> tiles -----------------------------------------------------------------------------------------------
   if constexpr (KDA) {
     // lane = channels lane, lane + 32, ..; warp = token pairs warp, warp + 8, ..; split into the two terms once
     uint4 kd[4][4];
-    float m = 0.f;
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const int c = lane + 32 * x;
@@ -498,22 +483,16 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
       for (int i = 0; i < 4; ++i) {
         const int r = 2 * (warp + 8 * i);
         BFrag<true> f;
-        const float y0 = bf(sK + r * LDH + c) * sRk[r] * ex2(gl - sG[r * LDG + c]), y1 = bf(sK + (r + 1) * LDH + c) * sRk[r + 1] * ex2(gl - sG[(r + 1) * LDG + c]);
-        f.set(y0, y1);
-        m = fmaxf(m, fmaxf(fabsf(y0), fabsf(y1)));
+        f.set(bf(sK + r * LDH + c) * sRk[r] * ex2(gl - sG[r * LDG + c]), bf(sK + (r + 1) * LDH + c) * sRk[r + 1] * ex2(gl - sG[(r + 1) * LDG + c]));
         kd[i][x] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
       }
     }
-    atomicMax(&sTop[2], __reduce_max_sync(0xffffffffu, __float_as_uint(m)));
     __syncthreads();   // every read of k, q, X and A is done
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int x = 0; x < 4; ++x) sKd[(warp + 8 * i) * LDK + lane + 32 * x] = kd[i][x];
     __syncthreads();
-    // |N| <= 64 |W| |Kd|: loose by some 2^7 of the 2^18 that the terms have to spare
-    topN = __float_as_uint(64.f * __uint_as_float(sTop[1]) * __uint_as_float(sTop[2]));
-    if (tid == 0) xat[kXTop + kTopN] = __uint_as_float(topN);
   }
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
@@ -542,7 +521,8 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
     uint8_t* dst = reinterpret_cast<uint8_t*>(p.nf) + chunk * kNTile + 2 * warp * sm100::RBS + 8 * half * 128 + g * 16 + 4 * t;
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      if constexpr (KDA) store_terms_h(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt], lift(topN)); else store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
+      if constexpr (KDA) store_f32(p.nf + (2 * chunk + half) * kHalf4, 16 * warp, nt, g, t, d[nt]);
+      else store_terms(dst + nt * 128, sm100::RBS, kNTile / 2, d[nt]);
     }
   }
   }
@@ -566,15 +546,23 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
 // while dS is zero does not change that).  Forward and backward together, 1 to 256 sequences: 1 to 9 % faster at five chunks, 4 to
 // 13 % at 16, 6 to 14 % at 64; from 48 sequences on ahead or level at every length.
 // =====================================================================================================================
-// Per-channel decays: two fp16 terms of operands whose largest entry is brought to 2^13 and above (22 bits; pre_kernel gives the bounds of N and Y),
-// the two products with accumulators of their own; four more warps find the power of two for d_o and turn it into fp16 where it lies.
+// Per-channel decays: the N of a strongly decaying chunk is as small as the decay, row by row, and what it adds to dS as large as the rest, so
+// float32 operands are three bf16 terms each (24 bits of every entry, float32's exponents), six products per pair.  N and Y arrive in float32 by
+// bulk copies; eight more warps turn them into terms in tensor memory, N in halves of 64 channels: the first as soon as the products with the chunk
+// before's first half are done, so that it is ready when they all are.  Y^T d_o has accumulators of its own.  B=2, T=4096, H=16: 153 us under ncu, where
+// two fp16 terms of operands scaled as a whole take 138 to 145 and lose N, and with it every gradient before such a chunk, from 0.35 nats a
+// token in every channel on; with the terms in shared memory and N by loads into registers 310 us (no L1 to load through).
 constexpr int kChThreads = 288, kChCols = 64;   // eight worker warps and one that issues
-constexpr int kChWarpsKda = 4;
-template <bool KDA> constexpr int ch_threads() { return kChThreads + (KDA ? 32 * kChWarpsKda : 0); }
+constexpr int kChSplit = 256;
+template <bool KDA> constexpr int ch_threads() { return kChThreads + (KDA ? kChSplit : 0); }
 // N hi twice, N lo, Y^T and d_o twice, the terms of dS, staging of its rows
-constexpr int kNTerm = kNTile / 2, kOTile = 64 * 128;
-constexpr int CH_H = 0, CH_L = CH_H + 2 * kNTerm, CH_Y = CH_L + kNTerm, CH_O = CH_Y + 2 * kYTile, CH_S = CH_O + 2 * kOTile, CH_G = CH_S + 2 * 128 * 128, CH_TOTAL = CH_G + 8 * 2048;
-static_assert(CH_O % 1024 == 0 && CH_S % 1024 == 0 && CH_TOTAL <= 232448 - 1024, "shared memory");
+constexpr int kNTerm = kNTile / 2, kSTerm = 128 * 128, kOTile = 64 * 128;
+constexpr int CH_H = 0, CH_L = CH_H + 2 * kNTerm, CH_Y = CH_L + kNTerm, CH_O = CH_Y + 2 * kYTile, CH_S = CH_O + 2 * kOTile, CH_G = CH_S + 2 * kSTerm, CH_TOTAL = CH_G + 8 * 2048;
+// per-channel decays: the terms of dS, d_o twice, staging, Y^T, three halves of N as they arrive
+constexpr int kHalfTile = kHalf4 * 16, kHalfSlots = 3;
+constexpr int CK_S = 0, CK_O = CK_S + 3 * kSTerm, CK_G = CK_O + 2 * kOTile, CK_Y = CK_G + 8 * 2048, CK_N = CK_Y + kHalfTile, CK_TOTAL = CK_N + kHalfSlots * kHalfTile;
+static_assert(CH_O % 1024 == 0 && CH_S % 1024 == 0 && CK_O % 1024 == 0 && CH_TOTAL <= 232448 - 1024 && CK_TOTAL <= 232448 - 1024, "shared memory");
+template <bool KDA> constexpr int ch_smem() { return KDA ? CK_TOTAL : CH_TOTAL; }
 struct alignas(64) ChainParams {
   CUtensorMap to;   // panels of d_o (see sm100::make_panel_map)
   Params p;
@@ -589,12 +577,13 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
   uint8_t* const smem = chain_smem;
   __shared__ __align__(8) struct {
     // (Y^T d_o of a chunk may be done before the slowest worker asks for the chunk before's, hence two barriers by turns; tests/test_chain_handover.py)
-    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y[2], bar_d, full_o[2];
+    // Per-channel decays: full_h: terms of N's halves, full_l: terms of Y, full_y[0]: Y has arrived, full_n: halves of N have, bar_e: products with N's first half
+    uint64_t full_h[2], full_l, full_y[2], rdy, bar_y[2], bar_d, full_o[2], full_n[kHalfSlots], bar_e;
     uint32_t tmem_base;
     int abort;
-    uint32_t top_s[4], top_o[8];   // largest entries of dS and d_o, by turns
   } ctl;
-  constexpr uint32_t kTmem = KDA ? 256 : 128, kTmemN = 128;   // (KDA: N dS behind the two accumulators of Y^T d_o)
+  // KDA: N dS behind the two accumulators of Y^T d_o, then the terms of N (64 columns each) and of Y
+  constexpr uint32_t kTmem = KDA ? 512 : 128, kTmemN = 128, kTmemA = 192, kTmemY = kTmemA + 3 * 64;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int unit = blockIdx.x / (kD / kChCols), v0 = blockIdx.x % (kD / kChCols) * kChCols;
   const int b = unit / p.map.H, h = unit % p.map.H;
@@ -602,14 +591,15 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
     tc::tmem_alloc(tc::smem_u32(&ctl.tmem_base), kTmem);
     tc::tmem_relinquish();
   }
-  if (tid < 8) ctl.top_s[tid & 3] = ctl.top_o[tid] = 0u;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(tc::smem_u32(&ctl.full_o[i]), 32 * kChWarpsKda);
-      tc::mbar_init(tc::smem_u32(&ctl.full_h[i]), 1);
+      tc::mbar_init(tc::smem_u32(&ctl.full_o[i]), 1);
+      tc::mbar_init(tc::smem_u32(&ctl.full_h[i]), KDA ? kChSplit : 1);
       tc::mbar_init(tc::smem_u32(&ctl.full_y[i]), 1);
     }
-    tc::mbar_init(tc::smem_u32(&ctl.full_l), 1);
+    for (int i = 0; i < kHalfSlots; ++i) tc::mbar_init(tc::smem_u32(&ctl.full_n[i]), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.bar_e), 1);
+    tc::mbar_init(tc::smem_u32(&ctl.full_l), KDA ? kChSplit : 1);
     tc::mbar_init(tc::smem_u32(&ctl.rdy), 256);
     tc::mbar_init(tc::smem_u32(&ctl.bar_y[0]), 1);
     tc::mbar_init(tc::smem_u32(&ctl.bar_y[1]), 1);
@@ -628,7 +618,65 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
   };
   const int64_t chunk0 = (int64_t)unit * p.N;
   const int steps = p.dh0 ? p.N : p.N - 1;   // the product of the first chunk gives the initial state's gradient alone
-  if (warp == 8) {
+  auto y_done = [&](int it) { wait_bar(ctl.bar_y[it & 1], (it >> 1) & 1); };
+  constexpr uint32_t id = tc::idesc_bf16(128, 64, 0, 1);
+  auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
+  if (KDA && warp == 8) {
+    if (tc::elect_one()) {
+      auto load_o = [&](int it) {
+        const uint32_t bar = tc::smem_u32(&ctl.full_o[it & 1]);
+        tc::mbar_arrive_expect_tx(bar, kOTile);
+        tc::tma_load_4d(sbase + CK_O + (it & 1) * kOTile, &P.to, v0, h, (p.N - 1 - it) * kC, b, bar);
+      };
+      auto load_y = [&](int it) {
+        const uint32_t bar = tc::smem_u32(&ctl.full_y[0]);
+        tc::mbar_arrive_expect_tx(bar, kHalfTile);
+        tc::bulk_g2s(sbase + CK_Y, p.yf + (chunk0 + p.N - 1 - it) * kHalf4, kHalfTile, bar);
+      };
+      auto load_n = [&](int i) {   // half i & 1 of chunk i / 2
+        const uint32_t bar = tc::smem_u32(&ctl.full_n[i % kHalfSlots]);
+        tc::mbar_arrive_expect_tx(bar, kHalfTile);
+        tc::bulk_g2s(sbase + CK_N + (i % kHalfSlots) * kHalfTile, p.nf + (2 * (chunk0 + p.N - 1 - (i >> 1)) + (i & 1)) * kHalf4, kHalfTile, bar);
+      };
+      if (steps > 0) { load_y(0); load_o(0); }
+      for (int i = 0; i < kHalfSlots && i < 2 * steps; ++i) load_n(i);
+      if (steps > 1) load_o(1);
+      const uint64_t sd = tc::smem_desc_sw128(sbase + CK_S, kSTerm, 1024);
+      const uint32_t acc_n = tbase + kTmemN;
+      constexpr uint32_t left[6] = {0, 0, 0, 1, 1, 2}, right[6] = {0, 1, 2, 0, 1, 0};   // terms of N and of dS
+#pragma unroll 1
+      for (int it = 0; it < steps; ++it) {
+        const uint32_t acc = tbase + (it & 1) * 64;   // (read for chunk it - 2 before its successor's dS was ready)
+        const uint64_t od = tc::smem_desc_sw128(sbase + CK_O + (it & 1) * kOTile, kSTerm, 1024);
+        wait_bar(ctl.full_o[it & 1], (it >> 1) & 1);
+        wait_bar(ctl.full_l, it & 1);
+        if (it + 1 < steps) load_y(it + 1);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+          for (int x = 0; x < 3; ++x) tc::mma_ts(acc, tbase + kTmemY + 32 * x + 8 * ks, adv(od, ks * 2048), id, ks + x > 0);
+        tc::mma_commit(tc::smem_u32(&ctl.bar_y[it & 1]));
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          wait_bar(ctl.full_h[hf], it & 1);
+          if (2 * it + hf + kHalfSlots < 2 * steps) load_n(2 * it + hf + kHalfSlots);
+          if (hf == 0) wait_bar(ctl.rdy, it & 1);
+          tc::tc_fence_after();
+#pragma unroll
+          for (int ks = 4 * hf; ks < 4 * hf + 4; ++ks)
+#pragma unroll
+            for (int x = 0; x < 6; ++x) tc::mma_ts(acc_n, tbase + kTmemA + 64 * left[x] + 8 * ks, adv(sd, right[x] * kSTerm + ks * 2048), id, ks + x > 0);
+          tc::mma_commit(tc::smem_u32(hf ? &ctl.bar_d : &ctl.bar_e));
+        }
+        if (it + 2 < steps) {
+          y_done(it);   // d_o has been read
+          load_o(it + 2);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 8) {
     if (tc::elect_one()) {
       auto n_at = [&](int it) { return reinterpret_cast<const uint8_t*>(p.nf) + (chunk0 + p.N - 1 - it) * kNTile; };
       auto y_at = [&](int it) { return reinterpret_cast<const uint8_t*>(p.yf) + (chunk0 + p.N - 1 - it) * kYTile; };
@@ -647,8 +695,6 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
       };
       if (steps > 0) { load_y(0); load_h(0); load_l(0); }
       if (steps > 1) { load_y(1); load_h(1); }
-      constexpr uint32_t id = KDA ? idesc_fp16(128, 64, 0, 1) : tc::idesc_bf16(128, 64, 0, 1);
-      auto adv = [](uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); };
       const uint64_t sd = tc::smem_desc_sw128(sbase + CH_S, 128 * 128, 1024), ld = tc::smem_desc(sbase + CH_L, 128, sm100::RBS);
 #pragma unroll 1
       for (int it = 0; it < steps; ++it) {
@@ -657,7 +703,6 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
         const uint64_t od = tc::smem_desc_sw128(sbase + CH_O + (it & 1) * kOTile, 128 * 128, 1024);
         const uint64_t hd = tc::smem_desc(sbase + CH_H + (it & 1) * kNTerm, 128, sm100::RBS);
         wait_bar(ctl.full_y[it & 1], (it >> 1) & 1);
-        if constexpr (KDA) wait_bar(ctl.full_o[it & 1], (it >> 1) & 1);
         tc::tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
@@ -668,18 +713,17 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
         wait_bar(ctl.full_h[it & 1], (it >> 1) & 1);
         wait_bar(ctl.rdy, it & 1);
         tc::tc_fence_after();
-        const uint32_t acc_n = KDA ? tbase + kTmemN : acc;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          tc::mma_ss(acc_n, adv(hd, ks * 256), adv(sd, ks * 2048), id, !KDA || ks > 0);
-          tc::mma_ss(acc_n, adv(hd, ks * 256), adv(sd, 128 * 128 + ks * 2048), id, 1);
+          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, ks * 2048), id, 1);
+          tc::mma_ss(acc, adv(hd, ks * 256), adv(sd, kSTerm + ks * 2048), id, 1);
         }
         wait_bar(ctl.full_l, it & 1);
         tc::tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc_n, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
+        for (int ks = 0; ks < 8; ++ks) tc::mma_ss(acc, adv(ld, ks * 256), adv(sd, ks * 2048), id, 1);
         tc::mma_commit(tc::smem_u32(&ctl.bar_d));
-        wait_bar(ctl.bar_y[it & 1], (it >> 1) & 1);   // Y^T and d_o have been read
+        y_done(it);   // Y^T and d_o have been read
         if (it + 2 < steps) load_y(it + 2);
         wait_bar(ctl.bar_d, it & 1);   // N has been read
         if (it + 1 < steps) load_l(it + 1);
@@ -688,41 +732,46 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
     }
     __syncwarp();
   } else if (KDA && warp > 8) {
-    // d_o, two threads to a token: its largest entry, then fp16 in place
-    const int at = (tid - kChThreads) * 64;
+    // thread = row; of 64 columns in shared memory half, as three terms to tensor memory
+    const int row = 32 * (warp & 3) + lane, hc = (warp - 9) >> 2;
+    const uint32_t at = (uint32_t)(32 * (warp & 3)) << 16;
+    auto split = [&](int from, uint32_t to, uint32_t term, uint64_t& full) {
+      const float4* src = reinterpret_cast<const float4*>(smem + from) + (row >> 3) * 64 + 4 * hc * 8 + (row & 7);
+      uint32_t h[16], m[16], l[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = src[8 * i], y = src[kHalf4 / 2 + 8 * i];
+        mma::split3_exact(x.x, x.y, h[4 * i], m[4 * i], l[4 * i]);
+        mma::split3_exact(x.z, x.w, h[4 * i + 1], m[4 * i + 1], l[4 * i + 1]);
+        mma::split3_exact(y.x, y.y, h[4 * i + 2], m[4 * i + 2], l[4 * i + 2]);
+        mma::split3_exact(y.z, y.w, h[4 * i + 3], m[4 * i + 3], l[4 * i + 3]);
+      }
+      to += tbase + at + 16 * hc;
+      tc::tmem_st16(to, h);
+      tc::tmem_st16(to + term, m);
+      tc::tmem_st16(to + 2 * term, l);
+      tc::tc_wait_st();
+      tc::tc_fence_before();
+      sm100::mbar_arrive(tc::smem_u32(&full));
+    };
 #pragma unroll 1
     for (int it = 0; it < steps; ++it) {
-      uint4* tile = reinterpret_cast<uint4*>(smem + CH_O + (it & 1) * kOTile + at);
-      wait_bar(ctl.full_y[it & 1], (it >> 1) & 1);
-      uint4 x[4];
-      float m = 0.f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        x[i] = tile[(i + (lane >> 1)) & 3];   // (pieces skewed by the token: no bank conflicts)
-        const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) m = fmaxf(m, fmaxf(fabsf(mma::lo_f(w[e])), fabsf(mma::hi_f(w[e]))));
+      wait_bar(ctl.full_y[0], it & 1);
+      if (it > 0) { y_done(it - 1); tc::tc_fence_after(); }
+      split(CK_Y, kTmemY, 32, ctl.full_l);
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+        const int i = 2 * it + hf;
+        wait_bar(ctl.full_n[i % kHalfSlots], (i / kHalfSlots) & 1);
+        if (it > 0) { wait_bar(hf ? ctl.bar_d : ctl.bar_e, (it - 1) & 1); tc::tc_fence_after(); }
+        split(CK_N + (i % kHalfSlots) * kHalfTile, kTmemA + 32 * hf, 64, ctl.full_h[hf]);
       }
-      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-      if (lane == 0) atomicMax(&ctl.top_o[it & 7], top);
-      asm volatile("bar.sync 2, 128;" ::: "memory");
-      if (tid == kChThreads) ctl.top_o[(it + 4) & 7] = 0u;   // (the workers are past its last use: this tile came after chunk it - 2's product)
-      const float s = lift(ctl.top_o[it & 7]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) w[e] = pack_h(s * mma::lo_f(w[e]), s * mma::hi_f(w[e]));
-        tile[(i + (lane >> 1)) & 3] = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      tc::fence_async_smem();
-      sm100::mbar_arrive(tc::smem_u32(&ctl.full_o[it & 1]));
     }
   } else {
     const int row = 32 * (warp & 3) + lane, hc = warp >> 2;   // this thread's channel and half of the columns
     const uint32_t lane_addr = (uint32_t)(32 * (warp & 3)) << 16;
     const int64_t at = (int64_t)row * kD + v0 + 32 * hc;
-    uint8_t* stage = smem + CH_G + warp * 2048;
+    uint8_t* stage = smem + (KDA ? CK_G : CH_G) + warp * 2048;
     float S[32];
 #pragma unroll
     for (int c = 0; c < 32; c += 2) {   // (d_hT and dh0 need not be aligned to more than eight bytes)
@@ -733,34 +782,19 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
     for (int it = 0; it < p.N; ++it) {
       const int64_t chunk = chunk0 + p.N - 1 - it;
       const float el = p.el[chunk * 128 + row];
-      float s = 1.f, fn = 1.f, fy = 1.f;
-      if (KDA && it < steps) {
-        const float* xat = p.xat + chunk * (3 * 64 * 64) + kXTop;
-        fn = drop(__float_as_uint(__ldcg(xat + kTopN)));
-        fy = drop(__float_as_uint(__ldcg(xat + kTopY)));
-        float m = 0.f;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) m = fmaxf(m, fabsf(S[c]));
-        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-        if (lane == 0) atomicMax(&ctl.top_s[it & 3], top);
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (tid == 0) ctl.top_s[(it + 2) & 3] = 0u;
-        const uint32_t all = ctl.top_s[it & 3];
-        s = lift(all);
-        fn = fminf(fn * drop(all), 3.4e38f);
-      }
       if (it < steps) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t hi[4], lo[4];
+          uint32_t hi[4], lo[4], last[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float x = S[8 * c + 2 * e], y = S[8 * c + 2 * e + 1];
-            if constexpr (KDA) split2h(s * x, s * y, hi[e], lo[e]); else split2(x, y, hi[e], lo[e]);
+            if constexpr (KDA) mma::split3_exact(x, y, hi[e], lo[e], last[e]); else split2(x, y, hi[e], lo[e]);
           }
-          uint8_t* dst = smem + CH_S + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
+          uint8_t* dst = smem + (KDA ? CK_S : CH_S) + row * 128 + (((4 * hc + c) ^ (row & 7)) << 4);
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(dst + 128 * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(dst + kSTerm) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          if constexpr (KDA) *reinterpret_cast<uint4*>(dst + 2 * kSTerm) = make_uint4(last[0], last[1], last[2], last[3]);
         }
         tc::fence_async_smem();
         sm100::mbar_arrive(tc::smem_u32(&ctl.rdy));
@@ -791,16 +825,15 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
         tc::tc_fence_after();
         tc::tmem_ld32(tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
         tc::tc_wait_ld();
-        fy = fminf(fy * drop(ctl.top_o[it & 7]), 3.4e38f);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) S[c] = S[c] * el + __uint_as_float(d[c]) * fy;
+        for (int c = 0; c < 32; ++c) S[c] = S[c] * el + __uint_as_float(d[c]);
       }
       wait_bar(ctl.bar_d, it & 1);
       tc::tc_fence_after();
       tc::tmem_ld32(KDA ? tbase + lane_addr + kTmemN + 32 * hc : tbase + lane_addr + (it & 1) * 64 + 32 * hc, d);
       tc::tc_wait_ld();
 #pragma unroll
-      for (int c = 0; c < 32; ++c) S[c] = KDA ? S[c] + __uint_as_float(d[c]) * fn : S[c] * el + __uint_as_float(d[c]);
+      for (int c = 0; c < 32; ++c) S[c] = KDA ? S[c] + __uint_as_float(d[c]) : S[c] * el + __uint_as_float(d[c]);
       tc::tc_fence_before();
     }
     if (p.dh0) {
@@ -1448,7 +1481,7 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
     if (KDA && e == cudaSuccess && at.numRegs != kLkRegs) e = cudaErrorInvalidConfiguration;   // its register split counts on them
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(pre_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_TOTAL);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_TOTAL);
+      e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_smem<KDA>());
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) attr_dev = dev;
   }
@@ -1503,7 +1536,7 @@ inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* sta
   c.p = p;
   c.status = status;
   c.to = lp.to;
-  e = launch_pdl(chain_kernel<KDA>, dim3((unsigned)(units * (kD / kChCols))), dim3(ch_threads<KDA>()), CH_TOTAL, stream, c);
+  e = launch_pdl(chain_kernel<KDA>, dim3((unsigned)(units * (kD / kChCols))), dim3(ch_threads<KDA>()), ch_smem<KDA>(), stream, c);
   if (e != cudaSuccess) return e;
   if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
       !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))

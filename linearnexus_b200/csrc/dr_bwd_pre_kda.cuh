@@ -31,7 +31,7 @@ struct PkCtl {
   uint64_t bar[4], full, free;
   alignas(16) float el[128];
   float beta[2][64];
-  uint32_t top[2][8];             // in the order of kTop (N: T diag(beta)); [6]: of W
+  uint32_t top[2][8];             // in the order of kTop, then kTopTb, kTopW
   uint32_t tmem_base;
   int rise[2], wide, abort;
 };
@@ -76,7 +76,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
   };
   // tensor memory: [X; A], W^T, its two terms, W^T A^T, N
   constexpr uint32_t tXA = 0, tW = 64, tWt = 128, tWA = 192, tN = 256;
-  constexpr int kTopW = 6;
+  constexpr int kTopTb = 4, kTopW = 5;   // T diag(beta), W
 
   if (warp == 16) {
     // (only the low word changes: the address field does not carry into the other)
@@ -366,10 +366,10 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           mb = fmaxf(mb, fabsf(y[e]));
         }
         raise(kTopT, m);
-        raise(kTopN, mb);
+        raise(kTopTb, mb);
         workers_sync();
         wait_at(ctl.free, ph ^ 1);
-        const float s = lift(top[kTopT]), sn = lift(top[kTopN]);
+        const float s = lift(top[kTopT]), sn = lift(top[kTopTb]);
         uint32_t h[4], l[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) split2h(s * x[2 * e], s * x[2 * e + 1], h[e], l[e]);
@@ -388,7 +388,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         uint32_t u[16];
         tc::tmem_ld16(ta + tW, u);
         tc::tc_wait_ld();
-        const float f = join(kTopK, kTopN);
+        const float f = join(kTopK, kTopTb);
         float w[16], m = 0.f;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -406,16 +406,11 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         tc::tc_wait_st();
       }
       hand_over(5);
-      // bounds (loose by some 2^7 of the 2^18 that the terms have to spare): |Y| <= |q^| + 64 |A| |W|,  |N| <= 64 |W| |k^|
-      const float w64 = 64.f * __uint_as_float(top[kTopW]);
-      const float top_y = __uint_as_float(top[kTopQ]) + w64 * __uint_as_float(top[kTopA]), top_n = w64 * __uint_as_float(top[kTopK]);
       if (tid == 0) {
         xat[kXTop + kTopA] = __uint_as_float(top[kTopA]);
         xat[kXTop + kTopT] = __uint_as_float(top[kTopT]);
         xat[kXTop + kTopK] = __uint_as_float(top[kTopK]);
         xat[kXTop + kTopQ] = __uint_as_float(top[kTopQ]);
-        xat[kXTop + kTopN] = top_n;
-        xat[kXTop + kTopY] = top_y;
       }
       // ---- Y^T = Qg^T - W^T A^T ------------------------------------------------------------------------------------------------------------------
       {
@@ -432,43 +427,30 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         uint32_t u[16];
         tc::tmem_ld16(ta + tWA, u);
         tc::tc_wait_ld();
-        const float f = join(kTopW, kTopA), s = lift(__float_as_uint(top_y));
-        uint8_t* dst = reinterpret_cast<uint8_t*>(p.yf) + (int64_t)c * kYTile + (row >> 3) * kYRbs + (row & 7) * 16 + 2 * cg * 128;
+        const float f = join(kTopW, kTopA);
+        float4* dst = p.yf + (int64_t)c * kHalf4 + (row >> 3) * 64 + 2 * cg * 8 + (row & 7);   // see store_f32
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t h[4], l[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int j = 8 * hf + 2 * e;
-            split2h(s * (y[j] - __uint_as_float(u[j]) * f), s * (y[j + 1] - __uint_as_float(u[j + 1]) * f), h[e], l[e]);
-          }
-          *reinterpret_cast<uint4*>(dst + hf * 128) = make_uint4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<uint4*>(dst + hf * 128 + kYTile / 2) = make_uint4(l[0], l[1], l[2], l[3]);
-        }
+        for (int e = 0; e < 4; ++e)
+          dst[(e & 1) * (kHalf4 / 2) + (e >> 1) * 8] = make_float4(y[4 * e] - __uint_as_float(u[4 * e]) * f, y[4 * e + 1] - __uint_as_float(u[4 * e + 1]) * f,
+                                                                   y[4 * e + 2] - __uint_as_float(u[4 * e + 2]) * f, y[4 * e + 3] - __uint_as_float(u[4 * e + 3]) * f);
       }
       // ---- N = -W^T Ki diag(e^{G_L}): thread = 32 columns -----------------------------------------------------------------------------------------
       {
         wait_at(ctl.bar[3], ph);
         tc::tc_fence_after();
-        const float f = -fminf(drop(top[kTopW]) * drop(top_i), 3.4e38f), s = lift(__float_as_uint(top_n));
-        uint8_t* dst = reinterpret_cast<uint8_t*>(p.nf) + (int64_t)c * kNTile + (row >> 3) * sm100::RBS + (row & 7) * 16 + 4 * cg * 128;
+        const float f = -fminf(drop(top[kTopW]) * drop(top_i), 3.4e38f);
+        float4* dst = p.nf + (2 * (int64_t)c + (cg >> 1)) * kHalf4 + (row >> 3) * 64 + 4 * (cg & 1) * 8 + (row & 7);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           uint32_t u[16];
           tc::tmem_ld16(ta + 16 * cg + tN + 16 * x, u);
           tc::tc_wait_ld();
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t h[4], l[4];
-#pragma unroll
-            for (int e4 = 0; e4 < 2; ++e4) {
-              const float4 d = *reinterpret_cast<const float4*>(ctl.el + 32 * cg + 16 * x + 8 * hf + 4 * e4);
-              const int j = 8 * hf + 4 * e4;
-              split2h(s * ((__uint_as_float(u[j]) * f) * d.x), s * ((__uint_as_float(u[j + 1]) * f) * d.y), h[2 * e4], l[2 * e4]);
-              split2h(s * ((__uint_as_float(u[j + 2]) * f) * d.z), s * ((__uint_as_float(u[j + 3]) * f) * d.w), h[2 * e4 + 1], l[2 * e4 + 1]);
-            }
-            *reinterpret_cast<uint4*>(dst + (2 * x + hf) * 128) = make_uint4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<uint4*>(dst + (2 * x + hf) * 128 + kNTile / 2) = make_uint4(l[0], l[1], l[2], l[3]);
+          for (int e = 0; e < 4; ++e) {
+            const float4 d = *reinterpret_cast<const float4*>(ctl.el + 32 * cg + 16 * x + 4 * e);
+            dst[(e & 1) * (kHalf4 / 2) + (2 * x + (e >> 1)) * 8] =
+                make_float4((__uint_as_float(u[4 * e]) * f) * d.x, (__uint_as_float(u[4 * e + 1]) * f) * d.y, (__uint_as_float(u[4 * e + 2]) * f) * d.z,
+                            (__uint_as_float(u[4 * e + 3]) * f) * d.w);
           }
         }
       }

@@ -273,3 +273,29 @@ def test_kda_local_passes(B, Hq, H, T, bthd, l2, decay):
         assert torch.equal(got[name], again[name]), name
         err = (got[name].double().cpu() - want).norm() / want.norm()
         assert err <= 1e-2, (name, err)
+
+
+@pytest.mark.parametrize("T,nats,loss", [(192, 0.4, "state"), (704, 0.25, "state"), (704, 0.4, "state"), (704, 1.0, "state"), (192, 0.6, "last"), (704, 0.25, "last"),
+                                         (704, 0.6, "last")])
+def test_kda_gradients_behind_chunks_that_decay_strongly(T, nats, loss):
+    """Every channel of every token decays by `nats`; the loss is of the final state or of the last token alone, so what reaches the chunks before
+    passes through N and Y of whole chunks, which are as small as the decay.  Chunk by chunk relative to itself, against float64: bf16 outputs
+    round at 2^-9 (2-norm 1.7e-3), the others carry the error of the chunk's inverse (tf32 products: measured 1.2e-4 at most); four times that."""
+    inp = O.make_inputs("kda", 1, 2, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["g"][...] = -nats
+    gen = torch.Generator().manual_seed(1)
+    do, dhT = torch.randn(1, 2, T, 128, generator=gen).bfloat16(), torch.randn(1, 2, 128, 128, generator=gen) * 0.1
+    do[:, :, :T if loss == "state" else T - 1] = 0
+    dhT = dhT if loss == "state" else None
+    args = [inp[x] for x in ("q", "k", "v", "g", "beta")]
+    got = ops.chunk_backward("kda", *(x.cuda() for x in args), do.cuda(), initial_state=inp["h0"].cuda(), d_final_state=None if dhT is None else dhT.cuda(),
+                             chunk_size=64)
+    L.check_device_status()
+    ref = O.delta_rule_grads("kda", *(x.double() for x in args), inp["h0"].double(), do.double(), None if dhT is None else dhT.double())
+    for name, tol in (("dq", 7e-3), ("dk", 7e-3), ("dv", 7e-3), ("dbeta", 5e-4), ("dg", 5e-4)):
+        for t0 in range(0, T, 64):
+            x, want = got[name][:, :, t0:t0 + 64].double().cpu(), ref[name][:, :, t0:t0 + 64]
+            if want.norm() > 1e-33:   # (what is left of float32's and bf16's range)
+                assert (x - want).norm() <= tol * want.norm(), (name, t0)
+    if ref["dh0"].norm() > 1e-33:
+        assert (got["dh0"].double().cpu() - ref["dh0"]).norm() <= 5e-4 * ref["dh0"].norm()
