@@ -13,7 +13,7 @@
 //                 chain rule of the normalisation and the reverse cumulative sum of dG, so that dq, dk, dv, dbeta, dg
 //                 leave in their final form (with grouped q/k heads dq^, dk^ leave as one fp32 copy per head for the
 //                 finalize kernel).  Scalar decays: local_sm100_kernel (dr_bwd_local_sm100.cuh), persistent, on tcgen05.  Per-channel
-//                 decays: local_sm100_kda_kernel (dr_bwd_local_kda.cuh), likewise, for chunks that decay by at most 2^16, and for the others
+//                 decays: local_sm100_kda_kernel (dr_bwd_local_kda.cuh), likewise, for chunks that decay by at most 2^40, and for the others
 //                 local_kernel, looping over four value slices with the sums over v in registers.
 //
 // The one-CTA-per-sequence-slice adjoint it replaces here walked all of a chunk's work in sequence (B=2, T=4096, H=16:
@@ -21,12 +21,10 @@
 //
 // DeltaNet / Gated DeltaNet: products on tcgen05 with two bf16 terms per float32 operand (16 bits); in pre_kernel mma.sync bf16 for the exact
 // ones of X and A and one tf32 product for W, Y and N.  KDA: three tf32 products per pair (x = hi + lo; see dr_tf32.cuh) on mma.sync, i.e.
-// float32 precision, as the CUDA-core adjoint it replaces, or three fp16 products of scaled operands on tcgen05.  Per-channel decays never appear as e^{-G}: inside a 16-row block the factors are
-// referred to the row before the block, between blocks they are carried by the blocks' total decays, and a block whose
-// decay range exceeds 2^64 is summed exactly.
+// float32 precision, as the CUDA-core adjoint it replaces; on tcgen05 two bf16 terms, in the state pass three.  On mma.sync per-channel decays never
+// appear as e^{-G}: inside a 16-row block the factors are referred to the row before the block, between blocks they are carried by
+// the blocks' total decays, and a block whose decay range exceeds 2^64 is summed exactly.
 #pragma once
-
-#include <cuda_fp16.h>
 
 #include "dr_common.cuh"
 #include "dr_mma.cuh"
@@ -96,31 +94,18 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   }
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
-// Per-channel decays: what the pre-pass leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32),
-// whether the chunk is pre_kernel's and local_kernel's (a channel decays by more than 2^16, or a decay is positive) or pre_sm100_kda_kernel's and
-// local_sm100_kda_kernel's, and the largest entries (A, T) or bounds of them (k^, q^), in the order of kTop.  local_kernel's chunks have X, A, T as rows, the others X by columns
-// in fours, A and T as two fp16 terms in tiles.
-constexpr float kWideKda = 16.f;   // log2 units
-constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096, kXTop = 2097;
-enum { kTopA, kTopT, kTopK, kTopQ, kTopS, kTopD, kTopO, kTopR, kTopdV, kTopVn, kTopdR, kTopP, kTopX };
+// Per-channel decays: what the pre-pass leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32) and
+// whether the chunk is pre_kernel's and local_kernel's (a channel decays by more than 2^40, or a decay is positive) or pre_sm100_kda_kernel's and
+// local_sm100_kda_kernel's.  local_kernel's chunks have X, A, T as rows, the others X by columns in fours, A and T - I as two bf16 terms in tiles.
+constexpr float kWideKda = 40.f;   // log2 units
+constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096;
 
-// the power of two that brings `top` to 2^13 .. 2^14 (none for zero and infinity); its inverse
+// The power of two that brings `top` to 2^40 .. 2^41 (none for zero and infinity; at most 2^126); its inverse
 __device__ __forceinline__ float lift(uint32_t top) {
   const uint32_t e = top >> 23;
-  return top == 0u || e == 255u ? 1.f : __uint_as_float(min(267u - e, 253u) << 23);
+  return top == 0u || e == 255u ? 1.f : __uint_as_float(min(294u - e, 253u) << 23);
 }
 __device__ __forceinline__ float drop(uint32_t top) { return __uint_as_float((254u << 23) - __float_as_uint(lift(top))); }
-__device__ __forceinline__ uint32_t pack_h(float x, float y) {
-  uint32_t r;
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
-  return r;
-}
-// two floats as two packed fp16 terms
-__device__ __forceinline__ void split2h(float x, float y, uint32_t& hi, uint32_t& lo) {
-  hi = pack_h(x, y);
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-  lo = pack_h(x - f.x, y - f.y);
-}
 // Per-channel decays: Y^T and the two halves of N's columns in float32, [128 rows][64 columns] each: eight columns of a row are a unit, eight rows'
 // units of the same columns follow each other; the first four columns of all units, then the others.  An m16n8 accumulator (lane g, t) of column
 // tile nt, rows r0 + g and eight further on.
@@ -129,10 +114,6 @@ __device__ __forceinline__ void store_f32(float4* dst, int r0, int nt, int g, in
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr)
     reinterpret_cast<float2*>(dst + (t >> 1) * (kHalf4 / 2) + ((r0 >> 3) + hr) * 64 + nt * 8 + g)[t & 1] = make_float2(d[2 * hr], d[2 * hr + 1]);
-}
-// Instruction descriptor for kind::f16 with fp16 operands and fp32 accumulation.
-__host__ __device__ constexpr uint32_t idesc_fp16(int M, int N, int a_mn_major, int b_mn_major) {
-  return tc::idesc_bf16(M, N, a_mn_major, b_mn_major) & ~((1u << 7) | (1u << 10));
 }
 // The chunks blockIdx.x, + gridDim.x, .. of one kind; warp-uniform, one read per 32 of them.
 template <bool WIDE>

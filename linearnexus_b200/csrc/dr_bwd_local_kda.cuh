@@ -2,28 +2,33 @@
 // gradient dS1 behind it and its inputs.  Formulas and names: header of dr_bwd.cuh; the kernels around it: dr_bwd_chunk.cuh; the form for
 // scalar decays, whose layout of work this one has: dr_bwd_local_sm100.cuh.
 //
-// float32 operands are two fp16 terms of a power of two times the operand, three products per pair: 22 bits of the largest entries, as the
-// three tf32 products of local_kernel have, and never less than 2^-39 of the tile's largest entry.  The power brings that entry to
-// 2^13 .. 2^14; it is found with one barrier per set of operands, and undone behind the product.  dO is a bf16 value: one term.
+// float32 operands are two bf16 terms, three products per pair: 17 bits of every entry, whatever lies beside it, with float32's exponents.  (Two fp16
+// terms of a power of two times the tile have 22 bits of its largest entries, none of those below 2^-39 of them; three bf16 terms
+// do not fit: the states alone would take 192 KB.)  dO is a bf16 value: one term.
 //
 // Decays: with Kg = k^ e^G, Qg = q^ e^G, Kd = k^ e^{G_L - G}, all at most the rows themselves,
 //   1  KS^T = S0^T Kg^T,  KD^T = dS1^T Kd^T,  AO^T = dO^T A,  dQ1^T = S0 dO^T
 //   2  Vn^T = R^T T^T,   dR^T = dVn^T T         R = beta (V - KS),  dVn = KD + AO   (terms in tensor memory)
 //   3  [dA; dM] = [dO; dR] Vn^T,  dKr1^T = S0 dR^T,  dKc1^T = dS1 Vn^T
 //   4  dQ2^T = Kd^T P^T,  dKr2^T = Kd^T Px^T,  dKc2^T = Qg^T P,  dKc3^T = Kg^T Px       P = dA, Px = dX below the diagonal
-//   dq^ = e^G (dQ1 + e^{-G_L} dQ2),  dk^ = e^G (-beta dKr1 + e^{-G_L} dKr2) + e^{G_L - G} dKc1 + e^{-G} (dKc2 + dKc3)
-// e^{-G_L} costs as many bits of the third term as it has, so the chunk may decay by at most 2^16 in any channel (kWideKda); pre_kernel says of
-// each chunk whether it does, and local_kernel, which refers the decays to 16-row blocks, takes the others.
+//   dq^ = e^G (dQ1 + e^{-G_L} dQ2) + diag(dA) k^,  dk^ = e^G (-beta dKr1 + e^{-G_L} dKr2) + e^{G_L - G} dKc1 + e^{-G} (dKc2 + dKc3) + diag(dA) q^
+// What the diagonals contribute is added in float32: T's (R and dVn lie in the accumulators that T - I adds to) and dA's, whose parts of q^ dq^
+// and k^ dk^ are equal and stay out of dG -- behind strong decays they are most of both.
+// The factors of a term multiply to decays of at most 1, so what each of them may reach is a matter of exponents alone.  P and Px, whose products
+// are the ones with a factor of more than 1 behind them, come with a power of two that brings their largest entries to 2^40, so that gradients as small as
+// float32 has them pass.  A chunk may decay by 2^40 in any channel (kWideKda).  The pre-pass says of each chunk whether it does, and local_kernel, which refers the decays to
+// 16-row blocks, takes the others.
 //
 // A thread of an epilogue owns one channel and sixteen tokens, and so does the one that forms Kg, Kd and Qg: G stays in its registers.  The
 // three are formed twice, before the products of 1 and of 4: beside the states (128 KB) there is no room to keep them.
 //
-// What bounds it: B=2, T=4096, H=16 (2048 chunks, 14 per CTA): 330 us, 48 K cycles per chunk, where local_kernel takes 882 us (three tf32 products on
-// mma.sync, 119 K); the training step 1490 -> 966 us, 265 -> 197 at B=1, T=1000.  Issue slots 34 %, tensor pipe 16 %: the element-wise work between the
-// products, 4.2 K instructions per warp, and the barriers around the largest entries.  Almost nothing is left for an L1, so what is not in
+// What bounds it: B=2, T=4096, H=16 (2048 chunks, 14 per CTA): 319 us, 46 K cycles per chunk, where local_kernel takes 884 us (three tf32 products on
+// mma.sync, 119 K).  Issue slots 34 %, tensor pipe 16 %: the element-wise work between the products, 4 K instructions per warp.  Almost nothing is left for an L1, so what is not in
 // shared memory costs an L2 access: with g, q, X, A and T by loads of the warps 71 K cycles, with everything the compiler would keep over the
 // chunk loop in spilled registers 57 K; hence the opaque thread index, and G parked in tensor memory.
-// Errors against float64 at one chunk as before: dbeta 3.7e-5, dg 3.7e-5 (T's inverse decides), dq, dk, dv 1.7e-3 (bf16 rounding).
+// Errors against float64 at one chunk (2-norm, 82 sequences; in brackets pre_kernel and local_kernel): dbeta 4.9e-5 (4.9e-5), dg 4.6e-5 (4.6e-5), dh0
+// 1.5e-5 (1.5e-5): T's tf32 merges decide; dq, dk, dv 1.7e-3 (bf16 rounding).  Where T is near I (beta a twentieth) 4.6e-6 (2.7e-6), 4.4e-6 (2.0e-6),
+// 2.2e-6 (1.3e-6).
 #pragma once
 
 namespace dr {
@@ -44,10 +49,10 @@ struct LkSums {
 static_assert(sizeof(LkSums) <= kTile, "over T");
 struct LkCtl {
   uint64_t bar[6], full_s, full_d, full_i, full_kv, full_t, full_x, full_q;
+  uint32_t top[2][2];             // largest entries (bits) of P and Px, by turns
   alignas(16) float beta[64];     // (read four at a time)
   float rk[64], rq[64];
-  float g[4][128];                // decay of sixteen tokens
-  uint32_t top[2][16];            // largest entries (bits), by turns
+  float g[4][128];                // decay of sixteen tokens, later the diagonal of dA
   uint32_t tmem_base;
   int abort;
 };
@@ -78,8 +83,8 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
     tc::mbar_init(tc::smem_u32(&ctl.full_q), 1);
     tc::fence_mbar_init();
     ctl.abort = 0;
+    ctl.top[0][0] = ctl.top[0][1] = 0u;
   }
-  if (tid < 32) ctl.top[tid >> 4][tid & 15] = 0u;
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -91,6 +96,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
   };
   auto wait_bar = [&](int i, uint32_t parity) { wait_at(ctl.bar[i], parity); };
   LkSums& sum = *reinterpret_cast<LkSums*>(smem + LK_T);
+  float(&dA)[64] = *reinterpret_cast<float(*)[64]>(ctl.g[0]);
   auto total = [](const float (&a)[4][64], int i) { return (a[0][i] + a[1][i]) + (a[2][i] + a[3][i]); };
   // tensor memory: columns of the accumulators and of the two terms of R^T, dVn^T
   constexpr uint32_t tKS = 0, tKD = 64, tAO = 128, tQ1 = 192, tR = 256, tV = 320, tVn = 384, tdR = 448;
@@ -137,7 +143,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
       load_part(ctl.full_i, LK_T, tile(c, 1), kTile);
     };
     // the token vectors of a chunk, lane = token and token + 32
-    float b0 = 0.f, b1 = 0.f, k0 = 0.f, k1 = 0.f, q0 = 0.f, q1 = 0.f, tops = 0.f;
+    float b0 = 0.f, b1 = 0.f, k0 = 0.f, k1 = 0.f, q0 = 0.f, q1 = 0.f;
     auto load_vectors = [&](int c) {
       const At x = place(c);
       const int rows = min(kC, p.map.T - x.t0);
@@ -147,19 +153,17 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
       if (lane + 32 < rows && in(at + (lane + 32) * tok)) b1 = p.beta[at + (lane + 32) * tok];
       const float* nrm = tile(c, 0) + kXNorms + lane;
       k0 = nrm[0]; k1 = nrm[kXNormRow]; q0 = nrm[2 * kXNormRow]; q1 = nrm[3 * kXNormRow];
-      tops = lane < 4 ? tile(c, 0)[kXTop + lane] : 0.f;
     };
-    auto store_vectors = [&](uint32_t turn) {   // before the inputs' barrier is armed: who waits for that sees them
+    auto store_vectors = [&]() {   // before the inputs' barrier is armed: who waits for that sees them
       ctl.beta[lane] = b0; ctl.beta[lane + 32] = b1;
       ctl.rk[lane] = k0; ctl.rk[lane + 32] = k1;
       ctl.rq[lane] = q0; ctl.rq[lane + 32] = q1;
-      if (lane < 4) ctl.top[turn][lane] = __float_as_uint(tops);
       __syncwarp();
     };
     int c = list.next(p, P.chunks, lane);
     if (c < P.chunks) {
       load_vectors(c);
-      store_vectors(0);
+      store_vectors();
       if (tc::elect_one()) {
         load_inputs(c);
         load_kv(c);
@@ -184,7 +188,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
           for (int x = 0; x < 3; ++x)
-            tc::mma_ss(tb + tKS, adv(sT, hi_lo[x] * 2048 + ks * 8192), adv(kd, lo_hi[x] * kTile + ks * 256), idesc_fp16(128, 64, 1, 1), ks + x > 0);
+            tc::mma_ss(tb + tKS, adv(sT, hi_lo[x] * 2048 + ks * 8192), adv(kd, lo_hi[x] * kTile + ks * 256), tc::idesc_bf16(128, 64, 1, 1), ks + x > 0);
       }
       __syncwarp();
       asm volatile("bar.sync 2, 544;" ::: "memory");
@@ -196,16 +200,16 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
           for (int x = 0; x < 3; ++x)
-            tc::mma_ss(tb + tKD, adv(dT, hi_lo[x] * 2048 + ks * 8192), adv(kd, lo_hi[x] * kTile + ks * 256), idesc_fp16(128, 64, 1, 1), ks + x > 0);
+            tc::mma_ss(tb + tKD, adv(dT, hi_lo[x] * 2048 + ks * 8192), adv(kd, lo_hi[x] * kTile + ks * 256), tc::idesc_bf16(128, 64, 1, 1), ks + x > 0);
 #pragma unroll
         for (int ks = 3; ks >= 0; --ks)
 #pragma unroll
-          for (int x = 0; x < 2; ++x) tc::mma_ss(tb + tAO, adv(odT, ks * 4096), adv(ad, x * 8192 + ks * 256), idesc_fp16(128, 16 * (ks + 1), 0, 1), ks < 3 || x > 0);
+          for (int x = 0; x < 2; ++x) tc::mma_ss(tb + tAO, adv(odT, ks * 4096), adv(ad, x * 8192 + ks * 256), tc::idesc_bf16(128, 16 * (ks + 1), 0, 1), ks < 3 || x > 0);
         commit(0);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
-          for (int x = 0; x < 2; ++x) tc::mma_ss(tb + tQ1, adv(sd, x * 2048 + ks * 256), adv(od, ks * 256), idesc_fp16(128, 64, 0, 1), ks + x > 0);
+          for (int x = 0; x < 2; ++x) tc::mma_ss(tb + tQ1, adv(sd, x * 2048 + ks * 256), adv(od, ks * 256), tc::idesc_bf16(128, 64, 0, 1), ks + x > 0);
         if (next < P.chunks) {   // what the next chunk reads
           const At x = place(next);
 #pragma unroll
@@ -231,15 +235,15 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         const uint64_t tk = tc::smem_desc(sb + LK_T, 1024, 128), tm = tc::smem_desc(sb + LK_T, 128, 1024);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          const uint32_t id = idesc_fp16(128, 64 - 16 * ks, 0, 0);
-          tc::mma_ts(tb + tVn + 16 * ks, tb + tR + 8 * ks, adv(tk, ks * 2304), id, ks > 0);
+          const uint32_t id = tc::idesc_bf16(128, 64 - 16 * ks, 0, 0);
+          tc::mma_ts(tb + tVn + 16 * ks, tb + tR + 8 * ks, adv(tk, ks * 2304), id, 1);
           tc::mma_ts(tb + tVn + 16 * ks, tb + tR + 32 + 8 * ks, adv(tk, ks * 2304), id, 1);
           tc::mma_ts(tb + tVn + 16 * ks, tb + tR + 8 * ks, adv(tk, 8192 + ks * 2304), id, 1);
         }
 #pragma unroll
         for (int ks = 3; ks >= 0; --ks) {
-          const uint32_t id = idesc_fp16(128, 16 * (ks + 1), 0, 1);
-          tc::mma_ts(tb + tdR, tb + tV + 8 * ks, adv(tm, ks * 256), id, ks < 3);
+          const uint32_t id = tc::idesc_bf16(128, 16 * (ks + 1), 0, 1);
+          tc::mma_ts(tb + tdR, tb + tV + 8 * ks, adv(tm, ks * 256), id, 1);
           tc::mma_ts(tb + tdR, tb + tV + 32 + 8 * ks, adv(tm, ks * 256), id, 1);
           tc::mma_ts(tb + tdR, tb + tV + 8 * ks, adv(tm, 8192 + ks * 256), id, 1);
         }
@@ -254,7 +258,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
       if (tc::elect_one()) {
         const uint64_t od = tc::smem_desc(sb + LK_O, 128, 2048), nd = tc::smem_desc(sb + LK_N, 128, 2048);
         const uint64_t sd = tc::smem_desc(sb + LK_S, 128, 4096), dd = tc::smem_desc(sb + LK_D, 128, 4096);
-        constexpr uint32_t id = idesc_fp16(128, 64, 1, 1), ik = idesc_fp16(128, 64, 0, 1);
+        constexpr uint32_t id = tc::idesc_bf16(128, 64, 1, 1), ik = tc::idesc_bf16(128, 64, 0, 1);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           tc::mma_ss(tb + tA, adv(od, ks * 256), adv(nd, ks * 256), id, ks > 0);
@@ -292,7 +296,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         const uint64_t pk = tc::smem_desc(sb + LK_P, 1024, 128), pm = tc::smem_desc(sb + LK_P, 128, 1024);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          const uint32_t id = idesc_fp16(128, 64 - 16 * ks, 0, 0);
+          const uint32_t id = tc::idesc_bf16(128, 64 - 16 * ks, 0, 0);
 #pragma unroll
           for (int x = 0; x < 3; ++x) {
             tc::mma_ss(tb + tQ2 + 16 * ks, adv(kd, hi_lo[x] * kTile + ks * 4096), adv(pk, lo_hi[x] * 8192 + ks * 2304), id, ks + x > 0);
@@ -301,7 +305,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         }
 #pragma unroll
         for (int ks = 3; ks >= 0; --ks) {
-          const uint32_t id = idesc_fp16(128, 16 * (ks + 1), 0, 1);
+          const uint32_t id = tc::idesc_bf16(128, 16 * (ks + 1), 0, 1);
 #pragma unroll
           for (int x = 0; x < 3; ++x) {
             tc::mma_ss(tb + tKc2, adv(qg, hi_lo[x] * kTile + ks * 4096), adv(pm, lo_hi[x] * 8192 + ks * 256), id, ks < 3 || x > 0);
@@ -346,7 +350,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         tc::bulk_commit();
       }
       __syncwarp();
-      store_vectors(ph ^ 1);
+      store_vectors();
       if (tc::elect_one()) {
         if (next < P.chunks) {
           tc::bulk_wait_read_all();
@@ -397,20 +401,15 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         return w[0] + __shfl_xor_sync(0xffffffffu, w[0], 1);
       };
       // sixteen tokens of this channel -> the two terms of a tile
-      auto put = [&](int base, const float (&y)[16], float s) {
+      auto put = [&](int base, const float (&y)[16]) {
   #pragma unroll
         for (int x = 0; x < 2; ++x) {
           uint32_t hi[4], lo[4];
   #pragma unroll
-          for (int e = 0; e < 4; ++e) split2h(s * y[8 * x + 2 * e], s * y[8 * x + 2 * e + 1], hi[e], lo[e]);
+          for (int e = 0; e < 4; ++e) split2(y[8 * x + 2 * e], y[8 * x + 2 * e + 1], hi[e], lo[e]);
           *reinterpret_cast<uint4*>(smem + base + own + x * 2048) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
           *reinterpret_cast<uint4*>(smem + base + kTile + own + x * 2048) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
-      };
-      uint32_t* const top = ctl.top[ph];
-      auto raise = [&](int i, float x) {
-        const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(x));
-        if (lane == 0) atomicMax(top + i, m);
       };
       // ---- G over this thread's tokens (log2 units); K, V, dO (warp = eight channels) -> registers ----------------------------------------------
       float G[16];
@@ -434,40 +433,17 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
       ctl.g[cg][row] = G[15];
       {
         const uint32_t src = sb + LK_O + (warp >> 3) * 8192 + (lane & 7) * 128 + (((warp & 7) ^ (lane & 7)) << 4);
-        float mo = 0.f;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           uint32_t r[4];
           mma::ldsm4t(r, src + (4 * x + (lane >> 3)) * 1024);
 #pragma unroll
-          for (int m = 0; m < 4; ++m) {
-            od[4 * x + m] = r[m];
-            mo = fmaxf(mo, fmaxf(fabsf(mma::lo_f(r[m])), fabsf(mma::hi_f(r[m]))));
-          }
+          for (int m = 0; m < 4; ++m) od[4 * x + m] = r[m];
         }
-        raise(kTopO, mo);
       }
-      // ---- S0, dS1: largest entries, <dS1, S0> per channel.  A lane's pieces of eight columns are skewed by the row, and rows 4 .. 7 read the
-      // halves of a piece in the other order: no bank conflicts on either side ----------------------------------------------------------------
-      float ts = 0.f;   // of channel 8 warp + (lane & 7)
+      // A lane's pieces of eight columns of the states are skewed by the row, and rows 4 .. 7 read the halves of a piece in the other order: no bank
+      // conflicts on either side
       const int r8 = lane & 7, turn = r8 >> 2;
-      wait_at(ctl.full_s, ph);
-      wait_at(ctl.full_d, ph);
-      {
-        float ms = 0.f, md = 0.f;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int at = warp * 4096 + r8 * 512 + ((4 * (it >> 1) + (lane >> 3) + r8) & 15) * 32 + 16 * ((it & 1) ^ turn);
-          const float4 s = *reinterpret_cast<const float4*>(smem + LK_S + at), d = *reinterpret_cast<const float4*>(smem + LK_D + at);
-          ts += (s.x * d.x + s.y * d.y) + (s.z * d.z + s.w * d.w);
-          ms = fmaxf(ms, fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fmaxf(fabsf(s.z), fabsf(s.w))));
-          md = fmaxf(md, fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fmaxf(fabsf(d.z), fabsf(d.w))));
-        }
-        ts += __shfl_xor_sync(0xffffffffu, ts, 8);
-        ts += __shfl_xor_sync(0xffffffffu, ts, 16);
-        raise(kTopS, ms);
-        raise(kTopD, md);
-      }
       workers_sync();
       // ---- G from the chunk's start; dO^T; Kg, the terms of S0; then Kd, dS1 --------------------------------------------------------------
       float GL;
@@ -482,7 +458,6 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
 #pragma unroll
         for (int e = 0; e < 16; ++e) G[e] += pre;
       }
-      auto join = [&](int i, int j) { return fminf(drop(top[i]) * drop(top[j]), 3.4e38f); };   // of one product
       // k^ or q^ times the decay from the chunk's start, or to its end
       auto decayed = [&](float (&y)[16], const uint32_t (&x)[8], const float (&r)[64], bool to_end) {
 #pragma unroll
@@ -493,7 +468,8 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
           for (int e = e4; e < e4 + 4; ++e) y[e] = f[e & 3] * half(x[e >> 1], e) * ex2(to_end ? GL - G[e] : G[e]);
         }
       };
-      auto split_state = [&](int base, float s) {
+      // the terms of a state in place of its rows
+      auto split_state = [&](int base) {
         float4 x[8];
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
@@ -505,28 +481,35 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
           uint32_t u[4], l[4];
-          split2h(s * x[2 * it].x, s * x[2 * it].y, u[0], l[0]);
-          split2h(s * x[2 * it].z, s * x[2 * it].w, u[1], l[1]);
-          split2h(s * x[2 * it + 1].x, s * x[2 * it + 1].y, u[2], l[2]);
-          split2h(s * x[2 * it + 1].z, s * x[2 * it + 1].w, u[3], l[3]);
+          split2(x[2 * it].x, x[2 * it].y, u[0], l[0]);
+          split2(x[2 * it].z, x[2 * it].w, u[1], l[1]);
+          split2(x[2 * it + 1].x, x[2 * it + 1].y, u[2], l[2]);
+          split2(x[2 * it + 1].z, x[2 * it + 1].w, u[3], l[3]);
           uint8_t* dst = smem + base + warp * 4096 + ((4 * it + (lane >> 3) + r8) & 15) * 128 + r8 * 16;
           *reinterpret_cast<uint4*>(dst) = turn ? make_uint4(u[2], u[3], u[0], u[1]) : make_uint4(u[0], u[1], u[2], u[3]);
           *reinterpret_cast<uint4*>(dst + 2048) = turn ? make_uint4(l[2], l[3], l[0], l[1]) : make_uint4(l[0], l[1], l[2], l[3]);
         }
       };
-      {
-        const float s = lift(top[kTopO]);
 #pragma unroll
-        for (int m = 0; m < 8; ++m)
-          *reinterpret_cast<uint32_t*>(smem + LK_O + m * 2048 + warp * 128 + lane * 4) = pack_h(s * mma::lo_f(od[m]), s * mma::hi_f(od[m]));
-      }
+      for (int m = 0; m < 8; ++m) *reinterpret_cast<uint32_t*>(smem + LK_O + m * 2048 + warp * 128 + lane * 4) = od[m];
       float y[16];
       decayed(y, kp, ctl.rk, false);
-      put(LK_N, y, lift(top[kTopK]));
-      split_state(LK_S, lift(top[kTopS]));
+      put(LK_N, y);
+      wait_at(ctl.full_s, ph);
+      wait_at(ctl.full_d, ph);
+      float ts = 0.f;   // <dS1, S0> of channel 8 warp + (lane & 7)
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int at = warp * 4096 + r8 * 512 + ((4 * (it >> 1) + (lane >> 3) + r8) & 15) * 32 + 16 * ((it & 1) ^ turn);
+        const float4 s = *reinterpret_cast<const float4*>(smem + LK_S + at), d = *reinterpret_cast<const float4*>(smem + LK_D + at);
+        ts += (s.x * d.x + s.y * d.y) + (s.z * d.z + s.w * d.w);
+      }
+      ts += __shfl_xor_sync(0xffffffffu, ts, 8);
+      ts += __shfl_xor_sync(0xffffffffu, ts, 16);
+      split_state(LK_S);
       hand_over(7);
       decayed(y, kp, ctl.rk, true);
-      put(LK_R, y, lift(top[kTopK]));
+      put(LK_R, y);
       // (G waits in tensor memory wherever it is not needed: registers are what these phases are short of)
       auto park = [&](uint32_t col) {
         uint32_t u[16];
@@ -543,80 +526,60 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         for (int e = 0; e < 16; ++e) G[e] = __uint_as_float(u[e]);
       };
       park(tVn);
-      split_state(LK_D, lift(top[kTopD]));
+      split_state(LK_D);
       hand_over(2);
       // ---- R and dVn, as two terms in tensor memory ----------------------------------------------------------------------------------
       wait_bar(0, ph);
       tc::tc_fence_after();
       {
-        float d[16], mr = 0.f, md = 0.f;
-        {
-          const float f1 = join(kTopK, kTopS), f2 = join(kTopK, kTopD), f3 = join(kTopO, kTopA);
+        fetch(tVn);   // (R goes there)
+        uint32_t u[16], l[16];
+        tc::tmem_ld16(ta + tKS, u);
+        tc::tc_wait_ld();
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t u[8], w[8], z[8];
-            tc::tmem_ld8(ta + tKS + 8 * hf, u);
-            tc::tmem_ld8(ta + tKD + 8 * hf, w);
-            tc::tmem_ld8(ta + tAO + 8 * hf, z);
-            tc::tc_wait_ld();
+        for (int e4 = 0; e4 < 16; e4 += 4) {
+          const float4 b4 = four(ctl.beta, e4);
+          const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-            for (int e4 = 0; e4 < 8; e4 += 4) {
-              const float4 b4 = four(ctl.beta, 8 * hf + e4);
-              const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-              for (int e = e4; e < e4 + 4; ++e) {
-                const int j = 8 * hf + e;
-                y[j] = bt[e & 3] * (half(vp[j >> 1], j) - __uint_as_float(u[e]) * f1);
-                d[j] = __uint_as_float(w[e]) * f2 + __uint_as_float(z[e]) * f3;
-                mr = fmaxf(mr, fabsf(y[j]));
-                md = fmaxf(md, fabsf(d[j]));
-              }
-            }
-          }
+          for (int e = e4; e < e4 + 4; ++e) y[e] = bt[e & 3] * (half(vp[e >> 1], e) - __uint_as_float(u[e]));
         }
-        raise(kTopR, mr);
-        raise(kTopdV, md);
-        workers_sync();
-        if (tid < 16) ctl.top[ph ^ 1][tid] = 0u;   // for the next chunk
-        const float sr = lift(top[kTopR]), sd = lift(top[kTopdV]);
         const uint32_t tt = ta - 8 * cg;   // eight columns for sixteen tokens
-        uint32_t u[8], l[8];
+        uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) split2h(sr * y[2 * e], sr * y[2 * e + 1], u[e], l[e]);
-        tc::tmem_st8(tt + tR, u);
-        tc::tmem_st8(tt + tR + 32, l);
+        for (int e = 0; e < 8; ++e) split2(y[2 * e], y[2 * e + 1], hi[e], lo[e]);
+        tc::tmem_st8(tt + tR, hi);
+        tc::tmem_st8(tt + tR + 32, lo);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) split2h(sd * d[2 * e], sd * d[2 * e + 1], u[e], l[e]);
-        tc::tmem_st8(tt + tV, u);
-        tc::tmem_st8(tt + tV + 32, l);
+        for (int e = 0; e < 16; ++e) u[e] = __float_as_uint(y[e]);
+        tc::tmem_st16(ta + tVn, u);
+        tc::tmem_ld16(ta + tKD, u);
+        tc::tmem_ld16(ta + tAO, l);
+        tc::tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) u[e] = __float_as_uint(__uint_as_float(u[e]) + __uint_as_float(l[e]));
+        tc::tmem_st16(ta + tdR, u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) split2(__uint_as_float(u[2 * e]), __uint_as_float(u[2 * e + 1]), hi[e], lo[e]);
+        tc::tmem_st8(tt + tV, hi);
+        tc::tmem_st8(tt + tV + 32, lo);
         tc::tc_wait_st();
       }
-      fetch(tVn);
       hand_over(3);
       // ---- Vn, dR -> tiles -----------------------------------------------------------------------------------------------------------------
       wait_bar(1, ph);
       tc::tc_fence_after();
       park(tV);
-      const float fdr = join(kTopdV, kTopT);   // dR from its accumulator
       {
         uint32_t u[16], w[16];
         tc::tmem_ld16(ta + tVn, u);
         tc::tmem_ld16(ta + tdR, w);
         tc::tc_wait_ld();
-        const float fvn = join(kTopR, kTopT);
-        float d[16], mn = 0.f, md = 0.f;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          y[e] = __uint_as_float(u[e]) * fvn;
-          d[e] = __uint_as_float(w[e]) * fdr;
-          mn = fmaxf(mn, fabsf(y[e]));
-          md = fmaxf(md, fabsf(d[e]));
-        }
-        raise(kTopVn, mn);
-        raise(kTopdR, md);
-        workers_sync();
-        put(LK_N, y, lift(top[kTopVn]));
-        put(LK_R, d, lift(top[kTopdR]));
+        for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(u[e]);
+        put(LK_N, y);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(w[e]);
+        put(LK_R, y);
       }
       hand_over(4);
       // ---- P = dA (rows 0 .. 63 of the product), Px = dX and dM . X (rows 64 ..); Kd, Kg, Qg once more -----------------------------------------
@@ -628,9 +591,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
         tc::tc_fence_after();
         uint32_t a[16];
         tc::tmem_ld16(ta + tA, a);
-        const int last = (second ? i - 1 : i) - 16 * cg;   // dX is strictly below the diagonal
-        const float fa = join(kTopVn, second ? kTopdR : kTopO);
-        float m = 0.f;
+        const int last = i - 1 - 16 * cg;   // below the diagonal
         if (second) {
           uint32_t a2[16];
           tc::tmem_ld16(ta + tM, a2);
@@ -643,46 +604,50 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
             const float x[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
             for (int e = 4 * f; e < 4 * f + 4; ++e) {
-              const float dm = -((__uint_as_float(a[e]) + __uint_as_float(a2[e])) * fa);
+              const float dm = -(__uint_as_float(a[e]) + __uint_as_float(a2[e]));
               xs += e <= last ? dm * x[e & 3] : 0.f;
               y[e] = e <= last ? bt * dm : 0.f;
-              m = fmaxf(m, fabsf(y[e]));
             }
           }
         } else {
           tc::tc_wait_ld();
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            y[e] = e <= last ? __uint_as_float(a[e]) * fa : 0.f;
-            m = fmaxf(m, fabsf(y[e]));
+            y[e] = e <= last ? __uint_as_float(a[e]) : 0.f;
+            if (e == last + 1) dA[i] = __uint_as_float(a[e]);
           }
         }
-        raise(second ? kTopX : kTopP, m);
-        workers_sync();
-        const float s = lift(top[second ? kTopX : kTopP]);
+        float m = 0.f;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) m = fmaxf(m, fabsf(y[e]));
+        const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if (lane == 0) atomicMax(&ctl.top[ph][second], most);
+        workers_sync();   // X has been read: Kd goes over it
+        if (tid < 2) ctl.top[ph ^ 1][tid] = 0u;   // for the next chunk
+        const float s = lift(ctl.top[ph][second]);
         wait_bar(3, ph);   // dO and dR have been read
         uint8_t* dst = smem + LK_P + (second ? 16384 : 0) + 2 * cg * 1024 + (i >> 3) * 128 + (i & 7) * 16;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t u[4], l[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split2h(s * y[8 * hf + 2 * e], s * y[8 * hf + 2 * e + 1], u[e], l[e]);
+          for (int e = 0; e < 4; ++e) split2(s * y[8 * hf + 2 * e], s * y[8 * hf + 2 * e + 1], u[e], l[e]);
           *reinterpret_cast<uint4*>(dst + hf * 1024) = make_uint4(u[0], u[1], u[2], u[3]);
           *reinterpret_cast<uint4*>(dst + 8192 + hf * 1024) = make_uint4(l[0], l[1], l[2], l[3]);
         }
       }
       fetch(tV);
       decayed(y, kp, ctl.rk, true);
-      put(LK_KD, y, lift(top[kTopK]));
+      put(LK_KD, y);
       uint32_t qp[8];
       wait_at(ctl.full_q, ph);
 #pragma unroll
       for (int e = 0; e < 8; ++e) qp[e] = raw2(LK_S, e);
       wait_bar(4, ph);   // Vn and dS1 have been read
       decayed(y, kp, ctl.rk, false);
-      put(LK_N, y, lift(top[kTopK]));
+      put(LK_N, y);
       decayed(y, qp, ctl.rq, false);
-      put(LK_QG, y, lift(top[kTopQ]));
+      put(LK_QG, y);
       hand_over(5);
       // ---- dV = beta dR, dR . V (while the last products run) ---------------------------------------------------------------------------------
       uint32_t dv[8];
@@ -697,7 +662,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
           const float bt[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
           for (int e = e4; e < e4 + 4; ++e) {
-            const float d = __uint_as_float(u[e]) * fdr;
+            const float d = __uint_as_float(u[e]);
             y[e] = d * half(vp[e >> 1], e);
             u[e] = __float_as_uint(bt[e & 3] * d);
           }
@@ -720,8 +685,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
       }
       float ex = 0.f;   // dKt . Kt
       {
-        const float el = ex2(GL), eli = ex2(-GL), f1 = join(kTopS, kTopO), f2 = join(kTopK, kTopP) * eli, f3 = join(kTopS, kTopdR), f4 = join(kTopK, kTopX) * eli;
-        const float f5 = join(kTopD, kTopVn) * el, f6 = join(kTopQ, kTopP), f7 = join(kTopK, kTopX);
+        const float el = ex2(GL), eli = ex2(-GL), fp = drop(ctl.top[ph][0]), fx = drop(ctl.top[ph][1]);
         // sums of eight values over the lanes: lane l ends up with value l >> 2
         auto reduce8 = [&](float (&w)[8]) -> float {
 #pragma unroll
@@ -749,15 +713,17 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
           tc::tc_wait_ld();
 #pragma unroll
           for (int e4 = 0; e4 < 8; e4 += 4) {
-            const float4 r4 = four(ctl.rq, 8 * hf + e4);
-            const float r[4] = {r4.x, r4.y, r4.z, r4.w};
+            const float4 q4 = four(ctl.rq, 8 * hf + e4), k4 = four(ctl.rk, 8 * hf + e4), a4 = four(dA, 8 * hf + e4);
+            const float rq[4] = {q4.x, q4.y, q4.z, q4.w}, rk[4] = {k4.x, k4.y, k4.z, k4.w}, da[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
             for (int e = e4; e < e4 + 4; ++e) {
               const int j = 8 * hf + e;
               eg[e] = ex2(__uint_as_float(gg[e]));
-              const float x = eg[e] * (__uint_as_float(u[e]) * f1 + __uint_as_float(w[e]) * f2);
-              s8[e] = dg[e] = r[e & 3] * half(qp[j >> 1], j) * x;
-              u[e] = __float_as_uint(x);
+              const float x = eg[e] * (__uint_as_float(u[e]) + (__uint_as_float(w[e]) * eli) * fp), qh = rq[e & 3] * half(qp[j >> 1], j);
+              const float all = x + da[e & 3] * (rk[e & 3] * half(kp[j >> 1], j));
+              dg[e] = qh * x;
+              s8[e] = qh * all;
+              u[e] = __float_as_uint(all);
             }
           }
           tc::tmem_st8(ta + tQ1 + 8 * hf, u);
@@ -773,8 +739,8 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
 #pragma unroll
             for (int e = e4; e < e4 + 4; ++e) {
               const int j = 8 * hf + e;
-              const float kh = r[e & 3] * half(kp[j >> 1], j), g1 = __uint_as_float(u[e]) * f3;
-              const float x = eg[e] * (__uint_as_float(w[e]) * f4 - bt[e & 3] * g1);
+              const float kh = r[e & 3] * half(kp[j >> 1], j), g1 = __uint_as_float(u[e]);
+              const float x = eg[e] * ((__uint_as_float(w[e]) * eli) * fx - bt[e & 3] * g1);
               dg[e] += kh * x;
               s8[e] = eg[e] * g1 * kh;
               u[e] = __float_as_uint(x);   // dk^_row
@@ -785,18 +751,22 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
           tc::tmem_ld8(ta + tKc3 + 8 * hf, z);
           tc::tc_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) s8[e] = __uint_as_float(w[e]) * f6 + __uint_as_float(z[e]) * f7;
+          for (int e = 0; e < 8; ++e) {
+            const float em = ex2(-__uint_as_float(gg[e]));
+            s8[e] = (em * __uint_as_float(w[e])) * fp + (em * __uint_as_float(z[e])) * fx;
+            gg[e] = __float_as_uint(em);
+          }
           tc::tmem_ld8(ta + tKc1 + 8 * hf, w);
           tc::tc_wait_ld();
 #pragma unroll
           for (int e4 = 0; e4 < 8; e4 += 4) {
-            const float4 r4 = four(ctl.rk, 8 * hf + e4);
-            const float r[4] = {r4.x, r4.y, r4.z, r4.w};
+            const float4 q4 = four(ctl.rq, 8 * hf + e4), k4 = four(ctl.rk, 8 * hf + e4), a4 = four(dA, 8 * hf + e4);
+            const float rq[4] = {q4.x, q4.y, q4.z, q4.w}, rk[4] = {k4.x, k4.y, k4.z, k4.w}, da[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
             for (int e = e4; e < e4 + 4; ++e) {
               const int j = 8 * hf + e;
-              const float kh = r[e & 3] * half(kp[j >> 1], j), em = ex2(-__uint_as_float(gg[e])), g3 = em * (__uint_as_float(w[e]) * f5);
-              const float kc = g3 + em * s8[e], x = __uint_as_float(u[e]) + kc;
+              const float kh = rk[e & 3] * half(kp[j >> 1], j), g3 = (__uint_as_float(gg[e]) * el) * __uint_as_float(w[e]);
+              const float kc = g3 + s8[e], x = (__uint_as_float(u[e]) + kc) + da[e & 3] * (rq[e & 3] * half(qp[j >> 1], j));
               ex += g3 * kh;
               dg[e] -= kh * kc;
               u[e] = __float_as_uint(x);

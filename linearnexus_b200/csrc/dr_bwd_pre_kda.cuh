@@ -1,22 +1,23 @@
 // The backward's pre-pass for per-channel decays (KDA) on tcgen05: X, A, T, N and Y of a chunk from q, k, g and beta.  Formulas and names:
 // headers of dr_bwd.cuh and dr_bwd_chunk.cuh.
 //
-// float32 operands are two fp16 terms of a power of two times the operand, three products per pair (22 bits of the largest entries; see
-// dr_bwd_local_kda.cuh).  With Kg = k^ e^G, Qg = q^ e^G, Ki = k^ e^{-G}:
+// float32 operands are two bf16 terms, three products per pair: 17 bits of every entry, float32's exponents (see dr_bwd_local_kda.cuh).  With
+// Kg = k^ e^G, Qg = q^ e^G, Ki = k^ e^{-G}:
 //   1  [X; A] = [Kg; Qg] Ki^T, then T by blocks
 //   2  W^T = Kg^T (T diag(beta))^T
 //   3  Y^T = Qg^T - W^T A^T,  N = -W^T Ki diag(e^{G_L})
-// Ki costs as many bits as the chunk decays by, so chunks of more than 2^16 in any channel are marked and left to pre_kernel, which refers the
-// decays to 16-row blocks.
+// The factors of a pair multiply to the pair's own decay whatever each of them is, so a chunk may decay by what their exponents have room for: 2^40
+// in any channel (kWideKda).  Others, and chunks with a positive log decay, are marked and left to pre_kernel, which refers the decays to 16-row
+// blocks.
 //
 // One persistent CTA per SM: sixteen warps that work, one that issues.  A worker warp owns four rows of the chunk up to the tiles, a lane four
 // channels of them; a thread of an epilogue one row of a product.  Rows arrive by TMA a chunk ahead, as soon as the tiles of the chunk before
 // are formed; A and T leave by bulk copies, X, N and Y as whole 128-byte lines.
 //
 // What bounds it: B=2, T=4096, H=16 (2048 chunks): 185 us on 116 SMs, 20 K cycles per chunk, where pre_kernel takes 266 us on 148 (65 K for two chunks at a
-// time: 15 K loads, 23 K for X and A, 18 K for W, Y and N); the training step 861 -> 743 us.  The phases of one chunk follow each other,
+// time: 15 K loads, 23 K for X and A, 18 K for W, Y and N).  The phases of one chunk follow each other,
 // sixteen warps on one: the tensor pipe has 4 K cycles of work.  210 KB of memory per chunk are 8 K cycles at the copy rate on all SMs.
-// Gradients against float64 as with pre_kernel: dbeta 4.6e-5, dg 5.0e-5, dh0 1.7e-5 at one chunk.
+// Gradients against float64 as with pre_kernel (T's tf32 merges decide): see dr_bwd_local_kda.cuh.
 #pragma once
 
 namespace dr {
@@ -31,7 +32,6 @@ struct PkCtl {
   uint64_t bar[4], full, free;
   alignas(16) float el[128];
   float beta[2][64];
-  uint32_t top[2][8];             // in the order of kTop, then kTopTb, kTopW
   uint32_t tmem_base;
   int rise[2], wide, abort;
 };
@@ -64,7 +64,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
     ctl.abort = 0;
     ctl.rise[0] = ctl.rise[1] = 0;
   }
-  if (tid < 16) ctl.top[tid >> 3][tid & 7] = 0u;
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -76,7 +75,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
   };
   // tensor memory: [X; A], W^T, its two terms, W^T A^T, N
   constexpr uint32_t tXA = 0, tW = 64, tWt = 128, tWA = 192, tN = 256;
-  constexpr int kTopTb = 4, kTopW = 5;   // T diag(beta), W
 
   if (warp == 16) {
     // (only the low word changes: the address field does not carry into the other)
@@ -117,7 +115,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
 #pragma unroll
           for (int x = 0; x < 3; ++x)
             tc::mma_ss(tb + tXA, adv(ad, hi_lo[x] * 32768 + (ks >> 2) * 16384 + (ks & 3) * 32), adv(bd, lo_hi[x] * kTile + (ks >> 2) * 8192 + (ks & 3) * 32),
-                       idesc_fp16(128, 64, 0, 0), ks + x > 0);
+                       tc::idesc_bf16(128, 64, 0, 0), ks + x > 0);
         commit(0);
       }
       __syncwarp();
@@ -135,7 +133,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
           for (int x = 0; x < 3; ++x)
-            tc::mma_ss(tb + tW + 16 * ks, adv(ad, hi_lo[x] * 32768 + ks * 2048), adv(bd, lo_hi[x] * 8192 + ks * 2304), idesc_fp16(128, 64 - 16 * ks, 1, 0), ks + x > 0);
+            tc::mma_ss(tb + tW + 16 * ks, adv(ad, hi_lo[x] * 32768 + ks * 2048), adv(bd, lo_hi[x] * 8192 + ks * 2304), tc::idesc_bf16(128, 64 - 16 * ks, 1, 0), ks + x > 0);
         commit(1);
         tc::bulk_s2g(xat + 8192, sb + PK_T, kTile);
         tc::bulk_commit();
@@ -149,13 +147,13 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
           for (int x = 0; x < 3; ++x)
-            tc::mma_ts(tb + tWA + 16 * ks, tb + tWt + 32 * hi_lo[x] + 8 * ks, adv(ad, lo_hi[x] * 8192 + ks * 2304), idesc_fp16(128, 64 - 16 * ks, 0, 0), ks + x > 0);
+            tc::mma_ts(tb + tWA + 16 * ks, tb + tWt + 32 * hi_lo[x] + 8 * ks, adv(ad, lo_hi[x] * 8192 + ks * 2304), tc::idesc_bf16(128, 64 - 16 * ks, 0, 0), ks + x > 0);
         commit(2);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
           for (int x = 0; x < 3; ++x)
-            tc::mma_ts(tb + tN, tb + tWt + 32 * hi_lo[x] + 8 * ks, adv(kd, lo_hi[x] * kTile + ks * 2048), idesc_fp16(128, 128, 0, 1), ks + x > 0);
+            tc::mma_ts(tb + tN, tb + tWt + 32 * hi_lo[x] + 8 * ks, adv(kd, lo_hi[x] * kTile + ks * 2048), tc::idesc_bf16(128, 128, 0, 1), ks + x > 0);
         commit(3);
         tc::bulk_wait_read_all();
         sm100::mbar_arrive(tc::smem_u32(&ctl.free));   // A and T have left
@@ -177,12 +175,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       asm volatile("" : "+r"(warp), "+r"(lane));
       warp = __shfl_sync(0xffffffffu, warp, 0);
       float* xat = p.xat + (int64_t)c * (3 * 64 * 64);
-      uint32_t* const top = ctl.top[turn];
-      auto raise = [&](int i, float x) {
-        const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(x));
-        if (lane == 0) atomicMax(top + i, m);
-      };
-      auto join = [&](int i, int j) { return fminf(drop(top[i]) * drop(top[j]), 3.4e38f); };   // of one product
       // ---- the warp's four rows: prefix sums over them, norm factors ---------------------------------------------------------------------------
       // byte of this lane's four channels in row 4 warp + r of a panel: + 128 r, piece ^ row
       const int piece = (lane & 15) >> 1, own = (4 * warp) * 128 + (lane & 1) * 8;
@@ -229,9 +221,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           }
         ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
         ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);   // lane l: q rows l >> 2, from lane 16 on k rows
-        const float s = lane < 16 ? p.scale : 1.f, nrm = sqrtf(ss[0]), m = p.l2norm ? s / (nrm + 1e-6f) : s, bound = fabsf(m * nrm);
-        raise(kTopQ, lane < 16 ? bound : 0.f);
-        raise(kTopK, lane < 16 ? 0.f : bound);
+        const float s = lane < 16 ? p.scale : 1.f, m = p.l2norm ? s / (sqrtf(ss[0]) + 1e-6f) : s;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           rq[r] = __shfl_sync(0xffffffffu, m, 4 * r);
@@ -244,7 +234,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       }
       workers_sync();
       bool wide;
-      float most;   // 2^(largest decay of a channel)
       {
         float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
 #pragma unroll
@@ -255,10 +244,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
-        const float low = fminf(fminf(run.x, run.y), fminf(run.z, run.w));
         const bool whole = run.x >= -kWideKda && run.y >= -kWideKda && run.z >= -kWideKda && run.w >= -kWideKda;   // (not for NaN)
         wide = ctl.rise[turn] || !__all_sync(0xffffffffu, whole);
-        most = ex2(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(-low, 0.f)))));
         if (warp == 0) {
           const float4 e = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
           *reinterpret_cast<float4*>(ctl.el + 4 * lane) = e;
@@ -269,10 +256,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           }
         }
       }
-      const uint32_t top_i = __float_as_uint(__uint_as_float(top[kTopK]) * most);   // of Ki
       if (!wide) {
         // ---- the tiles -----------------------------------------------------------------------------------------------------------------------
-        const float sk = lift(top[kTopK]), sq = lift(top[kTopQ]), si = lift(top_i);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const uint2 q = *at(PK_Q, 8192, r), k = *at(PK_K, 8192, r);
@@ -283,14 +268,14 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float x = ex2(gg[e]);
-            a[e] = sk * (kh[e] * x);
-            b[e] = sq * (qh[e] * x);
-            d[e] = si * (kh[e] * ex2(-gg[e]));
+            a[e] = kh[e] * x;
+            b[e] = qh[e] * x;
+            d[e] = kh[e] * ex2(-gg[e]);
           }
           auto put = [&](int base, int panel, int lo, const float (&x)[4]) {
             uint2 u, l;
-            split2h(x[0], x[1], u.x, l.x);
-            split2h(x[2], x[3], u.y, l.y);
+            split2(x[0], x[1], u.x, l.x);
+            split2(x[2], x[3], u.y, l.y);
             *at(base, panel, r) = u;
             *at(base + lo, panel, r) = l;
           };
@@ -301,9 +286,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       }
       hand_over(2);
       if (wide) {   // pre_kernel's
-        workers_sync();   // (the next chunk's maxima and totals wait for the readers of these)
-        if (tid < 8) top[tid] = 0u;
-        if (tid == 8) ctl.rise[turn] = 0;
+        workers_sync();   // (the next chunk's totals wait for the readers of these)
+        if (tid == 0) ctl.rise[turn] = 0;
         continue;
       }
       const int qd = warp & 3, cg = warp >> 2, row = 32 * qd + lane;   // this thread's row of a product and sixteen of its columns from 16 cg
@@ -317,14 +301,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         tc::tc_wait_ld();
         const bool second = row >= 64;
         const int i = row & 63, last = (second ? i : i - 1) - 16 * cg;   // X is strictly below the diagonal
-        const float f = fminf(drop(top[second ? kTopQ : kTopK]) * drop(top_i), 3.4e38f);
-        float x[16], m = 0.f;
+        float x[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          x[e] = e <= last ? __uint_as_float(u[e]) * f : 0.f;
-          m = fmaxf(m, fabsf(x[e]));
-        }
-        raise(kTopA, second ? m : 0.f);
+        for (int e = 0; e < 16; ++e) x[e] = e <= last ? __uint_as_float(u[e]) : 0.f;
         if (!second) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -333,15 +312,14 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
             if (cg <= (i >> 4)) reinterpret_cast<float4*>(xat)[(4 * cg + e) * 64 + i] = y;   // columns in fours
           }
         }
-        workers_sync();
+        workers_sync();   // (X for the inverse)
         if (second) {
           wait_at(ctl.free, ph ^ 1);   // the chunk before's has left
-          const float s = lift(top[kTopA]);
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
             uint32_t h[4], l[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2h(s * x[8 * hf + 2 * e], s * x[8 * hf + 2 * e + 1], h[e], l[e]);
+            for (int e = 0; e < 4; ++e) split2(x[8 * hf + 2 * e], x[8 * hf + 2 * e + 1], h[e], l[e]);
             uint4* dst = reinterpret_cast<uint4*>(smem + PK_AT) + (2 * cg + hf) * 64 + i;
             dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
             dst[512] = make_uint4(l[0], l[1], l[2], l[3]);
@@ -349,34 +327,29 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
         hand_over(3);
       }
-      // ---- T in place (eight warps), then T and T diag(beta) as tiles ----------------------------------------------------------------------------
+      // ---- T in place (eight warps), then T - I and T diag(beta) as tiles ----------------------------------------------------------------------------
       const float* beta = ctl.beta[turn];
       if (warp < 8) sm100::block_inverse_64(sX, beta, sX, 32 * warp + lane);
       workers_sync();
       {
         const int i = 32 * warp + lane, r = 8 * ((i >> 3) & 7) + (i & 7), cc = 8 * (i >> 6);
-        float x[8], y[8], m = 0.f, mb = 0.f;
+        float x[8], y[8];
         *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(sX + r * LDT + cc);
         *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(sX + r * LDT + cc + 4);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           x[e] = cc + e <= r ? x[e] : 0.f;
           y[e] = x[e] * beta[cc + e];
-          m = fmaxf(m, fabsf(x[e]));
-          mb = fmaxf(mb, fabsf(y[e]));
         }
-        raise(kTopT, m);
-        raise(kTopTb, mb);
-        workers_sync();
+        workers_sync();   // T has been read
         wait_at(ctl.free, ph ^ 1);
-        const float s = lift(top[kTopT]), sn = lift(top[kTopTb]);
         uint32_t h[4], l[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) split2h(s * x[2 * e], s * x[2 * e + 1], h[e], l[e]);
+        for (int e = 0; e < 4; ++e) split2(cc + 2 * e < r ? x[2 * e] : 0.f, cc + 2 * e + 1 < r ? x[2 * e + 1] : 0.f, h[e], l[e]);
         reinterpret_cast<uint4*>(smem + PK_T)[i] = make_uint4(h[0], h[1], h[2], h[3]);
         reinterpret_cast<uint4*>(smem + PK_T)[512 + i] = make_uint4(l[0], l[1], l[2], l[3]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) split2h(sn * y[2 * e], sn * y[2 * e + 1], h[e], l[e]);
+        for (int e = 0; e < 4; ++e) split2(y[2 * e], y[2 * e + 1], h[e], l[e]);
         reinterpret_cast<uint4*>(smem + PK_X)[i] = make_uint4(h[0], h[1], h[2], h[3]);
         reinterpret_cast<uint4*>(smem + PK_X)[512 + i] = make_uint4(l[0], l[1], l[2], l[3]);
       }
@@ -388,57 +361,38 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         uint32_t u[16];
         tc::tmem_ld16(ta + tW, u);
         tc::tc_wait_ld();
-        const float f = join(kTopK, kTopTb);
-        float w[16], m = 0.f;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          w[e] = __uint_as_float(u[e]) * f;
-          m = fmaxf(m, fabsf(w[e]));
-        }
-        raise(kTopW, m);
-        workers_sync();
-        const float s = lift(top[kTopW]);
         uint32_t h[8], l[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) split2h(s * w[2 * e], s * w[2 * e + 1], h[e], l[e]);
+        for (int e = 0; e < 8; ++e) split2(__uint_as_float(u[2 * e]), __uint_as_float(u[2 * e + 1]), h[e], l[e]);
         tc::tmem_st8(ta - 8 * cg + tWt, h);
         tc::tmem_st8(ta - 8 * cg + tWt + 32, l);
         tc::tc_wait_st();
       }
       hand_over(5);
-      if (tid == 0) {
-        xat[kXTop + kTopA] = __uint_as_float(top[kTopA]);
-        xat[kXTop + kTopT] = __uint_as_float(top[kTopT]);
-        xat[kXTop + kTopK] = __uint_as_float(top[kTopK]);
-        xat[kXTop + kTopQ] = __uint_as_float(top[kTopQ]);
-      }
       // ---- Y^T = Qg^T - W^T A^T ------------------------------------------------------------------------------------------------------------------
       {
         float y[16];
-        const float fq = drop(top[kTopQ]);
         const uint32_t el = (row >> 6) * 16384 + 8192 + 16 * cg * 128 + ((row >> 3) & 7) * 16 + (row & 7) * 2;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           const uint8_t* src = smem + PK_A + (el ^ ((e & 7) << 4)) + 128 * e;
-          y[e] = (__half2float(*reinterpret_cast<const __half*>(src)) + __half2float(*reinterpret_cast<const __half*>(src + 32768))) * fq;
+          y[e] = bf(reinterpret_cast<const __nv_bfloat16*>(src)) + bf(reinterpret_cast<const __nv_bfloat16*>(src + 32768));
         }
         wait_at(ctl.bar[2], ph);
         tc::tc_fence_after();
         uint32_t u[16];
         tc::tmem_ld16(ta + tWA, u);
         tc::tc_wait_ld();
-        const float f = join(kTopW, kTopA);
         float4* dst = p.yf + (int64_t)c * kHalf4 + (row >> 3) * 64 + 2 * cg * 8 + (row & 7);   // see store_f32
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          dst[(e & 1) * (kHalf4 / 2) + (e >> 1) * 8] = make_float4(y[4 * e] - __uint_as_float(u[4 * e]) * f, y[4 * e + 1] - __uint_as_float(u[4 * e + 1]) * f,
-                                                                   y[4 * e + 2] - __uint_as_float(u[4 * e + 2]) * f, y[4 * e + 3] - __uint_as_float(u[4 * e + 3]) * f);
+          dst[(e & 1) * (kHalf4 / 2) + (e >> 1) * 8] = make_float4(y[4 * e] - __uint_as_float(u[4 * e]), y[4 * e + 1] - __uint_as_float(u[4 * e + 1]),
+                                                                   y[4 * e + 2] - __uint_as_float(u[4 * e + 2]), y[4 * e + 3] - __uint_as_float(u[4 * e + 3]));
       }
       // ---- N = -W^T Ki diag(e^{G_L}): thread = 32 columns -----------------------------------------------------------------------------------------
       {
         wait_at(ctl.bar[3], ph);
         tc::tc_fence_after();
-        const float f = -fminf(drop(top[kTopW]) * drop(top_i), 3.4e38f);
         float4* dst = p.nf + (2 * (int64_t)c + (cg >> 1)) * kHalf4 + (row >> 3) * 64 + 4 * (cg & 1) * 8 + (row & 7);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
@@ -449,15 +403,14 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           for (int e = 0; e < 4; ++e) {
             const float4 d = *reinterpret_cast<const float4*>(ctl.el + 32 * cg + 16 * x + 4 * e);
             dst[(e & 1) * (kHalf4 / 2) + (2 * x + (e >> 1)) * 8] =
-                make_float4((__uint_as_float(u[4 * e]) * f) * d.x, (__uint_as_float(u[4 * e + 1]) * f) * d.y, (__uint_as_float(u[4 * e + 2]) * f) * d.z,
-                            (__uint_as_float(u[4 * e + 3]) * f) * d.w);
+                make_float4(-__uint_as_float(u[4 * e]) * d.x, -__uint_as_float(u[4 * e + 1]) * d.y, -__uint_as_float(u[4 * e + 2]) * d.z,
+                            -__uint_as_float(u[4 * e + 3]) * d.w);
           }
         }
       }
       ph ^= 1;
-      workers_sync();   // the maxima and e^{G_L} have been read
-      if (tid < 8) top[tid] = 0u;
-      if (tid == 8) ctl.rise[turn] = 0;
+      workers_sync();   // e^{G_L} has been read
+      if (tid == 0) ctl.rise[turn] = 0;
     }
   }
   tc::tc_fence_before();

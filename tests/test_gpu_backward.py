@@ -299,3 +299,53 @@ def test_kda_gradients_behind_chunks_that_decay_strongly(T, nats, loss):
                 assert (x - want).norm() <= tol * want.norm(), (name, t0)
     if ref["dh0"].norm() > 1e-33:
         assert (got["dh0"].double().cpu() - ref["dh0"]).norm() <= 5e-4 * ref["dh0"].norm()
+
+
+def _kda_backward(inp, do, dhT):
+    """Gradients, and float64's (on the device: many sequences)."""
+    cu = {n: x.cuda() for n, x in inp.items() if x is not None}
+    args = [cu[n] for n in ("q", "k", "v", "g", "beta")]
+    got = ops.chunk_backward("kda", *args, do.cuda(), initial_state=cu["h0"], d_final_state=dhT.cuda(), chunk_size=64)
+    L.check_device_status()
+    return got, O.delta_rule_grads("kda", *(x.double() for x in args), cu["h0"].double(), do.cuda().double(), dhT.cuda().double())
+
+
+@pytest.mark.parametrize("T,beta,nats,tol", [(64, 1.0, None, 2e-4), (63, 1.0, 0.2, 2e-4), (64, 0.05, None, 3e-5), (64, 1.0, 0.43, 2e-4), (17, 1.0, None, 2e-4)])
+def test_kda_float32_gradients_of_one_chunk(T, beta, nats, tol):
+    """One chunk, its states in float32: no bf16 checkpoint between.  Operands are two bf16 terms, 2^-17 of every entry; at most four products follow
+    each other (X, T, R or dVn, the gradient): 3e-5 where T is near I; its merges round to tf32, 2^-12 of its entries off the diagonal, of which those that
+    add up to a gradient are most of it at most: 2e-4.  A term that is left out is 2^-9.  bf16 outputs round at 2^-9 (2-norm 1.7e-3)."""
+    inp = O.make_inputs("kda", 81, 1, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["beta"] *= beta
+    if nats is not None:
+        inp["g"][...] = -nats
+    gen = torch.Generator().manual_seed(T + 1)
+    got, ref = _kda_backward(inp, torch.randn(81, 1, T, 128, generator=gen).bfloat16(), torch.randn(81, 1, 128, 128, generator=gen) * 0.1)
+    for name, tol in (("dbeta", tol), ("dg", tol), ("dh0", tol), ("dq", 3e-3), ("dk", 3e-3), ("dv", 3e-3)):
+        err = ((got[name].double() - ref[name]).norm() / ref[name].norm()).item()
+        assert err <= tol, (name, err)
+
+
+def test_kda_gradients_of_uneven_inputs():
+    """Half of the value channels 2^-60 of the others, and one of another head infinite in one token: a value channel's gradients know nothing of the
+    others, so each half keeps its own bits.  dv rounds to bf16; dh0 follows from N and Y, which T's tf32 merges decide: 2e-4."""
+    T = 705
+    inp = O.make_inputs("kda", 1, 2, T, 128, 128, seed=5, io_dtype=torch.bfloat16, h0_std=0.02)
+    gen = torch.Generator().manual_seed(6)
+    do, dhT = torch.randn(1, 2, T, 128, generator=gen).bfloat16(), torch.randn(1, 2, 128, 128, generator=gen) * 0.1
+    for x in (inp["v"], inp["h0"], do, dhT):
+        x[:, 0, :, 64:] *= 2.0 ** -60
+    do[:, 1, 300, 5] = float("inf")
+    got, ref = _kda_backward(inp, do, dhT)
+    rest = [v for v in range(128) if v != 5]
+    for name, tol in (("dv", 3e-3), ("dh0", 2e-4)):
+        for x, want in ((got[name][:, 0, :, :64], ref[name][:, 0, :, :64]), (got[name][:, 0, :, 64:], ref[name][:, 0, :, 64:]),
+                        (got[name][:, 1][..., rest], ref[name][:, 1][..., rest])):
+            err = ((x.double() - want).norm() / want.norm()).item()
+            assert err <= tol, (name, err)
+
+
+@pytest.mark.parametrize("decay", [27.7, 27.75, 39.0])
+def test_kda_local_passes_at_the_line(decay):
+    """The line between the two kinds of chunks: 2^40 (27.726 nats) in any channel."""
+    test_kda_local_passes(1, 2, 2, 703, True, True, decay)
