@@ -339,8 +339,8 @@ __device__ __forceinline__ void general_products(const float* sG, const __nv_bfl
 // Two persistent CTAs per SM: eight warps that work, one that issues copies and products.  A worker warp owns eight rows of the chunk, a lane
 // four channels of them, from the prefix sums to the tiles.
 //
-// With G summed from the chunk's start, e^{G_i - G_j} = e^{G_i} e^{-G_j}: while no channel decays by more than 2^64 over the chunk, the
-// factors fit bf16's exponents, and both chunk-local products are one tcgen05 product, [k^ e^G; q^ e^G] (k^ e^{-G})^T, of tiles
+// With G summed from the chunk's start, e^{G_i - G_j} = e^{G_i} e^{-G_j}: while no channel decays by more than 2^64 over the chunk and no log decay is
+// positive, the factors fit bf16's exponents, and both chunk-local products are one tcgen05 product, [k^ e^G; q^ e^G] (k^ e^{-G})^T, of tiles
 // of which the record and W need the first two anyway.  An entry above the diagonal may be as large as 2^64 |k|^2; none is used.
 // Chunks with a wider range (never with trained gates, but legal input) take general_products, which refers the decays to 16-row blocks.
 //
@@ -365,6 +365,7 @@ constexpr int IS_BETA = IS_X + 64 * LDT * 4;
 struct IntraCtl {
   float beta[64], rk[64], rq[64];
   uint64_t bar[2], full, free;
+  alignas(16) int up[8];   // per warp: a log decay of its rows is positive
   uint32_t tmem_base;
   int wide, abort;
 };
@@ -378,6 +379,14 @@ static __device__ __noinline__ void general_products_call(uint8_t* smem, const f
   general_products(reinterpret_cast<const float*>(smem), reinterpret_cast<const __nv_bfloat16*>(smem + IG_K),
                    reinterpret_cast<const __nv_bfloat16*>(smem + IG_Q), reinterpret_cast<float*>(smem + IS_X), reinterpret_cast<float*>(smem + IG_T),
                    reinterpret_cast<__nv_bfloat16*>(smem + IG_AQK), rk, rq, tid);
+}
+
+// Whether the chunk takes the general products, the same in every warp: a channel decays by more than 2^64 (run: this lane's four, whole chunk;
+// not a number counts), or a log decay is positive -- sums of others fall from row to row, so that e^G and e^{-G} of every row lie within 2^64.
+__device__ __forceinline__ bool any_wide(float4 run, const int (&up)[8]) {
+  const int4 a = *reinterpret_cast<const int4*>(up), b = *reinterpret_cast<const int4*>(up + 4);
+  const bool rise = (a.x | a.y | a.z | a.w) | (b.x | b.y | b.z | b.w);
+  return __any_sync(0xffffffffu, rise || !(run.x >= -64.f && run.y >= -64.f && run.z >= -64.f && run.w >= -64.f));
 }
 
 template <class Params>
@@ -586,12 +595,16 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           }
         }
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float up = 0.f;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
+          up = fmaxf(up, fmaxf(fmaxf(G[r].x, G[r].y), fmaxf(G[r].z, G[r].w)));
           acc.x += G[r].x * kLog2e; acc.y += G[r].y * kLog2e; acc.z += G[r].z * kLog2e; acc.w += G[r].w * kLog2e;
           G[r] = acc;
         }
         *reinterpret_cast<float4*>(smem + IS_TOT + warp * 512 + lane * 16) = acc;
+        const int rise = __any_sync(0xffffffffu, up > 0.f);
+        if (lane == 0) ctl.up[warp] = rise;
         // the sums are scattered over the lanes as they are reduced (16 shuffles), so that each lane takes one square root and one quotient
         float ss[16];
 #pragma unroll
@@ -633,16 +646,13 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
       float4 el;   // e^{G_L}
       {
         float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
-        float most = 0.f;
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
           if (s == warp) pre = run;
           const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
           run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
-          most = fmaxf(most, fmaxf(fmaxf(fabsf(run.x), fabsf(run.y)), fmaxf(fabsf(run.z), fabsf(run.w))));
         }
-        const float all = (run.x + run.y) + (run.z + run.w);   // NaN if any sum was
-        wide = __any_sync(0xffffffffu, !(most <= 64.f && all == all));
+        wide = any_wide(run, ctl.up);
         el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
 #pragma unroll
         for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
@@ -825,6 +835,7 @@ constexpr int IT_KD = IS_X - 16384;        // Kd; the log decay arrives over Kd 
 struct TransCtl {
   float beta[64], rk[64], rq[64];
   uint64_t bar[4], full, full_v;
+  alignas(16) int up[8];   // see IntraCtl
   uint32_t tmem_base;
   int abort;
 };
@@ -914,12 +925,16 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
       }
     }
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float up = 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
+      up = fmaxf(up, fmaxf(fmaxf(G[r].x, G[r].y), fmaxf(G[r].z, G[r].w)));
       acc.x += G[r].x * kLog2e; acc.y += G[r].y * kLog2e; acc.z += G[r].z * kLog2e; acc.w += G[r].w * kLog2e;
       G[r] = acc;
     }
     *reinterpret_cast<float4*>(smem + IT_TOT + warp * 512 + lane * 16) = acc;
+    const int rise = __any_sync(0xffffffffu, up > 0.f);
+    if (lane == 0) ctl.up[warp] = rise;
     // the sums are scattered over the lanes as they are reduced (16 shuffles), so that each lane takes one square root and one quotient
     float ss[16];
 #pragma unroll
@@ -950,16 +965,13 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
   float4 el;   // e^{G_L}
   {
     float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
-    float most = 0.f;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
       if (s == warp) pre = run;
       const float4 y = *reinterpret_cast<const float4*>(smem + IT_TOT + s * 512 + lane * 16);
       run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
-      most = fmaxf(most, fmaxf(fmaxf(fabsf(run.x), fabsf(run.y)), fmaxf(fabsf(run.z), fabsf(run.w))));
     }
-    const float all = (run.x + run.y) + (run.z + run.w);   // NaN if any sum was
-    wide = __any_sync(0xffffffffu, !(most <= 64.f && all == all));
+    wide = any_wide(run, ctl.up);
     el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
     if (warp == 0) *reinterpret_cast<float4*>(P.el + chunk * kD + 4 * lane) = el;
 #pragma unroll

@@ -135,3 +135,18 @@ def test_split_without_workspace_is_refused():
         assert st == want
     assert _lib.last_path() == "chunk_fp32"
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("path,T", [("split", 150), (None, 1100)])
+def test_kda_decays_that_climb_back(path, T):
+    """A channel that falls to 2^-130 of the chunk's start and climbs back to 2^-60 (a positive log decay): e^G and e^{-G} of the rows between have no float32,
+    the 16-row form refers them to their neighbours.  Both forms of the pass (T=1100, two sequences: the transition form)."""
+    inp = O.make_inputs("kda", 1, 2, T, 128, 128, seed=21, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["g"][:, 1, 64:128, 5] = 0.0
+    inp["g"][:, 1, 80:96, 5] = -90.0 / 16
+    inp["g"][:, 1, 96:128, 5] = 48.0 / 32
+    o, hT = _run("kda", inp, path)
+    assert _lib.last_path() == ("chunk_split_tcgen05" if path else "chunk_transition")
+    ro, rS = _truth("kda", inp)
+    for h in range(2):
+        assert _rel(o[:, h], ro[:, h]) <= BF16_TOL and _rel(hT[:, h], rS[:, h]) <= BF16_TOL
