@@ -1356,7 +1356,8 @@ inline cudaError_t bwd_side_stream(cudaStream_t* out) {
 // the chip as well, so there the fork lies between its kernels (KDA, B=2, T=4096, H=16: forward and pre-pass one after the
 // other took 590 us of a 1772 us step).
 // own_stream: the pre-pass may run on the library's side stream, forked from and joined to `stream` with events
-// (false for callers that must not create streams or events: the pre-pass then runs on `stream` before the forward).
+// (false for callers that must not create streams or events: the pre-pass then runs on `stream`, before the forward or, with per-channel decays,
+// behind it).
 cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                                       const float* beta, const float* h0, void* o, float* hT, void* workspace,
                                       int32_t* status, cudaStream_t stream, int* launches, bool own_stream) {
@@ -1375,8 +1376,6 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
           cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess)) {
       if (forked) cudaEventDestroy(forked);
       forked = joined = nullptr;
-      const cudaError_t ep = pre(stream);
-      if (ep != cudaSuccess) return ep;
     }
   }
   float* ckpt = reinterpret_cast<float*>(workspace);
@@ -1395,6 +1394,9 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
                      (!o || d->out_dtype == DR_BF16);
   const bool split = tc_shape && !fused && d->variant == DR_KDA;
   cudaError_t e = cudaSuccess;
+  // with per-channel decays the forward's first kernel says which chunks are the pre-pass's (WideMarks), so that one does not come before it
+  const bool after = split && chunked;
+  if (want_pre && !forked && !after) e = pre(stream);
   if (forked && !split) e = cudaEventRecord(forked, stream);
   if (e != cudaSuccess) {
   } else if (fused) {
@@ -1403,8 +1405,10 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
   } else if (split) {
     int n2 = 0;
     // its records lie where dS1 of every chunk will be written (bwdc::Params)
-    e = launch_chunk_split(f, bwdc::make_params(d, workspace).ds, stream, &n2, forked);
+    const bwdc::Params b = bwdc::make_params(d, workspace);
+    e = launch_chunk_split(f, b.ds, stream, &n2, forked, WideMarks{b.xat + bwdc::kXWide, 3 * 64 * 64, bwdc::kWideKda});
     *launches += n2;
+    if (want_pre && !forked && after && e == cudaSuccess) e = pre(stream);
   } else {
     // every other shape: the token recurrence (the same function of the inputs as the chunk form, and on the CUDA
     // cores 4-11x faster than the fp32 chunk kernel) leaves the state at each chunk start on its way

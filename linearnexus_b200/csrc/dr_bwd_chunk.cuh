@@ -94,11 +94,15 @@ __device__ __forceinline__ float4 load_g4(const void* g, int64_t at, int dt) {
   }
   return make_float4(x.x * kLog2e, x.y * kLog2e, x.z * kLog2e, x.w * kLog2e);
 }
-// Per-channel decays: what the pre-pass leaves among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32) and
+// Per-channel decays: what is kept among X, A, T in places that neither form of X uses: the norm factors of k and q (four rows of 32; the pre-pass) and
 // whether the chunk is pre_kernel's and local_kernel's (a channel decays by more than 2^40, or a decay is positive) or pre_sm100_kda_kernel's and
-// local_sm100_kda_kernel's.  local_kernel's chunks have X, A, T as rows, the others X by columns in fours, A and T - I as two bf16 terms in tiles.
+// local_sm100_kda_kernel's (the forward, see WideMarks).  local_kernel's chunks have X, A, T as rows, the others X by columns in fours, A and T - I as two bf16 terms in tiles.
 constexpr float kWideKda = 40.f;   // log2 units
 constexpr int kXNorms = 1056, kXNormRow = 256, kXWide = 2096;
+// pre_kernel's and local_kernel's chunks in a list, entry i beside chunk i's mark, and in chunk 0's place its length and how many of them either kernel has
+// taken; the forward's first kernel sets the three to zero, pre_sm100_kda_kernel fills the list.  CTAs take the entries one by one: dealt out
+// beforehand, those whose SM the forward's state pass holds would do their share behind it (training step of 2048 such chunks 1711 us).
+constexpr int kXList = kXWide + 1, kXCounts = kXWide + 2;
 
 // The power of two that brings `top` to 2^40 .. 2^41 (none for zero and infinity; at most 2^126); its inverse
 __device__ __forceinline__ float lift(uint32_t top) {
@@ -115,8 +119,13 @@ __device__ __forceinline__ void store_f32(float4* dst, int r0, int nt, int g, in
   for (int hr = 0; hr < 2; ++hr)
     reinterpret_cast<float2*>(dst + (t >> 1) * (kHalf4 / 2) + ((r0 >> 3) + hr) * 64 + nt * 8 + g)[t & 1] = make_float2(d[2 * hr], d[2 * hr + 1]);
 }
-// The chunks blockIdx.x, + gridDim.x, .. of one kind; warp-uniform, one read per 32 of them.
-template <bool WIDE>
+__device__ __forceinline__ void l2_panel(const void* tmap, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ void l2_bulk(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+// Those of the chunks blockIdx.x, + gridDim.x, .. that tcgen05 takes; warp-uniform, one read per 32 of them.
 struct ChunkList {
   int base;
   uint32_t mask;
@@ -126,7 +135,7 @@ struct ChunkList {
   }
   __device__ __forceinline__ void fetch(const Params& p, int chunks, int lane) {
     const int64_t c = base + (int64_t)lane * gridDim.x;
-    mask = __ballot_sync(0xffffffffu, c < chunks && ((WIDE && p.few) || (__ldcg(p.xat + c * (3 * 64 * 64) + kXWide) != 0.f) == WIDE));
+    mask = __ballot_sync(0xffffffffu, c < chunks && __ldcg(p.xat + c * (3 * 64 * 64) + kXWide) == 0.f);
   }
   __device__ __forceinline__ int next(const Params& p, int chunks, int lane) {   // `chunks` behind the last
     while (mask == 0u) {
@@ -139,6 +148,30 @@ struct ChunkList {
     return base + i * (int)gridDim.x;
   }
 };
+// The others: into the list (one warp per CTA) ..
+__device__ __forceinline__ void list_wide(const Params& p, int chunks, int lane) {
+  int* counts = reinterpret_cast<int*>(p.xat + kXCounts);
+  for (int64_t base = blockIdx.x; base < chunks; base += 32 * (int64_t)gridDim.x) {
+    const int64_t c = base + (int64_t)lane * gridDim.x;
+    const bool wide = c < chunks && __ldcg(p.xat + c * (3 * 64 * 64) + kXWide) != 0.f;
+    const uint32_t mask = __ballot_sync(0xffffffffu, wide);
+    if (mask == 0u) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(counts, __popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+    if (wide) reinterpret_cast<int*>(p.xat + (int64_t)at * (3 * 64 * 64))[kXList] = (int)c;
+  }
+}
+// .. and from it (one thread per CTA): a number, and the chunk that has it, or `chunks`.  Kernel 0: pre_kernel, 1: local_kernel.  Without a list (p.few): one
+// chunk per CTA.
+__device__ __forceinline__ int take_number(const Params& p, int kernel, bool first) {
+  int* counts = reinterpret_cast<int*>(p.xat + kXCounts);
+  return p.few ? (first ? (int)blockIdx.x : 0x7fffffff) : __ldcg(counts) == 0 ? 0x7fffffff : atomicAdd(counts + 1 + kernel, 1);
+}
+__device__ __forceinline__ int numbered(const Params& p, int chunks, int i) {
+  if (p.few) return min(i, chunks);
+  return i < __ldcg(reinterpret_cast<const int*>(p.xat + kXCounts)) ? __ldcg(reinterpret_cast<const int*>(p.xat + (int64_t)i * (3 * 64 * 64)) + kXList) : chunks;
+}
 // Few chunks, in short sequences: a training step is bound by the host, and the two launches that look for wide chunks cost more than the kernels on
 // tcgen05 give; every chunk is then treated as a wide one.  Whole step, so / as wide and narrow chunks: 20 chunks in 4 sequences 132 / 139 us, 40 in 4
 // 134 / 140, 80 in 16 133 / 138; 64 in 4 152 / 139, 128 in 8 159 / 139.
@@ -153,7 +186,8 @@ constexpr int PR_SC = PR_A + 64 * 72 * 4;     // beta, rk, rq, G, fw, fd (64 eac
 constexpr int LDG = 136;   // row stride of G: pairs of eight rows are read without bank conflicts
 constexpr int LDK = 130;   // row stride (16-byte entries) of the split Kd
 constexpr int PR_G = PR_SC + 6 * 64 * 4;      // KDA: log2(e) G [64][136]; Kd as token pairs [32][130] (hi, hi, lo, lo) later over k, q, X, A
-template <bool KDA> constexpr int pre_smem() { return KDA ? PR_G + 64 * LDG * 4 : PR_G; }
+constexpr int PR_TAKEN = PR_G + 64 * LDG * 4;
+template <bool KDA> constexpr int pre_smem() { return KDA ? PR_TAKEN + 16 : PR_G; }
 static_assert(PR_SC >= 32 * LDK * 16 && 2 * (pre_smem<true>() + 1024) <= 233472, "two CTAs per SM");
 
 template <bool KDA>
@@ -168,20 +202,25 @@ __global__ void __launch_bounds__(kPreThreads, 2) pre_kernel(const Params p, con
   float* sBeta = reinterpret_cast<float*>(smem + PR_SC);
   float *sRk = sBeta + 64, *sRq = sBeta + 128, *sGs = sBeta + 192, *sFw = sBeta + 256, *sFd = sBeta + 320;
   float* sG = reinterpret_cast<float*>(smem + PR_G);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  ChunkList<true> list;
-  if constexpr (KDA) list.start(p, chunks, lane);
+  int* const taken = reinterpret_cast<int*>(smem + PR_TAKEN);   // KDA: [2], by turns
+  if (KDA && threadIdx.x == 0) taken[0] = numbered(p, chunks, take_number(p, 0, true));
 #pragma unroll 1
-  for (int c = KDA ? list.next(p, chunks, lane) : blockIdx.x; c < chunks; c = KDA ? list.next(p, chunks, lane) : chunks) {
+  for (int turn = 0; KDA || turn == 0; turn ^= 1) {
+  int tid = threadIdx.x, c = blockIdx.x;
+  if constexpr (KDA) {
+    __syncthreads();   // the chunk before is done with shared memory
+    c = taken[turn];
+    if (c >= chunks) break;
+    asm volatile("" : "+r"(tid));   // (see local_kernel)
+    if (tid == 0) taken[turn ^ 1] = numbered(p, chunks, take_number(p, 0, false));
+  }
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int64_t chunk = c;
   const int unit = c / p.N, n = c % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
   const int64_t gk_base = p.map.base(b, h, kD), gk_tok = p.map.tok(kD);
   const int64_t s_base = p.map.base(b, h, 1), s_tok = p.map.tok(1);
-  if constexpr (KDA) {
-    __syncthreads();   // the chunk before is done with shared memory
-  }
   // ---- raw rows, norm factors, decay --------------------------------------------------------------------------------
   {
     uint2 qr[8], kr[8];
@@ -842,7 +881,8 @@ struct LoSmem {
   static constexpr int kV = kT + 64 * LDT * 4, kSl = 64 * LDV * 4;   // V, dO, Vn, dR
   static constexpr int kSD = kV + 4 * kSl, kS1 = 128 * LDV * 4;        // [2][S0, dS]
   static constexpr int kSc = kSD + 4 * kS1;
-  static constexpr int kTotal = kSc + (3 * 64 + 5 * 64 + 128 + 528) * 4;
+  static constexpr int kTaken = kSc + (3 * 64 + 5 * 64 + 128 + 528) * 4;
+  static constexpr int kTotal = kTaken + 16;
   // final phase: a map of its own from 0
   static constexpr int gQS = 0, gKS = 64 * 132 * 4, gKE = 2 * gKS, gG = 3 * gKS, gA = 4 * gKS, gX = gA + 64 * LDA * 4, gD = gX + 64 * LDA * 4;
   static constexpr int gSeg = gD + 4 * 128 * 4;   // [16][128] scan scratch
@@ -865,12 +905,18 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
   float *sdB = sBeta + 192, *sTS = sBeta + 512, *sU = sBeta + 640;   // dbeta [5][64]; <dS1, S0> per channel
   float *sEx = sU, *sUn = sU + 512;   // sums for dG_L [4][128], block flags
   float *sDq = F(L::kDot), *sDk = sDq + 256;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  ChunkList<true> list;
-  list.start(p, chunks, lane);
+  int* const taken = reinterpret_cast<int*>(smem + L::kTaken);   // [2], by turns
+  if (threadIdx.x == 0) taken[0] = numbered(p, chunks, take_number(p, 1, true));
 #pragma unroll 1
-  for (int at_chunk = list.next(p, chunks, lane); at_chunk < chunks; at_chunk = list.next(p, chunks, lane)) {
+  for (int turn = 0;; turn ^= 1) {
   __syncthreads();   // the chunk before is done with shared memory
+  const int at_chunk = taken[turn];
+  if (at_chunk >= chunks) break;
+  int tid = threadIdx.x;
+  asm volatile("" : "+r"(tid));   // (what follows from the thread's place is formed for each chunk: kept over the loop it costs the inner loops their registers)
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  int number = 0;   // (asked for early: the answer takes a while)
+  if (tid == 0) number = take_number(p, 1, false);
   const int unit = at_chunk / p.N, n = at_chunk % p.N;
   const int b = unit / p.map.H, h = unit % p.map.H, t0 = n * kC, rows = min(kC, p.map.T - t0);
   const int64_t qk_base = p.map.base_qk(b, h, kD), qk_tok = p.map.tok_qk(kD);
@@ -1121,6 +1167,14 @@ static __global__ void __launch_bounds__(kLoThreads, 1) local_kernel(const Param
       qr[i] = *reinterpret_cast<const uint2*>(gq + qk_base + (t0 + c) * qk_tok + 4 * lane);
       kr[i] = *reinterpret_cast<const uint2*>(gk + qk_base + (t0 + c) * qk_tok + 4 * lane);
       gr[i] = load_g4(p.g, gk_base + (t0 + c) * gk_tok + 4 * lane, p.g_dt);
+    }
+  }
+  if (tid == 0) {
+    const int next = numbered(p, chunks, number);
+    taken[turn ^ 1] = next;
+    if (next < chunks) {   // it begins with its states
+      l2_bulk(p.ckpt + (int64_t)next * (kD * kD), kD * kD * 4);
+      l2_bulk(p.ds + (int64_t)next * (kD * kD), kD * kD * 4);
     }
   }
   __syncthreads();   // phase 1 is over: its arrays may be written

@@ -101,7 +101,7 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
   // tensor memory: columns of the accumulators and of the two terms of R^T, dVn^T
   constexpr uint32_t tKS = 0, tKD = 64, tAO = 128, tQ1 = 192, tR = 256, tV = 320, tVn = 384, tdR = 448;
   constexpr uint32_t tKr1 = 0, tKc1 = 64, tA = 128, tM = 256, tQ2 = 128, tKr2 = 256, tKc2 = 320, tKc3 = 384;
-  ChunkList<false> list;
+  ChunkList list;
   list.start(p, P.chunks, lane);
 
   if (warp >= 16) {

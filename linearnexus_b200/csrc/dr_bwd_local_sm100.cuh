@@ -56,12 +56,6 @@ struct alignas(64) LocalParams {
   int32_t* status;
   int64_t n_tok, n_part;   // entries of the arrays with one number per token, of dq^ and dk^ per head (index checks of the debug build)
 };
-__device__ __forceinline__ void l2_panel(const void* tmap, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void l2_bulk(const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kernel(const __grid_constant__ LocalParams P) {
   const Params& p = P.p;
   extern __shared__ __align__(1024) uint8_t lt_smem[];

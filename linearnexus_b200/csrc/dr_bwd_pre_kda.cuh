@@ -7,8 +7,8 @@
 //   2  W^T = Kg^T (T diag(beta))^T
 //   3  Y^T = Qg^T - W^T A^T,  N = -W^T Ki diag(e^{G_L})
 // The factors of a pair multiply to the pair's own decay whatever each of them is, so a chunk may decay by what their exponents have room for: 2^40
-// in any channel (kWideKda).  Others, and chunks with a positive log decay, are marked and left to pre_kernel, which refers the decays to 16-row
-// blocks.
+// in any channel (kWideKda).  Others, and chunks with a positive log decay, are left to pre_kernel, which refers the decays to 16-row
+// blocks; the forward's first kernel, which forms the same sums before this one starts, marks them (launch_bwd_forward).
 //
 // One persistent CTA per SM: sixteen warps that work, one that issues.  A worker warp owns four rows of the chunk up to the tiles, a lane four
 // channels of them; a thread of an epilogue one row of a product.  Rows arrive by TMA a chunk ahead, as soon as the tiles of the chunk before
@@ -33,7 +33,7 @@ struct PkCtl {
   alignas(16) float el[128];
   float beta[2][64];
   uint32_t tmem_base;
-  int rise[2], wide, abort;
+  int abort;
 };
 constexpr int PK_TOTAL = PK_CTL + sizeof(PkCtl);
 static_assert(PK_TOTAL <= 232448 && PK_CTL % 16 == 0 && PK_X % 1024 == 0, "shared memory");
@@ -62,7 +62,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
     tc::mbar_init(tc::smem_u32(&ctl.free), 1);
     tc::fence_mbar_init();
     ctl.abort = 0;
-    ctl.rise[0] = ctl.rise[1] = 0;
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -73,6 +72,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
     const uint32_t at = tc::smem_u32(&bar);
     sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp == 16);
   };
+  ChunkList list;
+  list.start(p, P.chunks, lane);
   // tensor memory: [X; A], W^T, its two terms, W^T A^T, N
   constexpr uint32_t tXA = 0, tW = 64, tWt = 128, tWA = 192, tN = 256;
 
@@ -99,16 +100,18 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       }
       __syncwarp();
     };
-    load(blockIdx.x, 0);
+    int c = list.next(p, P.chunks, lane);
+    if (c < P.chunks) load(c, 0);
+    list_wide(p, P.chunks, lane);
     uint32_t turn = 0;
     constexpr uint32_t hi_lo[3] = {0, 1, 0}, lo_hi[3] = {0, 0, 1};   // terms of the left and of the right operand in the three products
 #pragma unroll 1
-    for (int c = blockIdx.x; c < P.chunks; c += gridDim.x, turn ^= 1) {
+    for (int next; c < P.chunks; c = next, turn ^= 1) {
       asm volatile("" : "+r"(sb), "+r"(tb));
+      next = list.next(p, P.chunks, lane);
       asm volatile("bar.sync 2, 544;" ::: "memory");
       tc::tc_fence_after();
-      const bool wide = ctl.wide;
-      if (!wide && tc::elect_one()) {
+      if (tc::elect_one()) {
         const uint64_t ad = tc::smem_desc_sw128(sb + PK_A, 128, 1024), bd = tc::smem_desc_sw128(sb + PK_KI, 128, 1024);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
@@ -119,8 +122,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         commit(0);
       }
       __syncwarp();
-      if (c + (int)gridDim.x < P.chunks) load(c + gridDim.x, turn ^ 1);
-      if (wide) continue;
+      if (next < P.chunks) load(next, turn ^ 1);
       float* xat = p.xat + (int64_t)c * (3 * 64 * 64);
       asm volatile("bar.sync 3, 544;" ::: "memory");
       if (tc::elect_one()) tc::bulk_s2g(xat + 4096, sb + PK_AT, kTile);
@@ -168,9 +170,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       tc::tc_fence_before();
       asm volatile("bar.arrive %0, 544;" ::"r"(id) : "memory");
     };
-    uint32_t ph = 0, turn = 0;   // narrow chunks, chunks so far
+    uint32_t ph = 0;
 #pragma unroll 1
-    for (int c = blockIdx.x; c < P.chunks; c += gridDim.x, turn ^= 1) {
+    for (int c = list.next(p, P.chunks, lane); c < P.chunks; c = list.next(p, P.chunks, lane), ph ^= 1) {
       int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       asm volatile("" : "+r"(warp), "+r"(lane));
       warp = __shfl_sync(0xffffffffu, warp, 0);
@@ -183,9 +185,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
       };
       float4 G[4];
       float rk[4], rq[4];
-      wait_at(ctl.full, turn);
+      wait_at(ctl.full, ph);
       {
-        float up = 0.f;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -196,12 +197,10 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           } else {
             x = *reinterpret_cast<const float4*>(smem + PK_G + (4 * warp + r) * 512 + lane * 16);
           }
-          up = fmaxf(up, fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
           acc.x += x.x * kLog2e; acc.y += x.y * kLog2e; acc.z += x.z * kLog2e; acc.w += x.w * kLog2e;
           G[r] = acc;
         }
         *reinterpret_cast<float4*>(smem + PK_TOT + warp * 512 + lane * 16) = acc;
-        if (__any_sync(0xffffffffu, up > 0.f) && lane == 0) ctl.rise[turn] = 1;
         float ss[8];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -233,7 +232,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
       }
       workers_sync();
-      bool wide;
       {
         float4 pre = make_float4(0.f, 0.f, 0.f, 0.f), run = pre;
 #pragma unroll
@@ -244,19 +242,13 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
-        const bool whole = run.x >= -kWideKda && run.y >= -kWideKda && run.z >= -kWideKda && run.w >= -kWideKda;   // (not for NaN)
-        wide = ctl.rise[turn] || !__all_sync(0xffffffffu, whole);
         if (warp == 0) {
           const float4 e = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
           *reinterpret_cast<float4*>(ctl.el + 4 * lane) = e;
           *reinterpret_cast<float4*>(p.el + (int64_t)c * 128 + 4 * lane) = e;
-          if (lane == 0) {
-            ctl.wide = wide;
-            xat[kXWide] = wide ? 1.f : 0.f;
-          }
         }
       }
-      if (!wide) {
+      {
         // ---- the tiles -----------------------------------------------------------------------------------------------------------------------
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -285,11 +277,6 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
       }
       hand_over(2);
-      if (wide) {   // pre_kernel's
-        workers_sync();   // (the next chunk's totals wait for the readers of these)
-        if (tid == 0) ctl.rise[turn] = 0;
-        continue;
-      }
       const int qd = warp & 3, cg = warp >> 2, row = 32 * qd + lane;   // this thread's row of a product and sixteen of its columns from 16 cg
       const uint32_t ta = tb + ((uint32_t)(32 * qd) << 16) + 16 * cg;
       // ---- X (rows 0 .. 63), A (rows 64 ..) --------------------------------------------------------------------------------------------------------
@@ -328,7 +315,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         hand_over(3);
       }
       // ---- T in place (eight warps), then T - I and T diag(beta) as tiles ----------------------------------------------------------------------------
-      const float* beta = ctl.beta[turn];
+      const float* beta = ctl.beta[ph];
       if (warp < 8) sm100::block_inverse_64(sX, beta, sX, 32 * warp + lane);
       workers_sync();
       {
@@ -408,9 +395,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           }
         }
       }
-      ph ^= 1;
-      workers_sync();   // e^{G_L} has been read
-      if (tid == 0) ctl.rise[turn] = 0;
+      workers_sync();   // e^{G_L} and the rows' totals have been read
     }
   }
   tc::tc_fence_before();

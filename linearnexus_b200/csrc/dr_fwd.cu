@@ -10,8 +10,8 @@ cudaError_t launch_chunk_fused_packed(const FwdParams& p, const SeqTable& seqs, 
   return sm100::launch_chunk_packed(p, seqs, stream);
 }
 int64_t split_workspace_bytes(int64_t units, int T) { return kda::workspace_bytes(units, T); }
-cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra) {
-  return kda::launch_chunk(p, workspace, stream, launches, after_intra);
+cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra, WideMarks marks) {
+  return kda::launch_chunk(p, workspace, stream, launches, after_intra, marks);
 }
 cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream) {
   return kda::launch_chunk_packed(p, seqs, workspace, stream);

@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "dr_chunk_sm100.cuh"
+#include "dr_launch.h"
 #include "dr_mma.cuh"
 
 namespace dr {
@@ -140,6 +141,7 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
 struct IntraParams {
   CUtensorMap tq, tk, tg;   // panels of q and k; g as boxes of 64 rows
   FwdParams p;
+  WideMarks marks;
   uint8_t* ws;
   int chunks, use_tma;
 };
@@ -383,10 +385,10 @@ static __device__ __noinline__ void general_products_call(uint8_t* smem, const f
 
 // Whether the chunk takes the general products, the same in every warp: a channel decays by more than 2^64 (run: this lane's four, whole chunk;
 // not a number counts), or a log decay is positive -- sums of others fall from row to row, so that e^G and e^{-G} of every row lie within 2^64.
-__device__ __forceinline__ bool any_wide(float4 run, const int (&up)[8]) {
+__device__ __forceinline__ bool any_wide(float4 run, const int (&up)[8], float limit = 64.f) {
   const int4 a = *reinterpret_cast<const int4*>(up), b = *reinterpret_cast<const int4*>(up + 4);
   const bool rise = (a.x | a.y | a.z | a.w) | (b.x | b.y | b.z | b.w);
-  return __any_sync(0xffffffffu, rise || !(run.x >= -64.f && run.y >= -64.f && run.z >= -64.f && run.w >= -64.f));
+  return __any_sync(0xffffffffu, rise || !(run.x >= -limit && run.y >= -limit && run.z >= -limit && run.w >= -limit));
 }
 
 template <class Params>
@@ -413,6 +415,8 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
   __syncthreads();
   tc::tc_fence_after();
   pdl_entry();
+  if constexpr (!kPacked)
+    if (P.marks.at && blockIdx.x == 0 && tid < 3) P.marks.at[2 + tid] = 0.f;
   const uint32_t tb = ctl.tmem_base, sb = tc::smem_u32(smem);
   auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
     const uint32_t at = tc::smem_u32(&bar);
@@ -638,6 +642,10 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
             run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
           }
           *reinterpret_cast<float4*>(P.ws + x.rec * WS_REC + WS_EGL + 16 * lane) = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
+          if (!kPacked && P.marks.at) {
+            const bool mark = any_wide(run, ctl.up, P.marks.limit);
+            if (lane == 0) P.marks.at[x.rec * P.marks.stride] = mark ? 1.f : 0.f;
+          }
         } else {
           sync();
         }
@@ -1826,9 +1834,10 @@ inline cudaError_t launch_pair(IP& I, SP& S, const FwdParams& p, void* workspace
   return launch_pdl(state_kernel<SP>, dim3((unsigned)units), dim3(kStateThreads), ST_TOTAL, stream, S);
 }
 
-inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra) {
+inline cudaError_t launch_chunk(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra, WideMarks marks) {
   IntraParams I;
   StateParams S;
+  I.marks = marks;
   const int64_t units = (int64_t)p.map.B * p.map.H;
   *launches = 2;
   return launch_pair(I, S, p, workspace, units * ((p.map.T + kC - 1) / kC), units, stream, after_intra);
@@ -1839,6 +1848,7 @@ inline cudaError_t launch_chunk_packed(const FwdParams& p, const SeqTable& seqs,
   IntraPackedParams I;
   StatePackedParams S;
   I.seqs = S.seqs = seqs;
+  I.marks = WideMarks{};
   return launch_pair(I, S, p, workspace, (int64_t)seqs.chunks * p.map.H, (int64_t)seqs.n * p.map.H, stream);
 }
 

@@ -13,7 +13,11 @@ cudaError_t launch_chunk_fused_packed(const FwdParams& p, const SeqTable& seqs, 
 // two-kernel forward (any variant); the workspace holds split_workspace_bytes
 int64_t split_workspace_bytes(int64_t units, int T);
 // after_intra: recorded on `stream` between the two kernels (null: not)
-cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra = nullptr);
+// Where the chunk-parallel pass notes (1 or 0) of each chunk whether a channel decays by more than `limit` (log2) or a log decay is positive; at[2 .. 4]
+// are set to zero.
+struct WideMarks { float* at; int64_t stride; float limit; };
+cudaError_t launch_chunk_split(const FwdParams& p, void* workspace, cudaStream_t stream, int* launches, cudaEvent_t after_intra = nullptr,
+                               WideMarks marks = WideMarks{});
 cudaError_t launch_chunk_split_packed(const FwdParams& p, const SeqTable& seqs, void* workspace, cudaStream_t stream);
 
 // forward in transition form (two kernels; K = V = 64 or 128); bf16_tensor: the bf16-operand kernels (dr_fwd.cu; bf16 q, k, v,

@@ -349,3 +349,16 @@ def test_kda_gradients_of_uneven_inputs():
 def test_kda_local_passes_at_the_line(decay):
     """The line between the two kinds of chunks: 2^40 (27.726 nats) in any channel."""
     test_kda_local_passes(1, 2, 2, 703, True, True, decay)
+
+
+def test_kda_wide_chunks_are_taken_one_by_one():
+    """160 chunks past the line, two of 162 are not: every CTA of the kernels with 16-row blocks takes several of the list."""
+    T = 1665
+    inp = O.make_inputs("kda", 3, 2, T, 128, 128, seed=8, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["g"] *= 20.0
+    inp["g"][0, 0, 64:192] = -0.01
+    gen = torch.Generator().manual_seed(9)
+    got, ref = _kda_backward(inp, torch.randn(3, 2, T, 128, generator=gen).bfloat16(), torch.randn(3, 2, 128, 128, generator=gen) * 0.1)
+    for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):   # bf16 operands in the forward's checkpoints: 1e-2 of the largest
+        err = ((got[name].double() - ref[name]).norm() / ref[name].norm()).item()
+        assert err <= 1e-2, (name, err)
