@@ -86,6 +86,15 @@ int validate_fwd_ptrs(const DrDesc* d, const void* q, const void* k, const void*
   return DR_OK;
 }
 
+// the two-kernel form (chunk-parallel intra pass + tcgen05 state pass over a workspace)
+bool split_eligible(const DrDesc* d) {
+  return d->K == 128 && d->V == 128 && d->chunk == 64 && d->qkv_dtype == DR_BF16;
+}
+// Rows of per-channel decays are read four channels at a time at the tensor-core shape.
+bool bwd_g_aligned(const DrDesc* d, const void* g) {
+  return d->variant != DR_KDA || !split_eligible(d) || (reinterpret_cast<uintptr_t>(g) & (d->g_dtype == DR_BF16 ? 7u : 15u)) == 0;
+}
+
 // SM count of the current device (cached per host thread and device)
 int sm_count() {
   thread_local int cached_dev = -1, cached = 0;
@@ -104,10 +113,6 @@ bool tcgen05_eligible(const DrDesc* d) {
          (d->variant == DR_DELTA || d->g_dtype == DR_F32);
 }
 
-// the two-kernel form (chunk-parallel intra pass + tcgen05 state pass over a workspace)
-bool split_eligible(const DrDesc* d) {
-  return d->K == 128 && d->V == 128 && d->chunk == 64 && d->qkv_dtype == DR_BF16;
-}
 // AUTO for a shape without a tensor-core kernel: the register-resident token recurrence.  It is the same function of
 // the inputs as the chunk form, does fewer multiply-adds (4 K V per token against the chunk form's 6CK + 4CV + 6KV
 // over C) and measured 4-11x faster than the fp32 chunk kernel on every fp32 shape tried; DR_PATH_FP32 still asks for
@@ -441,6 +446,7 @@ int dr_chunk_bwd(const DrDesc* d, const void* q, const void* k, const void* v, c
   if (!q || !k || !v || !beta || !d_o || !dq || !dk || !dv || !dbeta) return DR_ERR_NULL;
   if (d->variant == DR_DELTA ? (g != nullptr || dg != nullptr) : (g == nullptr || dg == nullptr))
     return DR_ERR_VARIANT;
+  if (!bwd_g_aligned(d, g)) return DR_ERR_ALIGN;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv) || !aligned16(workspace))
     return DR_ERR_ALIGN;
@@ -514,6 +520,7 @@ int dr_chunk_bwd_saved(const DrDesc* d, const void* q, const void* k, const void
   if (!q || !k || !v || !beta || !d_o || !dq || !dk || !dv || !dbeta) return DR_ERR_NULL;
   if (d->variant == DR_DELTA ? (g != nullptr || dg != nullptr) : (g == nullptr || dg == nullptr))
     return DR_ERR_VARIANT;
+  if (!bwd_g_aligned(d, g)) return DR_ERR_ALIGN;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv) || !aligned16(workspace))
     return DR_ERR_ALIGN;
@@ -566,6 +573,7 @@ int dr_chunk_bwd_static(const DrDesc* d, const void* q, const void* k, const voi
   if (!q || !k || !v || !beta || !d_o || !dq || !dk || !dv || !dbeta) return DR_ERR_NULL;
   if (d->variant == DR_DELTA ? (g != nullptr || dg != nullptr) : (g == nullptr || dg == nullptr))
     return DR_ERR_VARIANT;
+  if (!bwd_g_aligned(d, g)) return DR_ERR_ALIGN;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv))
     return DR_ERR_ALIGN;

@@ -1405,7 +1405,7 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
   } else if (split) {
     int n2 = 0;
     // its records lie where dS1 of every chunk will be written (bwdc::Params)
-    const bwdc::Params b = bwdc::make_params(d, workspace);
+    const bwdc::Params b = bwdc::make_params(d, workspace, g);
     e = launch_chunk_split(f, b.ds, stream, &n2, forked, WideMarks{b.xat + bwdc::kXWide, 3 * 64 * 64, bwdc::kWideKda});
     *launches += n2;
     if (want_pre && !forked && after && e == cudaSuccess) e = pre(stream);
@@ -1429,10 +1429,10 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
 cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, const void* v, const void* g,
                                       const float* beta, const void* d_o, const float* d_hT, void* dq, void* dk,
                                       void* dv, float* dbeta, float* dg, float* dh0, void* workspace,
-                                      int32_t* status, cudaStream_t stream, int* launches) {
+                                      int32_t* status, cudaStream_t stream, int* launches, const void* g_forward) {
   const int C = d->chunk, K = d->K, V = d->V;
   if (bwdc::eligible(d)) {
-    bwdc::Params p = bwdc::make_params(d, workspace);
+    bwdc::Params p = bwdc::make_params(d, workspace, g_forward);
     p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta; p.d_o = d_o; p.d_hT = d_hT;
     p.dq = dq; p.dk = dk; p.dv = dv; p.dbeta = dbeta; p.dg = dg; p.dh0 = dh0;
     const int64_t units = (int64_t)d->B * d->H;
@@ -1516,7 +1516,7 @@ cudaError_t launch_bwd(const DrDesc* d, const void* q, const void* k, const void
   cudaError_t e = launch_bwd_forward(d, q, k, v, g, beta, h0, nullptr, nullptr, workspace, status, stream, launches,
                                      own_stream);
   if (e != cudaSuccess) return e;
-  return launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace, status, stream, launches);
+  return launch_bwd_adjoint(d, q, k, v, g, beta, d_o, d_hT, dq, dk, dv, dbeta, dg, dh0, workspace, status, stream, launches, g);
 }
 
 }  // namespace dr

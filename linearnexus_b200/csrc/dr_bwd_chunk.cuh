@@ -51,7 +51,7 @@ struct Params {
   float* part;          // grouped heads: dq^ [units][N*64][128], then dk^ (over nf)
   SeqMap map;
   int N, variant, g_dt, l2norm;
-  int few;              // KDA: pre_kernel and local_kernel take every chunk (see kFewKda)
+  int few;              // KDA: pre_kernel and local_kernel take every chunk, one per CTA (see kFewKda, make_params)
   float scale;
 };
 
@@ -1483,11 +1483,14 @@ inline int64_t workspace_bytes(const DrDesc* d) {
   const int64_t N = (d->T + kC - 1) / kC;
   return (int64_t)d->B * d->H * N * kFloats * 4;
 }
-inline Params make_params(const DrDesc* d, void* workspace) {
+inline bool tma_base(const void* g) { return (reinterpret_cast<uintptr_t>(g) & 15u) == 0; }
+// Rows of per-channel decays where a tensor map does not take them (bf16 at eight bytes) leave every chunk to the kernels that load by themselves.  g: the
+// decays that the pre-pass reads.
+inline Params make_params(const DrDesc* d, void* workspace, const void* g) {
   Params p{};
   p.N = (d->T + kC - 1) / kC;
   const int64_t nc = (int64_t)d->B * d->H * p.N;
-  p.few = nc <= kFewKda && p.N <= kFewLength;
+  p.few = (nc <= kFewKda && p.N <= kFewLength) || (d->variant == DR_KDA && !tma_base(g));
   float* f = reinterpret_cast<float*>(workspace);
   p.ckpt = f; f += nc * kCkpt;
   p.nf = reinterpret_cast<float4*>(f); p.part = f; f += nc * kNf;
@@ -1545,41 +1548,45 @@ inline cudaError_t launch_pre_t(const Params& p, int64_t units, int32_t* status,
     if (e != cudaSuccess) return e;
   }
   ++*launches;
-  return launch_pdl(pre_kernel<KDA>, dim3((unsigned)(!KDA || chunks < 2 * sms ? chunks : 2 * sms)), dim3(kPreThreads), pre_smem<KDA>(), stream, p, (int)chunks);
+  return launch_pdl(pre_kernel<KDA>, dim3((unsigned)(!KDA || p.few || chunks < 2 * sms ? chunks : 2 * sms)), dim3(kPreThreads), pre_smem<KDA>(), stream, p, (int)chunks);
 }
 inline cudaError_t launch_pre(const DrDesc* d, const void* q, const void* k, const void* g, const float* beta, void* workspace,
                               int32_t* status, cudaStream_t stream, bool beside, int* launches) {
-  Params p = make_params(d, workspace);
+  Params p = make_params(d, workspace, g);
   p.q = q; p.k = k; p.g = g; p.beta = beta;
   const int64_t units = (int64_t)d->B * d->H;
   return d->variant == DR_KDA ? launch_pre_t<true>(p, units, status, stream, beside, launches) : launch_pre_t<false>(p, units, status, stream, beside, launches);
 }
 template <bool KDA>
-inline cudaError_t launch_adjoint_t(const Params& p, int64_t units, int32_t* status, cudaStream_t stream) {
+inline cudaError_t launch_adjoint_t(Params p, int64_t units, int32_t* status, cudaStream_t stream) {
   int sms = 0;
   cudaError_t e = set_attributes<KDA>(&sms);
   if (e != cudaSuccess) return e;
   const int64_t chunks = units * p.N;
+  // the forward that this is the adjoint of had its decays where a tensor map takes them: so that its chunks are read as it left them, they move to Y's
+  // place once that has been read (32 KB a chunk, 64 rows of 256 bytes)
+  const void* const g_from = KDA && !p.few && !tma_base(p.g) ? p.g : nullptr;
+  if (g_from) p.g = p.yf;
   const dim3 grid((unsigned)(chunks < sms ? chunks : sms));
   LocalParams lp;
   lp.p = p; lp.chunks = (int)chunks; lp.status = status;
   lp.n_tok = units * p.map.T; lp.n_part = 2 * chunks * (kC * kD);
   const SeqMap& m = p.map;
   auto panels = [&](CUtensorMap* t, const void* base, int heads) { return sm100::make_panel_map(t, base, m.B, heads, m.T, m.bthd != 0); };
-  if (!panels(&lp.to, p.d_o, m.H)) return cudaErrorInvalidValue;
+  // (every map before the first launch: a call that fails leaves nothing half done)
+  if (!panels(&lp.to, p.d_o, m.H) || !panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
+      !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
+    return cudaErrorInvalidValue;
+  if (KDA && !p.few && !sm100::make_output_map(&lp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4)) return cudaErrorInvalidValue;
   ChainParams c;
   c.p = p;
   c.status = status;
   c.to = lp.to;
   e = launch_pdl(chain_kernel<KDA>, dim3((unsigned)(units * (kD / kChCols))), dim3(ch_threads<KDA>()), ch_smem<KDA>(), stream, c);
+  if (g_from && e == cudaSuccess) e = cudaMemcpyAsync(p.yf, g_from, (size_t)units * m.T * kD * 2, cudaMemcpyDeviceToDevice, stream);
   if (e != cudaSuccess) return e;
-  if (!panels(&lp.tq, p.q, m.Hq) || !panels(&lp.tk, p.k, m.Hq) || !panels(&lp.tv, p.v, m.H) || !panels(&lp.tdq, p.dq, m.Hq) ||
-      !panels(&lp.tdk, p.dk, m.Hq) || !panels(&lp.tdv, p.dv, m.H))
-    return cudaErrorInvalidValue;
   if constexpr (KDA) {
-    if (p.few) return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
-    if (!sm100::make_output_map(&lp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
-      return cudaErrorInvalidValue;
+    if (p.few) return launch_pdl(local_kernel, dim3((unsigned)chunks), dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);
     e = launch_pdl(local_sm100_kda_kernel, grid, dim3(kLkThreads), LK_TOTAL, stream, lp);
     if (e != cudaSuccess) return e;
     return launch_pdl(local_kernel, grid, dim3(kLoThreads), LoSmem::kTotal, stream, p, (int)chunks);

@@ -34,7 +34,8 @@ cudaError_t launch_bwd_forward(const DrDesc* d, const void* q, const void* k, co
                                int* launches, bool own_stream = true);
 cudaError_t launch_bwd_adjoint(const DrDesc* d, const void* q, const void* k, const void* v, const void* g, const float* beta,
                                const void* d_o, const float* d_hT, void* dq, void* dk, void* dv, float* dbeta, float* dg,
-                               float* dh0, void* workspace, int32_t* status, cudaStream_t stream, int* launches);
+                               float* dh0, void* workspace, int32_t* status, cudaStream_t stream, int* launches,
+                               const void* g_forward = nullptr);   // the decays that launch_bwd_forward had (null: aligned ones, see dr_chunk_fwd_saving)
 // forward recomputation + adjoint
 cudaError_t launch_bwd(const DrDesc* d, const void* q, const void* k, const void* v, const void* g, const float* beta,
                        const float* h0, const void* d_o, const float* d_hT, void* dq, void* dk, void* dv, float* dbeta, float* dg,

@@ -362,3 +362,27 @@ def test_kda_wide_chunks_are_taken_one_by_one():
     for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):   # bf16 operands in the forward's checkpoints: 1e-2 of the largest
         err = ((got[name].double() - ref[name]).norm() / ref[name].norm()).item()
         assert err <= 1e-2, (name, err)
+
+
+@pytest.mark.parametrize("T,H", [(130, 2), (640, 8), (641, 2), (705, 27)])
+def test_kda_decays_at_eight_bytes(T, H):
+    """bf16 log decays whose rows start at eight bytes, where a tensor map does not take them: on both sides of the line of few chunks (ten a sequence, 80 in
+    all) as with aligned ones, and from a forward that had them aligned.  Against float64: the bf16 budget of the other tests."""
+    inp = O.make_inputs("kda", 1, H, T, 128, 128, seed=T, io_dtype=torch.bfloat16, h0_std=0.02, g_dtype=torch.bfloat16)
+    gen = torch.Generator().manual_seed(T)
+    do, dhT = torch.randn(1, H, T, 128, generator=gen).bfloat16().cuda(), (torch.randn(1, H, 128, 128, generator=gen) * 0.1).cuda()
+    cu = {n: x.cuda() for n, x in inp.items()}
+    apart = torch.empty(cu["g"].numel() + 4, dtype=torch.bfloat16, device="cuda")[4:].view_as(cu["g"]).copy_(cu["g"])
+    assert apart.data_ptr() % 16 == 8 and apart.is_contiguous()
+    def run(g, saved=None):
+        r = ops.chunk_backward("kda", cu["q"], cu["k"], cu["v"], g, cu["beta"], do, initial_state=cu["h0"], d_final_state=dhT, chunk_size=64, saved=saved)
+        L.check_device_status()
+        return r
+    ref = O.delta_rule_grads("kda", *(cu[n].double() for n in ("q", "k", "v", "g", "beta")), cu["h0"].double(), do.double(), dhT.double())
+    want, got = run(cu["g"]), run(apart)
+    save = lambda: ops.chunk_forward_saving("kda", cu["q"], cu["k"], cu["v"], cu["g"], cu["beta"], cu["h0"], chunk_size=64)[2]
+    kept, again = run(cu["g"], save()), run(apart, save())
+    for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):
+        for x in (want, got, kept, again):
+            assert (x[name].double() - ref[name]).norm() <= 1e-2 * ref[name].norm(), name
+        assert torch.equal(kept[name], again[name]), name
