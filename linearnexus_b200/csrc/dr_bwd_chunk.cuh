@@ -1483,14 +1483,31 @@ inline int64_t workspace_bytes(const DrDesc* d) {
   const int64_t N = (d->T + kC - 1) / kC;
   return (int64_t)d->B * d->H * N * kFloats * 4;
 }
+// Whether local_sm100_kda_kernel was given the registers that its split counts on (another compiler may give it others, and the split waits for good then).
+inline bool split_fits(int regs) { return regs == kLkRegs; }
+inline cudaError_t local_kernel_fits(bool* fits) {
+  thread_local int attr_dev = -1;
+  thread_local bool known = false;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && attr_dev != dev) {
+    cudaFuncAttributes at{};
+    e = cudaFuncGetAttributes(&at, local_sm100_kda_kernel);
+    if (e == cudaSuccess) { known = split_fits(at.numRegs); attr_dev = dev; }
+  }
+  *fits = known;
+  return e;
+}
 inline bool tma_base(const void* g) { return (reinterpret_cast<uintptr_t>(g) & 15u) == 0; }
-// Rows of per-channel decays where a tensor map does not take them (bf16 at eight bytes) leave every chunk to the kernels that load by themselves.  g: the
-// decays that the pre-pass reads.
+// Rows of per-channel decays where a tensor map does not take them (bf16 at eight bytes), and a local_sm100_kda_kernel that was not given its registers, leave
+// every chunk to the kernels with 16-row blocks.  g: the decays that the pre-pass reads.
 inline Params make_params(const DrDesc* d, void* workspace, const void* g) {
   Params p{};
+  bool fits = true;
+  if (d->variant == DR_KDA && local_kernel_fits(&fits) != cudaSuccess) fits = false;   // (the launches report what is wrong)
   p.N = (d->T + kC - 1) / kC;
   const int64_t nc = (int64_t)d->B * d->H * p.N;
-  p.few = (nc <= kFewKda && p.N <= kFewLength) || (d->variant == DR_KDA && !tma_base(g));
+  p.few = (nc <= kFewKda && p.N <= kFewLength) || (d->variant == DR_KDA && !(tma_base(g) && fits));
   float* f = reinterpret_cast<float*>(workspace);
   p.ckpt = f; f += nc * kCkpt;
   p.nf = reinterpret_cast<float4*>(f); p.part = f; f += nc * kNf;
@@ -1514,9 +1531,6 @@ inline cudaError_t set_attributes(int* sms = nullptr) {
       e = KDA ? cudaFuncSetAttribute(local_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_TOTAL)
               : cudaFuncSetAttribute(local_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_TOTAL);
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LoSmem::kTotal);
-    cudaFuncAttributes at{};
-    if (KDA && e == cudaSuccess) e = cudaFuncGetAttributes(&at, local_sm100_kda_kernel);
-    if (KDA && e == cudaSuccess && at.numRegs != kLkRegs) e = cudaErrorInvalidConfiguration;   // its register split counts on them
     if (KDA && e == cudaSuccess) e = cudaFuncSetAttribute(pre_sm100_kda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_TOTAL);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(chain_kernel<KDA>, cudaFuncAttributeMaxDynamicSharedMemorySize, ch_smem<KDA>());

@@ -59,7 +59,7 @@ struct LkCtl {
 constexpr int LK_TOTAL = LK_CTL + sizeof(LkCtl);
 static_assert(LK_TOTAL <= 232448 && LK_CTL % 16 == 0 && offsetof(LkCtl, beta) % 16 == 0 && offsetof(LkSums, f) % 16 == 0, "shared memory");
 // Registers: 640 threads of 96 (the fifth warp group is the issuing warp and three that leave); the workers take 104, the issuing group keeps 64, which
-// adds up to what the block was launched with (launch_adjoint_t asks for 96).  With 544 threads and 96 each 1.4 % slower, spills 308 bytes against 136.
+// adds up to what the block was launched with (make_params sees to it that it was 96).  With 544 threads and 96 each 1.4 % slower, spills 308 bytes against 136.
 constexpr int kLkThreads = 640, kLkRegs = 96, kLkWorkerRegs = 104, kLkIssueRegs = 64;
 static_assert(512 * kLkWorkerRegs + 128 * kLkIssueRegs <= kLkThreads * kLkRegs, "the split waits for good otherwise");
 static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(const __grid_constant__ LocalParams P) {
