@@ -823,6 +823,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
   }
   tc::tc_fence_before();
   __syncthreads();
+  sm100::settle(ctl.abort);
   if (warp == 8) tc::tmem_dealloc(tb, 128);
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
@@ -1248,6 +1249,7 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
   }
   tc::tc_fence_before();
   __syncthreads();
+  sm100::settle(ctl.abort);
   if (warp == 0) tc::tmem_dealloc(tb, 256);
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
@@ -1571,6 +1573,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   }
   tc::tc_fence_before();
   __syncthreads();
+  sm100::settle(ctl.abort);
   if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
 }
 
@@ -1641,6 +1644,7 @@ __global__ void __launch_bounds__(kTrThreads<STAGED>, 1) trans_state_kernel(cons
       if (lane >= 3 && lane < 11) tc::bulk_g2s(dst + L::kZ + (lane - 3) * NT * 512, P.zf + ((c * 8 + lane - 3) * 16 + v0 / 8) * 32, NT * 512, bar);
       if (lane >= 11 && lane < 15) tc::bulk_g2s(dst + L::kO + (lane - 11) * NT * 512, P.of + ((c * 4 + lane - 11) * 16 + v0 / 8) * 32, NT * 512, bar);
     }
+    sm100::settle(ctl.abort);
     return;
   }
   uint4 a[8];
