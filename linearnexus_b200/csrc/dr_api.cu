@@ -311,7 +311,8 @@ int dr_chunk_fwd_varlen(const DrDesc* d, const void* q, const void* k, const voi
       if (workspace && !aligned16(workspace)) return DR_ERR_ALIGN;
       cap = workspace ? (int64_t)workspace_bytes / dr::split_workspace_bytes(d->H, 64) : 0;
     }
-    const dr::FwdParams p = make_fwd(&da, q, k, v, g, beta, h0, o, hT, status_dev);
+    dr::FwdParams p = make_fwd(&da, q, k, v, g, beta, h0, o, hT, status_dev);
+    p.n_state *= n_seqs;   // (one state per sequence; index checks of the debug build)
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     std::vector<int32_t> order(n_seqs);   // longest first
     for (int i = 0; i < n_seqs; ++i) order[i] = i;

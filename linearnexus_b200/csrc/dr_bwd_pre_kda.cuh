@@ -228,7 +228,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         }
         if (!(lane & 3)) {
           const int i = 4 * warp + ((lane >> 2) & 3);
-          xat[kXNorms + ((lane < 16 ? 2 : 0) + (i >> 5)) * kXNormRow + (i & 31)] = m;
+          const int place = kXNorms + ((lane < 16 ? 2 : 0) + (i >> 5)) * kXNormRow + (i & 31);
+          if (in_bounds(P.status, (int64_t)c * (3 * 64 * 64) + place, (int64_t)P.chunks * (3 * 64 * 64))) xat[place] = m;
         }
       }
       workers_sync();
@@ -245,7 +246,7 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         if (warp == 0) {
           const float4 e = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
           *reinterpret_cast<float4*>(ctl.el + 4 * lane) = e;
-          *reinterpret_cast<float4*>(p.el + (int64_t)c * 128 + 4 * lane) = e;
+          if (in_bounds_run(P.status, (int64_t)c * 128 + 4 * lane, 4, (int64_t)P.chunks * 128)) *reinterpret_cast<float4*>(p.el + (int64_t)c * 128 + 4 * lane) = e;
         }
       }
       {
@@ -296,7 +297,8 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
           for (int e = 0; e < 4; ++e) {
             const float4 y = make_float4(x[4 * e], x[4 * e + 1], x[4 * e + 2], x[4 * e + 3]);
             *reinterpret_cast<float4*>(sX + i * LDT + 16 * cg + 4 * e) = y;
-            if (cg <= (i >> 4)) reinterpret_cast<float4*>(xat)[(4 * cg + e) * 64 + i] = y;   // columns in fours
+            if (cg <= (i >> 4) && in_bounds(P.status, (int64_t)c * (3 * 64 * 16) + (4 * cg + e) * 64 + i, (int64_t)P.chunks * (3 * 64 * 16)))
+              reinterpret_cast<float4*>(xat)[(4 * cg + e) * 64 + i] = y;   // columns in fours
           }
         }
         workers_sync();   // (X for the inverse)
@@ -370,17 +372,18 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
         uint32_t u[16];
         tc::tmem_ld16(ta + tWA, u);
         tc::tc_wait_ld();
-        float4* dst = p.yf + (int64_t)c * kHalf4 + (row >> 3) * 64 + 2 * cg * 8 + (row & 7);   // see store_f32
+        const int64_t dst = (int64_t)c * kHalf4 + (row >> 3) * 64 + 2 * cg * 8 + (row & 7);   // see store_f32
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          dst[(e & 1) * (kHalf4 / 2) + (e >> 1) * 8] = make_float4(y[4 * e] - __uint_as_float(u[4 * e]), y[4 * e + 1] - __uint_as_float(u[4 * e + 1]),
+          if (in_bounds(P.status, dst + (e & 1) * (kHalf4 / 2) + (e >> 1) * 8, (int64_t)P.chunks * kHalf4))
+            p.yf[dst + (e & 1) * (kHalf4 / 2) + (e >> 1) * 8] = make_float4(y[4 * e] - __uint_as_float(u[4 * e]), y[4 * e + 1] - __uint_as_float(u[4 * e + 1]),
                                                                    y[4 * e + 2] - __uint_as_float(u[4 * e + 2]), y[4 * e + 3] - __uint_as_float(u[4 * e + 3]));
       }
       // ---- N = -W^T Ki diag(e^{G_L}): thread = 32 columns -----------------------------------------------------------------------------------------
       {
         wait_at(ctl.bar[3], ph);
         tc::tc_fence_after();
-        float4* dst = p.nf + (2 * (int64_t)c + (cg >> 1)) * kHalf4 + (row >> 3) * 64 + 4 * (cg & 1) * 8 + (row & 7);
+        const int64_t dst = (2 * (int64_t)c + (cg >> 1)) * kHalf4 + (row >> 3) * 64 + 4 * (cg & 1) * 8 + (row & 7);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           uint32_t u[16];
@@ -389,8 +392,9 @@ static __global__ void __launch_bounds__(kLtThreads, 1) pre_sm100_kda_kernel(con
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float4 d = *reinterpret_cast<const float4*>(ctl.el + 32 * cg + 16 * x + 4 * e);
-            dst[(e & 1) * (kHalf4 / 2) + (2 * x + (e >> 1)) * 8] =
-                make_float4(-__uint_as_float(u[4 * e]) * d.x, -__uint_as_float(u[4 * e + 1]) * d.y, -__uint_as_float(u[4 * e + 2]) * d.z,
+            const int64_t at = dst + (e & 1) * (kHalf4 / 2) + (2 * x + (e >> 1)) * 8;
+            if (in_bounds(P.status, at, 2 * (int64_t)P.chunks * kHalf4))
+              p.nf[at] = make_float4(-__uint_as_float(u[4 * e]) * d.x, -__uint_as_float(u[4 * e + 1]) * d.y, -__uint_as_float(u[4 * e + 2]) * d.z,
                             -__uint_as_float(u[4 * e + 3]) * d.w);
           }
         }

@@ -155,6 +155,7 @@ struct IntraTransParams {
   uint4 *nf, *yf;     // [chunks][8 | 4 row tiles][8 k-steps][32 lanes]: A operands of m16n8k16
   float4 *zf, *of;    // [chunks][8 | 4 row tiles][16 column tiles][32 lanes]: addends
   float* el;          // [chunks][128] e^{G_L}
+  int64_t chunks;
 };
 
 // eight channels of one row: scale q^ e^G, k^ e^{G_L - G}, k^ e^G (G of the row and of the chunk's last row in log2 units)
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
         const At x = place(c);
         const int rows = x.rows - 8 * warp, tok = x.tok + 8 * warp;
         const int64_t s_tok = p.map.tok(1), s_at = p.map.base(x.b, x.h, 1) + tok * s_tok;
-        const float bt = lane < 8 && lane < rows ? p.beta[s_at + lane * s_tok] : 0.f;
+        const float bt = lane < 8 && lane < rows && in_bounds(p.status, s_at + lane * s_tok, p.n_tok) ? p.beta[s_at + lane * s_tok] : 0.f;
         if (P.use_tma) {
           wait_bar(ctl.full, ph);
           if (p.g_dt == DR_BF16) {
@@ -587,11 +588,11 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           for (int r = 0; r < 8; ++r) {
             uint2 q = make_uint2(0u, 0u), k = q;
             float y[4] = {0.f, 0.f, 0.f, 0.f};
-            if (r < rows) {
+            if (r < rows && in_bounds_run(p.status, at + r * st, 4, p.n_qk)) {
               q = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + at + r * st);
               k = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + at + r * st);
-              if (p.variant == DR_KDA) ld4(p.g, g_at + r * gst, p.g_dt, y);
-              else if (p.variant == DR_GATED) y[0] = y[1] = y[2] = y[3] = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
+              if (p.variant == DR_KDA && in_bounds_run(p.status, g_at + r * gst, 4, p.n_gk)) ld4(p.g, g_at + r * gst, p.g_dt, y);
+              else if (p.variant == DR_GATED && in_bounds(p.status, s_at + r * s_tok, p.n_tok)) y[0] = y[1] = y[2] = y[3] = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
             }
             G[r] = make_float4(y[0], y[1], y[2], y[3]);
             *entry(IS_Q, r) = q;
@@ -641,10 +642,11 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
             const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
             run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
           }
-          *reinterpret_cast<float4*>(P.ws + x.rec * WS_REC + WS_EGL + 16 * lane) = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
+          if (in_bounds(p.status, x.rec, P.chunks))
+            *reinterpret_cast<float4*>(P.ws + x.rec * WS_REC + WS_EGL + 16 * lane) = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
           if (!kPacked && P.marks.at) {
             const bool mark = any_wide(run, ctl.up, P.marks.limit);
-            if (lane == 0) P.marks.at[x.rec * P.marks.stride] = mark ? 1.f : 0.f;
+            if (lane == 0 && in_bounds(p.status, x.rec, P.chunks)) P.marks.at[x.rec * P.marks.stride] = mark ? 1.f : 0.f;
           }
         } else {
           sync();
@@ -913,11 +915,11 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
   float4 G[8];
   {
     const int64_t s_tok = p.map.tok(1), s_at = p.map.base(b, h, 1) + (t0 + 8 * warp) * s_tok;
-    const float bt = lane < 8 && lane < rows ? p.beta[s_at + lane * s_tok] : 0.f;
+    const float bt = lane < 8 && lane < rows && in_bounds(p.status, s_at + lane * s_tok, p.n_tok) ? p.beta[s_at + lane * s_tok] : 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       float x = 0.f;
-      if (p.variant == DR_GATED && r < rows) x = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
+      if (p.variant == DR_GATED && r < rows && in_bounds(p.status, s_at + r * s_tok, p.n_tok)) x = ld_elem(p.g, s_at + r * s_tok, p.g_dt);
       G[r] = make_float4(x, x, x, x);
     }
     wait_bar(ctl.full, 0);
@@ -982,7 +984,7 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
     }
     wide = any_wide(run, ctl.up);
     el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
-    if (warp == 0) *reinterpret_cast<float4*>(P.el + chunk * kD + 4 * lane) = el;
+    if (warp == 0 && in_bounds_run(p.status, chunk * kD + 4 * lane, 4, P.chunks * kD)) *reinterpret_cast<float4*>(P.el + chunk * kD + 4 * lane) = el;
 #pragma unroll
     for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
   }
@@ -1194,14 +1196,17 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
       uint32_t w[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) w[e] = mma::pack(-__uint_as_float(x[8 * ks + 2 * e]), -__uint_as_float(x[8 * ks + 2 * e + 1]));
-      P.nf[((chunk * 8 + mt) * 8 + 4 * hf + ks) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+      const int64_t at = ((chunk * 8 + mt) * 8 + 4 * hf + ks) * 32 + lane;
+      if (in_bounds(p.status, at, P.chunks * (8 * 8 * 32))) P.nf[at] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 128 + 64 * hf, x);
     tc::tc_wait_ld();
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-      P.zf[((chunk * 8 + mt) * 16 + 8 * hf + nt) * 32 + lane] =
-          make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+    for (int nt = 0; nt < 8; ++nt) {
+      const int64_t at = ((chunk * 8 + mt) * 16 + 8 * hf + nt) * 32 + lane;
+      if (in_bounds(p.status, at, P.chunks * (8 * 16 * 32)))
+        P.zf[at] = make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+    }
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -1237,14 +1242,17 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
           const int i = 8 * ks + 4 * (e >> 1) + 2 * (e & 1);
           w[e] = mma::pack(q.x - __uint_as_float(x[i]), q.y - __uint_as_float(x[i + 1]));
         }
-        P.yf[((chunk * 4 + mt) * 8 + 4 * hf + ks) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+        const int64_t at = ((chunk * 4 + mt) * 8 + 4 * hf + ks) * 32 + lane;
+        if (in_bounds(p.status, at, P.chunks * (4 * 8 * 32))) P.yf[at] = make_uint4(w[0], w[1], w[2], w[3]);
       }
       tc::tmem_ld_frag(ta + ((uint32_t)(16 * m) << 16) + 128 + 64 * hf, x);
       tc::tc_wait_ld();
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-        P.of[((chunk * 4 + mt) * 16 + 8 * hf + nt) * 32 + lane] =
-            make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+      for (int nt = 0; nt < 8; ++nt) {
+        const int64_t at = ((chunk * 4 + mt) * 16 + 8 * hf + nt) * 32 + lane;
+        if (in_bounds(p.status, at, P.chunks * (4 * 16 * 32)))
+          P.of[at] = make_float4(__uint_as_float(x[4 * nt]), __uint_as_float(x[4 * nt + 1]), __uint_as_float(x[4 * nt + 2]), __uint_as_float(x[4 * nt + 3]));
+      }
     }
   }
   tc::tc_fence_before();
@@ -1794,6 +1802,7 @@ inline cudaError_t launch_trans(const FwdParams& p, void* workspace, int sms, cu
   P.zf = reinterpret_cast<float4*>(w); w += nc * kTrZ;
   P.of = reinterpret_cast<float4*>(w); w += nc * kTrO;
   P.el = reinterpret_cast<float*>(w);
+  P.chunks = nc;
   const SeqMap& m = p.map;
   if (!sm100::make_panel_map(&P.tq, p.q, m.B, m.Hq, m.T, m.bthd != 0) || !sm100::make_panel_map(&P.tk, p.k, m.B, m.Hq, m.T, m.bthd != 0) ||
       !sm100::make_panel_map(&P.tv, p.v, m.B, m.H, m.T, m.bthd != 0) ||
