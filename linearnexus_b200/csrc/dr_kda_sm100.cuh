@@ -17,7 +17,7 @@
 //
 // Per-channel decay cannot be folded into row/column factors of a plain K K^T product the way a scalar
 // decay can, and e^{-G} alone overflows for strong decay.  A chunk that decays by at most 2^64 takes one product of decayed rows (see
-// intra_kernel); for the others, and in the transition form, the chunk-local products use 16-row
+// intra_kernel); for the others the chunk-local products use 16-row
 // sub-blocks: rows of sub-block bi against earlier columns are the bf16 tensor-core product of
 // x_i e^{G_i - G_n}  and  k_j e^{G_n - G_j}  with n the first row of bi, so both exponents are <= 0; the four diagonal
 // 16x16 blocks use the same form while their decay range stays below 2^64 and are summed exactly in fp32 otherwise.
@@ -36,8 +36,6 @@ namespace dr {
 namespace kda {
 
 using sm100::LDT;
-using sm100::RBS;
-using sm100::A_RBS;
 
 constexpr int kC = 64, kD = 128;
 constexpr int kThreads = 256;
@@ -56,11 +54,9 @@ constexpr int WS_ASKED = 82432;
 static_assert(WS_REC <= WS_ASKED, "records fit what callers provide");
 inline int64_t workspace_bytes(int64_t units, int T) { return units * ((T + kC - 1) / kC) * (int64_t)WS_ASKED; }
 
-// ---- the general products and the transition form's pass ----------------------------------------------------------
-// Shared memory is kept under half an SM's worth so that two CTAs are resident and one chunk's latency
-// (global loads, the serial prefix sum, the barriers between phases) hides behind the other's work.  The
-// inputs stay as raw bf16 with their l2-norm factors on the side, and the decayed bf16 operands of the
-// tensor-core products are formed in registers from them (no scaled copies in shared memory).
+// ---- the general products, for chunks past the line -----------------------------------------------------------------
+// The inputs lie as raw bf16 with their l2-norm factors on the side, and the decayed bf16 operands of the tensor-core products are formed in
+// registers from them (no scaled copies in shared memory).
 constexpr int LDF = 136;   // row stride (floats) of G: the products read pairs of eight rows without bank conflicts
 constexpr int LDH = 136;   // row stride (bf16) of the raw q, k rows and of the W staging tile
 constexpr int LDQ = 72;    // row stride (bf16) of A_qk
@@ -85,8 +81,6 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // packed pairs: one instruction per two products
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
@@ -118,23 +112,11 @@ __device__ __forceinline__ void ld4(const void* p, int64_t i, int dt, float (&x)
   }
 }
 
-// 16-byte piece number `piece` of a [64][128] tile in core-matrix order -> (row, first column)
-__device__ __forceinline__ void piece128(int piece, int& row, int& col) {
-  row = (piece >> 7) * 8 + (piece & 7);
-  col = ((piece >> 3) & 15) * 8;
-}
-// same for a [64][64] tile
+// 16-byte piece number `piece` of a [64][64] tile in core-matrix order -> (row, first column)
 __device__ __forceinline__ void piece64(int piece, int& row, int& col) {
   row = (piece >> 6) * 8 + (piece & 7);
   col = ((piece >> 3) & 7) * 8;
 }
-__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
-  uint4 u;
-  u.x = tc::pack_bf16(x[0], x[1]); u.y = tc::pack_bf16(x[2], x[3]);
-  u.z = tc::pack_bf16(x[4], x[5]); u.w = tc::pack_bf16(x[6], x[7]);
-  return u;
-}
-
 
 // Kernel parameters of the intra pass; a packed batch adds the table of its sequences (p then describes the packed
 // arrays: B = 1, T = all tokens, token-major).
