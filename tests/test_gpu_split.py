@@ -150,3 +150,19 @@ def test_kda_decays_that_climb_back(path, T):
     ro, rS = _truth("kda", inp)
     for h in range(2):
         assert _rel(o[:, h], ro[:, h]) <= BF16_TOL and _rel(hT[:, h], rS[:, h]) <= BF16_TOL
+
+
+@pytest.mark.parametrize("path", ["split", "transition"])
+def test_kda_one_token(path):
+    """A sequence of one token: q and k enter their product as they are, which then rounds to bf16 once, 2^-8 (v = beta = 1 and no state, so that the
+    output is the product; float32 sums of 128 terms add 2^-21 of their sizes)."""
+    inp = O.make_inputs("kda", 1, 512, 1, 128, 128, seed=31, io_dtype=torch.bfloat16)
+    inp["v"] = torch.ones_like(inp["v"])
+    inp["beta"] = torch.ones_like(inp["beta"])
+    inp["h0"] = None
+    o, hT = _run("kda", inp, path)
+    ro, rS = _truth("kda", inp)
+    q, k = (inp[x].double().abs() for x in ("q", "k"))
+    sizes = (q * k).sum(-1, keepdim=True) / (q.norm(dim=-1) * k.norm(dim=-1))[..., None] * 128 ** -0.5
+    assert ((o.double().cpu() - ro).abs() <= 2.0 ** -8 * ro.abs() + 2.0 ** -20 * sizes).all()
+    assert _rel(hT, rS) <= BF16_TOL
