@@ -133,3 +133,17 @@ def test_transition_form_bf16_wide_chunks(variant, T):
     ro, rS = ref(*(inp[x].double() for x in ("q", "k", "v", "g", "beta")), initial_state=inp["h0"].double(), compute_dtype=torch.float64)
     for got, want in ((o, ro), (hT, rS)):
         assert (got.double().cpu() - want).abs().max() <= 2e-2 * want.abs().max()
+
+
+@pytest.mark.parametrize("H,T,path", [(13, 2117, "chunk_transition"), (18, 2117, "chunk_transition"), (19, 2117, "chunk_split_tcgen05"), (18, 1024, "chunk_split_tcgen05")])
+def test_kda_route_by_sequences_and_chunks(H, T, path):
+    """KDA in bf16: up to 18 sequences of more than 16 chunks take the transition form, past 32 chunks as before them; the others the two-kernel form.  The budget
+    of the other bf16 forwards: 2e-2 of the largest value."""
+    inp = O.make_inputs("kda", 1, H, T, 128, 128, seed=H, io_dtype=torch.bfloat16, h0_std=0.02)
+    cu = {k: v.cuda() for k, v in inp.items()}
+    o, hT = L.kda_chunkwise(cu["q"], cu["k"], cu["v"], cu["g"], cu["beta"], initial_state=cu["h0"], chunk_size=64)
+    assert _lib.last_path() == path
+    L.check_device_status()
+    ro, rS = O.kda_recurrent(*(cu[x].double() for x in ("q", "k", "v", "g", "beta")), initial_state=cu["h0"].double(), compute_dtype=torch.float64)
+    for got, want in ((o, ro), (hT, rS)):
+        assert (got.double().cpu() - want.cpu()).abs().max() <= 2e-2 * want.cpu().abs().max()
