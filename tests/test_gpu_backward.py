@@ -386,3 +386,21 @@ def test_kda_decays_at_eight_bytes(T, H):
         for x in (want, got, kept, again):
             assert (x[name].double() - ref[name]).norm() <= 1e-2 * ref[name].norm(), name
         assert torch.equal(kept[name], again[name]), name
+
+
+def test_kda_two_backwards_behind_one_forward():
+    """The saved workspace serves a second adjoint, chunks past the line included (they are taken from a list, which begins anew)."""
+    T = 705
+    inp = O.make_inputs("kda", 1, 2, T, 128, 128, seed=12, io_dtype=torch.bfloat16, h0_std=0.02)
+    inp["g"][:, 1] *= 20.0
+    cu = {n: x.cuda() for n, x in inp.items()}
+    gen = torch.Generator().manual_seed(13)
+    do, dhT = torch.randn(1, 2, T, 128, generator=gen).bfloat16().cuda(), (torch.randn(1, 2, 128, 128, generator=gen) * 0.1).cuda()
+    args = [cu[n] for n in ("q", "k", "v", "g", "beta")]
+    saved = ops.chunk_forward_saving("kda", *args, cu["h0"], chunk_size=64)[2]
+    first, second = (ops.chunk_backward("kda", *args, do, initial_state=cu["h0"], d_final_state=dhT, chunk_size=64, saved=saved) for _ in range(2))
+    L.check_device_status()
+    ref = O.delta_rule_grads("kda", *(x.double() for x in args), cu["h0"].double(), do.double(), dhT.double())
+    for name in ("dq", "dk", "dv", "dbeta", "dg", "dh0"):
+        assert torch.equal(first[name], second[name]), name
+        assert (first[name].double() - ref[name]).norm() <= 1e-2 * ref[name].norm(), name
