@@ -339,7 +339,8 @@ __device__ __forceinline__ void general_products(const float* sG, const __nv_bfl
 // waiting for rows, 2.0 K prefix sums and norms, 2.0 K tiles, 1.4 K for the product, 3.8 K inverse, 0.9 K for W^T; issue slots 51 %.  With loads by
 // the warps into registers a chunk ahead they wait 6 K cycles for room in what the tiles leave of the L1 (690 us).  Fewer instructions in the
 // prefix sums and norms (packed adds, one barrier with a vote) made it 2 to 7 % slower.  Output error against float64 (2-norm, 64 heads,
-// T=500): 4.3e-3 -> 3.8e-3, one rounding per operand instead of two; T=1: 2.7e-3 -> 3.0e-3, where the general form's factors are 1.
+// T=500): 4.3e-3 -> 3.8e-3, one rounding per operand instead of two; without any decay, where the general form's factors are 1,
+// 2.9e-3 -> 3.4e-3.  A sequence of one token (2.8e-3 -> 4.1e-3) keeps the general form.
 constexpr int kIntraThreads = kThreads + 32;
 constexpr int IS_A = 0, IS_Q = 8192, IS_B = 16384, IS_PANEL = 24576;   // k^ e^G | q^ e^G | Kd of 64 channels, then of the other 64; A and B by turns
 constexpr int IS_G = 2 * IS_PANEL;         // log decay as it arrives [64][128]
