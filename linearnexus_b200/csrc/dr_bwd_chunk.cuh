@@ -631,6 +631,8 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
   __syncthreads();
   tc::tc_fence_after();
   pdl_entry();
+  // local_kernel, behind the next kernel, takes its chunks from the first on, also in a second backward behind one forward
+  if (KDA && blockIdx.x == 0 && tid == 0) reinterpret_cast<int*>(p.xat + kXCounts)[2] = 0;
   const uint32_t tbase = ctl.tmem_base, sbase = tc::smem_u32(smem);
   auto wait_bar = [&](uint64_t& bar, uint32_t parity) {
     const uint32_t at = tc::smem_u32(&bar);

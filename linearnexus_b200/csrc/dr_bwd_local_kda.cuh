@@ -103,8 +103,6 @@ static __global__ void __launch_bounds__(kLkThreads, 1) local_sm100_kda_kernel(c
   constexpr uint32_t tKr1 = 0, tKc1 = 64, tA = 128, tM = 256, tQ2 = 128, tKr2 = 256, tKc2 = 320, tKc3 = 384;
   ChunkList list;
   list.start(p, P.chunks, lane);
-  // local_kernel, which follows, takes its chunks from the first on, also in a second backward behind one forward
-  if (blockIdx.x == 0 && tid == 0) reinterpret_cast<int*>(p.xat + kXCounts)[2] = 0;
 
   if (warp >= 16) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLkIssueRegs));

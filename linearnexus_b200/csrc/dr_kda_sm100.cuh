@@ -353,7 +353,7 @@ struct IntraCtl {
   uint64_t bar[2], full, free;
   alignas(16) int up[8];   // per warp: a log decay of its rows is positive
   uint32_t tmem_base;
-  int wide, abort;
+  int wide, one, abort;
 };
 constexpr int IS_TOTAL = IS_BETA + sizeof(IntraCtl);
 // the arrays of the general products: A_kk where the inverse expects it
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
     sm100::wait_inline(at, parity, &ctl.abort, at - tc::smem_u32(&ctl), warp == 8);
   };
   // chunk number -> batch, head, first token, rows of it that exist, number of its record
-  struct At { int b, h, tok, rows, T; int64_t rec; };
+  struct At { int b, h, tok, rows, one; int64_t rec; };   // one: packed, a sequence of one token
   auto place = [&](int c) -> At {
     At x;
     if constexpr (kPacked) {   // heads outermost in the grid, innermost but one in the records
@@ -419,16 +419,16 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
         const int mid = (lo + hi + 1) >> 1;
         if (P.seqs.first[mid] <= c) lo = mid; else hi = mid - 1;
       }
-      const int n = c - P.seqs.first[lo], T = x.T = P.seqs.len[lo];
+      const int n = c - P.seqs.first[lo], T = P.seqs.len[lo];
       x.tok = P.seqs.start[lo] + n * kC;
       x.rows = min(kC, T - n * kC);
+      x.one = T == 1;
       x.rec = (int64_t)P.seqs.first[lo] * p.map.H + (int64_t)x.h * ((T + kC - 1) / kC) + n;
     } else {
       const int nchunks = (p.map.T + kC - 1) / kC, unit = c / nchunks, n = c - unit * nchunks;
       x.b = unit / p.map.H; x.h = unit - x.b * p.map.H;
       x.tok = n * kC;
-      x.T = p.map.T;
-      x.rows = min(kC, x.T - n * kC);
+      x.rows = min(kC, p.map.T - n * kC);
       x.rec = c;
     }
     return x;
@@ -541,10 +541,8 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
       auto entry = [&](int base, int r) { return reinterpret_cast<uint2*>(smem + base + own + r * 128 + ((piece ^ r) << 4)); };
       // ---- the warp's rows, prefix sums over them, norm factors ------------------------------------------------------------------------
       float4 G[8];
-      bool one;   // a sequence of one token: the 16-row form's operands are its rows as they are, which the tiles' rounding is worse than
       {
         const At x = place(c);
-        one = x.T == 1;
         const int rows = x.rows - 8 * warp, tok = x.tok + 8 * warp;
         const int64_t s_tok = p.map.tok(1), s_at = p.map.base(x.b, x.h, 1) + tok * s_tok;
         const float bt = lane < 8 && lane < rows && in_bounds(p.status, s_at + lane * s_tok, p.n_tok) ? p.beta[s_at + lane * s_tok] : 0.f;
@@ -620,6 +618,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           (lane < 16 ? ctl.rq : ctl.rk)[8 * warp + ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
         }
         if (lane < 8) ctl.beta[8 * warp + lane] = bt;
+        if (kPacked && tid == 0) ctl.one = x.one;
         if (warp == 0) {   // (the record's tail; its address is not worth keeping)
           sync();
           float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -648,7 +647,8 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
           run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
         }
-        wide = any_wide(run, ctl.up) || one;
+        // (a sequence of one token: the 16-row form's operands are its rows as they are, which the tiles' rounding is worse than)
+        wide = any_wide(run, ctl.up) || (kPacked ? ctl.one != 0 : p.map.T == 1);
         el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
 #pragma unroll
         for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
