@@ -866,8 +866,10 @@ __global__ void __launch_bounds__(ch_threads<KDA>(), 1) chain_kernel(const __gri
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 0) tc::tmem_dealloc(tbase, kTmem);
+  if (warp == 0) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tbase, kTmem);
+  }
   if (tid == 0) sm100::report_wait(P.status, ctl.abort);
 }
 

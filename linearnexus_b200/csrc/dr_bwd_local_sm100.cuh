@@ -676,8 +676,10 @@ static __global__ void __launch_bounds__(kLtThreads, 1) local_sm100_kernel(const
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 16) tc::tmem_dealloc(tb, 512);
+  if (warp == 16) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tb, 512);
+  }
   if (tid == 0) sm100::report_wait(P.status, ctl.abort);
 }
 

@@ -730,8 +730,10 @@ __global__ void __launch_bounds__(kThreads, 1) chunk_sm100_kernel(const __grid_c
   }
   tc::tc_fence_before();
   __syncthreads();
-  settle(ctl.abort);
-  if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
+  if (warp == 0) {
+    settle(ctl.abort);
+    tc::tmem_dealloc(tbase, TM_COLS);
+  }
 }
 
 template <class Params>

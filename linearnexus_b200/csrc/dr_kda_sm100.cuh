@@ -353,7 +353,7 @@ struct IntraCtl {
   uint64_t bar[2], full, free;
   alignas(16) int up[8];   // per warp: a log decay of its rows is positive
   uint32_t tmem_base;
-  int wide, one, abort;
+  int wide, abort;
 };
 constexpr int IS_TOTAL = IS_BETA + sizeof(IntraCtl);
 // the arrays of the general products: A_kk where the inverse expects it
@@ -584,7 +584,8 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           }
         }
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        float up = 0.f;
+        // (a sequence of one token counts as a rise: the 16-row form's operands are its rows as they are, which the tiles' rounding is worse than)
+        float up = (kPacked ? x.one : p.map.T == 1) ? 1.f : 0.f;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           up = fmaxf(up, fmaxf(fmaxf(G[r].x, G[r].y), fmaxf(G[r].z, G[r].w)));
@@ -618,7 +619,6 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           (lane < 16 ? ctl.rq : ctl.rk)[8 * warp + ((lane >> 1) & 7)] = p.l2norm ? top / (sqrtf(ss[0]) + 1e-6f) : top;
         }
         if (lane < 8) ctl.beta[8 * warp + lane] = bt;
-        if (kPacked && tid == 0) ctl.one = x.one;
         if (warp == 0) {   // (the record's tail; its address is not worth keeping)
           sync();
           float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -647,8 +647,7 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
           const float4 y = *reinterpret_cast<const float4*>(smem + IS_TOT + s * 512 + lane * 16);
           run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
         }
-        // (a sequence of one token: the 16-row form's operands are its rows as they are, which the tiles' rounding is worse than)
-        wide = any_wide(run, ctl.up) || (kPacked ? ctl.one != 0 : p.map.T == 1);
+        wide = any_wide(run, ctl.up);
         el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
 #pragma unroll
         for (int r = 0; r < 8; ++r) G[r] = make_float4(G[r].x + pre.x, G[r].y + pre.y, G[r].z + pre.z, G[r].w + pre.w);
@@ -811,8 +810,10 @@ __global__ void __launch_bounds__(kIntraThreads, 2) intra_kernel(const __grid_co
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 8) tc::tmem_dealloc(tb, 128);
+  if (warp == 8) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tb, 128);
+  }
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
@@ -922,7 +923,7 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
       }
     }
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float up = 0.f;
+    float up = T == 1 ? 1.f : 0.f;   // (see intra_kernel)
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       up = fmaxf(up, fmaxf(fmaxf(G[r].x, G[r].y), fmaxf(G[r].z, G[r].w)));
@@ -968,7 +969,7 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
       const float4 y = *reinterpret_cast<const float4*>(smem + IT_TOT + s * 512 + lane * 16);
       run.x += y.x; run.y += y.y; run.z += y.z; run.w += y.w;
     }
-    wide = any_wide(run, ctl.up) || T == 1;   // (see intra_kernel)
+    wide = any_wide(run, ctl.up);
     el = make_float4(ex2(run.x), ex2(run.y), ex2(run.z), ex2(run.w));
     if (warp == 0 && in_bounds_run(p.status, chunk * kD + 4 * lane, 4, P.chunks * kD)) *reinterpret_cast<float4*>(P.el + chunk * kD + 4 * lane) = el;
 #pragma unroll
@@ -1243,8 +1244,10 @@ static __global__ void __launch_bounds__(kThreads, 2) intra_trans_kernel(const _
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 0) tc::tmem_dealloc(tb, 256);
+  if (warp == 0) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tb, 256);
+  }
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
@@ -1567,8 +1570,10 @@ __global__ void __launch_bounds__(kStateThreads, 1) state_kernel(const __grid_co
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 0) tc::tmem_dealloc(tbase, TM_COLS);
+  if (warp == 0) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tbase, TM_COLS);
+  }
 }
 
 // ---- few sequences: the state pass in transition form ------------------------------------------------------------------------

@@ -63,8 +63,8 @@ __device__ __forceinline__ void wait_inline(uint32_t bar, uint32_t parity, int* 
   }
 }
 // Behind a wait that gave up a CTA runs on without waiting, in step with its named barriers, and starts the copies and products that are left.  Before it ends
-// or frees its tensor memory it gives them the time to finish (every thread, behind the last barrier; in a kernel whose copying warp ends by
-// itself, that warp): they take microseconds, this is two milliseconds.  One read of shared memory per CTA; with the flag asked before every copy
+// or frees its tensor memory it gives them the time to finish (the warp that frees it, behind the last barrier, which keeps the CTA; in a kernel whose copying
+// warp ends by itself, that warp): they take microseconds, this is two milliseconds.  One read of shared memory per CTA; with the flag asked before every copy
 // the kernels were 0.5 to 3 % slower, with each thread's own note of it in a register up to 9 %.
 __device__ __forceinline__ void settle(const int& abort_flag) {
   if (*(volatile const int*)&abort_flag == 0) return;

@@ -603,8 +603,10 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_sm100_kernel(const __grid_con
   }
   tc::tc_fence_before();
   __syncthreads();
-  sm100::settle(ctl.abort);
-  if (warp == 0) tc::tmem_dealloc(tbase, 512);
+  if (warp == 0) {
+    sm100::settle(ctl.abort);
+    tc::tmem_dealloc(tbase, 512);
+  }
   if (tid == 0) sm100::report_wait(p.status, ctl.abort);
 }
 
