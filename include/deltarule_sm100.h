@@ -217,6 +217,7 @@ int dr_chunk_bwd_saved(const DrDesc* desc, const void* q, const void* k, const v
  * Inputs: the forward inputs, d_o [like o, desc->qkv_dtype] and d_hT (float32 [B,H,K,V] or
  * null).  Outputs: dq,dk [like q], dv [like v] in desc->qkv_dtype; dbeta float32 [like beta];
  * dg float32 [like g] (null for DR_DELTA); dh0 float32 [B,H,K,V] or null.
+ * Activations and their gradients start at 16 bytes; KDA's g at the tensor-core shape (K = V = 128, chunk 64, bf16) at 16 bytes in float32, at 8 in bf16.
  */
 int dr_chunk_bwd(const DrDesc* desc, const void* q, const void* k, const void* v, const void* g,
                  const float* beta, const float* h0, const void* d_o, const float* d_hT, void* dq,
