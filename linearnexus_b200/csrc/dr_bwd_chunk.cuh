@@ -1559,9 +1559,9 @@ inline cudaError_t launch_pre_t(const Params& p, int64_t units, int32_t* status,
         !sm100::make_output_map(&pp.tg, const_cast<void*>(p.g), m, p.g_dt == DR_BF16 ? 2 : 4))
       return cudaErrorInvalidValue;
     ++*launches;
-    // Beside the forward's state pass, whose CTAs keep an SM each for 2.65 us a chunk (this kernel: 10.4 us), its own CTAs keep off those SMs while
-    // there are few of them: those that wait for one would do their share of the chunks behind it.  32 sequences of 64 chunks: 185 us on
-    // 116 SMs, by the same figures 170 + 144 on all of them; level at about 59 sequences.
+    // Beside the forward's state pass, whose CTAs keep an SM each for 2.65 us a chunk (this kernel: 9 us), its own CTAs keep off those SMs while
+    // there are few of them: those that wait for one would do their share of the chunks behind it.  32 sequences of 64 chunks: 160 us on
+    // 116 SMs, by the same figures 170 + 125 on all of them; level at about 61 sequences.
     const int64_t free = beside && 5 * units <= 2 * sms ? sms - units : sms;
     e = launch_pdl(pre_sm100_kda_kernel, dim3((unsigned)(chunks < free ? chunks : free)), dim3(kLtThreads), PK_TOTAL, stream, pp);
     if (e != cudaSuccess) return e;

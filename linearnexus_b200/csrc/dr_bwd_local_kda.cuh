@@ -16,8 +16,8 @@
 // and k^ dk^ are equal and stay out of dG -- behind strong decays they are most of both.
 // The factors of a term multiply to decays of at most 1, so what each of them may reach is a matter of exponents alone.  P and Px, whose products
 // are the ones with a factor of more than 1 behind them, come with a power of two that brings their largest entries to 2^40, so that gradients as small as
-// float32 has them pass.  A chunk may decay by 2^40 in any channel (kWideKda).  The pre-pass says of each chunk whether it does, and local_kernel, which refers the decays to
-// 16-row blocks, takes the others.
+// float32 has them pass.  A chunk may decay by 2^40 in any channel (kWideKda).  The forward marks those that
+// decay by more, and local_kernel, which refers the decays to 16-row blocks, takes them.
 //
 // A thread of an epilogue owns one channel and sixteen tokens, and so does the one that forms Kg, Kd and Qg: G stays in its registers.  The
 // three are formed twice, before the products of 1 and of 4: beside the states (128 KB) there is no room to keep them.
@@ -27,7 +27,7 @@
 // shared memory costs an L2 access: with g, q, X, A and T by loads of the warps 71 K cycles, with everything the compiler would keep over the
 // chunk loop in spilled registers 57 K; hence the opaque thread index, and G parked in tensor memory.
 // Errors against float64 at one chunk (2-norm, 82 sequences; in brackets pre_kernel and local_kernel): dbeta 4.9e-5 (4.9e-5), dg 4.6e-5 (4.6e-5), dh0
-// 1.5e-5 (1.5e-5): T's tf32 merges decide; dq, dk, dv 1.7e-3 (bf16 rounding).  Where T is near I (beta a twentieth) 4.6e-6 (2.7e-6), 4.4e-6 (2.0e-6),
+// 1.5e-5 (1.5e-5): T's tf32 merges decide; dq, dk, dv 1.7e-3 (bf16 rounding).  Where T is near I (beta a twentieth) 5.2e-6 (2.7e-6), 4.7e-6 (2.0e-6),
 // 2.2e-6 (1.3e-6).
 #pragma once
 

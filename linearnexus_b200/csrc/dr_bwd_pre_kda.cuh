@@ -14,7 +14,7 @@
 // channels of them; a thread of an epilogue one row of a product.  Rows arrive by TMA a chunk ahead, as soon as the tiles of the chunk before
 // are formed; A and T leave by bulk copies, X, N and Y as whole 128-byte lines.
 //
-// What bounds it: B=2, T=4096, H=16 (2048 chunks): 185 us on 116 SMs, 20 K cycles per chunk, where pre_kernel takes 266 us on 148 (65 K for two chunks at a
+// What bounds it: B=2, T=4096, H=16 (2048 chunks): 160 us on 116 SMs, 17 K cycles per chunk, where pre_kernel takes 266 us on 148 (65 K for two chunks at a
 // time: 15 K loads, 23 K for X and A, 18 K for W, Y and N).  The phases of one chunk follow each other,
 // sixteen warps on one: the tensor pipe has 4 K cycles of work.  210 KB of memory per chunk are 8 K cycles at the copy rate on all SMs.
 // Gradients against float64 as with pre_kernel (T's tf32 merges decide): see dr_bwd_local_kda.cuh.
